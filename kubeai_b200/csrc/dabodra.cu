@@ -78,7 +78,7 @@ struct LayerWeights {
   void* sh_down = nullptr;  // [width, sff]
   GemmPlan p_in, p_out, p_shin, p_shdown;
   GroupedPlan g_egu, g_edown;
-  CUtensorMap xg_h, xg_act;                                    // the grouped form's views of the sorted rows and of the hidden rows
+  GroupedX xg_h, xg_act;                                    // the grouped form's views of the sorted rows and of the hidden rows
   CUtensorMap xm_out[kGemmNumBlockN], xm_shact[kGemmNumBlockN];
   bool tc_in = false, tc_out = false, tc_shin = false, tc_shdown = false, tc_experts = false;
   // gate and up rows in alternating blocks of 64, so that one GEMM tile holds both and its epilogue can join them
@@ -389,6 +389,7 @@ class Dabodra : public Model {
     auto plan = [&](GemmPlan* p, const void* Wm, int N, int K) {
       if (N % 8 || K % 8 || gemm_plan_init(p, Wm, N, K, K, gemm_ws, gemm_counters, env.sms)) return false;
       p->ws_bytes = ws_bytes;
+      p->error = kernel_error;
       return true;
     };
     auto plan_maps = [&](GemmPlan* p, CUtensorMap* m, const void* X, const void* Wm, int N, int K) {
@@ -415,7 +416,7 @@ class Dabodra : public Model {
       }
       if (s.mlp && grouped)
         w.tc_experts = !gemm_grouped_plan(&w.g_egu, w.e_gu, s.experts, 2 * s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
-                       !gemm_grouped_x_map(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_map(&w.xg_act, eact, moe_cap, s.ff);
+                       !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);
     }
     return 0;
   }
@@ -576,9 +577,9 @@ class Dabodra : public Model {
   // The grouped kernel on one matrix: whole 256 x 256 tiles, the accumulator drained under the next tile.
   bool takes_whole(bool tc, int T) const { return tc && T > 256 && whole; }
   int run_whole(const GemmPlan& plan, const CUtensorMap* xm, bool glu, void* Y, int ldy, int T) {
-    GroupedPlan g;
-    g.tm_w = plan.tm_w; g.experts = 1; g.N = plan.N; g.K = plan.K;      // the same boxes: 128 rows x 64 columns on both sides
-    return gemm_grouped_run(g, xm[gemm_block_n_index(256)], nullptr, Y, ldy, glu, env.sms, kernel_error, env.stream, T);
+    const GroupedOut o = {Y, ldy, glu ? GROUPED_GATED : GROUPED_PLAIN, nullptr, INFINITY, 1.f, 0.f};
+    const int bn = gemm_block_n_for(T);
+    return gemm_whole_run(plan, xm[gemm_block_n_index(bn)], bn, T, o, env.stream);
   }
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
     if (takes_whole(tc, T)) return run_whole(plan, xm, false, Y, N, T);
@@ -712,12 +713,15 @@ class Dabodra : public Model {
       // the inputs in expert-sorted order, then one grouped GEMM per matrix; the row counts stay on the device
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
       if (w.il_e) {
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, expert_rows, eact, s.ff, true, env.sms, kernel_error, st));
+        const GroupedOut o = {eact, s.ff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
       } else {
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, expert_rows, egu, 2 * s.ff, false, env.sms, kernel_error, st));
+        const GroupedOut o = {egu, 2 * s.ff};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
         KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f));
       }
-      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, expert_rows, edown16, W, false, env.sms, kernel_error, st));
+      const GroupedOut o = {edown16, W};
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, o, env.sms, kernel_error, st));
       KRN("moe_combine", moe_combine_add(edown16, DT_BF16, pair_pos, topw, shared_out, nullptr, 0, fo, dt, T, s.top, W, st));
       return rc;
     }

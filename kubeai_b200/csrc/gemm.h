@@ -22,6 +22,7 @@ struct GemmPlan {
   int table_segs[65];  // partial segments the ntt-th schedule produces
   int max_ntt;
   size_t ws_bytes;     // capacity of ws
+  int* error;          // optional, host-visible: a kernel whose wait ran out leaves a mark here (gemm_grouped.cu)
 };
 
 // variant 2 (default): CTA-pair kernel (gemm2_tcgen05.cu); variant 1: single-CTA kernel (gemm_tcgen05.cu)
@@ -66,18 +67,39 @@ int gemm_run_deferred(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, v
 struct Gemm2Epi;
 int gemm2_run_fused(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int T, const Gemm2Epi& e, cudaStream_t st);
 // Grouped form (gemm_grouped.cu): the rows of every expert, sorted by expert, times that expert's matrix in one launch.  W: the
-// experts' [N, K] matrices stacked; expert_rows: device [experts][2] = {first row of X, rows}.  out[r, n] (leading dimension
-// ldo); with glu the rows of every matrix alternate in blocks of 64 gate rows and their 64 up rows (N % 128 == 0) and
-// out[r, i] = silu(gate_i) * up_i, i < N / 2.  N, K, ldo: multiples of 8.  error (optional, host-visible int): set to 1 when a
-// wait inside the kernel ran out.  expert_rows may be null for one matrix and `rows` rows: a plain product in whole tiles.
+// experts' [N, K] matrices stacked; expert_rows: device [experts][2] = {first row of X, rows}; most_rows: what no expert's row
+// count exceeds (the step's tokens).  N, K: multiples of 8, ldy of 8 (fp32 output: 4).  error (optional, host-visible int): set
+// to 1 when a wait inside the kernel ran out.
 struct GroupedPlan {
   CUtensorMap tm_w;
   int experts, N, K;
 };
+constexpr int kGroupedBoxes = 4;
+struct GroupedX { CUtensorMap box[kGroupedBoxes]; };
+// What happens to a sum s[r, n]: GROUPED_PLAIN / _RELU2 / _XIELU (a_pos = p0, a_neg = p1): y[r, n] = bf16(act(s + bias[n]));
+// GROUPED_F32: y[r, n] = s + bias[n] in fp32; GROUPED_GATED (limit p0, slope p1, up offset p2; the rows of every matrix alternate
+// in blocks of 64 gate rows and their 64 up rows, N % 128 == 0): g, u = bf16(s) of the two rows, y[r, i] = bf16(min(g, p0)
+// sigmoid(p1 min(g, p0)) (clamp(u, -p0, p0) + p2)), i < N / 2.  bias (optional): one matrix only.
+enum GroupedEpi { GROUPED_PLAIN = 0, GROUPED_RELU2, GROUPED_XIELU, GROUPED_F32, GROUPED_GATED };
+struct GroupedOut {
+  void* y;
+  int ldy;
+  int epi = GROUPED_PLAIN;
+  const float* bias = nullptr;
+  float p0 = 0.f, p1 = 0.f, p2 = 0.f;
+};
 int gemm_grouped_plan(GroupedPlan* p, const void* W, int experts, int N, int K);
-int gemm_grouped_x_map(CUtensorMap* tm, const void* X, int rows, int K);
-int gemm_grouped_run(const GroupedPlan& p, const CUtensorMap& tm_x, const int* expert_rows, void* out, int ldo, bool glu, int sms, int* error,
-                     cudaStream_t st, int rows = 0);
+int gemm_grouped_x_maps(GroupedX* x, const void* X, int rows, int K);
+int gemm_grouped_run(const GroupedPlan& p, const GroupedX& x, int most_rows, const int* expert_rows, const GroupedOut& o, int sms, int* error, cudaStream_t st);
+// The same kernel on one matrix and `rows` rows, in whole tiles of 256 weight rows x up to 256 rows; few tiles are cut along K.
+// tm_x: the activation's map for token-tile size block_n, which is gemm_block_n_for(rows) or anything from 256 up.
+int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int rows, const GroupedOut& o, cudaStream_t st);
+// whether a bf16 output of the plan's product can leave through it: N and ldo multiples of 8, out on a 16-byte boundary
+bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo);
+// ... with the choices made by the caller: box (16, 32, 64 or 128) is tm_x's, tile its rows per tile (a multiple of 16, at most
+// 2 * box), parts the pieces K is cut into (p.ws and p.counters hold them; a pair then has one item).
+int gemm_whole_run_as(const GemmPlan& p, const CUtensorMap& tm_x, int box, int tile, int parts, int rows, const GroupedOut& o, int* error, cudaStream_t st);
+int gemm_whole_parts(int N, int K, int tile, int tiles, int units);
 // Generic consumer: out[t, n] = bf16(sum of segments) — used by tests and by paths without a fused consumer.
 int reduce_partials(const PartialView& v, void* out, int ldo, int T, int N, cudaStream_t st);
 // out[t, n] (bf16, leading dimension ldo) for t < T.

@@ -957,6 +957,18 @@ int gemm2_x_box_rows(int block_n) { return (block_n > 256 ? 256 : block_n) / 2; 
 
 int gemm2_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, void* out, int ldo, int T, cudaStream_t st) {
   if (T <= 0) return 0;
+  // Whole tiles, or tiles cut along K with the last part finishing (gemm_grouped.cu), beat the stream-K form with its in-kernel
+  // fix-up (2048 x 2048, 512 tokens: 17 against 32 us; 8192 x 2048, 512 tokens: 20 against 102 us; 4096 x 14336, 2048 tokens:
+  // 194 against 447 us).  Left here: shapes whose rows are no whole 16-byte pieces, and long K where this kernel gives every
+  // pair one 512-token tile while 256-token tiles take two waves (4096 x 4096, 2048 tokens: 49.5 against 53.6 us; with K of
+  // 2048 the smaller tiles are the faster ones again, 4096 x 2048, 2048 tokens: 28.9 against 30.4).
+  const int slabs = (p.N + 2 * kSlab - 1) / (2 * kSlab);
+  const bool one_each = block_n == 512 && p.K > 2048 && slabs * ((T + 255) / 256) > p.max_ctas / 2 &&
+                        units_for(p, (T + 511) / 512) == slabs * ((T + 511) / 512);
+  if (gemm_whole_fits(p, out, ldo) && !one_each) {
+    const GroupedOut o = {out, ldo};
+    return gemm_whole_run(p, tm_x, block_n, T, o, st);
+  }
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   switch (block_n) {
     case 32: return launch2<32>(p, tm_x, o, ldo, T, st);

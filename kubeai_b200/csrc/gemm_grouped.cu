@@ -2,10 +2,15 @@
 // that expert's matrix, in ONE launch whose tile list is read from device memory.
 //     out[r, n] = sum_k X[r, k] * W[e(r) * N + n, k]        (bf16 x bf16 -> fp32 -> bf16)
 // X holds the rows of expert e at [first_e, first_e + rows_e) (the table moe_align leaves, so no count ever travels to the
-// host); W is the experts' matrices stacked row-wise.  With `glu` the rows of W alternate in blocks of 64 gate rows and their 64
-// up rows, and the epilogue writes silu(gate) * up, half as many columns.
+// host); W is the experts' matrices stacked row-wise.  What leaves the accumulators (gemm.h GroupedOut): the bf16 rounding of
+// bias and activation on the fp32 sums, the fp32 sums themselves, or a gated unit, for which the rows of W alternate in blocks
+// of 64 gate rows and their 64 up rows and the output has half as many columns.
 //
-// A CTA pair works on a tile of 256 weight rows x up to 256 rows of one expert; an expert's rows are cut into equal tiles.
+// A CTA pair works on a tile of 256 weight rows x up to 2 * box rows of one expert; an expert's rows are cut into equal tiles.
+// box, the rows of X that a CTA stages per k-block, is 16 to 128: a step of few tokens reads the weights once and is bound by
+// how fast an SM can take them in through TMA, and every byte of X that its tile does not need would come off that rate.
+// (24 tokens, 16 experts of 2 x 2048 x 2048, two a token: 128-row boxes move as many bytes of X as of weights.)  The ring
+// takes as many stages as fit beside the output staging.
 // Work items run expert by expert, weight tile by weight tile with its row tiles side by side, so that neighbouring pairs use
 // one weight slab at the same time, and are dealt to the pairs in turn.  Per CTA: one producer thread (TMA: its own 128
 // weight rows and its half of the row tile), one issuing thread in the leader, four epilogue warps that drain one of two
@@ -15,8 +20,10 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
+#include "activations.cuh"
 #include "gemm.h"
 #include "launch.h"
 #include "ptx.cuh"
@@ -27,14 +34,18 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 constexpr int kSlab = 128;      // weight rows per CTA
-constexpr int kRows = 256;      // rows of X per tile, at most
+constexpr int kRows = 256;      // rows of X per tile, at most; TMEM columns of one accumulator
 constexpr int kBlockK = 64, kUmmaK = 16;
 constexpr int kThreads = 192;
-constexpr int kABytes = kSlab * kBlockK * 2, kBBytes = kRows / 2 * kBlockK * 2, kStageBytes = kABytes + kBBytes;
-constexpr int kStages = 6;
-constexpr int kOutRows = 64;    // rows of X per epilogue round
+constexpr int kABytes = kSlab * kBlockK * 2;
+constexpr int kRingBytes = 6 * (kABytes + kRows / 2 * kBlockK * 2), kMaxStages = 10;
+constexpr int kOutRows = 64;    // rows of X per epilogue round (32 with fp32 output: the same bytes)
 constexpr int kOutBytes = kOutRows * kSlab * 2;
-constexpr int kSmem = 1024 + kStages * kStageBytes + 256 + 2 * kOutBytes;
+constexpr int kSmem = 1024 + kRingBytes + 256 + 2 * kOutBytes;
+__host__ __device__ constexpr int stage_bytes(int box) { return kABytes + box * kBlockK * 2; }
+__host__ __device__ constexpr int stages_for(int box) { return kRingBytes / stage_bytes(box) < kMaxStages ? kRingBytes / stage_bytes(box) : kMaxStages; }
+static_assert(stages_for(128) == 6 && stages_for(16) == kMaxStages, "ring depths");
+static_assert(8 * (2 * kMaxStages + 4) + 4 <= 256, "the barriers fit in front of the output staging");
 constexpr int kWaitLimit = 1 << 22;
 
 struct Tile {
@@ -42,22 +53,35 @@ struct Tile {
   int n0;        // the same within the expert's matrix
   int row0;      // first row of X
   int rows;      // rows of X (at most kRows)
+  int id;        // number of the tile (one matrix)
+  int part;      // which part of K
+  int kb0, kb1;  // its 64-wide steps
 };
 
 // Walks this pair's items: `next` advances by one item of the pair, expert by expert.
 struct Walk {
   const int* expert_rows;
-  int experts, mt, N, rows;   // without a table: one matrix, `rows` rows from 0
+  int experts, mt, N, rows, tile;   // without a table: one matrix, `rows` rows from 0; tile: rows of a tile at most
+  int parts, KB;                    // K in parts (one matrix only), in 64-wide steps
   int e = 0;
   long long base = 0;    // items of the experts before e
   __device__ bool at(long long item, Tile* t) {
     while (e < experts) {
       const int cnt = expert_rows ? expert_rows[2 * e + 1] : rows;
-      const int ntt = (cnt + kRows - 1) / kRows;
-      const long long n = static_cast<long long>(ntt) * mt;
+      const int ntt = (cnt + tile - 1) / tile;
+      const long long n = static_cast<long long>(ntt) * mt * parts;
       if (item < base + n) {
-        const int r = static_cast<int>(item - base), m = r / ntt, tt = r - m * ntt;
-        const int per = ((cnt + ntt - 1) / ntt + 15) & ~15;     // equal tiles, whole 16-row steps (at most kRows)
+        int r = static_cast<int>(item - base);
+        t->part = 0; t->kb0 = 0; t->kb1 = KB;
+        if (parts > 1) {
+          t->id = r / parts;
+          t->part = r - t->id * parts;
+          t->kb0 = KB * t->part / parts;
+          t->kb1 = KB * (t->part + 1) / parts;
+          r = t->id;
+        }
+        const int m = r / ntt, tt = r - m * ntt;
+        const int per = ((cnt + ntt - 1) / ntt + 15) & ~15;     // equal tiles, whole 16-row steps (at most `tile`)
         t->n0 = m * 2 * kSlab;
         t->wrow = e * N + t->n0;
         t->row0 = (expert_rows ? expert_rows[2 * e] : 0) + tt * per;
@@ -94,17 +118,109 @@ __device__ __forceinline__ bool all_epilogue(bool v) {
   return r != 0;
 }
 
+// Split K (one matrix, and fewer tiles than pairs): a tile's K is cut into parts, an item each, side by side on neighbouring
+// pairs.  Every part leaves its fp32 sums in the workspace and counts itself in; the part that comes last adds all of them
+// in their order and goes on to the epilogue, so nobody waits for anybody and the sum does not depend on who came last.
+struct SplitK {
+  float* ws;       // [tile][part][rank][rows of the tile][128]
+  int* counters;   // [tile][rank], zero between launches
+  int parts;
+  int tile;        // rows of a tile
+};
+__device__ __forceinline__ float gated_unit(float g, float u, bool clamp, const GroupedOut& o) {
+  if (clamp) { g = fminf(g, o.p0); u = fminf(fmaxf(u, -o.p0), o.p0); }
+  return __fdividef(g, 1.0f + __expf(-o.p1 * g)) * (u + o.p2);
+}
+// Eight neighbouring columns of one row: the parts' sums added in their order.
+__device__ __forceinline__ void add_parts(float* v, const float* p, int step, int parts) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = 0.f;
+  for (int k = 0; k < parts; ++k) {
+    const float4 a = *reinterpret_cast<const float4*>(p + k * step), b = *(reinterpret_cast<const float4*>(p + k * step) + 1);
+    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+    v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+  }
+}
+__device__ __forceinline__ void store8(bf16* p, const float* v) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+// n rows of a split tile, their parts in shared memory, to the rows from row0 of the output: a thread takes eight columns of a row
+template <int EPI>
+__device__ __forceinline__ void finish_rows(const float* sums, int step, int parts, int n, int row0, int n0, int N, const GroupedOut& o, int et) {
+  constexpr int kPieces = EPI == 1 ? 8 : 16;
+  for (int it = et; it < n * kPieces; it += 128) {
+    const int j = it / kPieces, c = (it % kPieces) * 8;
+    const float* p = sums + j * kSlab + c;
+    const size_t r = row0 + j;
+    float v[8];
+    if constexpr (EPI == 1) {
+      if (n0 + kSlab > N) continue;
+      float u[8];
+      add_parts(v, p, step, parts);
+      add_parts(u, p + 64, step, parts);
+      const bool clamp = o.p0 < INFINITY;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        v[i] = gated_unit(__bfloat162float(__float2bfloat16_rn(v[i])), __bfloat162float(__float2bfloat16_rn(u[i])), clamp, o);
+      store8(static_cast<bf16*>(o.y) + r * o.ldy + n0 / 2 + c, v);
+    } else {
+      if (n0 + c >= N) continue;
+      add_parts(v, p, step, parts);
+      if (EPI >= 2 && o.bias) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (n0 + c + i < N) v[i] += __ldg(o.bias + n0 + c + i);
+      }
+      if (EPI == 2) {
+        float* y = static_cast<float*>(o.y) + r * o.ldy + n0 + c;
+        *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]);
+        if (n0 + c + 4 < N) *reinterpret_cast<float4*>(y + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        continue;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (EPI == 3 && o.epi == GROUPED_RELU2) v[i] = fmaxf(v[i], 0.f) * fmaxf(v[i], 0.f);
+        if (EPI == 4) v[i] = xielu_fast(v[i], o.p0, o.p1);
+      }
+      store8(static_cast<bf16*>(o.y) + r * o.ldy + n0 + c, v);
+    }
+  }
+}
+// The epilogue of a split tile, from the workspace (`first`: the tile's first part, `step` floats to the next).  The parts come
+// through the operand ring, which is free (a split launch gives a pair one item), by cp.async: with plain loads the registers
+// bound what is in flight, and 256 rows in two parts took 25 us where this takes 13.
+template <int EPI>
+__device__ __forceinline__ void finish_parts(float* ring, const float* first, size_t step, int parts, const Tile& t, int n0, int N, const GroupedOut& o, int et) {
+  const int chunk = min(t.rows, kRingBytes / (kSlab * 4) / parts), sstep = chunk * kSlab;      // rows a round brings in
+  const uint32_t sring = smem_u32(ring);
+  for (int r0 = 0; r0 < t.rows; r0 += chunk) {
+    const int n = min(chunk, t.rows - r0);
+    for (int k = 0; k < parts; ++k)
+      for (int it = et; it < n * (kSlab / 4); it += 128)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sring + (k * sstep + it * 4) * 4), "l"(first + k * step + r0 * kSlab + it * 4) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    finish_rows<EPI>(ring, sstep, parts, n, t.row0 + r0, n0, N, o, et);
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+  }
+}
+
+// EPI 0: bf16(sum); 1: the gated unit; 2: fp32 sum + bias; 3: bf16(relu2(sum + bias)), or without an activation; 4: bf16(xielu(sum + bias)).
+// A form of its own for the plain product: looking the activation up per element made its drain a sixth of the launch longer.
+// FULL: 128-row boxes, their sizes known to the compiler.
+template <int EPI, bool FULL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const int* expert_rows, int experts, int rows,
-                    bf16* out, int ldo, int N, int K, int glu, int* error) {
+                    const __grid_constant__ GroupedOut o, int N, int K, int box_rows, const __grid_constant__ SplitK split, int* error) {
+  const int box = FULL ? 128 : box_rows, stages = stages_for(box);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + kStages * kStageBytes;
+  const uint32_t bar_base = smem_base + kRingBytes, stage_step = stage_bytes(box);
   auto full_bar = [&](int s) { return bar_base + 8u * s; };                     // the leader's copy is the live one
-  auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };        // both CTAs
-  auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kStages + a); };    // both CTAs
-  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kStages + 2 + a); };   // the leader's copy, 8 arrivals
-  const uint32_t tmem_slot = bar_base + 8u * (2 * kStages + 4);
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };        // both CTAs
+  auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + a); };    // both CTAs
+  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + 2 + a); };   // the leader's copy, 8 arrivals
+  const uint32_t tmem_slot = bar_base + 8u * (2 * kMaxStages + 4);
   uint8_t* stage_out = smem_raw + (bar_base + 256 - smem_u32(smem_raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -112,6 +228,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const int units = gridDim.x >> 1, unit = blockIdx.x >> 1, KB = (K + kBlockK - 1) / kBlockK;
   Walk walk;
   walk.expert_rows = expert_rows; walk.experts = experts; walk.mt = (N + 2 * kSlab - 1) / (2 * kSlab); walk.N = N; walk.rows = rows;
+  walk.tile = split.tile; walk.parts = split.parts; walk.KB = KB;
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_w);
@@ -119,7 +236,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   }
   if (warp == 1) {
     if (lane == 0) {
-      for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+      for (int s = 0; s < stages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
       for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 8); }   // 4 epilogue warps of each CTA
       fence_mbar_init();
     }
@@ -132,23 +249,38 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   bool ok = true;
+  griddep_launch();
+  if (expert_rows) griddep_wait();     // every role walks the table
 
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
+      int stage = 0, ahead = 0;
       uint32_t phase = 0;
       Tile t;
+      auto load_w = [&](int st, int kb) {
+        if (leader) mbar_arrive_expect_tx(full_bar(st), 2u * stage_step);
+        tma_load_2d_pair(smem_base + st * stage_step, &tm_w, full_bar(st), kb * kBlockK, t.wrow + static_cast<int>(rank) * kSlab, kEvictNormal);
+      };
+      if (!expert_rows) {
+        // the weights do not wait for the kernel in front: the ring's first stages of them are on their way before it ends
+        if (walk.at(unit, &t) && t.rows)
+          for (; ahead < min(stages, t.kb1 - t.kb0); ++ahead) load_w(ahead, t.kb0 + ahead);
+        griddep_wait();
+      }
       for (long long item = unit; ok && walk.at(item, &t); item += units) {
         if (!t.rows) continue;
         const int nc = (t.rows + 15) & ~15;
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!wait_limited(empty_bar(stage), phase ^ 1u)) { ok = false; break; }
-          const uint32_t sa = smem_base + stage * kStageBytes;
-          if (leader) mbar_arrive_expect_tx(full_bar(stage), 2u * kStageBytes);
-          tma_load_2d_pair(sa, &tm_w, full_bar(stage), kb * kBlockK, t.wrow + static_cast<int>(rank) * kSlab, kEvictNormal);
-          // this CTA stages the rank-th half of the row tile (the box is always kRows / 2 rows; rows past nc / 2 are not used)
+        for (int kb = t.kb0; kb < t.kb1; ++kb) {
+          const uint32_t sa = smem_base + stage * stage_step;
+          if (ahead > 0) {
+            --ahead;
+          } else {
+            if (!wait_limited(empty_bar(stage), phase ^ 1u)) { ok = false; break; }
+            load_w(stage, kb);
+          }
+          // this CTA stages the rank-th half of the row tile (rows of the box past nc / 2 are not used)
           tma_load_2d_pair(sa + kABytes, &tm_x, full_bar(stage), kb * kBlockK, t.row0 + static_cast<int>(rank) * (nc >> 1), kEvictLast);
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
     }
@@ -162,17 +294,17 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         const uint32_t idesc = umma_idesc_bf16(2 * kSlab, (t.rows + 15) & ~15);
         if (!wait_limited(tempty_bar(acc), acc_phase ^ 1u)) { ok = false; break; }
         tc_fence_after();
-        for (int kb = 0; kb < KB; ++kb) {
+        for (int kb = t.kb0; kb < t.kb1; ++kb) {
           if (!wait_limited(full_bar(stage), phase)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_base + stage * kStageBytes;
+          const uint32_t sa = smem_base + stage * stage_step;
           const uint64_t a_desc = umma_desc_kmajor_sw128(sa), b_desc = umma_desc_kmajor_sw128(sa + kABytes);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k)
-            umma2_bf16(tmem_base + acc * kRows, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma2_bf16(tmem_base + acc * kRows, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > t.kb0 || k > 0) ? 1u : 0u);
           umma2_commit_pair(empty_bar(stage), 3);
-          if (kb == KB - 1) umma2_commit_pair(tfull_bar(acc), 3);
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (kb == t.kb1 - 1) umma2_commit_pair(tfull_bar(acc), 3);
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
@@ -189,47 +321,102 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       tc_fence_after();
       const int n0 = t.n0 + static_cast<int>(rank) * kSlab;    // first column of this CTA's slab in the expert's output
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * kRows;
-      for (int c0 = 0; c0 < t.rows; c0 += kOutRows) {
-        const bool two = c0 + 32 < t.rows;
-        uint32_t v0[32], v1[32];
+      const float bias = EPI >= 2 && o.bias && n0 + row < N ? __ldg(o.bias + n0 + row) : 0.f;   // a thread's accumulator row is one output column
+      const bool relu2 = EPI == 3 && o.epi == GROUPED_RELU2;
+      bool whole = true;
+      if (split.parts > 1) {
+        whole = false;
+        const size_t slab = static_cast<size_t>(split.tile) * kSlab;
+        float* first = split.ws + (static_cast<size_t>(t.id) * split.parts * 2 + rank) * slab;
+        float* mine = first + 2 * t.part * slab + row;
+        for (int c0 = 0; c0 < t.rows; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld_32x32(taddr + c0, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (c0 + j < t.rows) __stcg(mine + static_cast<size_t>(c0 + j) * kSlab, __uint_as_float(v[j]));
+        }
+        __threadfence();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        bool last = false;
+        if (et == 0) {
+          last = atomicAdd(split.counters + 2 * t.id + rank, 1) == split.parts - 1;
+          if (last) split.counters[2 * t.id + rank] = 0;
+          __threadfence();
+        }
+        last = !all_epilogue(!last);       // thread 0's answer reaches all
+        if (last) finish_parts<EPI>(reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))), first, 2 * slab, split.parts, t, n0, N, o, et);
+      }
+      constexpr int kStep = EPI == 2 ? 32 : kOutRows;
+      for (int c0 = 0; whole && c0 < t.rows; c0 += kStep) {
+        const bool two = EPI != 2 && c0 + 32 < t.rows;
+        uint32_t v0[32], v1[EPI == 2 ? 1 : 32];
         tmem_ld_32x32(taddr + c0, v0);
-        if (two) tmem_ld_32x32(taddr + c0 + 32, v1);
+        if constexpr (EPI != 2) {
+          if (two) tmem_ld_32x32(taddr + c0 + 32, v1);
+        }
         tmem_ld_wait();
-        bf16* sb = reinterpret_cast<bf16*>(stage_out + sbuf * kOutBytes);
+        uint8_t* stage = stage_out + sbuf * kOutBytes;
+        const int left = t.rows - c0;
+        if constexpr (EPI == 2) {
+          float* sf = reinterpret_cast<float*>(stage);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sb[j * kSlab + row] = __float2bfloat16_rn(__uint_as_float(v0[j]));
-        if (two) {
+          for (int j = 0; j < 32; ++j) sf[j * kSlab + row] = __uint_as_float(v0[j]) + bias;
+        } else {
+          bf16* sb = reinterpret_cast<bf16*>(stage);
+          auto put = [&](int j, uint32_t u) {
+            float v = __uint_as_float(u);
+            if (EPI >= 3) v += bias;
+            if (EPI == 3) v = relu2 ? fmaxf(v, 0.f) * fmaxf(v, 0.f) : v;
+            if (EPI == 4) v = xielu_fast(v, o.p0, o.p1);
+            sb[j * kSlab + row] = __float2bfloat16_rn(v);
+          };
 #pragma unroll
-          for (int j = 0; j < 32; ++j) sb[(32 + j) * kSlab + row] = __float2bfloat16_rn(__uint_as_float(v1[j]));
+          for (int j = 0; j < 32; ++j) put(j, v0[j]);
+          if (two) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) put(32 + j, v1[j]);
+          }
         }
         // one barrier per round: a thread past it has finished its pass over the buffer staged two rounds ago
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        const int left = t.rows - c0;
-        bf16* dst = out + static_cast<size_t>(t.row0 + c0) * ldo;
-        if (glu) {
+        if constexpr (EPI == 2) {
+          float* dst = static_cast<float*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
+          const float* sf = reinterpret_cast<const float*>(stage);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int it = et + i * 128, j = it >> 5, c = (it & 31) * 4;
+            if (j < left && n0 + c < N)
+              *reinterpret_cast<float4*>(dst + static_cast<size_t>(j) * o.ldy + n0 + c) = *reinterpret_cast<const float4*>(sf + j * kSlab + c);
+          }
+        } else if constexpr (EPI == 1) {
           // rows 0..63 of the slab are gate rows, 64..127 the matching up rows: output columns n0 / 2 ..
+          bf16* dst = static_cast<bf16*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
+          const bf16* sb = reinterpret_cast<const bf16*>(stage);
+          const bool clamp = o.p0 < INFINITY;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int it = et + i * 128, j = it >> 3, c = (it & 7) * 8;
             if (j < left && n0 + kSlab <= N) {
               const uint4 g = *reinterpret_cast<const uint4*>(sb + j * kSlab + c), u = *reinterpret_cast<const uint4*>(sb + j * kSlab + 64 + c);
               const uint32_t gu[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w};
-              uint32_t o[4];
+              uint32_t r[4];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float g0 = __uint_as_float(gu[k] << 16), g1 = __uint_as_float(gu[k] & 0xffff0000u);
-                o[k] = pack_bf16x2(__fdividef(g0, 1.0f + __expf(-g0)) * __uint_as_float(uu[k] << 16),
-                                   __fdividef(g1, 1.0f + __expf(-g1)) * __uint_as_float(uu[k] & 0xffff0000u));
-              }
-              *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * ldo + n0 / 2 + c) = make_uint4(o[0], o[1], o[2], o[3]);
+              for (int k = 0; k < 4; ++k)
+                r[k] = pack_bf16x2(gated_unit(__uint_as_float(gu[k] << 16), __uint_as_float(uu[k] << 16), clamp, o),
+                                   gated_unit(__uint_as_float(gu[k] & 0xffff0000u), __uint_as_float(uu[k] & 0xffff0000u), clamp, o));
+              *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * o.ldy + n0 / 2 + c) = make_uint4(r[0], r[1], r[2], r[3]);
             }
           }
         } else {
+          bf16* dst = static_cast<bf16*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
+          const bf16* sb = reinterpret_cast<const bf16*>(stage);
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int it = et + i * 128, j = it >> 4, c = (it & 15) * 8;
             if (j < left && n0 + c < N)
-              *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * ldo + n0 + c) = *reinterpret_cast<const uint4*>(sb + j * kSlab + c);
+              *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * o.ldy + n0 + c) = *reinterpret_cast<const uint4*>(sb + j * kSlab + c);
           }
         }
         sbuf ^= 1;
@@ -259,15 +446,77 @@ int gemm_grouped_plan(GroupedPlan* p, const void* W, int experts, int N, int K) 
   return tmap_encode_bf16_2d(&p->tm_w, W, static_cast<uint64_t>(experts) * N, K, K, kSlab, kBlockK, 1);
 }
 
-int gemm_grouped_x_map(CUtensorMap* tm, const void* X, int rows, int K) { return tmap_encode_bf16_2d(tm, X, rows, K, K, kRows / 2, kBlockK, 1); }
+constexpr int kBoxes[kGroupedBoxes] = {16, 32, 64, 128};
 
-int gemm_grouped_run(const GroupedPlan& p, const CUtensorMap& tm_x, const int* expert_rows, void* out, int ldo, bool glu, int sms, int* error,
-                     cudaStream_t st, int rows) {
-  if ((!expert_rows && (p.experts != 1 || rows < 1)) || !out || ldo % 8 || reinterpret_cast<uintptr_t>(out) % 16 || sms < 2 || (glu && p.N % kSlab)) return -1;
-  static std::atomic<unsigned long long> attr{0};
-  if (!ensure_dynamic_smem(gemm_grouped_kernel, kSmem, &attr)) return -2;
-  gemm_grouped_kernel<<<sms / 2 * 2, kThreads, kSmem, st>>>(p.tm_w, tm_x, expert_rows, p.experts, rows, static_cast<bf16*>(out), ldo, p.N, p.K, glu ? 1 : 0, error);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+int gemm_grouped_x_maps(GroupedX* x, const void* X, int rows, int K) {
+  for (int i = 0; i < kGroupedBoxes; ++i)
+    if (const int rc = tmap_encode_bf16_2d(&x->box[i], X, rows, K, K, kBoxes[i], kBlockK, 1)) return rc;
+  return 0;
+}
+
+namespace {
+int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap& tm_x, int box, const int* expert_rows, int rows, const GroupedOut& o,
+           const SplitK& split, int units, int* error, cudaStream_t st) {
+  const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED;
+  if ((!expert_rows && (experts != 1 || rows < 1)) || !o.y || o.ldy % (f32 ? 4 : 8) || N % (f32 ? 4 : 8) || reinterpret_cast<uintptr_t>(o.y) % 16 || units < 1 ||
+      (gated && (N % kSlab || o.bias)) || (o.bias && experts != 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
+  static std::atomic<unsigned long long> attr[10];
+  auto start = [&](auto kernel, int i) {
+    if (!ensure_dynamic_smem(kernel, kSmem, &attr[i])) return -2;
+    return launch_pdl(kernel, dim3(2 * units), dim3(kThreads), kSmem, st, tm_w, tm_x, expert_rows, experts, rows, o, N, K, box, split, error) == cudaSuccess ? 0 : -2;
+  };
+#define RUN(E) return box == 128 ? start(gemm_grouped_kernel<E, true>, 2 * E) : start(gemm_grouped_kernel<E, false>, 2 * E + 1)
+  if (gated) RUN(1);
+  if (f32) RUN(2);
+  if (o.epi == GROUPED_XIELU) RUN(4);
+  if (o.epi == GROUPED_RELU2 || o.bias) RUN(3);
+  RUN(0);
+#undef RUN
+}
+}  // namespace
+
+int gemm_grouped_run(const GroupedPlan& p, const GroupedX& x, int most_rows, const int* expert_rows, const GroupedOut& o, int sms, int* error, cudaStream_t st) {
+  if (!expert_rows) return -1;
+  int i = 0;
+  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < most_rows) ++i;
+  return launch(p.tm_w, p.experts, p.N, p.K, x.box[i], kBoxes[i], expert_rows, 0, o, {nullptr, nullptr, 1, 2 * kBoxes[i]}, sms / 2, error, st);
+}
+
+int gemm_whole_run_as(const GemmPlan& p, const CUtensorMap& tm_x, int box, int tile, int parts, int rows, const GroupedOut& o, int* error, cudaStream_t st) {
+  if (rows < 1 || tile < 1 || parts < 1 || parts > (p.K + kBlockK - 1) / kBlockK) return -1;
+  const long long tiles = static_cast<long long>((p.N + 2 * kSlab - 1) / (2 * kSlab)) * ((rows + tile - 1) / tile);
+  if (parts > 1 && (tiles * parts > p.max_ctas / 2 || tiles * parts * 2 * tile * kSlab * static_cast<long long>(sizeof(float)) > static_cast<long long>(p.ws_bytes) ||
+                    !p.ws || !p.counters)) return -1;
+  const int units = static_cast<int>(std::min<long long>(p.max_ctas / 2, tiles * parts));
+  return launch(p.tm_w, 1, p.N, p.K, tm_x, box, nullptr, rows, o, {p.ws, p.counters, parts, tile}, units, error, st);
+}
+
+// The parts K is cut into.  A pair takes in a 64-wide step of K in 0.28 us whatever the tile (what an SM draws through TMA), so
+// a launch of few tiles is as long as its K; cutting it puts more pairs to work, down to the time the weights take from
+// memory, and costs the exchange, about 1 us + rows of the tile * (0.03 + 0.005 parts) us.  Measured, one part against the
+// rule's (N, K, tokens): 4096, 14336, 16: 72.7 against 33.8 us; 257: 74.8, 50.9; 512: 76.8, 57.0; 2048, 8192, 16: 45.4, 19.4;
+// 512: 46.1, 34.5; 4096, 4096, 64: 27.6, 20.8; 512: 29.7, 29.7; 2048, 2048, 16: 17.4, 13.3 (launch included).
+int gemm_whole_parts(int N, int K, int tile, int tiles, int units) {
+  const int KB = (K + kBlockK - 1) / kBlockK;
+  const double memory = 2.0 * N * K / 5.5e6;
+  int best = 1;
+  double least = 0;
+  for (int parts = 1; parts == 1 || (tiles * parts <= units && parts * 8 <= KB); ++parts) {
+    const double us = std::max((KB + parts - 1) / parts * 0.28, tiles < units ? memory : 0.0) + (parts > 1 ? 1.0 + tile * (0.03 + 0.005 * parts) : 0.0);
+    if (parts == 1 || us < least) { least = us; best = parts; }
+  }
+  return best;
+}
+
+int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int rows, const GroupedOut& o, cudaStream_t st) {
+  if (rows < 1) return 0;
+  const int box = gemm2_x_box_rows(block_n), ntt = (rows + 2 * box - 1) / (2 * box), tile = ((rows + ntt - 1) / ntt + 15) & ~15;
+  const int tiles = (p.N + 2 * kSlab - 1) / (2 * kSlab) * ((rows + tile - 1) / tile);
+  return gemm_whole_run_as(p, tm_x, box, tile, gemm_whole_parts(p.N, p.K, tile, tiles, p.max_ctas / 2), rows, o, p.error, st);
+}
+
+bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo) {
+  return gemm_variant() == 2 && p.N % 8 == 0 && ldo % 8 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
 }
 
 }  // namespace b200

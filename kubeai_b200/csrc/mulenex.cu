@@ -74,18 +74,21 @@ struct LayerWeights {
   float *up_b = nullptr, *down_b = nullptr;
   void* router = nullptr;   // [experts (+ 1), width]: the router rows, then the shared expert's gate row
   float* router_b = nullptr;   // [experts (+ 1)], 0 for the shared gate
-  void* e_gu = nullptr;     // [experts][2 ff][width]  gate rows, then up rows
+  void* e_gu = nullptr;     // [experts][2 ff][width]  gate rows, then up rows (or in turns, see il_e)
   void* e_down = nullptr;   // [experts][width][ff]
-  void* sh_in = nullptr;    // [n_sh, width]: gate [sff] | up [sff]
+  void* sh_in = nullptr;    // [n_sh, width]: gate [sff] | up [sff] (or in turns, see il_s)
   void* sh_down = nullptr;  // [width, sff]
   void* cache = nullptr;    // attention: [num_blocks * page][kv_heads * (dim + vdim)]
   float* state = nullptr;   // mlstm: [slots][heads][dim][vdim]
   float* nstate = nullptr;  // mlstm: [slots][heads][dim], the normaliser
   float* mstate = nullptr;  // mlstm: [slots][heads], the log-scale
   GemmPlan p_in, p_out, p_up, p_down, p_shin, p_shdown;
-  std::vector<GemmPlan> p_egu, p_edown;
+  GroupedPlan g_egu, g_edown;
+  GroupedX xg_h, xg_act;                                       // views of the sorted rows and of the hidden rows
   CUtensorMap xm_out[kGemmNumBlockN], xm_ffh[kGemmNumBlockN], xm_shact[kGemmNumBlockN];
-  bool tc_in = false, tc_out = false, tc_up = false, tc_down = false, tc_shin = false, tc_shdown = false;
+  bool tc_in = false, tc_out = false, tc_up = false, tc_down = false, tc_shin = false, tc_shdown = false, tc_experts = false;
+  // bf16: gate and up rows alternate in blocks of 64 (a product's epilogue then holds both parts of a gated unit)
+  bool il_e = false, il_s = false;
 };
 
 bool jnum(const JVal* o, const char* k, double* out) {
@@ -115,7 +118,9 @@ class Mulenex : public Model {
   int *topi = nullptr, *sorted_rows = nullptr, *tile_group = nullptr, *pair_pos = nullptr, *iota = nullptr;
   int row_cap = 0, moe_cap = 0, vfirst_ld = 0;
   void *hsorted = nullptr, *edown16 = nullptr;
-  int *expert_rows = nullptr, *expert_rows_host = nullptr;
+  int* expert_rows = nullptr;
+  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
+  int moe_tc_min = 1;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
@@ -131,10 +136,8 @@ class Mulenex : public Model {
       if (w.tc_down) gemm_plan_destroy(&w.p_down);
       if (w.tc_shin) gemm_plan_destroy(&w.p_shin);
       if (w.tc_shdown) gemm_plan_destroy(&w.p_shdown);
-      for (auto& p : w.p_egu) gemm_plan_destroy(&p);
-      for (auto& p : w.p_edown) gemm_plan_destroy(&p);
     }
-    if (expert_rows_host) cudaFreeHost(expert_rows_host);
+    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Mulenex"; }
@@ -285,6 +288,8 @@ class Mulenex : public Model {
         if (s.shared) { any_shared = true; max_nsh = std::max(max_nsh, s.n_sh); max_sff = std::max(max_sff, s.sff); }
       }
     }
+    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
+    *kernel_error = 0;
     int rc = 0;
     auto mat = [&](void** p, size_t rows, size_t cols) { return dalloc(p, rows * cols * es); };
     auto vec = [&](float** p, size_t n) { return dalloc(p, n * sizeof(float)); };
@@ -306,6 +311,8 @@ class Mulenex : public Model {
       if (s.mlp != MLP_NONE) rc |= vec(&w.norm2, W) | vec(&w.norm2b, W);
       if (s.mlp == MLP_DENSE) rc |= mat(&w.up, s.ff, W) | mat(&w.down, W, s.ff) | vec(&w.up_b, s.ff) | vec(&w.down_b, W);
       if (s.mlp == MLP_MOE) {
+        w.il_e = dt == DT_BF16 && s.ff % 64 == 0;
+        w.il_s = dt == DT_BF16 && s.shared && s.sff % 64 == 0;
         const int nr = s.experts + (s.shared ? 1 : 0);
         rc |= mat(&w.router, nr, W) | vec(&w.router_b, nr) | mat(&w.e_gu, static_cast<size_t>(s.experts) * 2 * s.ff, W) |
               mat(&w.e_down, static_cast<size_t>(s.experts) * W, s.ff);
@@ -344,8 +351,7 @@ class Mulenex : public Model {
   }
 
   // The projections of a bf16 model run on the tcgen05 pair GEMM (gemm2_tcgen05.cu) where their shapes allow it (K % 8 == 0):
-  // input and output projection, the dense feed-forward, the shared expert, and every expert for steps large enough to sort
-  // rows per expert.  B200_MX_TC=0 keeps every projection on linear.cu (A/B knob); fp32 models always do.
+  // input and output projection, the dense feed-forward, the shared expert; the experts on its grouped form (gemm_grouped.cu).  B200_MX_TC=0 keeps every projection on linear.cu (A/B knob); fp32 models always do.
   int setup_tc() {
     const char* ev = getenv("B200_MX_TC");
     use_tc = dt == DT_BF16 && !(ev && atoi(ev) == 0) && W % 8 == 0 && gemm_variant() == 2;
@@ -362,6 +368,7 @@ class Mulenex : public Model {
     auto plan = [&](GemmPlan* p, const void* Wm, int N, int K) {
       if (K % 8 || gemm_plan_init(p, Wm, N, K, K, gemm_ws, gemm_counters, env.sms)) return false;
       p->ws_bytes = ws_bytes;
+      p->error = kernel_error;
       return true;
     };
     auto maps = [&](CUtensorMap* xm, const void* X, int K) {
@@ -369,7 +376,13 @@ class Mulenex : public Model {
         if (gemm_make_x_map(&xm[j], X, env.Tcap, K, K, bns[j])) return false;
       return true;
     };
-    bool any_expert_tc = false;
+    int max_e = 1;
+    bool any_moe = false;
+    for (auto& s : spec)
+      if (s.mlp == MLP_MOE) { any_moe = true; max_e = std::max(max_e, s.experts); }
+    if (any_moe && (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
+                    dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int)))) return -3;
+    if (const char* e = getenv("B200_MX_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
     for (size_t i = 0; i < spec.size(); ++i) {
       const LayerSpec& s = spec[i];
       LayerWeights& w = wts[i];
@@ -386,30 +399,9 @@ class Mulenex : public Model {
         w.tc_shdown = plan(&w.p_shdown, w.sh_down, W, s.sff);
         if (w.tc_shdown && !maps(w.xm_shact, shact, s.sff)) { gemm_plan_destroy(&w.p_shdown); w.tc_shdown = false; }
       }
-      if (s.mlp == MLP_MOE && s.ff % 8 == 0) {
-        w.p_egu.resize(s.experts);
-        w.p_edown.resize(s.experts);
-        int made_u = 0, made_d = 0;
-        bool ok = true;
-        for (int e = 0; e < s.experts && ok; ++e) {
-          ok = plan(&w.p_egu[e], static_cast<bf16*>(w.e_gu) + static_cast<size_t>(e) * 2 * s.ff * W, 2 * s.ff, W);
-          if (ok) ++made_u;
-          ok = ok && plan(&w.p_edown[e], static_cast<bf16*>(w.e_down) + static_cast<size_t>(e) * W * s.ff, W, s.ff);
-          if (ok) ++made_d;
-        }
-        if (!ok) {
-          for (int e = 0; e < made_u; ++e) gemm_plan_destroy(&w.p_egu[e]);
-          for (int e = 0; e < made_d; ++e) gemm_plan_destroy(&w.p_edown[e]);
-          w.p_egu.clear(); w.p_edown.clear();
-        } else any_expert_tc = true;
-      }
-    }
-    if (any_expert_tc) {
-      int max_e = 1;
-      for (auto& s : spec) max_e = std::max(max_e, s.experts);
-      if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
-          dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
-      if (cudaMallocHost(&expert_rows_host, static_cast<size_t>(max_e) * 2 * sizeof(int)) != cudaSuccess) return -3;
+      if (s.mlp == MLP_MOE)
+        w.tc_experts = !gemm_grouped_plan(&w.g_egu, w.e_gu, s.experts, 2 * s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
+                       !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);
     }
     return 0;
   }
@@ -439,6 +431,17 @@ class Mulenex : public Model {
     uint8_t* d = static_cast<uint8_t*>(dst) + (row0 * ld + col0) * es;
     return cudaMemcpy2D(d, ld * es, tmp.data(), cols * es, cols * es, rows, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -2;
   }
+  // gate and up rows [F, cols] each, one below the other or in alternating blocks of 64
+  int put_pair(void* dst, size_t row0, const std::vector<float>& gate, const std::vector<float>& up, size_t F, size_t cols, bool in_turns) {
+    std::vector<float> both;
+    both.reserve(2 * F * cols);
+    const size_t block = (in_turns ? 64 : F) * cols;
+    for (size_t at = 0; at < F * cols; at += block) {
+      both.insert(both.end(), gate.begin() + at, gate.begin() + at + block);
+      both.insert(both.end(), up.begin() + at, up.begin() + at + block);
+    }
+    return put(dst, cols, row0, 0, both, 2 * F, cols);
+  }
   int putf(float* dst, const std::vector<float>& src, float offset = 0.f) {
     std::vector<float> t(src);
     for (auto& v : t) v += offset;
@@ -461,6 +464,8 @@ class Mulenex : public Model {
     };
     int rc = 0;
 #define MAT(name, dst, ld, row0, col0, rows, cols) do { if (!get(name, rows, cols)) return -4; rc |= put(dst, ld, row0, col0, v, rows, cols); } while (0)
+#define PAIR(name, dst, row0, F, cols, in_turns) do { if (!get((name) + "gate", F, cols)) return -4; const std::vector<float> gate_(v); \
+                                                      if (!get((name) + "up", F, cols)) return -4; rc |= put_pair(dst, row0, gate_, v, F, cols, in_turns); } while (0)
 #define VEC(name, dst, n) do { if (!get(name, 1, n)) return -4; rc |= putf(dst, v); } while (0)
 #define NORM(name, dst, n) do { if (!get(name, 1, n)) return -4; rc |= putf(dst, v, 1.0f); } while (0)   // stored as the offset from one
     MAT("embed", embed, W, 0, 0, V, W);
@@ -515,18 +520,17 @@ class Mulenex : public Model {
       }
       for (int e = 0; e < s.experts; ++e) {
         const std::string ep = f + "e" + std::to_string(e) + ".";
-        MAT(ep + "gate", w.e_gu, W, static_cast<size_t>(e) * 2 * s.ff, 0, s.ff, W);
-        MAT(ep + "up", w.e_gu, W, static_cast<size_t>(e) * 2 * s.ff + s.ff, 0, s.ff, W);
+        PAIR(ep, w.e_gu, static_cast<size_t>(e) * 2 * s.ff, s.ff, W, w.il_e);
         MAT(ep + "down", w.e_down, s.ff, static_cast<size_t>(e) * W, 0, W, s.ff);
       }
       if (s.shared) {
-        MAT(f + "shared.gate", w.sh_in, W, 0, 0, s.sff, W);
-        MAT(f + "shared.up", w.sh_in, W, s.sff, 0, s.sff, W);
+        PAIR(f + "shared.", w.sh_in, 0, s.sff, W, w.il_s);
         MAT(f + "shared.sg", w.router, W, s.experts, 0, 1, W);
         MAT(f + "shared.down", w.sh_down, s.sff, 0, 0, W, s.sff);
       }
     }
 #undef MAT
+#undef PAIR
 #undef VEC
 #undef NORM
     if (rc) { *err = "copying weights to the device failed"; return -2; }
@@ -576,7 +580,12 @@ class Mulenex : public Model {
               const float* bias = nullptr, int act = LIN_NONE) {
     if (tc) {
       const int bn = gemm_block_n_for(T);
-      int rc = gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
+      const CUtensorMap& tm = xm[gemm_block_n_index(bn)];
+      if ((bias || act != LIN_NONE) && gemm_whole_fits(plan, Y, N)) {
+        const GroupedOut o = {Y, N, act == LIN_RELU2 ? GROUPED_RELU2 : GROUPED_PLAIN, bias};
+        return gemm_whole_run(plan, tm, bn, T, o, env.stream);
+      }
+      int rc = gemm_run(plan, tm, bn, Y, N, T, env.stream);
       if (!rc && (bias || act != LIN_NONE)) rc = bias_act(Y, N, bias, act, dt, T, N, env.stream);
       return rc;
     }
@@ -691,22 +700,27 @@ class Mulenex : public Model {
     const void* shared_out = nullptr;
     const float* shared_gate = nullptr;
     if (s.shared) {
-      KRN("shared_in", project(w.p_shin, w.tc_shin, xm_h, h, w.sh_in, sh, T, s.n_sh, W));
-      KRN("glu", glu_clamped(sh, s.n_sh, shact, s.sff, dt, T, s.sff, INFINITY, 1.f, st, 0.f));
+      if (w.il_s && w.tc_shin && gemm_whole_fits(w.p_shin, shact, s.sff)) {
+        const GroupedOut o = {shact, s.sff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};     // the gated unit in the epilogue
+        const int bn = gemm_block_n_for(T);
+        KRN("shared_in", gemm_whole_run(w.p_shin, xm_h[gemm_block_n_index(bn)], bn, T, o, st));
+      } else {
+        KRN("shared_in", project(w.p_shin, w.tc_shin, xm_h, h, w.sh_in, sh, T, s.n_sh, W));
+        KRN("glu", glu_clamped(sh, s.n_sh, shact, s.sff, dt, T, s.sff, INFINITY, 1.f, st, 0.f, w.il_s));
+      }
       KRN("shared_down", project(w.p_shdown, w.tc_shdown, w.xm_shact, shact, w.sh_down, sdown, T, W, s.sff));
       shared_out = sdown;
       shared_gate = scores + s.experts;
     }
     const long long gu_stride = 2ll * s.ff * W, down_stride = static_cast<long long>(W) * s.ff;
-    static const int moe_tc_min = [] { const char* e = getenv("B200_MX_MOE_TC_MIN_T"); return e ? atoi(e) : 256; }();   // A/B knob
-    const bool per_expert = !w.p_egu.empty() && T >= moe_tc_min;
+    const bool grouped = w.tc_experts && T >= moe_tc_min;
     if (T * s.top <= 64) {
       // decode-sized steps: one weight-streaming pass per chosen (token, expert) pair, rows in pair order
       LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, T * s.top, 2 * s.ff, W);
       up.wbs = gu_stride;
       const PickedRows pu = {T * s.top, nullptr, s.top, iota, topi};
       KRN("moe_up", linear_picked_rows(up, pu, st));
-      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, T * s.top, s.ff, INFINITY, 1.f, st, 0.f));
+      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, T * s.top, s.ff, INFINITY, 1.f, st, 0.f, w.il_e));
       LinearArgs dn = linear_args(eact, dt, w.e_down, dt, edown, DT_F32, T * s.top, W, s.ff);
       dn.wbs = down_stride;
       const PickedRows pd = {T * s.top, iota, 1, iota, topi};
@@ -716,43 +730,29 @@ class Mulenex : public Model {
       return rc;
     }
     const int cap = (T * s.top + 63) / 64 * 64 + s.experts * 64;
-    KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, per_expert ? expert_rows : nullptr));
-    if (per_expert) {
-      // Large steps: every expert's rows are one tcgen05 GEMM.  The row counts come back to the host (one small copy and a
-      // wait per layer, paid only by steps of hundreds of tokens); the inputs are gathered into sorted order.
+    KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, grouped ? expert_rows : nullptr));
+    if (grouped) {
+      // the inputs in expert-sorted order, then one grouped GEMM per matrix; the row counts stay on the device.  Steps of
+      // fewer than 256 tokens keep the experts' outputs in fp32 until the combine, as the tile kernel below does.
+      const bool wide = T < 256;
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
-      if (cudaMemcpyAsync(expert_rows_host, expert_rows, static_cast<size_t>(s.experts) * 2 * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess) rc = -2;
-      prof_start();
-      for (int e = 0; e < s.experts && !rc; ++e) {
-        const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-        if (cnt <= 0) continue;
-        const int bn = gemm_block_n_for(cnt);
-        CUtensorMap tm;
-        if (gemm_make_x_map(&tm, static_cast<bf16*>(hsorted) + static_cast<size_t>(start) * W, cnt, W, W, bn)) { rc = -2; break; }
-        rc |= gemm_run(w.p_egu[e], tm, bn, static_cast<bf16*>(egu) + static_cast<size_t>(start) * 2 * s.ff, 2 * s.ff, cnt, st);
-        ++nl;
+      if (w.il_e) {
+        const GroupedOut o = {eact, s.ff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
+      } else {
+        const GroupedOut o = {egu, 2 * s.ff};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
+        KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f));
       }
-      prof_stop("moe_up");
-      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f));
-      prof_start();
-      for (int e = 0; e < s.experts && !rc; ++e) {
-        const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-        if (cnt <= 0) continue;
-        const int bn = gemm_block_n_for(cnt);
-        CUtensorMap tm;
-        if (gemm_make_x_map(&tm, static_cast<bf16*>(eact) + static_cast<size_t>(start) * s.ff, cnt, s.ff, s.ff, bn)) { rc = -2; break; }
-        rc |= gemm_run(w.p_edown[e], tm, bn, static_cast<bf16*>(edown16) + static_cast<size_t>(start) * W, W, cnt, st);
-        ++nl;
-      }
-      prof_stop("moe_down");
-      KRN("moe_combine", moe_combine_add(edown16, DT_BF16, pair_pos, topw, shared_out, shared_gate, nr, fo, dt, T, s.top, W, st));
+      const GroupedOut o = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, o, env.sms, kernel_error, st));
+      KRN("moe_combine", moe_combine_add(o.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, shared_out, shared_gate, nr, fo, dt, T, s.top, W, st));
       return rc;
     }
     LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, cap, 2 * s.ff, W);
     up.x_rows = sorted_rows; up.tile_group = tile_group; up.wbs = gu_stride;
     KRN("moe_up", linear(up, st));
-    KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f));
+    KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f, w.il_e));
     LinearArgs dn = linear_args(eact, dt, w.e_down, dt, edown, DT_F32, cap, W, s.ff);
     dn.tile_group = tile_group; dn.wbs = down_stride;
     KRN("moe_down", linear(dn, st));
@@ -765,6 +765,7 @@ class Mulenex : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
+    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Mulenex forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_sinusoid(embed, dt, b.ids, b.pos, pos_freq, x, T, W, V, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {

@@ -1,0 +1,69 @@
+"""The whole-tile product (csrc/gemm_grouped.cu): every size of its row tiles and operand boxes, K whole and in parts, and the
+expert form behind a model, against 64-bit products and against the tile kernel it replaces."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from mulenex_util import attention, layer, make_config, moe, mlstm, open_engine, feed_whole, random_weights, rel_err, write_model_dir, oracle_for
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(T, N, K, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") / math.sqrt(K)).to(torch.bfloat16)
+    return x, w
+
+
+@pytest.mark.parametrize("T,N,K", [
+    (1, 8, 8), (1, 4096, 4096), (16, 264, 72), (17, 2048, 2048), (32, 2048, 8192), (33, 1032, 4096),      # boxes of 16 and 32 rows, K in parts
+    (64, 256, 16384), (65, 2048, 2048), (128, 4096, 14336), (129, 2048, 4104), (255, 512, 2048), (256, 4096, 4096),   # 64 and 128; K no whole steps
+    (257, 4096, 14336), (300, 2048, 8192), (511, 264, 1032), (513, 2048, 2048),                       # two and three row tiles
+    (1000, 6144, 4096), (1999, 4096, 2048), (2048, 8192, 1024),                                          # several waves
+])
+def test_product_against_64_bits_and_repeatable(T, N, K):
+    from kubeai_b200 import ops
+    x, w = operands(T, N, K)
+    got = ops.gemm(x, w)
+    again = ops.gemm(x, w)          # counters are zero again, the parts are added in their order whoever comes last
+    assert torch.equal(got, again)
+    want = x.double() @ w.double().T
+    # one rounding to bf16 (8 significant bits: half a last place is at most 2^-8 of the value) and at most K + 16 fp32
+    # additions (2^-24 of the sum of magnitudes each)
+    bound = 2.0 ** -8 * want.abs() + (K + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert ((got.double() - want).abs() <= 1.01 * bound + 1e-30).all()
+
+
+def test_infinities_and_nan_stay_in_their_rows():
+    from kubeai_b200 import ops
+    x, w = operands(40, 512, 8192, seed=3)
+    x[3, 100], x[7, 5000] = float("nan"), float("inf")
+    got = ops.gemm(x, w)
+    assert torch.isnan(got[3]).all() and not torch.isfinite(got[7]).any()
+    rest = [i for i in range(40) if i not in (3, 7)]
+    assert torch.isfinite(got[rest]).all()
+
+
+@pytest.mark.parametrize("ff,shared", [(64, 64), (24, 40), (128, None)])
+@pytest.mark.parametrize("T", [33, 64, 65, 129, 255, 256, 300])
+def test_experts_agree_with_the_tile_kernel(tmp_path, monkeypatch, ff, shared, T):
+    """Interleaved and stacked gate and up rows, fp32 outputs below 256 tokens, every operand box."""
+    layers = [layer(attention(heads=2, kv_heads=1, dim=16, vdim=16), mlp=moe(experts=5, top=2, ff=ff, shared=shared)),
+              layer(mlstm(heads=2, dim=16, vdim=16), mlp=moe(experts=3, top=3, ff=ff, shared=shared))]
+    cfg = make_config(layers, width=64)
+    W = random_weights(cfg, seed=5)
+    d = write_model_dir(tmp_path / "m", cfg, W)
+    t = np.random.default_rng(T).integers(0, cfg["vocab"], T).tolist()
+    with open_engine(d, dtype="bfloat16") as e:
+        new = feed_whole(e, t)
+    monkeypatch.setenv("B200_MX_MOE_TC_MIN_T", "100000")
+    with open_engine(d, dtype="bfloat16") as e:
+        old = feed_whole(e, t)
+    want = oracle_for(cfg, W).forward(t)
+    # both round every projection to bf16, so a row's distance to the oracle is a few times 2^-8; rows whose routing is close
+    # to a tie may take another expert
+    assert np.median(rel_err(new, want)) < 0.03 and np.median(rel_err(new, old.astype(np.float64))) < 0.02
+    assert np.median(rel_err(new, want)) < 1.3 * np.median(rel_err(old, want)) + 1e-3

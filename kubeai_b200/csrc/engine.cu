@@ -259,6 +259,7 @@ struct Engine {
        *last_hidden = nullptr, *logits = nullptr;
   int* sampled = nullptr;
   int32_t* sampled_host = nullptr;  // pinned
+  int* kernel_error = nullptr;      // pinned: a kernel whose wait ran out leaves a mark here
   // decode-shape fused path (gemm3_tcgen05.cu): per-slab sums of squares of the residual, argmax candidates, stream-K flags
   float* ssq = nullptr;
   float2* cand = nullptr;
@@ -272,6 +273,7 @@ struct Engine {
   int attn_split_force = 0;  // B200_ATTN_SPLIT=<parts> (A/B knob; 1 = never split)
   static constexpr int kSplitMaxWork = 18, kSplitMaxParts = 32;
   bool fused2_ok = false;   // steps of more than 128 tokens: pair kernel with fused epilogues (gemm2 mode 2)
+  bool whole_ok = false;    // ... or the whole-tile product (gemm_grouped.cu), the default
   int chain_ctas = 0;
   unsigned long long* chain_bar = nullptr;
   unsigned long long chain_bar_count = 0;   // host mirror of the grid-barrier counter
@@ -416,6 +418,7 @@ Engine::~Engine() {
   if (feed_logits_host) cudaFreeHost(feed_logits_host);
   model.reset();   // frees the model's device memory while the context is current
   if (sampled_host) cudaFreeHost(sampled_host);
+  if (kernel_error) cudaFreeHost(kernel_error);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (stream) cudaStreamDestroy(stream);
@@ -541,9 +544,12 @@ int Engine::alloc_all() {
   CK(cudaMemset(gemm_counters, 0, n_counters * 4));
 
   // ---- GEMM plans + activation tensor maps (encoded once; kernels mask rows >= T)
+  CK(cudaMallocHost(&kernel_error, sizeof(int)));
+  *kernel_error = 0;
   auto plan = [&](GemmPlan* p, const void* W, int N, int K) {
     int rc = gemm_plan_init(p, W, N, K, K, gemm_ws, gemm_counters, sms);
     if (rc) return rc;
+    p->error = kernel_error;
     p->ws_bytes = gemm_ws_bytes;
     return gemm_variant() == 2 ? gemm_plan_build_table(p, std::max(Tcap, Scap)) : 0;
   };
@@ -582,6 +588,11 @@ int Engine::alloc_all() {
       const char* pe = getenv("B200_FUSED_PREFILL");   // A/B knob: 0 keeps the larger steps on fp32 segments + elementwise kernels
       fused2_ok = !(pe && atoi(pe) == 0) && gemm_variant() == 2 && QKV % 256 == 0 && H % 256 == 0 && (2 * I) % 256 == 0 && kD == 128 &&
                   gemm_ws_bytes >= static_cast<size_t>(sms / 2) * 2 * 512 * 128 * sizeof(float);
+      const char* he = getenv("B200_GEMM_HYBRID");     // A/B knob: 0 keeps them on the stream-K kernel in its plain form
+      // Models narrower than 1024 stay there too: their steps are promised to give the same tokens with and without fused
+      // epilogues, which holds for forms that add the same pieces (hidden 512: 142 against 134 us for a step of 150 tokens, 224
+      // against 178 for 512).
+      whole_ok = fused2_ok && H >= 1024 && !(he && atoi(he) == 0);
     }
     const char* ce = getenv("B200_CHAIN");
     chain_ok = fused_ok && deferred_ok && (ce && atoi(ce) != 0) && chain_max_ctas(&chain_ctas) == 0 && chain_ctas >= 128 && chain_ctas >= sms / 2 * 2 &&
@@ -742,6 +753,7 @@ int Engine::init(const b200_config& c) {
 // ------------------------------------------------------------------ forward pass (fixed kernel sequence)
 int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* logits_out) {
   if (model) return forward_model(m, dbuf, nullptr);
+  if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("forward: a wait inside a projection ran out"); return B200_ERR_CUDA; }
   const int T = m.T;
   const int* ids = dbuf + m.off_ids;
   const int* pos = dbuf + m.off_pos;
@@ -781,7 +793,11 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
   }();
   const bool dfr = deferred_ok && !all_logits && T <= defer_max_t;
   PartialView pv_x = no_partials();  // partials of the GEMM whose output is `x` (o_proj / down_proj)
-  // Steps of more than 128 tokens (prefill bursts and mixed steps), per projection: when the launch has at least one
+  // Steps of more than 128 tokens (prefill bursts and mixed steps) take the whole-tile product: complete bf16 tensors for
+  // the norms and RoPE instead of fp32 pieces they have to add, and SiLU * up in gate_up's epilogue.  One Llama-3-8B layer,
+  // 2048 tokens, against the two forms below: gate_up 312 against 410 us, down 165 against 260, o 49 against 62.
+  const bool wh = whole_ok && dfr && T > 128;
+  // B200_GEMM_HYBRID=0 / B200_FUSED_PREFILL=0 keep the stream-K kernel's forms.  Per projection: when the launch has at least one
   // (256-row x token-tile) tile per CTA pair — gate_up at every T, nothing else at Llama-3-8B's shapes — the pair kernel
   // finishes its few split tiles in-kernel and the elementwise neighbour rides in its epilogue (gemm2 mode 2, epi_pass.cuh).
   // With fewer tiles than pairs every tile is cut into several pieces and one finisher per tile would serialise the
@@ -790,7 +806,7 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
   // Both forms round at the same points and add the pieces in the same order
   // (tests/test_fullsize_gpu.py::test_full_size_prefill_burst_step_matches_oracle compares them bit for bit).
   auto f2_bn = [&](const GemmPlan& pl) {   // token-tile size of the fused form, 0 = keep the segment form
-    if (!fused2_ok || all_logits || !dfr || T <= 128) return 0;
+    if (!fused2_ok || wh || all_logits || !dfr || T <= 128) return 0;
     const int bn = gemm_block_n_for(T);    // same tiles, ranges and piece order as the segment form: bit-identical results
     const int ntt = (T + bn - 1) / bn;
     const int tiles = (pl.N / 256) * ntt;
@@ -825,7 +841,7 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
     } else {
       P(B200_K_GEMM_QKV);
       if (!on(B200_K_GEMM_QKV)) {}
-      else if (dfr) rc |= gemm_def(ly.p_qkv, xm_normed, qkv, QKV, T, &pv); else rc |= gemm(ly.p_qkv, xm_normed, qkv, QKV, T);
+      else if (dfr && !wh) rc |= gemm_def(ly.p_qkv, xm_normed, qkv, QKV, T, &pv); else rc |= gemm(ly.p_qkv, xm_normed, qkv, QKV, T);
       Q();
       P(B200_K_ROPE); if (on(B200_K_ROPE)) rc |= rope_kv_write(qkv, pos, slots, cos_sin, kv_l, T, Hq, Hkv, cfg.max_model_len, stream, pv); Q();
       launched(1);
@@ -840,7 +856,7 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
       x_pending = false;
     } else {
       if (!on(B200_K_GEMM_O)) {}
-      else if (dfr) rc |= gemm_def(ly.p_o, xm_attn, x, H, T, &pv_x); else { rc |= gemm(ly.p_o, xm_attn, x, H, T); pv_x = no_partials(); }
+      else if (dfr && !wh) rc |= gemm_def(ly.p_o, xm_attn, x, H, T, &pv_x); else { rc |= gemm(ly.p_o, xm_attn, x, H, T); pv_x = no_partials(); }
       x_pending = true;
     }
     Q();
@@ -851,7 +867,12 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
     Q();
     launched(1);
     pv = no_partials();
-    if (const int bn = f2_bn(ly.p_gu)) {
+    if (wh) {
+      const int bn = gemm_block_n_for(T);
+      const GroupedOut g = {act, I, GROUPED_SILU};
+      ++stats.kernel_launches;
+      P(B200_K_GEMM_GU); if (on(B200_K_GEMM_GU)) rc |= gemm_whole_run(ly.p_gu, xmap(xm_normed, bn), bn, T, g, stream); Q();
+    } else if (const int bn = f2_bn(ly.p_gu)) {
       Gemm2Epi g;
       memset(&g, 0, sizeof(g));
       g.epi = GEMM3_EPI_SILU; g.out = act; g.ldo = I;
@@ -870,7 +891,7 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
       x_pending = false;
     } else {
       if (!on(B200_K_GEMM_DOWN)) {}
-      else if (dfr) rc |= gemm_def(ly.p_down, xm_act, x, H, T, &pv_x); else { rc |= gemm(ly.p_down, xm_act, x, H, T); pv_x = no_partials(); }
+      else if (dfr && !wh) rc |= gemm_def(ly.p_down, xm_act, x, H, T, &pv_x); else { rc |= gemm(ly.p_down, xm_act, x, H, T); pv_x = no_partials(); }
       x_pending = true;
     }
     Q();

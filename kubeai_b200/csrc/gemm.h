@@ -79,8 +79,9 @@ struct GroupedX { CUtensorMap box[kGroupedBoxes]; };
 // What happens to a sum s[r, n]: GROUPED_PLAIN / _RELU2 / _XIELU (a_pos = p0, a_neg = p1): y[r, n] = bf16(act(s + bias[n]));
 // GROUPED_F32: y[r, n] = s + bias[n] in fp32; GROUPED_GATED (limit p0, slope p1, up offset p2; the rows of every matrix alternate
 // in blocks of 64 gate rows and their 64 up rows, N % 128 == 0): g, u = bf16(s) of the two rows, y[r, i] = bf16(min(g, p0)
-// sigmoid(p1 min(g, p0)) (clamp(u, -p0, p0) + p2)), i < N / 2.  bias (optional): one matrix only.
-enum GroupedEpi { GROUPED_PLAIN = 0, GROUPED_RELU2, GROUPED_XIELU, GROUPED_F32, GROUPED_GATED };
+// sigmoid(p1 min(g, p0)) (clamp(u, -p0, p0) + p2)), i < N / 2; GROUPED_SILU: likewise bf16(bf16(silu(g)) u).  bias (optional): one
+// matrix only.
+enum GroupedEpi { GROUPED_PLAIN = 0, GROUPED_RELU2, GROUPED_XIELU, GROUPED_F32, GROUPED_GATED, GROUPED_SILU };
 struct GroupedOut {
   void* y;
   int ldy;

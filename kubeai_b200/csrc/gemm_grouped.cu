@@ -131,6 +131,11 @@ __device__ __forceinline__ float gated_unit(float g, float u, bool clamp, const 
   if (clamp) { g = fminf(g, o.p0); u = fminf(fmaxf(u, -o.p0), o.p0); }
   return __fdividef(g, 1.0f + __expf(-o.p1 * g)) * (u + o.p2);
 }
+// EPI 5: SiLU rounded to bf16 before the product, the rounding points of the Llama path's own kernel (elementwise.cu silu_mul)
+template <int EPI>
+__device__ __forceinline__ float gated(float g, float u, bool clamp, const GroupedOut& o) {
+  return EPI == 5 ? __bfloat162float(silu_bf16(g)) * u : gated_unit(g, u, clamp, o);
+}
 // Eight neighbouring columns of one row: the parts' sums added in their order.
 __device__ __forceinline__ void add_parts(float* v, const float* p, int step, int parts) {
 #pragma unroll
@@ -147,13 +152,13 @@ __device__ __forceinline__ void store8(bf16* p, const float* v) {
 // n rows of a split tile, their parts in shared memory, to the rows from row0 of the output: a thread takes eight columns of a row
 template <int EPI>
 __device__ __forceinline__ void finish_rows(const float* sums, int step, int parts, int n, int row0, int n0, int N, const GroupedOut& o, int et) {
-  constexpr int kPieces = EPI == 1 ? 8 : 16;
+  constexpr int kPieces = EPI == 1 || EPI == 5 ? 8 : 16;
   for (int it = et; it < n * kPieces; it += 128) {
     const int j = it / kPieces, c = (it % kPieces) * 8;
     const float* p = sums + j * kSlab + c;
     const size_t r = row0 + j;
     float v[8];
-    if constexpr (EPI == 1) {
+    if constexpr (EPI == 1 || EPI == 5) {
       if (n0 + kSlab > N) continue;
       float u[8];
       add_parts(v, p, step, parts);
@@ -161,12 +166,12 @@ __device__ __forceinline__ void finish_rows(const float* sums, int step, int par
       const bool clamp = o.p0 < INFINITY;
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        v[i] = gated_unit(__bfloat162float(__float2bfloat16_rn(v[i])), __bfloat162float(__float2bfloat16_rn(u[i])), clamp, o);
+        v[i] = gated<EPI>(__bfloat162float(__float2bfloat16_rn(v[i])), __bfloat162float(__float2bfloat16_rn(u[i])), clamp, o);
       store8(static_cast<bf16*>(o.y) + r * o.ldy + n0 / 2 + c, v);
     } else {
       if (n0 + c >= N) continue;
       add_parts(v, p, step, parts);
-      if (EPI >= 2 && o.bias) {
+      if (EPI <= 4 && EPI >= 2 && o.bias) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           if (n0 + c + i < N) v[i] += __ldg(o.bias + n0 + c + i);
@@ -205,7 +210,8 @@ __device__ __forceinline__ void finish_parts(float* ring, const float* first, si
   }
 }
 
-// EPI 0: bf16(sum); 1: the gated unit; 2: fp32 sum + bias; 3: bf16(relu2(sum + bias)), or without an activation; 4: bf16(xielu(sum + bias)).
+// EPI 0: bf16(sum); 1: the gated unit; 2: fp32 sum + bias; 3: bf16(relu2(sum + bias)), or without an activation; 4: bf16(xielu(sum + bias));
+// 5: the SiLU-gated unit with its inner rounding.
 // A form of its own for the plain product: looking the activation up per element made its drain a sixth of the launch longer.
 // FULL: 128-row boxes, their sizes known to the compiler.
 template <int EPI, bool FULL>
@@ -321,7 +327,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       tc_fence_after();
       const int n0 = t.n0 + static_cast<int>(rank) * kSlab;    // first column of this CTA's slab in the expert's output
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * kRows;
-      const float bias = EPI >= 2 && o.bias && n0 + row < N ? __ldg(o.bias + n0 + row) : 0.f;   // a thread's accumulator row is one output column
+      const float bias = EPI >= 2 && EPI <= 4 && o.bias && n0 + row < N ? __ldg(o.bias + n0 + row) : 0.f;   // a thread's accumulator row is one output column
       const bool relu2 = EPI == 3 && o.epi == GROUPED_RELU2;
       bool whole = true;
       if (split.parts > 1) {
@@ -367,7 +373,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           bf16* sb = reinterpret_cast<bf16*>(stage);
           auto put = [&](int j, uint32_t u) {
             float v = __uint_as_float(u);
-            if (EPI >= 3) v += bias;
+            if (EPI == 3 || EPI == 4) v += bias;
             if (EPI == 3) v = relu2 ? fmaxf(v, 0.f) * fmaxf(v, 0.f) : v;
             if (EPI == 4) v = xielu_fast(v, o.p0, o.p1);
             sb[j * kSlab + row] = __float2bfloat16_rn(v);
@@ -390,7 +396,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             if (j < left && n0 + c < N)
               *reinterpret_cast<float4*>(dst + static_cast<size_t>(j) * o.ldy + n0 + c) = *reinterpret_cast<const float4*>(sf + j * kSlab + c);
           }
-        } else if constexpr (EPI == 1) {
+        } else if constexpr (EPI == 1 || EPI == 5) {
           // rows 0..63 of the slab are gate rows, 64..127 the matching up rows: output columns n0 / 2 ..
           bf16* dst = static_cast<bf16*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
           const bf16* sb = reinterpret_cast<const bf16*>(stage);
@@ -404,8 +410,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
               uint32_t r[4];
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                r[k] = pack_bf16x2(gated_unit(__uint_as_float(gu[k] << 16), __uint_as_float(uu[k] << 16), clamp, o),
-                                   gated_unit(__uint_as_float(gu[k] & 0xffff0000u), __uint_as_float(uu[k] & 0xffff0000u), clamp, o));
+                r[k] = pack_bf16x2(gated<EPI>(__uint_as_float(gu[k] << 16), __uint_as_float(uu[k] << 16), clamp, o),
+                                   gated<EPI>(__uint_as_float(gu[k] & 0xffff0000u), __uint_as_float(uu[k] & 0xffff0000u), clamp, o));
               *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * o.ldy + n0 / 2 + c) = make_uint4(r[0], r[1], r[2], r[3]);
             }
           }
@@ -457,15 +463,16 @@ int gemm_grouped_x_maps(GroupedX* x, const void* X, int rows, int K) {
 namespace {
 int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap& tm_x, int box, const int* expert_rows, int rows, const GroupedOut& o,
            const SplitK& split, int units, int* error, cudaStream_t st) {
-  const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED;
+  const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED || o.epi == GROUPED_SILU;
   if ((!expert_rows && (experts != 1 || rows < 1)) || !o.y || o.ldy % (f32 ? 4 : 8) || N % (f32 ? 4 : 8) || reinterpret_cast<uintptr_t>(o.y) % 16 || units < 1 ||
       (gated && (N % kSlab || o.bias)) || (o.bias && experts != 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
-  static std::atomic<unsigned long long> attr[10];
+  static std::atomic<unsigned long long> attr[12];
   auto start = [&](auto kernel, int i) {
     if (!ensure_dynamic_smem(kernel, kSmem, &attr[i])) return -2;
     return launch_pdl(kernel, dim3(2 * units), dim3(kThreads), kSmem, st, tm_w, tm_x, expert_rows, experts, rows, o, N, K, box, split, error) == cudaSuccess ? 0 : -2;
   };
 #define RUN(E) return box == 128 ? start(gemm_grouped_kernel<E, true>, 2 * E) : start(gemm_grouped_kernel<E, false>, 2 * E + 1)
+  if (o.epi == GROUPED_SILU) RUN(5);
   if (gated) RUN(1);
   if (f32) RUN(2);
   if (o.epi == GROUPED_XIELU) RUN(4);

@@ -94,7 +94,10 @@ struct LayerWeights {
   void* e_gu = nullptr;     // [experts][2 ff][width]  gate rows, then up rows
   void* e_down = nullptr;   // [experts][width][ff]
   GemmPlan p_in, p_lo, p_ro, p_rg2;
-  std::vector<GemmPlan> p_egu, p_edown;
+  GroupedPlan g_egu, g_edown;
+  GroupedX xg_h, xg_act;     // views of the sorted rows and of the hidden rows
+  bool tc_experts = false;
+  bool il_e = false;         // bf16: an expert's gate and up rows alternate in blocks of 64
   CUtensorMap xm_lo[kGemmNumBlockN], xm_ro[kGemmNumBlockN];
   bool tc_in = false, tc_lo = false, tc_ro = false, tc_rg2 = false;
 };
@@ -135,7 +138,9 @@ class Nagilix : public Model {
   int *topi = nullptr, *sorted_rows = nullptr, *tile_group = nullptr, *pair_pos = nullptr, *iota = nullptr;
   int row_cap = 0, moe_cap = 0;
   void *hsorted = nullptr, *edown16 = nullptr;
-  int *expert_rows = nullptr, *expert_rows_host = nullptr;
+  int* expert_rows = nullptr;
+  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
+  int moe_tc_min = 1;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
@@ -149,10 +154,8 @@ class Nagilix : public Model {
       if (w.tc_lo) gemm_plan_destroy(&w.p_lo);
       if (w.tc_ro) gemm_plan_destroy(&w.p_ro);
       if (w.tc_rg2) gemm_plan_destroy(&w.p_rg2);
-      for (auto& p : w.p_egu) gemm_plan_destroy(&p);
-      for (auto& p : w.p_edown) gemm_plan_destroy(&p);
     }
-    if (expert_rows_host) cudaFreeHost(expert_rows_host);
+    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Nagilix"; }
@@ -434,46 +437,40 @@ class Nagilix : public Model {
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
     for (int i = 0; i < kGemmNumBlockN; ++i)
       if (gemm_make_x_map(&xm_h[i], h, env.Tcap, W, W, bns[i])) { use_tc = false; return 0; }
-    bool any_expert_tc = false;
-    for (size_t i = 0; i < spec.size(); ++i) {
-      const LayerSpec& s = spec[i];
-      LayerWeights& w = wts[i];
-      w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-      if (w.tc_in) w.p_in.ws_bytes = ws_bytes;
-      const int k_lo = s.kind == MIX_PARALLEL ? s.hv_l : s.m.inner;
-      w.tc_lo = k_lo % 8 == 0 && gemm_plan_init(&w.p_lo, w.w_lo, W, k_lo, k_lo, gemm_ws, gemm_counters, env.sms) == 0;
-      for (int j = 0; j < kGemmNumBlockN && w.tc_lo; ++j)
-        if (gemm_make_x_map(&w.xm_lo[j], yl, env.Tcap, k_lo, k_lo, bns[j])) w.tc_lo = false;
-      if (w.tc_lo) w.p_lo.ws_bytes = ws_bytes;
-      if (s.kind == MIX_PARALLEL) {
-        w.tc_ro = s.hv_r % 8 == 0 && gemm_plan_init(&w.p_ro, w.w_ro, W, s.hv_r, s.hv_r, gemm_ws, gemm_counters, env.sms) == 0;
-        for (int j = 0; j < kGemmNumBlockN && w.tc_ro; ++j)
-          if (gemm_make_x_map(&w.xm_ro[j], yr, env.Tcap, s.hv_r, s.hv_r, bns[j])) w.tc_ro = false;
-        if (w.tc_ro) w.p_ro.ws_bytes = ws_bytes;
-      }
-      if (s.mlp && gated) {
-        w.tc_rg2 = gemm_plan_init(&w.p_rg2, w.rg2, W, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-        if (w.tc_rg2) w.p_rg2.ws_bytes = ws_bytes;
-      }
-      if (s.mlp && s.experts > 0 && s.ff % 8 == 0) {
-        w.p_egu.resize(s.experts);
-        w.p_edown.resize(s.experts);
-        bool ok = true;
-        for (int e = 0; e < s.experts && ok; ++e) {
-          ok = gemm_plan_init(&w.p_egu[e], static_cast<bf16*>(w.e_gu) + static_cast<size_t>(e) * 2 * s.ff * W, 2 * s.ff, W, W, gemm_ws, gemm_counters, env.sms) == 0 &&
-               gemm_plan_init(&w.p_edown[e], static_cast<bf16*>(w.e_down) + static_cast<size_t>(e) * W * s.ff, W, s.ff, s.ff, gemm_ws, gemm_counters, env.sms) == 0;
-          w.p_egu[e].ws_bytes = w.p_edown[e].ws_bytes = ws_bytes;
-        }
-        if (!ok) { w.p_egu.clear(); w.p_edown.clear(); }
-        else any_expert_tc = true;
-      }
-    }
-    if (any_expert_tc) {
+    if (moe_cap) {
       int max_e = 1;
       for (auto& s : spec) max_e = std::max(max_e, s.experts + s.identity);
       if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
           dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
-      if (cudaMallocHost(&expert_rows_host, static_cast<size_t>(max_e) * 2 * sizeof(int)) != cudaSuccess) return -3;
+    }
+    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
+    *kernel_error = 0;
+    if (const char* e = getenv("B200_NG_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
+    for (size_t i = 0; i < spec.size(); ++i) {
+      const LayerSpec& s = spec[i];
+      LayerWeights& w = wts[i];
+      w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
+      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = kernel_error; }
+      const int k_lo = s.kind == MIX_PARALLEL ? s.hv_l : s.m.inner;
+      w.tc_lo = k_lo % 8 == 0 && gemm_plan_init(&w.p_lo, w.w_lo, W, k_lo, k_lo, gemm_ws, gemm_counters, env.sms) == 0;
+      for (int j = 0; j < kGemmNumBlockN && w.tc_lo; ++j)
+        if (gemm_make_x_map(&w.xm_lo[j], yl, env.Tcap, k_lo, k_lo, bns[j])) w.tc_lo = false;
+      if (w.tc_lo) { w.p_lo.ws_bytes = ws_bytes; w.p_lo.error = kernel_error; }
+      if (s.kind == MIX_PARALLEL) {
+        w.tc_ro = s.hv_r % 8 == 0 && gemm_plan_init(&w.p_ro, w.w_ro, W, s.hv_r, s.hv_r, gemm_ws, gemm_counters, env.sms) == 0;
+        for (int j = 0; j < kGemmNumBlockN && w.tc_ro; ++j)
+          if (gemm_make_x_map(&w.xm_ro[j], yr, env.Tcap, s.hv_r, s.hv_r, bns[j])) w.tc_ro = false;
+        if (w.tc_ro) { w.p_ro.ws_bytes = ws_bytes; w.p_ro.error = kernel_error; }
+      }
+      if (s.mlp && gated) {
+        w.tc_rg2 = gemm_plan_init(&w.p_rg2, w.rg2, W, W, W, gemm_ws, gemm_counters, env.sms) == 0;
+        if (w.tc_rg2) { w.p_rg2.ws_bytes = ws_bytes; w.p_rg2.error = kernel_error; }
+      }
+      if (s.mlp && s.experts > 0) {
+        w.tc_experts = !gemm_grouped_plan(&w.g_egu, w.e_gu, s.experts, 2 * s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
+                       !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);
+        w.il_e = w.tc_experts && s.ff % 64 == 0;
+      }
     }
     return 0;
   }
@@ -498,6 +495,17 @@ class Nagilix : public Model {
     }
     uint8_t* d = static_cast<uint8_t*>(dst) + (row0 * ld + col0) * es;
     return cudaMemcpy2D(d, ld * es, tmp.data(), cols * es, cols * es, rows, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -2;
+  }
+  // gate and up rows [F, cols] each, one below the other or in alternating blocks of 64
+  int put_pair(void* dst, size_t row0, const std::vector<float>& gate, const std::vector<float>& up, size_t F, size_t cols, bool in_turns) {
+    std::vector<float> both;
+    both.reserve(2 * F * cols);
+    const size_t block = (in_turns ? 64 : F) * cols;
+    for (size_t at = 0; at < F * cols; at += block) {
+      both.insert(both.end(), gate.begin() + at, gate.begin() + at + block);
+      both.insert(both.end(), up.begin() + at, up.begin() + at + block);
+    }
+    return put(dst, cols, row0, 0, both, 2 * F, cols);
   }
   int putf(float* dst, const std::vector<float>& src) {
     return cudaMemcpy(dst, src.data(), src.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -2;
@@ -585,8 +593,10 @@ class Nagilix : public Model {
       VEC(f + "correction", w.correction, s.experts + s.identity);
       for (int e = 0; e < s.experts; ++e) {
         const std::string ep = f + "e" + std::to_string(e) + ".";
-        MAT(ep + "gate", w.e_gu, W, static_cast<size_t>(e) * 2 * s.ff, 0, s.ff, W);
-        MAT(ep + "up", w.e_gu, W, static_cast<size_t>(e) * 2 * s.ff + s.ff, 0, s.ff, W);
+        if (!get(ep + "gate", s.ff, W)) return -4;
+        const std::vector<float> gate(v);
+        if (!get(ep + "up", s.ff, W)) return -4;
+        rc |= put_pair(w.e_gu, static_cast<size_t>(e) * 2 * s.ff, gate, v, s.ff, W, w.il_e);
         MAT(ep + "down", w.e_down, s.ff, static_cast<size_t>(e) * W, 0, W, s.ff);
       }
     }
@@ -781,8 +791,7 @@ class Nagilix : public Model {
     KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, ne, W), st));
     KRN("moe_route", moe_route(scores, topi, topw, T, ne, 1, 1, s.top, st, MOE_SOFTMAX, ne, w.correction));
     const long long gu_stride = 2ll * s.ff * W, down_stride = static_cast<long long>(W) * s.ff;
-    static const int moe_tc_min = [] { const char* e = getenv("B200_NG_MOE_TC_MIN_T"); return e ? atoi(e) : 256; }();   // A/B knob
-    const bool per_expert = !w.p_egu.empty() && T >= moe_tc_min;
+    const bool grouped = w.tc_experts && T >= moe_tc_min;
     if (s.experts == 0) {
       // nothing but identity experts: the output is the input times the sum of the chosen weights
       KRN("moe_combine", moe_combine_identity(h, dt, iota, topw, topi, 0, h, fo, dt, T, s.top, W, st));
@@ -795,7 +804,7 @@ class Nagilix : public Model {
       PickedRows pu = {T * s.top, nullptr, s.top, iota, topi};
       pu.group_limit = s.experts;
       KRN("moe_up", linear_picked_rows(up, pu, st));
-      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, T * s.top, s.ff, s.limit, 1.702f, st));
+      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, T * s.top, s.ff, s.limit, 1.702f, st, 1.0f, w.il_e));
       LinearArgs dn = linear_args(eact, dt, w.e_down, dt, edown, DT_F32, T * s.top, W, s.ff);
       dn.wbs = down_stride;
       PickedRows pd = {T * s.top, iota, 1, iota, topi};
@@ -806,44 +815,29 @@ class Nagilix : public Model {
       return rc;
     }
     const int cap = (T * s.top + 63) / 64 * 64 + ne * 64;
-    KRN("moe_align", moe_align(topi, T, s.top, ne, sorted_rows, tile_group, pair_pos, cap, st, per_expert ? expert_rows : nullptr, nullptr, nullptr, s.experts));
-    if (per_expert) {
-      // Large steps: every expert's rows are one tcgen05 GEMM.  The row counts come back to the host (one small copy and a
-      // wait per layer, paid only by steps of hundreds of tokens); the inputs are gathered into sorted order.
-      KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st, nullptr));
-      if (cudaMemcpyAsync(expert_rows_host, expert_rows, static_cast<size_t>(ne) * 2 * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess) rc = -2;
-      prof_start();
-      for (int e = 0; e < s.experts && !rc; ++e) {
-        const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-        if (cnt <= 0) continue;
-        const int bn = gemm_block_n_for(cnt);
-        CUtensorMap tm;
-        if (gemm_make_x_map(&tm, static_cast<bf16*>(hsorted) + static_cast<size_t>(start) * W, cnt, W, W, bn)) { rc = -2; break; }
-        rc |= gemm_run(w.p_egu[e], tm, bn, static_cast<bf16*>(egu) + static_cast<size_t>(start) * 2 * s.ff, 2 * s.ff, cnt, st);
-        ++nl;
+    KRN("moe_align", moe_align(topi, T, s.top, ne, sorted_rows, tile_group, pair_pos, cap, st, grouped ? expert_rows : nullptr, nullptr, nullptr, s.experts));
+    if (grouped) {
+      // the inputs in expert-sorted order, then one grouped GEMM per matrix; the row counts stay on the device.  Identity experts
+      // come last in the order and have no rows of a matrix.  Steps of fewer than 256 tokens keep the outputs in fp32.
+      const bool wide = T < 256;
+      KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
+      if (w.il_e) {
+        const GroupedOut up = {eact, s.ff, GROUPED_GATED, nullptr, s.limit, 1.702f, 1.0f};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+      } else {
+        const GroupedOut up = {egu, 2 * s.ff};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+        KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
       }
-      prof_stop("moe_up");
-      const int real_rows = expert_rows_host[2 * (s.experts - 1)] + (expert_rows_host[2 * (s.experts - 1) + 1] + 63) / 64 * 64;   // rows of experts with matrices
-      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, real_rows, s.ff, s.limit, 1.702f, st));
-      prof_start();
-      for (int e = 0; e < s.experts && !rc; ++e) {
-        const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-        if (cnt <= 0) continue;
-        const int bn = gemm_block_n_for(cnt);
-        CUtensorMap tm;
-        if (gemm_make_x_map(&tm, static_cast<bf16*>(eact) + static_cast<size_t>(start) * s.ff, cnt, s.ff, s.ff, bn)) { rc = -2; break; }
-        rc |= gemm_run(w.p_edown[e], tm, bn, static_cast<bf16*>(edown16) + static_cast<size_t>(start) * W, W, cnt, st);
-        ++nl;
-      }
-      prof_stop("moe_down");
-      KRN("moe_combine", moe_combine_identity(edown16, DT_BF16, pair_pos, topw, topi, s.experts, h, fo, dt, T, s.top, W, st));
+      const GroupedOut dn = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, kernel_error, st));
+      KRN("moe_combine", moe_combine_identity(dn.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, topi, s.experts, h, fo, dt, T, s.top, W, st));
       return rc;
     }
     LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, cap, 2 * s.ff, W);
     up.x_rows = sorted_rows; up.tile_group = tile_group; up.wbs = gu_stride;
     KRN("moe_up", linear(up, st));
-    KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
+    KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st, 1.0f, w.il_e));
     LinearArgs dn = linear_args(eact, dt, w.e_down, dt, edown, DT_F32, cap, W, s.ff);
     dn.tile_group = tile_group; dn.wbs = down_stride;
     KRN("moe_down", linear(dn, st));
@@ -858,6 +852,7 @@ class Nagilix : public Model {
     int64_t nl = 0;
     const size_t es = dtype_bytes(dt);
     auto col = [&](void* base, size_t off) { return static_cast<void*>(static_cast<uint8_t*>(base) + off * es); };
+    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Nagilix forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_learned_pos(embed, pos_table, dt, b.ids, b.pos, x, T, W, V, max_pos, ns, xstride, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {

@@ -69,9 +69,10 @@ struct LayerWeights {
   void* e_up = nullptr;    // [experts][ff][width]
   void* e_down = nullptr;  // [experts][width][ff]
   GemmPlan p_in, p_out;    // tcgen05 projections (bf16 storage, K % 8 == 0)
-  std::vector<GemmPlan> p_eup, p_edown;   // per expert, for steps large enough to pay for a count read-back
+  GroupedPlan g_eup, g_edown;
+  GroupedX xg_h, xg_act;     // views of the sorted rows and of the hidden rows
   CUtensorMap xm_out[kGemmNumBlockN];   // activation maps over the output projection's input [Tcap, k_out]
-  bool tc_in = false, tc_out = false;
+  bool tc_in = false, tc_out = false, tc_experts = false;
 };
 
 struct LayerRun {
@@ -109,8 +110,10 @@ class Nomanex : public Model {
   int row_cap = 0, moe_cap = 0;
   float* split_ws = nullptr;       // partials of the split attention form (decode of a few long sequences)
   long long split_ws_floats = 0;
-  void *hsorted = nullptr, *edown16 = nullptr;   // per-expert tensor-core path: gathered inputs, bf16 expert outputs
-  int *expert_rows = nullptr, *expert_rows_host = nullptr;
+  void *hsorted = nullptr, *edown16 = nullptr;   // tensor-core experts: gathered inputs, bf16 expert outputs
+  int* expert_rows = nullptr;
+  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
+  int moe_tc_min = 1;
   std::vector<void*> allocs;
   // tcgen05 projections
   float* gemm_ws = nullptr;
@@ -124,7 +127,7 @@ class Nomanex : public Model {
       if (w.tc_in) gemm_plan_destroy(&w.p_in);
       if (w.tc_out) gemm_plan_destroy(&w.p_out);
     }
-    if (expert_rows_host) cudaFreeHost(expert_rows_host);
+    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   // (profiling events are released with the context)
@@ -381,34 +384,28 @@ class Nomanex : public Model {
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
     for (int i = 0; i < kGemmNumBlockN; ++i)
       if (gemm_make_x_map(&xm_h[i], h, env.Tcap, W, W, bns[i])) { use_tc = false; return 0; }
-    for (size_t i = 0; i < spec.size(); ++i) {
-      const LayerSpec& s = spec[i];
-      if (s.weights_of != static_cast<int>(i)) continue;
-      LayerWeights& w = wts[i];
-      w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-      if (w.tc_in) w.p_in.ws_bytes = ws_bytes;
-      w.tc_out = s.k_out % 8 == 0 && gemm_plan_init(&w.p_out, w.w_out, W, s.k_out, s.k_out, gemm_ws, gemm_counters, env.sms) == 0;
-      for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
-        if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
-      if (w.tc_out) w.p_out.ws_bytes = ws_bytes;
-      if (s.ff_kind == FF_MOE && s.ff % 8 == 0) {
-        w.p_eup.resize(s.experts);
-        w.p_edown.resize(s.experts);
-        bool ok = true;
-        for (int e = 0; e < s.experts && ok; ++e) {
-          ok = gemm_plan_init(&w.p_eup[e], static_cast<bf16*>(w.e_up) + static_cast<size_t>(e) * s.ff * W, s.ff, W, W, gemm_ws, gemm_counters, env.sms) == 0 &&
-               gemm_plan_init(&w.p_edown[e], static_cast<bf16*>(w.e_down) + static_cast<size_t>(e) * W * s.ff, W, s.ff, s.ff, gemm_ws, gemm_counters, env.sms) == 0;
-          w.p_eup[e].ws_bytes = w.p_edown[e].ws_bytes = ws_bytes;
-        }
-        if (!ok) { w.p_eup.clear(); w.p_edown.clear(); }
-      }
-    }
     if (moe_cap) {
       int max_e = 1;
       for (auto& s : spec) max_e = std::max(max_e, s.experts);
       if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
           dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
-      if (cudaMallocHost(&expert_rows_host, static_cast<size_t>(max_e) * 2 * sizeof(int)) != cudaSuccess) return -3;
+    }
+    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
+    *kernel_error = 0;
+    if (const char* e = getenv("B200_NX_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
+    for (size_t i = 0; i < spec.size(); ++i) {
+      const LayerSpec& s = spec[i];
+      if (s.weights_of != static_cast<int>(i)) continue;
+      LayerWeights& w = wts[i];
+      w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
+      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = kernel_error; }
+      w.tc_out = s.k_out % 8 == 0 && gemm_plan_init(&w.p_out, w.w_out, W, s.k_out, s.k_out, gemm_ws, gemm_counters, env.sms) == 0;
+      for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
+        if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
+      if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = kernel_error; }
+      if (s.ff_kind == FF_MOE)
+        w.tc_experts = !gemm_grouped_plan(&w.g_eup, w.e_up, s.experts, s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
+                       !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);
     }
     return 0;
   }
@@ -592,6 +589,7 @@ class Nomanex : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
+    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Nomanex forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_bigram(embed, bigram, dt, b.ids, b.prev_ids, x, T, W, V, buckets, mul_prev, mul_cur, st));
     const LayerWeights& w0 = wts[spec[0].weights_of];
     KRN("residual_norm", residual_dyt(x, nullptr, nullptr, dt, 0.f, w0.norm_w, w0.norm_b, w0.norm_alpha, h, dt, nullptr, T, W, st));
@@ -653,41 +651,19 @@ class Nomanex : public Model {
         KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, s.experts, W), st));
         KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, s.groups, s.keep, s.top, st));
         const int cap = (T * s.top + 63) / 64 * 64 + s.experts * 64;
-        const char* mte = getenv("B200_NX_MOE_TC_MIN_T");   // A/B knob
-        const int moe_tc_min = mte ? atoi(mte) : 256;
-        const bool per_expert = !w.p_eup.empty() && T >= moe_tc_min;
-        KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, per_expert ? expert_rows : nullptr));
-        if (per_expert) {
-          // Large steps: every expert's rows are one tcgen05 GEMM.  The row counts come back to the host (one small copy
-          // and a wait per layer, paid only by steps of hundreds of tokens), the inputs are gathered into sorted order.
+        const bool grouped = w.tc_experts && T >= moe_tc_min && T * s.top > 64;
+        KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, grouped ? expert_rows : nullptr));
+        if (grouped) {
+          // the inputs in expert-sorted order, then one grouped GEMM per matrix, the activation in the first one's epilogue; the
+          // row counts stay on the device.  Steps of fewer than 256 tokens keep the experts' outputs in fp32 until the combine.
+          const bool wide = T < 256;
           KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
-          if (cudaMemcpyAsync(expert_rows_host, expert_rows, static_cast<size_t>(s.experts) * 2 * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-              cudaStreamSynchronize(st) != cudaSuccess) rc = -2;
-          prof_start();
-          for (int e = 0; e < s.experts && !rc; ++e) {
-            const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-            if (cnt <= 0) continue;
-            const int bn = gemm_block_n_for(cnt);
-            CUtensorMap tm;
-            if (gemm_make_x_map(&tm, static_cast<bf16*>(hsorted) + static_cast<size_t>(start) * W, cnt, W, W, bn)) { rc = -2; break; }
-            rc |= gemm_run(w.p_eup[e], tm, bn, static_cast<bf16*>(eact) + static_cast<size_t>(start) * s.ff, s.ff, cnt, st);
-            ++nl;
-          }
-          prof_stop("moe_up");
-          KRN("moe_act", relu2_bf16(eact, static_cast<long long>(cap) * s.ff, st));
-          prof_start();
-          for (int e = 0; e < s.experts && !rc; ++e) {
-            const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-            if (cnt <= 0) continue;
-            const int bn = gemm_block_n_for(cnt);
-            CUtensorMap tm;
-            if (gemm_make_x_map(&tm, static_cast<bf16*>(eact) + static_cast<size_t>(start) * s.ff, cnt, s.ff, s.ff, bn)) { rc = -2; break; }
-            rc |= gemm_run(w.p_edown[e], tm, bn, static_cast<bf16*>(edown16) + static_cast<size_t>(start) * W, W, cnt, st);
-            ++nl;
-          }
-          prof_stop("moe_down");
-          KRN("moe_combine", moe_combine(edown16, DT_BF16, pair_pos, topw, fo, dt, T, s.top, W, st));
-          nl += 5;
+          const GroupedOut up = {eact, s.ff, GROUPED_RELU2};
+          KRN("moe_up", gemm_grouped_run(w.g_eup, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+          const GroupedOut dn = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
+          KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, kernel_error, st));
+          KRN("moe_combine", moe_combine(dn.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, fo, dt, T, s.top, W, st));
+          nl += 4;
         } else if (T * s.top <= 64) {
           // decode-sized steps: one weight-streaming pass per chosen (token, expert) pair
           LinearArgs up = linear_args(h, dt, w.e_up, dt, eact, dt, T * s.top, s.ff, W);

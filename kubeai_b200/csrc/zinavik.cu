@@ -81,7 +81,10 @@ struct LayerWeights {
   void* sh_in = nullptr;   // [n_sh, width]: gate [sff] | up [sff]
   void* sh_down = nullptr; // [width, sff]
   GemmPlan p_in, p_out, p_shin, p_shdown;
-  std::vector<GemmPlan> p_egu, p_edown;
+  GroupedPlan g_egu, g_edown;
+  GroupedX xg_h, xg_act;     // views of the sorted rows and of the hidden rows
+  bool tc_experts = false;
+  bool il_e = false;         // bf16: an expert's gate and up rows alternate in blocks of 64
   CUtensorMap xm_out[kGemmNumBlockN], xm_shact[kGemmNumBlockN];
   bool tc_in = false, tc_out = false, tc_shin = false, tc_shdown = false;
 };
@@ -121,7 +124,9 @@ class Zinavik : public Model {
   int *topi = nullptr, *sorted_rows = nullptr, *tile_group = nullptr, *pair_pos = nullptr, *iota = nullptr;
   int row_cap = 0, moe_cap = 0;
   void *hsorted = nullptr, *edown16 = nullptr;
-  int *expert_rows = nullptr, *expert_rows_host = nullptr;
+  int* expert_rows = nullptr;
+  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
+  int moe_tc_min = 256;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
@@ -135,10 +140,8 @@ class Zinavik : public Model {
       if (w.tc_out) gemm_plan_destroy(&w.p_out);
       if (w.tc_shin) gemm_plan_destroy(&w.p_shin);
       if (w.tc_shdown) gemm_plan_destroy(&w.p_shdown);
-      for (auto& p : w.p_egu) gemm_plan_destroy(&p);
-      for (auto& p : w.p_edown) gemm_plan_destroy(&p);
     }
-    if (expert_rows_host) cudaFreeHost(expert_rows_host);
+    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Zinavik"; }
@@ -403,43 +406,37 @@ class Zinavik : public Model {
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
     for (int i = 0; i < kGemmNumBlockN; ++i)
       if (gemm_make_x_map(&xm_h[i], h, env.Tcap, W, W, bns[i])) { use_tc = false; return 0; }
-    bool any_expert_tc = false;
-    for (size_t i = 0; i < spec.size(); ++i) {
-      const LayerSpec& s = spec[i];
-      LayerWeights& w = wts[i];
-      w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-      if (w.tc_in) w.p_in.ws_bytes = ws_bytes;
-      w.tc_out = s.k_out % 8 == 0 && gemm_plan_init(&w.p_out, w.w_out, W, s.k_out, s.k_out, gemm_ws, gemm_counters, env.sms) == 0;
-      for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
-        if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
-      if (w.tc_out) w.p_out.ws_bytes = ws_bytes;
-      if (s.mlp && s.shared) {
-        w.tc_shin = gemm_plan_init(&w.p_shin, w.sh_in, s.n_sh, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-        if (w.tc_shin) w.p_shin.ws_bytes = ws_bytes;
-        w.tc_shdown = s.sff % 8 == 0 && gemm_plan_init(&w.p_shdown, w.sh_down, W, s.sff, s.sff, gemm_ws, gemm_counters, env.sms) == 0;
-        for (int j = 0; j < kGemmNumBlockN && w.tc_shdown; ++j)
-          if (gemm_make_x_map(&w.xm_shact[j], shact, env.Tcap, s.sff, s.sff, bns[j])) w.tc_shdown = false;
-        if (w.tc_shdown) w.p_shdown.ws_bytes = ws_bytes;
-      }
-      if (s.mlp && s.ff % 8 == 0) {
-        w.p_egu.resize(s.experts);
-        w.p_edown.resize(s.experts);
-        bool ok = true;
-        for (int e = 0; e < s.experts && ok; ++e) {
-          ok = gemm_plan_init(&w.p_egu[e], static_cast<bf16*>(w.e_gu) + static_cast<size_t>(e) * 2 * s.ff * W, 2 * s.ff, W, W, gemm_ws, gemm_counters, env.sms) == 0 &&
-               gemm_plan_init(&w.p_edown[e], static_cast<bf16*>(w.e_down) + static_cast<size_t>(e) * W * s.ff, W, s.ff, s.ff, gemm_ws, gemm_counters, env.sms) == 0;
-          w.p_egu[e].ws_bytes = w.p_edown[e].ws_bytes = ws_bytes;
-        }
-        if (!ok) { w.p_egu.clear(); w.p_edown.clear(); }
-        else any_expert_tc = true;
-      }
-    }
-    if (any_expert_tc) {
+    if (moe_cap) {
       int max_e = 1;
       for (auto& s : spec) max_e = std::max(max_e, s.experts);
       if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
           dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
-      if (cudaMallocHost(&expert_rows_host, static_cast<size_t>(max_e) * 2 * sizeof(int)) != cudaSuccess) return -3;
+    }
+    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
+    *kernel_error = 0;
+    if (const char* e = getenv("B200_ZV_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
+    for (size_t i = 0; i < spec.size(); ++i) {
+      const LayerSpec& s = spec[i];
+      LayerWeights& w = wts[i];
+      w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
+      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = kernel_error; }
+      w.tc_out = s.k_out % 8 == 0 && gemm_plan_init(&w.p_out, w.w_out, W, s.k_out, s.k_out, gemm_ws, gemm_counters, env.sms) == 0;
+      for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
+        if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
+      if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = kernel_error; }
+      if (s.mlp && s.shared) {
+        w.tc_shin = gemm_plan_init(&w.p_shin, w.sh_in, s.n_sh, W, W, gemm_ws, gemm_counters, env.sms) == 0;
+        if (w.tc_shin) { w.p_shin.ws_bytes = ws_bytes; w.p_shin.error = kernel_error; }
+        w.tc_shdown = s.sff % 8 == 0 && gemm_plan_init(&w.p_shdown, w.sh_down, W, s.sff, s.sff, gemm_ws, gemm_counters, env.sms) == 0;
+        for (int j = 0; j < kGemmNumBlockN && w.tc_shdown; ++j)
+          if (gemm_make_x_map(&w.xm_shact[j], shact, env.Tcap, s.sff, s.sff, bns[j])) w.tc_shdown = false;
+        if (w.tc_shdown) { w.p_shdown.ws_bytes = ws_bytes; w.p_shdown.error = kernel_error; }
+      }
+      if (s.mlp) {
+        w.tc_experts = !gemm_grouped_plan(&w.g_egu, w.e_gu, s.experts, 2 * s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
+                       !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);
+        w.il_e = w.tc_experts && s.ff % 64 == 0;
+      }
     }
     return 0;
   }
@@ -467,6 +464,17 @@ class Zinavik : public Model {
     }
     uint8_t* d = static_cast<uint8_t*>(dst) + (row0 * ld + col0) * es;
     return cudaMemcpy2D(d, ld * es, tmp.data(), cols * es, cols * es, rows, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -2;
+  }
+  // gate and up rows [F, cols] each, one below the other or in alternating blocks of 64
+  int put_pair(void* dst, size_t row0, const std::vector<float>& gate, const std::vector<float>& up, size_t F, size_t cols, bool in_turns) {
+    std::vector<float> both;
+    both.reserve(2 * F * cols);
+    const size_t block = (in_turns ? 64 : F) * cols;
+    for (size_t at = 0; at < F * cols; at += block) {
+      both.insert(both.end(), gate.begin() + at, gate.begin() + at + block);
+      both.insert(both.end(), up.begin() + at, up.begin() + at + block);
+    }
+    return put(dst, cols, row0, 0, both, 2 * F, cols);
   }
   int putf(float* dst, const std::vector<float>& src) {
     return cudaMemcpy(dst, src.data(), src.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -2;
@@ -514,8 +522,10 @@ class Zinavik : public Model {
       MAT(f + "router", w.router, W, 0, 0, s.experts, W);
       for (int e = 0; e < s.experts; ++e) {
         const std::string ep = f + "e" + std::to_string(e) + ".";
-        MAT(ep + "gate", w.e_gu, W, static_cast<size_t>(e) * 2 * s.ff, 0, s.ff, W);
-        MAT(ep + "up", w.e_gu, W, static_cast<size_t>(e) * 2 * s.ff + s.ff, 0, s.ff, W);
+        if (!get(ep + "gate", s.ff, W)) return -4;
+        const std::vector<float> gate(v);
+        if (!get(ep + "up", s.ff, W)) return -4;
+        rc |= put_pair(w.e_gu, static_cast<size_t>(e) * 2 * s.ff, gate, v, s.ff, W, w.il_e);
         MAT(ep + "down", w.e_down, s.ff, static_cast<size_t>(e) * W, 0, W, s.ff);
       }
       if (s.shared) {
@@ -621,15 +631,14 @@ class Zinavik : public Model {
       shared_gate = scores + s.experts;
     }
     const long long gu_stride = 2ll * s.ff * W, down_stride = static_cast<long long>(W) * s.ff;
-    static const int moe_tc_min = [] { const char* e = getenv("B200_ZV_MOE_TC_MIN_T"); return e ? atoi(e) : 256; }();   // A/B knob
-    const bool per_expert = !w.p_egu.empty() && T >= moe_tc_min;
+    const bool grouped = w.tc_experts && T >= moe_tc_min;
     if (T * s.top <= 64) {
       // decode-sized steps: one weight-streaming pass per chosen (token, expert) pair, rows in pair order
       LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, T * s.top, 2 * s.ff, W);
       up.wbs = gu_stride; up.row_scale = topw;
       const PickedRows pu = {T * s.top, nullptr, s.top, iota, topi};
       KRN("moe_up", linear_picked_rows(up, pu, st));
-      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, T * s.top, s.ff, s.limit, 1.702f, st));
+      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, T * s.top, s.ff, s.limit, 1.702f, st, 1.0f, w.il_e));
       LinearArgs dn = linear_args(eact, dt, w.e_down, dt, edown, DT_F32, T * s.top, W, s.ff);
       dn.wbs = down_stride;
       const PickedRows pd = {T * s.top, iota, 1, iota, topi};
@@ -639,44 +648,28 @@ class Zinavik : public Model {
       return rc;
     }
     const int cap = (T * s.top + 63) / 64 * 64 + s.experts * 64;
-    KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, per_expert ? expert_rows : nullptr, topw, sorted_w));
-    if (per_expert) {
-      // Large steps: every expert's rows are one tcgen05 GEMM.  The row counts come back to the host (one small copy and a
-      // wait per layer, paid only by steps of hundreds of tokens); the inputs are gathered into sorted order, scaled by
-      // their router weight in fp32 and rounded once.
+    KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, grouped ? expert_rows : nullptr, topw, sorted_w));
+    if (grouped) {
+      // Large steps: the inputs in expert-sorted order, scaled by their router weight in fp32 and rounded once, then one grouped
+      // GEMM per matrix; the row counts stay on the device.  Smaller steps keep that scale on the fp32 sums (below).
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st, sorted_w));
-      if (cudaMemcpyAsync(expert_rows_host, expert_rows, static_cast<size_t>(s.experts) * 2 * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess) rc = -2;
-      prof_start();
-      for (int e = 0; e < s.experts && !rc; ++e) {
-        const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-        if (cnt <= 0) continue;
-        const int bn = gemm_block_n_for(cnt);
-        CUtensorMap tm;
-        if (gemm_make_x_map(&tm, static_cast<bf16*>(hsorted) + static_cast<size_t>(start) * W, cnt, W, W, bn)) { rc = -2; break; }
-        rc |= gemm_run(w.p_egu[e], tm, bn, static_cast<bf16*>(egu) + static_cast<size_t>(start) * 2 * s.ff, 2 * s.ff, cnt, st);
-        ++nl;
+      if (w.il_e) {
+        const GroupedOut up = {eact, s.ff, GROUPED_GATED, nullptr, s.limit, 1.702f, 1.0f};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+      } else {
+        const GroupedOut up = {egu, 2 * s.ff};
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+        KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
       }
-      prof_stop("moe_up");
-      KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
-      prof_start();
-      for (int e = 0; e < s.experts && !rc; ++e) {
-        const int start = expert_rows_host[2 * e], cnt = expert_rows_host[2 * e + 1];
-        if (cnt <= 0) continue;
-        const int bn = gemm_block_n_for(cnt);
-        CUtensorMap tm;
-        if (gemm_make_x_map(&tm, static_cast<bf16*>(eact) + static_cast<size_t>(start) * s.ff, cnt, s.ff, s.ff, bn)) { rc = -2; break; }
-        rc |= gemm_run(w.p_edown[e], tm, bn, static_cast<bf16*>(edown16) + static_cast<size_t>(start) * W, W, cnt, st);
-        ++nl;
-      }
-      prof_stop("moe_down");
+      const GroupedOut dn = {edown16, W};
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, kernel_error, st));
       KRN("moe_combine", moe_combine_add(edown16, DT_BF16, pair_pos, nullptr, shared_out, shared_gate, nr, fo, dt, T, s.top, W, st));
       return rc;
     }
     LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, cap, 2 * s.ff, W);
     up.x_rows = sorted_rows; up.tile_group = tile_group; up.wbs = gu_stride; up.row_scale = sorted_w;
     KRN("moe_up", linear(up, st));
-    KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
+    KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st, 1.0f, w.il_e));
     LinearArgs dn = linear_args(eact, dt, w.e_down, dt, edown, DT_F32, cap, W, s.ff);
     dn.tile_group = tile_group; dn.wbs = down_stride;
     KRN("moe_down", linear(dn, st));
@@ -694,6 +687,7 @@ class Zinavik : public Model {
     int64_t nl = 0;
     const size_t es = dtype_bytes(dt);
     auto col = [&](void* base, size_t off) { return static_cast<void*>(static_cast<uint8_t*>(base) + off * es); };
+    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Zinavik forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_scaled(embed, dt, b.ids, x, T, W, V, emb_scale, ns, xstride, st));
     Pending pend;
     for (size_t ri = 0; ri < run.size() && !rc; ++ri) {

@@ -109,8 +109,7 @@ class Soselix : public Model {
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
-  int* gemm_flags = nullptr;     // of the fused form: two per CTA pair, stamped with the launch's number
-  int gemm_epoch = 0;
+  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   bool fuse = true;
   int few_rows = 16;
   CUtensorMap xm_h[kGemmNumBlockN];
@@ -126,6 +125,7 @@ class Soselix : public Model {
       if (w.tc_down) gemm_plan_destroy(&w.p_down);
     }
     if (pe0) { cudaEventDestroy(pe0); cudaEventDestroy(pe1); }
+    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Soselix"; }
@@ -244,7 +244,7 @@ class Soselix : public Model {
       s.rec_floats = static_cast<size_t>(HD) * s.vdim;
     }
     s.n_in = at;
-    // a wide row is filled up to whole 256-row weight tiles (rows of zeros nobody reads), which the fused GEMM form asks for
+    // a wide row is filled up to whole 256-row weight tiles (rows of zeros nobody reads)
     const int full = (at + 255) / 256 * 256;
     if (at >= 1024 && full - at <= at / 8) s.n_in = full;
   }
@@ -360,7 +360,8 @@ class Soselix : public Model {
     const size_t ws_bytes = std::max(gemm_workspace_bytes(env.sms), gemm_deferred_ws_bytes(env.sms));
     if (dalloc(&gemm_ws, ws_bytes)) return -3;
     const size_t n_counters = 2ull * (maxN / 128 + 2) * (env.Tcap / 32 + 2);
-    if (dalloc(&gemm_counters, n_counters * sizeof(int)) || dalloc(&gemm_flags, static_cast<size_t>(env.sms) * 2 * sizeof(int))) return -3;
+    if (dalloc(&gemm_counters, n_counters * sizeof(int)) || cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
+    *kernel_error = 0;
     if (const char* e = getenv("B200_SX_FUSE")) fuse = atoi(e) != 0;              // A/B knobs
     if (const char* e = getenv("B200_SX_FEW_ROWS")) few_rows = atoi(e);
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
@@ -372,6 +373,7 @@ class Soselix : public Model {
     auto plan = [&](GemmPlan* p, const void* Wm, int N, int K) {
       if (N % 8 || K % 8 || gemm_plan_init(p, Wm, N, K, K, gemm_ws, gemm_counters, env.sms)) return false;
       p->ws_bytes = ws_bytes;
+      p->error = kernel_error;
       return true;
     };
     if (!maps(xm_h, h, W)) { use_tc = false; return 0; }
@@ -539,23 +541,17 @@ class Soselix : public Model {
 
   // ------------------------------------------------------------ forward
   // Y = X W^T, with bias and xIELU behind it where the epilogue is given.  Steps of up to 16 tokens stream the weights through
-  // linear.cu's fragment kernel.  Larger steps take the pair GEMM; in its fused form (whole 256-row tiles, at least one tile
-  // per CTA pair) every tile leaves through the epilogue, otherwise the epilogue is a pass of its own over the result.
+  // linear.cu's fragment kernel, larger steps take the whole-tile product with the epilogue on its fp32 sums (gemm_grouped.cu).
   struct Epilogue {
     const float* bias = nullptr;
     float a_pos = 0.f, a_neg = 0.f;
   };
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K, const Epilogue* ep = nullptr) {
     if (tc && T > few_rows) {
-      const int bn = block_n(plan, T);
-      if (fuse && N % 256 == 0 && T > 128 && N / 256 * ((T + bn - 1) / bn) >= plan.max_ctas / 2) {
-        Gemm2Epi e;
-        memset(&e, 0, sizeof(e));
-        e.epi = ep ? GEMM3_EPI_BIAS_XIELU : GEMM3_EPI_PLAIN;
-        e.out = static_cast<bf16*>(Y); e.ldo = N;
-        e.flags = gemm_flags; e.epoch = ++gemm_epoch;
-        if (ep) { e.bias = ep->bias; e.a_pos = ep->a_pos; e.a_neg = ep->a_neg; }
-        return gemm2_run_fused(plan, xm[gemm_block_n_index(bn)], bn, T, e, env.stream);
+      const int bn = gemm_block_n_for(T);
+      if (ep && fuse && gemm_whole_fits(plan, Y, N)) {
+        const GroupedOut o = {Y, N, GROUPED_XIELU, ep->bias, ep->a_pos, ep->a_neg};
+        return gemm_whole_run(plan, xm[gemm_block_n_index(bn)], bn, T, o, env.stream);
       }
       const int rc = gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
       return rc || !ep ? rc : bias_act(Y, N, ep->bias, LIN_XIELU, dt, T, N, env.stream, ep->a_pos, ep->a_neg);
@@ -564,16 +560,6 @@ class Soselix : public Model {
     if (ep) { la.bias = ep->bias; la.act = LIN_XIELU; la.a_pos = ep->a_pos; la.a_neg = ep->a_neg; }
     return linear(la, env.stream);
   }
-  // Token-tile size: where 512-token tiles neither fill the pairs nor are close enough to one whole tile per pair (that form
-  // takes up to 64 k-blocks), 256-token tiles give the fused form its tile per pair.
-  int block_n(const GemmPlan& p, int T) const {
-    const int bn = gemm_block_n_for(T), pairs = p.max_ctas / 2;
-    if (bn != 512 || !fuse || p.N % 256) return bn;
-    const int t512 = p.N / 256 * ((T + 511) / 512), t256 = p.N / 256 * ((T + 255) / 256);
-    const bool whole = p.K <= 4096 && t512 * 5 >= pairs * 3;
-    return t512 < pairs && !whole && t256 >= pairs ? 256 : bn;
-  }
-
   // per-kernel device time (b200_engine_kernel_times): with profiling on, every launch is bracketed by events and waited for
   cudaEvent_t pe0 = nullptr, pe1 = nullptr;
   void prof_start() {
@@ -695,6 +681,7 @@ class Soselix : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
+    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Soselix forward: a wait inside a projection ran out"); return -2; }
     KRN("embed", embed_scaled(embed, dt, b.ids, x, T, W, V, embed_scale, 1, 0, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {

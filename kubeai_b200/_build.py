@@ -30,6 +30,7 @@ SOURCES = [
     "norm_act.cu",
     "gla.cu",
     "scan_chunk.cu",
+    "scan_parallel.cu",
     "delta.cu",
     "delta_chunk.cu",
     "latent_attention.cu",

@@ -530,6 +530,14 @@ int gla_scan(const GlaArgs& a, cudaStream_t st) {
     const int from = e ? atoi(e) : 8;
     if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return scan_chunk(a, st);
   }
+  if ((a.nstate != nullptr) != (a.nq != nullptr) || (a.nstate && !a.tok_decay)) return -1;
+  if (a.tok_decay && (!a.tok_kscale || a.head_decay)) return -1;
+  if (!a.tok_decay && !a.head_decay && !a.dt_pre && !a.fgate_lower && (!a.z || !a.z_bias)) return -1;
+  if (!a.dt_pre && scan_parallel_fits(a)) {
+    const char* e = getenv("B200_SCAN_CHUNK");
+    const int from = e ? atoi(e) : 8;
+    if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return scan_parallel(a, st);
+  }
   int P = 1;
   while (P * kRows < a.dim) P <<= 1;
   if (P > 32) return -1;   // dim <= 1024
@@ -549,12 +557,8 @@ int gla_scan(const GlaArgs& a, cudaStream_t st) {
   while (G > 1 && smem_for(G) > 44 * 1024) G >>= 1;
   const size_t smem = smem_for(G);
   if (smem > 48 * 1024) return -1;
-  if ((a.nstate != nullptr) != (a.nq != nullptr) || (a.nstate && !a.tok_decay)) return -1;
   if (a.nstate && rows_per_part > kNormRows * tcols) return -1;
-  if (a.tok_decay) {
-    if (!a.tok_kscale || a.head_decay) return -1;
-  } else if (!a.head_decay && !a.dt_pre && !a.fgate_lower) {
-    if (!a.z || !a.z_bias) return -1;
+  if (!a.tok_decay && !a.head_decay && !a.dt_pre && !a.fgate_lower) {
     const long long total = static_cast<long long>(a.T) * a.heads * a.dim;
     if (total > 0) gla_decay_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(a.z, a.z_bias, a.heads * a.dim, a.inv_tau, total);
   }

@@ -131,12 +131,25 @@ struct GlaArgs {
   const float* fgate_lower = nullptr;
   const void* dt_pre = nullptr; int ld_dt = 0; const float* dt_bias = nullptr; const float* dt_rate = nullptr;
   int group = 1;
+  // workspace of the form whose chunks run side by side (scan_parallel.cu); without it, or where it is too small, the step's
+  // tokens run in a chain
+  float* par_ws = nullptr; size_t par_ws_floats = 0;
 };
 int gla_scan(const GlaArgs& a, cudaStream_t st);
 // The chunked tensor-core form of the dt_pre scan (scan_chunk.cu; same result up to fp32 rounding), for the shapes it takes;
 // gla_scan chooses it for bf16 steps of prompt portions.
 bool scan_chunk_fits(const GlaArgs& a);
 int scan_chunk(const GlaArgs& a, cudaStream_t st);
+// The form whose chunks run side by side (scan_parallel.cu; same result up to fp32 rounding), likewise chosen by gla_scan; its
+// workspace for steps of up to `tokens` tokens of up to `seqs` sequences (fgate: the HGRN2 form).
+size_t scan_parallel_ws_floats(int tokens, int seqs, int heads, int dim, int vdim, bool fgate);
+// (the sequences of a step it is chosen for bring 8 tokens and more each; at most 2 GB are asked for)
+inline size_t scan_parallel_ws_cap(int tokens, int slots, int heads, int dim, int vdim, bool fgate) {
+  const size_t need = scan_parallel_ws_floats(tokens, slots < tokens / 8 + 1 ? slots : tokens / 8 + 1, heads, dim, vdim, fgate), most = size_t(1) << 29;
+  return need < most ? need : most;
+}
+bool scan_parallel_fits(const GlaArgs& a);
+int scan_parallel(const GlaArgs& a, cudaStream_t st);
 // y[t, h * vdim + :] (leading dimension ldy) = o[t, h, :] / sqrt(mean(o^2) + eps) * w * silu(g[t, h, :])   (w: fp32 [vdim], shared by the heads)
 int gla_out_gate(const float* o, const void* g, int ldg, const float* w, float eps, void* y, int ldy, DType t, int T, int heads, int vdim,
                  cudaStream_t st);

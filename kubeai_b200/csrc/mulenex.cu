@@ -121,6 +121,8 @@ class Mulenex : public Model {
   int* expert_rows = nullptr;
   int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int moe_tc_min = 1;
+  float* scan_ws = nullptr;      // of the scan whose chunks run side by side
+  size_t scan_ws_floats = 0;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
@@ -328,6 +330,10 @@ class Mulenex : public Model {
     if (any_mlstm)
       rc |= dalloc(&o32, T * max_o * sizeof(float)) | dalloc(&gpre, T * 2 * max_h * sizeof(float)) | dalloc(&gkeep, T * max_h * sizeof(float)) |
             dalloc(&gtake, T * max_h * sizeof(float)) | dalloc(&gfloor, T * max_h * sizeof(float)) | dalloc(&gnq, T * max_h * sizeof(float));
+    if (dt == DT_BF16)
+      for (auto& s : spec)
+        if (s.mixer == MIX_MLSTM) scan_ws_floats = std::max(scan_ws_floats, scan_parallel_ws_cap(e.Tcap, e.num_slots, s.heads, s.dim, s.vdim, false));
+    if (scan_ws_floats) rc |= vec(&scan_ws, scan_ws_floats);
     if (any_dense) rc |= mat(&ffh, T, max_ff);
     if (any_dense || any_moe) rc |= mat(&fo, T, W);
     if (any_moe) {
@@ -672,6 +678,7 @@ class Mulenex : public Model {
     g.states = w.state; g.seqs = b.seqs; g.nseq = b.nseq;
     g.heads = s.heads; g.dim = s.dim; g.vdim = s.vdim; g.o = o32;
     g.tok_decay = gkeep; g.tok_kscale = gtake; g.nstate = w.nstate; g.nq = gnq;
+    g.par_ws = scan_ws; g.par_ws_floats = scan_ws_floats;
     KRN("mlstm_scan", gla_scan(g, st));
     OutGateArgs og;
     og.o = o32; og.g = col(inb, s.off_g); og.ldg = s.n_in; og.w = w.h_norm; og.eps = eps;

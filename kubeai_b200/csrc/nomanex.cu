@@ -114,6 +114,8 @@ class Nomanex : public Model {
   int* expert_rows = nullptr;
   int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int moe_tc_min = 1;
+  float* scan_ws = nullptr;      // of the scan whose chunks run side by side
+  size_t scan_ws_floats = 0;
   std::vector<void*> allocs;
   // tcgen05 projections
   float* gemm_ws = nullptr;
@@ -351,6 +353,10 @@ class Nomanex : public Model {
           mat(&hrow, row_cap, W);
     rc |= dalloc(&z, T * max_hd * sizeof(float)) | dalloc(&o32, T * max_hv * sizeof(float)) | dalloc(&qlat, T * max_ql * sizeof(float)) |
           dalloc(&olat, T * max_ol * sizeof(float)) | dalloc(&logits, static_cast<size_t>(row_cap) * V * sizeof(float));
+    if (dt == DT_BF16)
+      for (auto& s : spec)
+        if (s.mixer == MIX_GLA) scan_ws_floats = std::max(scan_ws_floats, scan_parallel_ws_cap(e.Tcap, e.num_slots, s.heads, s.dim, s.vdim, false));
+    if (scan_ws_floats) rc |= dalloc(&scan_ws, scan_ws_floats * sizeof(float));
     if (any_moe) {
       moe_cap = static_cast<int>((T * max_top + 63) / 64 * 64) + max_e * 64;
       rc |= dalloc(&scores, T * max_e * sizeof(float)) | dalloc(&topw, T * max_top * sizeof(float)) | dalloc(&topi, T * max_top * sizeof(int)) |
@@ -612,6 +618,7 @@ class Nomanex : public Model {
         g.z = z; g.T = T; g.z_bias = w.a2_b; g.inv_tau = 1.0f / s.tau; g.q_scale = 1.0f / sqrtf(static_cast<float>(s.dim));
         g.states = r.state; g.seqs = b.seqs; g.nseq = b.nseq;
         g.heads = s.heads; g.dim = s.dim; g.vdim = s.vdim; g.o = o32;
+        g.par_ws = scan_ws; g.par_ws_floats = scan_ws_floats;
         KRN("gla_scan", gla_scan(g, st));
         KRN("gla_out_gate", gla_out_gate(o32, col(inb, s.off_g), s.n_in, w.o_norm, eps, ycat, s.k_out, dt, T, s.heads, s.vdim, st));
         nl += 3;

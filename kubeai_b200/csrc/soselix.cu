@@ -106,6 +106,8 @@ class Soselix : public Model {
   long long split_ws_floats = 0;
   void *h = nullptr, *inb = nullptr, *cq = nullptr, *qb = nullptr, *xc = nullptr, *yb = nullptr, *ao = nullptr, *hid = nullptr, *fo = nullptr, *hrow = nullptr;
   int row_cap = 0;
+  float* scan_ws = nullptr;      // of the scan whose chunks run side by side
+  size_t scan_ws_floats = 0;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
@@ -334,6 +336,10 @@ class Soselix : public Model {
           vec(&logits, static_cast<size_t>(row_cap) * V);
     if (max_ql) rc |= mat(&cq, T, max_cq) | mat(&qb, T, max_q) | vec(&qlat, T * max_ql) | vec(&olat, T * max_ol);
     if (max_rec) rc |= vec(&o32, T * max_rec);
+    if (dt == DT_BF16)
+      for (auto& s : spec)
+        if (s.kind == MIX_HGRN2) scan_ws_floats = std::max(scan_ws_floats, scan_parallel_ws_cap(e.Tcap, e.num_slots, s.heads, s.dim, s.vdim, true));
+    if (scan_ws_floats) rc |= vec(&scan_ws, scan_ws_floats);
     if (max_xc) rc |= mat(&xc, T, max_xc);
     if (max_ff) rc |= mat(&hid, T, max_ff) | mat(&fo, T, W);
     if (max_ol && dt == DT_BF16) {
@@ -636,6 +642,7 @@ class Soselix : public Model {
     g.t = dt; g.inv_tau = 1.f; g.q_scale = 1.f; g.T = b.T;
     g.states = r.state; g.seqs = b.seqs; g.nseq = b.nseq;
     g.heads = s.heads; g.dim = s.dim; g.vdim = s.vdim; g.o = o32;
+    g.par_ws = scan_ws; g.par_ws_floats = scan_ws_floats;
     return g;
   }
 

@@ -522,6 +522,17 @@ int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int 
   return gemm_whole_run_as(p, tm_x, box, tile, gemm_whole_parts(p.N, p.K, tile, tiles, p.max_ctas / 2), rows, o, p.error, st);
 }
 
+int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, cudaStream_t st) {
+  CUtensorMap tm_w, tm_x;
+  int dev = 0, sms = 0, i = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
+  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < rows) ++i;
+  const int box = kBoxes[i], ntt = (rows + 2 * box - 1) / (2 * box), tile = ((rows + ntt - 1) / ntt + 15) & ~15;
+  if (tmap_encode_bf16_2d(&tm_w, W, N, K, ldw, kSlab, kBlockK, 1) || tmap_encode_bf16_2d(&tm_x, X, rows, K, ldx, box, kBlockK, 1)) return -2;
+  const long long tiles = static_cast<long long>((N + 2 * kSlab - 1) / (2 * kSlab)) * ((rows + tile - 1) / tile);
+  return launch(tm_w, 1, N, K, tm_x, box, nullptr, rows, o, {nullptr, nullptr, 1, tile}, static_cast<int>(std::min<long long>(sms / 2, tiles)), nullptr, st);
+}
+
 bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo) {
   return gemm_variant() == 2 && p.N % 8 == 0 && ldo % 8 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
 }

@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "activations.cuh"
+#include "gemm.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -427,6 +428,16 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
       if (a.T <= 8) linear_rows_mma_kernel<TX, TY, 1, U, false><<<grid, 256, 0, st>>>(a, KS);
       else linear_rows_mma_kernel<TX, TY, 2, U / 2, false><<<grid, 256, 0, st>>>(a, KS);
       return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    }
+    if constexpr (sizeof(TX) == 2 && sizeof(TY) == 4) {
+      // fp32 outputs of a wide matrix (the head's logits): whole tcgen05 tiles.  32 rows, 8192 x 2048: 76 us on the tile kernel
+      // below, 19 here (B200_LIN_WHOLE=0: A/B knob).
+      static const bool whole = [] { const char* e = getenv("B200_LIN_WHOLE"); return !e || atoi(e) != 0; }();
+      if (whole && vec && a.T > mma_rows && a.N >= 256 && a.N % 8 == 0 && a.ldy % 4 == 0 && reinterpret_cast<uintptr_t>(a.Y) % 16 == 0 && a.batch == 1 && !a.x_rows &&
+          !a.tile_group && !a.row_scale && a.act == LIN_NONE && gemm_variant() == 2) {
+        GroupedOut o = {a.Y, a.ldy, GROUPED_F32, a.bias};
+        return gemm_whole_direct(a.W, a.ldw, a.X, a.ldx, a.N, a.K, a.T, o, st);
+      }
     }
     if constexpr (sizeof(TX) == 2) {
       // B200_LIN_THIN: A/B knob, the most columns that take the exchanged form (0: none)

@@ -721,7 +721,7 @@ class Mulenex : public Model {
     }
     const long long gu_stride = 2ll * s.ff * W, down_stride = static_cast<long long>(W) * s.ff;
     const bool grouped = w.tc_experts && T >= moe_tc_min;
-    if (T * s.top <= 64) {
+    if (grouped ? picked_rows_pay(T * s.top, s.experts) : T * s.top <= 64) {
       // decode-sized steps: one weight-streaming pass per chosen (token, expert) pair, rows in pair order
       LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, T * s.top, 2 * s.ff, W);
       up.wbs = gu_stride;

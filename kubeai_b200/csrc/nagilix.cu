@@ -797,7 +797,7 @@ class Nagilix : public Model {
       KRN("moe_combine", moe_combine_identity(h, dt, iota, topw, topi, 0, h, fo, dt, T, s.top, W, st));
       return rc;
     }
-    if (T * s.top <= 64) {
+    if (grouped ? picked_rows_pay(T * s.top, s.experts) : T * s.top <= 64) {
       // decode-sized steps: one weight-streaming pass per chosen (token, expert) pair, rows in pair order; identity choices are skipped
       LinearArgs up = linear_args(h, dt, w.e_gu, dt, egu, dt, T * s.top, 2 * s.ff, W);
       up.wbs = gu_stride;

@@ -658,7 +658,7 @@ class Nomanex : public Model {
         KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, s.experts, W), st));
         KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, s.groups, s.keep, s.top, st));
         const int cap = (T * s.top + 63) / 64 * 64 + s.experts * 64;
-        const bool grouped = w.tc_experts && T >= moe_tc_min && T * s.top > 64;
+        const bool grouped = w.tc_experts && T >= moe_tc_min && !picked_rows_pay(T * s.top, s.experts);
         KRN("moe_align", moe_align(topi, T, s.top, s.experts, sorted_rows, tile_group, pair_pos, cap, st, grouped ? expert_rows : nullptr));
         if (grouped) {
           // the inputs in expert-sorted order, then one grouped GEMM per matrix, the activation in the first one's epilogue; the

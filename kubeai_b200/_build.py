@@ -37,6 +37,7 @@ SOURCES = [
     "moe.cu",
     "hyper.cu",
     "window_attention.cu",
+    "prompt_attention.cu",
     "ssm.cu",
     "nomanex.cu",
     "zinavik.cu",

@@ -711,6 +711,7 @@ int Engine::forward_model(const StepMeta& m, int32_t* dbuf, float* host_logits) 
   b.rows = dbuf + m.off_rows; b.seq_of_tok = dbuf + m.off_seqtok; b.seqs = dbuf + m.off_seqs; b.btab = dbuf + m.off_btab;
   b.max_blocks = max_blocks_per_seq;
   b.max_ctx = m.max_ctx;
+  b.fresh = m.kv_tokens == m.T;
   last_S = m.S;
   if (int rc = model->forward(b, sampled, host_logits, &stats.kernel_launches)) return rc == -1 ? B200_ERR_INVALID : B200_ERR_CUDA;
   return 0;

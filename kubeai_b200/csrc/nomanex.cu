@@ -3,7 +3,7 @@
 //   x_0[t]   = embed[token] + bigram[hash(previous token, token)]
 //   h        = dyt(x) = tanh(alpha x) w + b                         (Dynamic Tanh: no statistics)
 //   x       <- x + m (mixer(h) + ff(h))                             (one norm, both sublayers read it)
-//   mixer    = gated linear attention (gla.cu) | latent attention with a sliding window (latent_attention.cu)
+//   mixer    = gated linear attention (gla.cu) | latent attention with a sliding window (latent_attention.cu; whole prompts: prompt_attention.cu)
 //   ff       = clamped gated unit | group-limited mixture of squared-ReLU experts (moe.cu) | none
 //   logits   = head dyt_final(x)
 // A layer may name another layer whose weights it uses (`weights_of`); it keeps a cache / state of its own.
@@ -63,11 +63,15 @@ struct LayerWeights {
   float* c_norm = nullptr;
   void* uk_t = nullptr;    // [heads][kv_rank][dim]: W_uk transposed per head (the latent query projection)
   void* uv = nullptr;      // [heads * vdim, kv_rank]
+  void* ukv = nullptr;     // per head W_uk and W_uv one above the other [heads][256][kv_rank] (prompt_attention.cu)
   float2* rope = nullptr;  // [max_model_len][rot_dims / 2]
   // moe
   void* router = nullptr;  // [experts, width]
   void* e_up = nullptr;    // [experts][ff][width]
   void* e_down = nullptr;  // [experts][width][ff]
+  GemmPlan p_ukv;
+  CUtensorMap xm_c[kGemmNumBlockN];
+  bool tc_ukv = false;
   GemmPlan p_in, p_out;    // tcgen05 projections (bf16 storage, K % 8 == 0)
   GroupedPlan g_eup, g_edown;
   GroupedX xg_h, xg_act;     // views of the sorted rows and of the hidden rows
@@ -126,6 +130,7 @@ class Nomanex : public Model {
   explicit Nomanex(DType d) : dt(d) {}
   ~Nomanex() override {
     for (auto& w : wts) {
+      if (w.tc_ukv) gemm_plan_destroy(&w.p_ukv);
       if (w.tc_in) gemm_plan_destroy(&w.p_in);
       if (w.tc_out) gemm_plan_destroy(&w.p_out);
     }
@@ -382,7 +387,7 @@ class Nomanex : public Model {
     use_tc = dt == DT_BF16 && !(ev && atoi(ev) == 0) && W % 8 == 0 && gemm_variant() == 2;
     if (!use_tc) return 0;
     int maxN = W, max_kout = 8;
-    for (auto& s : spec) { maxN = std::max(maxN, s.n_in); max_kout = std::max(max_kout, s.k_out); }
+    for (auto& s : spec) { maxN = std::max(std::max(maxN, s.n_in), s.mixer == MIX_LATENT ? s.heads * (s.dim + s.vdim) : 0); max_kout = std::max(max_kout, s.k_out); }
     const size_t ws_bytes = std::max(gemm_workspace_bytes(env.sms), gemm_deferred_ws_bytes(env.sms));
     if (dalloc(&gemm_ws, ws_bytes)) return -3;
     const size_t n_counters = 2ull * (maxN / 128 + 2) * (env.Tcap / 32 + 2);
@@ -409,6 +414,14 @@ class Nomanex : public Model {
       for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
         if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
       if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = kernel_error; }
+      if (s.mixer == MIX_LATENT && s.rot_dims > 0 && latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank)) {
+        const int N = s.heads * (s.dim + s.vdim);
+        if (dalloc(&w.ukv, static_cast<size_t>(N) * s.kv_rank * 2)) return -3;
+        w.tc_ukv = gemm_plan_init(&w.p_ukv, w.ukv, N, s.kv_rank, s.kv_rank, gemm_ws, gemm_counters, env.sms) == 0;
+        for (int j = 0; j < kGemmNumBlockN && w.tc_ukv; ++j)
+          if (gemm_make_x_map(&w.xm_c[j], qlat, env.Tcap, s.kv_rank, s.kv_rank, bns[j])) w.tc_ukv = false;
+        if (w.tc_ukv) { w.p_ukv.ws_bytes = ws_bytes; w.p_ukv.error = kernel_error; }
+      }
       if (s.ff_kind == FF_MOE)
         w.tc_experts = !gemm_grouped_plan(&w.g_eup, w.e_up, s.experts, s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
                        !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);
@@ -519,7 +532,7 @@ class Nomanex : public Model {
     }
 #undef MAT
 #undef VEC
-    if (rc) { *err = "copying weights to the device failed"; return -2; }
+    if (rc || stack_latent() || cudaStreamSynchronize(env.stream) != cudaSuccess) { *err = "copying weights to the device failed"; return -2; }
     return 0;
   }
 
@@ -555,8 +568,14 @@ class Nomanex : public Model {
         M(w.e_down, static_cast<size_t>(s.experts) * W * s.ff, 1.7f / sqrtf(static_cast<float>(s.ff)));
       }
     }
-    if (rc) return -2;
+    if (rc || stack_latent()) return -2;
     return cudaStreamSynchronize(st) == cudaSuccess ? 0 : -2;
+  }
+  int stack_latent() {
+    int rc = 0;
+    for (size_t i = 0; i < spec.size(); ++i)
+      if (wts[i].tc_ukv) rc |= latent_prompt_stack(wts[i].uk_t, wts[i].uv, wts[i].ukv, spec[i].heads, spec[i].kv_rank, env.stream);
+    return rc;
   }
 
   // ------------------------------------------------------------ forward
@@ -629,21 +648,38 @@ class Nomanex : public Model {
         p.norm_w = w.c_norm; p.eps = eps; p.rope = w.rope; p.rot_dims = s.rot_dims;
         p.positions = b.pos; p.slots = b.slots; p.cache = r.cache; p.qlat = qlat;
         p.T = T; p.heads = s.heads; p.dim = s.dim; p.rot_dim = R; p.kv_rank = C;
-        KRN("latent_prep", latent_prep(p, st));
-        // latent query: per head [T, dim] x [kv_rank, dim]^T into the head's first kv_rank columns of qlat
-        LinearArgs lq = linear_args(col(inb, s.off_q), dt, w.uk_t, dt, qlat, DT_F32, T, C, s.dim);
-        lq.ldx = s.n_in; lq.ldy = s.heads * E; lq.batch = s.heads; lq.xbs = s.dim + R; lq.wbs = static_cast<long long>(C) * s.dim; lq.ybs = E;
-        KRN("latent_q_absorb", linear(lq, st));
-        LatentAttnArgs a;
-        a.qlat = qlat; a.cache = r.cache; a.t = dt; a.positions = b.pos; a.seq_of_tok = b.seq_of_tok; a.block_tables = b.btab;
-        a.max_blocks = b.max_blocks; a.page = env.page; a.olat = olat;
-        a.T = T; a.heads = s.heads; a.kv_rank = C; a.rot_dim = R; a.window = std::min(s.window, env.max_model_len); a.scale = s.scale;
-        a.seqs = b.seqs; a.nseq = b.nseq; a.max_ctx = b.max_ctx; a.split_ws = split_ws; a.split_ws_floats = split_ws_floats;
-        KRN("latent_attention", latent_attention(a, st));
-        // values: per head [T, kv_rank] x [vdim, kv_rank]^T into the head's columns of the output projection's input
-        LinearArgs lv = linear_args(olat, DT_F32, w.uv, dt, ycat, dt, T, s.vdim, C);
-        lv.ldx = s.heads * C; lv.ldy = s.k_out; lv.batch = s.heads; lv.xbs = C; lv.wbs = static_cast<long long>(s.vdim) * C; lv.ybs = s.vdim;
-        KRN("latent_v_expand", linear(lv, st));
+        const bool fresh = b.fresh && w.tc_ukv && latent_prompt_pays(T, b.nseq);
+        // whole prompts: per-head keys and values once per token, in the buffers of the latent form
+        bf16 *c = reinterpret_cast<bf16*>(qlat), *k2 = c + static_cast<size_t>(env.Tcap) * C, *q2 = k2 + static_cast<size_t>(env.Tcap) * R;
+        const int N = s.heads * (s.dim + s.vdim);
+        PromptAttnArgs pa = {};
+        pa.q = p.q; pa.ldq = s.n_in; pa.q_step = s.dim + R; pa.q2 = q2; pa.kv = olat; pa.ldkv = N; pa.k_step = pa.v_step = s.dim + s.vdim; pa.v_off = s.dim; pa.k2 = k2;
+        pa.y = ycat; pa.ldy = s.k_out; pa.T = T; pa.heads = pa.kv_heads = s.heads; pa.window = std::min(s.window, env.max_model_len); pa.scale = s.scale; pa.out_scale = 1.f;
+        pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = kernel_error;
+        if (fresh && prompt_attention_fits(pa)) {
+          LatentPromptPrepArgs pp = {r.cache, b.slots, b.pos, w.rope, s.rot_dims, p.half_pairs, p.q, p.ldq, c, k2, q2, T, s.heads, s.dim, R, C};
+          p.q = nullptr;
+          KRN("latent_prep", latent_prep(p, st));
+          KRN("latent_prompt_prep", latent_prompt_prep(pp, st));
+          KRN("latent_kv", project(w.p_ukv, true, w.xm_c, c, w.ukv, olat, T, N, C));
+          KRN("latent_attention", prompt_attention(pa, st));
+        } else {
+          KRN("latent_prep", latent_prep(p, st));
+          // latent query: per head [T, dim] x [kv_rank, dim]^T into the head's first kv_rank columns of qlat
+          LinearArgs lq = linear_args(col(inb, s.off_q), dt, w.uk_t, dt, qlat, DT_F32, T, C, s.dim);
+          lq.ldx = s.n_in; lq.ldy = s.heads * E; lq.batch = s.heads; lq.xbs = s.dim + R; lq.wbs = static_cast<long long>(C) * s.dim; lq.ybs = E;
+          KRN("latent_q_absorb", linear(lq, st));
+          LatentAttnArgs a;
+          a.qlat = qlat; a.cache = r.cache; a.t = dt; a.positions = b.pos; a.seq_of_tok = b.seq_of_tok; a.block_tables = b.btab;
+          a.max_blocks = b.max_blocks; a.page = env.page; a.olat = olat;
+          a.T = T; a.heads = s.heads; a.kv_rank = C; a.rot_dim = R; a.window = std::min(s.window, env.max_model_len); a.scale = s.scale;
+          a.seqs = b.seqs; a.nseq = b.nseq; a.max_ctx = b.max_ctx; a.split_ws = split_ws; a.split_ws_floats = split_ws_floats;
+          KRN("latent_attention", latent_attention(a, st));
+          // values: per head [T, kv_rank] x [vdim, kv_rank]^T into the head's columns of the output projection's input
+          LinearArgs lv = linear_args(olat, DT_F32, w.uv, dt, ycat, dt, T, s.vdim, C);
+          lv.ldx = s.heads * C; lv.ldy = s.k_out; lv.batch = s.heads; lv.xbs = C; lv.wbs = static_cast<long long>(s.vdim) * C; lv.ybs = s.vdim;
+          KRN("latent_v_expand", linear(lv, st));
+        }
         KRN("sigmoid_gate", sigmoid_gate(ycat, s.k_out, col(inb, s.off_g), s.n_in, dt, T, HV, st));
         nl += 5;
       }

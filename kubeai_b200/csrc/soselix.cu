@@ -7,7 +7,7 @@
 //              [c | kr] = W_dkv h, c RMS-normed, kr rotated: both cached, shared by the heads; per head
 //              score_j = (q . W_uk c_j + rot(q') . kr_j) * scale, causal softmax with exp(sink_h) in its denominator,
 //              W_uv on the weighted sum of the c_j, times sigmoid(W_g h)_h, W_o; rotation pairs (i, i + rot.dims / 2).
-//              With `kv_from`: j the layer has no W_dkv and reads the cache rows of layer j   (latent_attention.cu, absorbed form)
+//              With `kv_from`: j the layer has no W_dkv and reads the cache rows of layer j   (latent_attention.cu, absorbed form; whole prompts: prompt_attention.cu)
 //   hgrn2    : f = l + (1 - l) sigmoid(W_f h + b), S <- diag(f) S + (1 - f) v^T, o = S^T silu(W_q h); every head's o RMS-normed
 //              with one shared weight, W_o                                                       (gla.cu, fgate_lower form)
 //   mamba2   : [z | x | B | C | dt] = W_in h; x, B, C pass a short causal convolution and SiLU; d = softplus(dt + b);
@@ -63,6 +63,7 @@ struct LayerSpec {
 struct LayerWeights {
   void* w_in = nullptr;     // [n_in, width]
   void* w_out = nullptr;    // [width, k_out]
+  void* w_ukv = nullptr;   // per head W_uk and W_uv one above the other [heads][256][kv_rank] (prompt_attention.cu)
   void *w_uq = nullptr, *uk_t = nullptr, *w_uv = nullptr;   // [heads (dim + rot_dim), q_rank], [heads][kv_rank][dim], [heads][vdim][kv_rank]
   void *w_up = nullptr, *w_down = nullptr;                  // [ff, width], [width, ff]
   float *norm1 = nullptr, *norm2 = nullptr;                 // the norm's one number, spread over the width
@@ -72,9 +73,9 @@ struct LayerWeights {
   float *conv_w = nullptr, *conv_b = nullptr, *dt_b = nullptr, *dt_rate = nullptr, *skip = nullptr;
   float *up_b = nullptr, *down_b = nullptr;
   float act_pos = 0.f, act_neg = 0.f;
-  GemmPlan p_in, p_out, p_uq, p_up, p_down;
-  CUtensorMap xm_out[kGemmNumBlockN], xm_cq[kGemmNumBlockN], xm_hid[kGemmNumBlockN];
-  bool tc_in = false, tc_out = false, tc_uq = false, tc_up = false, tc_down = false;
+  GemmPlan p_in, p_out, p_uq, p_ukv, p_up, p_down;
+  CUtensorMap xm_out[kGemmNumBlockN], xm_cq[kGemmNumBlockN], xm_c[kGemmNumBlockN], xm_hid[kGemmNumBlockN];
+  bool tc_in = false, tc_ukv = false, tc_out = false, tc_uq = false, tc_up = false, tc_down = false;
 };
 
 struct LayerRun {
@@ -123,6 +124,7 @@ class Soselix : public Model {
       if (w.tc_in) gemm_plan_destroy(&w.p_in);
       if (w.tc_out) gemm_plan_destroy(&w.p_out);
       if (w.tc_uq) gemm_plan_destroy(&w.p_uq);
+      if (w.tc_ukv) gemm_plan_destroy(&w.p_ukv);
       if (w.tc_up) gemm_plan_destroy(&w.p_up);
       if (w.tc_down) gemm_plan_destroy(&w.p_down);
     }
@@ -362,7 +364,7 @@ class Soselix : public Model {
     use_tc = dt == DT_BF16 && !(ev && atoi(ev) == 0) && W % 8 == 0 && gemm_variant() == 2;
     if (!use_tc) return 0;
     int maxN = W;
-    for (auto& s : spec) maxN = std::max(std::max(maxN, s.n_in), std::max(s.ff, s.kind == MIX_LATENT ? s.heads * (s.dim + s.rot_dim) : 0));
+    for (auto& s : spec) maxN = std::max(std::max(maxN, s.n_in), std::max(s.ff, s.kind == MIX_LATENT ? s.heads * (s.dim + std::max(s.rot_dim, s.vdim)) : 0));
     const size_t ws_bytes = std::max(gemm_workspace_bytes(env.sms), gemm_deferred_ws_bytes(env.sms));
     if (dalloc(&gemm_ws, ws_bytes)) return -3;
     const size_t n_counters = 2ull * (maxN / 128 + 2) * (env.Tcap / 32 + 2);
@@ -389,6 +391,11 @@ class Soselix : public Model {
       w.tc_in = plan(&w.p_in, w.w_in, s.n_in, W);
       w.tc_out = plan(&w.p_out, w.w_out, W, s.k_out) && maps(w.xm_out, yb, s.k_out);
       if (s.kind == MIX_LATENT) w.tc_uq = plan(&w.p_uq, w.w_uq, s.heads * (s.dim + s.rot_dim), s.q_rank) && maps(w.xm_cq, cq, s.q_rank);
+      if (s.kind == MIX_LATENT && latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank)) {
+        const int N = s.heads * (s.dim + s.vdim);
+        if (dalloc(&w.w_ukv, static_cast<size_t>(N) * s.kv_rank * 2)) return -3;
+        w.tc_ukv = plan(&w.p_ukv, w.w_ukv, N, s.kv_rank) && maps(w.xm_c, qlat, s.kv_rank);
+      }
       if (s.mlp) {
         w.tc_up = plan(&w.p_up, w.w_up, s.ff, W);
         w.tc_down = plan(&w.p_down, w.w_down, W, s.ff) && maps(w.xm_hid, hid, s.ff);
@@ -502,7 +509,7 @@ class Soselix : public Model {
 #undef MAT
 #undef VEC
 #undef NORM1
-    if (rc) { *err = "copying weights to the device failed"; return -2; }
+    if (rc || stack_latent() || cudaStreamSynchronize(env.stream) != cudaSuccess) { *err = "copying weights to the device failed"; return -2; }
     return 0;
   }
 
@@ -541,8 +548,14 @@ class Soselix : public Model {
       M(w.w_down, static_cast<size_t>(W) * s.ff, by(s.ff)); F(w.down_b, W, 0.1f, 0.f);
       w.act_pos = 0.8f; w.act_neg = 1.2f;
     }
-    if (rc) return -2;
+    if (rc || stack_latent()) return -2;
     return cudaStreamSynchronize(st) == cudaSuccess ? 0 : -2;
+  }
+  int stack_latent() {
+    int rc = 0;
+    for (size_t i = 0; i < spec.size(); ++i)
+      if (wts[i].tc_ukv) rc |= latent_prompt_stack(wts[i].uk_t, wts[i].w_uv, wts[i].w_ukv, spec[i].heads, spec[i].kv_rank, env.stream);
+    return rc;
   }
 
   // ------------------------------------------------------------ forward
@@ -615,6 +628,22 @@ class Soselix : public Model {
     p.cq = col(inb, s.off_dq); p.ldcq = s.n_in; p.cq_w = w.cq_norm; p.q_rank = s.q_rank; p.cq_out = cq; p.ldcq_out = s.q_rank;
     KRN("latent_prep", latent_prep(p, st));
     KRN("proj_q", project(w.p_uq, w.tc_uq, w.xm_cq, cq, w.w_uq, qb, T, Q, s.q_rank));
+    if (b.fresh && w.tc_ukv && latent_prompt_pays(T, b.nseq)) {
+      // whole prompts: per-head keys and values once per token, in the buffers of the latent form
+      bf16 *c = reinterpret_cast<bf16*>(qlat), *k2 = c + static_cast<size_t>(env.Tcap) * C, *q2 = k2 + static_cast<size_t>(env.Tcap) * R;
+      LatentPromptPrepArgs pp = {r.cache, b.slots, b.pos, w.rope, s.rot_dims, true, qb, Q, c, k2, q2, T, s.heads, s.dim, R, C};
+      const int N = s.heads * (s.dim + s.vdim);
+      PromptAttnArgs pa = {};
+      pa.q = qb; pa.ldq = Q; pa.q_step = s.dim + R; pa.q2 = q2; pa.kv = olat; pa.ldkv = N; pa.k_step = pa.v_step = s.dim + s.vdim; pa.v_off = s.dim; pa.k2 = k2;
+      pa.y = yb; pa.ldy = s.k_out; pa.T = T; pa.heads = pa.kv_heads = s.heads; pa.window = env.max_model_len; pa.scale = s.scale; pa.out_scale = 1.f;
+      pa.sink = w.sink; pa.gate = col(inb, s.off_g); pa.ldg = s.n_in; pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = kernel_error;
+      if (prompt_attention_fits(pa)) {
+        KRN("latent_prompt_prep", latent_prompt_prep(pp, st));
+        KRN("latent_kv", project(w.p_ukv, true, w.xm_c, c, w.w_ukv, olat, T, N, C));
+        KRN("latent_attention", prompt_attention(pa, st));
+        return rc;
+      }
+    }
     if (R > 0) {
       pq.q = qb; pq.ldq = Q;
       KRN("latent_q_rotate", latent_prep(pq, st));

@@ -1,0 +1,71 @@
+"""Attention of whole prompts in latent layers (csrc/prompt_attention.cu) against the same tokens in portions (the latent-space
+kernels) and the oracles: lengths at the edges of its query and key tiles, windows from one key, one and more heads, sinks and
+gates, several sequences in one step, and a sequence whose neighbour holds no finite number."""
+import numpy as np
+import pytest
+
+import nomanex_util as nx
+import soselix_util as sx
+
+pytestmark = pytest.mark.gpu
+
+LENS = [32, 63, 64, 65, 127, 128, 129, 255, 256, 257, 320, 511, 513, 700]
+
+
+def check(cfg, e, oracle, lens):
+    rng = np.random.default_rng(len(lens))
+    for n in lens:
+        t = rng.integers(0, cfg["vocab"], n).tolist()
+        new, old = nx.feed_whole(e, t), nx.feed_portions(e, t, [1, 20, 300])
+        assert np.isfinite(new).all()
+        # each form rounds queries or keys, weights, sums or values and the output to bf16 (2^-9 of a value at most, each): four
+        # roundings a side, eight between the two
+        r = nx.rel_err(new, old.astype(np.float64))
+        assert np.median(r) < 8 * 2.0 ** -9 and r.max() < 10 * 8 * 2.0 ** -9, (n, np.median(r), r.max())
+        want = oracle.forward(t)
+        a, b = nx.rel_err(new, want), nx.rel_err(old, want)
+        assert np.median(a) < 1.1 * np.median(b) + 2.0 ** -11, (n, np.median(a), np.median(b))
+
+
+@pytest.mark.parametrize("heads,kv_rank", [(1, 128), (3, 136), (2, 512)])
+def test_sinks_gates_and_shared_rows(tmp_path, heads, kv_rank):
+    wide = dict(dim=128, rot_dim=64, vdim=128, kv_rank=kv_rank, q_rank=24, base=1000.0, mlp=None)
+    cfg = sx.make_config([sx.latent(heads=heads, **wide), sx.latent(heads=heads + 1, kv_from=0, **wide)], width=32)
+    W = sx.random_weights(cfg, seed=heads)
+    with sx.open_engine(sx.write_model_dir(tmp_path / "m", cfg, W), dtype="bfloat16", max_tokens=1024) as e:
+        check(cfg, e, sx.oracle_for(cfg, W), LENS if heads == 3 else LENS[:4])
+
+
+@pytest.mark.parametrize("window", [1, 2, 64, 100, 129, 4096])
+def test_windows(tmp_path, window):
+    cfg = nx.make_config([(nx.latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=128, window=window, base=1000.0, rot_dims=32), None)], width=32)
+    W = nx.random_weights(cfg, seed=window)
+    with nx.open_engine(nx.write_model_dir(tmp_path / "m", cfg, W), dtype="bfloat16", max_tokens=1024) as e:
+        check(cfg, e, nx.oracle_for(cfg, W), [65, 257, 700])
+
+
+def test_unequal_sequences_beside_one_without_finite_numbers(tmp_path):
+    cfg = sx.make_config([sx.latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=128, q_rank=24, base=1000.0, mlp=None)], width=32)
+    W = sx.random_weights(cfg, seed=9)
+    d = sx.write_model_dir(tmp_path / "m", cfg, W)
+    rng = np.random.default_rng(5)
+    lens = [1, 300, 65, 40, 63, 2] + [int(n) for n in rng.integers(1, 180, 34)] + [257]
+    assert sum(lens) >= 32 * len(lens)
+    seqs = [rng.integers(1, cfg["vocab"], n).tolist() for n in lens]
+    with sx.open_engine(d, dtype="bfloat16", max_tokens=400, max_seqs=64, budget=8192, blocks=2048) as e:
+        alone = [nx.feed_portions(e, s, [1, 400])[-1] for s in seqs]
+        ids = [e.feed_open() for _ in seqs]
+        together = e.feed_step([(r, s, [len(s) - 1]) for r, s in zip(ids, seqs)])
+        for r in ids:
+            e.feed_close(r)
+        r = nx.rel_err(together, np.stack(alone).astype(np.float64))
+        assert np.median(r) < 8 * 2.0 ** -9 and r.max() < 80 * 2.0 ** -9, (np.median(r), r.max())
+    W["embed"] = W["embed"].copy()
+    W["embed"][0] = np.inf
+    with sx.open_engine(sx.write_model_dir(tmp_path / "inf", cfg, W), dtype="bfloat16", max_tokens=400, max_seqs=64, budget=8192, blocks=2048) as e:
+        seqs = [[0] * n if i % 3 == 2 else s for i, (s, n) in enumerate(zip(seqs, lens))]
+        ids = [e.feed_open() for _ in seqs]
+        got = e.feed_step([(r, s, [len(s) - 1]) for r, s in zip(ids, seqs)])
+        for i in range(len(seqs)):
+            if i % 3 != 2:
+                np.testing.assert_array_equal(got[i], together[i])

@@ -233,8 +233,14 @@ struct Engine {
   // scheduling, pages, slots, packing and sampling
   std::unique_ptr<Model> model;
   std::vector<int> free_slots;
-  float* feed_logits_host = nullptr;   // pinned staging of b200_feed_step's logits
-  size_t feed_logits_cap = 0;
+  // Pinned staging of b200_feed_step's logits, two halves (engines that step by hand): the device's copies land here and the
+  // host converts or copies from it, one half while the other fills.  16 rows of 8192 logits from pageable memory and one by
+  // one took 150 us of a step.
+  static constexpr size_t kFeedHalf = 2u << 20;
+  uint8_t* feed_stage = nullptr;
+  cudaEvent_t feed_ev[2] = {nullptr, nullptr};
+  int init_feed();
+  int read_logits_f32(float* out, size_t count);
   std::vector<float> residual_dump;
   int L, H, Hq, Hkv, I, V, QKV;
   int Tcap, Scap, max_blocks_per_seq;
@@ -415,7 +421,8 @@ Engine::~Engine() {
   for (auto p : stage_dev)
     if (p) cudaFree(p);
   if (stage_host) cudaFreeHost(stage_host);
-  if (feed_logits_host) cudaFreeHost(feed_logits_host);
+  for (cudaEvent_t ev : feed_ev) if (ev) cudaEventDestroy(ev);
+  if (feed_stage) cudaFreeHost(feed_stage);
   model.reset();   // frees the model's device memory while the context is current
   if (sampled_host) cudaFreeHost(sampled_host);
   if (kernel_error) cudaFreeHost(kernel_error);
@@ -629,6 +636,7 @@ int Engine::alloc_all() {
   pool.init(nblocks, cfg.enable_prefix_caching != 0);
 
   if (int rc = alloc_step_ring()) return rc;
+  if (int rc = init_feed()) return rc;
   CK(cudaStreamSynchronize(stream));
   return 0;
 }
@@ -697,6 +705,7 @@ int Engine::init_model(const b200_config& c, std::unique_ptr<Model> mdl) {
   CK(cudaMalloc(&sampled, static_cast<size_t>(std::max(Scap, Tcap)) * 4));
   CK(cudaMallocHost(&sampled_host, static_cast<size_t>(Scap) * 4));
   if (int rc = alloc_step_ring()) return rc;
+  if (int rc = init_feed()) return rc;
   CK(cudaStreamSynchronize(stream));
   stats.kv_blocks_total = pool.total();
   stats.kv_blocks_free = pool.free_count();
@@ -1511,6 +1520,33 @@ int Engine::complete(InFlight& f, const StepMeta& m, b200_step_info* info) {
 // One step whose tokens the caller supplies (b200_feed_step): the listed sequences advance by exactly the given tokens, as
 // one batch, through the same page / slot bookkeeping, packing and forward pass as a scheduled step; nothing is sampled
 // into the sequences.  Logits of the wanted positions go to logits_out in the order of the entries.
+int Engine::init_feed() {
+  if (!cfg.manual_step) return 0;
+  CK(cudaMallocHost(&feed_stage, 2 * kFeedHalf));
+  for (cudaEvent_t& ev : feed_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  return 0;
+}
+
+// the first `count` bf16 logits on the device -> fp32 (same values) at `out`
+int Engine::read_logits_f32(float* out, size_t count) {
+  constexpr size_t part = kFeedHalf / 2;
+  const size_t parts = (count + part - 1) / part;
+  auto len = [&](size_t i) { return std::min(part, count - i * part); };
+  for (size_t i = 0; i <= parts; ++i) {
+    if (i < parts) {
+      CK(cudaMemcpyAsync(feed_stage + (i & 1) * kFeedHalf, logits + i * part, len(i) * 2, cudaMemcpyDeviceToHost, stream));
+      CK(cudaEventRecord(feed_ev[i & 1], stream));
+    }
+    if (i == 0) continue;
+    CK(cudaEventSynchronize(feed_ev[(i - 1) & 1]));
+    const uint16_t* in = reinterpret_cast<const uint16_t*>(feed_stage + ((i - 1) & 1) * kFeedHalf);
+    uint32_t* o = reinterpret_cast<uint32_t*>(out + (i - 1) * part);
+    const size_t n = len(i - 1);
+    for (size_t k = 0; k < n; ++k) o[k] = static_cast<uint32_t>(in[k]) << 16;
+  }
+  return 0;
+}
+
 int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, int64_t cap_floats) {
   InFlight& f = inflight_;
   f.sched.clear();
@@ -1562,22 +1598,19 @@ int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, 
     int32_t* dbuf = stage_dev[slot];
     CK(cudaMemcpyAsync(dbuf, stage_host, static_cast<size_t>(m.words) * 4, cudaMemcpyHostToDevice, stream));
     CK(cudaEventRecord(ev0, stream));
-    if (model) rc = forward_model(m, dbuf, logits_out);
+    const bool staged = model && static_cast<size_t>(S) * V * sizeof(float) <= 2 * kFeedHalf;
+    if (model) rc = forward_model(m, dbuf, staged ? reinterpret_cast<float*>(feed_stage) : logits_out);
     else {
       const bool keep = keep_logits;
       keep_logits = true;
       rc = forward(m, dbuf, false, nullptr);
       keep_logits = keep;
-      if (!rc && m.S) {
-        std::vector<bf16> tmp(static_cast<size_t>(m.S) * V);
-        CK(cudaMemcpyAsync(tmp.data(), logits, tmp.size() * 2, cudaMemcpyDeviceToHost, stream));
-        CK(cudaStreamSynchronize(stream));
-        for (size_t i = 0; i < tmp.size(); ++i) logits_out[i] = __bfloat162float(tmp[i]);
-      }
+      if (!rc && m.S) rc = read_logits_f32(logits_out, static_cast<size_t>(m.S) * V);
     }
     if (!rc) {
       CK(cudaEventRecord(ev1, stream));
       CK(cudaStreamSynchronize(stream));
+      if (staged && S) memcpy(logits_out, feed_stage, static_cast<size_t>(S) * V * sizeof(float));
     }
   }
   if (rc) {

@@ -4,10 +4,29 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass
+from operator import index
 
 import numpy as np
 
 from ._lib import Config, FeedEntry, Sampling, Stats, StepInfo, Usage, check, lib
+
+# FeedEntry for numpy
+FEED_DTYPE = np.dtype(dict(names=[f for f, _ in FeedEntry._fields_], formats=["u8", "u8", "i4", "u8", "i4"],
+                           offsets=[getattr(FeedEntry, f).offset for f, _ in FeedEntry._fields_], itemsize=C.sizeof(FeedEntry)))
+
+
+def _joined(values):
+    """int32 rows of the values one behind the other, and their lengths (of more dimensions: the first len(x) values)."""
+    make, int32 = np.ascontiguousarray, np.int32
+    rows = [make(v, int32) for v in values]
+    try:
+        flat = np.concatenate(rows)
+    except ValueError:                     # of different dimensions
+        flat = None
+    if flat is None or flat.ndim != 1:
+        flat = np.concatenate([r.reshape(-1)[:len(r)] for r in rows])
+    return flat, np.array([*map(len, rows)])
+
 
 FINISH = {0: None, 1: "stop", 2: "length", 3: "aborted", 4: "error"}
 
@@ -216,21 +235,21 @@ class Engine:
 
     def feed_step(self, entries) -> np.ndarray:
         """entries: [(rid, tokens, want offsets)]; returns fp32 logits [total wanted, vocab] in entry order."""
-        arr = (FeedEntry * len(entries))()
-        keep = []
+        # one array of entries whose pointers lead into two joined arrays: a ctypes pointer for each sequence's tokens and wanted
+        # offsets took 300 us of a step of 128 sequences
+        n = len(entries)
+        arr = np.zeros(n, dtype=FEED_DTYPE)
         total = 0
-        for i, (rid, toks, want) in enumerate(entries):
-            t = np.ascontiguousarray(toks, dtype=np.int32)
-            w = np.ascontiguousarray(want, dtype=np.int32)
-            keep += [t, w]
-            arr[i].req_id = rid
-            arr[i].tokens = t.ctypes.data_as(C.POINTER(C.c_int32))
-            arr[i].n_tokens = len(t)
-            arr[i].want = w.ctypes.data_as(C.POINTER(C.c_int32)) if len(w) else None
-            arr[i].n_want = len(w)
-            total += len(w)
+        if n:
+            rids, toks, wants = zip(*entries, strict=True)
+            arr["req_id"] = [index(r) & 0xFFFFFFFFFFFFFFFF for r in rids]
+            (tok, n_tok), (want, n_want) = _joined(toks), _joined(wants)
+            arr["tokens"], arr["n_tokens"] = tok.ctypes.data + 4 * (np.cumsum(n_tok) - n_tok), n_tok
+            arr["want"], arr["n_want"] = want.ctypes.data + 4 * (np.cumsum(n_want) - n_want), n_want
+            arr["want"][n_want == 0] = 0
+            total = len(want)
         out = np.empty((total, self.cfg.vocab), dtype=np.float32)
-        check(self._l.b200_feed_step(self._h, arr, len(entries), out.ctypes.data_as(C.POINTER(C.c_float)), out.size))
+        check(self._l.b200_feed_step(self._h, arr.ctypes.data_as(C.POINTER(FeedEntry)), n, out.ctypes.data_as(C.POINTER(C.c_float)), out.size))
         return out
 
     def profile_kernels(self, on: bool):

@@ -1,0 +1,52 @@
+"""Fed steps: the entries as they reach the C call, whatever the caller's sequences are made of, and the logits that come back
+in more than one part."""
+import numpy as np
+import pytest
+
+from kubeai_b200 import engine as E
+
+
+class Recorder:
+    def b200_feed_step(self, h, arr, n, out, size):
+        self.seen = [(arr[i].req_id, arr[i].tokens[:arr[i].n_tokens], arr[i].want[:arr[i].n_want] if arr[i].want else None) for i in range(n)]
+        return 0
+
+
+def fed(entries):
+    e = E.Engine.__new__(E.Engine)
+    e._l, e._h, e.cfg = Recorder(), None, E.Config(vocab=7)
+    out = e.feed_step(entries)
+    assert out.dtype == np.float32 and out.shape == (sum(len(w) for _, _, w in entries), 7)
+    return e._l.seen
+
+
+@pytest.mark.parametrize("entries,want", [
+    ([(3, [1, 2, 3], [0, 2])], [(3, [1, 2, 3], [0, 2])]),
+    ([(1, np.arange(8)[::2], []), (2, (7,), np.array([0]))], [(1, [0, 2, 4, 6], None), (2, [7], [0])]),
+    ([(2 ** 63 + 5, np.array([4], dtype=np.uint8), [0]), (9, [], [])], [(2 ** 63 + 5, [4], [0]), (9, [], None)]),
+    ([(1, np.array([[5, 6], [7, 8]]), []), (np.uint64(2), [1], [0])], [(1, [5, 6], None), (2, [1], [0])]),
+    ([], []),
+])
+def test_entries(entries, want):
+    assert fed(entries) == want
+
+
+@pytest.mark.parametrize("entries,error", [([(1.5, [1], [])], TypeError), ([(1, [2 ** 40], [])], OverflowError), ([(1, [1])], ValueError),
+                                           ([(1, [1], []), (1, [1], [], 0)], ValueError), ([(1, ["a"], [])], ValueError)])
+def test_refused_entries(entries, error):
+    with pytest.raises(error):
+        fed(entries)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 64])
+def test_logits_in_parts(rows):
+    """32 rows of 32768 are one part."""
+    cfg = E.default_config(num_layers=1, hidden=512, q_heads=8, kv_heads=2, intermediate=1024, vocab=32768, manual_step=1, max_num_seqs=64,
+                           max_batched_tokens=128, max_model_len=64, num_kv_blocks=256)
+    with E.Engine(cfg) as e:
+        e.set_keep_logits(True)
+        ids = [e.feed_open() for _ in range(rows)]
+        got = e.feed_step([(r, [i + 1, 2 * i + 1], [1]) for i, r in enumerate(ids)])
+        assert np.isfinite(got).all() and got.std(axis=1).min() > 0
+        np.testing.assert_array_equal(got, e.read_logits(rows))

@@ -108,7 +108,7 @@ paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16
 
   // All S stages are put in flight as early as the data allows.  Decode: every cached token except the newest was
   // written by an earlier step, so tiles that end before the newest token are gathered BEFORE the dependency wait
-  // (ptx.cuh griddep_enter) and overlap the RoPE/KV-write kernel upstream.  Prefill tiles may hold rows written by
+  // (griddep.cuh griddep_enter) and overlap the RoPE/KV-write kernel upstream.  Prefill tiles may hold rows written by
   // this step: wait first.
   const int safe_tiles = DECODE ? wk.q_pos0 / kTile : 0;
   bool waited = false;

@@ -71,7 +71,7 @@ template <int VPT>  // uint4 vectors per thread (H = VPT * 8 * blockDim)
 __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                const int* __restrict__ row_index, int H, float eps, PartialView pv) {
-  // ---- before the dependency wait (ptx.cuh griddep_enter): everything that does not come from the producer GEMM —
+  // ---- before the dependency wait (griddep.cuh griddep_enter): everything that does not come from the producer GEMM —
   // the row index (step input), the residual (written four or more launches upstream), the norm weight and the
   // partial-segment table entries (static)
   const int s = blockIdx.x;

@@ -27,6 +27,8 @@
 
 #include <algorithm>
 
+#include "griddep.cuh"
+#include "launch.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -52,6 +54,8 @@ constexpr int kThreads = 128;
 // The decay of every (token, head, key channel), once per step and in place over the pre-activation:
 // alpha = exp(inv_tau * logsigmoid(z + bias)), log sigmoid(z) = min(z, 0) - log1p(exp(-|z|)), accurate fp32 functions.
 __global__ void gla_decay_kernel(float* z, const float* bias, int HD, float inv_tau, long long total) {
+  griddep_launch();
+  griddep_wait();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const float v = z[i] + bias[i % HD];
@@ -78,6 +82,8 @@ __global__ void gla_decay_kernel(float* z, const float* bias, int HD, float inv_
 constexpr int kNormRows = 8;
 template <typename T, int NC, int MODE, int NE>
 __global__ void __launch_bounds__(kThreads) gla_scan_kernel(GlaArgs a, int P, int rpp, int G) {
+  griddep_launch();
+  griddep_wait();
   constexpr bool CD = MODE == 1 || MODE == 2;
   constexpr bool NRM = NE > 0;
   extern __shared__ __align__(16) float sm[];
@@ -337,6 +343,8 @@ __device__ __forceinline__ void stf4(bf16* p, float4 v) {
 // The per-head output stage for whole fours of columns: a warp per (token, head), the head's row in registers.
 template <typename T, int NF>
 __global__ void __launch_bounds__(128) out_gate_vec_kernel(OutGateArgs a, long long units) {
+  griddep_launch();
+  griddep_wait();
   const int lane = threadIdx.x & 31;
   const long long p = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (p >= units) return;
@@ -377,6 +385,8 @@ __global__ void __launch_bounds__(128) out_gate_vec_kernel(OutGateArgs a, long l
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) gated_group_norm_kernel(GatedGroupNormArgs a) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ __align__(16) float us[];
   __shared__ float red[8];
   const long long t = blockIdx.x;
@@ -430,6 +440,8 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(GatedGroupNormArg
 // three factors the scan and the output stage read.
 constexpr int kGateRound = 512;
 __global__ void __launch_bounds__(128) mlstm_gates_kernel(MlstmGateArgs a) {
+  griddep_launch();
+  griddep_wait();
   __shared__ float li[kGateRound], lf[kGateRound], ms[kGateRound + 1];
   const int head = blockIdx.x, seq = blockIdx.y;
   const int tok0 = a.seqs[seq * 8 + 0], n = a.seqs[seq * 8 + 1], pos0 = a.seqs[seq * 8 + 2], slot = a.seqs[seq * 8 + 3];
@@ -469,7 +481,7 @@ __global__ void __launch_bounds__(128) mlstm_gates_kernel(MlstmGateArgs a) {
 int mlstm_gates(const MlstmGateArgs& a, cudaStream_t st) {
   if (a.nseq <= 0) return 0;
   if (!a.pre || !a.keep || !a.take || !a.floor || !a.mstate || !a.seqs || a.heads < 1 || a.ld < 2 * a.heads) return -1;
-  mlstm_gates_kernel<<<dim3(a.heads, a.nseq), 128, 0, st>>>(a);
+  launch_pdl(mlstm_gates_kernel, dim3(a.heads, a.nseq), 128, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -486,9 +498,9 @@ int gated_group_norm(const GatedGroupNormArgs& a, cudaStream_t st) {
   const int th = work >= 256 ? 256 : (work >= 128 ? 128 : 64);
   dim3 grid(a.T, a.groups);
   if (a.t == DT_BF16) {
-    if (vec) gated_group_norm_kernel<bf16, true><<<grid, th, smem, st>>>(a); else gated_group_norm_kernel<bf16, false><<<grid, th, smem, st>>>(a);
+    if (vec) launch_pdl(gated_group_norm_kernel<bf16, true>, grid, th, smem, st, a); else launch_pdl(gated_group_norm_kernel<bf16, false>, grid, th, smem, st, a);
   } else {
-    if (vec) gated_group_norm_kernel<float, true><<<grid, th, smem, st>>>(a); else gated_group_norm_kernel<float, false><<<grid, th, smem, st>>>(a);
+    if (vec) launch_pdl(gated_group_norm_kernel<float, true>, grid, th, smem, st, a); else launch_pdl(gated_group_norm_kernel<float, false>, grid, th, smem, st, a);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -503,9 +515,9 @@ int recurrent_out_gate(const OutGateArgs& a, cudaStream_t st) {
   if (!a.joint && a.vdim % 4 == 0 && a.vdim <= 256 && a.ldg % 4 == 0 && a.ldy % 4 == 0 && al16(a.o) && al16(a.g) && al16(a.y) && al16(a.w)) {
     const unsigned ctas = static_cast<unsigned>((units + 3) / 4);
     if (a.t == DT_BF16) {
-      if (a.vdim <= 128) out_gate_vec_kernel<bf16, 1><<<ctas, 128, 0, st>>>(a, units); else out_gate_vec_kernel<bf16, 2><<<ctas, 128, 0, st>>>(a, units);
+      if (a.vdim <= 128) launch_pdl(out_gate_vec_kernel<bf16, 1>, ctas, 128, 0, st, a, units); else launch_pdl(out_gate_vec_kernel<bf16, 2>, ctas, 128, 0, st, a, units);
     } else {
-      if (a.vdim <= 128) out_gate_vec_kernel<float, 1><<<ctas, 128, 0, st>>>(a, units); else out_gate_vec_kernel<float, 2><<<ctas, 128, 0, st>>>(a, units);
+      if (a.vdim <= 128) launch_pdl(out_gate_vec_kernel<float, 1>, ctas, 128, 0, st, a, units); else launch_pdl(out_gate_vec_kernel<float, 2>, ctas, 128, 0, st, a, units);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
@@ -560,15 +572,15 @@ int gla_scan(const GlaArgs& a, cudaStream_t st) {
   if (a.nstate && rows_per_part > kNormRows * tcols) return -1;
   if (!a.tok_decay && !a.head_decay && !a.dt_pre && !a.fgate_lower) {
     const long long total = static_cast<long long>(a.T) * a.heads * a.dim;
-    if (total > 0) gla_decay_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(a.z, a.z_bias, a.heads * a.dim, a.inv_tau, total);
+    if (total > 0) launch_pdl(gla_decay_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, st, a.z, a.z_bias, a.heads * a.dim, a.inv_tau, total);
   }
   const bool one_row = rows_per_part <= tcols;
-#define SCAN(T_, NC_) do { if (a.tok_decay && a.nstate && one_row) gla_scan_kernel<T_, NC_, 2, 1><<<grid, kThreads, smem, st>>>(a, P, rows_per_part, G); \
-                          else if (a.tok_decay && a.nstate) gla_scan_kernel<T_, NC_, 2, kNormRows><<<grid, kThreads, smem, st>>>(a, P, rows_per_part, G); \
-                          else if (a.tok_decay || a.dt_pre) gla_scan_kernel<T_, NC_, 2, 0><<<grid, kThreads, smem, st>>>(a, P, rows_per_part, G); \
-                          else if (a.fgate_lower) gla_scan_kernel<T_, NC_, 3, 0><<<grid, kThreads, smem, st>>>(a, P, rows_per_part, G); \
-                          else if (a.head_decay) gla_scan_kernel<T_, NC_, 1, 0><<<grid, kThreads, smem, st>>>(a, P, rows_per_part, G); \
-                          else gla_scan_kernel<T_, NC_, 0, 0><<<grid, kThreads, smem, st>>>(a, P, rows_per_part, G); } while (0)
+#define SCAN(T_, NC_) do { if (a.tok_decay && a.nstate && one_row) launch_pdl(gla_scan_kernel<T_, NC_, 2, 1>, grid, kThreads, smem, st, a, P, rows_per_part, G); \
+                          else if (a.tok_decay && a.nstate) launch_pdl(gla_scan_kernel<T_, NC_, 2, kNormRows>, grid, kThreads, smem, st, a, P, rows_per_part, G); \
+                          else if (a.tok_decay || a.dt_pre) launch_pdl(gla_scan_kernel<T_, NC_, 2, 0>, grid, kThreads, smem, st, a, P, rows_per_part, G); \
+                          else if (a.fgate_lower) launch_pdl(gla_scan_kernel<T_, NC_, 3, 0>, grid, kThreads, smem, st, a, P, rows_per_part, G); \
+                          else if (a.head_decay) launch_pdl(gla_scan_kernel<T_, NC_, 1, 0>, grid, kThreads, smem, st, a, P, rows_per_part, G); \
+                          else launch_pdl(gla_scan_kernel<T_, NC_, 0, 0>, grid, kThreads, smem, st, a, P, rows_per_part, G); } while (0)
   if (a.t == DT_BF16) {
     if (NC == 2) SCAN(bf16, 2); else SCAN(bf16, 1);
   } else {

@@ -24,6 +24,8 @@
 
 #include <vector>
 
+#include "griddep.cuh"
+#include "launch.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -38,6 +40,8 @@ __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn
 
 template <typename TW>
 __global__ void embed_scaled_kernel(const TW* embed, const int* ids, float* x, int W, int vocab, float scale, int streams, long long stride) {
+  griddep_launch();
+  griddep_wait();
   const long long t = blockIdx.x;
   int id = ids[t];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
@@ -320,6 +324,8 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
 // VEC: four neighbouring columns per thread and round (W % 4 == 0, every row start 16-byte aligned)
 template <typename TY, typename TH, bool VEC>
 __global__ void __launch_bounds__(256) sandwich_step_kernel(SandwichArgs a) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ __align__(16) float row[];   // [W]: the sublayer output with its bias, then the new residual row
   __shared__ float red[8];
   const int r = blockIdx.x;
@@ -436,7 +442,7 @@ int sandwich_step(const SandwichArgs& a, cudaStream_t st) {
   auto al16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool vec = a.W % 4 == 0 && al16(a.x) && al16(a.y) && al16(a.h) && al16(a.y_bias) && al16(a.post_w) && al16(a.pre_w);
   const int th = vec ? (a.W >= 1024 ? 256 : (a.W >= 512 ? 128 : 64)) : threads_for(a.W);
-#define SW(TY, TH) do { if (vec) sandwich_step_kernel<TY, TH, true><<<a.rows, th, smem, st>>>(a); else sandwich_step_kernel<TY, TH, false><<<a.rows, th, smem, st>>>(a); } while (0)
+#define SW(TY, TH) do { if (vec) launch_pdl(sandwich_step_kernel<TY, TH, true>, a.rows, th, smem, st, a); else launch_pdl(sandwich_step_kernel<TY, TH, false>, a.rows, th, smem, st, a); } while (0)
   const bool y16 = a.y && a.ty == DT_BF16, h16 = a.h && a.th == DT_BF16;
   if (y16 && h16) SW(bf16, bf16);
   else if (y16) SW(bf16, float);
@@ -450,8 +456,8 @@ int embed_scaled(const void* embed, DType tw, const int* ids, float* x, int T, i
                  long long stream_stride, cudaStream_t st) {
   if (T <= 0) return 0;
   if (W < 1 || streams < 1) return -1;
-  if (tw == DT_BF16) embed_scaled_kernel<bf16><<<T, threads_for(W), 0, st>>>(static_cast<const bf16*>(embed), ids, x, W, vocab, scale, streams, stream_stride);
-  else embed_scaled_kernel<float><<<T, threads_for(W), 0, st>>>(static_cast<const float*>(embed), ids, x, W, vocab, scale, streams, stream_stride);
+  if (tw == DT_BF16) launch_pdl(embed_scaled_kernel<bf16>, T, threads_for(W), 0, st, static_cast<const bf16*>(embed), ids, x, W, vocab, scale, streams, stream_stride);
+  else launch_pdl(embed_scaled_kernel<float>, T, threads_for(W), 0, st, static_cast<const float*>(embed), ids, x, W, vocab, scale, streams, stream_stride);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

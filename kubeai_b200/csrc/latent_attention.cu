@@ -21,6 +21,7 @@
 #include <atomic>
 #include <vector>
 
+#include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
 
@@ -73,13 +74,19 @@ __device__ __forceinline__ float out_gate(const LatentAttnArgs& a, long long t, 
   return 1.0f / (1.0f + expf(-ldf(static_cast<const T*>(a.gate) + t * a.ldg + h)));
 }
 
-// one CTA per token
+// per token, each its own CTA: the query latent's norm, the cache row, the queries' rotated parts (one after the other in one CTA,
+// 8 tokens took 13 us)
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepArgs a) {
+  griddep_launch();
+  griddep_wait();
   __shared__ float red[8];
   const int t = blockIdx.x;
   const int C = a.kv_rank, R = a.rot_dim, D = a.dim;
-  if (a.cq) {
+  int part = blockIdx.y;     // of those that the call asks for
+  if (!a.cq) ++part;
+  if (part >= 1 && !a.dkv) ++part;
+  if (part == 0 && a.cq) {
     const T* u = static_cast<const T*>(a.cq) + static_cast<long long>(t) * a.ldcq;
     T* o = static_cast<T*>(a.cq_out) + static_cast<long long>(t) * a.ldcq_out;
     float ss = 0.f;
@@ -90,7 +97,7 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepArgs a) {
   }
   const int half = a.rot_dims / 2;
   const float2* cs = a.rope + static_cast<long long>(a.positions[t]) * half;
-  if (a.dkv) {
+  if (part == 1 && a.dkv) {
     const T* d = static_cast<const T*>(a.dkv) + static_cast<long long>(t) * a.lddkv;
     T* row = static_cast<T*>(a.cache) + static_cast<long long>(a.slots[t]) * (C + R);
     float ss = 0.f;
@@ -101,7 +108,7 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepArgs a) {
     // shared rotated key part
     for (int i = threadIdx.x; i < R; i += blockDim.x) stf(row + C + i, rotated(d + C, i, half, a.half_pairs, cs));
   }
-  if (a.q) {
+  if (part == 2 && a.q) {
     // rotated part of every query head -> tail of the latent query
     const T* q = static_cast<const T*>(a.q) + static_cast<long long>(t) * a.ldq;
     float* ql = a.qlat + static_cast<long long>(t) * a.heads * (C + R);
@@ -206,6 +213,8 @@ constexpr int kMaxPairs = 4;   // 16-column pairs of the latent value width per 
 // MB = 16-row blocks per CTA: two for steps made of prompt portions (each key tile then serves twice the rows)
 template <int MB>
 __global__ void __launch_bounds__(256) latent_attn_mma_kernel(LatentAttnArgs a, const int* seqs, int nseq, int TQ, int HB, int nsplit, float* split_ws) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int R = 16 * MB;
   const int C = a.kv_rank, E = a.kv_rank + a.rot_dim, LDE = E + 8;
@@ -425,6 +434,8 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(LatentAttnArgs a, 
 
 // one warp per (token, head): combine the splits' partials
 __global__ void latent_attn_merge_kernel(LatentAttnArgs a, const float* ws, float* olat, int C, int nsplit, long long rows) {
+  griddep_launch();
+  griddep_wait();
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -722,8 +733,10 @@ int latent_prep(const LatentPrepArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   if (a.rot_dims > a.rot_dim || a.rot_dims % 2) return -1;
   if (a.cq && (!a.cq_w || !a.cq_out || a.q_rank < 1)) return -1;
-  if (a.t == DT_BF16) latent_prep_kernel<bf16><<<a.T, 128, 0, st>>>(a);
-  else latent_prep_kernel<float><<<a.T, 128, 0, st>>>(a);
+  const int parts = (a.cq != nullptr) + (a.dkv != nullptr) + (a.q != nullptr);
+  if (!parts) return 0;
+  if (a.t == DT_BF16) launch_pdl(latent_prep_kernel<bf16>, dim3(a.T, parts), 128, 0, st, a);
+  else launch_pdl(latent_prep_kernel<float>, dim3(a.T, parts), 128, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -768,15 +781,15 @@ int latent_attention(const LatentAttnArgs& a, cudaStream_t st) {
     dim3 grid((a.T + TQ - 1) / TQ + a.nseq, (a.heads + HB - 1) / HB, nsplit);
     if (two) {
       if (!ensure_dynamic_smem(latent_attn_mma_kernel<2>, 220 * 1024, &attr2)) return -2;
-      latent_attn_mma_kernel<2><<<grid, 256, latent_mma_smem(E, 2), st>>>(a, a.seqs, a.nseq, TQ, HB, nsplit, a.split_ws);
+      launch_pdl(latent_attn_mma_kernel<2>, grid, 256, latent_mma_smem(E, 2), st, a, a.seqs, a.nseq, TQ, HB, nsplit, a.split_ws);
     } else {
       if (!ensure_dynamic_smem(latent_attn_mma_kernel<1>, 220 * 1024, &attr1)) return -2;
-      latent_attn_mma_kernel<1><<<grid, 256, latent_mma_smem(E, 1), st>>>(a, a.seqs, a.nseq, TQ, HB, nsplit, a.split_ws);
+      launch_pdl(latent_attn_mma_kernel<1>, grid, 256, latent_mma_smem(E, 1), st, a, a.seqs, a.nseq, TQ, HB, nsplit, a.split_ws);
     }
     if (cudaGetLastError() != cudaSuccess) return -2;
     if (nsplit > 1) {
       const long long rows = static_cast<long long>(a.T) * a.heads;
-      latent_attn_merge_kernel<<<static_cast<unsigned>((rows + 3) / 4), 128, 0, st>>>(a, a.split_ws, a.olat, a.kv_rank, nsplit, rows);
+      launch_pdl(latent_attn_merge_kernel, static_cast<unsigned>((rows + 3) / 4), 128, 0, st, a, a.split_ws, a.olat, a.kv_rank, nsplit, rows);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }

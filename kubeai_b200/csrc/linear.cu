@@ -18,6 +18,8 @@
 
 #include "activations.cuh"
 #include "gemm.h"
+#include "griddep.cuh"
+#include "launch.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -328,6 +330,14 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
   const int steps = (a.K + 31) >> 5, per = (steps + KS - 1) / KS, s1 = min(steps, (ks + 1) * per);
+  griddep_launch();
+  if (!THIN) {
+    // while the kernel before this one ends: this warp's share of the weights (16 rows, 128-byte lines, at most 32 KB) into L2
+    const int k0 = ks * per * 32, lines = (min(a.K, s1 * 32) - k0 + 63) >> 6;
+    for (int i = lane; i < min(16 * lines, 256); i += 32)
+      if (n0 + (i & 15) < rows) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + static_cast<long long>(n0 + (i & 15)) * ldw + k0 + (i >> 4) * 64));
+  }
+  griddep_wait();
   const uint4 zero = make_uint4(0, 0, 0, 0);
   for (int s = ks * per; s < s1; s += U) {
     uint4 wa[U], wb[U], xv[U][NB], xl[U][SPLIT ? NB : 1];
@@ -382,6 +392,8 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
 // streaming rate instead of walking 64-row tiles that are almost empty.
 template <typename TX, typename TW, typename TY, int VEC>
 __global__ void __launch_bounds__(256) linear_picked_rows_kernel(LinearArgs a, PickedRows p) {
+  griddep_launch();
+  griddep_wait();
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
   const int n = blockIdx.x * 8 + wrp, r = blockIdx.y;
   if (n >= a.N) return;
@@ -407,8 +419,8 @@ int launch_picked(const LinearArgs& a, const PickedRows& p, cudaStream_t st) {
   const bool vec = a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.wbs % 8 == 0 && reinterpret_cast<uintptr_t>(a.X) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(a.W) % 16 == 0;
   dim3 grid((a.N + 7) / 8, p.rows);
-  if (vec) linear_picked_rows_kernel<TX, TW, TY, 8><<<grid, 256, 0, st>>>(a, p);
-  else linear_picked_rows_kernel<TX, TW, TY, 1><<<grid, 256, 0, st>>>(a, p);
+  if (vec) launch_pdl(linear_picked_rows_kernel<TX, TW, TY, 8>, grid, 256, 0, st, a, p);
+  else launch_pdl(linear_picked_rows_kernel<TX, TW, TY, 1>, grid, 256, 0, st, a, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -425,8 +437,8 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
       const int KS = steps >= 32 ? 8 : (steps >= 16 ? 4 : (steps >= 8 ? 2 : 1));
       dim3 grid((a.N + 128 / KS - 1) / (128 / KS), 1, a.batch);
       constexpr int U = sizeof(TX) == 4 ? 4 : 8;
-      if (a.T <= 8) linear_rows_mma_kernel<TX, TY, 1, U, false><<<grid, 256, 0, st>>>(a, KS);
-      else linear_rows_mma_kernel<TX, TY, 2, U / 2, false><<<grid, 256, 0, st>>>(a, KS);
+      if (a.T <= 8) launch_pdl(linear_rows_mma_kernel<TX, TY, 1, U, false>, grid, 256, 0, st, a, KS);
+      else launch_pdl(linear_rows_mma_kernel<TX, TY, 2, U / 2, false>, grid, 256, 0, st, a, KS);
       return cudaGetLastError() == cudaSuccess ? 0 : -2;
     }
     if constexpr (sizeof(TX) == 2 && sizeof(TY) == 4) {
@@ -446,7 +458,7 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
         const int steps = (a.K + 31) / 32;
         const int KS = steps >= 32 ? 8 : (steps >= 16 ? 4 : (steps >= 8 ? 2 : 1));
         dim3 grid((a.T + 128 / KS - 1) / (128 / KS), (a.N + 15) / 16);
-        linear_rows_mma_kernel<TX, TY, 2, 4, true><<<grid, 256, 0, st>>>(a, KS);
+        launch_pdl(linear_rows_mma_kernel<TX, TY, 2, 4, true>, grid, 256, 0, st, a, KS);
         return cudaGetLastError() == cudaSuccess ? 0 : -2;
       }
     }

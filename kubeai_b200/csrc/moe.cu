@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <float.h>
 
+#include "griddep.cuh"
+#include "launch.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -20,6 +22,8 @@ typedef __nv_bfloat16 bf16;
 // one warp per token; scores row in global memory is the scratch (chosen entries are overwritten with -1)
 __global__ void moe_route_kernel(float* scores, int* topk_ids, float* topk_w, int T, int E, int groups, int keep, int top, int score_fn, int ld,
                                  const float* bias, MoeRouteForm form) {
+  griddep_launch();
+  griddep_wait();
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
   const int lane = threadIdx.x & 31;
@@ -111,6 +115,8 @@ __global__ void moe_route_kernel(float* scores, int* topk_ids, float* topk_w, in
 // single CTA: histogram, padded offsets, scatter
 __global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, int pairs, int top, int E, int* sorted_rows, int* tile_group,
                                                          int* pair_pos, int cap, int* expert_rows, const float* topk_w, float* sorted_w, int matrices) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ int sh[];   // count[E], start[E + 1], fill[E]
   int* count = sh;
   int* start = sh + E;
@@ -169,6 +175,8 @@ __global__ void moe_combine_kernel(const TYIN* y, const int* pair_pos, const flo
 // bf16 rows of whole 16-byte pieces: a thread forms eight neighbouring columns, the same sums in the same order
 __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const bf16* y, const int* pair_pos, const float* topk_w, bf16* out, int top, int W, const bf16* add,
                                                               const float* add_gate, int ld_gate) {
+  griddep_launch();
+  griddep_wait();
   const long long t = blockIdx.x;
   const float gate = add && add_gate ? 1.0f / (1.0f + expf(-add_gate[t * ld_gate])) : 1.f;
   auto fma8 = [](float* acc, float s, const bf16* p) {
@@ -203,7 +211,7 @@ int moe_route(float* scores, int* topk_ids, float* topk_w, int T, int E, int gro
   if (E < 1 || groups < 1 || groups > 64 || E % groups || keep < 1 || keep > groups || top < 1 || top > keep * (E / groups)) return -1;
   if ((select_bias || form.normalize) && score_fn == MOE_TOP_SOFTMAX) return -1;
   if (form.group_best < 1 || form.group_best > 2) return -1;
-  moe_route_kernel<<<(T + 3) / 4, 128, 0, st>>>(scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, ld > 0 ? ld : E, select_bias, form);
+  launch_pdl(moe_route_kernel, (T + 3) / 4, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, ld > 0 ? ld : E, select_bias, form);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -213,7 +221,7 @@ int moe_align(const int* topk_ids, int T, int top, int E, int* sorted_rows, int*
   if (cap % 64 || cap < T * top + E * 64 || (sorted_w && !topk_w)) return -1;
   const size_t smem = static_cast<size_t>(3 * E + 1) * sizeof(int);
   if (smem > 48 * 1024) return -1;
-  moe_align_kernel<<<1, 1024, smem, st>>>(topk_ids, T * top, top, E, sorted_rows, tile_group, pair_pos, cap, expert_rows, topk_w, sorted_w, matrices > 0 ? matrices : E);
+  launch_pdl(moe_align_kernel, 1, 1024, smem, st, topk_ids, T * top, top, E, sorted_rows, tile_group, pair_pos, cap, expert_rows, topk_w, sorted_w, matrices > 0 ? matrices : E);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -235,7 +243,7 @@ int moe_combine_add(const void* y, DType ty, const int* pair_pos, const float* t
   const int th = W >= 1024 ? 256 : 128;
   auto al16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (ty == DT_BF16 && W % 8 == 0 && al16(y) && al16(out) && al16(add))
-    moe_combine_vec_kernel<<<T, W >= 2048 ? 256 : 128, 0, st>>>(static_cast<const bf16*>(y), pair_pos, topk_w, static_cast<bf16*>(out), top, W,
+    launch_pdl(moe_combine_vec_kernel, T, W >= 2048 ? 256 : 128, 0, st, static_cast<const bf16*>(y), pair_pos, topk_w, static_cast<bf16*>(out), top, W,
                                                                 static_cast<const bf16*>(add), add_gate, ld_gate);
   else if (ty == DT_BF16)
     moe_combine_kernel<bf16, bf16><<<T, th, 0, st>>>(static_cast<const bf16*>(y), pair_pos, topk_w, static_cast<bf16*>(out), top, W,
@@ -269,6 +277,8 @@ int moe_combine_identity(const void* y, DType ty, const int* pair_pos, const flo
 namespace {
 // rows of x in expert-sorted order (16-byte pieces; W % 8 == 0): a negative source row becomes zeros
 __global__ void moe_gather_kernel(const uint4* x, const int* sorted_rows, uint4* out, int pieces, long long total, const float* row_scale) {
+  griddep_launch();
+  griddep_wait();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long r = i / pieces;
@@ -300,7 +310,7 @@ int moe_gather_bf16(const void* x, const int* sorted_rows, void* out, int rows, 
   if (rows <= 0) return 0;
   if (W % 8) return -1;
   const long long total = static_cast<long long>(rows) * (W / 8);
-  moe_gather_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(static_cast<const uint4*>(x), sorted_rows, static_cast<uint4*>(out), W / 8, total, row_scale);
+  launch_pdl(moe_gather_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, st, static_cast<const uint4*>(x), sorted_rows, static_cast<uint4*>(out), W / 8, total, row_scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

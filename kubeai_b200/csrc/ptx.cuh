@@ -6,27 +6,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "griddep.cuh"
+
 namespace b200 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// ---------------------------------------------------------------- programmatic dependent launch
-// wait: block until every grid this one depends on has completed and its memory is visible.
-// launch_dependents: allow the next kernel in the stream to start launching (it still waits
-// at its own griddepcontrol.wait for our completion before touching dependent data).
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Dependency point of every non-GEMM kernel: wait for the producer, THEN let the consumer launch.  GEMMs release their
-// consumer at entry (before their own wait).  Consequence used by the kernels' pre-wait prologues: code that runs
-// before griddep_enter() in kernel K_n may read
-//   * anything written by K_{n-2} or earlier when K_{n-1} is a non-GEMM kernel,
-//   * anything written by K_{n-3} or earlier when K_{n-1} is a GEMM (two GEMMs are never adjacent),
-//   * per-step inputs uploaded before the step's first kernel, and static tables (weights, cos/sin, segment tables).
-__device__ __forceinline__ void griddep_enter() {
-  griddep_wait();
-  griddep_launch();
 }
 
 // ---------------------------------------------------------------- mbarrier

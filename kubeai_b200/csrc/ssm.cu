@@ -22,6 +22,8 @@
 
 #include <algorithm>
 
+#include "griddep.cuh"
+#include "launch.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -85,6 +87,8 @@ __device__ __forceinline__ void stv(float* p, const float* v) { *reinterpret_cas
 // sequence (or at its start) the window is filled again, from the rows before, the sequence's carried inputs or zeros.
 template <int VEC, int TAPS>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConvArgs a, int TB) {
+  griddep_launch();
+  griddep_wait();
   typedef typename VecOf<VEC>::type T;
   const int groups = a.C / VEC;
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
@@ -157,6 +161,8 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConvArgs a, in
 
 template <typename TU>
 __global__ void short_conv_carry_kernel(ShortConvArgs a) {
+  griddep_launch();
+  griddep_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
   if (c >= a.C) return;
   const int* sq = a.seqs + s * 8;
@@ -273,7 +279,7 @@ int short_conv(const ShortConvArgs& a, cudaStream_t st) {
     int TB = 16;
     while (TB > 1 && static_cast<long long>((a.T + TB - 1) / TB) * ((groups + 127) / 128) < 4 * 148) TB >>= 1;
     dim3 vgrid((groups + 127) / 128, (a.T + TB - 1) / TB);
-#define SC(V_, K_) short_conv_vec_kernel<V_, K_><<<vgrid, 128, 0, st>>>(a, TB)
+#define SC(V_, K_) launch_pdl(short_conv_vec_kernel<V_, K_>, vgrid, 128, 0, st, a, TB)
     if (a.t == DT_BF16) { switch (a.taps) { case 1: SC(8, 1); break; case 2: SC(8, 2); break; case 3: SC(8, 3); break; default: SC(8, 4); } }
     else { switch (a.taps) { case 1: SC(4, 1); break; case 2: SC(4, 2); break; case 3: SC(4, 3); break; default: SC(4, 4); } }
 #undef SC
@@ -294,8 +300,8 @@ int short_conv_carry(const ShortConvArgs& a, cudaStream_t st) {
   if (a.nseq <= 0 || a.taps <= 1) return 0;
   if (!a.u || !a.state || a.C < 1 || !a.seqs) return -1;
   dim3 grid((a.C + 127) / 128, a.nseq);
-  if (a.t == DT_BF16) short_conv_carry_kernel<bf16><<<grid, 128, 0, st>>>(a);
-  else short_conv_carry_kernel<float><<<grid, 128, 0, st>>>(a);
+  if (a.t == DT_BF16) launch_pdl(short_conv_carry_kernel<bf16>, grid, 128, 0, st, a);
+  else launch_pdl(short_conv_carry_kernel<float>, grid, 128, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

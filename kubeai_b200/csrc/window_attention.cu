@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
 
@@ -47,6 +48,8 @@ __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf
 // lane 0's.  Value rows are copied by all threads.
 template <typename T>
 __global__ void __launch_bounds__(128) qk_prep_kernel(QkPrepArgs a) {
+  griddep_launch();
+  griddep_wait();
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int p = a.positions[t];
@@ -121,6 +124,8 @@ __global__ void __launch_bounds__(128) qk_prep_kernel(QkPrepArgs a) {
 // queries and writes qn or the key part of the cache row.
 template <typename T>
 __global__ void __launch_bounds__(1024) conv_qk_prep_kernel(ConvQkPrepArgs a) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ float cv[];   // [(heads + kv_heads) * dim] convolved projections
   __shared__ float red[2][32];
   const long long t = blockIdx.x;
@@ -198,6 +203,8 @@ __global__ void __launch_bounds__(1024) conv_qk_prep_kernel(ConvQkPrepArgs a) {
 // The same without a convolution, for bf16 rows of whole 16-byte pieces and neighbouring rotation pairs: a thread owns eight
 // columns of the query or key row from the load to the store, so only the two sums go through shared memory.
 __global__ void __launch_bounds__(1024) qk_rows_prep_kernel(ConvQkPrepArgs a) {
+  griddep_launch();
+  griddep_wait();
   __shared__ float red[2][32];
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -292,6 +299,8 @@ __device__ __forceinline__ float dot_row(const float* q, const T* k, int D, bool
 
 template <typename T>
 __global__ void __launch_bounds__(kWarpsDecode * 32) window_attn_kernel(WindowAttnArgs a, bool vec) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ float sm[];   // q [dim] | per warp: m, l, acc [vdim]
   const long long t = blockIdx.x / a.heads;
   const int h = blockIdx.x % a.heads;
@@ -423,6 +432,8 @@ constexpr float kMasked = -1e30f;
 
 template <int NV>   // value n-tiles of 8 columns held per thread: vdim <= 8 * NV
 __global__ void __launch_bounds__(kMmaThreads, kMmaCtasPerSm) window_attn_mma_kernel(WindowAttnArgs a, int gs, int TQ, int page_shift) {
+  griddep_launch();
+  griddep_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ long long rowoff[kTileKeys];                // cache row (in elements) of every key of a tile, looked up once
   const int D = a.dim, Dv = a.vdim, LDK = D + 8, LDV = Dv + 8;
@@ -703,8 +714,8 @@ int rope_table_yarn(float2* table, int max_pos, int dims, double base, const Rop
 int qk_rope_norm_cache(const QkPrepArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   if (a.heads < 1 || a.kv_heads < 1 || a.dim < 1 || a.vdim < 1 || a.rot_dims < 0 || a.rot_dims > a.dim || a.rot_dims % 2 || (a.rot_dims && !a.rope)) return -1;
-  if (a.t == DT_BF16) qk_prep_kernel<bf16><<<a.T, 128, 0, st>>>(a);
-  else qk_prep_kernel<float><<<a.T, 128, 0, st>>>(a);
+  if (a.t == DT_BF16) launch_pdl(qk_prep_kernel<bf16>, a.T, 128, 0, st, a);
+  else launch_pdl(qk_prep_kernel<float>, a.T, 128, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -721,16 +732,16 @@ int conv_qk_prep(const ConvQkPrepArgs& a, cudaStream_t st) {
   auto al16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (a.t == DT_BF16 && !a.conv_w && (a.interleaved || !a.rot_dims) && a.dim % 8 == 0 && a.ld % 8 == 0 && C <= 8192 && al16(a.qk) && al16(a.cache) && al16(a.qn) &&
       al16(a.q_norm_w) && al16(a.k_norm_w)) {
-    qk_rows_prep_kernel<<<a.T, (C / 8 + 31) / 32 * 32, 0, st>>>(a);
+    launch_pdl(qk_rows_prep_kernel, a.T, (C / 8 + 31) / 32 * 32, 0, st, a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   const int th = a.T >= 256 ? (C >= 2048 ? 256 : 128) : std::min(1024, std::max(128, (C + 31) / 32 * 32));
   if (a.t == DT_BF16) {
     if (smem > 48 * 1024 && !ensure_dynamic_smem(conv_qk_prep_kernel<bf16>, 200 * 1024, &set16)) return -2;
-    conv_qk_prep_kernel<bf16><<<a.T, th, smem, st>>>(a);
+    launch_pdl(conv_qk_prep_kernel<bf16>, a.T, th, smem, st, a);
   } else {
     if (smem > 48 * 1024 && !ensure_dynamic_smem(conv_qk_prep_kernel<float>, 200 * 1024, &set32)) return -2;
-    conv_qk_prep_kernel<float><<<a.T, th, smem, st>>>(a);
+    launch_pdl(conv_qk_prep_kernel<float>, a.T, th, smem, st, a);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -758,11 +769,11 @@ int window_attention(const WindowAttnArgs& a, cudaStream_t st) {
     if (a.vdim <= 64) {
       if (!ensure_dynamic_smem(window_attn_mma_kernel<8>, 112 * 1024, &set8)) return -2;
       cudaFuncSetAttribute(window_attn_mma_kernel<8>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      window_attn_mma_kernel<8><<<grid, kMmaThreads, smem, st>>>(a, gs, TQ, page_shift);
+      launch_pdl(window_attn_mma_kernel<8>, grid, kMmaThreads, smem, st, a, gs, TQ, page_shift);
     } else {
       if (!ensure_dynamic_smem(window_attn_mma_kernel<16>, 112 * 1024, &set16)) return -2;
       cudaFuncSetAttribute(window_attn_mma_kernel<16>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      window_attn_mma_kernel<16><<<grid, kMmaThreads, smem, st>>>(a, gs, TQ, page_shift);
+      launch_pdl(window_attn_mma_kernel<16>, grid, kMmaThreads, smem, st, a, gs, TQ, page_shift);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
@@ -773,8 +784,8 @@ int window_attention(const WindowAttnArgs& a, cudaStream_t st) {
   const size_t smem = (static_cast<size_t>((a.dim + 3) & ~3) + warps * (a.vdim + 2)) * sizeof(float);
   if (smem > 48 * 1024) return -1;
   const unsigned grid = static_cast<unsigned>(static_cast<long long>(a.T) * a.heads);
-  if (a.t == DT_BF16) window_attn_kernel<bf16><<<grid, warps * 32, smem, st>>>(a, vec);
-  else window_attn_kernel<float><<<grid, warps * 32, smem, st>>>(a, vec);
+  if (a.t == DT_BF16) launch_pdl(window_attn_kernel<bf16>, grid, warps * 32, smem, st, a, vec);
+  else launch_pdl(window_attn_kernel<float>, grid, warps * 32, smem, st, a, vec);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -118,6 +118,7 @@ class Dabodra : public Model {
   int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int row_cap = 0, moe_cap = 0;
   std::vector<void*> allocs;
+  void* attn_ws = nullptr;       // of the attention of whole prompts
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
   int few_rows = 16;
@@ -342,6 +343,10 @@ class Dabodra : public Model {
     rc |= vec(&x, T * W) | mat(&h, T, W) | mat(&inb, T, max_in) | mat(&yb, T, max_out) | mat(&ao, T, W) | mat(&hrow, row_cap, W) |
           vec(&logits, static_cast<size_t>(row_cap) * V);
     if (max_qn) rc |= vec(&qn, T * max_qn);
+    size_t aw = 0;
+    for (auto& s : spec)
+      if (dt == DT_BF16 && s.kind == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(e.Tcap, s.heads, s.kv_heads));
+    if (aw) rc |= dalloc(&attn_ws, aw);
     if (max_rec) rc |= mat(&xc, T, max_xc) | vec(&o32, T * max_rec);
     if (any_moe) {
       moe_cap = static_cast<int>((T * max_top + 63) / 64 * 64) + max_e * 64;
@@ -643,6 +648,7 @@ class Dabodra : public Model {
     wa.T = b.T; wa.heads = s.heads; wa.kv_heads = s.kv_heads; wa.dim = s.dim; wa.vdim = s.vdim;
     wa.window = s.window; wa.scale = s.scale; wa.sink = w.sink;
     wa.seqs = b.seqs; wa.nseq = b.nseq; wa.max_ctx = b.max_ctx;
+    wa.fresh = b.fresh; wa.slots = b.slots; wa.ws = attn_ws; wa.error = kernel_error;
     KRN("window_attention", window_attention(wa, st));
     return rc;
   }

@@ -291,6 +291,9 @@ struct LatentPromptPrepArgs {
   int T, heads, dim, rot_dim, kv_rank;
 };
 int latent_prompt_prep(const LatentPromptPrepArgs& a, cudaStream_t st);
+// Attention from per-head keys and values: the tokens' cache rows [kv_heads * 256] side by side -> kv, qn (fp32) -> q (bf16).
+int window_prompt_prep(const void* cache, const int* slots, const float* qn, void* kv, void* q, int T, int heads, int kv_heads, cudaStream_t st);
+bool window_prompt_pays(int T, int nseq, int heads);
 bool latent_prompt_fits(int dim, int vdim, int rot_dim, int kv_rank);   // the widths this form is built for
 bool latent_prompt_pays(int T, int nseq);                               // steps of long enough prompts
 int latent_prompt_stack(const void* uk_t, const void* uv, void* out, int heads, int kv_rank, cudaStream_t st);
@@ -365,7 +368,11 @@ struct WindowAttnArgs {
   const int* seqs; int nseq; int max_ctx;
   float softcap = 0.f; bool gate_per_head = false;
   int chunk = 0; const float* sink = nullptr;
+  // steps whose sequences all start at their first token (StepBatch::fresh): the cache row of every token, a workspace of
+  // window_prompt_ws_bytes and a host-visible mark for a wait that ran out (prompt_attention.cu); ws null: never that form
+  bool fresh = false; const int* slots = nullptr; void* ws = nullptr; int* error = nullptr;
 };
+size_t window_prompt_ws_bytes(int rows, int heads, int kv_heads);
 int window_attention(const WindowAttnArgs& a, cudaStream_t st);
 
 // ---------------------------------------------------------------- short causal convolution, selective scan (ssm.cu)

@@ -124,6 +124,7 @@ class Mulenex : public Model {
   float* scan_ws = nullptr;      // of the scan whose chunks run side by side
   size_t scan_ws_floats = 0;
   std::vector<void*> allocs;
+  void* attn_ws = nullptr;       // of the attention of whole prompts
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
   CUtensorMap xm_h[kGemmNumBlockN];
@@ -327,6 +328,10 @@ class Mulenex : public Model {
     rc |= dalloc(&x, T * W * sizeof(float)) | mat(&h, T, W) | mat(&inb, T, max_in) | mat(&ycat, T, max_kout) | mat(&ao, T, W) | mat(&hrow, row_cap, W);
     rc |= dalloc(&qn, T * max_qn * sizeof(float)) | dalloc(&logits, static_cast<size_t>(row_cap) * V * sizeof(float));
     if (vfirst_ld) rc |= mat(&vfirst, T, vfirst_ld);
+    size_t aw = 0;
+    for (auto& s : spec)
+      if (dt == DT_BF16 && s.mixer == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(e.Tcap, s.heads, s.kv_heads));
+    if (aw) rc |= dalloc(&attn_ws, aw);
     if (any_mlstm)
       rc |= dalloc(&o32, T * max_o * sizeof(float)) | dalloc(&gpre, T * 2 * max_h * sizeof(float)) | dalloc(&gkeep, T * max_h * sizeof(float)) |
             dalloc(&gtake, T * max_h * sizeof(float)) | dalloc(&gfloor, T * max_h * sizeof(float)) | dalloc(&gnq, T * max_h * sizeof(float));
@@ -655,6 +660,7 @@ class Mulenex : public Model {
     wa.T = b.T; wa.heads = s.heads; wa.kv_heads = s.kv_heads; wa.dim = s.dim; wa.vdim = s.vdim;
     wa.window = 1 << 30; wa.keep_first = 0; wa.scale = s.scale; wa.softcap = s.softcap;
     wa.seqs = b.seqs; wa.nseq = b.nseq; wa.max_ctx = b.max_ctx;
+    wa.fresh = b.fresh; wa.slots = b.slots; wa.ws = attn_ws; wa.error = kernel_error;
     KRN("attention", window_attention(wa, st));
     return rc;
   }

@@ -13,6 +13,9 @@
 // sequence's end belong to the next one: their keys are masked and their values cleared, so that nothing of another sequence
 // can reach a result.  Every wait has a limit; a CTA that gives up sets an error mark and still meets at the end.
 //
+// With keys and values per head (window_prompt_prep gathers them from the cache): sequences of 455, 1365 and 2275 tokens, 16 query
+// and 4 key heads, cap: 291 us on mma.sync -> 120.
+//
 // What bounds it: the exponentials and the tensor cores about evenly.  16 heads, 192 + 128 dimensions, sequences of 455, 1365
 // and 2275 tokens: 87 us (37 GFLOP), with the product that rebuilds keys and values and the gather of the latents 126; the
 // latent-space kernel on mma.sync took 883, with its two per-head products 1109.
@@ -374,6 +377,16 @@ __global__ void __launch_bounds__(128) latent_prompt_prep_kernel(LatentPromptPre
   }
 }
 
+// one CTA per token
+__global__ void __launch_bounds__(128) window_prompt_prep_kernel(const uint4* cache, const int* slots, const float4* qn, uint4* kv, uint4* q, int kv_pieces, int q_pieces) {
+  const long long t = blockIdx.x, row = slots[t];
+  for (int i = threadIdx.x; i < kv_pieces; i += blockDim.x) kv[t * kv_pieces + i] = cache[row * kv_pieces + i];
+  for (int i = threadIdx.x; i < q_pieces; i += blockDim.x) {
+    const float4 a = qn[(t * q_pieces + i) * 2], b = qn[(t * q_pieces + i) * 2 + 1];
+    q[t * q_pieces + i] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+  }
+}
+
 // per head: rows 0 .. 127 W_uk (kept transposed), rows 128 .. 255 W_uv
 __global__ void latent_stack_kernel(const bf16* uk_t, const bf16* uv, bf16* out, int C, long long total) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -410,6 +423,25 @@ int latent_prompt_prep(const LatentPromptPrepArgs& a, cudaStream_t st) {
   if (a.kv_rank % 8 || a.rot_dim % 8 || a.rot_dims > a.rot_dim) return -1;
   latent_prompt_prep_kernel<<<a.T, 128, 0, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int window_prompt_prep(const void* cache, const int* slots, const float* qn, void* kv, void* q, int T, int heads, int kv_heads, cudaStream_t st) {
+  if (T <= 0) return 0;
+  window_prompt_prep_kernel<<<T, 128, 0, st>>>(static_cast<const uint4*>(cache), slots, reinterpret_cast<const float4*>(qn), static_cast<uint4*>(kv), static_cast<uint4*>(q),
+                                               kv_heads * 2 * kD / 8, heads * kD / 8);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+size_t window_prompt_ws_bytes(int rows, int heads, int kv_heads) { return static_cast<size_t>(rows) * (heads + 2 * kv_heads) * kD * 2; }
+
+// Measured with 16 query and 4 key heads under a cap, window kernel on mma.sync -> this one with its gather, in us: one prompt of 32
+// tokens 22 -> 15, of 128 26 -> 17, of 512 49 -> 32; 64 prompts of 64 95 -> 64, 16 of 128 56 -> 29, 8 of 512 128 -> 56; 4095
+// tokens under a window of 1024 211 -> 95.  Many prompts of 32 fill a quarter of a CTA's 128 rows and break even (64 of them
+// 63 -> 62, 32 of them 32 -> 35): below 64 tokens only while one wave of CTAs holds them all.
+bool window_prompt_pays(int T, int nseq, int heads) {
+  static const int least = [] { const char* e = getenv("B200_WINDOW_PROMPT"); return e ? atoi(e) : 32; }();   // A/B knob: fewest tokens a prompt, 0 = never
+  const long long n = nseq;
+  return least > 0 && T >= least * n && (T >= 2 * least * n || n * heads <= 148);
 }
 
 bool latent_prompt_fits(int dim, int vdim, int rot_dim, int kv_rank) {

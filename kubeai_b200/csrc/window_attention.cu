@@ -757,6 +757,19 @@ int window_attention(const WindowAttnArgs& a, cudaStream_t st) {
   const bool fits = a.t == DT_BF16 && a.dim % 16 == 0 && a.vdim % 16 == 0 && a.dim <= 128 && a.vdim <= 128 && a.seqs && a.nseq > 0 && a.ldy % 2 == 0 &&
                     (!a.gate || a.gate_per_head || a.ldg % 2 == 0) && reinterpret_cast<uintptr_t>(a.cache) % 16 == 0;
   const bool want = force >= 0 ? force != 0 : (a.T >= 32 && a.T >= 8 * a.nseq);
+  // whole prompts: every key is one of the step's own rows, tcgen05 (prompt_attention.cu)
+  if (force < 0 && a.fresh && a.ws && a.slots && a.t == DT_BF16 && a.dim == 128 && a.vdim == 128 && a.keep_first == 0 && a.chunk == 0 && (!a.gate || a.gate_per_head) &&
+      window_prompt_pays(a.T, a.nseq, a.heads)) {
+    PromptAttnArgs pa = {};
+    bf16* kv = static_cast<bf16*>(a.ws) + static_cast<size_t>(a.T) * a.heads * 128;
+    pa.q = a.ws; pa.ldq = a.heads * 128; pa.q_step = 128; pa.kv = kv; pa.ldkv = a.kv_heads * 256; pa.k_step = pa.v_step = 128; pa.v_off = a.kv_heads * 128;
+    pa.y = a.y; pa.ldy = a.ldy; pa.T = a.T; pa.heads = a.heads; pa.kv_heads = a.kv_heads; pa.window = a.window; pa.scale = a.scale; pa.softcap = a.softcap;
+    pa.out_scale = a.out_scale; pa.sink = a.sink; pa.gate = a.gate; pa.ldg = a.ldg; pa.seqs = a.seqs; pa.nseq = a.nseq; pa.error = a.error;
+    if (prompt_attention_fits(pa)) {
+      const int rc = window_prompt_prep(a.cache, a.slots, a.qn, kv, a.ws, a.T, a.heads, a.kv_heads, st);
+      return rc ? rc : prompt_attention(pa, st);
+    }
+  }
   if (fits && want) {
     const int group = a.heads / a.kv_heads;
     const int gs = kTileRows % group == 0 ? group : 1;

@@ -1,9 +1,11 @@
-"""Attention of whole prompts in latent layers (csrc/prompt_attention.cu) against the same tokens in portions (the latent-space
-kernels) and the oracles: lengths at the edges of its query and key tiles, windows from one key, one and more heads, sinks and
+"""Attention of whole prompts (csrc/prompt_attention.cu) against the same tokens in portions (the kernels over the paged cache:
+latent-space, window) and the oracles: lengths at the edges of its query and key tiles, windows from one key, one and more heads, sinks and
 gates, several sequences in one step, and a sequence whose neighbour holds no finite number."""
 import numpy as np
 import pytest
 
+import dabodra_util as db
+import mulenex_util as mx
 import nomanex_util as nx
 import soselix_util as sx
 
@@ -42,6 +44,23 @@ def test_windows(tmp_path, window):
     W = nx.random_weights(cfg, seed=window)
     with nx.open_engine(nx.write_model_dir(tmp_path / "m", cfg, W), dtype="bfloat16", max_tokens=1024) as e:
         check(cfg, e, nx.oracle_for(cfg, W), [65, 257, 700])
+
+
+@pytest.mark.parametrize("heads,kv_heads,softcap,scale", [(1, 1, None, 0.09), (4, 2, 6.0, 0.2), (6, 2, 30.0, 1.0), (3, 3, None, 0.09)])
+def test_caps_and_grouped_heads(tmp_path, heads, kv_heads, softcap, scale):
+    wide = dict(heads=heads, kv_heads=kv_heads, dim=128, vdim=128, scale=scale, softcap=softcap)
+    cfg = mx.make_config([mx.layer(mx.attention(v_mix=False, **wide), mlp=None), mx.layer(mx.attention(**wide), mlp=None)], width=32)
+    W = mx.random_weights(cfg, seed=heads)
+    with mx.open_engine(mx.write_model_dir(tmp_path / "m", cfg, W), dtype="bfloat16", max_tokens=1024) as e:
+        check(cfg, e, mx.oracle_for(cfg, W), LENS if heads == 4 else LENS[:4])
+
+
+@pytest.mark.parametrize("window", [1, 65, 128, 4096])
+def test_windows_and_sinks_over_grouped_heads(tmp_path, window):
+    cfg = db.make_config([db.attention(heads=4, kv_heads=1, dim=128, window=window, rot_dims=32, base=1000.0, mlp=None)], width=32)
+    W = db.random_weights(cfg, seed=window)
+    with db.open_engine(db.write_model_dir(tmp_path / "m", cfg, W), dtype="bfloat16", max_tokens=1024) as e:
+        check(cfg, e, db.oracle_for(cfg, W), [32, 65, 257, 700])
 
 
 def test_unequal_sequences_beside_one_without_finite_numbers(tmp_path):

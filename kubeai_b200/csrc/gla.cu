@@ -555,11 +555,13 @@ int gla_scan(const GlaArgs& a, cudaStream_t st) {
   if (P > 32) return -1;   // dim <= 1024
   const int rows_per_part = ((a.dim + P - 1) / P + 3) / 4 * 4;
   const int tcols = kThreads / P;
-  // two columns per thread when that still leaves at least two CTAs per SM's worth of work
+  // two columns per thread when that still leaves at least two CTAs per SM's worth of work and there is a chain of tokens to walk;
+  // a decode step only loads and stores states, and twice the CTAs of half the registers keep more of that in flight (Soselix, 8
+  // sequences, Mamba-2's 64 heads and HGRN2's 16: the step 298 us with two columns, 274 with one)
   int sms = 148;
   { int dev = 0; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   const long long ctas2 = static_cast<long long>((a.vdim + 2 * tcols - 1) / (2 * tcols)) * a.heads * a.nseq;
-  int NC = (a.vdim >= 2 * tcols && ctas2 >= sms) ? 2 : 1;
+  int NC = (a.vdim >= 2 * tcols && ctas2 >= sms && a.T >= 2 * a.nseq) ? 2 : 1;
   if (const char* e = getenv("B200_GLA_NC")) NC = atoi(e) == 2 && a.vdim >= 2 * tcols ? 2 : 1;   // A/B knob
   const int cols = tcols * NC;
   dim3 grid((a.vdim + cols - 1) / cols, a.heads, a.nseq);

@@ -35,8 +35,8 @@ namespace b200 {
 namespace {
 
 typedef __nv_bfloat16 bf16;
-__device__ __forceinline__ float ldf(const float* p) { return __ldg(p); }
-__device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(__ldg(p)); }
+__device__ __forceinline__ float ldf(const float* p) { return *p; }
+__device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 __device__ __forceinline__ float siluf_(float x) { return x / (1.0f + expf(-x)); }
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kThreads) gla_scan_kernel(GlaArgs a, int P, in
           }
           s3[(tt * 3) * Dp] = qv * a.q_scale;
           s3[(tt * 3 + 1) * Dp] = kv * a.k_scale;
-          if (MODE == 0) s3[(tt * 3 + 2) * Dp] = __ldg(a.z + row * (a.heads * D) + c);
+          if (MODE == 0) s3[(tt * 3 + 2) * Dp] = a.z[row * (a.heads * D) + c];
         }
       } else {
         for (int tt = 0; tt < gn; ++tt) { s3[(tt * 3) * Dp] = 0.f; s3[(tt * 3 + 1) * Dp] = 0.f; s3[(tt * 3 + 2) * Dp] = 0.f; }
@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(kThreads) gla_scan_kernel(GlaArgs a, int P, in
           ds[tt] = expf(__ldg(a.dt_rate + head) * d);
           ds[G + tt] = d;
         } else {
-          ds[tt] = __ldg(a.tok_decay + row * a.heads + head);
-          ds[G + tt] = __ldg(a.tok_kscale + row * a.heads + head);
+          ds[tt] = a.tok_decay[row * a.heads + head];
+          ds[G + tt] = a.tok_kscale[row * a.heads + head];
         }
       }
     __syncthreads();
@@ -330,9 +330,9 @@ __global__ void recurrent_out_gate_kernel(OutGateArgs a, long long units) {
 // The output stage with the gate in front of the norm (GatedGroupNormArgs): one CTA per (token, part).  VEC: four
 // neighbouring columns per thread and round (every part a whole number of fours inside a head).  The gated row stays in
 // shared memory between the two passes; the warps' sums of squares are added in warp order.
-__device__ __forceinline__ float4 ldf4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ldf4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 ldf4(const bf16* p) {
-  const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
   return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
 }
 __device__ __forceinline__ void stf4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }

@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(LatentAttnArgs a, 
     for (int e = tid; e < R * e4; e += 256) {
       const int r = e / e4, c = (e - r * e4) * 4, tq = r / HB, h = h0 + r % HB;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (tq < ntq && h < a.heads) v = __ldg(reinterpret_cast<const float4*>(a.qlat + (static_cast<long long>(tok0 + tq0 + tq) * a.heads + h) * E + c));
+      if (tq < ntq && h < a.heads) v = *reinterpret_cast<const float4*>(a.qlat + (static_cast<long long>(tok0 + tq0 + tq) * a.heads + h) * E + c);
       *reinterpret_cast<__nv_bfloat162*>(Qs + r * LDE + c) = __floats2bfloat162_rn(v.x, v.y);
       *reinterpret_cast<__nv_bfloat162*>(Qs + r * LDE + c + 2) = __floats2bfloat162_rn(v.z, v.w);
     }
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(256) latent_attn_mma_wide_kernel(LatentAttnArg
     for (int e = tid; e < R * e4; e += 256) {
       const int r = e / e4, c = (e - r * e4) * 4, tq = r / HB, h = h0 + r % HB;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (tq < ntq && h < a.heads) v = __ldg(reinterpret_cast<const float4*>(a.qlat + (static_cast<long long>(tok0 + tq0 + tq) * a.heads + h) * E + c));
+      if (tq < ntq && h < a.heads) v = *reinterpret_cast<const float4*>(a.qlat + (static_cast<long long>(tok0 + tq0 + tq) * a.heads + h) * E + c);
       *reinterpret_cast<__nv_bfloat162*>(Qs + r * LDE + c) = __floats2bfloat162_rn(v.x, v.y);
       *reinterpret_cast<__nv_bfloat162*>(Qs + r * LDE + c + 2) = __floats2bfloat162_rn(v.z, v.w);
     }

@@ -338,6 +338,8 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
       if (n0 + (i & 15) < rows) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + static_cast<long long>(n0 + (i & 15)) * ldw + k0 + (i >> 4) * 64));
   }
   griddep_wait();
+  // the read-only path is for weights alone: rows of X may be written while this kernel waits
+  auto fetch = [](const bf16* p) { return THIN ? *reinterpret_cast<const uint4*>(p) : __ldg(reinterpret_cast<const uint4*>(p)); };
   const uint4 zero = make_uint4(0, 0, 0, 0);
   for (int s = ks * per; s < s1; s += U) {
     uint4 wa[U], wb[U], xv[U][NB], xl[U][SPLIT ? NB : 1];
@@ -345,8 +347,8 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
     for (int u = 0; u < U; ++u) {
       const int k = (s + u) * 32 + t4 * 8;
       const bool in = s + u < s1 && k < a.K;      // K is a multiple of 8: a piece is inside or outside as a whole
-      wa[u] = in && r0 ? __ldg(reinterpret_cast<const uint4*>(w0 + k)) : zero;
-      wb[u] = in && r1 ? __ldg(reinterpret_cast<const uint4*>(w1 + k)) : zero;
+      wa[u] = in && r0 ? fetch(w0 + k) : zero;
+      wb[u] = in && r1 ? fetch(w1 + k) : zero;
 #pragma unroll
       for (int i = 0; i < NB; ++i) {
         xv[u][i] = zero;

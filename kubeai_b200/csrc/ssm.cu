@@ -30,8 +30,8 @@ namespace b200 {
 namespace {
 
 typedef __nv_bfloat16 bf16;
-__device__ __forceinline__ float ldf(const float* p) { return __ldg(p); }
-__device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(__ldg(p)); }
+__device__ __forceinline__ float ldf(const float* p) { return *p; }
+__device__ __forceinline__ float ldf(const bf16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 __device__ __forceinline__ float siluf_(float x) { return x / (1.0f + expf(-x)); }

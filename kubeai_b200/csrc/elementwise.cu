@@ -71,9 +71,9 @@ template <int VPT>  // uint4 vectors per thread (H = VPT * 8 * blockDim)
 __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                const int* __restrict__ row_index, int H, float eps, PartialView pv) {
-  // ---- before the dependency wait (griddep.cuh griddep_enter): everything that does not come from the producer GEMM —
-  // the row index (step input), the residual (written four or more launches upstream), the norm weight and the
-  // partial-segment table entries (static)
+  // ---- before the dependency wait (griddep.cuh griddep_enter): the row index (step input), the norm weight and the
+  // partial-segment table entries (static).  The residual comes after it: its writer, the norm before, is only three launches
+  // upstream where gate_up's epilogue holds the gate, and the two GEMMs between release their consumers at entry.
   const int s = blockIdx.x;
   const int r = row_index ? row_index[s] : s;
   const uint4* xin = reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * H);
@@ -88,10 +88,12 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat1
     const int idx = threadIdx.x + i * blockDim.x;
     n0[i] = idx * 8;
     ww[i].u = __ldg(reinterpret_cast<const uint4*>(w) + idx);
-    if (res) rb[i].u = res[idx];
   }
   if (pv.ws) partial_entries<VPT>(pv, r, n0, ent);
   griddep_enter();
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (res) rb[i].u = res[threadIdx.x + i * blockDim.x];
   float xa[VPT][8];
   if (pv.ws) {
     load8xM_entries<VPT>(pv, ent, r, n0, xa);  // x = bf16(sum of the GEMM's stream-K segments)

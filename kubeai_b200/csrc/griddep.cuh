@@ -8,12 +8,13 @@ namespace b200 {
 // at its own griddepcontrol.wait for our completion before touching dependent data).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Dependency point of every non-GEMM kernel: wait for the producer, THEN let the consumer launch.  GEMMs release their
-// consumer at entry (before their own wait).  Consequence used by the kernels' pre-wait prologues: code that runs
-// before griddep_enter() in kernel K_n may read
-//   * anything written by K_{n-2} or earlier when K_{n-1} is a non-GEMM kernel,
-//   * anything written by K_{n-3} or earlier when K_{n-1} is a GEMM (two GEMMs are never adjacent),
-//   * per-step inputs uploaded before the step's first kernel, and static tables (weights, cos/sin, segment tables).
+// Dependency point of every non-GEMM kernel of the Llama path: wait for the producer, THEN let the consumer launch.  GEMMs
+// release their consumer at entry (before their own wait).  Consequence used by the kernels' pre-wait prologues: code that
+// runs before griddep_enter() in kernel K_n may read per-step inputs uploaded before the step's first kernel, static tables
+// (weights, cos/sin, segment tables), and of what the step's kernels write only
+//   * the output of K_{n-2} or earlier when K_{n-1} is a non-GEMM kernel (it was released after K_{n-2} had completed),
+//   * with g GEMMs directly in front, the output of K_{n-g-2} or earlier: the last non-GEMM kernel in front of them is known
+//     to have STARTED, not to have completed.
 __device__ __forceinline__ void griddep_enter() {
   griddep_wait();
   griddep_launch();

@@ -119,6 +119,9 @@ int b200_stats_get(b200_engine* e, b200_stats* out);
 /* 1 when a CUDA failure has poisoned this replica (every request fails with B200_FINISH_ERROR / B200_ERR_CUDA from then on):
  * the serving shell drops such a replica from the router's endpoint set (internal/loadbalancer/group.go:119-131). */
 int b200_engine_is_failed(b200_engine* e);
+/* Tests: whether the engine's kernels have left the mark of a wait that ran out (0 / 1); set >= 0 then makes it so.  A step that ends
+ * with the mark set returns B200_ERR_CUDA and no results. */
+int b200_engine_kernel_mark(b200_engine* e, int32_t set);
 
 /* manual_step mode: run one scheduler iteration + forward; *info may be NULL. Returns 1 if a step ran, 0 if idle. */
 int b200_engine_step(b200_engine* e, b200_step_info* info);
@@ -368,6 +371,9 @@ int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, i
  * NULL turns it off.  Stamps: 0 entry, 1 after prologue, 2 first tile accumulated, 3 main loop + partial stores
  * done, 4 peers' partials visible, 5 bulk pull landed, 6 before final cluster sync, 7 exit. */
 int b200_op_gemm_trace(void* trace_dev);
+/* Tests: the mark of b200_op_gemm's kernels for a wait that ran out (0 / 1); set >= 0 makes it so.  The next b200_op_gemm reports a mark
+ * once (B200_ERR_CUDA) and clears it. */
+int b200_op_kernel_mark(int32_t set);
 /* Same contraction, but the GEMM only dumps fp32 stream-K partials and a second kernel reduces them to bf16 —
  * the engine's T <= 512 path (there the reduction is fused into the consumer kernels). */
 int b200_op_gemm_deferred(const void* w, const void* x, void* out, int32_t N, int32_t T, int32_t K, void* stream);

@@ -124,6 +124,8 @@ SYMBOLS = {
     "b200_release": (C.c_int, [_vp, _u64]),
     "b200_stats_get": (C.c_int, [_vp, C.POINTER(Stats)]),
     "b200_engine_is_failed": (C.c_int, [_vp]),
+    "b200_engine_kernel_mark": (C.c_int, [_vp, _i32]),
+    "b200_op_kernel_mark": (C.c_int, [_i32]),
     "b200_engine_step": (C.c_int, [_vp, C.POINTER(StepInfo)]),
     "b200_engine_run": (C.c_int, [_vp, _i32, _i64, C.POINTER(StepInfo), C.POINTER(_i32)]),
     "b200_engine_replay": (C.c_int, [_vp, _i32, _i32, C.POINTER(C.c_double), C.POINTER(_i64), C.POINTER(_i64),

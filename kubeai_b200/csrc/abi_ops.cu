@@ -49,6 +49,7 @@ std::mutex g_mu;
 float* g_ws = nullptr;
 size_t g_ws_bytes = 0;
 int* g_counters = nullptr;
+int* g_mark = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
 constexpr int kCounterInts = 1 << 20;
 
 int ensure_scratch() {
@@ -61,7 +62,22 @@ int ensure_scratch() {
   if (cudaMalloc(&g_ws, g_ws_bytes) != cudaSuccess) return -1;
   if (cudaMalloc(&g_counters, kCounterInts * sizeof(int)) != cudaSuccess) return -1;
   cudaMemset(g_counters, 0, kCounterInts * sizeof(int));
+  if (cudaMallocHost(&g_mark, sizeof(int)) != cudaSuccess) return -1;
+  *g_mark = 0;
   return 0;
+}
+
+// The operations return before their kernels have run, so one that gave up waiting is reported by the next: an error once, and
+// the split counters it left behind are cleared.
+int report_mark() {
+  std::lock_guard<std::mutex> lk(g_mu);
+  volatile int* mark = g_mark;
+  if (!*mark) return 0;
+  cudaDeviceSynchronize();
+  cudaMemset(g_counters, 0, kCounterInts * sizeof(int));
+  *mark = 0;
+  set_error("a wait inside the kernel of an earlier product ran out: its output is not valid");
+  return B200_ERR_CUDA;
 }
 }  // namespace
 }  // namespace b200
@@ -84,9 +100,11 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
     set_error("b200_op_gemm: workspace allocation failed");
     return B200_ERR_OOM;
   }
+  if (int rc = report_mark()) return rc;
   GemmPlan plan;
   int rc = gemm_plan_init(&plan, w, N, K, K, g_ws, g_counters, 0);
   if (rc) return cuda_fail("gemm_plan_init", rc);
+  plan.error = g_mark;
   const int bn = gemm_block_n_for(T);
   const int slabs = (N + 127) / 128, ntt = (T + bn - 1) / bn;
   if (2ll * slabs * ntt > kCounterInts) {
@@ -99,6 +117,15 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
   rc = gemm_run(plan, tmx, bn, out, N, T, static_cast<cudaStream_t>(stream));
   if (rc) return cuda_fail("gemm_run", rc);
   return 0;
+}
+
+int b200_op_kernel_mark(int32_t set) {
+  if (int rc = require_device()) return rc;
+  if (ensure_scratch()) { set_error("b200_op_kernel_mark: workspace allocation failed"); return B200_ERR_OOM; }
+  volatile int* mark = g_mark;
+  const int was = *mark ? 1 : 0;
+  if (set >= 0) *mark = set ? 1 : 0;
+  return was;
 }
 
 int b200_op_gemm_deferred(const void* w, const void* x, void* out, int32_t N, int32_t T, int32_t K, void* stream) {

@@ -115,7 +115,6 @@ class Dabodra : public Model {
   void *egu = nullptr, *eact = nullptr, *sh = nullptr, *shact = nullptr, *sdown = nullptr, *hsorted = nullptr, *edown16 = nullptr;
   int *topi = nullptr, *sorted_rows = nullptr, *tile_group = nullptr, *pair_pos = nullptr, *iota = nullptr;
   int* expert_rows = nullptr;
-  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int row_cap = 0, moe_cap = 0;
   std::vector<void*> allocs;
   void* attn_ws = nullptr;       // of the attention of whole prompts
@@ -135,7 +134,6 @@ class Dabodra : public Model {
       if (w.tc_shdown) gemm_plan_destroy(&w.p_shdown);
     }
     if (pe0) { cudaEventDestroy(pe0); cudaEventDestroy(pe1); }
-    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Dabodra"; }
@@ -336,8 +334,6 @@ class Dabodra : public Model {
       if (s.shared) rc |= mat(&w.sh_in, s.n_sh, W) | mat(&w.sh_down, W, s.sff);
     }
     if (rc) return rc;
-    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
-    *kernel_error = 0;
     const size_t T = e.Tcap;
     row_cap = static_cast<int>(std::min<size_t>(T, 256));
     rc |= vec(&x, T * W) | mat(&h, T, W) | mat(&inb, T, max_in) | mat(&yb, T, max_out) | mat(&ao, T, W) | mat(&hrow, row_cap, W) |
@@ -394,7 +390,7 @@ class Dabodra : public Model {
     auto plan = [&](GemmPlan* p, const void* Wm, int N, int K) {
       if (N % 8 || K % 8 || gemm_plan_init(p, Wm, N, K, K, gemm_ws, gemm_counters, env.sms)) return false;
       p->ws_bytes = ws_bytes;
-      p->error = kernel_error;
+      p->error = env.kernel_error;
       return true;
     };
     auto plan_maps = [&](GemmPlan* p, CUtensorMap* m, const void* X, const void* Wm, int N, int K) {
@@ -648,7 +644,7 @@ class Dabodra : public Model {
     wa.T = b.T; wa.heads = s.heads; wa.kv_heads = s.kv_heads; wa.dim = s.dim; wa.vdim = s.vdim;
     wa.window = s.window; wa.scale = s.scale; wa.sink = w.sink;
     wa.seqs = b.seqs; wa.nseq = b.nseq; wa.max_ctx = b.max_ctx;
-    wa.fresh = b.fresh; wa.slots = b.slots; wa.ws = attn_ws; wa.error = kernel_error;
+    wa.fresh = b.fresh; wa.slots = b.slots; wa.ws = attn_ws; wa.error = env.kernel_error;
     KRN("window_attention", window_attention(wa, st));
     return rc;
   }
@@ -682,7 +678,7 @@ class Dabodra : public Model {
   int moe(const LayerSpec& s, const LayerWeights& w, int T, int64_t& nl) {
     cudaStream_t st = env.stream;
     int rc = 0;
-    KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, s.experts, W), st));
+    KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, s.experts, W, env.kernel_error), st));
     MoeRouteForm form;
     form.group_best = 2; form.normalize = true; form.sum_eps = kWeightSumEps; form.scale = s.route_scale;
     KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, s.groups, s.keep, s.top, st, MOE_SIGMOID, s.experts, w.correction, form));
@@ -720,15 +716,15 @@ class Dabodra : public Model {
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
       if (w.il_e) {
         const GroupedOut o = {eact, s.ff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, env.kernel_error, st));
       } else {
         const GroupedOut o = {egu, 2 * s.ff};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, env.kernel_error, st));
         KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f));
       }
       const bool wide = T * s.top <= 64;     // fp32 until the combine, as the passes per pair leave them
       const GroupedOut o = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
-      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, o, env.sms, kernel_error, st));
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, o, env.sms, env.kernel_error, st));
       KRN("moe_combine", moe_combine_add(o.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, shared_out, nullptr, 0, fo, dt, T, s.top, W, st));
       return rc;
     }
@@ -748,7 +744,6 @@ class Dabodra : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
-    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Dabodra forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_normed(embed, dt, b.ids, emb_w, eps, x, h, dt, T, W, V, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {
@@ -780,7 +775,7 @@ class Dabodra : public Model {
     for (int r0 = 0; r0 < b.S && !rc; r0 += row_cap) {
       const int n = std::min(row_cap, b.S - r0);
       KRN("residual_norm", sandwich_step(boundary(Pending(), fin_w, hrow, b.rows + r0, n), st));
-      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W), st));
+      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
       KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
       if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
                                          cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -2;

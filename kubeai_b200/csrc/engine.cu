@@ -240,6 +240,7 @@ struct Engine {
   uint8_t* feed_stage = nullptr;
   cudaEvent_t feed_ev[2] = {nullptr, nullptr};
   int init_feed();
+  int check_kernels();
   int read_logits_f32(float* out, size_t count);
   std::vector<float> residual_dump;
   int L, H, Hq, Hkv, I, V, QKV;
@@ -551,8 +552,6 @@ int Engine::alloc_all() {
   CK(cudaMemset(gemm_counters, 0, n_counters * 4));
 
   // ---- GEMM plans + activation tensor maps (encoded once; kernels mask rows >= T)
-  CK(cudaMallocHost(&kernel_error, sizeof(int)));
-  *kernel_error = 0;
   auto plan = [&](GemmPlan* p, const void* W, int N, int K) {
     int rc = gemm_plan_init(p, W, N, K, K, gemm_ws, gemm_counters, sms);
     if (rc) return rc;
@@ -672,6 +671,8 @@ int Engine::init_model(const b200_config& c, std::unique_ptr<Model> mdl) {
   Scap = c.max_num_seqs;
   memset(&stats, 0, sizeof(stats));
   CK(cudaSetDevice(c.device));
+  CK(cudaMallocHost(&kernel_error, sizeof(int)));
+  *kernel_error = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
   CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ev0));
@@ -695,7 +696,7 @@ int Engine::init_model(const b200_config& c, std::unique_ptr<Model> mdl) {
   }
   ModelEnv env;
   env.stream = stream; env.device = c.device; env.sms = sms; env.Tcap = Tcap; env.max_model_len = cfg.max_model_len;
-  env.page = kPage; env.num_blocks = nblocks; env.num_slots = Scap;
+  env.page = kPage; env.num_blocks = nblocks; env.num_slots = Scap; env.kernel_error = kernel_error;
   if (int rc = model->init(env)) return rc == -3 ? B200_ERR_OOM : (rc == -1 ? B200_ERR_INVALID : B200_ERR_CUDA);
   // pages of a sequence with recurrent state cannot be shared by prefix: the state after the prefix is not in them
   pool.init(nblocks, cfg.enable_prefix_caching != 0 && model->state_bytes_per_slot() == 0);
@@ -749,6 +750,8 @@ int Engine::init(const b200_config& c) {
   Scap = c.max_num_seqs;
   memset(&stats, 0, sizeof(stats));
   CK(cudaSetDevice(c.device));
+  CK(cudaMallocHost(&kernel_error, sizeof(int)));
+  *kernel_error = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
   CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ev0));
@@ -763,7 +766,6 @@ int Engine::init(const b200_config& c) {
 // ------------------------------------------------------------------ forward pass (fixed kernel sequence)
 int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* logits_out) {
   if (model) return forward_model(m, dbuf, nullptr);
-  if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("forward: a wait inside a projection ran out"); return B200_ERR_CUDA; }
   const int T = m.T;
   const int* ids = dbuf + m.off_ids;
   const int* pos = dbuf + m.off_pos;
@@ -1440,6 +1442,7 @@ int Engine::launch(InFlight* f, StepMeta* mp) {
 int Engine::complete(InFlight& f, const StepMeta& m, b200_step_info* info) {
   static const bool timing = [] { const char* e = getenv("B200_STEP_TIMING"); return e && atoi(e) != 0; }();
   CK(cudaStreamSynchronize(stream));
+  if (int rc = check_kernels()) return rc;
   const double ht3 = timing ? now_s() : 0.0;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ev0, ev1);
@@ -1517,9 +1520,16 @@ int Engine::complete(InFlight& f, const StepMeta& m, b200_step_info* info) {
   return 1;
 }
 
-// One step whose tokens the caller supplies (b200_feed_step): the listed sequences advance by exactly the given tokens, as
-// one batch, through the same page / slot bookkeeping, packing and forward pass as a scheduled step; nothing is sampled
-// into the sequences.  Logits of the wanted positions go to logits_out in the order of the entries.
+// After the wait for a step: whether one of its kernels gave up waiting (a bounded wait inside it ran out), so that what the step
+// computed is not valid.  Nothing of it may leave the engine, and no later step can build on it.
+int Engine::check_kernels() {
+  if (!*static_cast<volatile int*>(kernel_error)) return 0;
+  set_error("a wait inside a kernel of the step ran out");
+  std::lock_guard<std::mutex> lk(mu_);
+  fatal = true;
+  return B200_ERR_CUDA;
+}
+
 int Engine::init_feed() {
   if (!cfg.manual_step) return 0;
   CK(cudaMallocHost(&feed_stage, 2 * kFeedHalf));
@@ -1547,6 +1557,9 @@ int Engine::read_logits_f32(float* out, size_t count) {
   return 0;
 }
 
+// One step whose tokens the caller supplies (b200_feed_step): the listed sequences advance by exactly the given tokens, as
+// one batch, through the same page / slot bookkeeping, packing and forward pass as a scheduled step; nothing is sampled
+// into the sequences.  Logits of the wanted positions go to logits_out in the order of the entries.
 int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, int64_t cap_floats) {
   InFlight& f = inflight_;
   f.sched.clear();
@@ -1610,7 +1623,8 @@ int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, 
     if (!rc) {
       CK(cudaEventRecord(ev1, stream));
       CK(cudaStreamSynchronize(stream));
-      if (staged && S) memcpy(logits_out, feed_stage, static_cast<size_t>(S) * V * sizeof(float));
+      rc = check_kernels();
+      if (!rc && staged && S) memcpy(logits_out, feed_stage, static_cast<size_t>(S) * V * sizeof(float));
     }
   }
   if (rc) {
@@ -1881,6 +1895,14 @@ int b200_engine_is_failed(b200_engine* e) {
   return e->impl.fatal ? 1 : 0;
 }
 
+int b200_engine_kernel_mark(b200_engine* e, int32_t set) {
+  if (!e) { set_error("null engine"); return B200_ERR_INVALID; }
+  volatile int* mark = e->impl.kernel_error;
+  const int was = *mark ? 1 : 0;
+  if (set >= 0) *mark = set ? 1 : 0;
+  return was;
+}
+
 int b200_engine_step(b200_engine* e, b200_step_info* info) {
   if (!e) { set_error("null engine"); return B200_ERR_INVALID; }
   if (!e->impl.cfg.manual_step) { set_error("engine was not created with manual_step"); return B200_ERR_INVALID; }
@@ -1919,6 +1941,7 @@ int b200_engine_replay(b200_engine* e, int32_t n, int32_t repeat, double* ms_tot
   }
   CK(cudaEventRecord(g.ev1, g.stream));
   CK(cudaStreamSynchronize(g.stream));
+  if (int rc = g.check_kernels()) return rc;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, g.ev0, g.ev1);
   if (ms_total) *ms_total = ms;
@@ -1962,6 +1985,7 @@ int b200_engine_profile_range(b200_engine* e, int32_t n, int32_t min_tokens, int
     g.profiling = false;
     if (rc) return rc;
     CK(cudaStreamSynchronize(g.stream));
+    if ((rc = g.check_kernels())) return rc;
     for (size_t k = 0; k + 1 < g.prof_used; k += 2) {
       float ms = 0.f;
       cudaEventElapsedTime(&ms, g.prof_events[k].second, g.prof_events[k + 1].second);
@@ -2115,6 +2139,7 @@ int b200_engine_forward_logits(b200_engine* e, const int32_t* ids, int32_t n, vo
     ce = cudaMemcpyAsync(host_logits_bf16, dl, static_cast<size_t>(n) * g.V * 2, cudaMemcpyDeviceToHost, g.stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(g.stream);
     if (ce != cudaSuccess) { set_error("forward_logits: %s", cudaGetErrorString(ce)); rc = B200_ERR_CUDA; }
+    else rc = g.check_kernels();
   }
   cudaFree(dl);
   for (auto it = s.blocks.rbegin(); it != s.blocks.rend(); ++it) g.pool.unref(*it);

@@ -101,7 +101,7 @@ bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo);
 // 2 * box), parts the pieces K is cut into (p.ws and p.counters hold them; a pair then has one item).
 int gemm_whole_run_as(const GemmPlan& p, const CUtensorMap& tm_x, int box, int tile, int parts, int rows, const GroupedOut& o, int* error, cudaStream_t st);
 // ... without a plan: the maps are made for the call (K, ldw, ldx multiples of 8, W and X on 16-byte boundaries, K whole).
-int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, cudaStream_t st);
+int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, int* error, cudaStream_t st);
 int gemm_whole_parts(int N, int K, int tile, int tiles, int units);
 // Generic consumer: out[t, n] = bf16(sum of segments) — used by tests and by paths without a fused consumer.
 int reduce_partials(const PartialView& v, void* out, int ldo, int T, int N, cudaStream_t st);

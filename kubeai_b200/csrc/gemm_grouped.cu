@@ -256,11 +256,13 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   bool ok = true;
   griddep_launch();
-  if (expert_rows) griddep_wait();     // every role walks the table
+  // Every role walks the table.  Without one only the loading thread has something to do before the kernel in front has ended; the
+  // others wait for that here, so that no limited wait below runs out over the length of another kernel.
+  if (expert_rows || warp != 0) griddep_wait();
 
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0, ahead = 0;
+      int stage = 0, ahead = 0, filled = 0;
       uint32_t phase = 0;
       Tile t;
       auto load_w = [&](int st, int kb) {
@@ -284,11 +286,19 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             if (!wait_limited(empty_bar(stage), phase ^ 1u)) { ok = false; break; }
             load_w(stage, kb);
           }
+          filled = min(filled + 1, stages);
           // this CTA stages the rank-th half of the row tile (rows of the box past nc / 2 are not used)
           tma_load_2d_pair(sa + kABytes, &tm_x, full_bar(stage), kb * kBlockK, t.row0 + static_cast<int>(rank) * (nc >> 1), kEvictLast);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
+      // The copies started last have landed before the CTA ends, also where a role gave up: the leader's barriers count both CTAs'
+      // bytes.  (Where none did, they were waited for long ago.)
+      if (leader)
+        for (int i = 0; i < filled; ++i) {
+          if (--stage < 0) { stage = stages - 1; phase ^= 1u; }
+          wait_limited(full_bar(stage), phase);
+        }
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {
@@ -522,7 +532,7 @@ int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int 
   return gemm_whole_run_as(p, tm_x, box, tile, gemm_whole_parts(p.N, p.K, tile, tiles, p.max_ctas / 2), rows, o, p.error, st);
 }
 
-int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, cudaStream_t st) {
+int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, int* error, cudaStream_t st) {
   CUtensorMap tm_w, tm_x;
   int dev = 0, sms = 0, i = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
@@ -530,7 +540,7 @@ int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int
   const int box = kBoxes[i], ntt = (rows + 2 * box - 1) / (2 * box), tile = ((rows + ntt - 1) / ntt + 15) & ~15;
   if (tmap_encode_bf16_2d(&tm_w, W, N, K, ldw, kSlab, kBlockK, 1) || tmap_encode_bf16_2d(&tm_x, X, rows, K, ldx, box, kBlockK, 1)) return -2;
   const long long tiles = static_cast<long long>((N + 2 * kSlab - 1) / (2 * kSlab)) * ((rows + tile - 1) / tile);
-  return launch(tm_w, 1, N, K, tm_x, box, nullptr, rows, o, {nullptr, nullptr, 1, tile}, static_cast<int>(std::min<long long>(sms / 2, tiles)), nullptr, st);
+  return launch(tm_w, 1, N, K, tm_x, box, nullptr, rows, o, {nullptr, nullptr, 1, tile}, static_cast<int>(std::min<long long>(sms / 2, tiles)), error, st);
 }
 
 bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo) {

@@ -450,7 +450,7 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
       if (whole && vec && a.T > mma_rows && a.N >= 256 && a.N % 8 == 0 && a.ldy % 4 == 0 && reinterpret_cast<uintptr_t>(a.Y) % 16 == 0 && a.batch == 1 && !a.x_rows &&
           !a.tile_group && !a.row_scale && a.act == LIN_NONE && gemm_variant() == 2) {
         GroupedOut o = {a.Y, a.ldy, GROUPED_F32, a.bias};
-        return gemm_whole_direct(a.W, a.ldw, a.X, a.ldx, a.N, a.K, a.T, o, st);
+        return gemm_whole_direct(a.W, a.ldw, a.X, a.ldx, a.N, a.K, a.T, o, a.error, st);
       }
     }
     if constexpr (sizeof(TX) == 2) {

@@ -43,6 +43,7 @@ struct ModelEnv {
   int page;              // tokens per page of the block pool
   int64_t num_blocks;    // pages in the pool
   int num_slots;         // recurrent-state slots (one per live sequence)
+  int* kernel_error;     // pinned: a kernel whose wait ran out leaves a mark here; the engine looks at it after every step
 };
 
 struct TensorRef {

@@ -119,7 +119,6 @@ class Mulenex : public Model {
   int row_cap = 0, moe_cap = 0, vfirst_ld = 0;
   void *hsorted = nullptr, *edown16 = nullptr;
   int* expert_rows = nullptr;
-  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int moe_tc_min = 1;
   float* scan_ws = nullptr;      // of the scan whose chunks run side by side
   size_t scan_ws_floats = 0;
@@ -140,7 +139,6 @@ class Mulenex : public Model {
       if (w.tc_shin) gemm_plan_destroy(&w.p_shin);
       if (w.tc_shdown) gemm_plan_destroy(&w.p_shdown);
     }
-    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Mulenex"; }
@@ -291,8 +289,6 @@ class Mulenex : public Model {
         if (s.shared) { any_shared = true; max_nsh = std::max(max_nsh, s.n_sh); max_sff = std::max(max_sff, s.sff); }
       }
     }
-    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
-    *kernel_error = 0;
     int rc = 0;
     auto mat = [&](void** p, size_t rows, size_t cols) { return dalloc(p, rows * cols * es); };
     auto vec = [&](float** p, size_t n) { return dalloc(p, n * sizeof(float)); };
@@ -379,7 +375,7 @@ class Mulenex : public Model {
     auto plan = [&](GemmPlan* p, const void* Wm, int N, int K) {
       if (K % 8 || gemm_plan_init(p, Wm, N, K, K, gemm_ws, gemm_counters, env.sms)) return false;
       p->ws_bytes = ws_bytes;
-      p->error = kernel_error;
+      p->error = env.kernel_error;
       return true;
     };
     auto maps = [&](CUtensorMap* xm, const void* X, int K) {
@@ -660,7 +656,7 @@ class Mulenex : public Model {
     wa.T = b.T; wa.heads = s.heads; wa.kv_heads = s.kv_heads; wa.dim = s.dim; wa.vdim = s.vdim;
     wa.window = 1 << 30; wa.keep_first = 0; wa.scale = s.scale; wa.softcap = s.softcap;
     wa.seqs = b.seqs; wa.nseq = b.nseq; wa.max_ctx = b.max_ctx;
-    wa.fresh = b.fresh; wa.slots = b.slots; wa.ws = attn_ws; wa.error = kernel_error;
+    wa.fresh = b.fresh; wa.slots = b.slots; wa.ws = attn_ws; wa.error = env.kernel_error;
     KRN("attention", window_attention(wa, st));
     return rc;
   }
@@ -671,7 +667,7 @@ class Mulenex : public Model {
     auto col = [&](void* base, size_t off) { return static_cast<void*>(static_cast<uint8_t*>(base) + off * es); };
     int rc = 0;
     // gate pre-activations in fp32 straight from the accumulator, bias included
-    LinearArgs ga = linear_args(h, dt, w.w_gates, dt, gpre, DT_F32, b.T, 2 * s.heads, W);
+    LinearArgs ga = linear_args(h, dt, w.w_gates, dt, gpre, DT_F32, b.T, 2 * s.heads, W, env.kernel_error);
     ga.bias = w.b_gates;
     KRN("mlstm_gate_proj", linear(ga, st));
     MlstmGateArgs mg;
@@ -706,7 +702,7 @@ class Mulenex : public Model {
     cudaStream_t st = env.stream;
     int rc = 0;
     const int nr = s.experts + (s.shared ? 1 : 0);   // router logits and, behind them, the shared expert's gate logit
-    LinearArgs ra = linear_args(h, dt, w.router, dt, scores, DT_F32, T, nr, W);
+    LinearArgs ra = linear_args(h, dt, w.router, dt, scores, DT_F32, T, nr, W, env.kernel_error);
     ra.bias = w.router_b;
     KRN("moe_router", linear(ra, st));
     KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, 1, 1, s.top, st, MOE_TOP_SOFTMAX, nr));
@@ -751,14 +747,14 @@ class Mulenex : public Model {
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
       if (w.il_e) {
         const GroupedOut o = {eact, s.ff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, env.kernel_error, st));
       } else {
         const GroupedOut o = {egu, 2 * s.ff};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, env.kernel_error, st));
         KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, INFINITY, 1.f, st, 0.f));
       }
       const GroupedOut o = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
-      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, o, env.sms, kernel_error, st));
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, o, env.sms, env.kernel_error, st));
       KRN("moe_combine", moe_combine_add(o.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, shared_out, shared_gate, nr, fo, dt, T, s.top, W, st));
       return rc;
     }
@@ -778,7 +774,6 @@ class Mulenex : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
-    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Mulenex forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_sinusoid(embed, dt, b.ids, b.pos, pos_freq, x, T, W, V, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {
@@ -811,7 +806,7 @@ class Mulenex : public Model {
     for (int r0 = 0; r0 < b.S && !rc; r0 += row_cap) {
       const int n = std::min(row_cap, b.S - r0);
       KRN("residual_norm", sandwich_step(boundary(Pending(), fin_w, hrow, dt, b.rows + r0, n), st));
-      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W), st));
+      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
       KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
       if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
                                          cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -2;

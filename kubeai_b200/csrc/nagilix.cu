@@ -139,7 +139,6 @@ class Nagilix : public Model {
   int row_cap = 0, moe_cap = 0;
   void *hsorted = nullptr, *edown16 = nullptr;
   int* expert_rows = nullptr;
-  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int moe_tc_min = 1;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
@@ -155,7 +154,6 @@ class Nagilix : public Model {
       if (w.tc_ro) gemm_plan_destroy(&w.p_ro);
       if (w.tc_rg2) gemm_plan_destroy(&w.p_rg2);
     }
-    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Nagilix"; }
@@ -443,28 +441,26 @@ class Nagilix : public Model {
       if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
           dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
     }
-    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
-    *kernel_error = 0;
     if (const char* e = getenv("B200_NG_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
     for (size_t i = 0; i < spec.size(); ++i) {
       const LayerSpec& s = spec[i];
       LayerWeights& w = wts[i];
       w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = kernel_error; }
+      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = env.kernel_error; }
       const int k_lo = s.kind == MIX_PARALLEL ? s.hv_l : s.m.inner;
       w.tc_lo = k_lo % 8 == 0 && gemm_plan_init(&w.p_lo, w.w_lo, W, k_lo, k_lo, gemm_ws, gemm_counters, env.sms) == 0;
       for (int j = 0; j < kGemmNumBlockN && w.tc_lo; ++j)
         if (gemm_make_x_map(&w.xm_lo[j], yl, env.Tcap, k_lo, k_lo, bns[j])) w.tc_lo = false;
-      if (w.tc_lo) { w.p_lo.ws_bytes = ws_bytes; w.p_lo.error = kernel_error; }
+      if (w.tc_lo) { w.p_lo.ws_bytes = ws_bytes; w.p_lo.error = env.kernel_error; }
       if (s.kind == MIX_PARALLEL) {
         w.tc_ro = s.hv_r % 8 == 0 && gemm_plan_init(&w.p_ro, w.w_ro, W, s.hv_r, s.hv_r, gemm_ws, gemm_counters, env.sms) == 0;
         for (int j = 0; j < kGemmNumBlockN && w.tc_ro; ++j)
           if (gemm_make_x_map(&w.xm_ro[j], yr, env.Tcap, s.hv_r, s.hv_r, bns[j])) w.tc_ro = false;
-        if (w.tc_ro) { w.p_ro.ws_bytes = ws_bytes; w.p_ro.error = kernel_error; }
+        if (w.tc_ro) { w.p_ro.ws_bytes = ws_bytes; w.p_ro.error = env.kernel_error; }
       }
       if (s.mlp && gated) {
         w.tc_rg2 = gemm_plan_init(&w.p_rg2, w.rg2, W, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-        if (w.tc_rg2) { w.p_rg2.ws_bytes = ws_bytes; w.p_rg2.error = kernel_error; }
+        if (w.tc_rg2) { w.p_rg2.ws_bytes = ws_bytes; w.p_rg2.error = env.kernel_error; }
       }
       if (s.mlp && s.experts > 0) {
         w.tc_experts = !gemm_grouped_plan(&w.g_egu, w.e_gu, s.experts, 2 * s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
@@ -770,7 +766,7 @@ class Nagilix : public Model {
     KRN("conv_carry", short_conv_carry(cc, st));
     // [dt | B | C] and the step sizes' pre-activations leave their products in fp32
     const int nx = m.dt_rank + 2 * m.state;
-    KRN("ssm_x_proj", linear(linear_args(xc, dt, w.w_x, dt, xdbc, DT_F32, T, nx, m.inner), st));
+    KRN("ssm_x_proj", linear(linear_args(xc, dt, w.w_x, dt, xdbc, DT_F32, T, nx, m.inner, env.kernel_error), st));
     LinearArgs dl = linear_args(xdbc, DT_F32, w.w_dt, dt, dtp, DT_F32, T, m.inner, m.dt_rank);
     dl.ldx = nx; dl.bias = w.dt_b;
     KRN("ssm_dt_proj", linear(dl, st));
@@ -788,7 +784,7 @@ class Nagilix : public Model {
     cudaStream_t st = env.stream;
     int rc = 0;
     const int ne = s.experts + s.identity;    // router outputs: the experts, then the identity experts
-    KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, ne, W), st));
+    KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, ne, W, env.kernel_error), st));
     KRN("moe_route", moe_route(scores, topi, topw, T, ne, 1, 1, s.top, st, MOE_SOFTMAX, ne, w.correction));
     const long long gu_stride = 2ll * s.ff * W, down_stride = static_cast<long long>(W) * s.ff;
     const bool grouped = w.tc_experts && T >= moe_tc_min;
@@ -823,14 +819,14 @@ class Nagilix : public Model {
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
       if (w.il_e) {
         const GroupedOut up = {eact, s.ff, GROUPED_GATED, nullptr, s.limit, 1.702f, 1.0f};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, env.kernel_error, st));
       } else {
         const GroupedOut up = {egu, 2 * s.ff};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, env.kernel_error, st));
         KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
       }
       const GroupedOut dn = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
-      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, kernel_error, st));
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, env.kernel_error, st));
       KRN("moe_combine", moe_combine_identity(dn.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, topi, s.experts, h, fo, dt, T, s.top, W, st));
       return rc;
     }
@@ -852,7 +848,6 @@ class Nagilix : public Model {
     int64_t nl = 0;
     const size_t es = dtype_bytes(dt);
     auto col = [&](void* base, size_t off) { return static_cast<void*>(static_cast<uint8_t*>(base) + off * es); };
-    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Nagilix forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_learned_pos(embed, pos_table, dt, b.ids, b.pos, x, T, W, V, max_pos, ns, xstride, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {
@@ -893,7 +888,7 @@ class Nagilix : public Model {
     for (int r0 = 0; r0 < b.S && !rc; r0 += row_cap) {
       const int n = std::min(row_cap, b.S - r0);
       KRN("stream_norm", hyper_step(boundary(Pending(), nullptr, fin_w, hrow, dt, b.rows + r0, n), st));
-      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W), st));
+      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
       KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
       if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
                                          cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -2;

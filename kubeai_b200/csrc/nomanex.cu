@@ -116,7 +116,6 @@ class Nomanex : public Model {
   long long split_ws_floats = 0;
   void *hsorted = nullptr, *edown16 = nullptr;   // tensor-core experts: gathered inputs, bf16 expert outputs
   int* expert_rows = nullptr;
-  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int moe_tc_min = 1;
   float* scan_ws = nullptr;      // of the scan whose chunks run side by side
   size_t scan_ws_floats = 0;
@@ -134,7 +133,6 @@ class Nomanex : public Model {
       if (w.tc_in) gemm_plan_destroy(&w.p_in);
       if (w.tc_out) gemm_plan_destroy(&w.p_out);
     }
-    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   // (profiling events are released with the context)
@@ -401,26 +399,24 @@ class Nomanex : public Model {
       if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
           dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
     }
-    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
-    *kernel_error = 0;
     if (const char* e = getenv("B200_NX_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
     for (size_t i = 0; i < spec.size(); ++i) {
       const LayerSpec& s = spec[i];
       if (s.weights_of != static_cast<int>(i)) continue;
       LayerWeights& w = wts[i];
       w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = kernel_error; }
+      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = env.kernel_error; }
       w.tc_out = s.k_out % 8 == 0 && gemm_plan_init(&w.p_out, w.w_out, W, s.k_out, s.k_out, gemm_ws, gemm_counters, env.sms) == 0;
       for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
         if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
-      if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = kernel_error; }
+      if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = env.kernel_error; }
       if (s.mixer == MIX_LATENT && s.rot_dims > 0 && latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank)) {
         const int N = s.heads * (s.dim + s.vdim);
         if (dalloc(&w.ukv, static_cast<size_t>(N) * s.kv_rank * 2)) return -3;
         w.tc_ukv = gemm_plan_init(&w.p_ukv, w.ukv, N, s.kv_rank, s.kv_rank, gemm_ws, gemm_counters, env.sms) == 0;
         for (int j = 0; j < kGemmNumBlockN && w.tc_ukv; ++j)
           if (gemm_make_x_map(&w.xm_c[j], qlat, env.Tcap, s.kv_rank, s.kv_rank, bns[j])) w.tc_ukv = false;
-        if (w.tc_ukv) { w.p_ukv.ws_bytes = ws_bytes; w.p_ukv.error = kernel_error; }
+        if (w.tc_ukv) { w.p_ukv.ws_bytes = ws_bytes; w.p_ukv.error = env.kernel_error; }
       }
       if (s.ff_kind == FF_MOE)
         w.tc_experts = !gemm_grouped_plan(&w.g_eup, w.e_up, s.experts, s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
@@ -614,7 +610,6 @@ class Nomanex : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
-    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Nomanex forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_bigram(embed, bigram, dt, b.ids, b.prev_ids, x, T, W, V, buckets, mul_prev, mul_cur, st));
     const LayerWeights& w0 = wts[spec[0].weights_of];
     KRN("residual_norm", residual_dyt(x, nullptr, nullptr, dt, 0.f, w0.norm_w, w0.norm_b, w0.norm_alpha, h, dt, nullptr, T, W, st));
@@ -629,7 +624,7 @@ class Nomanex : public Model {
       const size_t es = dtype_bytes(dt);
       auto col = [&](void* base, size_t off) { return static_cast<void*>(static_cast<uint8_t*>(base) + off * es); };
       if (s.mixer == MIX_GLA) {
-        LinearArgs la = linear_args(col(inb, s.off_a1), dt, w.a2, dt, z, DT_F32, T, s.heads * s.dim, s.a_rank);
+        LinearArgs la = linear_args(col(inb, s.off_a1), dt, w.a2, dt, z, DT_F32, T, s.heads * s.dim, s.a_rank, env.kernel_error);
         la.ldx = s.n_in;
         KRN("gla_decay_proj", linear(la, st));
         GlaArgs g;
@@ -655,7 +650,7 @@ class Nomanex : public Model {
         PromptAttnArgs pa = {};
         pa.q = p.q; pa.ldq = s.n_in; pa.q_step = s.dim + R; pa.q2 = q2; pa.kv = olat; pa.ldkv = N; pa.k_step = pa.v_step = s.dim + s.vdim; pa.v_off = s.dim; pa.k2 = k2;
         pa.y = ycat; pa.ldy = s.k_out; pa.T = T; pa.heads = pa.kv_heads = s.heads; pa.window = std::min(s.window, env.max_model_len); pa.scale = s.scale; pa.out_scale = 1.f;
-        pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = kernel_error;
+        pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = env.kernel_error;
         if (fresh && prompt_attention_fits(pa)) {
           LatentPromptPrepArgs pp = {r.cache, b.slots, b.pos, w.rope, s.rot_dims, p.half_pairs, p.q, p.ldq, c, k2, q2, T, s.heads, s.dim, R, C};
           p.q = nullptr;
@@ -691,7 +686,7 @@ class Nomanex : public Model {
       ++nl;
       const void* f_out = nullptr;
       if (s.ff_kind == FF_MOE) {
-        KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, s.experts, W), st));
+        KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, s.experts, W, env.kernel_error), st));
         KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, s.groups, s.keep, s.top, st));
         const int cap = (T * s.top + 63) / 64 * 64 + s.experts * 64;
         const bool grouped = w.tc_experts && T >= moe_tc_min && !picked_rows_pay(T * s.top, s.experts);
@@ -702,9 +697,9 @@ class Nomanex : public Model {
           const bool wide = T < 256;
           KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
           const GroupedOut up = {eact, s.ff, GROUPED_RELU2};
-          KRN("moe_up", gemm_grouped_run(w.g_eup, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+          KRN("moe_up", gemm_grouped_run(w.g_eup, w.xg_h, T, expert_rows, up, env.sms, env.kernel_error, st));
           const GroupedOut dn = {wide ? static_cast<void*>(edown) : edown16, W, wide ? GROUPED_F32 : GROUPED_PLAIN};
-          KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, kernel_error, st));
+          KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, env.kernel_error, st));
           KRN("moe_combine", moe_combine(dn.y, wide ? DT_F32 : DT_BF16, pair_pos, topw, fo, dt, T, s.top, W, st));
           nl += 4;
         } else if (T * s.top <= 64) {
@@ -748,7 +743,7 @@ class Nomanex : public Model {
     for (int r0 = 0; r0 < b.S && !rc; r0 += row_cap) {
       const int n = std::min(row_cap, b.S - r0);
       KRN("residual_norm", residual_dyt(x, nullptr, nullptr, dt, 0.f, fin_w, fin_b, fin_alpha, hrow, dt, b.rows + r0, n, W, st));
-      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W), st));
+      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
       KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
       nl += 3;
       if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),

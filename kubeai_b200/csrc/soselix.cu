@@ -112,7 +112,6 @@ class Soselix : public Model {
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
   int* gemm_counters = nullptr;
-  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   bool fuse = true;
   int few_rows = 16;
   CUtensorMap xm_h[kGemmNumBlockN];
@@ -129,7 +128,6 @@ class Soselix : public Model {
       if (w.tc_down) gemm_plan_destroy(&w.p_down);
     }
     if (pe0) { cudaEventDestroy(pe0); cudaEventDestroy(pe1); }
-    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Soselix"; }
@@ -368,8 +366,7 @@ class Soselix : public Model {
     const size_t ws_bytes = std::max(gemm_workspace_bytes(env.sms), gemm_deferred_ws_bytes(env.sms));
     if (dalloc(&gemm_ws, ws_bytes)) return -3;
     const size_t n_counters = 2ull * (maxN / 128 + 2) * (env.Tcap / 32 + 2);
-    if (dalloc(&gemm_counters, n_counters * sizeof(int)) || cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
-    *kernel_error = 0;
+    if (dalloc(&gemm_counters, n_counters * sizeof(int))) return -3;
     if (const char* e = getenv("B200_SX_FUSE")) fuse = atoi(e) != 0;              // A/B knobs
     if (const char* e = getenv("B200_SX_FEW_ROWS")) few_rows = atoi(e);
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
@@ -381,7 +378,7 @@ class Soselix : public Model {
     auto plan = [&](GemmPlan* p, const void* Wm, int N, int K) {
       if (N % 8 || K % 8 || gemm_plan_init(p, Wm, N, K, K, gemm_ws, gemm_counters, env.sms)) return false;
       p->ws_bytes = ws_bytes;
-      p->error = kernel_error;
+      p->error = env.kernel_error;
       return true;
     };
     if (!maps(xm_h, h, W)) { use_tc = false; return 0; }
@@ -636,7 +633,7 @@ class Soselix : public Model {
       PromptAttnArgs pa = {};
       pa.q = qb; pa.ldq = Q; pa.q_step = s.dim + R; pa.q2 = q2; pa.kv = olat; pa.ldkv = N; pa.k_step = pa.v_step = s.dim + s.vdim; pa.v_off = s.dim; pa.k2 = k2;
       pa.y = yb; pa.ldy = s.k_out; pa.T = T; pa.heads = pa.kv_heads = s.heads; pa.window = env.max_model_len; pa.scale = s.scale; pa.out_scale = 1.f;
-      pa.sink = w.sink; pa.gate = col(inb, s.off_g); pa.ldg = s.n_in; pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = kernel_error;
+      pa.sink = w.sink; pa.gate = col(inb, s.off_g); pa.ldg = s.n_in; pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = env.kernel_error;
       if (prompt_attention_fits(pa)) {
         KRN("latent_prompt_prep", latent_prompt_prep(pp, st));
         KRN("latent_kv", project(w.p_ukv, true, w.xm_c, c, w.w_ukv, olat, T, N, C));
@@ -717,7 +714,6 @@ class Soselix : public Model {
     const int T = b.T;
     int rc = 0;
     int64_t nl = 0;
-    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Soselix forward: a wait inside a projection ran out"); return -2; }
     KRN("embed", embed_scaled(embed, dt, b.ids, x, T, W, V, embed_scale, 1, 0, st));
     Pending pend;
     for (size_t li = 0; li < spec.size() && !rc; ++li) {
@@ -754,7 +750,7 @@ class Soselix : public Model {
     for (int r0 = 0; r0 < b.S && !rc; r0 += row_cap) {
       const int n = std::min(row_cap, b.S - r0);
       KRN("residual_norm", sandwich_step(boundary(Pending(), fin_w, hrow, b.rows + r0, n), st));
-      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W), st));
+      KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
       KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
       if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
                                          cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -2;

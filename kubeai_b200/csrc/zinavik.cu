@@ -125,7 +125,6 @@ class Zinavik : public Model {
   int row_cap = 0, moe_cap = 0;
   void *hsorted = nullptr, *edown16 = nullptr;
   int* expert_rows = nullptr;
-  int* kernel_error = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
   int moe_tc_min = 256;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
@@ -141,7 +140,6 @@ class Zinavik : public Model {
       if (w.tc_shin) gemm_plan_destroy(&w.p_shin);
       if (w.tc_shdown) gemm_plan_destroy(&w.p_shdown);
     }
-    if (kernel_error) cudaFreeHost(kernel_error);
     for (void* p : allocs) cudaFree(p);
   }
   const char* arch() const override { return "Zinavik"; }
@@ -412,25 +410,23 @@ class Zinavik : public Model {
       if (dalloc(&hsorted, static_cast<size_t>(moe_cap) * W * 2) || dalloc(&edown16, static_cast<size_t>(moe_cap) * W * 2) ||
           dalloc(&expert_rows, static_cast<size_t>(max_e) * 2 * sizeof(int))) return -3;
     }
-    if (cudaMallocHost(&kernel_error, sizeof(int)) != cudaSuccess) return -3;
-    *kernel_error = 0;
     if (const char* e = getenv("B200_ZV_MOE_TC_MIN_T")) moe_tc_min = atoi(e);   // A/B knob: the fewest tokens that take the grouped GEMM
     for (size_t i = 0; i < spec.size(); ++i) {
       const LayerSpec& s = spec[i];
       LayerWeights& w = wts[i];
       w.tc_in = gemm_plan_init(&w.p_in, w.w_in, s.n_in, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = kernel_error; }
+      if (w.tc_in) { w.p_in.ws_bytes = ws_bytes; w.p_in.error = env.kernel_error; }
       w.tc_out = s.k_out % 8 == 0 && gemm_plan_init(&w.p_out, w.w_out, W, s.k_out, s.k_out, gemm_ws, gemm_counters, env.sms) == 0;
       for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
         if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
-      if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = kernel_error; }
+      if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = env.kernel_error; }
       if (s.mlp && s.shared) {
         w.tc_shin = gemm_plan_init(&w.p_shin, w.sh_in, s.n_sh, W, W, gemm_ws, gemm_counters, env.sms) == 0;
-        if (w.tc_shin) { w.p_shin.ws_bytes = ws_bytes; w.p_shin.error = kernel_error; }
+        if (w.tc_shin) { w.p_shin.ws_bytes = ws_bytes; w.p_shin.error = env.kernel_error; }
         w.tc_shdown = s.sff % 8 == 0 && gemm_plan_init(&w.p_shdown, w.sh_down, W, s.sff, s.sff, gemm_ws, gemm_counters, env.sms) == 0;
         for (int j = 0; j < kGemmNumBlockN && w.tc_shdown; ++j)
           if (gemm_make_x_map(&w.xm_shact[j], shact, env.Tcap, s.sff, s.sff, bns[j])) w.tc_shdown = false;
-        if (w.tc_shdown) { w.p_shdown.ws_bytes = ws_bytes; w.p_shdown.error = kernel_error; }
+        if (w.tc_shdown) { w.p_shdown.ws_bytes = ws_bytes; w.p_shdown.error = env.kernel_error; }
       }
       if (s.mlp) {
         w.tc_experts = !gemm_grouped_plan(&w.g_egu, w.e_gu, s.experts, 2 * s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
@@ -619,7 +615,7 @@ class Zinavik : public Model {
     cudaStream_t st = env.stream;
     int rc = 0;
     const int nr = s.experts + (s.shared ? 1 : 0);   // router logits and, behind them, the shared expert's gate logit
-    KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, nr, W), st));
+    KRN("moe_router", linear(linear_args(h, dt, w.router, dt, scores, DT_F32, T, nr, W, env.kernel_error), st));
     KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, 1, 1, s.top, st, MOE_SIGMOID, nr));
     const void* shared_out = nullptr;
     const float* shared_gate = nullptr;
@@ -655,14 +651,14 @@ class Zinavik : public Model {
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st, sorted_w));
       if (w.il_e) {
         const GroupedOut up = {eact, s.ff, GROUPED_GATED, nullptr, s.limit, 1.702f, 1.0f};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, env.kernel_error, st));
       } else {
         const GroupedOut up = {egu, 2 * s.ff};
-        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, kernel_error, st));
+        KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, up, env.sms, env.kernel_error, st));
         KRN("glu", glu_clamped(egu, 2 * s.ff, eact, s.ff, dt, cap, s.ff, s.limit, 1.702f, st));
       }
       const GroupedOut dn = {edown16, W};
-      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, kernel_error, st));
+      KRN("moe_down", gemm_grouped_run(w.g_edown, w.xg_act, T, expert_rows, dn, env.sms, env.kernel_error, st));
       KRN("moe_combine", moe_combine_add(edown16, DT_BF16, pair_pos, nullptr, shared_out, shared_gate, nr, fo, dt, T, s.top, W, st));
       return rc;
     }
@@ -687,7 +683,6 @@ class Zinavik : public Model {
     int64_t nl = 0;
     const size_t es = dtype_bytes(dt);
     auto col = [&](void* base, size_t off) { return static_cast<void*>(static_cast<uint8_t*>(base) + off * es); };
-    if (kernel_error && *static_cast<volatile int*>(kernel_error)) { set_error("Zinavik forward: a wait inside the grouped GEMM ran out"); return -2; }
     KRN("embed", embed_scaled(embed, dt, b.ids, x, T, W, V, emb_scale, ns, xstride, st));
     Pending pend;
     for (size_t ri = 0; ri < run.size() && !rc; ++ri) {
@@ -745,7 +740,7 @@ class Zinavik : public Model {
     for (int r0 = 0; r0 < b.S && !rc; r0 += row_cap) {
       const int n = std::min(row_cap, b.S - r0);
       KRN("stream_norm", hyper_step(boundary(Pending(), nullptr, fin_w, hrow, dt, b.rows + r0, n), st));
-      KRN("head", linear(linear_args(hrow, dt, embed, dt, logits, DT_F32, n, V, W), st));
+      KRN("head", linear(linear_args(hrow, dt, embed, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
       KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
       if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
                                          cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -2;

@@ -129,7 +129,7 @@ struct SplitK {
 };
 __device__ __forceinline__ float gated_unit(float g, float u, bool clamp, const GroupedOut& o) {
   if (clamp) { g = fminf(g, o.p0); u = fminf(fmaxf(u, -o.p0), o.p0); }
-  return __fdividef(g, 1.0f + __expf(-o.p1 * g)) * (u + o.p2);
+  return g * (1.0f / (1.0f + expf(-(o.p1 * g)))) * (u + o.p2);     // accurate functions, as norm_act.cu's glu_clamped
 }
 // EPI 5: SiLU rounded to bf16 before the product, the rounding points of the Llama path's own kernel (elementwise.cu silu_mul)
 template <int EPI>

@@ -67,3 +67,27 @@ def test_experts_agree_with_the_tile_kernel(tmp_path, monkeypatch, ff, shared, T
     # to a tie may take another expert
     assert np.median(rel_err(new, want)) < 0.03 and np.median(rel_err(new, old.astype(np.float64))) < 0.02
     assert np.median(rel_err(new, want)) < 1.3 * np.median(rel_err(old, want)) + 1e-3
+
+
+def picks(rng, rows, cols):
+    """One power of two per row: every product with it is exact, whatever the order of the sum."""
+    m = np.zeros((rows, cols), dtype=np.float32)
+    m[np.arange(rows), rng.integers(0, cols, rows)] = 2.0 ** rng.integers(-1, 4, rows) * rng.choice([-1.0, 1.0], rows)
+    return m
+
+
+@pytest.mark.parametrize("T", [40, 250])
+def test_gated_unit_in_the_epilogue_is_the_one_of_its_own_kernel(tmp_path, monkeypatch, T):
+    """Same accurate exponential and quotient: where the sums are exact, so are the two forms equal, bit for bit."""
+    cfg = make_config([layer(attention(heads=2, kv_heads=1, dim=16, vdim=16), mlp=moe(experts=4, top=2, ff=512, shared=None))], width=512)
+    W, rng = random_weights(cfg, seed=6), np.random.default_rng(7)
+    for e in range(4):
+        W["l0.mlp.e%d.gate" % e], W["l0.mlp.e%d.up" % e], W["l0.mlp.e%d.down" % e] = (picks(rng, 512, 512) for _ in range(3))
+    d = write_model_dir(tmp_path / "m", cfg, W)
+    t = rng.integers(0, cfg["vocab"], T).tolist()
+    out = []
+    for least in ("1", "100000"):            # tokens from which the experts take the grouped product
+        monkeypatch.setenv("B200_MX_MOE_TC_MIN_T", least)
+        with open_engine(d, dtype="bfloat16") as e:
+            out.append(feed_whole(e, t))
+    np.testing.assert_array_equal(out[0], out[1])

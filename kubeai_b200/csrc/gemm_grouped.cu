@@ -136,6 +136,7 @@ template <int EPI>
 __device__ __forceinline__ float gated(float g, float u, bool clamp, const GroupedOut& o) {
   return EPI == 5 ? __bfloat162float(silu_bf16(g)) * u : gated_unit(g, u, clamp, o);
 }
+__device__ __forceinline__ float left_over(float s) { return s - __bfloat162float(__float2bfloat16_rn(s)); }
 // Eight neighbouring columns of one row: the parts' sums added in their order.
 __device__ __forceinline__ void add_parts(float* v, const float* p, int step, int parts) {
 #pragma unroll
@@ -188,6 +189,11 @@ __device__ __forceinline__ void finish_rows(const float* sums, int step, int par
         if (EPI == 4) v[i] = xielu_fast(v[i], o.p0, o.p1);
       }
       store8(static_cast<bf16*>(o.y) + r * o.ldy + n0 + c, v);
+      if (EPI == 6 && (n0 & kSlab)) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = left_over(v[i]);
+        store8(static_cast<bf16*>(o.y2) + r * (N / 2) + (n0 - kSlab) / 2 + c, v);
+      }
     }
   }
 }
@@ -211,7 +217,7 @@ __device__ __forceinline__ void finish_parts(float* ring, const float* first, si
 }
 
 // EPI 0: bf16(sum); 1: the gated unit; 2: fp32 sum + bias; 3: bf16(relu2(sum + bias)), or without an activation; 4: bf16(xielu(sum + bias));
-// 5: the SiLU-gated unit with its inner rounding.
+// 5: the SiLU-gated unit with its inner rounding; 6: bf16(sum), and of the pair's second slab what that rounding left.
 // A form of its own for the plain product: looking the activation up per element made its drain a sixth of the launch longer.
 // FULL: 128-row boxes, their sizes known to the compiler.
 template <int EPI, bool FULL>
@@ -434,6 +440,23 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             if (j < left && n0 + c < N)
               *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * o.ldy + n0 + c) = *reinterpret_cast<const uint4*>(sb + j * kSlab + c);
           }
+          if (EPI == 6 && rank == 1) {      // one more round for the second terms
+            sbuf ^= 1;
+            bf16* s2 = reinterpret_cast<bf16*>(stage_out + sbuf * kOutBytes);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) s2[j * kSlab + row] = __float2bfloat16_rn(left_over(__uint_as_float(v0[j])));
+            if (two) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) s2[(32 + j) * kSlab + row] = __float2bfloat16_rn(left_over(__uint_as_float(v1[j])));
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            bf16* d2 = static_cast<bf16*>(o.y2) + static_cast<size_t>(t.row0 + c0) * (N / 2) + t.n0 / 2;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int it = et + i * 128, j = it >> 4, c = (it & 15) * 8;
+              if (j < left) *reinterpret_cast<uint4*>(d2 + static_cast<size_t>(j) * (N / 2) + c) = *reinterpret_cast<const uint4*>(s2 + j * kSlab + c);
+            }
+          }
         }
         sbuf ^= 1;
       }
@@ -475,14 +498,15 @@ int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap
            const SplitK& split, int units, int* error, cudaStream_t st) {
   const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED || o.epi == GROUPED_SILU;
   if ((!expert_rows && (experts != 1 || rows < 1)) || !o.y || o.ldy % (f32 ? 4 : 8) || N % (f32 ? 4 : 8) || reinterpret_cast<uintptr_t>(o.y) % 16 || units < 1 ||
-      (gated && (N % kSlab || o.bias)) || (o.bias && experts != 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
-  static std::atomic<unsigned long long> attr[12];
+      (gated && (N % kSlab || o.bias)) || (o.epi == GROUPED_TWO_TERMS && (N % (2 * kSlab) || o.bias || !o.y2 || reinterpret_cast<uintptr_t>(o.y2) % 16)) || (o.bias && experts != 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
+  static std::atomic<unsigned long long> attr[14];
   auto start = [&](auto kernel, int i) {
     if (!ensure_dynamic_smem(kernel, kSmem, &attr[i])) return -2;
     return launch_pdl(kernel, dim3(2 * units), dim3(kThreads), kSmem, st, tm_w, tm_x, expert_rows, experts, rows, o, N, K, box, split, error) == cudaSuccess ? 0 : -2;
   };
 #define RUN(E) return box == 128 ? start(gemm_grouped_kernel<E, true>, 2 * E) : start(gemm_grouped_kernel<E, false>, 2 * E + 1)
   if (o.epi == GROUPED_SILU) RUN(5);
+  if (o.epi == GROUPED_TWO_TERMS) RUN(6);
   if (gated) RUN(1);
   if (f32) RUN(2);
   if (o.epi == GROUPED_XIELU) RUN(4);

@@ -268,13 +268,14 @@ int latent_attention(const LatentAttnArgs& a, cudaStream_t st);
 // For steps whose sequences all start at their first token (StepBatch::fresh), bf16: keys and values are the step's own rows.
 // q [T, ldq]: head h's 128 columns at h * q_step; kv [T, ldkv]: key head g's columns at k_off + g * k_step and its values at
 // v_off + g * v_step (128 each; query heads share key heads in equal groups).  q2 [T, heads * 64] with k2 [T, 64] (optional):
-// 64 more dimensions per head against a key part all heads share.  score = q . k * scale, then softcap * tanh(score /
+// 64 more dimensions per head against a key part all heads share, and then v2 [T, heads * 128]: second terms of the values, which
+// are the sum of both (every head has its own key head).  score = q . k * scale, then softcap * tanh(score /
 // softcap) where softcap > 0; key j is visible from position p when max(0, p - window + 1) <= j <= p.  sink (optional, fp32
 // [heads]) joins the denominator as exp(sink); y [T, ldy]: head h's 128 columns = sum * out_scale * sigmoid(gate[t, h])
 // (gate optional, bf16, leading dimension ldg).  error (optional, host-visible): set to 1 when a wait ran out.
 struct PromptAttnArgs {
   const void* q; int ldq, q_step; const void* q2;
-  const void* kv; int ldkv, k_off, k_step, v_off, v_step; const void* k2;
+  const void* kv; int ldkv, k_off, k_step, v_off, v_step; const void *k2, *v2;
   void* y; int ldy;
   int T, heads, kv_heads, window; float scale, softcap, out_scale;
   const float* sink; const void* gate; int ldg;
@@ -286,7 +287,7 @@ int prompt_attention(const PromptAttnArgs& a, cudaStream_t st);
 // Latent attention this way: per token the cached latent -> c [T, kv_rank], the cached rotated key part -> k2 [T, rot_dim] and
 // the rotated part of every query head (q as for LatentPrepArgs) -> q2 [T, heads * rot_dim]; the per-head keys and values are
 // then c times the stacked matrix [heads][128 rows of W_uk, 128 rows of W_uv][kv_rank] that latent_prompt_stack makes from
-// uk_t [heads][kv_rank][128] and uv [heads][128][kv_rank].
+// uk_t [heads][kv_rank][128] and uv [heads][128][kv_rank] (GROUPED_TWO_TERMS: the values' second terms apart).
 struct LatentPromptPrepArgs {
   const void* cache; const int* slots; const int* positions; const float2* rope; int rot_dims; bool half_pairs;
   const void* q; int ldq; void *c, *k2, *q2;

@@ -645,18 +645,20 @@ class Nomanex : public Model {
         p.T = T; p.heads = s.heads; p.dim = s.dim; p.rot_dim = R; p.kv_rank = C;
         const bool fresh = b.fresh && w.tc_ukv && latent_prompt_pays(T, b.nseq);
         // whole prompts: per-head keys and values once per token, in the buffers of the latent form
-        bf16 *c = reinterpret_cast<bf16*>(qlat), *k2 = c + static_cast<size_t>(env.Tcap) * C, *q2 = k2 + static_cast<size_t>(env.Tcap) * R;
-        const int N = s.heads * (s.dim + s.vdim);
+        bf16 *c = reinterpret_cast<bf16*>(qlat), *k2 = c + static_cast<size_t>(env.Tcap) * C, *q2 = k2 + static_cast<size_t>(env.Tcap) * R, *v2 = q2 + static_cast<size_t>(env.Tcap) * s.heads * R;
+        const int N = s.heads * (s.dim + s.vdim), bn = gemm_block_n_for(T);
+        GroupedOut kv = {olat, N, GROUPED_TWO_TERMS};
+        kv.y2 = v2;
         PromptAttnArgs pa = {};
-        pa.q = p.q; pa.ldq = s.n_in; pa.q_step = s.dim + R; pa.q2 = q2; pa.kv = olat; pa.ldkv = N; pa.k_step = pa.v_step = s.dim + s.vdim; pa.v_off = s.dim; pa.k2 = k2;
+        pa.q = p.q; pa.ldq = s.n_in; pa.q_step = s.dim + R; pa.q2 = q2; pa.kv = olat; pa.ldkv = N; pa.k_step = pa.v_step = s.dim + s.vdim; pa.v_off = s.dim; pa.k2 = k2; pa.v2 = v2;
         pa.y = ycat; pa.ldy = s.k_out; pa.T = T; pa.heads = pa.kv_heads = s.heads; pa.window = std::min(s.window, env.max_model_len); pa.scale = s.scale; pa.out_scale = 1.f;
         pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = env.kernel_error;
-        if (fresh && prompt_attention_fits(pa)) {
+        if (fresh && prompt_attention_fits(pa) && gemm_whole_fits(w.p_ukv, olat, N)) {
           LatentPromptPrepArgs pp = {r.cache, b.slots, b.pos, w.rope, s.rot_dims, p.half_pairs, p.q, p.ldq, c, k2, q2, T, s.heads, s.dim, R, C};
           p.q = nullptr;
           KRN("latent_prep", latent_prep(p, st));
           KRN("latent_prompt_prep", latent_prompt_prep(pp, st));
-          KRN("latent_kv", project(w.p_ukv, true, w.xm_c, c, w.ukv, olat, T, N, C));
+          KRN("latent_kv", gemm_whole_run(w.p_ukv, w.xm_c[gemm_block_n_index(bn)], bn, T, kv, st));
           KRN("latent_attention", prompt_attention(pa, st));
         } else {
           KRN("latent_prep", latent_prep(p, st));

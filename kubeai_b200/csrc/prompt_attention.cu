@@ -1,8 +1,9 @@
 // Softmax attention of whole prompts on the 5th-generation tensor cores (mixers.h PromptAttnArgs): every sequence of the step
 // starts at its first token, so its keys and values are the step's own rows and lie densely in memory.  Causal, with an
 // optional window, sink, cap and per-head gate; 128 dimensions a head, or 128 of its own and 64 more against a key part that
-// all heads share (latent attention, whose per-head keys and values one product rebuilds from the latents: that and 192 + 128
-// dimensions a pair are a third of the work of scores and sums in 576 + 512 latent dimensions).
+// all heads share (latent attention, whose per-head keys and values one product rebuilds from the latents: that and 192 + 256
+// dimensions a pair are 0.4 of the work of scores and sums in 576 + 512 latent dimensions).  There a value is two bf16 terms, the
+// rounded sum and what the rounding left: the absorbed form it stands for keeps the weighted latents in fp32 up to W_uv.
 //
 // A CTA owns 256 query tokens of one head as two 128-row tiles that share every 64-key tile.  One thread loads (TMA, 128-byte
 // swizzle, keys and values in rings of their own), one issues every tcgen05.mma:
@@ -43,7 +44,8 @@ constexpr int kVTile = 2 * kKSlab, kPTile = kRows * 128;
 constexpr int kThreads = 320;                        // warp 0: loads, warps 1-4 and 5-8: rows of tile 0 and 1, warp 9: products
 constexpr int kWaitLimit = 1 << 22;
 template <int NS>
-constexpr int smem_bytes() { return 1024 + 2 * NS * kQSlab + 2 * NS * kKSlab + 2 * kVTile + 2 * kPTile + 256; }
+constexpr int smem_bytes() { return 1024 + 2 * NS * kQSlab + 2 * NS * kKSlab + 2 * kVTile + 2 * kPTile + (NS == 3 ? kVTile : 0) + 256; }
+static_assert(smem_bytes<3>() <= 227 * 1024, "one buffer of the values' second terms is what fits");
 
 __device__ __forceinline__ uint32_t idesc_bf16(uint32_t m, uint32_t n, uint32_t b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
@@ -65,11 +67,12 @@ __device__ __forceinline__ float exp2_ftz(float x) {
   return y;
 }
 
-// NS: 64-column slabs of a query or key row (2, or 3 with the shared part)
+// NS: 64-column slabs of a query or key row (2, or 3 with the shared part and values in two terms)
 template <int NS, bool CAP>
 __global__ void __launch_bounds__(kThreads, 1)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_q2, const __grid_constant__ CUtensorMap tm_kv,
-                   const __grid_constant__ CUtensorMap tm_k2, const __grid_constant__ PromptAttnArgs a) {
+                   const __grid_constant__ CUtensorMap tm_k2, const __grid_constant__ CUtensorMap tm_v2, const __grid_constant__ PromptAttnArgs a) {
+  constexpr bool LO = NS == 3;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (sbase - smem_u32(smem_raw));
@@ -77,7 +80,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const uint32_t k_s = q_s + 2 * NS * kQSlab;               // [stage][slab]
   const uint32_t v_s = k_s + 2 * NS * kKSlab;               // [stage][half]
   const uint32_t p_s = v_s + 2 * kVTile;                    // [tile]
-  const uint32_t bars = p_s + 2 * kPTile;
+  const uint32_t v2_s = p_s + 2 * kPTile;                   // the values' second terms, one tile
+  const uint32_t bars = v2_s + (LO ? kVTile : 0);
   auto k_full = [&](int s) { return bars + 8u * s; };
   auto k_empty = [&](int s) { return bars + 8u * (2 + s); };
   auto v_full = [&](int s) { return bars + 8u * (4 + s); };
@@ -85,14 +89,14 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   auto s_full = [&](int i, int b) { return bars + 8u * (8 + 2 * i + b); };
   auto p_ready = [&](int i) { return bars + 8u * (12 + i); };     // 4 warps: P_i written, S_i read, O_i rescaled
   auto pv_full = [&](int i) { return bars + 8u * (14 + i); };
-  const uint32_t q_bar = bars + 8u * 16, tmem_slot = bars + 8u * 17;
+  const uint32_t q_bar = bars + 8u * 16, v2_full = bars + 8u * 17, v2_empty = bars + 8u * 18, tmem_slot = bars + 8u * 19;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (warp == 0) {
     if (lane == 0) {
       for (int s = 0; s < 2; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(s_full(i, 0), 1); mbar_init(s_full(i, 1), 1); mbar_init(p_ready(i), 4); mbar_init(pv_full(i), 1); }
-      mbar_init(q_bar, 1);
+      mbar_init(q_bar, 1); mbar_init(v2_full, 1); mbar_init(v2_empty, 1);
       fence_mbar_init();
     }
     __syncwarp();
@@ -149,22 +153,38 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int i = 0; i < tiles; ++i)
           for (int s = 0; s < NS; ++s)
             tma_load_2d(q_s + (i * NS + s) * kQSlab, s < 2 ? &tm_q : &tm_q2, q_bar, s < 2 ? head * a.q_step + 64 * s : head * 64, tok0 + q0 + i * kRows, kEvictNormal);
-        int it = 0;
-        for (int t = t_begin; ok && t < t_end; ++t, ++it) {
-          const int st = it & 1;
-          const uint32_t ph = (it >> 1) & 1;
-          const int row = tok0 + t * kKeys;
-          if (!(ok = wait_limited(k_empty(st), ph ^ 1u))) break;
+        int nk = 0, nv = 0, nl = 0;      // tiles of keys, values and second terms on their way
+        auto keys = [&] {
+          const int st = nk & 1;
+          if (!wait_limited(k_empty(st), ((nk >> 1) & 1) ^ 1u)) return false;
           mbar_arrive_expect_tx(k_full(st), NS * kKSlab);
           for (int s = 0; s < NS; ++s)
-            tma_load_2d(k_s + (st * NS + s) * kKSlab, s < 2 ? &tm_kv : &tm_k2, k_full(st), s < 2 ? a.k_off + kvh * a.k_step + 64 * s : 0, row, kEvictLast);
-          if (!(ok = wait_limited(v_empty(st), ph ^ 1u))) { ++it; break; }
+            tma_load_2d(k_s + (st * NS + s) * kKSlab, s < 2 ? &tm_kv : &tm_k2, k_full(st), s < 2 ? a.k_off + kvh * a.k_step + 64 * s : 0, tok0 + (t_begin + nk) * kKeys,
+                        kEvictLast);
+          ++nk;
+          return true;
+        };
+        if (LO) ok = keys();
+        for (int t = t_begin; ok && t < t_end; ++t) {
+          // with one buffer of second terms that wait is the long one: the next keys go ahead of it
+          if ((!LO || t + 1 < t_end) && !(ok = keys())) break;
+          const int st = nv & 1, row = tok0 + t * kKeys;
+          if (!(ok = wait_limited(v_empty(st), ((nv >> 1) & 1) ^ 1u))) break;
           mbar_arrive_expect_tx(v_full(st), kVTile);
           for (int s = 0; s < 2; ++s) tma_load_2d(v_s + st * kVTile + s * kKSlab, &tm_kv, v_full(st), a.v_off + kvh * a.v_step + 64 * s, row, kEvictLast);
+          ++nv;
+          if constexpr (LO) {
+            if (!(ok = wait_limited(v2_empty, (nl & 1) ^ 1u))) break;
+            mbar_arrive_expect_tx(v2_full, kVTile);
+            for (int s = 0; s < 2; ++s) tma_load_2d(v2_s + s * kKSlab, &tm_v2, v2_full, head * kD + 64 * s, row, kEvictLast);
+            ++nl;
+          }
         }
         // the copies in flight land before the CTA ends, also where it gives up
         wait_limited(q_bar, 0);
-        for (int j = max(0, it - 2); j < it; ++j) { wait_limited(k_full(j & 1), (j >> 1) & 1); wait_limited(v_full(j & 1), (j >> 1) & 1); }
+        for (int j = max(0, nk - 2); j < nk; ++j) wait_limited(k_full(j & 1), (j >> 1) & 1);
+        for (int j = max(0, nv - 2); j < nv; ++j) wait_limited(v_full(j & 1), (j >> 1) & 1);
+        if (nl > 0) wait_limited(v2_full, (nl - 1) & 1);
       }
     } else if (warp == 9) {
       if (lane == 0) {
@@ -202,9 +222,17 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int k = 0; k < kKeys / 16; ++k)
               umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v_s + st * kVTile + k * 2048, kKSlab, 1024), id_o,
                         (t > first[i] || k > 0) ? 1u : 0u);
+            if constexpr (LO) {
+              if (!(ok = wait_limited(v2_full, it & 1))) break;
+              tc_fence_after();
+#pragma unroll
+              for (int k = 0; k < kKeys / 16; ++k)
+                umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v2_s + k * 2048, kKSlab, 1024), id_o, 1u);
+            }
             umma_commit(pv_full(i));
           }
           umma_commit(v_empty(st));
+          if constexpr (LO) umma_commit(v2_empty);
         }
       }
     } else {
@@ -289,12 +317,16 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (kv0 + kKeys > n && (gi == 0 || !active(0, t))) {
           // values behind the sequence's end: cleared before the first product that reads the tile (that of row tile 0, where it is active)
           const int it = t - t_begin;
-          if (!__all_sync(0xffffffffu, wait_limited(v_full(it & 1), (it >> 1) & 1))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, wait_limited(v_full(it & 1), (it >> 1) & 1) && (!LO || wait_limited(v2_full, it & 1)))) { ok = false; break; }
           const int r = row & 63;
           if (kv0 + r >= n) {
             uint4* d = reinterpret_cast<uint4*>(smem + (v_s - sbase) + (it & 1) * kVTile + (row >> 6) * kKSlab + r * 128);
+            uint4* d2 = reinterpret_cast<uint4*>(smem + (v2_s - sbase) + (row >> 6) * kKSlab + r * 128);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) d[c] = make_uint4(0, 0, 0, 0);
+            for (int c = 0; c < 8; ++c) {
+              d[c] = make_uint4(0, 0, 0, 0);
+              if (LO) d2[c] = make_uint4(0, 0, 0, 0);
+            }
           }
         }
         fence_proxy_async();
@@ -341,11 +373,11 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 }
 
 template <int NS, bool CAP>
-int launch(const PromptAttnArgs& a, const CUtensorMap& q, const CUtensorMap& q2, const CUtensorMap& kv, const CUtensorMap& k2, cudaStream_t st) {
+int launch(const PromptAttnArgs& a, const CUtensorMap& q, const CUtensorMap& q2, const CUtensorMap& kv, const CUtensorMap& k2, const CUtensorMap& v2, cudaStream_t st) {
   static std::atomic<unsigned long long> attr{0};
   constexpr int smem = smem_bytes<NS>();
   if (!ensure_dynamic_smem(prompt_attn_kernel<NS, CAP>, smem, &attr)) return -2;
-  prompt_attn_kernel<NS, CAP><<<dim3(a.heads, a.T / (2 * kRows) + a.nseq), kThreads, smem, st>>>(q, q2, kv, k2, a);
+  prompt_attn_kernel<NS, CAP><<<dim3(a.heads, a.T / (2 * kRows) + a.nseq), kThreads, smem, st>>>(q, q2, kv, k2, v2, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -402,20 +434,21 @@ __global__ void latent_stack_kernel(const bf16* uk_t, const bf16* uv, bf16* out,
 bool prompt_attention_fits(const PromptAttnArgs& a) {
   auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   return gemm_variant() == 2 && a.heads > 0 && a.kv_heads > 0 && a.heads % a.kv_heads == 0 && a.ldq % 8 == 0 && a.q_step % 8 == 0 && a.ldkv % 8 == 0 && a.k_off % 8 == 0 &&
-         a.k_step % 8 == 0 && a.v_off % 8 == 0 && a.v_step % 8 == 0 && a.ldy % 8 == 0 && al(a.q) && al(a.q2) && al(a.kv) && al(a.k2) && al(a.y) && !a.q2 == !a.k2 &&
+         a.k_step % 8 == 0 && a.v_off % 8 == 0 && a.v_step % 8 == 0 && a.ldy % 8 == 0 && al(a.q) && al(a.q2) && al(a.kv) && al(a.k2) && al(a.v2) && al(a.y) && !a.q2 == !a.k2 && !a.q2 == !a.v2 && (!a.v2 || a.kv_heads == a.heads) &&
          a.window > 0 && a.softcap >= 0.f && a.scale > 0.f;
 }
 
 int prompt_attention(const PromptAttnArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.nseq <= 0) return 0;
   if (!prompt_attention_fits(a)) return -1;
-  CUtensorMap q, q2, kv, k2;
+  CUtensorMap q, q2, kv, k2, v2;
   const int kcols = a.k_off + (a.kv_heads - 1) * a.k_step + kD, vcols = a.v_off + (a.kv_heads - 1) * a.v_step + kD;
   if (tmap_encode_bf16_2d(&q, a.q, a.T, (a.heads - 1) * a.q_step + kD, a.ldq, kRows, 64, 1) ||
       tmap_encode_bf16_2d(&kv, a.kv, a.T, kcols > vcols ? kcols : vcols, a.ldkv, kKeys, 64, 1)) return -2;
-  if (!a.q2) return a.softcap > 0.f ? launch<2, true>(a, q, q, kv, kv, st) : launch<2, false>(a, q, q, kv, kv, st);
-  if (tmap_encode_bf16_2d(&q2, a.q2, a.T, a.heads * 64, a.heads * 64, kRows, 64, 1) || tmap_encode_bf16_2d(&k2, a.k2, a.T, 64, 64, kKeys, 64, 1)) return -2;
-  return a.softcap > 0.f ? launch<3, true>(a, q, q2, kv, k2, st) : launch<3, false>(a, q, q2, kv, k2, st);
+  if (!a.q2) return a.softcap > 0.f ? launch<2, true>(a, q, q, kv, kv, kv, st) : launch<2, false>(a, q, q, kv, kv, kv, st);
+  if (tmap_encode_bf16_2d(&q2, a.q2, a.T, a.heads * 64, a.heads * 64, kRows, 64, 1) || tmap_encode_bf16_2d(&k2, a.k2, a.T, 64, 64, kKeys, 64, 1) ||
+      tmap_encode_bf16_2d(&v2, a.v2, a.T, a.heads * kD, a.heads * kD, kKeys, 64, 1)) return -2;
+  return a.softcap > 0.f ? launch<3, true>(a, q, q2, kv, k2, v2, st) : launch<3, false>(a, q, q2, kv, k2, v2, st);
 }
 
 int latent_prompt_prep(const LatentPromptPrepArgs& a, cudaStream_t st) {

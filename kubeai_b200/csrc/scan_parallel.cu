@@ -286,6 +286,7 @@ __device__ __forceinline__ void mma6(float* c, const uint32_t (*A)[4], const uin
   mma(c, A[0], B[1][0], B[1][1]);
   mma(c, A[0], B[0][0], B[0][1]);
 }
+__device__ __forceinline__ bool finite2(uint32_t x) { return (x & 0x7f80u) != 0x7f80u && (x & 0x7f800000u) != 0x7f800000u; }
 __device__ __forceinline__ float2 mul2(float2 x, float2 y) { return make_float2(x.x * y.x, x.y * y.y); }
 
 // grid (chunks, heads, column blocks).  Warp w: tokens of block w / 2, value columns of half w % 2.
@@ -487,7 +488,32 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
         const int t = g + 8 * (e >> 1), j = nt * 8 + 2 * t4 + (e & 1);
         d[nt][e] = sm.diag[2 * b][t][j] + sm.diag[2 * b + 1][t][j];
       }
-    values(d, b);
+    // A token's weight for the block's later keys is 0, which a product would turn into NaN where their value is infinite or NaN:
+    // such a block is summed key by key, up to the token.
+    bool finite = true;
+#pragma unroll
+    for (int e = 0; e < kB * 8; e += 32) {
+      const uint4 v = *reinterpret_cast<const uint4*>(sm.V + (b * kB + (e + lane) / 8) * kLd + half * 64 + (e + lane) % 8 * 8);
+      finite = finite && finite2(v.x) && finite2(v.y) && finite2(v.z) && finite2(v.w);
+    }
+    if (__all_sync(0xffffffffu, finite)) {
+      values(d, b);
+    } else {
+      if (NRM) {
+        nq[0] += (d[0][0] + d[0][1]) + (d[1][0] + d[1][1]);
+        nq[1] += (d[0][2] + d[0][3]) + (d[1][2] + d[1][3]);
+      }
+      for (int r = 0; r < 2; ++r)
+        for (int j = 0; j <= g + 8 * r; ++j) {
+          const float w = sm.diag[2 * b][g + 8 * r][j] + sm.diag[2 * b + 1][g + 8 * r][j];
+          const bf16* v = sm.V + (b * kB + j) * kLd + half * 64 + 2 * t4;
+#pragma unroll
+          for (int nt = 0; nt < 8; ++nt) {
+            if (r == 0) { o[nt][0] = fmaf(w, __bfloat162float(v[nt * 8]), o[nt][0]); o[nt][1] = fmaf(w, __bfloat162float(v[nt * 8 + 1]), o[nt][1]); }
+            else { o[nt][2] = fmaf(w, __bfloat162float(v[nt * 8]), o[nt][2]); o[nt][3] = fmaf(w, __bfloat162float(v[nt * 8 + 1]), o[nt][3]); }
+          }
+        }
+    }
   }
   // ---- the incoming state's part
   if (has_state) {

@@ -85,3 +85,26 @@ def test_unequal_sequences_in_one_step_and_their_states(tmp_path, monkeypatch):
             out[knob] = np.concatenate([a, b])
     r = nx.rel_err(out["1"], out["0"].astype(np.float64))
     assert np.median(r) < 2e-3 and r.max() < 2e-2, (np.median(r), r.max())
+
+
+@pytest.mark.parametrize("family", ["hgrn2", "mlstm"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [1, 15, 16, 40, 63, 64, 70])
+def test_tokens_in_front_of_one_without_finite_numbers(tmp_path, family, bad, at):
+    """A token whose values are not finite, in every place of a block and a chunk: what came before it does not depend on it."""
+    if family == "hgrn2":
+        cfg = sx.make_config([sx.hgrn2(heads=2, dim=48, vdim=72, mlp=None)], width=32)
+        W = sx.random_weights(cfg, seed=4)
+    else:
+        cfg = mx.make_config([mx.layer(mx.mlstm(heads=2, dim=48, vdim=72), mlp=None)], width=32)
+        W = mx.random_weights(cfg, seed=4)
+    W["embed"] = W["embed"].copy()
+    t = np.random.default_rng(at).integers(1, cfg["vocab"], 90)
+    t[at] = 0
+    out = []
+    for row in (W["embed"][1].copy(), np.full(32, bad, dtype=np.float32)):
+        W["embed"][0] = row
+        with sx.open_engine(sx.write_model_dir(tmp_path / ("m%d" % len(out)), cfg, W), dtype="bfloat16") as e:
+            out.append(nx.feed_whole(e, t.tolist()))
+    assert np.isfinite(out[0]).all() and not np.isfinite(out[1][at:]).all()
+    np.testing.assert_array_equal(out[1][:at], out[0][:at])

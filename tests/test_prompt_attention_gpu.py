@@ -117,3 +117,35 @@ def test_unequal_sequences_beside_one_without_finite_numbers(tmp_path):
         for i in range(len(seqs)):
             if i % 3 != 2:
                 np.testing.assert_array_equal(got[i], together[i])
+
+
+@pytest.mark.parametrize("family", ["latent", "cap", "window"])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_tokens_in_front_of_one_without_finite_numbers(tmp_path, family, bad):
+    """A token whose values are not finite: what came before it, and what its window no longer reaches, does not depend on it."""
+    if family == "latent":
+        cfg = sx.make_config([sx.latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=128, q_rank=24, base=1000.0, mlp=None)], width=32)
+        W = sx.random_weights(cfg, seed=9)
+    elif family == "cap":
+        cfg = mx.make_config([mx.layer(mx.attention(heads=4, kv_heads=2, dim=128, vdim=128, scale=0.2, softcap=6.0, v_mix=False), mlp=None)], width=32)
+        W = mx.random_weights(cfg, seed=9)
+    else:
+        cfg = db.make_config([db.attention(heads=4, kv_heads=1, dim=128, window=65, rot_dims=32, base=1000.0, mlp=None)], width=32)
+        W = db.random_weights(cfg, seed=9)
+    W["embed"] = W["embed"].copy()
+    for at in (1, 63, 64, 127, 128, 200, 255, 256, 300, 389):
+        t = np.random.default_rng(at).integers(1, cfg["vocab"], 390)
+        t[at] = 0
+        out = []
+        for row in (W["embed"][1].copy(), np.full(32, bad, dtype=np.float32)):
+            W["embed"][0] = row
+            with sx.open_engine(sx.write_model_dir(tmp_path / ("%d_%d" % (at, len(out))), cfg, W), dtype="bfloat16") as e:
+                out.append(nx.feed_whole(e, t.tolist()))
+        good = np.arange(390) < at
+        if family == "window":
+            good |= np.arange(390) >= at + 65
+        assert np.isfinite(out[0]).all() and not np.isfinite(out[1][~good]).any(axis=-1).any()
+        assert np.isfinite(out[1][good]).all(), (at, np.flatnonzero(good & ~np.isfinite(out[1]).all(axis=-1)))
+        # rows formed again key by key: the same values without the roundings of weights and of the output's terms
+        r = nx.rel_err(out[1][good], out[0][good].astype(np.float64))
+        assert np.median(r) < 4 * 2.0 ** -9 and r.max() < 10 * 4 * 2.0 ** -9, (at, np.median(r), r.max())

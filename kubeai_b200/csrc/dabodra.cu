@@ -339,10 +339,6 @@ class Dabodra : public Model {
     rc |= vec(&x, T * W) | mat(&h, T, W) | mat(&inb, T, max_in) | mat(&yb, T, max_out) | mat(&ao, T, W) | mat(&hrow, row_cap, W) |
           vec(&logits, static_cast<size_t>(row_cap) * V);
     if (max_qn) rc |= vec(&qn, T * max_qn);
-    size_t aw = 0;
-    for (auto& s : spec)
-      if (dt == DT_BF16 && s.kind == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(e.Tcap, s.heads, s.kv_heads));
-    if (aw) rc |= dalloc(&attn_ws, aw);
     if (max_rec) rc |= mat(&xc, T, max_xc) | vec(&o32, T * max_rec);
     if (any_moe) {
       moe_cap = static_cast<int>((T * max_top + 63) / 64 * 64) + max_e * 64;
@@ -361,7 +357,22 @@ class Dabodra : public Model {
     register_tensors();
     rc = setup_tc();
     if (rc) return rc;
+    setup_spare();
     return cudaStreamSynchronize(e.stream) == cudaSuccess ? 0 : -2;
+  }
+
+  // workspaces of forms that a step can also do without: last, and only from memory to spare
+  template <typename P>
+  bool spare(P** p, size_t bytes) {
+    if (memory_to_spare(bytes) && !dalloc(p, bytes)) return true;
+    cudaGetLastError();
+    return false;
+  }
+  void setup_spare() {
+    size_t aw = 0;
+    for (auto& s : spec)
+      if (dt == DT_BF16 && s.kind == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(env.Tcap, s.heads, s.kv_heads));
+    if (aw) spare(&attn_ws, aw);
   }
 
   // The projections of a bf16 model run on the tcgen05 pair GEMM (gemm2_tcgen05.cu) where their shapes allow it (rows and

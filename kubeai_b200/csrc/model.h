@@ -46,6 +46,13 @@ struct ModelEnv {
   int* kernel_error;     // pinned: a kernel whose wait ran out leaves a mark here; the engine looks at it after every step
 };
 
+// Whether `bytes` may go to a form that a step can also do without, once everything a model needs has been allocated: half a
+// gigabyte stays free for what comes after.
+inline bool memory_to_spare(size_t bytes) {
+  size_t fr = 0, tot = 0;
+  return cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr >= bytes + (static_cast<size_t>(512) << 20);
+}
+
 struct TensorRef {
   void* ptr;
   size_t bytes;

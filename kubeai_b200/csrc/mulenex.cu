@@ -324,17 +324,9 @@ class Mulenex : public Model {
     rc |= dalloc(&x, T * W * sizeof(float)) | mat(&h, T, W) | mat(&inb, T, max_in) | mat(&ycat, T, max_kout) | mat(&ao, T, W) | mat(&hrow, row_cap, W);
     rc |= dalloc(&qn, T * max_qn * sizeof(float)) | dalloc(&logits, static_cast<size_t>(row_cap) * V * sizeof(float));
     if (vfirst_ld) rc |= mat(&vfirst, T, vfirst_ld);
-    size_t aw = 0;
-    for (auto& s : spec)
-      if (dt == DT_BF16 && s.mixer == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(e.Tcap, s.heads, s.kv_heads));
-    if (aw) rc |= dalloc(&attn_ws, aw);
     if (any_mlstm)
       rc |= dalloc(&o32, T * max_o * sizeof(float)) | dalloc(&gpre, T * 2 * max_h * sizeof(float)) | dalloc(&gkeep, T * max_h * sizeof(float)) |
             dalloc(&gtake, T * max_h * sizeof(float)) | dalloc(&gfloor, T * max_h * sizeof(float)) | dalloc(&gnq, T * max_h * sizeof(float));
-    if (dt == DT_BF16)
-      for (auto& s : spec)
-        if (s.mixer == MIX_MLSTM) scan_ws_floats = std::max(scan_ws_floats, scan_parallel_ws_cap(e.Tcap, e.num_slots, s.heads, s.dim, s.vdim, false));
-    if (scan_ws_floats) rc |= vec(&scan_ws, scan_ws_floats);
     if (any_dense) rc |= mat(&ffh, T, max_ff);
     if (any_dense || any_moe) rc |= mat(&fo, T, W);
     if (any_moe) {
@@ -354,7 +346,26 @@ class Mulenex : public Model {
     register_tensors();
     rc = setup_tc();
     if (rc) return rc;
+    setup_spare();
     return cudaStreamSynchronize(e.stream) == cudaSuccess ? 0 : -2;
+  }
+
+  // workspaces of forms that a step can also do without: last, and only from memory to spare
+  template <typename P>
+  bool spare(P** p, size_t bytes) {
+    if (memory_to_spare(bytes) && !dalloc(p, bytes)) return true;
+    cudaGetLastError();
+    return false;
+  }
+  void setup_spare() {
+    if (dt != DT_BF16) return;
+    size_t aw = 0, sw = 0;
+    for (auto& s : spec) {
+      if (s.mixer == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(env.Tcap, s.heads, s.kv_heads));
+      if (s.mixer == MIX_MLSTM) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim, false));
+    }
+    if (aw) spare(&attn_ws, aw);
+    if (sw && spare(&scan_ws, sw * sizeof(float))) scan_ws_floats = sw;
   }
 
   // The projections of a bf16 model run on the tcgen05 pair GEMM (gemm2_tcgen05.cu) where their shapes allow it (K % 8 == 0):

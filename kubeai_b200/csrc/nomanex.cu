@@ -122,6 +122,7 @@ class Nomanex : public Model {
   std::vector<void*> allocs;
   // tcgen05 projections
   float* gemm_ws = nullptr;
+  size_t gemm_ws_bytes = 0;
   int* gemm_counters = nullptr;
   CUtensorMap xm_h[kGemmNumBlockN];
   bool use_tc = false;
@@ -356,10 +357,6 @@ class Nomanex : public Model {
           mat(&hrow, row_cap, W);
     rc |= dalloc(&z, T * max_hd * sizeof(float)) | dalloc(&o32, T * max_hv * sizeof(float)) | dalloc(&qlat, T * max_ql * sizeof(float)) |
           dalloc(&olat, T * max_ol * sizeof(float)) | dalloc(&logits, static_cast<size_t>(row_cap) * V * sizeof(float));
-    if (dt == DT_BF16)
-      for (auto& s : spec)
-        if (s.mixer == MIX_GLA) scan_ws_floats = std::max(scan_ws_floats, scan_parallel_ws_cap(e.Tcap, e.num_slots, s.heads, s.dim, s.vdim, false));
-    if (scan_ws_floats) rc |= dalloc(&scan_ws, scan_ws_floats * sizeof(float));
     if (any_moe) {
       moe_cap = static_cast<int>((T * max_top + 63) / 64 * 64) + max_e * 64;
       rc |= dalloc(&scores, T * max_e * sizeof(float)) | dalloc(&topw, T * max_top * sizeof(float)) | dalloc(&topi, T * max_top * sizeof(int)) |
@@ -374,7 +371,36 @@ class Nomanex : public Model {
     register_tensors();
     rc = setup_tc();
     if (rc) return rc;
+    setup_spare();
     return cudaStreamSynchronize(e.stream) == cudaSuccess ? 0 : -2;
+  }
+
+  // workspaces of forms that a step can also do without: last, and only from memory to spare
+  template <typename P>
+  bool spare(P** p, size_t bytes) {
+    if (memory_to_spare(bytes) && !dalloc(p, bytes)) return true;
+    cudaGetLastError();
+    return false;
+  }
+  void setup_spare() {
+    if (dt != DT_BF16) return;
+    size_t sw = 0;
+    for (auto& s : spec)
+      if (s.mixer == MIX_GLA) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim, false));
+    if (sw && spare(&scan_ws, sw * sizeof(float))) scan_ws_floats = sw;
+    if (!use_tc) return;
+    const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
+    for (size_t i = 0; i < spec.size(); ++i) {
+      const LayerSpec& s = spec[i];
+      LayerWeights& w = wts[i];
+      if (s.weights_of != static_cast<int>(i) || s.mixer != MIX_LATENT || s.rot_dims <= 0 || !latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank)) continue;
+      const int N = s.heads * (s.dim + s.vdim);
+      if (!spare(&w.ukv, static_cast<size_t>(N) * s.kv_rank * 2)) continue;
+      w.tc_ukv = gemm_plan_init(&w.p_ukv, w.ukv, N, s.kv_rank, s.kv_rank, gemm_ws, gemm_counters, env.sms) == 0;
+      for (int j = 0; j < kGemmNumBlockN && w.tc_ukv; ++j)
+        if (gemm_make_x_map(&w.xm_c[j], qlat, env.Tcap, s.kv_rank, s.kv_rank, bns[j])) w.tc_ukv = false;
+      if (w.tc_ukv) { w.p_ukv.ws_bytes = gemm_ws_bytes; w.p_ukv.error = env.kernel_error; }
+    }
   }
 
   // The large projections of a bf16 model run on the tcgen05 pair GEMM (gemm2_tcgen05.cu) when their shapes allow it: the
@@ -388,6 +414,7 @@ class Nomanex : public Model {
     for (auto& s : spec) { maxN = std::max(std::max(maxN, s.n_in), s.mixer == MIX_LATENT ? s.heads * (s.dim + s.vdim) : 0); max_kout = std::max(max_kout, s.k_out); }
     const size_t ws_bytes = std::max(gemm_workspace_bytes(env.sms), gemm_deferred_ws_bytes(env.sms));
     if (dalloc(&gemm_ws, ws_bytes)) return -3;
+    gemm_ws_bytes = ws_bytes;
     const size_t n_counters = 2ull * (maxN / 128 + 2) * (env.Tcap / 32 + 2);
     if (dalloc(&gemm_counters, n_counters * sizeof(int))) return -3;
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
@@ -410,14 +437,6 @@ class Nomanex : public Model {
       for (int j = 0; j < kGemmNumBlockN && w.tc_out; ++j)
         if (gemm_make_x_map(&w.xm_out[j], ycat, env.Tcap, s.k_out, s.k_out, bns[j])) w.tc_out = false;
       if (w.tc_out) { w.p_out.ws_bytes = ws_bytes; w.p_out.error = env.kernel_error; }
-      if (s.mixer == MIX_LATENT && s.rot_dims > 0 && latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank)) {
-        const int N = s.heads * (s.dim + s.vdim);
-        if (dalloc(&w.ukv, static_cast<size_t>(N) * s.kv_rank * 2)) return -3;
-        w.tc_ukv = gemm_plan_init(&w.p_ukv, w.ukv, N, s.kv_rank, s.kv_rank, gemm_ws, gemm_counters, env.sms) == 0;
-        for (int j = 0; j < kGemmNumBlockN && w.tc_ukv; ++j)
-          if (gemm_make_x_map(&w.xm_c[j], qlat, env.Tcap, s.kv_rank, s.kv_rank, bns[j])) w.tc_ukv = false;
-        if (w.tc_ukv) { w.p_ukv.ws_bytes = ws_bytes; w.p_ukv.error = env.kernel_error; }
-      }
       if (s.ff_kind == FF_MOE)
         w.tc_experts = !gemm_grouped_plan(&w.g_eup, w.e_up, s.experts, s.ff, W) && !gemm_grouped_plan(&w.g_edown, w.e_down, s.experts, W, s.ff) &&
                        !gemm_grouped_x_maps(&w.xg_h, hsorted, moe_cap, W) && !gemm_grouped_x_maps(&w.xg_act, eact, moe_cap, s.ff);

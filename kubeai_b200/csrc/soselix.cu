@@ -111,6 +111,7 @@ class Soselix : public Model {
   size_t scan_ws_floats = 0;
   std::vector<void*> allocs;
   float* gemm_ws = nullptr;
+  size_t gemm_ws_bytes = 0;
   int* gemm_counters = nullptr;
   bool fuse = true;
   int few_rows = 16;
@@ -336,10 +337,6 @@ class Soselix : public Model {
           vec(&logits, static_cast<size_t>(row_cap) * V);
     if (max_ql) rc |= mat(&cq, T, max_cq) | mat(&qb, T, max_q) | vec(&qlat, T * max_ql) | vec(&olat, T * max_ol);
     if (max_rec) rc |= vec(&o32, T * max_rec);
-    if (dt == DT_BF16)
-      for (auto& s : spec)
-        if (s.kind == MIX_HGRN2) scan_ws_floats = std::max(scan_ws_floats, scan_parallel_ws_cap(e.Tcap, e.num_slots, s.heads, s.dim, s.vdim, true));
-    if (scan_ws_floats) rc |= vec(&scan_ws, scan_ws_floats);
     if (max_xc) rc |= mat(&xc, T, max_xc);
     if (max_ff) rc |= mat(&hid, T, max_ff) | mat(&fo, T, W);
     if (max_ol && dt == DT_BF16) {
@@ -350,7 +347,35 @@ class Soselix : public Model {
     register_tensors();
     rc = setup_tc();
     if (rc) return rc;
+    setup_spare();
     return cudaStreamSynchronize(e.stream) == cudaSuccess ? 0 : -2;
+  }
+
+  // workspaces of forms that a step can also do without: last, and only from memory to spare
+  template <typename P>
+  bool spare(P** p, size_t bytes) {
+    if (memory_to_spare(bytes) && !dalloc(p, bytes)) return true;
+    cudaGetLastError();
+    return false;
+  }
+  void setup_spare() {
+    if (dt != DT_BF16) return;
+    size_t sw = 0;
+    for (auto& s : spec)
+      if (s.kind == MIX_HGRN2) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim, true));
+    if (sw && spare(&scan_ws, sw * sizeof(float))) scan_ws_floats = sw;
+    if (!use_tc) return;
+    const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};
+    for (size_t i = 0; i < spec.size(); ++i) {
+      const LayerSpec& s = spec[i];
+      LayerWeights& w = wts[i];
+      const int N = s.heads * (s.dim + s.vdim);
+      if (s.kind != MIX_LATENT || !latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank) || !spare(&w.w_ukv, static_cast<size_t>(N) * s.kv_rank * 2)) continue;
+      w.tc_ukv = gemm_plan_init(&w.p_ukv, w.w_ukv, N, s.kv_rank, s.kv_rank, gemm_ws, gemm_counters, env.sms) == 0;
+      for (int j = 0; j < kGemmNumBlockN && w.tc_ukv; ++j)
+        if (gemm_make_x_map(&w.xm_c[j], qlat, env.Tcap, s.kv_rank, s.kv_rank, bns[j])) w.tc_ukv = false;
+      if (w.tc_ukv) { w.p_ukv.ws_bytes = gemm_ws_bytes; w.p_ukv.error = env.kernel_error; }
+    }
   }
 
   // The projections of a bf16 model run on the tcgen05 pair GEMM (gemm2_tcgen05.cu) where their shapes allow it (rows and
@@ -365,6 +390,7 @@ class Soselix : public Model {
     for (auto& s : spec) maxN = std::max(std::max(maxN, s.n_in), std::max(s.ff, s.kind == MIX_LATENT ? s.heads * (s.dim + std::max(s.rot_dim, s.vdim)) : 0));
     const size_t ws_bytes = std::max(gemm_workspace_bytes(env.sms), gemm_deferred_ws_bytes(env.sms));
     if (dalloc(&gemm_ws, ws_bytes)) return -3;
+    gemm_ws_bytes = ws_bytes;
     const size_t n_counters = 2ull * (maxN / 128 + 2) * (env.Tcap / 32 + 2);
     if (dalloc(&gemm_counters, n_counters * sizeof(int))) return -3;
     if (const char* e = getenv("B200_SX_FUSE")) fuse = atoi(e) != 0;              // A/B knobs
@@ -388,11 +414,6 @@ class Soselix : public Model {
       w.tc_in = plan(&w.p_in, w.w_in, s.n_in, W);
       w.tc_out = plan(&w.p_out, w.w_out, W, s.k_out) && maps(w.xm_out, yb, s.k_out);
       if (s.kind == MIX_LATENT) w.tc_uq = plan(&w.p_uq, w.w_uq, s.heads * (s.dim + s.rot_dim), s.q_rank) && maps(w.xm_cq, cq, s.q_rank);
-      if (s.kind == MIX_LATENT && latent_prompt_fits(s.dim, s.vdim, s.rot_dim, s.kv_rank)) {
-        const int N = s.heads * (s.dim + s.vdim);
-        if (dalloc(&w.w_ukv, static_cast<size_t>(N) * s.kv_rank * 2)) return -3;
-        w.tc_ukv = plan(&w.p_ukv, w.w_ukv, N, s.kv_rank) && maps(w.xm_c, qlat, s.kv_rank);
-      }
       if (s.mlp) {
         w.tc_up = plan(&w.p_up, w.w_up, s.ff, W);
         w.tc_down = plan(&w.p_down, w.w_down, W, s.ff) && maps(w.xm_hid, hid, s.ff);

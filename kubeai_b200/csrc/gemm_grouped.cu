@@ -172,16 +172,10 @@ __device__ __forceinline__ void finish_rows(const float* sums, int step, int par
     } else {
       if (n0 + c >= N) continue;
       add_parts(v, p, step, parts);
-      if (EPI <= 4 && EPI >= 2 && o.bias) {
+      if ((EPI == 3 || EPI == 4) && o.bias) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           if (n0 + c + i < N) v[i] += __ldg(o.bias + n0 + c + i);
-      }
-      if (EPI == 2) {
-        float* y = static_cast<float*>(o.y) + r * o.ldy + n0 + c;
-        *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]);
-        if (n0 + c + 4 < N) *reinterpret_cast<float4*>(y + 4) = make_float4(v[4], v[5], v[6], v[7]);
-        continue;
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -346,7 +340,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       const float bias = EPI >= 2 && EPI <= 4 && o.bias && n0 + row < N ? __ldg(o.bias + n0 + row) : 0.f;   // a thread's accumulator row is one output column
       const bool relu2 = EPI == 3 && o.epi == GROUPED_RELU2;
       bool whole = true;
-      if (split.parts > 1) {
+      if (EPI != 2 && split.parts > 1) {
         whole = false;
         const size_t slab = static_cast<size_t>(split.tile) * kSlab;
         float* first = split.ws + (static_cast<size_t>(t.id) * split.parts * 2 + rank) * slab;
@@ -368,7 +362,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           __threadfence();
         }
         last = !all_epilogue(!last);       // thread 0's answer reaches all
-        if (last) finish_parts<EPI>(reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))), first, 2 * slab, split.parts, t, n0, N, o, et);
+        if constexpr (EPI != 2)
+          if (last) finish_parts<EPI>(reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))), first, 2 * slab, split.parts, t, n0, N, o, et);
       }
       constexpr int kStep = EPI == 2 ? 32 : kOutRows;
       for (int c0 = 0; whole && c0 < t.rows; c0 += kStep) {
@@ -498,7 +493,7 @@ int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap
            const SplitK& split, int units, int* error, cudaStream_t st) {
   const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED || o.epi == GROUPED_SILU;
   if ((!expert_rows && (experts != 1 || rows < 1)) || !o.y || o.ldy % (f32 ? 4 : 8) || N % (f32 ? 4 : 8) || reinterpret_cast<uintptr_t>(o.y) % 16 || units < 1 ||
-      (gated && (N % kSlab || o.bias)) || (o.epi == GROUPED_TWO_TERMS && (N % (2 * kSlab) || o.bias || !o.y2 || reinterpret_cast<uintptr_t>(o.y2) % 16)) || (o.bias && experts != 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
+      (gated && (N % kSlab || o.bias)) || (o.epi == GROUPED_TWO_TERMS && (N % (2 * kSlab) || o.bias || !o.y2 || reinterpret_cast<uintptr_t>(o.y2) % 16)) || (o.bias && experts != 1) || (f32 && split.parts > 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
   static std::atomic<unsigned long long> attr[14];
   auto start = [&](auto kernel, int i) {
     if (!ensure_dynamic_smem(kernel, kSmem, &attr[i])) return -2;
@@ -553,7 +548,8 @@ int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int 
   if (rows < 1) return 0;
   const int box = gemm2_x_box_rows(block_n), ntt = (rows + 2 * box - 1) / (2 * box), tile = ((rows + ntt - 1) / ntt + 15) & ~15;
   const int tiles = (p.N + 2 * kSlab - 1) / (2 * kSlab) * ((rows + tile - 1) / tile);
-  return gemm_whole_run_as(p, tm_x, box, tile, gemm_whole_parts(p.N, p.K, tile, tiles, p.max_ctas / 2), rows, o, p.error, st);
+  // (fp32 outputs have no split form)
+  return gemm_whole_run_as(p, tm_x, box, tile, o.epi == GROUPED_F32 ? 1 : gemm_whole_parts(p.N, p.K, tile, tiles, p.max_ctas / 2), rows, o, p.error, st);
 }
 
 int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, int* error, cudaStream_t st) {

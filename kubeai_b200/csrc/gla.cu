@@ -545,7 +545,7 @@ int gla_scan(const GlaArgs& a, cudaStream_t st) {
   if ((a.nstate != nullptr) != (a.nq != nullptr) || (a.nstate && !a.tok_decay)) return -1;
   if (a.tok_decay && (!a.tok_kscale || a.head_decay)) return -1;
   if (!a.tok_decay && !a.head_decay && !a.dt_pre && !a.fgate_lower && (!a.z || !a.z_bias)) return -1;
-  if (!a.dt_pre && scan_parallel_fits(a)) {
+  if (scan_parallel_fits(a)) {
     const char* e = getenv("B200_SCAN_CHUNK");
     const int from = e ? atoi(e) : 8;
     if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return scan_parallel(a, st);

@@ -519,8 +519,7 @@ int moe_combine_add(const void* y, DType ty, const int* pair_pos, const float* t
 int moe_combine_identity(const void* y, DType ty, const int* pair_pos, const float* topk_w, const int* topk_ids, int matrices, const void* x,
                          void* out, DType t, int T, int top, int W, cudaStream_t st);
 // bf16 helpers of the per-expert tensor-core path: x rows in sorted order (negative source row -> zeros; with row_scale the
-// row is multiplied by row_scale[r] in fp32 and rounded once), max(p, 0)^2 in place
+// row is multiplied by row_scale[r] in fp32 and rounded once)
 int moe_gather_bf16(const void* x, const int* sorted_rows, void* out, int rows, int W, cudaStream_t st, const float* row_scale = nullptr);
-int relu2_bf16(void* p, long long n, cudaStream_t st);
 
 }  // namespace b200

@@ -297,13 +297,6 @@ __global__ void moe_gather_kernel(const uint4* x, const int* sorted_rows, uint4*
   }
   out[i] = v;
 }
-__global__ void relu2_kernel(__nv_bfloat162* p, long long n2) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n2) return;
-  float2 v = __bfloat1622float2(p[i]);
-  v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f);
-  p[i] = __floats2bfloat162_rn(v.x * v.x, v.y * v.y);
-}
 }  // namespace
 
 int moe_gather_bf16(const void* x, const int* sorted_rows, void* out, int rows, int W, cudaStream_t st, const float* row_scale) {
@@ -311,13 +304,6 @@ int moe_gather_bf16(const void* x, const int* sorted_rows, void* out, int rows, 
   if (W % 8) return -1;
   const long long total = static_cast<long long>(rows) * (W / 8);
   launch_pdl(moe_gather_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, st, static_cast<const uint4*>(x), sorted_rows, static_cast<uint4*>(out), W / 8, total, row_scale);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-
-int relu2_bf16(void* p, long long n, cudaStream_t st) {
-  if (n <= 0) return 0;
-  if (n % 2) return -1;
-  relu2_kernel<<<static_cast<unsigned>((n / 2 + 255) / 256), 256, 0, st>>>(static_cast<__nv_bfloat162*>(p), n / 2);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

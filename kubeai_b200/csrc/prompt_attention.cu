@@ -540,7 +540,9 @@ size_t window_prompt_ws_bytes(int rows, int heads, int kv_heads) { return static
 bool window_prompt_pays(int T, int nseq, int heads) {
   static const int least = [] { const char* e = getenv("B200_WINDOW_PROMPT"); return e ? atoi(e) : 32; }();   // A/B knob: fewest tokens a prompt, 0 = never
   const long long n = nseq;
-  return least > 0 && T >= least * n && (T >= 2 * least * n || n * heads <= 148);
+  int sms = 0, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+  return least > 0 && T >= least * n && (T >= 2 * least * n || n * heads <= sms);
 }
 
 bool latent_prompt_fits(int dim, int vdim, int rot_dim, int kv_rank) {

@@ -1,5 +1,5 @@
 // The recurrent scan (mixers.h GlaArgs) for steps of prompt portions, every chunk of 64 tokens by itself: learned decays per
-// key channel (gated linear attention, HGRN2) and scalar gates per token (mLSTM with its normaliser, Mamba-2).
+// key channel (gated linear attention, HGRN2) and scalar gates per token (mLSTM with its normaliser).
 //
 // With l_t the log decay of token t (a vector over the key channels), S <- diag(e^l_t) S + k_t v_t^T and o_t = S^T q_t unroll
 // inside a chunk, whose incoming state is S_0 and c_t = l_1 + ... + l_t, to
@@ -45,7 +45,6 @@ struct Work {
 };
 
 __device__ __forceinline__ float floor_log(float x) { return x < kLowest ? kLowest : x; }   // keeps NaN
-__device__ __forceinline__ float softplus_(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float bf(const bf16* p) { return __bfloat162float(__ldg(p)); }
 
 // The sequence and chunk that number `id` is (chunks are numbered sequence by sequence); false past the last one.
@@ -82,14 +81,8 @@ __device__ __forceinline__ void forget_gate(float g, float lower, float* la, flo
 }
 // log decay and key scale of a token's scalar gates
 __device__ __forceinline__ void scalar_gate(const GlaArgs& a, long long row, int head, float* la, float* ks) {
-  if (a.dt_pre) {
-    const float d = softplus_(bf(static_cast<const bf16*>(a.dt_pre) + row * a.ld_dt + head) + __ldg(a.dt_bias + head));
-    *la = floor_log(__ldg(a.dt_rate + head) * d);
-    *ks = d;
-  } else {
-    *la = floor_log(logf(__ldg(a.tok_decay + row * a.heads + head)));
-    *ks = __ldg(a.tok_kscale + row * a.heads + head);
-  }
+  *la = floor_log(logf(__ldg(a.tok_decay + row * a.heads + head)));
+  *ks = __ldg(a.tok_kscale + row * a.heads + head);
 }
 
 // z -> log decay in place: inv_tau * logsigmoid(z + bias)
@@ -611,8 +604,8 @@ size_t scan_parallel_ws_floats(int tokens, int seqs, int heads, int dim, int vdi
 
 bool scan_parallel_fits(const GlaArgs& a) {
   auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-  return a.par_ws && a.t == DT_BF16 && (a.act == GLA_ACT_NONE || a.act == GLA_ACT_SILU_Q) && !a.rope && !a.head_decay && a.dim % 16 == 0 && a.dim <= kMaxD &&
-         a.vdim % 8 == 0 && a.ld % 8 == 0 && a.v_off % 8 == 0 && al(a.qkv) && al(a.states) && al(a.o) && al(a.par_ws) && (a.tok_decay || a.dt_pre || a.fgate_lower || al(a.z)) &&
+  return a.par_ws && a.t == DT_BF16 && (a.act == GLA_ACT_NONE || a.act == GLA_ACT_SILU_Q) && !a.rope && !a.head_decay && !a.dt_pre && !a.tok_decay == !a.nstate && a.dim % 16 == 0 && a.dim <= kMaxD &&
+         a.vdim % 8 == 0 && a.ld % 8 == 0 && a.v_off % 8 == 0 && al(a.qkv) && al(a.states) && al(a.o) && al(a.par_ws) && (a.tok_decay || a.fgate_lower || al(a.z)) &&
          scan_parallel_ws_floats(a.T, a.nseq, a.heads, a.dim, a.vdim, a.fgate_lower != nullptr) <= a.par_ws_floats;
 }
 
@@ -625,7 +618,7 @@ int scan_parallel(const GlaArgs& a, cudaStream_t st) {
   w.d = w.s + rows * a.vdim;
   w.n = w.d + rows;
   w.la = w.n + rows;
-  if (a.tok_decay || a.dt_pre) return a.nstate ? run<SCALAR, true>(a, w, chunks, st) : run<SCALAR, false>(a, w, chunks, st);
+  if (a.tok_decay) return run<SCALAR, true>(a, w, chunks, st);
   if (a.fgate_lower) return run<VEC_FGATE, false>(a, w, chunks, st);
   const long long total = static_cast<long long>(a.T) * a.heads * a.dim;
   if (total > 0) log_decay_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(a.z, a.z_bias, a.heads * a.dim, a.inv_tau, total);

@@ -1,4 +1,4 @@
-// In-process inference engine: one instance per GPU replica (SURVEY.md §8a K1-K11, §8b).
+// In-process inference engine: one instance per GPU replica.
 // It stands where the reference launches a backend pod (internal/modelcontroller/engine_vllm.go:82-100)
 // and is reached through the C ABI in include/b200engine.h instead of the HTTP hop at
 // internal/modelproxy/handler.go:158.
@@ -594,11 +594,11 @@ int Engine::alloc_all() {
       const char* pe = getenv("B200_FUSED_PREFILL");   // A/B knob: 0 keeps the larger steps on fp32 segments + elementwise kernels
       fused2_ok = !(pe && atoi(pe) == 0) && gemm_variant() == 2 && QKV % 256 == 0 && H % 256 == 0 && (2 * I) % 256 == 0 && kD == 128 &&
                   gemm_ws_bytes >= static_cast<size_t>(sms / 2) * 2 * 512 * 128 * sizeof(float);
-      const char* he = getenv("B200_GEMM_HYBRID");     // A/B knob: 0 keeps them on the stream-K kernel in its plain form
-      // Models narrower than 1024 stay there too: their steps are promised to give the same tokens with and without fused
-      // epilogues, which holds for forms that add the same pieces (hidden 512: 142 against 134 us for a step of 150 tokens, 224
-      // against 178 for 512).
-      whole_ok = fused2_ok && H >= 1024 && !(he && atoi(he) == 0);
+      const char *wo = getenv("B200_GEMM_WHOLE"), *he = getenv("B200_GEMM_HYBRID");     // A/B knobs: 0 keeps them on the pair kernel (HYBRID=0: with plain stream-K ranges)
+      // Models narrower than 1024 stay there too, although whole tiles are a little faster (hidden 512, a step of 150 tokens 142 us
+      // on the pair kernel against 134, of 512 tokens 224 against 178): their steps are promised to give the same tokens with
+      // and without fused epilogues, which holds for forms that add the same pieces.
+      whole_ok = fused2_ok && H >= 1024 && !(wo && atoi(wo) == 0) && !(he && atoi(he) == 0);
     }
     const char* ce = getenv("B200_CHAIN");
     chain_ok = fused_ok && deferred_ok && (ce && atoi(ce) != 0) && chain_max_ctas(&chain_ctas) == 0 && chain_ctas >= 128 && chain_ctas >= sms / 2 * 2 &&
@@ -809,7 +809,7 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
   // the norms and RoPE instead of fp32 pieces they have to add, and SiLU * up in gate_up's epilogue.  One Llama-3-8B layer,
   // 2048 tokens, against the two forms below: gate_up 312 against 410 us, down 165 against 260, o 49 against 62.
   const bool wh = whole_ok && dfr && T > 128;
-  // B200_GEMM_HYBRID=0 / B200_FUSED_PREFILL=0 keep the stream-K kernel's forms.  Per projection: when the launch has at least one
+  // Narrow models and B200_GEMM_WHOLE=0 / B200_GEMM_HYBRID=0 / B200_FUSED_PREFILL=0 keep the pair kernel's forms.  Per projection: when the launch has at least one
   // (256-row x token-tile) tile per CTA pair — gate_up at every T, nothing else at Llama-3-8B's shapes — the pair kernel
   // finishes its few split tiles in-kernel and the elementwise neighbour rides in its epilogue (gemm2 mode 2, epi_pass.cuh).
   // With fewer tiles than pairs every tile is cut into several pieces and one finisher per tile would serialise the
@@ -1420,7 +1420,7 @@ int Engine::launch(InFlight* f, StepMeta* mp) {
   ring_meta[slot] = m;
   int32_t* dbuf = stage_dev[slot];
   f->t_packed = timing ? now_s() : 0.0;
-  // NVTX range per step (SURVEY.md §5): visible in nsys / ncu --nvtx timelines as "step T=<tokens> dec=<n> pre=<n>"
+  // NVTX range per step: visible in nsys / ncu --nvtx timelines as "step T=<tokens> dec=<n> pre=<n>"
   char nv[64];
   snprintf(nv, sizeof(nv), "step T=%d dec=%d pre=%d", m.T, f->ndec_seq, f->npre_seq);
   nvtxRangePushA(nv);

@@ -39,14 +39,36 @@ def test_refused_entries(entries, error):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows", [1, 31, 32, 33, 64])
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 64, 65, 97, 128])
 def test_logits_in_parts(rows):
-    """32 rows of 32768 are one part."""
-    cfg = E.default_config(num_layers=1, hidden=512, q_heads=8, kv_heads=2, intermediate=1024, vocab=32768, manual_step=1, max_num_seqs=64,
-                           max_batched_tokens=128, max_model_len=64, num_kv_blocks=256)
+    """32 rows of 32768 are one part; from the third part on a half of the staging memory is used again."""
+    cfg = E.default_config(num_layers=1, hidden=512, q_heads=8, kv_heads=2, intermediate=1024, vocab=32768, manual_step=1, max_num_seqs=128,
+                           max_batched_tokens=256, max_model_len=64, num_kv_blocks=512)
     with E.Engine(cfg) as e:
         e.set_keep_logits(True)
         ids = [e.feed_open() for _ in range(rows)]
         got = e.feed_step([(r, [i + 1, 2 * i + 1], [1]) for i, r in enumerate(ids)])
         assert np.isfinite(got).all() and got.std(axis=1).min() > 0
         np.testing.assert_array_equal(got, e.read_logits(rows))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 64])
+def test_logits_of_a_design_around_the_staging_limit(tmp_path, rows):
+    """32 rows of 32768 fp32 logits are staged, 33 go to the caller's memory at once: the same numbers row by row."""
+    import soselix_util as sx
+    cfg = sx.make_config([sx.hgrn2(mlp=None)], vocab=32768)
+    W = sx.random_weights(cfg, seed=2)
+    with sx.open_engine(sx.write_model_dir(tmp_path / "m", cfg, W), dtype="bfloat16", max_tokens=128) as e:
+        t = np.random.default_rng(1).integers(0, 32768, rows).tolist()
+        r = e.feed_open()
+        got = e.feed_step([(r, t, list(range(rows)))])
+        e.feed_close(r)
+        parts = []
+        for lo in range(0, rows, 20):        # the same step, twenty positions of it at a time
+            r = e.feed_open()
+            parts.append(e.feed_step([(r, t, list(range(lo, min(rows, lo + 20))))]))
+            e.feed_close(r)
+    assert np.isfinite(got).all() and got.std(axis=1).min() > 0
+    # other numbers of rows take other product kernels: the same sums in another order
+    np.testing.assert_allclose(got, np.concatenate(parts), rtol=0, atol=2.0 ** -20 * 64 * np.abs(got).max())

@@ -1,5 +1,5 @@
-"""Parity at BASELINE config 2's model size (Llama-3-8B shapes: hidden 4096, 32 query / 8 KV heads of 128, intermediate 14336,
-vocab 128256), default-on in the GPU suite (VERDICT r1 item 1):
+"""Parity at the headline benchmark's model size (Llama-3-8B shapes: hidden 4096, 32 query / 8 KV heads of 128, intermediate 14336,
+vocab 128256), default-on in the GPU suite:
 
   * one full-size decoder layer + lm_head through the engine against the oracle's ops on the same weights, for a
     T=128 prefill, a T=1536 prefill and a 128-sequence decode step over contexts 16..2047 (the production decode batch);
@@ -150,15 +150,17 @@ def test_full_size_decode_step_of_128_sequences_matches_oracle(layer):
     assert (G.argmax(-1)[solid] == Wn.argmax(-1)[solid]).all()
 
 
-@pytest.mark.parametrize("mode", ["fused_epilogues", "fused_stream_k_only", "fp32_segments"])
+@pytest.mark.parametrize("mode", ["fused_epilogues", "fused_whole_waves", "fused_stream_k_only", "fp32_segments"])
 def test_full_size_prefill_burst_step_matches_oracle(layer, mode, monkeypatch):
     """A prefill burst as the scheduler runs it (T = 1500 new tokens of four prompts in ONE step, the sampled rows only):
-    the pair kernel with SiLU*up in gate_up's epilogue and the whole-tile-waves + stream-K-tail schedule (default), the same
-    with plain stream-K ranges (B200_GEMM_HYBRID=0), and the fp32-segment form (B200_FUSED_PREFILL=0), each against the
-    oracle; the last two cut the tiles at the same k-blocks and must agree bit for bit."""
+    the whole-tile product with SiLU*up in gate_up's epilogue (default), the pair kernel with the same epilogue and the
+    whole-tile-waves + stream-K-tail schedule (B200_GEMM_WHOLE=0), the same with plain stream-K ranges (B200_GEMM_HYBRID=0), and
+    the fp32-segment form (B200_FUSED_PREFILL=0), each against the oracle; the last two cut the tiles at the same k-blocks and
+    must agree bit for bit."""
     from kubeai_b200.engine import Engine, default_config
     _, cfg, w, cs = layer
     monkeypatch.setenv("B200_FUSED_PREFILL", "0" if mode == "fp32_segments" else "1")
+    monkeypatch.setenv("B200_GEMM_WHOLE", "0" if mode == "fused_whole_waves" else "1")
     monkeypatch.setenv("B200_GEMM_HYBRID", "0" if mode == "fused_stream_k_only" else "1")
     rng = np.random.default_rng(77)
     lens = [700, 450, 300, 50]
@@ -175,9 +177,9 @@ def test_full_size_prefill_burst_step_matches_oracle(layer, mode, monkeypatch):
     want = np.stack([oracle_layer(cfg, w, cs, p, [len(p) - 1])[0] for p in prompts])
     logits_close(got, want, f"prefill burst T={sum(lens)} ({mode})")
     _BURST[mode] = (got, launches)
-    if len(_BURST) == 3:
+    if len(_BURST) == 4:
         assert np.array_equal(_BURST["fused_stream_k_only"][0], _BURST["fp32_segments"][0]), "the two forms differ"
-        assert _BURST["fused_epilogues"][1] == _BURST["fused_stream_k_only"][1] < _BURST["fp32_segments"][1]
+        assert _BURST["fused_epilogues"][1] == _BURST["fused_whole_waves"][1] == _BURST["fused_stream_k_only"][1] < _BURST["fp32_segments"][1]
 
 
 _BURST = {}

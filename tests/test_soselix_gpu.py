@@ -228,9 +228,9 @@ def test_bfloat16_large_prompt_step_takes_the_64_row_attention_kernel_by_itself(
 
 
 def test_fused_large_step_products_equal_the_plain_ones(tmp_path, monkeypatch):
-    """Matrices of whole 256-row tiles in a step with a tile per CTA pair and more take the fused GEMM form: bias and xIELU in
-    the epilogue of a wide up-projection, 256-token tiles for a deep down-projection, the filled-up input projection.  The
-    step's last token tiles are partial.  Rows of the first tokens are the oracle's; all rows are those of the plain form."""
+    """Large steps take the whole-tile product: bias and xIELU in the epilogue of a wide up-projection (in a kernel of their own
+    with B200_SX_FUSE=0), a deep down-projection, the filled-up input projection.  The step's last token tiles are partial.
+    Rows of the first tokens are the oracle's; all rows are those of the plain form."""
     layers = [hgrn2(heads=4, dim=96, vdim=104, mlp=dense(4352)), mamba2(heads=8, vdim=120, state=16, groups=1, norm_groups=4, conv=4, mlp=None)]
     cfg, W, d = build(tmp_path, layers, seed=81, width=2048, vocab=64)
     T = 4700

@@ -6,7 +6,8 @@ import numpy as np
 import pytest
 import torch
 
-from mulenex_util import attention, layer, make_config, moe, mlstm, open_engine, feed_whole, random_weights, rel_err, write_model_dir, oracle_for
+import soselix_util as sx
+from mulenex_util import attention, bf16_round, dense, layer, make_config, moe, mlstm, open_engine, feed_whole, random_weights, rel_err, write_model_dir, oracle_for
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +92,25 @@ def test_gated_unit_in_the_epilogue_is_the_one_of_its_own_kernel(tmp_path, monke
         with open_engine(d, dtype="bfloat16") as e:
             out.append(feed_whole(e, t))
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("T", [17, 64, 130, 300])
+def test_split_products_with_an_epilogue(tmp_path, monkeypatch, T):
+    """Few weight tiles and a long K: the last part adds the others and goes on to the bias and squared ReLU, the gated unit of a
+    shared expert, or the bias and xIELU."""
+    monkeypatch.setenv("B200_SX_FEW_ROWS", "1")
+    mxc = make_config([layer(attention(heads=2, kv_heads=1, dim=16, vdim=16), mlp=dense(ff=264)),
+                       layer(attention(heads=2, kv_heads=1, dim=16, vdim=16, v_mix=False), mlp=moe(experts=2, top=1, ff=64, shared=192))], width=2048)
+    sxc = sx.make_config([sx.latent(), dict(sx.hgrn2(), mlp=sx.dense(ff=520))], width=2048)
+    for name, cfg, weights, oracle, knob in (("mx", mxc, random_weights, oracle_for, "B200_MX_TC"), ("sx", sxc, sx.random_weights, sx.oracle_for, "B200_SX_TC")):
+        W = weights(cfg, seed=T)
+        d = write_model_dir(tmp_path / name, cfg, W)
+        t = np.random.default_rng(T).integers(0, cfg["vocab"], T).tolist()
+        out = []
+        for on in ("1", "0"):                # "0": unsplit tile kernels of linear.cu and the epilogues' own kernels
+            monkeypatch.setenv(knob, on)
+            with open_engine(d, dtype="bfloat16") as e:
+                out.append(rel_err(feed_whole(e, t), oracle(cfg, W).forward(t)))
+        # the fused form rounds once less per product; otherwise the same roundings
+        assert np.median(out[0]) < 0.03 and np.median(out[0]) < 1.1 * np.median(out[1]) + 2.0 ** -11, (name, np.median(out[0]), np.median(out[1]))
+        assert out[0].max() < 3 * out[1].max() + 2.0 ** -8, (name, out[0].max(), out[1].max())

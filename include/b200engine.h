@@ -1,6 +1,6 @@
 /* b200engine.h — C ABI of the in-process B200 inference engine.
  *
- * This is the drop-in boundary described in SURVEY.md §8(b).  The reference (kubeai-project/kubeai)
+ * This is the drop-in boundary.  The reference (kubeai-project/kubeai)
  * has no FFI: a backend is an HTTP server reached through
  *     internal/modelproxy/handler.go:158   proxy.ServeHTTP(w, pr.httpRequest())
  * after internal/loadbalancer/load_balancer.go:191 AwaitBestAddress picked an "ip:port".
@@ -167,7 +167,7 @@ int b200_engine_forward_logits(b200_engine* e, const int32_t* ids, int32_t n, vo
 int b200_engine_set_keep_logits(b200_engine* e, int32_t keep);
 int b200_engine_read_logits(b200_engine* e, void* host_logits_bf16, int32_t rows);
 
-/* ------------------------------------------------------------------ checkpoints (SURVEY.md §8f-2)
+/* ------------------------------------------------------------------ checkpoints
  * HF-layout Llama checkpoints: <dir>/config.json + model.safetensors[.index.json] (BF16/F16/F32 tensors).
  * The reference mounts such a directory into the backend pod (internal/modelcontroller/model_source.go:231-287). */
 /* Fill the architecture fields of cfg from <dir>/config.json; rejects head_dim != 128 and GQA != 4:1. */
@@ -250,7 +250,7 @@ uint64_t b200_xxh64(const void* data, size_t len);
  * (openaiserver/handler.go:20-49), ServeHTTP/proxyHTTP incl. error bodies and <=max_retries re-picks
  * (modelproxy/handler.go:57-159, request.go:45-63), ParseRequest (apiutils/request.go:64-225),
  * Prefix (api/openai/v1/chat_completions.go:525-543), the requests-active gauge
- * (metrics/metrics.go:16-27); plus tokenizer/chat template and vLLM-framed SSE (SURVEY.md K12/K13).
+ * (metrics/metrics.go:16-27); plus tokenizer/chat template and vLLM-framed SSE.
  * A Go http.Handler calls b200_server_handle with a writer that forwards to http.ResponseWriter. */
 typedef struct b200_server b200_server;
 typedef struct {
@@ -287,7 +287,7 @@ int b200_server_metrics(b200_server* s, char* buf, size_t cap);
  * stands for an engine in the failed state: the first failure drops the replica from the router's endpoint set. */
 /* Attach a tokenizer (b200_tokenizer_load; not owned, must outlive the server; NULL detaches): prompts are then rendered with
  * the Llama-3 chat framing / <|begin_of_text|> + encoded text, <|eot_id|> and <|end_of_text|> end a generation, and output text is
- * detokenised incrementally.  Without one the server keeps the synthetic tokenizer (SURVEY.md §8d). */
+ * detokenised incrementally.  Without one the server keeps the synthetic tokenizer. */
 int b200_server_set_tokenizer(b200_server* s, const b200_tokenizer* t);
 /* Host-only: the token ids the server would submit for this request body (parse + chat template + tokenizer).  Returns the
  * count (may exceed cap), -1 with b200_last_error() = "<status> <message>" when the request is rejected. */
@@ -322,7 +322,7 @@ typedef struct {
   double request_duration_mean_s, chunks_per_request_mean;
   double run_output_throughput, run_total_throughput;   /* tokens/s over the whole run incl. ramp */
   double ttft_mean_s, itl_mean_s;                        /* runner.go:228-229 arithmetic */
-  double ttft_p50_s, ttft_p90_s, ttft_p99_s, itl_p50_s, itl_p99_s;   /* added for BASELINE.json's metric */
+  double ttft_p50_s, ttft_p90_s, ttft_p99_s, itl_p50_s, itl_p99_s;   /* for the headline metric */
   int64_t prompt_tokens, cached_prompt_tokens, completion_tokens, total_tokens;
   char first_error[256];
 } b200_harness_result;

@@ -1,4 +1,4 @@
-// Paged causal attention for the per-step hot path (SURVEY.md §8a K6 decode, K7 chunked prefill).
+// Paged causal attention for the per-step hot path.
 // Computes softmax(q . K^T / sqrt(128)) . V over the tokens reachable through a sequence's block
 // table, GQA 4:1 — the operation the reference backend delegates to FlashInfer/FlashAttention
 // (vllm/model_executor/models/llama.py:223-233, vllm/v1/attention/backends/flashinfer.py).

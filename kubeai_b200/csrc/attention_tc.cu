@@ -1,9 +1,9 @@
-// Chunked-prefill paged attention on the 5th-generation tensor cores (SURVEY.md §8a K7): softmax(q K^T / sqrt(128)) V for
+// Chunked-prefill paged attention on the 5th-generation tensor cores: softmax(q K^T / sqrt(128)) V for
 // blocks of new tokens on top of a cached prefix, GQA 4:1, the operation the reference backend delegates to FlashInfer's
 // prefill kernel (vllm/v1/attention/backends/flashinfer.py; trtllm-gen FMHA on sm_100).
 //
-// Round 1 ran prefill on the decode kernel's mma.sync path with 16-query tiles: K/V were re-read from L2 once per 16
-// queries and the math was issue-bound.  Here a CTA owns 64 query tokens x the 4 query heads
+// On the decode kernel's mma.sync path with 16-query tiles K/V are re-read from L2 once per 16 queries and the math is
+// issue-bound.  Here a CTA owns 64 query tokens x the 4 query heads
 // of one KV head = 256 query rows, as TWO 128-row UMMA tiles (32 tokens x 4 heads each) that share every K/V tile:
 //   * one driver thread gathers a 64-token K/V tile by TMA (16 boxes: 4 pages x {K,V} x two 64-column halves, 128B swizzle —
 //     the same page gather as the decode kernel) and issues every tcgen05.mma:

@@ -1,7 +1,7 @@
 // Decode-step "projection chain": o_proj -> (residual add + RMSNorm) -> gate_up (+SiLU) -> down_proj -> (residual add +
 // RMSNorm) -> next layer's qkv_proj -> (RoPE + KV write) as ONE persistent kernel, T <= 128 tokens.
 //
-// Why.  Round 1 ran each projection and each elementwise op as its own launch: ~11 us per GEMM -> elementwise -> GEMM
+// Why.  With each projection and each elementwise op a launch of its own: ~11 us per GEMM -> elementwise -> GEMM
 // boundary, a decode step at 0.57 of the HBM roofline.  Fusing the elementwise ops into per-GEMM launches (gemm3_tcgen05.cu)
 // removed the elementwise kernels but not the per-launch cost: every GEMM launch pays ~4 us before its first MMA (CTA start,
 // barrier / TMEM set-up, the first HBM round trip) and ~3-5 us after its last one, the weight stream stops in between, and

@@ -1,4 +1,4 @@
-// Bandwidth-bound per-step ops of the Llama forward (SURVEY.md §8a K2, K3, K5, K9-act, K11-argmax).
+// Bandwidth-bound per-step ops of the Llama forward.
 // Rounding points follow the reference backend so greedy tokens match:
 //   RMSNorm:              vllm/ir/ops/layernorm.py:9-21;  fused add: vllm/_custom_ops.py:323-327 (_C op: bf16 sum, norm of it)
 //   RoPE (neox):          vllm/model_executor/layers/rotary_embedding/base.py:140-198 (bf16 cos/sin cache)

@@ -1,4 +1,4 @@
-// Dense projection GEMM for the per-step hot path (SURVEY.md §8a K4/K8/K9/K10/K11):
+// Dense projection GEMM for the per-step hot path:
 //     out[t, n] = sum_k X[t, k] * W[n, k]        (bf16 x bf16 -> fp32 -> bf16)
 // which is what the reference backend computes for qkv_proj / o_proj /
 // gate_up_proj / down_proj / lm_head (vLLM model_executor/models/llama.py:81-121,

@@ -3,8 +3,8 @@
 //   benchmark/runner.go:153-187  Run: semaphore of max_concurrent_threads, one worker per thread
 //   benchmark/runner.go:263-352  RunThread: one streaming chat completion per input message, history grows
 //   benchmark/runner.go:189-250  summarizeResults: TTFT / ITL / throughput arithmetic
-// Extensions the metric needs: p50/p99 TTFT (the Go Result only has means) and a
-// synthetic thread generator with the published workload's shape (SURVEY.md §8d) because the
+// Extensions the headline metric needs: p50/p99 TTFT (the Go Result only has means) and a
+// synthetic thread generator with the published workload's shape because the
 // ShareGPT file is not available offline.  Transports: in-process (b200_server_handle) or HTTP/1.1.
 #include <arpa/inet.h>
 #include <errno.h>
@@ -266,7 +266,7 @@ double percentile(std::vector<double>& v, double q) {
   return v[lo] + (v[hi] - v[lo]) * (idx - static_cast<double>(lo));
 }
 
-// Synthetic threads with the shape of the reference's large-exact.json (SURVEY.md §8d):
+// Synthetic threads with the shape of the reference's large-exact.json:
 // 5..30 user messages per thread (clipped geometric, mean ~7.4), message length log-normal with
 // mean ~50 tokens, total user content clipped to the prep script's 500..3000 characters
 // (benchmarks/multi-turn-chat-go/Makefile:34-37, data/prepare-input-threads.py:49-58).

@@ -1,7 +1,7 @@
 // Host-side helpers shared by the serving shell (server.cc) and the load generator (harness.cc):
 // a small JSON DOM (parse + serialise), UTF-8 rune handling (Go's []rune semantics for
 // api/openai/v1/utils.go:5-8 firstNChars), and the synthetic tokenizer / chat template
-// (SURVEY.md §8d: no Llama-3 tokenizer offline).
+// (no Llama-3 tokenizer offline).
 #pragma once
 #include <stdint.h>
 #include <stdio.h>

@@ -1,4 +1,4 @@
-// HF-layout checkpoint loading (SURVEY.md §8f-2 "next": real weights).  The reference mounts a model
+// HF-layout checkpoint loading.  The reference mounts a model
 // directory into the backend pod (internal/modelcontroller/model_source.go:231-287, hf:// / pvc:// sources)
 // and vLLM reads its *.safetensors; the in-process engine reads the same files itself:
 //   <dir>/config.json                       -> b200_config (b200_config_from_hf)

@@ -2,7 +2,7 @@
 //   internal/loadbalancer/group.go:25-150          (group, getBestAddr, reconcileEndpoints, broadcast)
 //   internal/loadbalancer/balance_chwbl.go:14-162  (CHWBL: XXH64 ring, bounded-load walk)
 //   internal/loadbalancer/balance_least_load.go:3-23
-// Data-parallel strategy of the reference: independent replicas, no collective (SURVEY.md §2a).
+// Data-parallel strategy of the reference: independent replicas, no collective.
 #include <stdio.h>
 #include <string.h>
 

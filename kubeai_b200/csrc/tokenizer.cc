@@ -1,5 +1,4 @@
-// Byte-level BPE tokenizer that reads a local HF `tokenizer.json` of the Llama-3 family ("real weights /
-// tokenizer").  The reference never tokenizes: its backend pod does (vLLM loading the checkpoint's tokenizer.json through HF
+// Byte-level BPE tokenizer that reads a local HF `tokenizer.json` of the Llama-3 family.  The reference never tokenizes: its backend pod does (vLLM loading the checkpoint's tokenizer.json through HF
 // `tokenizers`, chat template included; internal/modelcontroller/engine_vllm.go:34-41 hands it the model directory).  This is
 // that step restated on the host side of the C ABI:
 //   added / special tokens   split out of the raw text first, leftmost-longest (tokenizers AddedVocabulary, normalized=false)

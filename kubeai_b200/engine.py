@@ -42,7 +42,7 @@ def default_config(**kw) -> Config:
 
 
 def config_from_hf(model_dir: str, **kw) -> Config:
-    """Engine config whose architecture comes from an HF config.json (SURVEY.md §8f-2)."""
+    """Engine config whose architecture comes from an HF config.json."""
     cfg = default_config(**kw)
     check(lib().b200_config_from_hf(str(model_dir).encode(), C.byref(cfg)))
     return cfg

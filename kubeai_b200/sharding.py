@@ -1,4 +1,4 @@
-"""Data-parallel sharding of the session list across replicas (SURVEY.md §8e): independent replicas,
+"""Data-parallel sharding of the session list across replicas: independent replicas,
 no collective on the data path.  Each rank keeps the conversation threads that the reference's CHWBL
 ring (internal/loadbalancer/balance_chwbl.go:14-84, key = first user message's first 100 runes)
 assigns to it; torch.distributed is used only to agree on the start time and to sum / max the

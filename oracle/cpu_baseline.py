@@ -2,7 +2,7 @@
 and `bench.py --impl reference`).
 
 The literal reference path (KubeAI Go proxy -> Ollama/vLLM CPU pod) cannot run here (no Go, no
-Ollama, no weights; BASELINE.md §3), so the CPU number is the oracle's restatement of the backend
+Ollama, no weights), so the CPU number is the oracle's restatement of the backend
 math (oracle/llama_oracle.py) on the host cores: one decode step of the Llama-3-8B shape, sampled as
 `layers` decoder layers + the lm_head at batch `batch`, mean context `ctx`, extrapolated to 32
 layers.  kind = "port".

@@ -1,4 +1,4 @@
-"""TEST/BENCH INFRASTRUCTURE — BASELINE.json configs[0] ("plumbing"): the reference's own CPU-runnable case,
+"""TEST/BENCH INFRASTRUCTURE — the plumbing workload: the reference's own CPU-runnable case,
 benchmarks/multi-turn-chat-go -> openaiserver/modelproxy -> loadbalancer -> local CPU backend (qwen2:0.5b),
 restated so that it can be timed on the GPU box's host cores next to the engine (bench.py cpu_baseline leg).
 

@@ -1,8 +1,8 @@
 """TEST INFRASTRUCTURE — CPU restatement of the reference backend's per-step model math.
 
 The reference (kubeai-project/kubeai) holds no model arithmetic: its backend is the third-party
-vLLM pod (`vllm/vllm-openai:v0.10.2`, /root/reference/charts/kubeai/values.yaml:45-46, launched by
-/root/reference/internal/modelcontroller/engine_vllm.go:82-100).  This file restates the published
+vLLM pod (`vllm/vllm-openai:v0.10.2`, charts/kubeai/values.yaml:45-46, launched by
+internal/modelcontroller/engine_vllm.go:82-100).  This file restates the published
 vLLM Llama forward with its rounding points (paths inside the vllm 0.22.0 wheel of this image, the
 closest available version):
 
@@ -14,8 +14,7 @@ closest available version):
   decoder layer / MLP / attention vllm/model_executor/models/llama.py:81-121,223-233,316-340
   greedy sampling                 vllm/v1/sample/sampler.py:91,235-236
 
-Pinning: the reference's own tests hold NO vector for model math (SURVEY.md §8c "parity unpinned"
-at the reference level); this restatement is pinned against HF transformers 5.5 LlamaForCausalLM
+Pinning: the reference's own tests hold NO vector for model math; this restatement is pinned against HF transformers 5.5 LlamaForCausalLM
 run in this container (oracle/gen_golden.py -> tests/golden/llama_mini.npz).
 
 Every tensor here is a float32 torch tensor whose values are bf16-representable wherever the

@@ -1,6 +1,6 @@
 """TEST INFRASTRUCTURE — pure-Python restatement of the reference's endpoint group.
 
-Follows /root/reference/internal/loadbalancer/group.go:25-150, balance_chwbl.go:14-162 and
+Follows internal/loadbalancer/group.go:25-150, balance_chwbl.go:14-162 and
 balance_least_load.go:3-23 line by line (single-threaded: the blocking/broadcast part is reduced
 to "returns None when the Go code would block").  Pinned by replaying the reference's own tables
 (load_balancer_test.go:131-427, :19-129) in tests/test_router.py; the C++ router

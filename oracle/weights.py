@@ -4,7 +4,7 @@ The engine fills its weights on the GPU with a counter-hash generator
 (kubeai_b200/csrc/elementwise.cu: init_uniform_kernel; tensor list and scales in
 kubeai_b200/csrc/engine.cu: Engine::alloc_all).  This file restates it in numpy so that the CPU
 oracle, HF transformers and the engine all see bit-identical bf16 weights without shipping
-checkpoints (there is no network; SURVEY.md §8d "Synthetic weights").
+checkpoints (there is no network).
 """
 from __future__ import annotations
 
@@ -33,7 +33,7 @@ def _merge(acc, v):
 
 def xxh64(data: bytes, seed: int = 0) -> int:
     """XXH64 from the published specification (== cespare/xxhash Sum64 for seed 0,
-    /root/reference/internal/loadbalancer/balance_chwbl.go:140-142)."""
+    internal/loadbalancer/balance_chwbl.go:140-142)."""
     n = len(data)
     p = 0
     if n >= 32:

@@ -1,5 +1,5 @@
 """Per-kernel timings on the B200 (CUDA events, L2 flushed between iterations), with cuBLAS /
-FlashInfer on the same box as the bars to beat (SURVEY.md Appendix B).  Not a bench.py number."""
+FlashInfer on the same box as the bars to beat.  Not a bench.py number."""
 import json
 import math
 import sys

@@ -1,4 +1,4 @@
-"""BASELINE.json configs[0] (the reference's CPU-runnable plumbing case) on the host cores: the product's load generator
+"""The reference's CPU-runnable plumbing case on the host cores: the product's load generator
 over HTTP -> oracle/cpu_server.py (restated proxy + router + CPU backend).  Tiny model here; bench.py's cpu_baseline leg
 runs the same path at qwen2:0.5b's dimensions."""
 import json

@@ -232,7 +232,7 @@ def test_pipelined_run_matches_single_steps_and_delivers_to_waiting_threads():
 
 
 def test_full_size_llama3_8b_run_is_deterministic_and_accounts_prefix_reuse():
-    """BASELINE config 2 shape (Llama-3-8B, 128 sequences, <=2k context) — too big for the CPU oracle, so checked through
+    """The headline benchmark's shape (Llama-3-8B, 128 sequences, <=2k context) — too big for the CPU oracle, so checked through
     size-independent properties: two independent engines produce identical token streams for the same multi-turn
     workload (fixed schedules, no atomics in any reduction), every id is a vocabulary id, each request yields exactly
     max_tokens ids, and the second turn's cached prefix is what the block-hash chain must give."""
@@ -293,7 +293,7 @@ def test_engines_on_two_devices_in_one_process_agree():
 
 
 def test_llama3_rope_scaling_matches_hf_golden():
-    """Llama-3.1 style RoPE frequency scaling (ADVICE r1): cos/sin table vs the numpy replica, logits vs HF."""
+    """Llama-3.1 style RoPE frequency scaling: cos/sin table vs the numpy replica, logits vs HF."""
     from kubeai_b200.engine import Engine, mini_config
     from oracle.gen_golden import ROPE3
     gold = np.load(Path(__file__).parent / "golden" / "llama_mini_rope3.npz")
@@ -317,7 +317,7 @@ def test_llama3_rope_scaling_matches_hf_golden():
 
 
 def test_create_time_validation_of_pool_and_shapes():
-    """a pool that cannot hold one max_model_len sequence, and shapes the kernels reject, fail at create."""
+    """A pool that cannot hold one max_model_len sequence, and shapes the kernels reject, fail at create."""
     from kubeai_b200 import B200Error
     from kubeai_b200.engine import Engine, mini_config
     with pytest.raises(B200Error, match="KV pool too small"):

@@ -1,4 +1,4 @@
-"""HF checkpoint loading (SURVEY.md §8f-2).  CPU part: safetensors / config.json parsing through the C ABI against
+"""HF checkpoint loading.  CPU part: safetensors / config.json parsing through the C ABI against
 files written by the `safetensors` package.  GPU part: an engine loaded from a checkpoint written by HF transformers
 reproduces the golden logits."""
 import json

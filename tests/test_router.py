@@ -14,7 +14,7 @@ A1, A2, B1, B2 = "10.0.0.1:8000", "10.0.0.2:8000", "10.0.0.3:8000", "10.0.0.4:80
 
 
 def test_xxh64_known_answers():
-    # SURVEY.md §7 step 1a (python-xxhash == cespare/xxhash Sum64) + XXH64 spec test vector for ""
+    # python-xxhash == cespare/xxhash Sum64, and the XXH64 spec test vector for ""
     kat = {b"": 0xEF46DB3751D8E999, b"pod-a-10": 689047897566398072, b"pod-a-20": 8996271527020827053}
     l = lib()
     for s, h in kat.items():

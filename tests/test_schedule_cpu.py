@@ -1,6 +1,6 @@
 """Host-side scheduling rules of the large-step projection GEMM and of split-KV decode attention, through the C ABI without
-a GPU (b200_schedule_query / b200_attn_split_query are pure host functions).  These are the decisions DESIGN.md §4 and
-profiles/r02_prefill_fused.md describe for Llama-3-8B on a 148-SM part; the test pins them so that a change of a threshold
+a GPU (b200_schedule_query / b200_attn_split_query are pure host functions).  These are the decisions that
+profiles/r02_prefill_fused.md describes for Llama-3-8B on a 148-SM part; the test pins them so that a change of a threshold
 shows up as a diff here and not as a silent 5 % in the bench."""
 import ctypes as C
 

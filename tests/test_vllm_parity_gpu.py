@@ -1,6 +1,6 @@
 """Parity of the engine against the vLLM wheel of this image — the closest runnable stand-in for the reference's backend
 pod (the repo pins vllm/vllm-openai:v0.10.2, charts/kubeai/values.yaml:45; the image has 0.22) — both loading the SAME HF
-checkpoint.  Default-on whenever `import vllm` works (VERDICT r1 item 1c); B200_SKIP_VLLM=1 skips it (vLLM needs a few
+checkpoint.  Default-on whenever `import vllm` works; B200_SKIP_VLLM=1 skips it (vLLM needs a few
 minutes to start).  Two things are compared on >= 32 prompts:
 
   * LOGITS, through vLLM's prompt logprobs: for every prompt position the log-probabilities vLLM reports (the prompt's own
@@ -140,7 +140,7 @@ def test_logits_and_greedy_tokens_match_vllm_on_the_test_model(tmp_path):
 
 @pytest.mark.skipif(os.environ.get("B200_SKIP_VLLM_8B") == "1", reason="B200_SKIP_VLLM_8B=1 (writes a 16 GB checkpoint)")
 def test_full_size_llama3_8b_logits_and_greedy_tokens_match_vllm(tmp_path):
-    """BASELINE config 2's model: the engine's seeded Llama-3-8B weights are exported as an HF checkpoint, vLLM loads it,
+    """The headline benchmark's model: the engine's seeded Llama-3-8B weights are exported as an HF checkpoint, vLLM loads it,
     and both sides' logits (prompt logprobs) and greedy streams are compared on 32 prompts of 5..700 tokens."""
     from safetensors.torch import save_file
     from transformers import LlamaConfig

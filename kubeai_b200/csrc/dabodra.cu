@@ -589,7 +589,7 @@ class Dabodra : public Model {
   // The grouped kernel on one matrix: whole 256 x 256 tiles, the accumulator drained under the next tile.
   bool takes_whole(bool tc, int T) const { return tc && T > 256 && whole; }
   int run_whole(const GemmPlan& plan, const CUtensorMap* xm, bool glu, void* Y, int ldy, int T) {
-    const GroupedOut o = {Y, ldy, glu ? GROUPED_GATED : GROUPED_PLAIN, nullptr, INFINITY, 1.f, 0.f};
+    const GroupedOut o = {Y, ldy, glu ? GROUPED_GATED_FAST : GROUPED_PLAIN, nullptr, INFINITY, 1.f, 0.f};
     const int bn = gemm_block_n_for(T);
     return gemm_whole_run(plan, xm[gemm_block_n_index(bn)], bn, T, o, env.stream);
   }
@@ -726,7 +726,7 @@ class Dabodra : public Model {
       // the inputs in expert-sorted order, then one grouped GEMM per matrix; the row counts stay on the device
       KRN("moe_gather", moe_gather_bf16(h, sorted_rows, hsorted, cap, W, st));
       if (w.il_e) {
-        const GroupedOut o = {eact, s.ff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};
+        const GroupedOut o = {eact, s.ff, GROUPED_GATED_FAST, nullptr, INFINITY, 1.f, 0.f};
         KRN("moe_up", gemm_grouped_run(w.g_egu, w.xg_h, T, expert_rows, o, env.sms, env.kernel_error, st));
       } else {
         const GroupedOut o = {egu, 2 * s.ff};

@@ -79,10 +79,11 @@ struct GroupedX { CUtensorMap box[kGroupedBoxes]; };
 // What happens to a sum s[r, n]: GROUPED_PLAIN / _RELU2 / _XIELU (a_pos = p0, a_neg = p1): y[r, n] = bf16(act(s + bias[n]));
 // GROUPED_F32: y[r, n] = s + bias[n] in fp32; GROUPED_GATED (limit p0, slope p1, up offset p2; the rows of every matrix alternate
 // in blocks of 64 gate rows and their 64 up rows, N % 128 == 0): g, u = bf16(s) of the two rows, y[r, i] = bf16(min(g, p0)
-// sigmoid(p1 min(g, p0)) (clamp(u, -p0, p0) + p2)), i < N / 2; GROUPED_SILU: likewise bf16(bf16(silu(g)) u); GROUPED_TWO_TERMS
+// sigmoid(p1 min(g, p0)) (clamp(u, -p0, p0) + p2)), i < N / 2; GROUPED_GATED_FAST: the same with the fast exponential and quotient
+// (about 2^-21 of the unit ahead of its rounding to bf16); GROUPED_SILU: likewise bf16(bf16(silu(g)) u); GROUPED_TWO_TERMS
 // (N % 256 == 0): y as GROUPED_PLAIN, and of the second 128 columns h of every 256 what the rounding left, y2[r, 128 h + j] =
 // bf16(s - y[r, 256 h + 128 + j]), y2 [rows, N / 2].  bias (optional): one matrix only, GROUPED_PLAIN to _F32.
-enum GroupedEpi { GROUPED_PLAIN = 0, GROUPED_RELU2, GROUPED_XIELU, GROUPED_F32, GROUPED_GATED, GROUPED_SILU, GROUPED_TWO_TERMS };
+enum GroupedEpi { GROUPED_PLAIN = 0, GROUPED_RELU2, GROUPED_XIELU, GROUPED_F32, GROUPED_GATED, GROUPED_SILU, GROUPED_TWO_TERMS, GROUPED_GATED_FAST };
 struct GroupedOut {
   void* y;
   int ldy;

@@ -127,14 +127,18 @@ struct SplitK {
   int parts;
   int tile;        // rows of a tile
 };
+template <bool FAST>
 __device__ __forceinline__ float gated_unit(float g, float u, bool clamp, const GroupedOut& o) {
   if (clamp) { g = fminf(g, o.p0); u = fminf(fmaxf(u, -o.p0), o.p0); }
+  if (FAST) return __fdividef(g, 1.0f + __expf(-o.p1 * g)) * (u + o.p2);
   return g * (1.0f / (1.0f + expf(-(o.p1 * g)))) * (u + o.p2);     // accurate functions, as norm_act.cu's glu_clamped
 }
+template <int EPI>
+constexpr bool gates = EPI == 1 || EPI == 5 || EPI == 7;
 // EPI 5: SiLU rounded to bf16 before the product, the rounding points of the Llama path's own kernel (elementwise.cu silu_mul)
 template <int EPI>
 __device__ __forceinline__ float gated(float g, float u, bool clamp, const GroupedOut& o) {
-  return EPI == 5 ? __bfloat162float(silu_bf16(g)) * u : gated_unit(g, u, clamp, o);
+  return EPI == 5 ? __bfloat162float(silu_bf16(g)) * u : gated_unit<EPI == 7>(g, u, clamp, o);
 }
 __device__ __forceinline__ float left_over(float s) { return s - __bfloat162float(__float2bfloat16_rn(s)); }
 // Eight neighbouring columns of one row: the parts' sums added in their order.
@@ -153,13 +157,13 @@ __device__ __forceinline__ void store8(bf16* p, const float* v) {
 // n rows of a split tile, their parts in shared memory, to the rows from row0 of the output: a thread takes eight columns of a row
 template <int EPI>
 __device__ __forceinline__ void finish_rows(const float* sums, int step, int parts, int n, int row0, int n0, int N, const GroupedOut& o, int et) {
-  constexpr int kPieces = EPI == 1 || EPI == 5 ? 8 : 16;
+  constexpr int kPieces = gates<EPI> ? 8 : 16;
   for (int it = et; it < n * kPieces; it += 128) {
     const int j = it / kPieces, c = (it % kPieces) * 8;
     const float* p = sums + j * kSlab + c;
     const size_t r = row0 + j;
     float v[8];
-    if constexpr (EPI == 1 || EPI == 5) {
+    if constexpr (gates<EPI>) {
       if (n0 + kSlab > N) continue;
       float u[8];
       add_parts(v, p, step, parts);
@@ -211,7 +215,9 @@ __device__ __forceinline__ void finish_parts(float* ring, const float* first, si
 }
 
 // EPI 0: bf16(sum); 1: the gated unit; 2: fp32 sum + bias; 3: bf16(relu2(sum + bias)), or without an activation; 4: bf16(xielu(sum + bias));
-// 5: the SiLU-gated unit with its inner rounding; 6: bf16(sum), and of the pair's second slab what that rounding left.
+// 5: the SiLU-gated unit with its inner rounding; 6: bf16(sum), and of the pair's second slab what that rounding left;
+// 7: the gated unit with fast functions, for the design whose units are formed so in every kernel with an epilogue (Dabodra; 4095 tokens 1577 us,
+// 1659 with the accurate ones: a tile's drain then outlasts the next tile's products).
 // A form of its own for the plain product: looking the activation up per element made its drain a sixth of the launch longer.
 // FULL: 128-row boxes, their sizes known to the compiler.
 template <int EPI, bool FULL>
@@ -407,7 +413,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             if (j < left && n0 + c < N)
               *reinterpret_cast<float4*>(dst + static_cast<size_t>(j) * o.ldy + n0 + c) = *reinterpret_cast<const float4*>(sf + j * kSlab + c);
           }
-        } else if constexpr (EPI == 1 || EPI == 5) {
+        } else if constexpr (gates<EPI>) {
           // rows 0..63 of the slab are gate rows, 64..127 the matching up rows: output columns n0 / 2 ..
           bf16* dst = static_cast<bf16*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
           const bf16* sb = reinterpret_cast<const bf16*>(stage);
@@ -491,10 +497,10 @@ int gemm_grouped_x_maps(GroupedX* x, const void* X, int rows, int K) {
 namespace {
 int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap& tm_x, int box, const int* expert_rows, int rows, const GroupedOut& o,
            const SplitK& split, int units, int* error, cudaStream_t st) {
-  const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED || o.epi == GROUPED_SILU;
+  const bool f32 = o.epi == GROUPED_F32, gated = o.epi == GROUPED_GATED || o.epi == GROUPED_GATED_FAST || o.epi == GROUPED_SILU;
   if ((!expert_rows && (experts != 1 || rows < 1)) || !o.y || o.ldy % (f32 ? 4 : 8) || N % (f32 ? 4 : 8) || reinterpret_cast<uintptr_t>(o.y) % 16 || units < 1 ||
       (gated && (N % kSlab || o.bias)) || (o.epi == GROUPED_TWO_TERMS && (N % (2 * kSlab) || o.bias || !o.y2 || reinterpret_cast<uintptr_t>(o.y2) % 16)) || (o.bias && experts != 1) || (f32 && split.parts > 1) || split.tile < 16 || split.tile % 16 || split.tile > 2 * box) return -1;
-  static std::atomic<unsigned long long> attr[14];
+  static std::atomic<unsigned long long> attr[16];
   auto start = [&](auto kernel, int i) {
     if (!ensure_dynamic_smem(kernel, kSmem, &attr[i])) return -2;
     return launch_pdl(kernel, dim3(2 * units), dim3(kThreads), kSmem, st, tm_w, tm_x, expert_rows, experts, rows, o, N, K, box, split, error) == cudaSuccess ? 0 : -2;
@@ -502,6 +508,7 @@ int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap
 #define RUN(E) return box == 128 ? start(gemm_grouped_kernel<E, true>, 2 * E) : start(gemm_grouped_kernel<E, false>, 2 * E + 1)
   if (o.epi == GROUPED_SILU) RUN(5);
   if (o.epi == GROUPED_TWO_TERMS) RUN(6);
+  if (o.epi == GROUPED_GATED_FAST) RUN(7);
   if (gated) RUN(1);
   if (f32) RUN(2);
   if (o.epi == GROUPED_XIELU) RUN(4);

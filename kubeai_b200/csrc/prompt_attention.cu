@@ -12,8 +12,8 @@
 // Two groups of four softmax warps (thread = row) work in fp32 with base-2 exponentials and rescale O_i in TMEM only when a row
 // of the warp moved its maximum.  Key tiles outside a row tile's triangle or window are skipped for that tile.  Rows behind a
 // sequence's end belong to the next one: their keys are masked and their values cleared, so that nothing of another sequence
-// can reach a result.  A masked key has weight 0, which a product would turn into NaN where its value is infinite or NaN: row
-// tiles that find such a value in a tile they mask a part of form their rows again, key by key.  Every wait has a limit; a CTA that gives up sets an error mark and still meets at the end.
+// can reach a result.  A masked key has weight 0, which a product turns into NaN where its value is infinite or NaN: a row that
+// comes out not finite looks for such a key and is then formed again, key by key.  Every wait has a limit; a CTA that gives up sets an error mark and still meets at the end.
 //
 // With keys and values per head (window_prompt_prep gathers them from the cache): sequences of 455, 1365 and 2275 tokens, 16 query
 // and 4 key heads, cap: 291 us on mma.sync -> 120.
@@ -68,23 +68,25 @@ __device__ __forceinline__ float exp2_ftz(float x) {
   return y;
 }
 
-__device__ __forceinline__ bool finite8(uint4 v) {
-  bool f = true;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t x = k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
-    f = f && (x & 0x7f80u) != 0x7f80u && (x & 0x7f800000u) != 0x7f800000u;
-  }
-  return f;
-}
-
-// One row from the keys it sees and from no other (a thread; for rows beside values that are not finite).
+// A row that came out not finite: where a key that it masks but its tiles hold ([begin, end)) has a value that is not finite, the
+// row is formed again from the keys it sees and from no other (a thread; what it sees itself decides otherwise).
 template <int NS, bool CAP>
-__device__ __noinline__ void plain_row(const PromptAttnArgs& a, int tok0, int p, int head, int kvh) {
+__device__ __noinline__ void plain_row(const PromptAttnArgs& a, int tok0, int p, int head, int kvh, int begin, int end) {
   const long long tok = tok0 + p;
   const bf16 *q = static_cast<const bf16*>(a.q) + tok * a.ldq + head * a.q_step, *q2 = static_cast<const bf16*>(a.q2) + tok * a.heads * 64 + head * 64;
   const bf16 *kv = static_cast<const bf16*>(a.kv), *k2 = static_cast<const bf16*>(a.k2), *v2 = static_cast<const bf16*>(a.v2);
   const int lo = max(0, p - a.window + 1);
+  bool beside = false;
+  for (int j = begin; j < end && !beside; ++j) {
+    if (j >= lo && j <= p) { j = p; continue; }
+    const uint4* v = reinterpret_cast<const uint4*>(kv + static_cast<long long>(tok0 + j) * a.ldkv + a.v_off + kvh * a.v_step);
+    for (int c = 0; c < kD / 8; ++c) {
+      const uint4 x = v[c];
+      auto odd = [](uint32_t u) { return (u & 0x7f80u) == 0x7f80u || (u & 0x7f800000u) == 0x7f800000u; };
+      beside = beside || odd(x.x) || odd(x.y) || odd(x.z) || odd(x.w);
+    }
+  }
+  if (!beside) return;
   auto score = [&](int j) {
     const bf16* k = kv + static_cast<long long>(tok0 + j) * a.ldkv + a.k_off + kvh * a.k_step;
     float s = 0.f;
@@ -140,14 +142,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   auto p_ready = [&](int i) { return bars + 8u * (12 + i); };     // 4 warps: P_i written, S_i read, O_i rescaled
   auto pv_full = [&](int i) { return bars + 8u * (14 + i); };
   const uint32_t q_bar = bars + 8u * 16, v2_full = bars + 8u * 17, v2_empty = bars + 8u * 18, tmem_slot = bars + 8u * 19;
-  volatile int* odd = reinterpret_cast<volatile int*>(smem + (bars - sbase) + 8 * 20);     // [row tile]: a value that is not finite beside its mask
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (warp == 0) {
     if (lane == 0) {
       for (int s = 0; s < 2; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(s_full(i, 0), 1); mbar_init(s_full(i, 1), 1); mbar_init(p_ready(i), 4); mbar_init(pv_full(i), 1); }
-      odd[0] = odd[1] = 0;
       mbar_init(q_bar, 1); mbar_init(v2_full, 1); mbar_init(v2_empty, 1);
       fence_mbar_init();
     }
@@ -366,18 +366,6 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
         for (int c = 0; c < 8; ++c)
           *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
-        if (kv0 + kKeys - 1 > q0 + gi * kRows || kv0 < min(q0 + (gi + 1) * kRows, n) - a.window) {
-          // a tile that some row of this row tile masks a part of: are its values finite (each thread half a key's)?
-          const int it = t - t_begin;
-          if (!__all_sync(0xffffffffu, wait_limited(v_full(it & 1), (it >> 1) & 1))) { ok = false; break; }
-          if (kv0 + (row & 63) < n) {
-            const uint4* d = reinterpret_cast<const uint4*>(smem + (v_s - sbase) + (it & 1) * kVTile + (row >> 6) * kKSlab + (row & 63) * 128);
-            bool finite = true;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) finite = finite && finite8(d[c]);
-            if (!finite) odd[gi] = 1;
-          }
-        }
         if (kv0 + kKeys > n && (gi == 0 || !active(0, t))) {
           // values behind the sequence's end: cleared before the first product that reads the tile (that of row tile 0, where it is active)
           const int it = t - t_begin;
@@ -399,10 +387,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (lane == 0) mbar_arrive(p_ready(gi));
       }
       if (ok && last[gi] >= 0) ok = __all_sync(0xffffffffu, wait_limited(pv_full(gi), ph_pv));
-      if (ok && last[gi] >= 0 && __any_sync(0xffffffffu, odd[gi])) {
-        if (valid) plain_row<NS, CAP>(a, tok0, p, head, kvh);
-      } else if (ok && last[gi] >= 0) {
+      if (ok && last[gi] >= 0) {
         tc_fence_after();
+        bool finite = true;
         float inv = l > 0.f ? 1.f / l : 0.f;
         if (a.sink) {
           const float sk = a.sink[head] * 1.4426950408889634f, ml = m * mul, mm = fmaxf(ml, sk), back = exp2f(ml - mm);
@@ -419,12 +406,15 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           tmem_ld_wait();
           if (valid) {
 #pragma unroll
+            for (int c = 0; c < 32; ++c) finite = finite && (v[c] & 0x7f800000u) != 0x7f800000u;
+#pragma unroll
             for (int c = 0; c < 32; c += 8)
               *reinterpret_cast<uint4*>(dst + c0 + c) =
                   make_uint4(pack_bf16x2(__uint_as_float(v[c]) * inv, __uint_as_float(v[c + 1]) * inv), pack_bf16x2(__uint_as_float(v[c + 2]) * inv, __uint_as_float(v[c + 3]) * inv),
                              pack_bf16x2(__uint_as_float(v[c + 4]) * inv, __uint_as_float(v[c + 5]) * inv), pack_bf16x2(__uint_as_float(v[c + 6]) * inv, __uint_as_float(v[c + 7]) * inv));
           }
         }
+        if (valid && !finite) plain_row<NS, CAP>(a, tok0, p, head, kvh, first[gi] * kKeys, min(n, (last[gi] + 1) * kKeys));
       }
     }
     if (!ok && a.error) *reinterpret_cast<volatile int*>(a.error) = 1;

@@ -964,7 +964,15 @@ int gemm2_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, void* out
   const int slabs = (p.N + 2 * kSlab - 1) / (2 * kSlab);
   const bool one_each = block_n == 512 && p.K > 2048 && slabs * ((T + 255) / 256) > p.max_ctas / 2 &&
                         units_for(p, (T + 511) / 512) == slabs * ((T + 511) / 512);
-  if (gemm_whole_fits(p, out, ldo) && !one_each) {
+  // ... and few weight tiles with a long K and 64 to 256 tokens: cut into at most KB / 8 parts they leave most pairs idle, and a
+  // part's exchange grows with its tokens, while this kernel spreads their k-steps over all pairs (K 4096, 128 tokens, N 256 to
+  // 1024: 14.6 to 16.0 against 18.1 to 18.6 us; N 512, K 14336, 256 tokens: 27.1 against 38.2; the line: N 1536, K 3072, 128
+  // tokens 15.7 against 16.8, N 1536, K 4096 even; 320 tokens 28.5 against 32.3, 384 39.9 against 32.4; K 2048, N 1024, 128 tokens
+  // 13.6 against 14.3, 144 15.6 against 14.7).
+  const int KB = (p.K + kBlockK - 1) / kBlockK;
+  const bool few = slabs <= 2 ? (KB >= 48 && T > 63 && T <= 256) || (KB >= 128 && T > 256 && T <= 320) || (KB >= 32 && T > 96 && T <= 128)
+                              : (KB >= 48 && slabs * KB <= 300 && T > 64 && T <= 256) || (KB >= 32 && slabs <= 4 && slabs * KB <= 300 && T > 96 && T <= 128);
+  if (gemm_whole_fits(p, out, ldo) && !one_each && !few) {
     const GroupedOut o = {out, ldo};
     return gemm_whole_run(p, tm_x, block_n, T, o, st);
   }

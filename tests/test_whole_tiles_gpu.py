@@ -38,6 +38,19 @@ def test_product_against_64_bits_and_repeatable(T, N, K):
     assert ((got.double() - want).abs() <= 1.01 * bound + 1e-30).all()
 
 
+@pytest.mark.parametrize("T", [63, 64, 65, 96, 97, 128, 129, 256, 257, 320, 321])
+@pytest.mark.parametrize("N,K", [(256, 3072), (512, 8200), (768, 2048), (1024, 4104), (1536, 3080), (1544, 3072)])
+def test_few_weight_tiles_and_a_long_k(T, N, K):
+    """Both sides of the lines between the whole tiles and the stream-K kernel: the same bound."""
+    from kubeai_b200 import ops
+    x, w = operands(T, N, K, seed=2)
+    got, again = ops.gemm(x, w), ops.gemm(x, w)
+    assert torch.equal(got, again)
+    want = x.double() @ w.double().T
+    bound = 2.0 ** -8 * want.abs() + (K + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert ((got.double() - want).abs() <= 1.01 * bound + 1e-30).all()
+
+
 def test_infinities_and_nan_stay_in_their_rows():
     from kubeai_b200 import ops
     x, w = operands(40, 512, 8192, seed=3)

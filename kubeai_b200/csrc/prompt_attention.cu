@@ -16,11 +16,12 @@
 // comes out not finite looks for such a key and is then formed again, key by key.  Every wait has a limit; a CTA that gives up sets an error mark and still meets at the end.
 //
 // With keys and values per head (window_prompt_prep gathers them from the cache): sequences of 455, 1365 and 2275 tokens, 16 query
-// and 4 key heads, cap: 291 us on mma.sync -> 120.
+// and 4 key heads, cap: 291 us on mma.sync -> 119.
 //
-// What bounds it: the exponentials and the tensor cores about evenly.  16 heads, 192 + 128 dimensions, sequences of 455, 1365
-// and 2275 tokens: 87 us (37 GFLOP), with the product that rebuilds keys and values and the gather of the latents 126; the
-// latent-space kernel on mma.sync took 883, with its two per-head products 1109.
+// What bounds it: the chain scores, softmax, weights, sums inside the one CTA an SM holds; the tensor pipe is active 28 % of the
+// time, the exponentials' unit 17 % (profiles/prompt_kernels_ncu.md).  16 heads, 192 + 128 dimensions with values in two terms, sequences
+// of 455, 1365 and 2275 tokens: 111 us (52 GFLOP), with the product that rebuilds keys and values and the gather of the latents
+// 166; the latent-space kernel on mma.sync took 883, with its two per-head products 1109.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -62,6 +63,7 @@ __device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+// (From 2^-126 to 1, where weights and rescaling factors lie, the same bits as exp2f for every argument; below, 0.)
 __device__ __forceinline__ float exp2_ftz(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -524,7 +526,7 @@ int window_prompt_prep(const void* cache, const int* slots, const float* qn, voi
 size_t window_prompt_ws_bytes(int rows, int heads, int kv_heads) { return static_cast<size_t>(rows) * (heads + 2 * kv_heads) * kD * 2; }
 
 // Measured with 16 query and 4 key heads under a cap, window kernel on mma.sync -> this one with its gather, in us: one prompt of 32
-// tokens 22 -> 15, of 128 26 -> 17, of 512 49 -> 32; 64 prompts of 64 95 -> 64, 16 of 128 56 -> 29, 8 of 512 128 -> 56; 4095
+// tokens 22 -> 14, of 128 26 -> 15, of 512 49 -> 31; 64 prompts of 64 95 -> 66, 16 of 128 56 -> 29, 8 of 512 127 -> 58; 4095
 // tokens under a window of 1024 211 -> 95.  Many prompts of 32 fill a quarter of a CTA's 128 rows and break even (64 of them
 // 63 -> 62, 32 of them 32 -> 35): below 64 tokens only while one wave of CTAs holds them all.
 bool window_prompt_pays(int T, int nseq, int heads) {
@@ -539,10 +541,10 @@ bool latent_prompt_fits(int dim, int vdim, int rot_dim, int kv_rank) {
   return dim == kD && vdim == kD && rot_dim == 64 && kv_rank >= kD && kv_rank % 8 == 0;
 }
 
-// Measured with 16 heads, latent-space form -> this one, in us: one prompt of 32 tokens 46 -> 21, of 128 54 -> 25, of 512
-// 125 -> 41; 64 prompts of 32 227 -> 75, 128 of 16 274 -> 128, 512 of 8 1011 -> 580, 256 of 1 175 -> 222.  The line lies at 32
-// because below it the rounding of a value is averaged over few keys: the error against 64 bits is 2.8e-3 of the output in both
-// forms at 32 tokens, but 2.6e-3 against 2.3e-3 at 8.
+// Measured with 16 heads, latent-space form -> this one, in us: one prompt of 40 tokens 42 -> 25, of 128 50 -> 28, of 512
+// 122 -> 47; 64 prompts of 32 223 -> 90, 128 of 16 275 -> 156, 512 of 8 1008 -> 670, 512 of 2 566 -> 619, 256 of 1 170 -> 267: a
+// quarter of a CTA's 128 rows is where it wins by half, a few tokens a prompt are where it loses.  Error against 64 bits, of the
+// output: 2.8e-3 -> 2.4e-3 at 64 tokens, 2.3e-3 -> 2.1e-3 at 8, 2.4e-3 -> 1.8e-3 at 2 (with values in one term 2.6e-3 at 8).
 bool latent_prompt_pays(int T, int nseq) {
   static const int least = [] { const char* e = getenv("B200_LATENT_PROMPT"); return e ? atoi(e) : 32; }();   // A/B knob: fewest tokens a prompt, 0 = never
   return least > 0 && T >= static_cast<long long>(least) * nseq;

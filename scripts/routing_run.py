@@ -4,7 +4,7 @@ against LeastLoad.  The experiment of the reference's runs/llama-3.1-8x-l4/run.i
 docs/benchmarks/prefix-aware-load-balancing.md:64-80 (same harness parameters: 40 completion tokens, temperature 0,
 seeded synthetic conversation threads of the ShareGPT shape).
 
-  python scripts/routing_run.py --gpus 8 [--sessions-per-gpu 128] [--threads-per-session 5] [--out gpurun_out/routing.json]
+  python scripts/routing_run.py --gpus 8 [--sessions-per-gpu 128] [--threads-per-session 5] [--out routing.json]
 """
 from __future__ import annotations
 

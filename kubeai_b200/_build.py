@@ -27,6 +27,7 @@ SOURCES = [
     "attention_tc.cu",
     "elementwise.cu",
     "linear.cu",
+    "linear_stream.cu",
     "norm_act.cu",
     "gla.cu",
     "scan_chunk.cu",

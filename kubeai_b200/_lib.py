@@ -183,6 +183,7 @@ SYMBOLS = {
     "b200_set_gemm_variant": (C.c_int, [_i32]),
     "b200_op_gemm_trace": (C.c_int, [_vp]),
     "b200_op_gemm_deferred": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp]),
+    "b200_op_linear_rows": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, C.c_float, C.c_float, C.c_float, _vp]),
     "b200_op_gemm": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp]),
     "b200_op_gemm3": (C.c_int, [C.POINTER(Gemm3Args), _vp, _pi32]),
     "b200_op_embed": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp]),

@@ -16,4 +16,13 @@ __device__ __forceinline__ float xielu_fast(float z, float a_pos, float a_neg) {
   return fmaf(z > 0.f ? a_pos * z : 0.5f, z, z > 0.f ? 0.5f * z : a_neg * (e - 1.0f - z));
 }
 
+// A gated unit: min(g, limit) sigmoid(slope min(g, limit)) (clamp(u, -limit, limit) + up_offset); without `clamp` the limit is
+// infinite.  FAST: the hardware exponential and quotient, about 2^-21 of the unit ahead of its rounding.
+template <bool FAST>
+__device__ __forceinline__ float gated_unit(float g, float u, bool clamp, float limit, float slope, float up_offset) {
+  if (clamp) { g = fminf(g, limit); u = fminf(fmaxf(u, -limit), limit); }
+  if (FAST) return __fdividef(g, 1.0f + __expf(-slope * g)) * (u + up_offset);
+  return g * (1.0f / (1.0f + expf(-(slope * g)))) * (u + up_offset);     // accurate functions, as norm_act.cu's glu_clamped
+}
+
 }  // namespace b200

@@ -595,11 +595,12 @@ class Dabodra : public Model {
   }
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
     if (takes_whole(tc, T)) return run_whole(plan, xm, false, Y, N, T);
-    if (tc && T > few_rows) {
+    const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
+    if (tc && T > few_rows && !linear_streams(la)) {
       const int bn = gemm_block_n_for(T);
       return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
     }
-    return linear(linear_args(X, dt, Wm, dt, Y, dt, T, N, K), env.stream);
+    return linear(la, env.stream);
   }
   // per-kernel device time (b200_engine_kernel_times): with profiling on, every launch is bracketed by events and waited for
   cudaEvent_t pe0 = nullptr, pe1 = nullptr;
@@ -695,7 +696,13 @@ class Dabodra : public Model {
     KRN("moe_route", moe_route(scores, topi, topw, T, s.experts, s.groups, s.keep, s.top, st, MOE_SIGMOID, s.experts, w.correction, form));
     const void* shared_out = nullptr;
     if (s.shared) {
-      if (w.il_s && takes_whole(w.tc_shin, T)) {
+      LinearArgs sg = linear_args(h, dt, w.sh_in, dt, shact, dt, T, 2 * s.sff, W);
+      sg.ldy = s.sff;
+      LinearPairs unit;
+      unit.limit = INFINITY;
+      if (w.il_s && linear_streams(sg, &unit)) {
+        KRN("shared_in", linear_stream(sg, &unit, st));
+      } else if (w.il_s && takes_whole(w.tc_shin, T)) {
         KRN("shared_in", run_whole(w.p_shin, xm_h, true, shact, s.sff, T));     // the gated unit in the epilogue
       } else {
         KRN("shared_in", project(w.p_shin, w.tc_shin, xm_h, h, w.sh_in, sh, T, s.n_sh, W));

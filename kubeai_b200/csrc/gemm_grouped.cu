@@ -127,18 +127,12 @@ struct SplitK {
   int parts;
   int tile;        // rows of a tile
 };
-template <bool FAST>
-__device__ __forceinline__ float gated_unit(float g, float u, bool clamp, const GroupedOut& o) {
-  if (clamp) { g = fminf(g, o.p0); u = fminf(fmaxf(u, -o.p0), o.p0); }
-  if (FAST) return __fdividef(g, 1.0f + __expf(-o.p1 * g)) * (u + o.p2);
-  return g * (1.0f / (1.0f + expf(-(o.p1 * g)))) * (u + o.p2);     // accurate functions, as norm_act.cu's glu_clamped
-}
 template <int EPI>
 constexpr bool gates = EPI == 1 || EPI == 5 || EPI == 7;
 // EPI 5: SiLU rounded to bf16 before the product, the rounding points of the Llama path's own kernel (elementwise.cu silu_mul)
 template <int EPI>
 __device__ __forceinline__ float gated(float g, float u, bool clamp, const GroupedOut& o) {
-  return EPI == 5 ? __bfloat162float(silu_bf16(g)) * u : gated_unit<EPI == 7>(g, u, clamp, o);
+  return EPI == 5 ? __bfloat162float(silu_bf16(g)) * u : gated_unit<EPI == 7>(g, u, clamp, o.p0, o.p1, o.p2);
 }
 __device__ __forceinline__ float left_over(float s) { return s - __bfloat162float(__float2bfloat16_rn(s)); }
 // Eight neighbouring columns of one row: the parts' sums added in their order.

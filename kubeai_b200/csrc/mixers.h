@@ -56,6 +56,23 @@ inline LinearArgs linear_args(const void* X, DType tx, const void* W, DType tw, 
   return a;
 }
 int linear(const LinearArgs& a, cudaStream_t st);
+// The same for a few rows against a bf16 matrix, as one pass over the weights (linear_stream.cu); `linear` takes it wherever it
+// serves.  W must not be anything that a kernel still in flight writes: it is read ahead of the wait for the kernel in front.
+// With pairs, rows i and i + 64 of every 128 rows of W give one result from their two sums g, u, each rounded to bf16:
+//   PAIRS_GATED, PAIRS_SILU: Y[t, N / 2] as GROUPED_GATED, GROUPED_SILU (gemm.h);
+//   PAIRS_ROPE_KV: 128 rows are a head; query heads rotated to Y, key heads rotated and value heads to the token's cache row
+//     (kv_layer [page][K|V][kv_heads][16][128], slots < 0: none), as rope_kv_write (elementwise.cu).
+enum LinearPairsKind { PAIRS_GATED = 0, PAIRS_SILU, PAIRS_ROPE_KV };
+struct LinearPairs {
+  int kind = PAIRS_GATED;
+  float limit = 0.f, slope = 1.f, up_offset = 0.f;
+  const int *positions = nullptr, *slots = nullptr;
+  const void* cos_sin = nullptr;
+  void* kv_layer = nullptr;
+  int heads = 0, kv_heads = 0, max_pos = 0;
+};
+bool linear_streams(const LinearArgs& a, const LinearPairs* q = nullptr);
+int linear_stream(const LinearArgs& a, const LinearPairs* q, cudaStream_t st);
 // `rows` rows (a handful: the expert choices of a decode step), row r reading X row src_rows[r] (or r / src_div), writing Y row
 // dst_rows[r], with weight matrix W + groups[r] * wbs (row_scale[r] applies); a.T, a.batch, x_rows and tile_group are not used.
 // group_limit > 0: a row whose group is negative or >= group_limit has no weight matrix and is skipped (its output row is

@@ -596,7 +596,8 @@ class Mulenex : public Model {
   // ------------------------------------------------------------ forward
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K,
               const float* bias = nullptr, int act = LIN_NONE) {
-    if (tc) {
+    LinearArgs a = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
+    if (tc && !linear_streams(a)) {
       const int bn = gemm_block_n_for(T);
       const CUtensorMap& tm = xm[gemm_block_n_index(bn)];
       if ((bias || act != LIN_NONE) && gemm_whole_fits(plan, Y, N)) {
@@ -607,7 +608,6 @@ class Mulenex : public Model {
       if (!rc && (bias || act != LIN_NONE)) rc = bias_act(Y, N, bias, act, dt, T, N, env.stream);
       return rc;
     }
-    LinearArgs a = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
     a.bias = bias; a.act = act;
     return linear(a, env.stream);
   }
@@ -720,7 +720,13 @@ class Mulenex : public Model {
     const void* shared_out = nullptr;
     const float* shared_gate = nullptr;
     if (s.shared) {
-      if (w.il_s && w.tc_shin && gemm_whole_fits(w.p_shin, shact, s.sff)) {
+      LinearArgs sg = linear_args(h, dt, w.sh_in, dt, shact, dt, T, 2 * s.sff, W);
+      sg.ldy = s.sff;
+      LinearPairs unit;
+      unit.limit = INFINITY;
+      if (w.il_s && linear_streams(sg, &unit)) {
+        KRN("shared_in", linear_stream(sg, &unit, st));
+      } else if (w.il_s && w.tc_shin && gemm_whole_fits(w.p_shin, shact, s.sff)) {
         const GroupedOut o = {shact, s.sff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};     // the gated unit in the epilogue
         const int bn = gemm_block_n_for(T);
         KRN("shared_in", gemm_whole_run(w.p_shin, xm_h[gemm_block_n_index(bn)], bn, T, o, st));

@@ -654,11 +654,12 @@ class Nagilix : public Model {
 
   // ------------------------------------------------------------ forward
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
-    if (tc) {
+    const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
+    if (tc && !linear_streams(la)) {
       const int bn = gemm_block_n_for(T);
       return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
     }
-    return linear(linear_args(X, dt, Wm, dt, Y, dt, T, N, K), env.stream);
+    return linear(la, env.stream);
   }
 
   // per-kernel device time (b200_engine_kernel_times): with profiling on, every launch is bracketed by events and waited for

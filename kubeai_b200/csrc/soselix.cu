@@ -577,14 +577,15 @@ class Soselix : public Model {
   }
 
   // ------------------------------------------------------------ forward
-  // Y = X W^T, with bias and xIELU behind it where the epilogue is given.  Steps of up to 16 tokens stream the weights through
-  // linear.cu's fragment kernel, larger steps take the whole-tile product with the epilogue on its fp32 sums (gemm_grouped.cu).
+  // Y = X W^T, with bias and xIELU behind it where the epilogue is given.  Steps of few tokens are one pass over the weights
+  // (linear_stream.cu, from linear.cu), larger steps take the whole-tile product with the epilogue on its fp32 sums (gemm_grouped.cu).
   struct Epilogue {
     const float* bias = nullptr;
     float a_pos = 0.f, a_neg = 0.f;
   };
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K, const Epilogue* ep = nullptr) {
-    if (tc && T > few_rows) {
+    LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
+    if (tc && T > few_rows && !linear_streams(la)) {
       const int bn = gemm_block_n_for(T);
       if (ep && fuse && gemm_whole_fits(plan, Y, N)) {
         const GroupedOut o = {Y, N, GROUPED_XIELU, ep->bias, ep->a_pos, ep->a_neg};
@@ -593,7 +594,6 @@ class Soselix : public Model {
       const int rc = gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
       return rc || !ep ? rc : bias_act(Y, N, ep->bias, LIN_XIELU, dt, T, N, env.stream, ep->a_pos, ep->a_neg);
     }
-    LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
     if (ep) { la.bias = ep->bias; la.act = LIN_XIELU; la.a_pos = ep->a_pos; la.a_neg = ep->a_neg; }
     return linear(la, env.stream);
   }

@@ -32,6 +32,17 @@ def gemm(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def linear_rows(x, w, bias=None, act=0, p=(0.0, 0.0, 0.0), dtype=torch.bfloat16, out=None):
+    """A few rows of x against w, one pass over the weights (b200_op_linear_rows); x and w may be wider buffers' leading columns."""
+    assert x.is_cuda and w.is_cuda and x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == w.stride(1) == 1
+    T, K = x.shape
+    N = w.shape[0]
+    out = torch.empty(T, N if act < 3 else N // 2, dtype=dtype, device=x.device) if out is None else out
+    check(lib().b200_op_linear_rows(_p(x), _p(w), _p(out), _p(bias) if bias is not None else None, T, N, K, x.stride(0), w.stride(0), out.stride(0),
+                                    int(out.dtype == torch.float32), act, *p, _stream()))
+    return out
+
+
 def gemm_deferred(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """Pair GEMM in deferred-reduction mode + the generic partial reducer (T <= 512)."""
     _chk(x), _chk(w)

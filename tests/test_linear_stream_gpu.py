@@ -1,0 +1,96 @@
+"""A few rows against a wide matrix in one pass over the weights (csrc/linear_stream.cu), at the sizes where its split can go
+wrong: rows that do not fill a block, fewer rows than SMs, K that is no whole number of pieces, every token block's edges."""
+import pytest
+import torch
+
+from kubeai_b200 import B200Error
+
+pytestmark = pytest.mark.gpu
+# 1, 47 and 149 rows (fewer than a CTA each, one more than the SMs), 16- and 48-row blocks' edges, several blocks a CTA
+SHAPES = [(1, 64), (47, 8), (149, 72), (16 * 148, 192), (16 * 148 + 1, 520), (32 * 148, 136), (32 * 148 + 8, 136), (48 * 148, 64), (48 * 148 + 3, 1000),
+          (97 * 148, 72), (576, 2048), (2048, 8192)]
+
+
+def operands(T, N, K, pad=0):
+    g = torch.Generator(device="cuda").manual_seed(T * 131 + N * 7 + K)
+    x = torch.randn(T, K + pad, generator=g, device="cuda").to(torch.bfloat16)[:, :K]
+    w = torch.randn(N, K + 2 * pad, generator=g, device="cuda").mul(K ** -0.5).to(torch.bfloat16)[:, :K]
+    return x, w
+
+
+def close(y, want, K):
+    # fp32 sums of exact products in two orders differ by at most K 2^-24 of the sum of their sizes (about sqrt(K) here: 0.8^2
+    # |x||w| with |w| ~ K^-1/2), and a bf16 result by half an ulp of its own
+    lim = K * 2.0 ** -24 * K ** 0.5 + (2.0 ** -8 * want.abs() if y.dtype == torch.bfloat16 else 0.0) + 1e-7
+    assert ((y.double() - want).abs() <= lim).all(), ((y.double() - want).abs() - lim).max()
+
+
+@pytest.mark.parametrize("N,K", SHAPES)
+def test_product_matches_64_bits(N, K):
+    from kubeai_b200 import ops
+    for T in (1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 48):
+        if T > (48 if N <= 32 * 148 else 32 if N <= 80 * 148 else 16):
+            x, w = operands(T, N, K)
+            with pytest.raises(B200Error):
+                ops.linear_rows(x, w)
+            continue
+        x, w = operands(T, N, K, pad=8)
+        want = x.double() @ w.double().T
+        y = ops.linear_rows(x, w, dtype=torch.float32)
+        close(y, want, K)
+        assert torch.equal(ops.linear_rows(x, w), y.to(torch.bfloat16))     # the same sums, rounded once
+        # a row's sums do not depend on what else is in the batch (within one matrix)
+        assert torch.equal(ops.linear_rows(x[-1:], w, dtype=torch.float32)[0], y[-1])
+
+
+def test_rows_of_other_tokens_and_of_other_blocks_stay_apart():
+    """Values that are not finite reach the outputs of their own row of x or of w, and nothing is written past the sizes."""
+    from kubeai_b200 import ops
+    x, w = operands(9, 49 * 148 + 5, 200)
+    ref = ops.linear_rows(x, w, dtype=torch.float32)
+    x[3, 7], w[148, 0] = float("nan"), float("inf")
+    out = torch.full((10, w.shape[0] + 8), 7.0, device="cuda")
+    y = ops.linear_rows(x, w, out=out[:9, :w.shape[0]])
+    assert torch.isnan(y[3]).all() and not torch.isfinite(y[:, 148]).any()
+    keep = torch.ones_like(ref, dtype=torch.bool)
+    keep[3], keep[:, 148] = False, False
+    assert torch.equal(y[keep], ref[keep])
+    assert (out[9] == 7).all() and (out[:, w.shape[0]:] == 7).all()
+
+
+@pytest.mark.parametrize("N,K", [(128, 64), (2048, 192), (4096, 2048), (14336 * 2, 136)])
+@pytest.mark.parametrize("act", [3, 4])
+def test_pairs_match_their_plain_sums(N, K, act):
+    """Gated units and silu(g) u of rows i, i + 64 of every 128: the arithmetic of the separate kernels on the plain sums."""
+    from kubeai_b200 import ops
+    for T in (1, 8, 13, 16, 24, 31):
+        if T > (32 if N <= 80 * 148 else 16):
+            continue
+        x, w = operands(T, N, K)
+        # the paired form deals rows out in another order but sums each of them in the same one when the split of K is the same:
+        # it is, for every N
+        s = ops.linear_rows(x, w).reshape(T, -1, 2, 64)
+        g, u = s[:, :, 0].reshape(T, -1), s[:, :, 1].reshape(T, -1)
+        if act == 4:
+            assert torch.equal(ops.linear_rows(x, w, act=4), ops.silu_mul(torch.cat([g, u], 1).contiguous()))
+            continue
+        for lim, slope, off in ((float("inf"), 1.0, 0.0), (0.5, 1.702, 1.0)):
+            gd, ud = g.double().clamp(max=lim), u.double().clamp(-lim, lim)
+            want = gd * torch.sigmoid(slope * gd) * (ud + off)
+            got = ops.linear_rows(x, w, act=3, p=(lim, slope, off)).double()
+            assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("act", [0, 1, 2])
+def test_bias_and_activations(act):
+    from kubeai_b200 import ops
+    x, w = operands(11, 600, 256)
+    bias = torch.randn(600, device="cuda")
+    z = ops.linear_rows(x, w, dtype=torch.float32).double() + bias.double()
+    if act == 1:
+        z = z.clamp(min=0) ** 2
+    elif act == 2:
+        neg = z.clamp(max=0)
+        z = torch.where(z > 0, 0.8 * z * z, 1.2 * (torch.expm1(neg) - neg)) + 0.5 * z
+    y = ops.linear_rows(x, w, bias=bias, act=act, p=(0.8, 1.2, 0.0), dtype=torch.float32).double()
+    assert ((y - z).abs() <= 1e-5 * (1 + z.abs())).all()

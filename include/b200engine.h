@@ -391,7 +391,8 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
  * 2: out [T, N/2] = silu(gate) * up with gate/up rows interleaved in 64-row blocks of w; 3: neox RoPE of q/k heads, q ->
  * out (the fused qkv buffer, ldo), k/v -> kv_layer pages; 4: argmax_out [T] = argmax_n acc[t, n < n_valid]).
  * force: 0 automatic schedule, 1..4 pairs per tile (cluster split-K through distributed shared memory), < 0 stream-K.
- * schedule_out (optional, 3 ints): pairs per tile, stream-K flag, CTAs launched. */
+ * schedule_out (optional, 3 ints): pairs per tile, stream-K flag, CTAs launched.  epi 2 without a prologue and with force 0
+ * takes b200_op_linear_rows's kernel where that serves the sizes (no pairs per tile then). */
 typedef struct {
   int32_t N, T, K, x_rows;
   int32_t pro, epi, force;

@@ -272,6 +272,7 @@ struct Engine {
   float2* cand = nullptr;
   int* g3_flags = nullptr;
   int g3_epoch = 0;
+  bool few_ok = true;       // steps of few tokens on linear_stream.cu (B200_FEW_ROWS=0: A/B knob)
   bool fused_ok = false;
   Gemm3Schedule sch_qkv, sch_o, sch_gu, sch_down, sch_lm;
   // projection chain (chain_tcgen05.cu): o -> norm -> gate_up -> down -> norm -> next qkv -> rope in one persistent launch
@@ -600,6 +601,7 @@ int Engine::alloc_all() {
       // and without fused epilogues, which holds for forms that add the same pieces.
       whole_ok = fused2_ok && H >= 1024 && !(wo && atoi(wo) == 0) && !(he && atoi(he) == 0);
     }
+    if (const char* fe = getenv("B200_FEW_ROWS")) few_ok = atoi(fe) != 0;
     const char* ce = getenv("B200_CHAIN");
     chain_ok = fused_ok && deferred_ok && (ce && atoi(ce) != 0) && chain_max_ctas(&chain_ctas) == 0 && chain_ctas >= 128 && chain_ctas >= sms / 2 * 2 &&
                gemm_ws_bytes >= (48ull << 20) + static_cast<size_t>(chain_ctas) * 128 * 128 * 4;
@@ -974,45 +976,96 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
   P(B200_K_EMBED); if (on(B200_K_EMBED)) rc |= embed_gather(embed, ids, res, T, H, V, stream); Q();
   P(B200_K_NORM); if (on(B200_K_NORM)) rc |= rmsnorm(res, nullptr, layers[0].norm1, normed, nullptr, T, H, cfg.rms_eps, stream); Q();
   stats.kernel_launches += 2;
+  // Few tokens: projections as passes over the weights on every SM (linear_stream.cu), the residual added by the norm behind
+  // them.  The clusters that share a tile in gemm3 run on 96 of 148 SMs, and their exchange has to pay for 128 tokens.  One
+  // Llama-3-8B layer, 1 token: qkv 17.5 us -> 10, o 16 -> 7 and a norm of 3, gate and up 42.5 -> 36, down 32 -> 19 and a norm.
+  // Narrow models keep one form for all steps: theirs are promised to give the same tokens with and without fused epilogues.
+  const bool few = few_ok && H >= 1024;
+  auto product = [&](const bf16* X, const bf16* Wm, bf16* Y, int ldy, int rows_n, int N, int K) {
+    LinearArgs a = linear_args(X, DT_BF16, Wm, DT_BF16, Y, DT_BF16, rows_n, N, K);
+    a.ldy = ldy;
+    return a;
+  };
+  bool x_pending = false;   // `x` holds a projection's output that the next RMSNorm still has to add to the residual
   for (int l = 0; l < L && !rc; ++l) {
     Layer& ly = layers[l];
     bf16* kv_l = kv + static_cast<size_t>(l) * kv_layer_elems;
-    {
+    if (x_pending) {
+      P(B200_K_NORM); if (on(B200_K_NORM)) rc |= rmsnorm(x, res, ly.norm1, normed, nullptr, T, H, cfg.rms_eps, stream); Q();
+      ++stats.kernel_launches;
+      x_pending = false;
+    }
+    LinearPairs pairs;
+    pairs.kind = PAIRS_ROPE_KV;
+    pairs.positions = pos; pairs.slots = slots; pairs.cos_sin = cos_sin; pairs.kv_layer = kv_l;
+    pairs.heads = Hq; pairs.kv_heads = Hkv; pairs.max_pos = cfg.max_model_len;
+    const LinearArgs qa = product(normed, ly.wqkv, qkv, QKV, T, QKV, H);
+    P(B200_K_GEMM_QKV);
+    if (few && linear_streams(qa, &pairs)) {
+      if (on(B200_K_GEMM_QKV)) rc |= linear_stream(qa, &pairs, stream);
+    } else {
       Gemm3Params p = base(ly.p_qkv, xmap(xm_normed, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_ROPE_KV);
       p.out = qkv; p.ldo = QKV;
       p.positions = pos; p.slots = slots; p.cos_sin = cos_sin; p.kv_layer = kv_l; p.Hq = Hq; p.Hkv = Hkv; p.max_pos = cfg.max_model_len;
-      P(B200_K_GEMM_QKV); if (on(B200_K_GEMM_QKV)) rc |= gemm3_launch(p, sch_qkv, stream); Q();
+      if (on(B200_K_GEMM_QKV)) rc |= gemm3_launch(p, sch_qkv, stream);
     }
+    Q();
     if (m.nd) { P(B200_K_ATTN_DECODE); if (on(B200_K_ATTN_DECODE)) rc |= decode_attention(m, kv_l, btab, dwork, scale); Q(); ++stats.kernel_launches; }
     if (m.np) { P(B200_K_ATTN_PREFILL); if (on(B200_K_ATTN_PREFILL)) rc |= prefill_attention(kv_l, btab, pwork, m.np, scale); Q(); ++stats.kernel_launches; }
-    {
+    const LinearArgs oa = product(attn, ly.wo, x, H, T, H, Hq * kD);
+    if (few && linear_streams(oa)) {
+      P(B200_K_GEMM_O); if (on(B200_K_GEMM_O)) rc |= linear_stream(oa, nullptr, stream); Q();
+      P(B200_K_NORM); if (on(B200_K_NORM)) rc |= rmsnorm(x, res, ly.norm2, normed, nullptr, T, H, cfg.rms_eps, stream); Q();
+      ++stats.kernel_launches;
+    } else {
       Gemm3Params p = base(ly.p_o, xmap(xm_attn, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_RESADD);
       p.out = res; p.ldo = H; p.ssq_out = ssq;
       p.normed_out = normed; p.norm_w_out = ly.norm2; p.row_flags = g3_flags + 4096;
       P(B200_K_GEMM_O); if (on(B200_K_GEMM_O)) rc |= gemm3_launch(p, sch_o, stream); Q();
     }
-    {
+    LinearPairs unit;
+    unit.kind = PAIRS_SILU;
+    const LinearArgs ga = product(normed, ly.wgu, act, I, T, 2 * I, H);
+    P(B200_K_GEMM_GU);
+    if (few && linear_streams(ga, &unit)) {
+      if (on(B200_K_GEMM_GU)) rc |= linear_stream(ga, &unit, stream);
+    } else {
       Gemm3Params p = base(ly.p_gu, xmap(xm_normed, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_SILU);
       p.out = act; p.ldo = I;
-      P(B200_K_GEMM_GU); if (on(B200_K_GEMM_GU)) rc |= gemm3_launch(p, sch_gu, stream); Q();
+      if (on(B200_K_GEMM_GU)) rc |= gemm3_launch(p, sch_gu, stream);
     }
-    {
+    Q();
+    const LinearArgs da = product(act, ly.wdown, x, H, T, H, I);
+    P(B200_K_GEMM_DOWN);
+    if (few && linear_streams(da)) {
+      if (on(B200_K_GEMM_DOWN)) rc |= linear_stream(da, nullptr, stream);
+      x_pending = true;
+    } else {
       Gemm3Params p = base(ly.p_down, xmap(xm_act, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_RESADD);
       p.out = res; p.ldo = H; p.ssq_out = ssq;
       if (l + 1 < L) { p.normed_out = normed; p.norm_w_out = layers[l + 1].norm1; p.row_flags = g3_flags + 4096; }
-      P(B200_K_GEMM_DOWN); if (on(B200_K_GEMM_DOWN)) rc |= gemm3_launch(p, sch_down, stream); Q();
+      if (on(B200_K_GEMM_DOWN)) rc |= gemm3_launch(p, sch_down, stream);
     }
+    Q();
     stats.kernel_launches += 4;
   }
   if (rc) return cuda_fail("forward_fused", -2);
   if (m.S > 0) {
-    // the residual already holds the summed stream: the final norm is a plain RMSNorm of the sampled rows
-    P(B200_K_NORM); rc |= rmsnorm(res, nullptr, final_norm, last_hidden, rows, m.S, H, cfg.rms_eps, stream); Q();
-    Gemm3Params p = base(p_lm, xmap(xm_last, 128), m.S, GEMM3_PRO_NONE, keep_logits ? GEMM3_EPI_PLAIN : GEMM3_EPI_ARGMAX);
-    p.out = logits; p.ldo = V; p.cand = cand;
-    P(B200_K_GEMM_LM); rc |= gemm3_launch(p, sch_lm, stream); Q();
+    // the final norm of the sampled rows: plain where the residual already holds the summed stream
+    P(B200_K_NORM); rc |= rmsnorm(x_pending ? x : res, x_pending ? res : nullptr, final_norm, last_hidden, rows, m.S, H, cfg.rms_eps, stream); Q();
+    const LinearArgs la = product(last_hidden, lm_head, logits, V, m.S, V, H);
+    const bool stream_lm = few && linear_streams(la);
+    P(B200_K_GEMM_LM);
+    if (stream_lm) {
+      rc |= linear_stream(la, nullptr, stream);
+    } else {
+      Gemm3Params p = base(p_lm, xmap(xm_last, 128), m.S, GEMM3_PRO_NONE, keep_logits ? GEMM3_EPI_PLAIN : GEMM3_EPI_ARGMAX);
+      p.out = logits; p.ldo = V; p.cand = cand;
+      rc |= gemm3_launch(p, sch_lm, stream);
+    }
+    Q();
     P(B200_K_ARGMAX);
-    if (keep_logits) rc |= argmax_rows(logits, sampled, m.S, V, V, stream);
+    if (stream_lm || keep_logits) rc |= argmax_rows(logits, sampled, m.S, V, V, stream);
     else rc |= argmax_candidates(cand, sampled, m.S, V / 128, stream);
     Q();
     last_S = m.S;

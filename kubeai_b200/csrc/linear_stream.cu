@@ -61,7 +61,7 @@ template <int NB, int MT> struct Layout {
 };
 // In the paired form rows i and i + 64 of every 128 of W belong together (gate and up rows of the same outputs, the two halves
 // of a head): a CTA takes them as neighbours, row n of this order being row_of_pair(n) of W.
-__device__ __forceinline__ int row_of_pair(int n) { const int p = n >> 1; return ((p >> 6) << 7) + (p & 63) + ((n & 1) << 6); }
+__device__ __forceinline__ int row_of_pair(int n) { const int p = n >> 1; return p + (p & ~63) + ((n & 1) << 6); }
 
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 // Both rows of pair p of token t, rounded to bf16, to their output; the arithmetic is that of gemm_grouped.cu's gated epilogues
@@ -109,12 +109,14 @@ __global__ void __launch_bounds__(kWarps * 32) linear_stream_kernel(LinearArgs a
   const int lr = lane >> 3, lp = lane & 7;
   auto load_w = [&](int first, int piece, int slot) {
     const int live = min(rows, n1 - first), k = piece * kPiece + lp * 8;
-    const bf16* src = W + (PAIRS ? 0 : static_cast<long long>(first + lr) * a.ldw) + (k < a.K ? k : 0);
+    const bf16* src = W + static_cast<long long>(PAIRS ? row_of_pair(first + lr) : first + lr) * a.ldw + (k < a.K ? k : 0);
     const uint32_t dst = ring + slot * L::kStage;
+    // paired rows step by two of W, and by 64 more past the end of their 64 (a block is shorter than that)
+    const int end = PAIRS ? 63 - (((first + lr) >> 1) & 63) : 0;
 #pragma unroll
     for (int i = 0; i < 4 * MT; ++i) {
-      const int r = lr + 4 * i;
-      if (r < live) copy16(dst + r * 128 + ((lp ^ (r & 7)) << 4), src + static_cast<long long>(PAIRS ? row_of_pair(first + r) : 4 * i) * a.ldw, k < a.K ? 16 : 0);
+      const int r = lr + 4 * i, step = PAIRS ? 2 * i + (2 * i > end ? 64 : 0) : 4 * i;
+      if (r < live) copy16(dst + r * 128 + ((lp ^ (r & 7)) << 4), src + static_cast<long long>(step) * a.ldw, k < a.K ? 16 : 0);
     }
   };
   auto load_x = [&](int piece, int slot) {
@@ -234,14 +236,19 @@ int launch(const LinearArgs& a, const LinearPairs& q, int per_cta, int rows, cud
   launch_pdl(linear_stream_kernel<TY, NB, MT, PAIRS>, ctas, kWarps * 32, Layout<NB, MT>::kBytes, st, a, q, per_cta, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
+int sm_count() {
+  int dev = 0, sms = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? sms : 0;
+}
+// n rows in `parts` shares, whole pairs each
+int share(int n, int parts, bool pairs) { return pairs ? (n / 2 + parts - 1) / parts * 2 : (n + parts - 1) / parts; }
 template <typename TY, int NB, bool PAIRS>
 int pick_rows(const LinearArgs& a, const LinearPairs& q, int sms, cudaStream_t st) {
   // rows of W at a time: more of them use a token's row more often, fewer leave room for more stages.  28672 x 4096, 8 tokens:
-  // 64 at a time 38.7 us, 48 35.8, 32 35.8, 16 37.5; 6144 x 2048, 41 rows a CTA: 5.5 at once, 6.1 as twice 21.
+  // 64 at a time 38.7 us, 48 35.8, 32 35.8, 16 37.5 (all rows of a CTA side by side, so that a piece of X is read once: 38.5,
+  // and 36 -> 38 with one token: neighbouring pieces of a row are better read together); 6144 x 2048, 41 rows a CTA: 5.5 at once, 6.1 as twice 21.
   constexpr int kMost = NB <= 4 ? 48 : 32;
-  const int unit = PAIRS ? 2 : 1;
-  auto split = [&](int n, int parts) { return (n / unit + parts - 1) / parts * unit; };
-  const int per_cta = split(a.N, sms), rows = split(per_cta, (per_cta + kMost - 1) / kMost);
+  const int per_cta = share(a.N, sms, PAIRS), rows = share(per_cta, (per_cta + kMost - 1) / kMost, PAIRS);
   switch ((rows + 15) / 16) {
     case 1: return launch<TY, NB, 1, PAIRS>(a, q, per_cta, rows, st);
     case 2: return launch<TY, NB, 2, PAIRS>(a, q, per_cta, rows, st);
@@ -250,8 +257,8 @@ int pick_rows(const LinearArgs& a, const LinearPairs& q, int sms, cudaStream_t s
 }
 template <typename TY, bool PAIRS>
 int pick_tokens(const LinearArgs& a, const LinearPairs& q, cudaStream_t st) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
+  const int sms = sm_count();
+  if (sms < 1) return -2;
   if (a.T <= 8) return pick_rows<TY, 1, PAIRS>(a, q, sms, st);
   if (a.T <= 16) return pick_rows<TY, 2, PAIRS>(a, q, sms, st);
   if (a.T <= 24) return pick_rows<TY, 3, PAIRS>(a, q, sms, st);
@@ -266,11 +273,11 @@ int pick_tokens(const LinearArgs& a, const LinearPairs& q, cudaStream_t st) {
 //   2048 x 8192:   8 tokens 7.0 / 13.0   32 tokens 10.5 / 14.4   48 tokens 14.5 / 15.3
 //   1792 x 2048:   8 tokens 3.0 /  8.3   32 tokens  4.1 /  9.5   48 tokens  5.5 / 10.4
 //   8192 x 2048:   8 tokens 6.6 / 11.7   32 tokens  9.4 / 12.4   48 tokens 13.2 / 13.4
-//   28672 x 4096:  8 tokens 35.8 / 46.6  16 tokens 38.8 / 46.8
+//   28672 x 4096:  8 tokens 36.1 / 42.5  16 tokens 39.0 / 43.0, in a second of nothing else 38.5 / 43.5 and 43.7 / 44.0
 // More tokens cost their rows once a CTA and block of its rows, which is what narrow matrices can afford longest.
 bool linear_streams(const LinearArgs& a, const LinearPairs* q) {
   static const int most = [] { const char* e = getenv("B200_LIN_STREAM"); return e ? atoi(e) : 48; }();     // A/B knob: the most rows, 0: none
-  if (a.T > most || a.T > (a.N <= 32 * 148 ? 48 : a.N <= 80 * 148 ? 32 : 16)) return false;
+  if (a.T > most || a.T > (a.N <= 32 * 148 ? 48 : a.N <= 80 * 148 ? 32 : 8)) return false;
   if (q && (a.N % 128 || a.ty != DT_BF16 || a.bias || a.row_scale || a.act != LIN_NONE)) return false;
   return a.T > 0 && a.N > 0 && a.K > 0 && a.tx == DT_BF16 && a.tw == DT_BF16 && a.batch == 1 && !a.x_rows && !a.tile_group && a.K % 8 == 0 && a.ldx % 8 == 0 &&
          a.ldw % 8 == 0 && (reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.W)) % 16 == 0;
@@ -280,6 +287,11 @@ int linear_stream(const LinearArgs& a, const LinearPairs* q, cudaStream_t st) {
   if (!linear_streams(a, q)) return -1;
   if (q) return pick_tokens<bf16, true>(a, *q, st);
   return a.ty == DT_BF16 ? pick_tokens<bf16, false>(a, LinearPairs(), st) : pick_tokens<float, false>(a, LinearPairs(), st);
+}
+
+int linear_stream_ctas(const LinearArgs& a, const LinearPairs* q) {
+  const int per_cta = share(a.N, std::max(1, sm_count()), q != nullptr);
+  return (a.N + per_cta - 1) / per_cta;
 }
 
 }  // namespace b200

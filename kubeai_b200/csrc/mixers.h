@@ -73,6 +73,7 @@ struct LinearPairs {
 };
 bool linear_streams(const LinearArgs& a, const LinearPairs* q = nullptr);
 int linear_stream(const LinearArgs& a, const LinearPairs* q, cudaStream_t st);
+int linear_stream_ctas(const LinearArgs& a, const LinearPairs* q);   // CTAs such a launch has on this device
 // `rows` rows (a handful: the expert choices of a decode step), row r reading X row src_rows[r] (or r / src_div), writing Y row
 // dst_rows[r], with weight matrix W + groups[r] * wbs (row_scale[r] applies); a.T, a.batch, x_rows and tile_group are not used.
 // group_limit > 0: a row whose group is negative or >= group_limit has no weight matrix and is skipped (its output row is

@@ -29,7 +29,7 @@ def close(y, want, K):
 def test_product_matches_64_bits(N, K):
     from kubeai_b200 import ops
     for T in (1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 48):
-        if T > (48 if N <= 32 * 148 else 32 if N <= 80 * 148 else 16):
+        if T > (48 if N <= 32 * 148 else 32 if N <= 80 * 148 else 8):
             x, w = operands(T, N, K)
             with pytest.raises(B200Error):
                 ops.linear_rows(x, w)
@@ -64,7 +64,7 @@ def test_pairs_match_their_plain_sums(N, K, act):
     """Gated units and silu(g) u of rows i, i + 64 of every 128: the arithmetic of the separate kernels on the plain sums."""
     from kubeai_b200 import ops
     for T in (1, 8, 13, 16, 24, 31):
-        if T > (32 if N <= 80 * 148 else 16):
+        if T > (32 if N <= 80 * 148 else 8):
             continue
         x, w = operands(T, N, K)
         # the paired form deals rows out in another order but sums each of them in the same one when the split of K is the same:

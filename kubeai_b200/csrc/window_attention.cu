@@ -115,6 +115,79 @@ __global__ void __launch_bounds__(128) qk_prep_kernel(QkPrepArgs a) {
   }
 }
 
+// The same for bf16 rows of whole 16-byte pieces: LP = dim / 8 lanes own a head's row from the load to the store, so the row is
+// read once; the lanes behind the heads' copy value pieces.  4096 tokens of 16 + 4 heads of 128: 35 us above, 19 here; 24 tokens 9 and 4.
+template <int LP>
+__global__ void __launch_bounds__(1024) qk_prep_vec_kernel(QkPrepArgs a) {
+  griddep_launch();
+  griddep_wait();
+  const long long t = blockIdx.x;
+  const int p = a.positions[t], D = 8 * LP, half = a.rot_dims / 2;
+  const float q_gain = a.q_gain_every > 0 ? 1.0f + a.q_gain_coef * logf(static_cast<float>((p + 1) / a.q_gain_every + 1)) : 1.0f;
+  bf16* cache = static_cast<bf16*>(a.cache) + static_cast<long long>(a.slots[t]) * a.kv_heads * (D + a.vdim);
+  const int heads = a.heads + a.kv_heads, vpieces = a.kv_heads * a.vdim / 8;
+  for (int x0 = 0; x0 < heads * LP + vpieces; x0 += blockDim.x) {
+    const int x = x0 + threadIdx.x, u = x / LP, c0 = (x % LP) * 8;
+    const bool row = u < heads, isq = u < a.heads;
+    float v[8];
+    float ss = 0.f;
+    if (row) {
+      const bf16* src = isq ? static_cast<const bf16*>(a.q) + t * a.ld + static_cast<long long>(u) * D + c0
+                            : static_cast<const bf16*>(a.k) + t * a.ld + static_cast<long long>(u - a.heads) * D + c0;
+      const uint4 r = *reinterpret_cast<const uint4*>(src);
+      const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x0_ = __uint_as_float(w[i] << 16), x1 = __uint_as_float(w[i] & 0xffff0000u);
+        if (c0 / 2 + i < half) {
+          const float2 c = a.rope[static_cast<long long>(p) * half + c0 / 2 + i];
+          const float r0 = x0_ * c.x - x1 * c.y, r1 = x1 * c.x + x0_ * c.y;
+          x0_ = r0; x1 = r1;
+        }
+        v[2 * i] = x0_; v[2 * i + 1] = x1;
+        ss = fmaf(x0_, x0_, ss);
+        ss = fmaf(x1, x1, ss);
+      }
+    }
+#pragma unroll
+    for (int o = LP / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (row) {
+      const float inv = (a.unit_norm ? 1.0f / sqrtf(ss / static_cast<float>(D) + a.eps) : 1.0f) * (isq ? q_gain : 1.0f);
+      const float* nw = isq ? a.q_norm_w : a.k_norm_w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { v[i] *= inv; if (nw) v[i] *= nw[c0 + i]; }
+      if (isq) {
+        float4* dst = reinterpret_cast<float4*>(a.qn + (t * a.heads + u) * D + c0);
+        dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+        dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+      } else {
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]); o[i] = *reinterpret_cast<const uint32_t*>(&b); }
+        *reinterpret_cast<uint4*>(cache + static_cast<long long>(u - a.heads) * D + c0) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    } else if (x < heads * LP + vpieces) {
+      const int i0 = (x - heads * LP) * 8;
+      const uint4 r = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(a.v) + t * a.ld + i0);
+      if (a.v_raw_out) *reinterpret_cast<uint4*>(static_cast<bf16*>(a.v_raw_out) + t * a.ld_raw + i0) = r;
+      uint4 o4 = r;
+      if (a.v_blend) {
+        const uint4 b4 = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(a.v_blend) + t * a.ld_blend + i0);
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const __nv_bfloat162 z = __floats2bfloat162_rn((1.0f - a.v_lambda) * __uint_as_float(w[i] << 16) + a.v_lambda * __uint_as_float(b[i] << 16),
+                                                         (1.0f - a.v_lambda) * __uint_as_float(w[i] & 0xffff0000u) + a.v_lambda * __uint_as_float(b[i] & 0xffff0000u));
+          o[i] = *reinterpret_cast<const uint32_t*>(&z);
+        }
+        o4 = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      *reinterpret_cast<uint4*>(cache + static_cast<long long>(a.kv_heads) * D + i0) = o4;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------- convolved queries and keys
 // One CTA per token (ConvQkPrepArgs).  Pass 1: a thread per channel convolves the projections over time (its taps come
 // from the step's own rows or from the sequence's carried inputs), leaves the result in shared memory, writes the
@@ -401,6 +474,152 @@ __global__ void __launch_bounds__(kWarpsDecode * 32) window_attn_kernel(WindowAt
     o *= inv;
     if (gate) o *= sigmoidf_(ldf(gate + t * a.ldg + (a.gate_per_head ? h : static_cast<long long>(h) * Dv + c)));
     stf(y + c, o * a.out_scale);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- attention of single tokens, bf16
+// A CTA takes a token and GS query heads of one key/value head, so a key's row is read once for all of them.  Sixteen lanes
+// hold a key (eight dimensions or value columns each, whole 16-byte pieces): half-warp r takes the visible keys r, r + 16,
+// r + 32, ... (8 warps), kRowKeys of them in flight, their keys and their values, and keeps an online softmax of its own in
+// fp32 with the accurate functions; the sixteen partial results are merged in a fixed order.  Which keys a half-warp takes,
+// and in which groups, depends on the token's position alone.
+// What bounds a step of short contexts is the chain positions -> block table -> rows -> exponentials -> merge; the general
+// kernel below added a chain of 16 loads a key (a lane a key) and of loads four values at a time behind it.  24 sequences of
+// 22 tokens, 16 heads of 128 in 4 groups: 37 us there, 10 here; 16 of 250: 34
+// and 21; one of 2000, 87 and 64.
+constexpr int kRowWarps = 8, kRowKeys = 4;
+__device__ __forceinline__ void unpack8(const uint4& r, float* v) {
+  const uint32_t u[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(u[i] << 16);
+    v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+  }
+}
+
+template <int GS>
+__global__ void __launch_bounds__(kRowWarps * 32) window_attn_rows_kernel(WindowAttnArgs a, int page_shift) {
+  griddep_launch();
+  griddep_wait();
+  extern __shared__ float sm[];   // [warp][GS][m, l, acc [vdim]]
+  const int D = a.dim, Dv = a.vdim, groups = a.heads / GS;
+  const long long t = blockIdx.x / groups;
+  const int h0 = (blockIdx.x % groups) * GS, g = h0 / (a.heads / a.kv_heads);
+  const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, c0 = (lane & 15) * 8;
+  const int p = a.positions[t];
+  const int* bt = a.block_tables + static_cast<long long>(a.seq_of_tok[t]) * a.max_blocks;
+  const int lo = a.chunk > 0 ? p / a.chunk * a.chunk : max(0, p - a.window + 1);
+  const int nk = min(a.keep_first, lo), n = nk + (p - lo + 1);
+  const long long crow = static_cast<long long>(a.kv_heads) * (D + Dv);
+  const bf16* keys = static_cast<const bf16*>(a.cache) + static_cast<long long>(g) * D + c0;
+  const bf16* vals = static_cast<const bf16*>(a.cache) + static_cast<long long>(a.kv_heads) * D + static_cast<long long>(g) * Dv + c0;
+  const bool kin = c0 < D, vin = c0 < Dv;
+  float q[GS][8], acc[GS][8], m[GS], l[GS];
+#pragma unroll
+  for (int h = 0; h < GS; ++h) {
+    const float* qp = a.qn + (t * a.heads + h0 + h) * D + c0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { q[h][e] = kin ? qp[e] * a.scale : 0.f; acc[h][e] = 0.f; }
+    m[h] = -FLT_MAX; l[h] = 0.f;
+  }
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int i0 = 2 * wrp + (lane >> 4); i0 - (lane >> 4) < n; i0 += 2 * kRowWarps * kRowKeys) {      // whole warps go round together
+    uint4 kr[kRowKeys], vr[kRowKeys];
+#pragma unroll
+    for (int u = 0; u < kRowKeys; ++u) {
+      const int i = i0 + u * 2 * kRowWarps;
+      kr[u] = zero; vr[u] = zero;
+      if (i < n) {
+        const int j = i < nk ? i : lo + (i - nk);
+        const long long row = page_shift >= 0 ? (static_cast<long long>(bt[j >> page_shift]) << page_shift) + (j & ((1 << page_shift) - 1))
+                                              : static_cast<long long>(bt[j / a.page]) * a.page + j % a.page;
+        if (kin) kr[u] = *reinterpret_cast<const uint4*>(keys + row * crow);
+        if (vin) vr[u] = *reinterpret_cast<const uint4*>(vals + row * crow);
+      }
+    }
+    float sc[GS][kRowKeys];
+#pragma unroll
+    for (int u = 0; u < kRowKeys; ++u) {
+      float k8[8];
+      unpack8(kr[u], k8);
+#pragma unroll
+      for (int h = 0; h < GS; ++h) {
+        float d = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d = fmaf(q[h][e], k8[e], d);
+        sc[h][u] = d;
+      }
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int h = 0; h < GS; ++h)
+#pragma unroll
+        for (int u = 0; u < kRowKeys; ++u) sc[h][u] += __shfl_xor_sync(0xffffffffu, sc[h][u], o);
+#pragma unroll
+    for (int h = 0; h < GS; ++h) {
+      float mn = m[h];
+#pragma unroll
+      for (int u = 0; u < kRowKeys; ++u) {
+        if (a.softcap > 0.f) sc[h][u] = a.softcap * tanhf(sc[h][u] / a.softcap);
+        if (i0 + u * 2 * kRowWarps >= n) sc[h][u] = -FLT_MAX;
+        mn = fmaxf(mn, sc[h][u]);
+      }
+      const float corr = expf(m[h] - mn);
+      m[h] = mn;
+      l[h] *= corr;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[h][e] *= corr;
+#pragma unroll
+      for (int u = 0; u < kRowKeys; ++u) {
+        sc[h][u] = i0 + u * 2 * kRowWarps < n ? expf(sc[h][u] - mn) : 0.f;
+        l[h] += sc[h][u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRowKeys; ++u) {
+      float v8[8];
+      unpack8(vr[u], v8);
+#pragma unroll
+      for (int h = 0; h < GS; ++h)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[h][e] = fmaf(sc[h][u], v8[e], acc[h][e]);
+    }
+  }
+  // the halves of a warp, then the warps in their order
+#pragma unroll
+  for (int h = 0; h < GS; ++h) {
+    const float mo = __shfl_xor_sync(0xffffffffu, m[h], 16), lo_ = __shfl_xor_sync(0xffffffffu, l[h], 16);
+    const float mn = fmaxf(m[h], mo), f0 = m[h] == -FLT_MAX ? 0.f : expf(m[h] - mn), f1 = mo == -FLT_MAX ? 0.f : expf(mo - mn);
+    float* mine = sm + (wrp * GS + h) * (Dv + 2);
+    if (lane == 0) { mine[0] = mn; mine[1] = l[h] * f0 + lo_ * f1; }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float o = __shfl_xor_sync(0xffffffffu, acc[h][e], 16);
+      if (lane < 16 && vin) mine[2 + c0 + e] = acc[h][e] * f0 + o * f1;
+    }
+  }
+  __syncthreads();
+  const bf16* gate = static_cast<const bf16*>(a.gate);
+  for (int x = threadIdx.x; x < GS * Dv; x += kRowWarps * 32) {
+    const int h = x / Dv, c = x - h * Dv, head = h0 + h;
+    const float* pt = sm + h * (Dv + 2);
+    const int step = GS * (Dv + 2);
+    // the sink adds exp(sink) to the denominator and nothing to the numerator; it is taken as it is, outside scale and cap
+    const float sink = a.sink ? a.sink[head] : -FLT_MAX;
+    float mm = sink;
+#pragma unroll
+    for (int w = 0; w < kRowWarps; ++w) mm = fmaxf(mm, pt[w * step]);
+    float ll = a.sink ? expf(sink - mm) : 0.f, o = 0.f;
+#pragma unroll
+    for (int w = 0; w < kRowWarps; ++w) {
+      const float f = pt[w * step] == -FLT_MAX ? 0.f : expf(pt[w * step] - mm);
+      ll = fmaf(pt[w * step + 1], f, ll);
+      o = fmaf(pt[w * step + 2 + c], f, o);
+    }
+    o *= 1.0f / ll;
+    if (gate) o *= sigmoidf_(ldf(gate + t * a.ldg + (a.gate_per_head ? head : static_cast<long long>(head) * Dv + c)));
+    stf(static_cast<bf16*>(a.y) + t * a.ldy + static_cast<long long>(head) * Dv + c, o * a.out_scale);
   }
 }
 
@@ -725,6 +944,15 @@ int rope_table_yarn(float2* table, int max_pos, int dims, double base, const Rop
 int qk_rope_norm_cache(const QkPrepArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   if (a.heads < 1 || a.kv_heads < 1 || a.dim < 1 || a.vdim < 1 || a.rot_dims < 0 || a.rot_dims > a.dim || a.rot_dims % 2 || (a.rot_dims && !a.rope)) return -1;
+  auto piece = [](const void* p, int ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 8 == 0; };
+  if (a.t == DT_BF16 && a.vdim % 8 == 0 && (a.dim == 32 || a.dim == 64 || a.dim == 128 || a.dim == 256) && piece(a.q, a.ld) && piece(a.k, a.ld) && piece(a.v, a.ld) &&
+      piece(a.cache, 0) && piece(a.qn, 0) && piece(a.v_blend, a.v_blend ? a.ld_blend : 0) && piece(a.v_raw_out, a.v_raw_out ? a.ld_raw : 0)) {
+    const int items = (a.heads + a.kv_heads) * (a.dim / 8) + a.kv_heads * a.vdim / 8;
+    const int threads = std::min(a.T >= 256 ? 256 : 512, (items + 31) / 32 * 32);
+    auto run = a.dim == 32 ? qk_prep_vec_kernel<4> : a.dim == 64 ? qk_prep_vec_kernel<8> : a.dim == 128 ? qk_prep_vec_kernel<16> : qk_prep_vec_kernel<32>;
+    launch_pdl(run, a.T, threads, 0, st, a);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   if (a.t == DT_BF16) launch_pdl(qk_prep_kernel<bf16>, a.T, 128, 0, st, a);
   else launch_pdl(qk_prep_kernel<float>, a.T, 128, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -799,6 +1027,22 @@ int window_attention(const WindowAttnArgs& a, cudaStream_t st) {
       cudaFuncSetAttribute(window_attn_mma_kernel<16>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
       launch_pdl(window_attn_mma_kernel<16>, grid, kMmaThreads, smem, st, a, gs, TQ, page_shift);
     }
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  // B200_WATTN_ROWS=0 keeps single tokens on the general kernel (A/B knob)
+  const char* re = getenv("B200_WATTN_ROWS");
+  if (!(re && atoi(re) == 0) && a.t == DT_BF16 && a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && reinterpret_cast<uintptr_t>(a.cache) % 16 == 0) {
+    // as many heads of a group to a CTA as keep every SM busy; the result does not depend on it
+    const int group = a.heads / a.kv_heads;
+    int gs = 1;
+    for (int c = 2; c <= 8; c *= 2)
+      if (group % c == 0 && static_cast<long long>(a.T) * a.heads / c >= 2 * 148) gs = c;
+    int page_shift = -1;
+    for (int b = 0; b < 31; ++b) if ((1 << b) == a.page) page_shift = b;
+    const unsigned grid = static_cast<unsigned>(static_cast<long long>(a.T) * (a.heads / gs));
+    const size_t smem = static_cast<size_t>(kRowWarps) * gs * (a.vdim + 2) * sizeof(float);     // at most 34 KB
+    auto run = gs == 8 ? window_attn_rows_kernel<8> : gs == 4 ? window_attn_rows_kernel<4> : gs == 2 ? window_attn_rows_kernel<2> : window_attn_rows_kernel<1>;
+    launch_pdl(run, grid, kRowWarps * 32, smem, st, a, page_shift);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   const int vl = a.t == DT_BF16 ? 8 : 4;

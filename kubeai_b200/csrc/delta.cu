@@ -17,6 +17,8 @@
 
 #include <algorithm>
 
+#include "griddep.cuh"
+#include "launch.h"
 #include "mixers.h"
 
 namespace b200 {
@@ -147,6 +149,113 @@ __global__ void __launch_bounds__(kThreads) delta_scan_kernel(DeltaArgs a, int P
   }
 }
 
+// Steps in which every sequence brings one token: a pass over the states as in gla.cu's gla_step_kernel, with the sums S^T k and
+// S^T q taken before the write.  A CTA takes 64 value columns of a (head, sequence): sixteen lanes a row in 16-byte pieces, RPT
+// rows a thread, every load in flight at once.  100 sequences of 16 heads of 128 x 128: 74 us in the scan, 37 here.
+constexpr int kStepCols = 64, kStepWarps = 8;
+template <typename T, int RPT>
+__global__ void __launch_bounds__(kStepWarps * 32) delta_step_kernel(DeltaArgs a) {
+  griddep_launch();
+  __shared__ __align__(16) float qs[16 * RPT], ks[16 * RPT];
+  __shared__ __align__(16) float part[2][kStepWarps][kStepCols];
+  __shared__ float sc[3];
+  const int seq = blockIdx.z, head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5, D = a.dim, Dv = a.vdim;
+  const int tok = a.seqs[seq * 8 + 0], pos = a.seqs[seq * 8 + 2], slot = a.seqs[seq * 8 + 3];     // the step's inputs, uploaded before its first kernel
+  const int jc = (tid & 15) * 4, j0 = blockIdx.x * kStepCols + jc, r0 = tid >> 4;
+  const bool live = j0 < Dv, held = pos > 0;
+  float* Sg = a.states + (static_cast<long long>(slot) * a.heads + head) * D * Dv + j0;
+  if (held && live && (tid & 7) == 0)
+    for (int m = 0; m < RPT; ++m)
+      if (r0 + 16 * m < D) asm volatile("prefetch.global.L2 [%0];" ::"l"(Sg + static_cast<long long>(r0 + 16 * m) * Dv));
+  griddep_wait();
+  float4 S[RPT];
+#pragma unroll
+  for (int m = 0; m < RPT; ++m) {
+    const int i = r0 + 16 * m;
+    S[m] = held && live && i < D ? *reinterpret_cast<const float4*>(Sg + static_cast<long long>(i) * Dv) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  auto ld = [](const T* p) { return static_cast<float>(*p); };      // rows that an earlier kernel of the step wrote
+  const T* row = static_cast<const T*>(a.qkv) + static_cast<long long>(tok) * a.ld;
+  if (wrp == 0) {
+    const int g = head / (a.heads / a.kv_heads);
+    const T *q = row + a.q_off + static_cast<long long>(g) * D, *k = row + a.k_off + static_cast<long long>(g) * D;
+    float qq = 0.f, kk = 0.f, qk = 0.f;
+    for (int i = lane; i < D; i += 32) {
+      const float x = ld(q + i), y = ld(k + i);
+      qs[i] = x; ks[i] = y;
+      qq = fmaf(x, x, qq); kk = fmaf(y, y, kk); qk = fmaf(x, y, qk);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      qq += __shfl_xor_sync(0xffffffffu, qq, o);
+      kk += __shfl_xor_sync(0xffffffffu, kk, o);
+      qk += __shfl_xor_sync(0xffffffffu, qk, o);
+    }
+    const float iq = a.q_scale / sqrtf(qq + a.unit_eps), ik = 1.0f / sqrtf(kk + a.unit_eps);
+    for (int i = lane; i < 16 * RPT; i += 32) {
+      qs[i] = i < D ? qs[i] * iq : 0.f;
+      ks[i] = i < D ? ks[i] * ik : 0.f;
+    }
+    if (lane == 0) sc[2] = qk * iq * ik;
+  } else if (tid == 32) {
+    const float b = ld(static_cast<const T*>(a.beta_pre) + static_cast<long long>(tok) * a.ld_gate + head);
+    const float d = softplusf_(ld(static_cast<const T*>(a.dt_pre) + static_cast<long long>(tok) * a.ld_gate + head) + a.dt_bias[head]);
+    sc[0] = expf(a.rate[head] * d);
+    sc[1] = 1.0f / (1.0f + expf(-b));
+  }
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (live) {
+    const T* vp = row + a.v_off + static_cast<long long>(head) * Dv + j0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = ld(vp + e);
+  }
+  __syncthreads();
+  const float decay = sc[0];
+  float sk[4] = {0.f, 0.f, 0.f, 0.f}, sq[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int m = 0; m < RPT; ++m) {
+    const float k = ks[r0 + 16 * m], q = qs[r0 + 16 * m], s4[4] = {S[m].x, S[m].y, S[m].z, S[m].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { sk[e] = fmaf(s4[e], k, sk[e]); sq[e] = fmaf(s4[e], q, sq[e]); }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    sk[e] += __shfl_xor_sync(0xffffffffu, sk[e], 16);
+    sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], 16);
+  }
+  if (lane < 16) {
+    *reinterpret_cast<float4*>(&part[0][wrp][jc]) = make_float4(sk[0], sk[1], sk[2], sk[3]);
+    *reinterpret_cast<float4*>(&part[1][wrp][jc]) = make_float4(sq[0], sq[1], sq[2], sq[3]);
+  }
+  __syncthreads();
+  float u[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float tk = 0.f;
+#pragma unroll
+    for (int w = 0; w < kStepWarps; ++w) tk += part[0][w][jc + e];
+    u[e] = sc[1] * fmaf(-decay, tk, v[e]);
+  }
+  if (r0 == 0 && live) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float tq = 0.f;
+#pragma unroll
+      for (int w = 0; w < kStepWarps; ++w) tq += part[1][w][jc + e];
+      a.o[static_cast<long long>(tok) * (static_cast<long long>(a.heads) * Dv) + static_cast<long long>(head) * Dv + j0 + e] = fmaf(sc[2], u[e], decay * tq);
+    }
+  }
+  if (live) {
+#pragma unroll
+    for (int m = 0; m < RPT; ++m) {
+      const int i = r0 + 16 * m;
+      const float k = ks[i];
+      if (i < D)
+        *reinterpret_cast<float4*>(Sg + static_cast<long long>(i) * Dv) =
+            make_float4(fmaf(k, u[0], decay * S[m].x), fmaf(k, u[1], decay * S[m].y), fmaf(k, u[2], decay * S[m].z), fmaf(k, u[3], decay * S[m].w));
+    }
+  }
+}
+
 }  // namespace
 
 int delta_scan(const DeltaArgs& a, cudaStream_t st) {
@@ -158,6 +267,16 @@ int delta_scan(const DeltaArgs& a, cudaStream_t st) {
     const char* e = getenv("B200_DELTA_CHUNK");
     const int from = e ? atoi(e) : 8;
     if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return delta_chunk(a, st);
+  }
+  // B200_SCAN_STEP=0 keeps single tokens in the scan (A/B knob); fp32 models stay there, whose outputs are promised to be the same
+  // bits however a sequence was cut into steps
+  const char* se = getenv("B200_SCAN_STEP");
+  if (a.t == DT_BF16 && a.T == a.nseq && a.dim <= 256 && a.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(a.states) % 16 == 0 && !(se && atoi(se) == 0)) {
+    dim3 grid((a.vdim + kStepCols - 1) / kStepCols, a.heads, a.nseq);
+    if (a.dim <= 64) launch_pdl(delta_step_kernel<bf16, 4>, grid, kStepWarps * 32, 0, st, a);
+    else if (a.dim <= 128) launch_pdl(delta_step_kernel<bf16, 8>, grid, kStepWarps * 32, 0, st, a);
+    else launch_pdl(delta_step_kernel<bf16, 16>, grid, kStepWarps * 32, 0, st, a);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   int P = 1;
   while (P * 4 * kPieces < a.dim) P <<= 1;

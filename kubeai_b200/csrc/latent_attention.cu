@@ -24,6 +24,7 @@
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
+#include "seq_tiles.cuh"
 
 namespace b200 {
 namespace {
@@ -226,13 +227,8 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(LatentAttnArgs a, 
   float* Ls = Ms + R;
   float* As = Ls + R;
   // which (sequence, token tile) is this CTA's
-  int idx = blockIdx.x, seq = -1, tile = 0;
-  for (int s = 0; s < nseq; ++s) {
-    const int tiles = (seqs[s * 8 + 1] + TQ - 1) / TQ;
-    if (idx < tiles) { seq = s; tile = idx; break; }
-    idx -= tiles;
-  }
-  if (seq < 0) return;
+  int seq, tile;
+  if (!find_tile(seqs, nseq, TQ, blockIdx.x, &seq, &tile)) return;
   const int tok0 = seqs[seq * 8 + 0], n = seqs[seq * 8 + 1], pos0 = seqs[seq * 8 + 2];
   const int tq0 = tile * TQ, ntq = min(TQ, n - tq0);
   const int h0 = blockIdx.y * HB;
@@ -478,13 +474,8 @@ __global__ void __launch_bounds__(256) latent_attn_mma_wide_kernel(LatentAttnArg
   float* Ms = reinterpret_cast<float*>(Ps + R * LDP);         // running max [R], sum [R], rescale [R]
   float* Ls = Ms + R;
   float* As = Ls + R;
-  int idx = blockIdx.x, seq = -1, tile = 0;
-  for (int s = 0; s < nseq; ++s) {
-    const int tiles = (seqs[s * 8 + 1] + TQ - 1) / TQ;
-    if (idx < tiles) { seq = s; tile = idx; break; }
-    idx -= tiles;
-  }
-  if (seq < 0) return;
+  int seq, tile;
+  if (!find_tile(seqs, nseq, TQ, blockIdx.x, &seq, &tile)) return;
   const int tok0 = seqs[seq * 8 + 0], n = seqs[seq * 8 + 1], pos0 = seqs[seq * 8 + 2];
   const int tq0 = tile * TQ, ntq = min(TQ, n - tq0);
   const int h0 = blockIdx.y * HB;

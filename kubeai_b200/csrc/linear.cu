@@ -300,6 +300,8 @@ __device__ __forceinline__ uint4 ldx8(const float* p, uint4* lo) {
   return make_uint4(h[0], h[1], h[2], h[3]);
 }
 
+// More rows than 8 * NB (one product per head, steps of up to 128 tokens): grid row y takes its own 8 * NB, the weights come from L2
+// again.  16 heads, 512 x 128 and 128 x 512, 100 rows: 22 us and 9 on the 64-row tiles below, 9 and 8 here; 40 rows 23 and 9, 7 and 6.
 // THIN: the same with the operands' parts exchanged, for many rows of X against few rows of W (router logits, scalar gates):
 // X streams as the 16-row operand, W's rows 16 y .. 16 y + 15 of grid row y are the "tokens".  One output element is summed in
 // the same order as above.
@@ -311,11 +313,11 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
   const int ks = wrp % KS, RG = 8 / KS;
   const int n0 = (blockIdx.x * RG + wrp / KS) * 16;
   const long long b = blockIdx.z;
-  const int col0 = THIN ? blockIdx.y * 8 * NB : 0;
+  const int col0 = THIN ? blockIdx.y * 8 * NB : 0, row0 = THIN ? 0 : blockIdx.y * 8 * NB;
   // the 16-row operand and its rows, the 8-row operand and its rows
   const bf16* W = THIN ? static_cast<const bf16*>(a.X) : static_cast<const bf16*>(a.W) + b * a.wbs;
-  const TX* X = THIN ? static_cast<const TX*>(a.W) + static_cast<long long>(col0) * a.ldw : static_cast<const TX*>(a.X) + b * a.xbs;
-  const int ldw = THIN ? a.ldx : a.ldw, ldx = THIN ? a.ldw : a.ldx, rows = THIN ? a.T : a.N, toks = THIN ? min(8 * NB, a.N - col0) : a.T;
+  const TX* X = THIN ? static_cast<const TX*>(a.W) + static_cast<long long>(col0) * a.ldw : static_cast<const TX*>(a.X) + b * a.xbs + static_cast<long long>(row0) * a.ldx;
+  const int ldw = THIN ? a.ldx : a.ldw, ldx = THIN ? a.ldw : a.ldx, rows = THIN ? a.T : a.N, toks = min(8 * NB, THIN ? a.N - col0 : a.T - row0);
   TY* Y = static_cast<TY*>(a.Y) + b * a.ybs;
   const bool r0 = n0 + g < rows, r1 = n0 + g + 8 < rows;
   const bf16* w0 = W + static_cast<long long>(n0 + g) * ldw;
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
     if (t >= toks || n >= rows) continue;
     float v = 0.f;
     for (int k = 0; k < KS; ++k) v += part[rg * KS + k][r & 15][t];
-    const int yr = THIN ? n : t, yc = THIN ? col0 + t : n;
+    const int yr = THIN ? n : row0 + t, yc = THIN ? col0 + t : n;
     st1(Y + static_cast<long long>(yr) * a.ldy + yc, finish<TY>(a, a.row_scale ? v * a.row_scale[yr] : v, yc));
   }
 }
@@ -434,10 +436,10 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
     static const int mma_rows = [] { const char* e = getenv("B200_LIN_MMA_ROWS"); return e ? std::min(16, std::max(0, atoi(e))) : 16; }();
     const bool vec = a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.xbs % 8 == 0 && a.wbs % 8 == 0 &&
                      reinterpret_cast<uintptr_t>(a.X) % 16 == 0 && reinterpret_cast<uintptr_t>(a.W) % 16 == 0;
-    if (vec && a.T <= mma_rows && !a.x_rows && !a.tile_group) {
+    if (vec && (a.T <= mma_rows || (a.batch > 1 && mma_rows == 16 && a.T <= 128)) && !a.x_rows && !a.tile_group) {
       const int steps = (a.K + 31) / 32;
       const int KS = steps >= 32 ? 8 : (steps >= 16 ? 4 : (steps >= 8 ? 2 : 1));
-      dim3 grid((a.N + 128 / KS - 1) / (128 / KS), 1, a.batch);
+      dim3 grid((a.N + 128 / KS - 1) / (128 / KS), a.T <= 8 ? 1 : (a.T + 15) / 16, a.batch);
       constexpr int U = sizeof(TX) == 4 ? 4 : 8;
       if (a.T <= 8) launch_pdl(linear_rows_mma_kernel<TX, TY, 1, U, false>, grid, 256, 0, st, a, KS);
       else launch_pdl(linear_rows_mma_kernel<TX, TY, 2, U / 2, false>, grid, 256, 0, st, a, KS);

@@ -25,6 +25,7 @@
 
 #include "launch.h"
 #include "mixers.h"
+#include "seq_tiles.cuh"
 #include "mma_frag.cuh"
 
 namespace b200 {
@@ -46,30 +47,6 @@ struct Work {
 
 __device__ __forceinline__ float floor_log(float x) { return x < kLowest ? kLowest : x; }   // keeps NaN
 __device__ __forceinline__ float bf(const bf16* p) { return __bfloat162float(__ldg(p)); }
-
-// The sequence and chunk that number `id` is (chunks are numbered sequence by sequence); false past the last one.
-__device__ __forceinline__ bool find_chunk(const int* seqs, int nseq, int id, int* seq, int* chunk) {
-  const int lane = threadIdx.x & 31;
-  int before = 0;
-  for (int s0 = 0; s0 < nseq; s0 += 32) {
-    const int s = s0 + lane, c = s < nseq ? (seqs[s * 8 + 1] + kQ - 1) / kQ : 0;
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, id < before + incl);
-    if (hit) {
-      const int l = __ffs(hit) - 1;
-      *seq = s0 + l;
-      *chunk = id - before - __shfl_sync(0xffffffffu, incl - c, l);
-      return true;
-    }
-    before += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  return false;
-}
 
 // forget gate pre-activation -> (log decay, key); 1 - f keeps its low bits where f is near 1, and f where it is near 0
 __device__ __forceinline__ void forget_gate(float g, float lower, float* la, float* key) {
@@ -128,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_sums_kernel(GlaArgs a, Work
   float* nsum = reinterpret_cast<float*>(half + 2 * kMaxD);  // [2][kMaxD]
   float* gates = nsum + 2 * kMaxD;               // [2][kQ] a scalar gate's log decays and key scales
   int seq, chunk;
-  if (!find_chunk(a.seqs, a.nseq, blockIdx.x, &seq, &chunk)) return;
+  if (!find_tile(a.seqs, a.nseq, kQ, blockIdx.x, &seq, &chunk)) return;
   const int head = blockIdx.y, p0 = blockIdx.z * kCols, D = a.dim, P = a.vdim, HD = a.heads * D;
   const int tok0 = a.seqs[seq * 8] + chunk * kQ, q = min(kQ, a.seqs[seq * 8 + 1] - chunk * kQ);
   const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5, g = lane >> 2, t4 = lane & 3;
@@ -301,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
   extern __shared__ __align__(16) unsigned char smraw[];
   OutSmem& sm = *reinterpret_cast<OutSmem*>(smraw);
   int seq, chunk;
-  if (!find_chunk(a.seqs, a.nseq, blockIdx.x, &seq, &chunk)) return;
+  if (!find_tile(a.seqs, a.nseq, kQ, blockIdx.x, &seq, &chunk)) return;
   const int head = blockIdx.y, p0 = blockIdx.z * kCols, D = a.dim, P = a.vdim, HD = a.heads * D, nk = D / 16;
   const int tok0 = a.seqs[seq * 8] + chunk * kQ, q = min(kQ, a.seqs[seq * 8 + 1] - chunk * kQ);
   const bool has_state = chunk > 0 || a.seqs[seq * 8 + 2] > 0;

@@ -31,6 +31,7 @@
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
+#include "seq_tiles.cuh"
 
 namespace b200 {
 namespace {
@@ -672,14 +673,10 @@ __global__ void __launch_bounds__(kMmaThreads, kMmaCtasPerSm) window_attn_mma_ke
   bf16* Vs = Ks + kTileKeys * LDK;                           // [64][LDV]
   const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   // which sequence and which tile of it
-  int tile = blockIdx.x, s = 0, n = 0;
-  for (; s < a.nseq; ++s) {
-    n = a.seqs[s * 8 + 1];
-    const int nt = (n + TQ - 1) / TQ;
-    if (tile < nt) { tile = nt - 1 - tile; break; }   // a sequence's last tiles see the most keys: they start first
-    tile -= nt;
-  }
-  if (s >= a.nseq) return;
+  int tile, s;
+  if (!find_tile(a.seqs, a.nseq, TQ, blockIdx.x, &s, &tile)) return;
+  const int n = a.seqs[s * 8 + 1];
+  tile = (n + TQ - 1) / TQ - 1 - tile;   // a sequence's last tiles see the most keys: they start first
   const int tok0 = a.seqs[s * 8] + tile * TQ, ntq = min(TQ, n - tile * TQ);
   const int p0 = a.seqs[s * 8 + 2] + tile * TQ, p1 = p0 + ntq - 1;
   const int hy = blockIdx.y;                                // group of query heads

@@ -11,7 +11,12 @@
 // operand (state, weighted scores, weighted x) needs more than one bf16 term, and it is split into three, 24 bits
 // (mma_frag.cuh).  The result differs from the token-by-token scan by fp32 rounding alone.
 //
-// One CTA owns 64 value columns of a (head, sequence) and walks its chunks: 4 warps, each with 16 value columns.  The state
+// Few long sequences leave most of the device to a chain of chunks on few CTAs.  They are cut into segments of kSegment
+// tokens: the sums of all segments at once (PART_SUMS), a pass that turns them into incoming states, the outputs of all segments at
+// once (PART_OUT).  64 heads of 128 x 64, 3 sequences of 455, 1365 and 2275 tokens: one chain each (PART_ALL) 460 us, segments 270.
+// The sums cost a third of the products again, so sequences enough to fill the device stay whole (segments_pay).
+//
+// One CTA owns 64 value columns of a (head, sequence or segment) and walks its chunks: 4 warps, each with 16 value columns.  The state
 // lives transposed (value columns x state rows) in the warps' accumulators, which are the left operand of the next chunk's
 // y without leaving the registers; the scores B C^T are computed 16 rows per warp and shared through shared memory.
 #include <cuda_bf16.h>
@@ -24,6 +29,7 @@
 #include "launch.h"
 #include "mixers.h"
 #include "mma_frag.cuh"
+#include "seq_tiles.cuh"
 
 namespace b200 {
 namespace {
@@ -40,9 +46,16 @@ size_t chunk_smem(int N) {
   return static_cast<size_t>(2) * kQ * (N + 8) * 2 + static_cast<size_t>(kQ) * kLdX * 2 + 3ull * kQ * kLdM * 2 + 4 * kQ * sizeof(float);
 }
 
+enum Part { PART_ALL = 0, PART_SUMS, PART_OUT };
+constexpr int kSegment = 256;
+// of every segment and head: its sums [dim][vdim], then the state in front of it; the decay over it
+struct Segments {
+  float *s, *d;
+};
+
 // NK: state rows in units of 16, at most (N = a.dim is any multiple of 16 up to 16 NK)
-template <int NK>
-__global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a) {
+template <int NK, int PART>
+__global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a, Segments sg) {
   using namespace frag;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int N = a.dim, P = a.vdim, nk = N / 16, LDN = N + 8;
@@ -54,13 +67,18 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
   float* ecum = cum + kQ;                        // [kQ] exp(c_t)
   float* dts = ecum + kQ;                        // [kQ] d_t (0 past the portion)
   float* wts = dts + kQ;                         // [kQ] exp(c_last - c_t) d_t
-  const int seq = blockIdx.z, head = blockIdx.y, p0 = blockIdx.x * kCols;
-  const int tok0 = a.seqs[seq * 8 + 0], n = a.seqs[seq * 8 + 1], pos0 = a.seqs[seq * 8 + 2], slot = a.seqs[seq * 8 + 3];
+  const int head = blockIdx.y, p0 = (PART == PART_ALL ? blockIdx.x : blockIdx.z) * kCols;
+  int seq = blockIdx.z, segment = 0;
+  if (PART != PART_ALL && !find_tile(a.seqs, a.nseq, kSegment, blockIdx.x, &seq, &segment)) return;
+  const int tok0 = a.seqs[seq * 8 + 0] + segment * kSegment, pos0 = a.seqs[seq * 8 + 2] + segment * kSegment, slot = a.seqs[seq * 8 + 3];
+  const int n = PART == PART_ALL ? a.seqs[seq * 8 + 1] : min(kSegment, a.seqs[seq * 8 + 1] - segment * kSegment);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t4 = lane & 3;
   const bf16* base = static_cast<const bf16*>(a.qkv);
   const int qk0 = (head / a.group) * N;
   const bool live = p0 + 16 * w < P;             // warps past the last value column only help with the scores
-  float* Sg = a.states + (static_cast<long long>(slot) * a.heads + head) * N * P;
+  float* Sg = PART == PART_ALL ? a.states + (static_cast<long long>(slot) * a.heads + head) * N * P
+                               : sg.s + (static_cast<long long>(blockIdx.x) * a.heads + head) * N * P;
+  float total = 0.f;                             // log decay over the segment
   const int pr[2] = {p0 + 16 * w + g, p0 + 16 * w + g + 8};
   float S[NK][2][4];                             // [16 state rows][half][c]: value column pr[c / 2], state row 16 k + 8 half + 2 t4 + c % 2
 #pragma unroll
@@ -70,7 +88,7 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int nn = 16 * k + 8 * h + 2 * t4 + (c & 1), p = pr[c >> 1];
-        S[k][h][c] = (k < nk && p < P && pos0 > 0) ? Sg[static_cast<long long>(nn) * P + p] : 0.f;
+        S[k][h][c] = (PART != PART_SUMS && k < nk && p < P && pos0 > 0) ? Sg[static_cast<long long>(nn) * P + p] : 0.f;
       }
   const float rate = a.dt_rate[head], dbias = a.dt_bias[head];
   const int npiece = N / 8, xpiece = kCols / 8;
@@ -85,10 +103,10 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
       if (t < q) {
         const bf16* r = rows + static_cast<long long>(t) * a.ld + qk0 + c;
         cp_async16(smem_addr(db), r + a.k_off);
-        cp_async16(smem_addr(dc), r + a.q_off);
+        if (PART != PART_SUMS) cp_async16(smem_addr(dc), r + a.q_off);
       } else {
         *reinterpret_cast<uint4*>(db) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(dc) = make_uint4(0, 0, 0, 0);
+        if (PART != PART_SUMS) *reinterpret_cast<uint4*>(dc) = make_uint4(0, 0, 0, 0);
       }
     }
     for (int e = tid; e < kQ * xpiece; e += kThreads) {
@@ -113,6 +131,7 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
         if (lane >= o) run += v;
       }
       const float last = __shfl_sync(0xffffffffu, run, 31);
+      total += last;
       const float before = __shfl_up_sync(0xffffffffu, run, 1);
       const float cc[2] = {(lane ? before : 0.f) + s[0], run};
 #pragma unroll
@@ -128,7 +147,7 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
     __syncthreads();
 
     // ---- weighted scores: this warp's 16 keys j against the tokens t >= j's block
-    {
+    if (PART != PART_SUMS) {
       float G[4][2][4];
 #pragma unroll
       for (int tb = 0; tb < 4; ++tb)
@@ -171,8 +190,8 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
             }
         }
       }
+      __syncthreads();
     }
-    __syncthreads();
 
     if (live) {
       // ---- y^T [16 value columns x 64 tokens]: the state's part, scaled per token, then the chunk's own
@@ -185,7 +204,7 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
           for (int c = 0; c < 4; ++c) Y[tb][h][c] = 0.f;
 #pragma unroll
       for (int k = 0; k < NK; ++k) {
-        if (k < nk) {
+        if (PART != PART_SUMS && k < nk) {
           uint32_t s0[4], s1[4], s2[4];
           split3(S[k][0][0], S[k][0][1], &s0[0], &s1[0], &s2[0]);
           split3(S[k][0][2], S[k][0][3], &s0[1], &s1[1], &s2[1]);
@@ -225,7 +244,7 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
         ldsm_x4_trans(xf, at_addr(Xs, kLdX, 16 * jb, 16 * w, lane));
 #pragma unroll
         for (int tb = 0; tb < 4; ++tb) {
-          if (tb >= jb) {
+          if (PART != PART_SUMS && tb >= jb) {
 #pragma unroll
             for (int s = 2; s >= 0; --s) {
               uint32_t b[4];
@@ -256,6 +275,7 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
           }
         }
       }
+      if (PART == PART_SUMS) continue;
       float* out = a.o + static_cast<long long>(tok0 + c0) * (a.heads * P) + head * P;
 #pragma unroll
       for (int tb = 0; tb < 4; ++tb)
@@ -268,6 +288,8 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
           }
     }
   }
+  if (PART == PART_SUMS && p0 == 0 && tid == 0) sg.d[static_cast<long long>(blockIdx.x) * a.heads + head] = expf(total);
+  if (PART == PART_OUT) return;
 #pragma unroll
   for (int k = 0; k < NK; ++k)
 #pragma unroll
@@ -279,16 +301,75 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a)
       }
 }
 
+// grid (four state entries a thread, heads, sequences): each segment's sums replaced by the state in front of it, S <- d S + sums
+__global__ void __launch_bounds__(256) segment_states_kernel(GlaArgs a, Segments sg) {
+  const int seq = blockIdx.z, head = blockIdx.y, NP = a.dim * a.vdim, lane = threadIdx.x & 31;
+  int first = 0;
+  for (int s0 = 0; s0 < seq; s0 += 32) {
+    int c = s0 + lane < seq ? (a.seqs[(s0 + lane) * 8 + 1] + kSegment - 1) / kSegment : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    first += c;
+  }
+  const int e = (blockIdx.x * 256 + threadIdx.x) * 4, segs = (a.seqs[seq * 8 + 1] + kSegment - 1) / kSegment, slot = a.seqs[seq * 8 + 3];
+  if (e >= NP || segs <= 0) return;
+  const bool old = a.seqs[seq * 8 + 2] > 0;
+  float4* state = reinterpret_cast<float4*>(a.states + (static_cast<long long>(slot) * a.heads + head) * NP + e);
+  float4 s = old ? *state : make_float4(0.f, 0.f, 0.f, 0.f);
+  constexpr int U = 4;      // segments in flight
+  for (int i = 0; i < segs; i += U) {
+    float4 t[U];
+    float d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u < segs) {
+        const long long r = static_cast<long long>(first + i + u) * a.heads + head;
+        t[u] = *reinterpret_cast<const float4*>(sg.s + r * NP + e);
+        d[u] = sg.d[r];
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u < segs) {
+        *reinterpret_cast<float4*>(sg.s + (static_cast<long long>(first + i + u) * a.heads + head) * NP + e) = s;
+        s = make_float4(fmaf(d[u], s.x, t[u].x), fmaf(d[u], s.y, t[u].y), fmaf(d[u], s.z, t[u].z), fmaf(d[u], s.w, t[u].w));
+      }
+  }
+  *state = s;
+}
+
+template <int NK, int PART>
+int launch_part(const GlaArgs& a, const Segments& sg, dim3 grid, cudaStream_t st) {
+  static std::atomic<unsigned long long> attr{0};
+  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK, PART>, static_cast<int>(chunk_smem(16 * NK)), &attr)) return -2;
+  scalar_decay_chunk_kernel<NK, PART><<<grid, kThreads, chunk_smem(a.dim), st>>>(a, sg);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+// Segments where the chains of whole sequences would leave SMs idle, and their workspace is there.
+bool segments_pay(const GlaArgs& a) {
+  const char* e = getenv("B200_SCAN_SEGMENTS");      // A/B knob: 0 = never, 1 = wherever they fit
+  const int force = e ? atoi(e) : -1;
+  if (force == 0 || !a.par_ws || scan_segments_ws_floats(a.T, a.nseq, a.heads, a.dim, a.vdim) > a.par_ws_floats || a.vdim % 4 ||
+      (reinterpret_cast<uintptr_t>(a.par_ws) | reinterpret_cast<uintptr_t>(a.states)) % 16) return false;
+  return force == 1 || (a.T >= 2 * kSegment * a.nseq && a.nseq <= 6);
+}
 template <int NK>
 int launch(const GlaArgs& a, cudaStream_t st) {
-  static std::atomic<unsigned long long> attr{0};
-  const size_t smem = chunk_smem(a.dim);
-  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK>, static_cast<int>(chunk_smem(16 * NK)), &attr)) return -2;
-  scalar_decay_chunk_kernel<NK><<<dim3((a.vdim + kCols - 1) / kCols, a.heads, a.nseq), kThreads, smem, st>>>(a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  const int cb = (a.vdim + kCols - 1) / kCols;
+  Segments sg = {nullptr, nullptr};
+  if (!segments_pay(a)) return launch_part<NK, PART_ALL>(a, sg, dim3(cb, a.heads, a.nseq), st);
+  const int segs = a.T / kSegment + a.nseq;
+  sg.s = a.par_ws;
+  sg.d = sg.s + static_cast<size_t>(segs) * a.heads * a.dim * a.vdim;
+  if (const int rc = launch_part<NK, PART_SUMS>(a, sg, dim3(segs, a.heads, cb), st)) return rc;
+  segment_states_kernel<<<dim3((a.dim * a.vdim / 4 + 255) / 256, a.heads, a.nseq), 256, 0, st>>>(a, sg);
+  return launch_part<NK, PART_OUT>(a, sg, dim3(segs, a.heads, cb), st);
 }
 
 }  // namespace
+
+size_t scan_segments_ws_floats(int tokens, int seqs, int heads, int dim, int vdim) {
+  return (static_cast<size_t>(tokens) / kSegment + seqs) * heads * (static_cast<size_t>(dim) * vdim + 1);
+}
 
 bool scan_chunk_fits(const GlaArgs& a) {
   auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };

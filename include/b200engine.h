@@ -377,7 +377,8 @@ int b200_op_kernel_mark(int32_t set);
 /* Same contraction, but the GEMM only dumps fp32 stream-K partials and a second kernel reduces them to bf16 —
  * the engine's T <= 512 path (there the reduction is fused into the consumer kernels). */
 int b200_op_gemm_deferred(const void* w, const void* x, void* out, int32_t N, int32_t T, int32_t K, void* stream);
-/* A few rows of x against w as one pass over the weights (csrc/linear_stream.cu): bf16 x [T, K] and w [N, K] (rows ldx, ldw
+/* A few rows of x against w as one pass over the weights (csrc/linear_stream.cu), or up to 256 rows against a matrix of about 1000
+ * to 3000 rows with K cut over clusters (csrc/linear_cluster.cu, act 0 to 2): bf16 x [T, K] and w [N, K] (rows ldx, ldw
  * apart), y [T, .] rows ldy apart, bf16 or fp32 (y_f32).  act 0: y = x w^T + bias; 1: max(.,0)^2; 2: xIELU with p0, p1;
  * 3: gated units of rows that alternate in blocks of 64 gate and 64 up rows (limit p0, slope p1, up offset p2), y [T, N / 2];
  * 4: silu(gate) up of the same rows.  B200_ERR_INVALID for sizes it does not serve.  w is read ahead of the kernel in front. */

@@ -28,6 +28,7 @@ SOURCES = [
     "elementwise.cu",
     "linear.cu",
     "linear_stream.cu",
+    "linear_cluster.cu",
     "norm_act.cu",
     "gla.cu",
     "scan_chunk.cu",

@@ -93,18 +93,20 @@ const char* b200_version(void) { return "kubeai-b200 0.1.0 sm_100a"; }
 int b200_op_linear_rows(const void* x, const void* w, void* y, const float* bias, int32_t T, int32_t N, int32_t K, int32_t ldx, int32_t ldw,
                         int32_t ldy, int32_t y_f32, int32_t act, float p0, float p1, float p2, void* stream) {
   if (int rc = require_device()) return rc;
-  LinearArgs a = linear_args(x, DT_BF16, w, DT_BF16, y, y_f32 ? DT_F32 : DT_BF16, T, N, K);
+  if (ensure_scratch()) { set_error("workspace allocation failed"); return B200_ERR_OOM; }
+  if (int rc = report_mark()) return rc;
+  LinearArgs a = linear_args(x, DT_BF16, w, DT_BF16, y, y_f32 ? DT_F32 : DT_BF16, T, N, K, g_mark);
   a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.bias = bias;
   LinearPairs q;
   q.kind = act == 4 ? PAIRS_SILU : PAIRS_GATED;
   q.limit = p0; q.slope = p1; q.up_offset = p2;
   if (act < 3) { a.act = act == 1 ? LIN_RELU2 : act == 2 ? LIN_XIELU : LIN_NONE; a.a_pos = p0; a.a_neg = p1; }
-  if (!x || !w || !y || act < 0 || act > 4 || ldx < K || ldw < K || ldy < (act < 3 ? N : N / 2) || !linear_streams(a, act < 3 ? nullptr : &q)) {
+  if (!x || !w || !y || act < 0 || act > 4 || ldx < K || ldw < K || ldy < (act < 3 ? N : N / 2) || !(act < 3 ? linear_few(a) : linear_streams(a, &q))) {
     set_error("b200_op_linear_rows: not served (T=%d N=%d K=%d act=%d)", T, N, K, act);
     return B200_ERR_INVALID;
   }
-  const int rc = linear_stream(a, act < 3 ? nullptr : &q, static_cast<cudaStream_t>(stream));
-  return rc ? cuda_fail("linear_stream", rc) : 0;
+  const int rc = act < 3 ? linear(a, static_cast<cudaStream_t>(stream)) : linear_stream(a, &q, static_cast<cudaStream_t>(stream));
+  return rc ? cuda_fail("b200_op_linear_rows", rc) : 0;
 }
 
 int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, int32_t K, void* stream) {

@@ -595,8 +595,8 @@ class Dabodra : public Model {
   }
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
     if (takes_whole(tc, T)) return run_whole(plan, xm, false, Y, N, T);
-    const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
-    if (tc && T > few_rows && !linear_streams(la)) {
+    const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
+    if (tc && T > few_rows && !linear_few(la)) {
       const int bn = gemm_block_n_for(T);
       return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
     }

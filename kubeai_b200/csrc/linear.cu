@@ -6,7 +6,7 @@
 //
 // Kernels: a 64 x 64 x 32 shared-memory tile kernel (fp32 weights: FMA, k ascending; bf16 weights: mma.sync tensor-core
 // products; either way one output element is accumulated in an order that does not depend on what else is in the batch), and
-// two kernels for the few rows of a decode step that linear_stream.cu does not take (one product per head, fp32 rows): up to
+// two kernels for the few rows of a decode step that linear_stream.cu and linear_cluster.cu do not take (one product per head, fp32 rows): up to
 // 16 rows of a bf16 matrix whose rows are whole 16-byte pieces go through mma.sync with the weights as the 16-row operand
 // (every weight byte is loaded once, straight into fragments), anything else of up to 8 rows through one warp per output row.
 // Many rows against up to 64 columns take the fragment kernel with the operands exchanged.
@@ -495,6 +495,7 @@ int linear(const LinearArgs& a, cudaStream_t st) {
   if (!a.X || !a.W || !a.Y || a.K <= 0 || a.batch < 1) return -1;
   if (a.tile_group && a.T % BM) return -1;
   if (linear_streams(a)) return linear_stream(a, nullptr, st);
+  if (linear_clusters(a)) return linear_cluster(a, st);
   const int key = (a.tx == DT_F32 ? 4 : 0) | (a.tw == DT_F32 ? 2 : 0) | (a.ty == DT_F32 ? 1 : 0);
   switch (key) {
     case 0: return launch_linear<bf16, bf16, bf16>(a, st);

@@ -17,16 +17,15 @@
 
 #include <algorithm>
 
-#include "activations.cuh"
 #include "griddep.cuh"
 #include "launch.h"
+#include "linear_finish.cuh"
 #include "mixers.h"
-#include "ptx.cuh"
 
 namespace b200 {
 namespace {
 
-typedef __nv_bfloat16 bf16;
+using namespace linfin;
 constexpr int kPiece = 64;     // values of K in one stage: a 128-byte line of a row
 
 __device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes) {
@@ -43,8 +42,6 @@ __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void put(float* p, float v) { *p = v; }
-__device__ __forceinline__ void put(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
 constexpr int kWarps = 8;
 // The shape of a launch: tokens in blocks of 8 (NB), 16-row blocks of W in a stage (MT).  A warp's ring has as many stages as
@@ -59,39 +56,6 @@ template <int NB, int MT> struct Layout {
   static_assert(kStages >= 2, "a ring of at least two stages");
   static constexpr int kRing = kWarps * kStages * kStage, kBytes = kRing + kPart;
 };
-// In the paired form rows i and i + 64 of every 128 of W belong together (gate and up rows of the same outputs, the two halves
-// of a head): a CTA takes them as neighbours, row n of this order being row_of_pair(n) of W.
-__device__ __forceinline__ int row_of_pair(int n) { const int p = n >> 1; return p + (p & ~63) + ((n & 1) << 6); }
-
-__device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-// Both rows of pair p of token t, rounded to bf16, to their output; the arithmetic is that of gemm_grouped.cu's gated epilogues
-// and of elementwise.cu's rope_kv_kernel.
-__device__ __forceinline__ void finish_pair(const LinearArgs& a, const LinearPairs& q, int t, int p, float x, float y) {
-  bf16* Y = static_cast<bf16*>(a.Y) + static_cast<long long>(t) * a.ldy;
-  if (q.kind == PAIRS_GATED) Y[p] = __float2bfloat16_rn(gated_unit<false>(x, y, q.limit < INFINITY, q.limit, q.slope, q.up_offset));
-  else if (q.kind == PAIRS_SILU) Y[p] = __float2bfloat16_rn(__bfloat162float(silu_bf16(x)) * y);
-  else {
-    const int head = p >> 6, i = p & 63, slot = q.slots[t];
-    bf16* dst = Y + head * 128 + i;
-    if (head >= q.heads) {     // a key or value head: its row of the page, and nothing for a token without one
-      if (slot < 0) return;
-      const long long page = static_cast<long long>(q.kv_heads) * 16 * 128;
-      const int kv_head = head - q.heads, value = kv_head >= q.kv_heads;
-      dst = static_cast<bf16*>(q.kv_layer) + (2 * static_cast<long long>(slot >> 4) + value) * page + ((kv_head - (value ? q.kv_heads : 0)) * 16 + (slot & 15)) * 128 + i;
-    }
-    if (head < q.heads + q.kv_heads) {
-      const int pos = min(max(q.positions[t], 0), q.max_pos - 1);
-      const bf16* cs = static_cast<const bf16*>(q.cos_sin) + static_cast<long long>(pos) * 128;
-      const float c = __bfloat162float(cs[i]), s = __bfloat162float(cs[64 + i]);
-      const float xc = bf16r(__fmul_rn(x, c)), ys = bf16r(__fmul_rn(y, s)), yc = bf16r(__fmul_rn(y, c)), xs = bf16r(__fmul_rn(x, s));
-      x = xc - ys;
-      y = yc + xs;
-    }
-    dst[0] = __float2bfloat16_rn(x);
-    dst[64] = __float2bfloat16_rn(y);
-  }
-}
-
 // CTA b: rows [b * per_cta, + per_cta) of W in `blocks` blocks of at most `rows` <= 16 MT rows.
 template <typename TY, int NB, int MT, bool PAIRS>
 __global__ void __launch_bounds__(kWarps * 32) linear_stream_kernel(LinearArgs a, LinearPairs q, int per_cta, int rows) {
@@ -216,12 +180,7 @@ __global__ void __launch_bounds__(kWarps * 32) linear_stream_kernel(LinearArgs a
     } else {
       for (int e = threadIdx.x; e < live * a.T; e += kWarps * 32) {
         const int t = e / live, r = e - t * live, n = first + r;
-        float v = sum(t, r);
-        if (a.row_scale) v *= a.row_scale[t];
-        if (a.bias) v += a.bias[n];
-        if (a.act == LIN_RELU2) { v = fmaxf(v, 0.f); v = v * v; }
-        else if (a.act == LIN_XIELU) v = sizeof(TY) == 2 ? xielu_fast(v, a.a_pos, a.a_neg) : xielu(v, a.a_pos, a.a_neg);
-        put(static_cast<TY*>(a.Y) + static_cast<long long>(t) * a.ldy + n, v);
+        put(static_cast<TY*>(a.Y) + static_cast<long long>(t) * a.ldy + n, finish_one<TY>(a, sum(t, r), t, n));
       }
     }
     if (first + rows < n1) __syncthreads();

@@ -596,8 +596,8 @@ class Mulenex : public Model {
   // ------------------------------------------------------------ forward
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K,
               const float* bias = nullptr, int act = LIN_NONE) {
-    LinearArgs a = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
-    if (tc && !linear_streams(a)) {
+    LinearArgs a = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
+    if (tc && !linear_few(a)) {
       const int bn = gemm_block_n_for(T);
       const CUtensorMap& tm = xm[gemm_block_n_index(bn)];
       if ((bias || act != LIN_NONE) && gemm_whole_fits(plan, Y, N)) {

@@ -596,8 +596,8 @@ class Nomanex : public Model {
   // ------------------------------------------------------------ forward
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
     static const int tc_min_t = [] { const char* e = getenv("B200_NX_TC_MIN_T"); return e ? atoi(e) : 1; }();   // A/B knob
-    const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
-    if (tc && T >= tc_min_t && !linear_streams(la)) {
+    const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
+    if (tc && T >= tc_min_t && !linear_few(la)) {
       const int bn = gemm_block_n_for(T);
       return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
     }

@@ -586,8 +586,8 @@ class Soselix : public Model {
     float a_pos = 0.f, a_neg = 0.f;
   };
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K, const Epilogue* ep = nullptr) {
-    LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K);
-    if (tc && T > few_rows && !linear_streams(la)) {
+    LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
+    if (tc && T > few_rows && !linear_few(la)) {
       const int bn = gemm_block_n_for(T);
       if (ep && fuse && gemm_whole_fits(plan, Y, N)) {
         const GroupedOut o = {Y, N, GROUPED_XIELU, ep->bias, ep->a_pos, ep->a_neg};

@@ -284,7 +284,9 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(LinearArgs a) {
 // mma, its second half the second), so no fragment goes through shared memory.  The 8 warps of a CTA are KS slices of K times
 // 8 / KS groups of 16 weight rows; the slices' sums meet in shared memory and are added in a fixed order.  An fp32 X is split
 // into two bf16 terms, x = hi + lo up to 2^-16 of x.  The order of the sums depends on K alone.
+template <bool SPLIT>
 __device__ __forceinline__ uint4 ldx8(const bf16* p, uint4*) { return *reinterpret_cast<const uint4*>(p); }
+template <bool SPLIT>
 __device__ __forceinline__ uint4 ldx8(const float* p, uint4* lo) {
   float v[8];
   ld8(p, v);
@@ -296,18 +298,18 @@ __device__ __forceinline__ uint4 ldx8(const float* p, uint4* lo) {
     h[i] = *reinterpret_cast<const uint32_t*>(&b);
     l[i] = *reinterpret_cast<const uint32_t*>(&r);
   }
-  *lo = make_uint4(l[0], l[1], l[2], l[3]);
+  if (SPLIT) *lo = make_uint4(l[0], l[1], l[2], l[3]);
   return make_uint4(h[0], h[1], h[2], h[3]);
 }
 
 // More rows than 8 * NB (one product per head, steps of up to 128 tokens): grid row y takes its own 8 * NB, the weights come from L2
-// again.  16 heads, 512 x 128 and 128 x 512, 100 rows: 22 us and 9 on the 64-row tiles below, 9 and 8 here; 40 rows 23 and 9, 7 and 6.
+// again; an fp32 X is rounded to one bf16 term, as in the 64-row tiles above that these steps used.  16 heads, 512 x 128 and 128 x 512,
+// 100 rows: 22 us and 9 on the tiles, 9 and 8 here; 40 rows 23 and 9, 7 and 6.
 // THIN: the same with the operands' parts exchanged, for many rows of X against few rows of W (router logits, scalar gates):
 // X streams as the 16-row operand, W's rows 16 y .. 16 y + 15 of grid row y are the "tokens".  One output element is summed in
 // the same order as above.
-template <typename TX, typename TY, int NB, int U, bool THIN>
+template <typename TX, typename TY, int NB, int U, bool THIN, bool SPLIT = sizeof(TX) == 4>
 __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int KS) {
-  constexpr bool SPLIT = sizeof(TX) == 4;
   __shared__ float part[8][16][8 * NB + 1];   // [warp][weight row][token]
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
   const int ks = wrp % KS, RG = 8 / KS;
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(LinearArgs a, int 
       for (int i = 0; i < NB; ++i) {
         xv[u][i] = zero;
         if (SPLIT) xl[u][i] = zero;
-        if (in && xin[i]) xv[u][i] = ldx8(xr[i] + k, &xl[u][SPLIT ? i : 0]);
+        if (in && xin[i]) xv[u][i] = ldx8<SPLIT>(xr[i] + k, &xl[u][SPLIT ? i : 0]);
       }
     }
 #pragma unroll
@@ -441,7 +443,8 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
       const int KS = steps >= 32 ? 8 : (steps >= 16 ? 4 : (steps >= 8 ? 2 : 1));
       dim3 grid((a.N + 128 / KS - 1) / (128 / KS), a.T <= 8 ? 1 : (a.T + 15) / 16, a.batch);
       constexpr int U = sizeof(TX) == 4 ? 4 : 8;
-      if (a.T <= 8) launch_pdl(linear_rows_mma_kernel<TX, TY, 1, U, false>, grid, 256, 0, st, a, KS);
+      if (a.T > 16) launch_pdl(linear_rows_mma_kernel<TX, TY, 2, 4, false, false>, grid, 256, 0, st, a, KS);
+      else if (a.T <= 8) launch_pdl(linear_rows_mma_kernel<TX, TY, 1, U, false>, grid, 256, 0, st, a, KS);
       else launch_pdl(linear_rows_mma_kernel<TX, TY, 2, U / 2, false>, grid, 256, 0, st, a, KS);
       return cudaGetLastError() == cudaSuccess ? 0 : -2;
     }

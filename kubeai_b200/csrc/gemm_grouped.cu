@@ -13,7 +13,7 @@
 // takes as many stages as fit beside the output staging.
 // Work items run expert by expert, weight tile by weight tile with its row tiles side by side, so that neighbouring pairs use
 // one weight slab at the same time, and are dealt to the pairs in turn.  Per CTA: one producer thread (TMA: its own 128
-// weight rows and its half of the row tile), one issuing thread in the leader, four epilogue warps that drain one of two
+// weight rows and its half of the row tile), one issuing thread in the leader, four or eight epilogue warps that drain one of two
 // accumulators while the other is being filled.  Every wait has an iteration limit: a pair that gives up stops its work, sets
 // an error flag for the host, and still meets its peer before the tensor memory is freed.
 #include <cuda.h>
@@ -36,10 +36,15 @@ typedef __nv_bfloat16 bf16;
 constexpr int kSlab = 128;      // weight rows per CTA
 constexpr int kRows = 256;      // rows of X per tile, at most; TMEM columns of one accumulator
 constexpr int kBlockK = 64, kUmmaK = 16;
-constexpr int kThreads = 192;
+// A warp that loads, one that issues the products, and one or two groups of four that drain a tile's rows in turns.  Two where
+// the drain of one group outlasts the next tile's products: gated units with the accurate functions (4096 tokens, 16 experts of 4096 x
+// 2048, two a token: 133 us with one group, 122 with two; one such matrix for all 70 and 58; of 500 tokens with K cut, 27 and 21) and
+// the sums of two terms (34, 28).  The others keep one, whose rounds of 64 rows pass fewer barriers (Llama's gated product of 2048 tokens 310 us, 317 with two).
+__host__ __device__ constexpr int groups_of(int epi) { return epi == 1 || epi == 6 ? 2 : 1; }
+__host__ __device__ constexpr int threads_of(int epi) { return 64 + groups_of(epi) * 128; }
 constexpr int kABytes = kSlab * kBlockK * 2;
 constexpr int kRingBytes = 6 * (kABytes + kRows / 2 * kBlockK * 2), kMaxStages = 10;
-constexpr int kOutRows = 64;    // rows of X per epilogue round (32 with fp32 output: the same bytes)
+constexpr int kOutRows = 64;    // rows of X in the output staging, twice: an epilogue round of one group (32 rows with fp32 output), or of two
 constexpr int kOutBytes = kOutRows * kSlab * 2;
 constexpr int kSmem = 1024 + kRingBytes + 256 + 2 * kOutBytes;
 __host__ __device__ constexpr int stage_bytes(int box) { return kABytes + box * kBlockK * 2; }
@@ -102,18 +107,21 @@ __device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
-// whether all 128 epilogue threads say yes (they also meet here)
+template <int EPI>
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(groups_of(EPI) * 128) : "memory"); }
+// whether all epilogue threads say yes (they also meet here)
+template <int EPI>
 __device__ __forceinline__ bool all_epilogue(bool v) {
   uint32_t r;
   asm volatile(
       "{\n"
       ".reg .pred p, q;\n"
       "setp.ne.u32 p, %1, 0;\n"
-      "barrier.cta.red.and.pred q, 2, 128, p;\n"
+      "barrier.cta.red.and.pred q, 2, %2, p;\n"
       "selp.u32 %0, 1, 0, q;\n"
       "}\n"
       : "=r"(r)
-      : "r"(v ? 1u : 0u)
+      : "r"(v ? 1u : 0u), "n"(groups_of(EPI) * 128)
       : "memory");
   return r != 0;
 }
@@ -152,7 +160,7 @@ __device__ __forceinline__ void store8(bf16* p, const float* v) {
 template <int EPI>
 __device__ __forceinline__ void finish_rows(const float* sums, int step, int parts, int n, int row0, int n0, int N, const GroupedOut& o, int et) {
   constexpr int kPieces = gates<EPI> ? 8 : 16;
-  for (int it = et; it < n * kPieces; it += 128) {
+  for (int it = et; it < n * kPieces; it += groups_of(EPI) * 128) {
     const int j = it / kPieces, c = (it % kPieces) * 8;
     const float* p = sums + j * kSlab + c;
     const size_t r = row0 + j;
@@ -199,12 +207,12 @@ __device__ __forceinline__ void finish_parts(float* ring, const float* first, si
   for (int r0 = 0; r0 < t.rows; r0 += chunk) {
     const int n = min(chunk, t.rows - r0);
     for (int k = 0; k < parts; ++k)
-      for (int it = et; it < n * (kSlab / 4); it += 128)
+      for (int it = et; it < n * (kSlab / 4); it += groups_of(EPI) * 128)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sring + (k * sstep + it * 4) * 4), "l"(first + k * step + r0 * kSlab + it * 4) : "memory");
     asm volatile("cp.async.wait_all;" ::: "memory");
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    epilogue_sync<EPI>();
     finish_rows<EPI>(ring, sstep, parts, n, t.row0 + r0, n0, N, o, et);
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    epilogue_sync<EPI>();
   }
 }
 
@@ -215,9 +223,10 @@ __device__ __forceinline__ void finish_parts(float* ring, const float* first, si
 // A form of its own for the plain product: looking the activation up per element made its drain a sixth of the launch longer.
 // FULL: 128-row boxes, their sizes known to the compiler.
 template <int EPI, bool FULL>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads_of(EPI), 1)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const int* expert_rows, int experts, int rows,
                     const __grid_constant__ GroupedOut o, int N, int K, int box_rows, const __grid_constant__ SplitK split, int* error) {
+  constexpr int G = groups_of(EPI), kTurn = EPI == 2 ? 32 : kOutRows / G;      // groups, rows of a round
   const int box = FULL ? 128 : box_rows, stages = stages_for(box);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -225,7 +234,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   auto full_bar = [&](int s) { return bar_base + 8u * s; };                     // the leader's copy is the live one
   auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };        // both CTAs
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + a); };    // both CTAs
-  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + 2 + a); };   // the leader's copy, 8 arrivals
+  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + 2 + a); };   // the leader's copy
   const uint32_t tmem_slot = bar_base + 8u * (2 * kMaxStages + 4);
   uint8_t* stage_out = smem_raw + (bar_base + 256 - smem_u32(smem_raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -243,7 +252,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   if (warp == 1) {
     if (lane == 0) {
       for (int s = 0; s < stages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-      for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 8); }   // 4 epilogue warps of each CTA
+      for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 8 * G); }   // the epilogue warps of both CTAs
       fence_mbar_init();
     }
     __syncwarp();
@@ -326,13 +335,14 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
       }
     }
   } else {
-    const int q = warp & 3, row = q * 32 + lane, et = threadIdx.x - 64;
+    const int q = warp & 3, row = q * 32 + lane, ea = threadIdx.x - 64, grp = ea >> 7, et = ea & 127;
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(3 + grp) : "memory"); };
     int acc = 0, sbuf = 0;
     uint32_t acc_phase = 0;
     Tile t;
     for (long long item = unit; ok && walk.at(item, &t); item += units) {
       if (!t.rows) continue;
-      ok = all_epilogue(wait_limited(tfull_bar(acc), acc_phase));
+      ok = all_epilogue<EPI>(wait_limited(tfull_bar(acc), acc_phase));
       if (!ok) break;
       tc_fence_after();
       const int n0 = t.n0 + static_cast<int>(rank) * kSlab;    // first column of this CTA's slab in the expert's output
@@ -345,7 +355,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         const size_t slab = static_cast<size_t>(split.tile) * kSlab;
         float* first = split.ws + (static_cast<size_t>(t.id) * split.parts * 2 + rank) * slab;
         float* mine = first + 2 * t.part * slab + row;
-        for (int c0 = 0; c0 < t.rows; c0 += 32) {
+        for (int c0 = 32 * grp; c0 < t.rows; c0 += 32 * G) {
           uint32_t v[32];
           tmem_ld_32x32(taddr + c0, v);
           tmem_ld_wait();
@@ -354,27 +364,26 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             if (c0 + j < t.rows) __stcg(mine + static_cast<size_t>(c0 + j) * kSlab, __uint_as_float(v[j]));
         }
         __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        epilogue_sync<EPI>();
         bool last = false;
-        if (et == 0) {
+        if (ea == 0) {
           last = atomicAdd(split.counters + 2 * t.id + rank, 1) == split.parts - 1;
           if (last) split.counters[2 * t.id + rank] = 0;
           __threadfence();
         }
-        last = !all_epilogue(!last);       // thread 0's answer reaches all
+        last = !all_epilogue<EPI>(!last);       // thread 0's answer reaches all
         if constexpr (EPI != 2)
-          if (last) finish_parts<EPI>(reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))), first, 2 * slab, split.parts, t, n0, N, o, et);
+          if (last) finish_parts<EPI>(reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw))), first, 2 * slab, split.parts, t, n0, N, o, ea);
       }
-      constexpr int kStep = EPI == 2 ? 32 : kOutRows;
-      for (int c0 = 0; whole && c0 < t.rows; c0 += kStep) {
-        const bool two = EPI != 2 && c0 + 32 < t.rows;
-        uint32_t v0[32], v1[EPI == 2 ? 1 : 32];
+      for (int c0 = grp * kTurn; whole && c0 < t.rows; c0 += G * kTurn) {
+        const bool two = kTurn == 64 && c0 + 32 < t.rows;
+        uint32_t v0[32], v1[kTurn == 64 ? 32 : 1];
         tmem_ld_32x32(taddr + c0, v0);
-        if constexpr (EPI != 2) {
+        if constexpr (kTurn == 64) {
           if (two) tmem_ld_32x32(taddr + c0 + 32, v1);
         }
         tmem_ld_wait();
-        uint8_t* stage = stage_out + sbuf * kOutBytes;
+        uint8_t* stage = stage_out + (2 * grp + sbuf) * (kOutBytes / G);
         const int left = t.rows - c0;
         if constexpr (EPI == 2) {
           float* sf = reinterpret_cast<float*>(stage);
@@ -391,13 +400,15 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           };
 #pragma unroll
           for (int j = 0; j < 32; ++j) put(j, v0[j]);
-          if (two) {
+          if constexpr (kTurn == 64) {
+            if (two) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) put(32 + j, v1[j]);
+              for (int j = 0; j < 32; ++j) put(32 + j, v1[j]);
+            }
           }
         }
         // one barrier per round: a thread past it has finished its pass over the buffer staged two rounds ago
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        group_sync();
         if constexpr (EPI == 2) {
           float* dst = static_cast<float*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
           const float* sf = reinterpret_cast<const float*>(stage);
@@ -413,7 +424,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           const bf16* sb = reinterpret_cast<const bf16*>(stage);
           const bool clamp = o.p0 < INFINITY;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < kTurn / 16; ++i) {
             const int it = et + i * 128, j = it >> 3, c = (it & 7) * 8;
             if (j < left && n0 + kSlab <= N) {
               const uint4 g = *reinterpret_cast<const uint4*>(sb + j * kSlab + c), u = *reinterpret_cast<const uint4*>(sb + j * kSlab + 64 + c);
@@ -430,24 +441,20 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           bf16* dst = static_cast<bf16*>(o.y) + static_cast<size_t>(t.row0 + c0) * o.ldy;
           const bf16* sb = reinterpret_cast<const bf16*>(stage);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < kTurn / 8; ++i) {
             const int it = et + i * 128, j = it >> 4, c = (it & 15) * 8;
             if (j < left && n0 + c < N)
               *reinterpret_cast<uint4*>(dst + static_cast<size_t>(j) * o.ldy + n0 + c) = *reinterpret_cast<const uint4*>(sb + j * kSlab + c);
           }
           if (EPI == 6 && rank == 1) {      // one more round for the second terms
             sbuf ^= 1;
-            bf16* s2 = reinterpret_cast<bf16*>(stage_out + sbuf * kOutBytes);
+            bf16* s2 = reinterpret_cast<bf16*>(stage_out + (2 * grp + sbuf) * (kOutBytes / G));
 #pragma unroll
             for (int j = 0; j < 32; ++j) s2[j * kSlab + row] = __float2bfloat16_rn(left_over(__uint_as_float(v0[j])));
-            if (two) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) s2[(32 + j) * kSlab + row] = __float2bfloat16_rn(left_over(__uint_as_float(v1[j])));
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            group_sync();
             bf16* d2 = static_cast<bf16*>(o.y2) + static_cast<size_t>(t.row0 + c0) * (N / 2) + t.n0 / 2;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < kTurn / 8; ++i) {
               const int it = et + i * 128, j = it >> 4, c = (it & 15) * 8;
               if (j < left) *reinterpret_cast<uint4*>(d2 + static_cast<size_t>(j) * (N / 2) + c) = *reinterpret_cast<const uint4*>(s2 + j * kSlab + c);
             }
@@ -497,7 +504,7 @@ int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap
   static std::atomic<unsigned long long> attr[16];
   auto start = [&](auto kernel, int i) {
     if (!ensure_dynamic_smem(kernel, kSmem, &attr[i])) return -2;
-    return launch_pdl(kernel, dim3(2 * units), dim3(kThreads), kSmem, st, tm_w, tm_x, expert_rows, experts, rows, o, N, K, box, split, error) == cudaSuccess ? 0 : -2;
+    return launch_pdl(kernel, dim3(2 * units), dim3(threads_of(i / 2)), kSmem, st, tm_w, tm_x, expert_rows, experts, rows, o, N, K, box, split, error) == cudaSuccess ? 0 : -2;
   };
 #define RUN(E) return box == 128 ? start(gemm_grouped_kernel<E, true>, 2 * E) : start(gemm_grouped_kernel<E, false>, 2 * E + 1)
   if (o.epi == GROUPED_SILU) RUN(5);

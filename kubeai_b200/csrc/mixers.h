@@ -174,11 +174,11 @@ bool scan_chunk_fits(const GlaArgs& a);
 size_t scan_segments_ws_floats(int tokens, int seqs, int heads, int dim, int vdim);
 int scan_chunk(const GlaArgs& a, cudaStream_t st);
 // The form whose chunks run side by side (scan_parallel.cu; same result up to fp32 rounding), likewise chosen by gla_scan; its
-// workspace for steps of up to `tokens` tokens of up to `seqs` sequences (fgate: the HGRN2 form).
-size_t scan_parallel_ws_floats(int tokens, int seqs, int heads, int dim, int vdim, bool fgate);
+// workspace for steps of up to `tokens` tokens of up to `seqs` sequences.
+size_t scan_parallel_ws_floats(int tokens, int seqs, int heads, int dim, int vdim);
 // (the sequences of a step it is chosen for bring 8 tokens and more each; at most 2 GB are asked for)
-inline size_t scan_parallel_ws_cap(int tokens, int slots, int heads, int dim, int vdim, bool fgate) {
-  const size_t need = scan_parallel_ws_floats(tokens, slots < tokens / 8 + 1 ? slots : tokens / 8 + 1, heads, dim, vdim, fgate), most = size_t(1) << 29;
+inline size_t scan_parallel_ws_cap(int tokens, int slots, int heads, int dim, int vdim) {
+  const size_t need = scan_parallel_ws_floats(tokens, slots < tokens / 8 + 1 ? slots : tokens / 8 + 1, heads, dim, vdim), most = size_t(1) << 29;
   return need < most ? need : most;
 }
 bool scan_parallel_fits(const GlaArgs& a);

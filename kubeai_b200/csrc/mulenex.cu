@@ -362,7 +362,7 @@ class Mulenex : public Model {
     size_t aw = 0, sw = 0;
     for (auto& s : spec) {
       if (s.mixer == MIX_ATTENTION && s.dim == 128 && s.vdim == 128) aw = std::max(aw, window_prompt_ws_bytes(env.Tcap, s.heads, s.kv_heads));
-      if (s.mixer == MIX_MLSTM) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim, false));
+      if (s.mixer == MIX_MLSTM) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim));
     }
     if (aw) spare(&attn_ws, aw);
     if (sw && spare(&scan_ws, sw * sizeof(float))) scan_ws_floats = sw;

@@ -386,7 +386,7 @@ class Nomanex : public Model {
     if (dt != DT_BF16) return;
     size_t sw = 0;
     for (auto& s : spec)
-      if (s.mixer == MIX_GLA) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim, false));
+      if (s.mixer == MIX_GLA) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim));
     if (sw && spare(&scan_ws, sw * sizeof(float))) scan_ws_floats = sw;
     if (!use_tc) return;
     const int bns[kGemmNumBlockN] = {32, 64, 128, 256, 512};

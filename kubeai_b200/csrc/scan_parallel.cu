@@ -10,7 +10,13 @@
 // Three launches: the sums over a chunk's own tokens for all (chunk, head) at once, a pass over them that turns each into the
 // chunk's incoming state (elementwise, in place, and the slot's new state), the outputs for all (chunk, head) at once.  The
 // token-by-token form (gla.cu) is a chain as long as the longest sequence on as many CTAs as there are heads and sequences:
-// HGRN2, 16 heads of 128 x 128, 3 sequences of 455 to 2275 tokens took 3255 us there.
+// HGRN2, 16 heads of 128 x 128, 3 sequences of 455 to 2275 tokens took 3255 us there, 226 here (GLA 200, mLSTM 193; 380, 365 and
+// 296 while a thread waited for each token's load before it issued the next one's: two thirds of both kernels' cycles).
+//
+// What bounds it: two CTAs of eight warps an SM (shared memory and registers allow no more) go through phases that each lean on
+// something else: loads, the blocks on the diagonal (issue slots), scores and state (tensor cores, mma.sync: a third of the time
+// at its peak rate).  Cycles of a CTA with a second one beside it, GLA: sums 7.8k loads, 3.4k terms, 7k products and stores; outputs
+// 9.6k loads, 8.2k diagonal, 3.6k carrying, 6.5k scores, 5.3k values, 13k state.  Three CTAs of the first kernel an SM spill: slower.
 //
 // Precision is that of fp32.  No factor is the inverse of a decay: a chunk's four blocks of 16 tokens carry their queries from
 // the block's start and their keys to its end, both with exponents of at most 0, and what lies between two blocks is a third
@@ -22,6 +28,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "launch.h"
 #include "mixers.h"
@@ -42,19 +49,33 @@ constexpr float kLowest = -87.f;            // log decays below it are as good a
 enum Mode { VEC_Z = 0, VEC_FGATE = 1, SCALAR = 2 };
 
 struct Work {
-  float *s, *d, *n, *la;   // [chunk][head][dim][vdim] sums, then incoming states; [chunk][head][dim] decays, normaliser; [T][heads * dim]
+  float *s, *d, *n;   // [chunk][head][dim][vdim] sums, then incoming states; [chunk][head][dim] decays, normaliser
 };
 
 __device__ __forceinline__ float floor_log(float x) { return x < kLowest ? kLowest : x; }   // keeps NaN
-__device__ __forceinline__ float bf(const bf16* p) { return __bfloat162float(__ldg(p)); }
 
-// forget gate pre-activation -> (log decay, key); 1 - f keeps its low bits where f is near 1, and f where it is near 0
+// sigmoid(x) and sigmoid(-x) without a branch, so that the gates of several tokens are under way at once: quotients over
+// d = 1 + e^-|x| from an approximate reciprocal with a Newton step each, whose residuals count what the rounding of d left out
+__device__ __forceinline__ void sigmoids(float x, float* pos, float* neg) {
+  const float e = expf(-fabsf(x)), d = 1.0f + e, dd = e - (d - 1.0f);
+  float r = __fdividef(1.0f, d);
+  r = fmaf(r, fmaf(-dd, r, fmaf(-d, r, 1.0f)), r);
+  float er = e * r;
+  er = fmaf(r, fmaf(-dd, er, fmaf(-d, er, e)), er);
+  *pos = x >= 0.f ? r : er;
+  *neg = x >= 0.f ? er : r;
+}
+// forget gate pre-activation -> (log decay, key); 1 - f keeps its low bits where f is near 1, and f where it is near 0.  There
+// log f is that of the rounded f plus what the rounding left out, (1 - w) - f, over f (Kahan's way to log(1 + x); 1 - f is exact
+// above a half): one logarithm, where two on either side of a branch had every warp take both, one token after the other (a
+// gate 150 cycles of a warp's share of an SM, now 75; against 64 bits both the largest and the mean error are smaller).
 __device__ __forceinline__ void forget_gate(float g, float lower, float* la, float* key) {
-  const float e = expf(-fabsf(g)), r = 1.0f / (1.0f + e), er = e * r;
-  const float hi = g >= 0.f ? r : er, lo = g >= 0.f ? er : r;
+  float hi, lo;
+  sigmoids(g, &hi, &lo);
   const float f = fmaf(1.0f - lower, hi, lower), w = (1.0f - lower) * lo;
   *key = w;
-  *la = floor_log(f > 0.5f ? log1pf(-w) : logf(f));
+  const float left = f > 0.5f ? (1.0f - f) - w : 0.0f;    // over f = 1 - w: times 1 + w + w^2 + w^3
+  *la = floor_log(logf(f) + fmaf(left * w, fmaf(w, 1.0f + w, 1.0f), left));
 }
 // log decay and key scale of a token's scalar gates
 __device__ __forceinline__ void scalar_gate(const GlaArgs& a, long long row, int head, float* la, float* ks) {
@@ -62,12 +83,17 @@ __device__ __forceinline__ void scalar_gate(const GlaArgs& a, long long row, int
   *ks = __ldg(a.tok_kscale + row * a.heads + head);
 }
 
-// z -> log decay in place: inv_tau * logsigmoid(z + bias)
-__global__ void log_decay_kernel(float* z, const float* bias, int HD, float inv_tau, long long total) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const float v = z[i] + bias[i % HD];
-  z[i] = floor_log((fminf(v, 0.f) - log1pf(expf(-fabsf(v)))) * inv_tau);
+// z -> log decay in place: inv_tau * logsigmoid(z + bias); grid (tokens, blocks of 1024 channels)
+__global__ void __launch_bounds__(256) log_decay_kernel(float* z, const float* bias, int HD, float inv_tau) {
+  const int i = (blockIdx.y * 256 + threadIdx.x) * 4;
+  if (i >= HD) return;
+  float4* p = reinterpret_cast<float4*>(z + static_cast<long long>(blockIdx.x) * HD + i);
+  const float4 x = *p;
+  auto decay = [&](float a, int n) {
+    const float v = a + __ldg(bias + i + n);
+    return floor_log((fminf(v, 0.f) - log1pf(expf(-fabsf(v)))) * inv_tau);
+  };
+  *p = make_float4(decay(x.x, 0), decay(x.y, 1), decay(x.z, 2), decay(x.w, 3));
 }
 
 // 64 tokens x 128 columns of values into shared memory; zeros past the portion and past the last column
@@ -78,6 +104,16 @@ __device__ __forceinline__ void fetch_values(const GlaArgs& a, bf16* Vs, int tok
     bf16* d = Vs + t * kLd + c;
     if (t < q && p0 + c < a.vdim) cp_async16(smem_addr(d), base + static_cast<long long>(tok0 + t) * a.ld + c);
     else *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
+  }
+}
+
+// 64 tokens x dim of keys into the first bf16 tile; what is past the portion or the last channel stays unwritten
+__device__ __forceinline__ void fetch_keys(const GlaArgs& a, bf16* Ks, int tok0, int q, int head) {
+  const bf16* base = static_cast<const bf16*>(a.qkv) + a.k_off + (head / a.group) * a.dim;
+  for (int e = threadIdx.x; e < kQ * (kMaxD / 8); e += kThreads) {
+    const int t = e / (kMaxD / 8), c = (e % (kMaxD / 8)) * 8;
+    if (t >= q || c >= a.dim) continue;
+    cp_async16(smem_addr(Ks + t * kLd + c), base + static_cast<long long>(tok0 + t) * a.ld + c);
   }
 }
 
@@ -110,29 +146,33 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_sums_kernel(GlaArgs a, Work
   const int tok0 = a.seqs[seq * 8] + chunk * kQ, q = min(kQ, a.seqs[seq * 8 + 1] - chunk * kQ);
   const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   fetch_values(a, Vs, tok0, q, head, p0);
-  if (MODE == SCALAR) fetch_gates(a, gates, tok0, q, head);
   const int i = tid & (kMaxD - 1), hf = tid / kMaxD;
   const bool ch = i < D;
   float la[kQ / 2], kv[kQ / 2];
+  // every load of the chunk is in flight before the first is waited for: the keys on their way to shared memory, where their
+  // terms go afterwards, the decays to registers
+  fetch_keys(a, Ks, tok0, q, head);
+  if (MODE == VEC_Z) {
+    const float* zp = a.z + static_cast<long long>(tok0) * HD + head * D + (ch ? i : 0);
+#pragma unroll
+    for (int jj = 0; jj < kQ / 2; ++jj) la[jj] = __ldg(zp + static_cast<long long>(min(hf * (kQ / 2) + jj, q - 1)) * HD);
+  }
+  if (MODE == SCALAR) fetch_gates(a, gates, tok0, q, head);
+  cp_async_wait_all();
+  __syncthreads();
   {
-    const bf16* kp = static_cast<const bf16*>(a.qkv) + a.k_off + (head / a.group) * D + i;
+    const bf16* kp = Ks + i;
     const float fb = MODE == VEC_FGATE && ch ? __ldg(a.z_bias + head * D + i) : 0.f, fl = MODE == VEC_FGATE && ch ? __ldg(a.fgate_lower + head * D + i) : 0.f;
     double sum = 0.0;
 #pragma unroll
     for (int jj = 0; jj < kQ / 2; ++jj) {
       const int j = hf * (kQ / 2) + jj;
-      la[jj] = 0.f; kv[jj] = 0.f;
-      if (ch && j < q) {
-        const long long row = tok0 + j;
-        float k = bf(kp + row * a.ld);
-        if (MODE == VEC_Z) la[jj] = __ldg(a.z + row * HD + head * D + i);
-        if (MODE == VEC_FGATE) {
-          forget_gate(k + fb, fl, &la[jj], &k);
-          if (blockIdx.z == 0) w.la[row * HD + head * D + i] = la[jj];
-        }
-        if (MODE == SCALAR) { la[jj] = gates[j]; k *= gates[kQ + j]; }
-        kv[jj] = k * a.k_scale;
-      }
+      const bool in = ch && j < q;
+      float k = __bfloat162float(kp[j * kLd]);
+      if (MODE == VEC_FGATE) forget_gate(k + fb, fl, &la[jj], &k);
+      if (MODE == SCALAR) { la[jj] = gates[j]; k *= gates[kQ + j]; }
+      if (!in) la[jj] = 0.f;
+      kv[jj] = in ? k * a.k_scale : 0.f;
       sum += la[jj];
     }
     half[hf * kMaxD + i] = sum;
@@ -158,7 +198,6 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_sums_kernel(GlaArgs a, Work
     if (hf == 0 && ch && blockIdx.z == 0) w.d[r] = expf(static_cast<float>(rest));
     if (NRM) nsum[hf * kMaxD + i] = ns;
   }
-  cp_async_wait_all();
   __syncthreads();
   if (NRM && tid < D && blockIdx.z == 0) w.n[(static_cast<long long>(blockIdx.x) * a.heads + head) * D + tid] = nsum[tid] + nsum[kMaxD + tid];
   if (16 * wrp >= D) return;
@@ -211,7 +250,7 @@ __global__ void __launch_bounds__(kThreads) chunk_states_kernel(GlaArgs a, Work 
   const bool old = a.seqs[seq * 8 + 2] > 0;
   const long long cstep = static_cast<long long>(a.heads) * D, hrow = static_cast<long long>(first) * cstep + head * D;
   const int e = (blockIdx.x * kThreads + threadIdx.x) * 4;
-  constexpr int U = 4;
+  constexpr int U = 8;
   if (e < D * P) {
     const int i = e / P;
     float* sp = w.s + hrow * P + e;
@@ -248,24 +287,27 @@ __global__ void __launch_bounds__(kThreads) chunk_states_kernel(GlaArgs a, Work 
 }
 
 // ---------------------------------------------------------------- a chunk's outputs
-__device__ __forceinline__ void mma6(float* c, const uint32_t (*A)[4], const uint32_t (*B)[2]) {
-  mma(c, A[2], B[0][0], B[0][1]);
-  mma(c, A[0], B[2][0], B[2][1]);
-  mma(c, A[1], B[1][0], B[1][1]);
-  mma(c, A[1], B[0][0], B[0][1]);
-  mma(c, A[0], B[1][0], B[1][1]);
-  mma(c, A[0], B[0][0], B[0][1]);
+// N tiles of one left operand, term pairs outside: neighbouring products go to different sums, so none waits for the one in front
+template <int N>
+__device__ __forceinline__ void mma6(float* const* c, const uint32_t (*A)[4], const uint32_t (*B)[3][2]) {
+  constexpr int ta[6] = {2, 0, 1, 1, 0, 0}, tb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+  for (int p = 0; p < 6; ++p)
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma(c[n], A[ta[p]], B[n][tb[p]][0], B[n][tb[p]][1]);
 }
 __device__ __forceinline__ bool finite2(uint32_t x) { return (x & 0x7f80u) != 0x7f80u && (x & 0x7f800000u) != 0x7f800000u; }
 __device__ __forceinline__ float2 mul2(float2 x, float2 y) { return make_float2(x.x * y.x, x.y * y.y); }
 
-// grid (chunks, heads, column blocks).  Warp w: tokens of block w / 2, value columns of half w % 2.
+// grid (chunks, heads, column blocks).  Warp w: tokens of block w / 2, key channels and then value columns of half w % 2.  All
+// loads of a phase are issued before the first is waited for; a lane's queries, keys and decays are its own until the scores.
 constexpr int kRows = 32;     // state rows staged per round, in three terms, where the keys were
 struct OutSmem {
   float Q[kQ * kLd];          // queries, then carried from their block's start
   float K[kQ * kLd];          // keys, then carried to their block's end; then [3][kRows][kLd] bf16 terms of the state
   bf16 V[kQ * kLd];
   float diag[8][kB][kB + 1];  // scores inside a block, one half of the key channels each
+  float cross[6][kB][24];     // scores between two blocks: of block b against x in b (b - 1) / 2 + x
   float tot[4][kMaxD];        // log decay over a block
   float from0[4][kMaxD];      // decay from the chunk's start to a block's start
   float mid[3][kMaxD];        // decay over block 1, block 2, both
@@ -283,46 +325,61 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
   const int tok0 = a.seqs[seq * 8] + chunk * kQ, q = min(kQ, a.seqs[seq * 8 + 1] - chunk * kQ);
   const bool has_state = chunk > 0 || a.seqs[seq * 8 + 2] > 0;
   const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-  const float* lap = MODE == VEC_Z ? a.z : w.la;
+  const int b = wrp >> 1, half = wrp & 1;
+  const long long hrow = (static_cast<long long>(blockIdx.x) * a.heads + head) * D;
   fetch_values(a, sm.V, tok0, q, head, p0);
-  if (MODE == SCALAR) fetch_gates(a, sm.gates, tok0, q, head);
+  // A lane's own part: the 16 tokens of its warp's block, two channels.  All of its loads are in flight before the first is waited
+  // for (addresses of tokens and channels that are not there are those of ones that are).
+  const int c = half * 64 + 2 * lane;
+  const bool ch = c < D;
+  float2 la[kB];               // log decays; scalar gates: in shared memory
   {
-    const int i = tid & (kMaxD - 1), hf = tid / kMaxD;
-    const bool ch = i < D;
-    const bf16* base = static_cast<const bf16*>(a.qkv) + (head / a.group) * D + i;
-    const float fb = MODE == VEC_FGATE && ch ? __ldg(a.z_bias + head * D + i) : 0.f, fl = MODE == VEC_FGATE && ch ? __ldg(a.fgate_lower + head * D + i) : 0.f;
-#pragma unroll 8
-    for (int jj = 0; jj < kQ / 2; ++jj) {
-      const int j = hf * (kQ / 2) + jj;
-      float qv = 0.f, kv = 0.f;
-      if (ch && j < q) {
-        const long long row = tok0 + j;
-        qv = bf(base + row * a.ld + a.q_off);
-        kv = bf(base + row * a.ld + a.k_off);
-        if (a.act == GLA_ACT_SILU_Q) qv = qv / (1.0f + expf(-qv));
-        if (MODE == VEC_FGATE) { float l; forget_gate(kv + fb, fl, &l, &kv); }
-        if (MODE == SCALAR) kv *= sm.gates[kQ + j];
-      }
-      sm.Q[j * kLd + i] = qv * a.q_scale;
-      sm.K[j * kLd + i] = kv * a.k_scale;
+    uint32_t qr[kB], kr[kB];
+    const int c1 = ch ? c : 0;
+    const bf16* base = static_cast<const bf16*>(a.qkv) + (head / a.group) * D + c1;
+#pragma unroll
+    for (int t = 0; t < kB; ++t) {
+      const long long row = tok0 + min(b * kB + t, q - 1);
+      qr[t] = __ldg(reinterpret_cast<const unsigned int*>(base + row * a.ld + a.q_off));
+      kr[t] = __ldg(reinterpret_cast<const unsigned int*>(base + row * a.ld + a.k_off));
+      if (MODE == VEC_Z) la[t] = *reinterpret_cast<const float2*>(a.z + row * HD + head * D + c1);
     }
-    if (NRM && tid < kMaxD) sm.n0[tid] = has_state && tid < D ? w.n[(static_cast<long long>(blockIdx.x) * a.heads + head) * D + tid] : 0.f;
+    float2 fb = make_float2(0.f, 0.f), fl = fb;
+    if (MODE == VEC_FGATE) {
+      fb = make_float2(__ldg(a.z_bias + head * D + c1), __ldg(a.z_bias + head * D + c1 + 1));
+      fl = make_float2(__ldg(a.fgate_lower + head * D + c1), __ldg(a.fgate_lower + head * D + c1 + 1));
+    }
+    if (MODE == SCALAR) fetch_gates(a, sm.gates, tok0, q, head);
+    const bool silu = a.act == GLA_ACT_SILU_Q;
+#pragma unroll
+    for (int t = 0; t < kB; ++t) {
+      const int tt = b * kB + t;
+      const bool in = ch && tt < q;
+      float2 qv = make_float2(low(qr[t]), high(qr[t])), kv = make_float2(low(kr[t]), high(kr[t]));
+      if (silu) {
+        float2 s, rest;
+        sigmoids(qv.x, &s.x, &rest.x);
+        sigmoids(qv.y, &s.y, &rest.y);
+        qv = mul2(qv, s);
+      }
+      if (MODE == VEC_FGATE) { forget_gate(kv.x + fb.x, fl.x, &la[t].x, &kv.x); forget_gate(kv.y + fb.y, fl.y, &la[t].y, &kv.y); }
+      if (MODE == SCALAR) { kv.x *= sm.gates[kQ + tt]; kv.y *= sm.gates[kQ + tt]; }
+      else if (!in) la[t] = make_float2(0.f, 0.f);
+      *reinterpret_cast<float2*>(sm.Q + tt * kLd + c) = in ? make_float2(qv.x * a.q_scale, qv.y * a.q_scale) : make_float2(0.f, 0.f);
+      *reinterpret_cast<float2*>(sm.K + tt * kLd + c) = in ? make_float2(kv.x * a.k_scale, kv.y * a.k_scale) : make_float2(0.f, 0.f);
+    }
+    if (NRM && tid < kMaxD) sm.n0[tid] = has_state && tid < D ? w.n[hrow + tid] : 0.f;
   }
-  __syncthreads();
   // ---- blocks on the diagonal, token by token: a lane holds the decayed keys of its two channels
   {
-    const int b = wrp >> 1, c = (wrp & 1) * 64 + 2 * lane;
     float2 W[kB];
 #pragma unroll
     for (int t = 0; t < kB; ++t) {
       const int tt = b * kB + t;
       float2 al = make_float2(1.f, 1.f);
-      if (tt < q && t > 0) {
+      if (t > 0) {
         if (MODE == SCALAR) al.x = al.y = expf(sm.gates[tt]);
-        else if (c < D) {
-          const float2 l = *reinterpret_cast<const float2*>(lap + static_cast<long long>(tok0 + tt) * HD + head * D + c);
-          al = make_float2(expf(l.x), expf(l.y));
-        }
+        else al = make_float2(expf(la[t].x), expf(la[t].y));
       }
       const float2 qt = *reinterpret_cast<const float2*>(sm.Q + tt * kLd + c), kt = *reinterpret_cast<const float2*>(sm.K + tt * kLd + c);
       float p[kB];
@@ -347,32 +404,23 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
       if (!(lane & 1)) sm.diag[wrp][t][lane >> 1] = p[0];
     }
   }
-  __syncthreads();
-  // ---- queries from their block's start, keys to their block's end
-  {
-    const int i = tid & (kMaxD - 1), hf = tid / kMaxD;
-    if (i < D) {
+  // ---- the lane's queries from the block's start, its keys to the block's end
+  if (ch) {
+    float2 run = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int bb = 0; bb < 2; ++bb) {
-        const int b = 2 * hf + bb;
-        float la[kB];
+    for (int t = 0; t < kB; ++t) {
+      if (MODE == SCALAR) la[t].x = la[t].y = sm.gates[b * kB + t];
+      run.x += la[t].x; run.y += la[t].y;
+      float2* p = reinterpret_cast<float2*>(sm.Q + (b * kB + t) * kLd + c);
+      *p = mul2(*p, make_float2(expf(run.x), expf(run.y)));
+    }
+    *reinterpret_cast<float2*>(sm.tot[b] + c) = run;
+    run = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int t = 0; t < kB; ++t) {
-          const int tt = b * kB + t;
-          la[t] = 0.f;
-          if (tt < q) {
-            if (MODE == SCALAR) la[t] = sm.gates[tt];
-            else la[t] = lap[static_cast<long long>(tok0 + tt) * HD + head * D + i];
-          }
-        }
-        float run = 0.f;
-#pragma unroll
-        for (int t = 0; t < kB; ++t) { run += la[t]; sm.Q[(b * kB + t) * kLd + i] *= expf(run); }
-        sm.tot[b][i] = run;
-        run = 0.f;
-#pragma unroll
-        for (int t = kB - 1; t >= 0; --t) { sm.K[(b * kB + t) * kLd + i] *= expf(run); run += la[t]; }
-      }
+    for (int t = kB - 1; t >= 0; --t) {
+      float2* p = reinterpret_cast<float2*>(sm.K + (b * kB + t) * kLd + c);
+      *p = mul2(*p, make_float2(expf(run.x), expf(run.y)));
+      run.x += la[t].x; run.y += la[t].y;
     }
   }
   __syncthreads();
@@ -383,44 +431,69 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
   }
   cp_async_wait_all();
   __syncthreads();
-  // ---- scores of the warp's 16 tokens against the blocks in front
-  const int b = wrp >> 1, half = wrp & 1, ncol = min(64, P - p0 - 64 * half);
-  const float* Qr = sm.Q + (b * kB + g) * kLd + 2 * t4;
-  float sc[3][2][4];
+  // the state's first rows, on their way during the scores
+  const float* S = w.s + hrow * P + p0;
+  const int r0 = tid >> 5, c0 = (tid & 31) * 4;      // rows r0, r0 + 8, ... of a round
+  float4 nx[kRows / 8];
+  auto fetch = [&](int i0) {
 #pragma unroll
-  for (int x = 0; x < 3; ++x)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) sc[x][nt][0] = sc[x][nt][1] = sc[x][nt][2] = sc[x][nt][3] = 0.f;
+    for (int u = 0; u < kRows / 8; ++u) {
+      const int i = i0 + r0 + 8 * u;
+      nx[u] = i < D && p0 + c0 < P ? *reinterpret_cast<const float4*>(S + static_cast<long long>(i) * P + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (has_state) fetch(0);
+  // ---- scores against the blocks in front: six pairs of blocks, at most two for the two warps of a block, which take eight keys
+  // each; block 0's warps have block 3's first pair
   const bool live = b * kB < q;
-  if (live && b > 0) {
-    for (int ks = 0; ks < nk; ++ks) {
-      uint32_t A[3][4];
+  const int ncol = min(64, P - p0 - 64 * half);
+  const float* Qr = sm.Q + (b * kB + g) * kLd + 2 * t4;
+  {
+    const int qb = b == 0 ? 3 : b, x0 = b == 3 ? 1 : 0;
+    const float* Qs = sm.Q + (qb * kB + g) * kLd + 2 * t4;
+    auto scores = [&](auto pairs) {
+      constexpr int N = decltype(pairs)::value;
+      float sc[N][4];
+      float* at[N];
+      const float* m[N];       // from block x's end to block qb's start: nothing, block 1, block 2 or both
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float2 v = *reinterpret_cast<const float2*>(Qr + (r & 1) * 8 * kLd + ks * 16 + (r >> 1) * 8);
-        split3(v.x, v.y, &A[0][r], &A[1][r], &A[2][r]);
+      for (int n = 0; n < N; ++n) {
+        const int x = x0 + n;
+        at[n] = sc[n];
+        sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
+        m[n] = qb - x == 1 ? nullptr : (qb - x == 3 ? sm.mid[2] : sm.mid[x]);
       }
+      for (int ks = 0; ks < nk; ++ks) {
+        uint32_t A[3][4], B[N][3][2];
 #pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        if (x < b) {
-          // from block x's end to block b's start: nothing, block 1, block 2 or both
-          const float* m = b - x == 1 ? nullptr : (b - x == 3 ? sm.mid[2] : sm.mid[x]);
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            uint32_t B[3][2];
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const int col = ks * 16 + r * 8 + 2 * t4;
-              float2 v = *reinterpret_cast<const float2*>(sm.K + (x * kB + nt * 8 + g) * kLd + col);
-              if (m) v = mul2(v, *reinterpret_cast<const float2*>(m + col));
-              split3(v.x, v.y, &B[0][r], &B[1][r], &B[2][r]);
-            }
-            mma6(sc[x][nt], A, B);
-          }
+        for (int r = 0; r < 4; ++r) {
+          const float2 v = *reinterpret_cast<const float2*>(Qs + (r & 1) * 8 * kLd + ks * 16 + (r >> 1) * 8);
+          split3(v.x, v.y, &A[0][r], &A[1][r], &A[2][r]);
         }
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int col = ks * 16 + r * 8 + 2 * t4;
+            float2 v = *reinterpret_cast<const float2*>(sm.K + ((x0 + n) * kB + half * 8 + g) * kLd + col);
+            if (m[n]) v = mul2(v, *reinterpret_cast<const float2*>(m[n] + col));
+            split3(v.x, v.y, &B[n][0][r], &B[n][1][r], &B[n][2][r]);
+          }
+        mma6<N>(at, A, B);
       }
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        float (*d)[24] = sm.cross[qb * (qb - 1) / 2 + x0 + n];
+        *reinterpret_cast<float2*>(&d[g][half * 8 + 2 * t4]) = make_float2(sc[n][0], sc[n][1]);
+        *reinterpret_cast<float2*>(&d[g + 8][half * 8 + 2 * t4]) = make_float2(sc[n][2], sc[n][3]);
+      }
+    };
+    if (qb * kB < q) {
+      if (b < 2) scores(std::integral_constant<int, 1>());
+      else scores(std::integral_constant<int, 2>());
     }
   }
+  __syncthreads();
   float o[8][4];
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
@@ -434,22 +507,32 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
       nq[1] += (s[0][2] + s[0][3]) + (s[1][2] + s[1][3]);
     }
 #pragma unroll
-    for (int np = 0; np < 4; ++np) {
-      if (np * 16 < ncol) {
-        uint32_t v[4];
-        ldsm_x4_trans(v, bt_addr(sm.V, kLd, blk * kB, half * 64 + np * 16, lane));
+    for (int np = 0; np < 4; np += 2) {
+      if (np * 16 < ncol) {      // two 16-column tiles at a time; what is past the last column is zero
+        uint32_t v[2][4];
+        ldsm_x4_trans(v[0], bt_addr(sm.V, kLd, blk * kB, half * 64 + np * 16, lane));
+        ldsm_x4_trans(v[1], bt_addr(sm.V, kLd, blk * kB, half * 64 + np * 16 + 16, lane));
 #pragma unroll
-        for (int k = 2; k >= 0; --k) {
-          mma(o[2 * np], A[k], v[0], v[1]);
-          mma(o[2 * np + 1], A[k], v[2], v[3]);
-        }
+        for (int k = 2; k >= 0; --k)
+#pragma unroll
+          for (int n = 0; n < 4; ++n) mma(o[2 * np + n], A[k], v[n >> 1][2 * (n & 1)], v[n >> 1][2 * (n & 1) + 1]);
       }
     }
   };
   if (live) {
 #pragma unroll
     for (int x = 0; x < 3; ++x)
-      if (x < b) values(sc[x], x);
+      if (x < b) {
+        float s[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float2 v = *reinterpret_cast<const float2*>(&sm.cross[b * (b - 1) / 2 + x][g + 8 * r][nt * 8 + 2 * t4]);
+            s[nt][2 * r] = v.x; s[nt][2 * r + 1] = v.y;
+          }
+        values(s, x);
+      }
     float d[2][4];
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
@@ -488,19 +571,8 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
   // ---- the incoming state's part
   if (has_state) {
     bf16* Ss = reinterpret_cast<bf16*>(sm.K);
-    const float* S = w.s + ((static_cast<long long>(blockIdx.x) * a.heads + head) * D) * P + p0;
-    const int r0 = tid >> 5, c0 = (tid & 31) * 4;      // rows r0, r0 + 8, ... of a round
-    float4 nx[kRows / 8];
-    auto fetch = [&](int i0) {
-#pragma unroll
-      for (int u = 0; u < kRows / 8; ++u) {
-        const int i = i0 + r0 + 8 * u;
-        nx[u] = i < D && p0 + c0 < P ? *reinterpret_cast<const float4*>(S + static_cast<long long>(i) * P + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    };
-    fetch(0);
     for (int i0 = 0; i0 < D; i0 += kRows) {
-      __syncthreads();       // the keys, or the last rows, are no longer read
+      if (i0 > 0) __syncthreads();       // the last rows are no longer read (nor the keys, since the barrier behind the scores)
 #pragma unroll
       for (int u = 0; u < kRows / 8; ++u) {
         uint32_t x[3], y[3];
@@ -528,15 +600,22 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_out_kernel(GlaArgs a, Work 
             split3(v.x, v.y, &A[0][r], &A[1][r], &A[2][r]);
           }
 #pragma unroll
-          for (int np = 0; np < 4; ++np) {
+          for (int np = 0; np < 4; np += 2) {
             if (np * 16 < ncol) {
-              uint32_t t[3][4];
+              uint32_t B[4][3][2];
+              float* at[4];
 #pragma unroll
-              for (int k = 0; k < 3; ++k) ldsm_x4_trans(t[k], bt_addr(Ss + k * kRows * kLd, kLd, kk * 16, half * 64 + np * 16, lane));
-              const uint32_t B0[3][2] = {{t[0][0], t[0][1]}, {t[1][0], t[1][1]}, {t[2][0], t[2][1]}};
-              const uint32_t B1[3][2] = {{t[0][2], t[0][3]}, {t[1][2], t[1][3]}, {t[2][2], t[2][3]}};
-              mma6(o[2 * np], A, B0);
-              mma6(o[2 * np + 1], A, B1);
+              for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                  uint32_t t[4];
+                  ldsm_x4_trans(t, bt_addr(Ss + k * kRows * kLd, kLd, kk * 16, half * 64 + (np + n) * 16, lane));
+                  B[2 * n][k][0] = t[0]; B[2 * n][k][1] = t[1];
+                  B[2 * n + 1][k][0] = t[2]; B[2 * n + 1][k][1] = t[3];
+                }
+#pragma unroll
+              for (int n = 0; n < 4; ++n) at[n] = o[2 * np + n];
+              mma6<4>(at, A, B);
             }
           }
         }
@@ -574,16 +653,16 @@ int run(const GlaArgs& a, const Work& w, int chunks, cudaStream_t st) {
 
 }  // namespace
 
-size_t scan_parallel_ws_floats(int tokens, int seqs, int heads, int dim, int vdim, bool fgate) {
+size_t scan_parallel_ws_floats(int tokens, int seqs, int heads, int dim, int vdim) {
   const size_t chunks = static_cast<size_t>(tokens) / kQ + seqs;
-  return chunks * heads * dim * (static_cast<size_t>(vdim) + 2) + (fgate ? static_cast<size_t>(tokens) * heads * dim : 0);
+  return chunks * heads * dim * (static_cast<size_t>(vdim) + 2);
 }
 
 bool scan_parallel_fits(const GlaArgs& a) {
   auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   return a.par_ws && a.t == DT_BF16 && (a.act == GLA_ACT_NONE || a.act == GLA_ACT_SILU_Q) && !a.rope && !a.head_decay && !a.dt_pre && !a.tok_decay == !a.nstate && a.dim % 16 == 0 && a.dim <= kMaxD &&
-         a.vdim % 8 == 0 && a.ld % 8 == 0 && a.v_off % 8 == 0 && al(a.qkv) && al(a.states) && al(a.o) && al(a.par_ws) && (a.tok_decay || a.fgate_lower || al(a.z)) &&
-         scan_parallel_ws_floats(a.T, a.nseq, a.heads, a.dim, a.vdim, a.fgate_lower != nullptr) <= a.par_ws_floats;
+         a.vdim % 8 == 0 && a.ld % 8 == 0 && a.q_off % 8 == 0 && a.k_off % 8 == 0 && a.v_off % 8 == 0 && al(a.qkv) && al(a.states) && al(a.o) && al(a.par_ws) && (a.tok_decay || a.fgate_lower || al(a.z)) &&
+         scan_parallel_ws_floats(a.T, a.nseq, a.heads, a.dim, a.vdim) <= a.par_ws_floats;
 }
 
 int scan_parallel(const GlaArgs& a, cudaStream_t st) {
@@ -594,11 +673,9 @@ int scan_parallel(const GlaArgs& a, cudaStream_t st) {
   w.s = a.par_ws;
   w.d = w.s + rows * a.vdim;
   w.n = w.d + rows;
-  w.la = w.n + rows;
   if (a.tok_decay) return run<SCALAR, true>(a, w, chunks, st);
   if (a.fgate_lower) return run<VEC_FGATE, false>(a, w, chunks, st);
-  const long long total = static_cast<long long>(a.T) * a.heads * a.dim;
-  if (total > 0) log_decay_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(a.z, a.z_bias, a.heads * a.dim, a.inv_tau, total);
+  if (a.T > 0) log_decay_kernel<<<dim3(a.T, (a.heads * a.dim / 4 + 255) / 256), 256, 0, st>>>(a.z, a.z_bias, a.heads * a.dim, a.inv_tau);
   return run<VEC_Z, false>(a, w, chunks, st);
 }
 

@@ -362,7 +362,7 @@ class Soselix : public Model {
     if (dt != DT_BF16) return;
     size_t sw = 0;
     for (auto& s : spec) {
-      if (s.kind == MIX_HGRN2) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim, true));
+      if (s.kind == MIX_HGRN2) sw = std::max(sw, scan_parallel_ws_cap(env.Tcap, env.num_slots, s.heads, s.dim, s.vdim));
       if (s.kind == MIX_MAMBA2) sw = std::max(sw, scan_segments_ws_floats(env.Tcap, std::min(env.num_slots, 6), s.heads, s.dim, s.vdim));
     }
     if (sw && spare(&scan_ws, sw * sizeof(float))) scan_ws_floats = sw;

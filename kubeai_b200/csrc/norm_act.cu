@@ -34,7 +34,17 @@ __global__ void embed_bigram_kernel(const TW* embed, const TW* bigram, const int
   const long long row = prev < 0 ? buckets : (static_cast<long long>(prev) * mul_prev + static_cast<long long>(id) * mul_cur) % buckets;
   const TW* e = embed + static_cast<long long>(id) * W;
   const TW* g = bigram + row * W;
-  for (int i = threadIdx.x; i < W; i += blockDim.x) x[static_cast<long long>(t) * W + i] = ldf(e + i) + ldf(g + i);
+  float* xr = x + static_cast<long long>(t) * W;
+  if (sizeof(TW) == 2 && W % 4 == 0 && (reinterpret_cast<unsigned long long>(embed) | reinterpret_cast<unsigned long long>(bigram) | reinterpret_cast<unsigned long long>(x)) % 16 == 0) {
+    for (int i = threadIdx.x * 4; i < W; i += blockDim.x * 4) {
+      const uint2 u = *reinterpret_cast<const uint2*>(e + i), v = *reinterpret_cast<const uint2*>(g + i);
+      auto lo = [](uint32_t q) { return __uint_as_float(q << 16); };
+      auto hi = [](uint32_t q) { return __uint_as_float(q & 0xffff0000u); };
+      *reinterpret_cast<float4*>(xr + i) = make_float4(lo(u.x) + lo(v.x), hi(u.x) + hi(v.x), lo(u.y) + lo(v.y), hi(u.y) + hi(v.y));
+    }
+    return;
+  }
+  for (int i = threadIdx.x; i < W; i += blockDim.x) xr[i] = ldf(e + i) + ldf(g + i);
 }
 
 template <typename TA, typename TY>

@@ -1,0 +1,54 @@
+"""Norms between sublayers, embeddings and latent rows at widths around the edges of their pieces (csrc/hyper.cu, norm_act.cu,
+latent_attention.cu): one, two and four pieces of four columns a thread, more than that, and rows that allow no wide access."""
+import numpy as np
+import pytest
+
+import dabodra_util as dx
+import mulenex_util as mx
+import nomanex_util as nx
+import soselix_util as sx
+
+pytestmark = pytest.mark.gpu
+
+WIDTHS = [4, 36, 252, 256, 260, 510, 516, 1020, 1028, 2044, 2052, 4096, 4100]
+
+
+def model(family, width):
+    if family == "mulenex":
+        cfg = mx.make_config([mx.layer(mx.mlstm(heads=2, dim=16, vdim=8), mlp=None), mx.layer(mx.mlstm(heads=2, dim=16, vdim=8), mlp=None)], width=width)
+        return cfg, mx.random_weights(cfg, seed=1), mx.oracle_for
+    if family == "soselix":
+        cfg = sx.make_config([sx.latent(q_rank=24, kv_rank=20, mlp=None), sx.hgrn2(mlp=None)], width=width)
+        return cfg, sx.random_weights(cfg, seed=2), sx.oracle_for
+    if family == "dabodra":
+        cfg = dx.make_config([dx.attention(mlp=None), dx.delta(mlp=None)], width=width)
+        return cfg, dx.random_weights(cfg, seed=3), dx.oracle_for
+    cfg = nx.make_config([(nx.gla(), None), (nx.latent(), None)], width=width)
+    return cfg, nx.random_weights(cfg, seed=4), nx.oracle_for
+
+
+@pytest.mark.parametrize("family", ["mulenex", "soselix", "dabodra", "nomanex"])
+@pytest.mark.parametrize("width", WIDTHS)
+def test_rows_of_every_number_of_pieces(tmp_path, family, width):
+    cfg, W, oracle = model(family, width)
+    d = nx.write_model_dir(tmp_path / "m", cfg, W)
+    t = np.random.default_rng(width).integers(0, cfg["vocab"], 21).tolist()
+    want = oracle(cfg, W).forward(t)
+    # fp32: sums of at most 4100 products, some sixty roundings of 2^-24 each where their signs are random, in about eight sublayers'
+    # worth of operators: 3e-5; small widths divide by sums of few terms
+    with nx.open_engine(d) as e:
+        assert np.median(nx.rel_err(nx.feed_whole(e, t), want)) < 1e-4
+        assert np.median(nx.rel_err(nx.feed_portions(e, t, [9] + [1] * 12), want)) < 1e-4
+    # bf16: eight operators' outputs rounded to 2^-9 of their size each
+    with nx.open_engine(d, dtype="bfloat16") as e:
+        assert np.median(nx.rel_err(nx.feed_portions(e, t, [9] + [1] * 12), want)) < 0.06
+
+
+@pytest.mark.parametrize("q_rank,kv_rank", [(1, 1), (127, 129), (1024, 512), (1025, 1023), (40, 1100)])
+def test_latent_rows_that_stay_in_registers_and_longer_ones(tmp_path, q_rank, kv_rank):
+    cfg = sx.make_config([sx.latent(heads=2, q_rank=q_rank, kv_rank=kv_rank, mlp=None)], width=32)
+    W = sx.random_weights(cfg, seed=q_rank)
+    d = nx.write_model_dir(tmp_path / "m", cfg, W)
+    t = np.random.default_rng(5).integers(0, cfg["vocab"], 17).tolist()
+    with nx.open_engine(d) as e:
+        assert np.median(nx.rel_err(nx.feed_portions(e, t, [8] + [1] * 9), sx.oracle_for(cfg, W).forward(t))) < 1e-4

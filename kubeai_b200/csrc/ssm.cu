@@ -64,16 +64,15 @@ __global__ void short_conv_kernel(ShortConvArgs a) {
 template <int VEC> struct VecOf;
 template <> struct VecOf<8> { typedef bf16 type; };
 template <> struct VecOf<4> { typedef float type; };
-__device__ __forceinline__ void ldv(const bf16* p, float* v) {
-  const uint4 r = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void unpack(uint4 r, const bf16*, float* v) {
   const uint32_t u[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(u[i] << 16); v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
 }
-__device__ __forceinline__ void ldv(const float* p, float* v) {
-  const float4 r = *reinterpret_cast<const float4*>(p);
-  v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+__device__ __forceinline__ void unpack(uint4 r, const float*, float* v) {
+  v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2] = __uint_as_float(r.z); v[3] = __uint_as_float(r.w);
 }
+template <typename T> __device__ __forceinline__ void ldv(const T* p, float* v) { unpack(*reinterpret_cast<const uint4*>(p), p, v); }
 __device__ __forceinline__ void stv(bf16* p, const float* v) {
   uint32_t u[4];
 #pragma unroll
@@ -85,10 +84,11 @@ __device__ __forceinline__ void stv(float* p, const float* v) { *reinterpret_cas
 // A thread owns VEC neighbouring channels and walks TB consecutive token rows with the last TAPS - 1 inputs in registers:
 // every input row is loaded once, the weights of the thread's channels once per walk.  Where the walk enters another
 // sequence (or at its start) the window is filled again, from the rows before, the sequence's carried inputs or zeros.
+// Rows come four at a time, as loaded, with their sequences' numbers, and the next four while these are worked on: a walk is bound
+// by that many loads in flight.  4095 tokens x 6144 channels: 57 us with a wait for every four rows, 40 now (15.5 at the copy rate).
 template <int VEC, int TAPS>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConvArgs a, int TB) {
   griddep_launch();
-  griddep_wait();
   typedef typename VecOf<VEC>::type T;
   const int groups = a.C / VEC;
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConvArgs a, in
   const int c = gi * VEC;
   const long long t0 = static_cast<long long>(blockIdx.y) * TB, t1 = min(static_cast<long long>(a.T), t0 + TB);
   const T* u = static_cast<const T*>(a.u);
-  float w[TAPS][VEC], hist[TAPS > 1 ? TAPS - 1 : 1][VEC], bias[VEC], rows[4][VEC];
+  float w[TAPS][VEC], hist[TAPS > 1 ? TAPS - 1 : 1][VEC], bias[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
     bias[e] = a.bias ? a.bias[c + e] : 0.f;
@@ -108,54 +108,69 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConvArgs a, in
       w[0][e] = q.x; w[1][e] = q.y; w[2][e] = q.z; w[3][e] = q.w;
     }
   }
+  griddep_wait();
   int cur = -1;
-  for (long long t = t0; t < t1; ++t) {
-    const int s = a.seq_of_tok[t];
-    if (s != cur) {
-      // hist[k] = the input TAPS - 1 - k tokens before t
-      cur = s;
-      const int* sq = a.seqs + s * 8;
-      const int i = static_cast<int>(t) - sq[0];
-      const bool carried = sq[2] > 0;
-      const float* st = a.state + static_cast<long long>(sq[3]) * (TAPS - 1) * a.C;
+  constexpr int G = 4;
+  uint4 next[G];
+  int next_seq[G];
+  auto fetch = [&](long long t) {
 #pragma unroll
-      for (int k = 0; k < TAPS - 1; ++k) {
-        const int d = TAPS - 1 - k;
-        if (i - d >= 0) ldv(u + (t - d) * a.ldu + c, hist[k]);
-        else {
+    for (int r = 0; r < G; ++r) {
+      const long long tt = min(t + r, t1 - 1);
+      next[r] = *reinterpret_cast<const uint4*>(u + tt * a.ldu + c);
+      next_seq[r] = a.seq_of_tok[tt];
+    }
+  };
+  fetch(t0);
+  for (long long t4 = t0; t4 < t1; t4 += G) {
+    uint4 raw[G];
+    int seq[G];
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) hist[k][e] = carried ? st[static_cast<long long>(TAPS - 1 + i - d) * a.C + c + e] : 0.f;
+    for (int r = 0; r < G; ++r) { raw[r] = next[r]; seq[r] = next_seq[r]; }
+    if (t4 + G < t1) fetch(t4 + G);
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+      const long long t = t4 + r;
+      if (t >= t1) break;
+      const int s = seq[r];
+      if (s != cur) {
+        // hist[k] = the input TAPS - 1 - k tokens before t
+        cur = s;
+        const int* sq = a.seqs + s * 8;
+        const int i = static_cast<int>(t) - sq[0];
+        const bool carried = sq[2] > 0;
+        const float* st = a.state + static_cast<long long>(sq[3]) * (TAPS - 1) * a.C;
+#pragma unroll
+        for (int k = 0; k < TAPS - 1; ++k) {
+          const int d = TAPS - 1 - k;
+          if (i - d >= 0) ldv(u + (t - d) * a.ldu + c, hist[k]);
+          else {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) hist[k][e] = carried ? st[static_cast<long long>(TAPS - 1 + i - d) * a.C + c + e] : 0.f;
+          }
         }
       }
+      float v[VEC], acc[VEC];
+      unpack(raw[r], static_cast<T*>(nullptr), v);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        float x = bias[e];
+#pragma unroll
+        for (int k = 0; k < TAPS - 1; ++k) x = fmaf(w[k][e], hist[k][e], x);     // oldest tap first, the token's own last
+        x = fmaf(w[TAPS - 1][e], v[e], x);
+        // an output that is rounded to bf16 takes the fast exponential and division
+        acc[e] = a.act == CONV_SILU ? (VEC == 8 ? __fdividef(x, 1.0f + __expf(-x)) : siluf_(x)) : x;
+      }
+#pragma unroll
+      for (int k = 0; k + 1 < TAPS - 1; ++k)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) hist[k][e] = hist[k + 1][e];
+      if (TAPS > 1) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) hist[TAPS - 2][e] = v[e];
+      }
+      stv(static_cast<T*>(a.y) + t * a.ldy + c, acc);
     }
-    // the loads of up to four rows are issued together, ahead of the arithmetic of the first
-    const int q = static_cast<int>(t - t0) & 3;
-    if (q == 0) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (t + r < t1) ldv(u + (t + r) * a.ldu + c, rows[r]);
-    }
-    float v[VEC], acc[VEC];
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) v[e] = q == 0 ? rows[0][e] : (q == 1 ? rows[1][e] : (q == 2 ? rows[2][e] : rows[3][e]));
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      float r = bias[e];
-#pragma unroll
-      for (int k = 0; k < TAPS - 1; ++k) r = fmaf(w[k][e], hist[k][e], r);     // oldest tap first, the token's own last
-      r = fmaf(w[TAPS - 1][e], v[e], r);
-      // an output that is rounded to bf16 takes the fast exponential and division
-      acc[e] = a.act == CONV_SILU ? (VEC == 8 ? __fdividef(r, 1.0f + __expf(-r)) : siluf_(r)) : r;
-    }
-#pragma unroll
-    for (int k = 0; k + 1 < TAPS - 1; ++k)
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) hist[k][e] = hist[k + 1][e];
-    if (TAPS > 1) {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) hist[TAPS - 2][e] = v[e];
-    }
-    stv(static_cast<T*>(a.y) + t * a.ldy + c, acc);
   }
 }
 

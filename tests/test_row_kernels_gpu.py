@@ -52,3 +52,22 @@ def test_latent_rows_that_stay_in_registers_and_longer_ones(tmp_path, q_rank, kv
     t = np.random.default_rng(5).integers(0, cfg["vocab"], 17).tolist()
     with nx.open_engine(d) as e:
         assert np.median(nx.rel_err(nx.feed_portions(e, t, [8] + [1] * 9), sx.oracle_for(cfg, W).forward(t))) < 1e-4
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_short_convolution_over_sequences_that_end_inside_its_rounds(tmp_path, taps):
+    """Rows come in rounds of four and walks of up to sixteen; sequences begin and end anywhere in them and go on from what they carry."""
+    cfg = dx.make_config([dx.delta(heads=4, kv_heads=2, dim=8, vdim=8, conv=taps, mlp=None)], width=32)
+    W = dx.random_weights(cfg, seed=taps)
+    d = nx.write_model_dir(tmp_path / "m", cfg, W)
+    rng = np.random.default_rng(taps)
+    first = [1, 2, 3, 4, 5, 7, 16, 17, 1, 31, 6, 1, 1, 64, 3, 33]
+    seqs = [rng.integers(0, cfg["vocab"], n + 1 + i % 5) for i, n in enumerate(first)]
+    want = [dx.oracle_for(cfg, W).forward(s.tolist()) for s in seqs]
+    for dtype, tol in (("float32", 1e-4), ("bfloat16", 0.06)):     # fp32 sums; three operators' outputs rounded to 2^-9 each
+        with nx.open_engine(d, dtype=dtype, max_tokens=128, max_seqs=16, budget=512, blocks=128) as e:
+            ids = [e.feed_open() for _ in seqs]
+            a = e.feed_step([(r, s[:n].tolist(), [n - 1]) for r, s, n in zip(ids, seqs, first)])
+            b = e.feed_step([(r, s[n:].tolist(), [len(s) - n - 1]) for r, s, n in zip(ids, seqs, first)])
+        assert np.median(nx.rel_err(np.asarray(a), np.stack([w[n - 1] for w, n in zip(want, first)]))) < tol
+        assert np.median(nx.rel_err(np.asarray(b), np.stack([w[-1] for w in want]))) < tol

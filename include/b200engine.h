@@ -367,6 +367,10 @@ int64_t b200_tokenizer_chat_llama3(const b200_tokenizer* t, const char* const* r
 int b200_schedule_query(int32_t N, int32_t K, int32_t T, int32_t sms, int32_t* out8);
 /* Host-only: CTAs per (sequence, KV head) the engine gives decode attention when `num_work` sequences decode. */
 int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, int32_t sms);
+/* Host-only: what a rule of csrc/dispatch_rules.h answers for the n sizes v (1 or 0), B200_ERR_INVALID for another rule or count.
+ * B200_RULE_PICKED_ALONE {rows, N, K, bytes a value}: rows that pick their matrix run behind their predecessor, not overlapping it. */
+enum { B200_RULE_PICKED_ALONE = 0 };
+int b200_rule_query(int32_t rule, const int32_t* v, int32_t n);
 /* Debug: subsequent pair-GEMM launches write 8 clock64() phase stamps per CTA into trace_dev (int64[grid][8]);
  * NULL turns it off.  Stamps: 0 entry, 1 after prologue, 2 first tile accumulated, 3 main loop + partial stores
  * done, 4 peers' partials visible, 5 bulk pull landed, 6 before final cluster sync, 7 exit. */

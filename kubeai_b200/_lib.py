@@ -206,6 +206,7 @@ SYMBOLS = {
     "b200_tokenizer_chat_llama3": (C.c_int64, [C.c_void_p, _vp, _vp, _i32, _i32, _vp, C.c_size_t]),
     "b200_schedule_query": (C.c_int, [_i32, _i32, _i32, _i32, _vp]),
     "b200_attn_split_query": (C.c_int, [_i32, _i32, _i32, _i32]),
+    "b200_rule_query": (C.c_int, [_i32, _pi32, _i32]),
     "b200_op_paged_attn_decode_split": (C.c_int, [_vp, _i32, _vp, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _i32, _f, _i32, _vp]),
     "b200_op_paged_attn_prefill_tc": (C.c_int, [_vp, _i32, _i32, _vp, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _i32, _f, _vp]),
     "b200_op_init_uniform": (C.c_int, [_vp, _u64, C.c_uint32, _f, _f, _vp]),

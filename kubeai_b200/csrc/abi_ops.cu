@@ -10,6 +10,7 @@
 #include "../../include/b200engine.h"
 #include "errors.h"
 #include "gemm.h"
+#include "dispatch_rules.h"
 #include "mixers.h"
 #include "gemm3.h"
 #include "epi_pass.cuh"
@@ -274,6 +275,12 @@ int b200_schedule_query(int32_t N, int32_t K, int32_t T, int32_t sms, int32_t* o
   if (N <= 0 || K <= 0 || T <= 0 || sms < 2 || !out8) { set_error("b200_schedule_query: bad arguments"); return B200_ERR_INVALID; }
   gemm2_schedule_query(N, K, T, sms, out8);
   return 0;
+}
+
+int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
+  if (v && rule == B200_RULE_PICKED_ALONE && n == 4) return rules::picked_rows_alone(v[0], v[1], v[2], v[3]);
+  set_error("b200_rule_query: rule %d with %d sizes", rule, n);
+  return B200_ERR_INVALID;
 }
 
 int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, int32_t sms) {

@@ -18,6 +18,7 @@
 
 #include "activations.cuh"
 #include "gemm.h"
+#include "dispatch_rules.h"
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
@@ -425,8 +426,9 @@ int launch_picked(const LinearArgs& a, const PickedRows& p, cudaStream_t st) {
   const bool vec = a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.wbs % 8 == 0 && reinterpret_cast<uintptr_t>(a.X) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(a.W) % 16 == 0;
   dim3 grid((a.N + 7) / 8, p.rows);
-  if (vec) launch_pdl(linear_picked_rows_kernel<TX, TW, TY, 8>, grid, 256, 0, st, a, p);
-  else launch_pdl(linear_picked_rows_kernel<TX, TW, TY, 1>, grid, 256, 0, st, a, p);
+  auto kernel = vec ? linear_picked_rows_kernel<TX, TW, TY, 8> : linear_picked_rows_kernel<TX, TW, TY, 1>;
+  if (rules::picked_rows_alone(p.rows, a.N, a.K, sizeof(TW))) kernel<<<grid, 256, 0, st>>>(a, p);
+  else launch_pdl(kernel, grid, 256, 0, st, a, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

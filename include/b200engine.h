@@ -368,8 +368,9 @@ int b200_schedule_query(int32_t N, int32_t K, int32_t T, int32_t sms, int32_t* o
 /* Host-only: CTAs per (sequence, KV head) the engine gives decode attention when `num_work` sequences decode. */
 int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, int32_t sms);
 /* Host-only: what a rule of csrc/dispatch_rules.h answers for the n sizes v (1 or 0), B200_ERR_INVALID for another rule or count.
- * B200_RULE_PICKED_ALONE {rows, N, K, bytes a value}: rows that pick their matrix run behind their predecessor, not overlapping it. */
-enum { B200_RULE_PICKED_ALONE = 0 };
+ * B200_RULE_PICKED_ALONE {rows, N, K, bytes a value}: rows that pick their matrix run behind their predecessor, not overlapping it.
+ * B200_RULE_KEY_LANES {tokens, heads, the larger head dimension, most keys a token sees, scores capped}: sixteen lanes hold a key. */
+enum { B200_RULE_PICKED_ALONE = 0, B200_RULE_KEY_LANES = 1 };
 int b200_rule_query(int32_t rule, const int32_t* v, int32_t n);
 /* Debug: subsequent pair-GEMM launches write 8 clock64() phase stamps per CTA into trace_dev (int64[grid][8]);
  * NULL turns it off.  Stamps: 0 entry, 1 after prologue, 2 first tile accumulated, 3 main loop + partial stores

@@ -279,6 +279,7 @@ int b200_schedule_query(int32_t N, int32_t K, int32_t T, int32_t sms, int32_t* o
 
 int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_PICKED_ALONE && n == 4) return rules::picked_rows_alone(v[0], v[1], v[2], v[3]);
+  if (v && rule == B200_RULE_KEY_LANES && n == 5) return rules::sixteen_lanes_a_key(static_cast<long long>(v[0]) * v[1], v[2], v[3], v[4] != 0);
   set_error("b200_rule_query: rule %d with %d sizes", rule, n);
   return B200_ERR_INVALID;
 }

@@ -31,6 +31,17 @@ inline bool ensure_dynamic_smem(Kernel kernel, int bytes, std::atomic<unsigned l
   return true;
 }
 
+// SMs of the current device (of this design's part where there is none to ask), looked up once a device
+inline int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if ((sms = known[dev & 63].load(std::memory_order_relaxed)) > 0) return sms;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 148;
+  known[dev & 63].store(sms, std::memory_order_relaxed);
+  return sms;
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args&&... args) {

@@ -195,10 +195,6 @@ int launch(const LinearArgs& a, const LinearPairs& q, int per_cta, int rows, cud
   launch_pdl(linear_stream_kernel<TY, NB, MT, PAIRS>, ctas, kWarps * 32, Layout<NB, MT>::kBytes, st, a, q, per_cta, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
-int sm_count() {
-  int dev = 0, sms = 0;
-  return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? sms : 0;
-}
 // n rows in `parts` shares, whole pairs each
 int share(int n, int parts, bool pairs) { return pairs ? (n / 2 + parts - 1) / parts * 2 : (n + parts - 1) / parts; }
 template <typename TY, int NB, bool PAIRS>
@@ -217,7 +213,6 @@ int pick_rows(const LinearArgs& a, const LinearPairs& q, int sms, cudaStream_t s
 template <typename TY, bool PAIRS>
 int pick_tokens(const LinearArgs& a, const LinearPairs& q, cudaStream_t st) {
   const int sms = sm_count();
-  if (sms < 1) return -2;
   if (a.T <= 8) return pick_rows<TY, 1, PAIRS>(a, q, sms, st);
   if (a.T <= 16) return pick_rows<TY, 2, PAIRS>(a, q, sms, st);
   if (a.T <= 24) return pick_rows<TY, 3, PAIRS>(a, q, sms, st);
@@ -249,7 +244,7 @@ int linear_stream(const LinearArgs& a, const LinearPairs* q, cudaStream_t st) {
 }
 
 int linear_stream_ctas(const LinearArgs& a, const LinearPairs* q) {
-  const int per_cta = share(a.N, std::max(1, sm_count()), q != nullptr);
+  const int per_cta = share(a.N, sm_count(), q != nullptr);
   return (a.N + per_cta - 1) / per_cta;
 }
 

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "dispatch_rules.h"
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
@@ -1026,14 +1027,16 @@ int window_attention(const WindowAttnArgs& a, cudaStream_t st) {
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
-  // B200_WATTN_ROWS=0 keeps single tokens on the general kernel (A/B knob)
+  // B200_WATTN_ROWS: A/B knob, 0 = every other step on the general kernel, 1 = on the other one wherever that takes its sizes
   const char* re = getenv("B200_WATTN_ROWS");
-  if (!(re && atoi(re) == 0) && a.t == DT_BF16 && a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && reinterpret_cast<uintptr_t>(a.cache) % 16 == 0) {
+  const long long seen = a.chunk > 0 ? a.chunk : static_cast<long long>(a.window) + a.keep_first;
+  if ((re ? atoi(re) != 0 : rules::sixteen_lanes_a_key(static_cast<long long>(a.T) * a.heads, std::max(a.dim, a.vdim), std::min<long long>(seen, a.max_ctx), a.softcap > 0.f)) &&
+      a.t == DT_BF16 && a.dim % 8 == 0 && a.vdim % 8 == 0 && a.dim <= 128 && a.vdim <= 128 && reinterpret_cast<uintptr_t>(a.cache) % 16 == 0) {
     // as many heads of a group to a CTA as keep every SM busy; the result does not depend on it
     const int group = a.heads / a.kv_heads;
     int gs = 1;
     for (int c = 2; c <= 8; c *= 2)
-      if (group % c == 0 && static_cast<long long>(a.T) * a.heads / c >= 2 * 148) gs = c;
+      if (group % c == 0 && static_cast<long long>(a.T) * a.heads / c >= 2 * sm_count()) gs = c;
     int page_shift = -1;
     for (int b = 0; b < 31; ++b) if ((1 << b) == a.page) page_shift = b;
     const unsigned grid = static_cast<unsigned>(static_cast<long long>(a.T) * (a.heads / gs));

@@ -102,7 +102,7 @@ int b200_op_linear_rows(const void* x, const void* w, void* y, const float* bias
   q.kind = act == 4 ? PAIRS_SILU : PAIRS_GATED;
   q.limit = p0; q.slope = p1; q.up_offset = p2;
   if (act < 3) { a.act = act == 1 ? LIN_RELU2 : act == 2 ? LIN_XIELU : LIN_NONE; a.a_pos = p0; a.a_neg = p1; }
-  if (!x || !w || !y || act < 0 || act > 4 || ldx < K || ldw < K || ldy < (act < 3 ? N : N / 2) || !(act < 3 ? linear_few(a) : linear_streams(a, &q))) {
+  if (!x || !w || !y || act < 0 || act > 4 || ldx < K || ldw < K || ldy < (act < 3 ? N : N / 2) || !(act < 3 ? linear_streams(a) || linear_clusters(a) : linear_streams(a, &q))) {
     set_error("b200_op_linear_rows: not served (T=%d N=%d K=%d act=%d)", T, N, K, act);
     return B200_ERR_INVALID;
   }
@@ -227,7 +227,7 @@ int b200_op_gemm3(const b200_gemm3_args* a, void* stream, int32_t* schedule_out)
     la.ldy = a->ldo;
     LinearPairs q;
     q.kind = PAIRS_SILU;
-    if (gemm_variant() == 2 && a->N % 256 == 0 && a->K % 64 == 0 && linear_streams(la, &q)) {
+    if (gemm_variant() == 2 && a->N % 256 == 0 && a->K % 64 == 0 && linear_few(la, &q)) {
       if (schedule_out) { schedule_out[0] = 0; schedule_out[1] = 0; schedule_out[2] = linear_stream_ctas(la, &q); }
       const int rs = linear_stream(la, &q, st);
       return rs ? cuda_fail("linear_stream", rs) : 0;
@@ -280,6 +280,8 @@ int b200_schedule_query(int32_t N, int32_t K, int32_t T, int32_t sms, int32_t* o
 int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_PICKED_ALONE && n == 4) return rules::picked_rows_alone(v[0], v[1], v[2], v[3]);
   if (v && rule == B200_RULE_KEY_LANES && n == 5) return rules::sixteen_lanes_a_key(static_cast<long long>(v[0]) * v[1], v[2], v[3], v[4] != 0);
+  if (v && rule == B200_RULE_STREAM && n == 4) return rules::stream_pays(v[0], v[1], v[2], v[3] != 0);
+  if (v && rule == B200_RULE_CLUSTER && n == 3) return rules::cluster_pays(v[0], v[1], v[2]);
   set_error("b200_rule_query: rule %d with %d sizes", rule, n);
   return B200_ERR_INVALID;
 }

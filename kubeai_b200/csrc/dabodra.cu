@@ -700,7 +700,7 @@ class Dabodra : public Model {
       sg.ldy = s.sff;
       LinearPairs unit;
       unit.limit = INFINITY;
-      if (w.il_s && linear_streams(sg, &unit)) {
+      if (w.il_s && linear_few(sg, &unit)) {
         KRN("shared_in", linear_stream(sg, &unit, st));
       } else if (w.il_s && takes_whole(w.tc_shin, T)) {
         KRN("shared_in", run_whole(w.p_shin, xm_h, true, shact, s.sff, T));     // the gated unit in the epilogue

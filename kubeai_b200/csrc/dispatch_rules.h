@@ -30,5 +30,23 @@ inline bool sixteen_lanes_a_key(long long units, int width, long long keys, bool
   return width > 64 && !cap && keys >= 64;
 }
 
+// Products of few rows that have a whole-tile form too: where the passes over the weights (linear_stream.cu) and the clusters
+// (linear_cluster.cu) are still ahead of it.  Both read all of X in every CTA, T * K values through each SM's port, and a long K makes
+// that the larger part.  Ratio of their time to the whole tiles', weights from HBM; N rows of W, passes:
+//   K 4096   40 tokens, N 1024 .. 4736 0.67 .. 0.82     K 8192   N 64 .. 4736 0.82 .. 1.0      K 14336  N 64 .. 3168 1.06 .. 1.18, 4096 0.95
+//   K 14336  32 tokens, N 64 .. 3168 0.77 .. 0.93       K 28672  N 64 .. 1536 1.06 .. 1.20, 2048 0.95     16 tokens, N 64 .. 3168 0.80 .. 1.0
+// In a design's step (ff_down, us, whole tiles / here): 1024 x 28672 40 tokens 33 / 51, 200 tokens 57 / 71; 2048 x 14336 24 tokens 29 / 20, 100 tokens 35 / 32.
+//   pairs of rows (against the kernel of a decode step's pairs), 7168 x 16384: 24 tokens 46.4 / 49.9 us, 32 tokens 53.0 / 50.0
+// Llama-3-8B's down projection (4096 x 14336) and the norm behind it, 33 to 48 tokens: a step of 4 layers 530 .. 537 us, fused 580 .. 584.
+inline bool stream_pays(int T, int N, int K, bool pairs) {
+  if (K <= 8192) return true;
+  if (pairs) return T <= 24;
+  return T <= 16 || (T <= 32 ? K <= 16384 || N >= 2048 : N >= 4096);
+}
+// clusters, 49 .. 256 tokens:
+//   K 4096   N 1024 .. 2112 0.67 .. 0.83, 2560 .. 3168 0.77 .. 0.91     K 8192   0.73 .. 0.93, 0.93 .. 1.08
+//   K 14336  0.83 .. 1.08 (to 128 tokens), 1.0 .. 1.12 (129 on); 1.08 .. 1.19     K 28672  1.12 .. 1.52, 1.28 .. 1.42
+inline bool cluster_pays(int T, int N, int K) { return K <= (N > 2112 ? 6144 : T <= 128 ? 16384 : 10240); }
+
 }  // namespace rules
 }  // namespace b200

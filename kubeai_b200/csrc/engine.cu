@@ -1001,7 +1001,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     pairs.heads = Hq; pairs.kv_heads = Hkv; pairs.max_pos = cfg.max_model_len;
     const LinearArgs qa = product(normed, ly.wqkv, qkv, QKV, T, QKV, H);
     P(B200_K_GEMM_QKV);
-    if (few && linear_streams(qa, &pairs)) {
+    if (few && linear_few(qa, &pairs)) {
       if (on(B200_K_GEMM_QKV)) rc |= linear_stream(qa, &pairs, stream);
     } else {
       Gemm3Params p = base(ly.p_qkv, xmap(xm_normed, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_ROPE_KV);
@@ -1013,7 +1013,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     if (m.nd) { P(B200_K_ATTN_DECODE); if (on(B200_K_ATTN_DECODE)) rc |= decode_attention(m, kv_l, btab, dwork, scale); Q(); ++stats.kernel_launches; }
     if (m.np) { P(B200_K_ATTN_PREFILL); if (on(B200_K_ATTN_PREFILL)) rc |= prefill_attention(kv_l, btab, pwork, m.np, scale); Q(); ++stats.kernel_launches; }
     const LinearArgs oa = product(attn, ly.wo, x, H, T, H, Hq * kD);
-    if (few && linear_streams(oa)) {
+    if (few && linear_few(oa)) {
       P(B200_K_GEMM_O); if (on(B200_K_GEMM_O)) rc |= linear_stream(oa, nullptr, stream); Q();
       P(B200_K_NORM); if (on(B200_K_NORM)) rc |= rmsnorm(x, res, ly.norm2, normed, nullptr, T, H, cfg.rms_eps, stream); Q();
       ++stats.kernel_launches;
@@ -1027,7 +1027,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     unit.kind = PAIRS_SILU;
     const LinearArgs ga = product(normed, ly.wgu, act, I, T, 2 * I, H);
     P(B200_K_GEMM_GU);
-    if (few && linear_streams(ga, &unit)) {
+    if (few && linear_few(ga, &unit)) {
       if (on(B200_K_GEMM_GU)) rc |= linear_stream(ga, &unit, stream);
     } else {
       Gemm3Params p = base(ly.p_gu, xmap(xm_normed, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_SILU);
@@ -1037,7 +1037,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     Q();
     const LinearArgs da = product(act, ly.wdown, x, H, T, H, I);
     P(B200_K_GEMM_DOWN);
-    if (few && linear_streams(da)) {
+    if (few && linear_few(da)) {
       if (on(B200_K_GEMM_DOWN)) rc |= linear_stream(da, nullptr, stream);
       x_pending = true;
     } else {
@@ -1054,7 +1054,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     // the final norm of the sampled rows: plain where the residual already holds the summed stream
     P(B200_K_NORM); rc |= rmsnorm(x_pending ? x : res, x_pending ? res : nullptr, final_norm, last_hidden, rows, m.S, H, cfg.rms_eps, stream); Q();
     const LinearArgs la = product(last_hidden, lm_head, logits, V, m.S, V, H);
-    const bool stream_lm = few && linear_streams(la);
+    const bool stream_lm = few && linear_few(la);
     P(B200_K_GEMM_LM);
     if (stream_lm) {
       rc |= linear_stream(la, nullptr, stream);

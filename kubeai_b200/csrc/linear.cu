@@ -495,6 +495,11 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
 
 }  // namespace
 
+bool linear_few(const LinearArgs& a, const LinearPairs* q) {
+  if (linear_streams(a, q)) return rules::stream_pays(a.T, a.N, a.K, q != nullptr);
+  return !q && linear_clusters(a) && rules::cluster_pays(a.T, a.N, a.K);
+}
+
 int linear(const LinearArgs& a, cudaStream_t st) {
   if (a.T <= 0 || a.N <= 0) return 0;
   if (!a.X || !a.W || !a.Y || a.K <= 0 || a.batch < 1) return -1;

@@ -228,10 +228,12 @@ int pick_tokens(const LinearArgs& a, const LinearPairs& q, cudaStream_t st) {
 //   1792 x 2048:   8 tokens 3.0 /  8.3   32 tokens  4.1 /  9.5   48 tokens  5.5 / 10.4
 //   8192 x 2048:   8 tokens 6.6 / 11.7   32 tokens  9.4 / 12.4   48 tokens 13.2 / 13.4
 //   28672 x 4096:  8 tokens 36.1 / 42.5  16 tokens 39.0 / 43.0, in a second of nothing else 38.5 / 43.5 and 43.7 / 44.0
-// More tokens cost their rows once a CTA and block of its rows, which is what narrow matrices can afford longest.
+// More tokens cost their rows once a CTA and block of its rows, which is what narrow matrices can afford longest.  With a long K the
+// whole tiles win earlier (rules::stream_pays); a product without a plan for them still comes here.
 bool linear_streams(const LinearArgs& a, const LinearPairs* q) {
   static const int most = [] { const char* e = getenv("B200_LIN_STREAM"); return e ? atoi(e) : 48; }();     // A/B knob: the most rows, 0: none
-  if (a.T > most || a.T > (a.N <= 32 * 148 ? 48 : a.N <= 80 * 148 ? 32 : 8)) return false;
+  const int sms = sm_count();
+  if (a.T > most || a.T > (a.N <= 32 * sms ? 48 : a.N <= 80 * sms ? 32 : 8)) return false;
   if (q && (a.N % 128 || a.ty != DT_BF16 || a.bias || a.row_scale || a.act != LIN_NONE)) return false;
   return a.T > 0 && a.N > 0 && a.K > 0 && a.tx == DT_BF16 && a.tw == DT_BF16 && a.batch == 1 && !a.x_rows && !a.tile_group && a.K % 8 == 0 && a.ldx % 8 == 0 &&
          a.ldw % 8 == 0 && (reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.W)) % 16 == 0;

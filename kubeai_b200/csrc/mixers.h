@@ -77,7 +77,8 @@ int linear_stream(const LinearArgs& a, const LinearPairs* q, cudaStream_t st);
 // `linear` takes it wherever it serves, with the same promise about W.
 bool linear_clusters(const LinearArgs& a);
 int linear_cluster(const LinearArgs& a, cudaStream_t st);
-inline bool linear_few(const LinearArgs& a) { return linear_streams(a) || linear_clusters(a); }
+// Which of them a product that also has a whole-tile form should take; without one (`linear`), either is ahead of what is left.
+bool linear_few(const LinearArgs& a, const LinearPairs* q = nullptr);
 int linear_stream_ctas(const LinearArgs& a, const LinearPairs* q);   // CTAs such a launch has on this device
 // `rows` rows (a handful: the expert choices of a decode step), row r reading X row src_rows[r] (or r / src_div), writing Y row
 // dst_rows[r], with weight matrix W + groups[r] * wbs (row_scale[r] applies); a.T, a.batch, x_rows and tile_group are not used.

@@ -724,7 +724,7 @@ class Mulenex : public Model {
       sg.ldy = s.sff;
       LinearPairs unit;
       unit.limit = INFINITY;
-      if (w.il_s && linear_streams(sg, &unit)) {
+      if (w.il_s && linear_few(sg, &unit)) {
         KRN("shared_in", linear_stream(sg, &unit, st));
       } else if (w.il_s && w.tc_shin && gemm_whole_fits(w.p_shin, shact, s.sff)) {
         const GroupedOut o = {shact, s.sff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};     // the gated unit in the epilogue

@@ -6,7 +6,7 @@ import pytest
 
 from kubeai_b200._lib import lib
 
-PICKED_ALONE, KEY_LANES = range(2)
+PICKED_ALONE, KEY_LANES, STREAM, CLUSTER = range(4)
 
 
 def rule(which, *v):
@@ -36,3 +36,18 @@ def test_large_streams_of_picked_rows_run_behind_their_predecessor(rows, N, K, a
 def test_sixteen_lanes_hold_a_key_where_that_is_faster(tokens, heads, width, keys, cap, lanes):
     """Everywhere, they took 294 us against 124 for 8 heads of 8 over 16000 keys, and 56 against 36 for 100 tokens of up to 10 keys, 32 capped heads of 128."""
     assert rule(KEY_LANES, tokens, heads, width, keys, cap) == lanes
+
+
+@pytest.mark.parametrize("T,N,K,pairs,pays", [(48, 2048, 8192, 0, 1), (40, 1024, 14336, 0, 0), (48, 3168, 14336, 0, 0), (40, 4096, 14336, 0, 1), (48, 4096, 14336, 0, 1), (32, 2048, 14336, 0, 1),
+                                               (32, 1024, 28672, 0, 0), (32, 2048, 28672, 0, 1), (16, 1024, 28672, 0, 1), (48, 1024, 28672, 0, 0), (8, 576, 28672, 0, 1),
+                                               (24, 7168, 16384, 1, 1), (32, 7168, 16384, 1, 0), (32, 7168, 8192, 1, 1), (8, 28672, 4096, 1, 1)])
+def test_passes_over_the_weights_end_where_a_long_k_makes_x_the_larger_part(T, N, K, pairs, pays):
+    """Lines drawn by T and N alone sent 40 rows of 1024 x 28672 through them: 49 us against 33 in whole tiles."""
+    assert rule(STREAM, T, N, K, pairs) == pays
+
+
+@pytest.mark.parametrize("T,N,K,pays", [(100, 2048, 2048, 1), (256, 2112, 8192, 1), (100, 1024, 14336, 1), (129, 1024, 14336, 0), (100, 2048, 28672, 0), (64, 3072, 4096, 1), (64, 3072, 8192, 0),
+                                         (128, 3168, 648, 1)])
+def test_clusters_end_there_too(T, N, K, pays):
+    """129 rows of 2048 x 28672: 72 us in clusters, 53 in whole tiles."""
+    assert rule(CLUSTER, T, N, K) == pays

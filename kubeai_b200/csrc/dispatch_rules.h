@@ -1,6 +1,7 @@
 // Rules that choose between two kernels with the same result by the sizes of a call alone, as plain host functions: the kernels'
 // launchers use them, and b200_rule_query answers from them without a GPU.
 #pragma once
+#include <math.h>
 
 namespace b200 {
 namespace rules {
@@ -47,6 +48,23 @@ inline bool stream_pays(int T, int N, int K, bool pairs) {
 //   K 4096   N 1024 .. 2112 0.67 .. 0.83, 2560 .. 3168 0.77 .. 0.91     K 8192   0.73 .. 0.93, 0.93 .. 1.08
 //   K 14336  0.83 .. 1.08 (to 128 tokens), 1.0 .. 1.12 (129 on); 1.08 .. 1.19     K 28672  1.12 .. 1.52, 1.28 .. 1.42
 inline bool cluster_pays(int T, int N, int K) { return K <= (N > 2112 ? 6144 : T <= 128 ? 16384 : 10240); }
+
+// Mamba-2 prompts (scan_chunk.cu): sequences cut into segments of 256 tokens, or one chain of 64-token chunks each.  Times in chunks
+// of a chain's CTA with a second one on its SM (13.4 us at 128 state rows; alone on its SM 0.83 of that).  A chain takes its longest
+// sequence, and where not all CTAs (heads, column blocks) run at once as many rounds of equal ones, or the sum of unequal ones and a part of the
+// longest, which comes last at worst; the segments' three launches take about 3 to 5 and then 4 to 4.5 for every time that all of them fill the device.  us, segments / chains, 64 columns, 128 state rows:
+//   8 heads   1 x 4096 83 / 691    6 x 682 89 / 128        64 heads   1 x 512 89 / 97    1 x 4096 269 / 721    3 x 1365 279 / 289
+//   32 heads  4 x 512 103 / 98     6 x 682 162 / 147                  4 x 512 171 / 114  4 x 1024 270 / 217    6 x 682 274 / 281
+//   128 heads 1 x 1024 167 / 185   2 x 512 168 / 113       256 heads  1 x 512 169 / 115  1 x 4096 911 / 823    3 x 1365 965 / 882
+//   unequal: 64 heads 455 + 1365 + 2275 277 / 461; 128 heads 300 + 700 + 1100 + 2000 499 / 550; 256 heads 300 + 2000 561 / 484
+// longest 0: not known, all taken as equal.  From seven sequences on, or with a mean below 512, chains.
+inline bool segments_pay(long long T, int nseq, int longest, int heads, int blocks, int dim, int slots, int sms) {
+  if (nseq < 1 || nseq > 6 || T < 512LL * nseq) return false;
+  const double mean = T / 64.0 / nseq, most = ceil(longest > 0 ? longest / 64.0 : mean), per_slot = static_cast<double>(heads) * blocks / slots, rounds = ceil(nseq * per_slot);
+  const double chain = rounds <= 1 ? (nseq * heads * blocks <= sms ? 0.83 : 1.0) * most : most <= 1.1 * mean + 1 ? rounds * most : fmax(most, T / 64.0 * per_slot + 0.7 * fmax(0.0, 1.0 - per_slot) * most);
+  const double fills = (T / 256.0 + nseq / 2.0) * per_slot;
+  return (dim <= 32 ? 5.5 + 4.2 * fills : 2.7 + dim / 128.0 + (3.55 + 0.9 * dim / 128.0) * fills) < chain + 0.7;
+}
 
 }  // namespace rules
 }  // namespace b200

@@ -166,12 +166,13 @@ struct GlaArgs {
   // workspace of the form whose chunks run side by side (scan_parallel.cu); without it, or where it is too small, the step's
   // tokens run in a chain
   float* par_ws = nullptr; size_t par_ws_floats = 0;
+  int max_rows = 0;   // most tokens that a sequence brings (0: not known)
 };
 int gla_scan(const GlaArgs& a, cudaStream_t st);
 // The chunked tensor-core form of the dt_pre scan (scan_chunk.cu; same result up to fp32 rounding), for the shapes it takes;
 // gla_scan chooses it for bf16 steps of prompt portions.
 bool scan_chunk_fits(const GlaArgs& a);
-// floats of par_ws with which it cuts few long sequences into segments that run side by side
+// floats of par_ws with which it cuts up to six long sequences into segments that run side by side
 size_t scan_segments_ws_floats(int tokens, int seqs, int heads, int dim, int vdim);
 int scan_chunk(const GlaArgs& a, cudaStream_t st);
 // The form whose chunks run side by side (scan_parallel.cu; same result up to fp32 rounding), likewise chosen by gla_scan; its

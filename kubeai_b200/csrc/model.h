@@ -33,6 +33,7 @@ struct StepBatch {
   int max_blocks = 0;
   bool fresh = false;               // every sequence of the step starts at its first token
   int max_ctx = 0;                  // longest context in the step: max over sequences of first position + rows
+  int max_rows = 0;                 // most rows of a sequence in the step
 };
 
 struct ModelEnv {

@@ -14,7 +14,7 @@
 // Few long sequences leave most of the device to a chain of chunks on few CTAs.  They are cut into segments of kSegment
 // tokens: the sums of all segments at once (PART_SUMS), a pass that turns them into incoming states, the outputs of all segments at
 // once (PART_OUT).  64 heads of 128 x 64, 3 sequences of 455, 1365 and 2275 tokens: one chain each (PART_ALL) 460 us, segments 270.
-// The sums cost a third of the products again, so sequences enough to fill the device stay whole (segments_pay).
+// The sums cost a third of the products again, so sequences whose chains fill the device stay whole (rules::segments_pay).
 //
 // One CTA owns 64 value columns of a (head, sequence or segment) and walks its chunks: 4 warps, each with 16 value columns.  The state
 // lives transposed (value columns x state rows) in the warps' accumulators, which are the left operand of the next chunk's
@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "dispatch_rules.h"
 #include "launch.h"
 #include "mixers.h"
 #include "mma_frag.cuh"
@@ -344,19 +345,23 @@ int launch_part(const GlaArgs& a, const Segments& sg, dim3 grid, cudaStream_t st
   scalar_decay_chunk_kernel<NK, PART><<<grid, kThreads, chunk_smem(a.dim), st>>>(a, sg);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
-// Segments where the chains of whole sequences would leave SMs idle, and their workspace is there.
-bool segments_pay(const GlaArgs& a) {
+// Segments where they are the shorter way (slots: CTAs of the chain that run at once), and their workspace is there.
+bool cut_into_segments(const GlaArgs& a, int slots) {
   const char* e = getenv("B200_SCAN_SEGMENTS");      // A/B knob: 0 = never, 1 = wherever they fit
   const int force = e ? atoi(e) : -1;
   if (force == 0 || !a.par_ws || scan_segments_ws_floats(a.T, a.nseq, a.heads, a.dim, a.vdim) > a.par_ws_floats || a.vdim % 4 ||
       (reinterpret_cast<uintptr_t>(a.par_ws) | reinterpret_cast<uintptr_t>(a.states)) % 16) return false;
-  return force == 1 || (a.T >= 2 * kSegment * a.nseq && a.nseq <= 6);
+  return force == 1 || rules::segments_pay(a.T, a.nseq, a.max_rows, a.heads, (a.vdim + kCols - 1) / kCols, a.dim, slots, sm_count());
 }
 template <int NK>
 int launch(const GlaArgs& a, cudaStream_t st) {
   const int cb = (a.vdim + kCols - 1) / kCols;
   Segments sg = {nullptr, nullptr};
-  if (!segments_pay(a)) return launch_part<NK, PART_ALL>(a, sg, dim3(cb, a.heads, a.nseq), st);
+  static std::atomic<unsigned long long> attr{0};
+  int per_sm = 0;
+  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK, PART_ALL>, static_cast<int>(chunk_smem(16 * NK)), &attr) ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scalar_decay_chunk_kernel<NK, PART_ALL>, kThreads, chunk_smem(a.dim)) != cudaSuccess) return -2;
+  if (!cut_into_segments(a, std::max(1, per_sm) * sm_count())) return launch_part<NK, PART_ALL>(a, sg, dim3(cb, a.heads, a.nseq), st);
   const int segs = a.T / kSegment + a.nseq;
   sg.s = a.par_ws;
   sg.d = sg.s + static_cast<size_t>(segs) * a.heads * a.dim * a.vdim;

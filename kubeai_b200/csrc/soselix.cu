@@ -693,7 +693,7 @@ class Soselix : public Model {
     g.t = dt; g.inv_tau = 1.f; g.q_scale = 1.f; g.T = b.T;
     g.states = r.state; g.seqs = b.seqs; g.nseq = b.nseq;
     g.heads = s.heads; g.dim = s.dim; g.vdim = s.vdim; g.o = o32;
-    g.par_ws = scan_ws; g.par_ws_floats = scan_ws_floats;
+    g.par_ws = scan_ws; g.par_ws_floats = scan_ws_floats; g.max_rows = b.max_rows;
     return g;
   }
 

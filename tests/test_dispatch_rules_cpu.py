@@ -6,7 +6,7 @@ import pytest
 
 from kubeai_b200._lib import lib
 
-PICKED_ALONE, KEY_LANES, STREAM, CLUSTER = range(4)
+PICKED_ALONE, KEY_LANES, STREAM, CLUSTER, SEGMENTS = range(5)
 
 
 def rule(which, *v):
@@ -51,3 +51,21 @@ def test_passes_over_the_weights_end_where_a_long_k_makes_x_the_larger_part(T, N
 def test_clusters_end_there_too(T, N, K, pays):
     """129 rows of 2048 x 28672: 72 us in clusters, 53 in whole tiles."""
     assert rule(CLUSTER, T, N, K) == pays
+
+
+# heads, column blocks, state rows, sequences, tokens of each
+@pytest.mark.parametrize("heads,blocks,dim,nseq,each,cut", [
+    (8, 1, 128, 1, 4096, 1), (8, 1, 128, 6, 682, 1), (16, 1, 128, 4, 1024, 1), (32, 1, 128, 4, 512, 0), (32, 1, 128, 6, 682, 0), (32, 1, 128, 4, 1024, 1),
+    (64, 1, 128, 1, 512, 1), (64, 1, 128, 1, 4096, 1), (64, 1, 128, 2, 512, 0), (64, 1, 128, 3, 1365, 1), (64, 1, 128, 4, 512, 0), (64, 1, 128, 4, 1024, 0),
+    (128, 1, 128, 1, 1024, 1), (128, 1, 128, 2, 512, 0), (128, 1, 128, 2, 2048, 0), (128, 1, 128, 4, 1024, 0), (256, 1, 128, 1, 512, 0), (256, 1, 128, 1, 4096, 0),
+    (256, 1, 128, 3, 1365, 0), (32, 2, 128, 4, 512, 0), (64, 4, 64, 1, 512, 0), (64, 1, 16, 5, 820, 0), (64, 1, 16, 1, 4096, 1), (8, 1, 128, 7, 1024, 0), (8, 1, 128, 4, 500, 0)])
+def test_sequences_are_cut_where_their_chains_leave_the_device_idle(heads, blocks, dim, nseq, each, cut):
+    """By sequences and tokens alone, four of 512 tokens with 64 heads were cut: 171 us against 114 in chains."""
+    for longest in (each, 0):
+        assert rule(SEGMENTS, nseq * each, nseq, longest, heads, blocks, dim, 444 if dim <= 32 else 296, 148) == cut
+
+
+def test_a_chain_is_as_long_as_its_longest_sequence():
+    assert rule(SEGMENTS, 4095, 3, 2275, 64, 1, 128, 296, 148) == 1 and rule(SEGMENTS, 4096, 4, 3000, 64, 1, 128, 296, 148) == 1
+    assert rule(SEGMENTS, 4100, 4, 2000, 128, 1, 128, 296, 148) == 1 and rule(SEGMENTS, 2300, 2, 2000, 256, 1, 128, 296, 148) == 0
+    assert rule(SEGMENTS, 4000, 6, 1200, 64, 1, 128, 296, 148) == 1 and rule(SEGMENTS, 4000, 6, 1200, 128, 1, 128, 296, 148) == 0

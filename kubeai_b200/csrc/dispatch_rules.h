@@ -66,5 +66,11 @@ inline bool segments_pay(long long T, int nseq, int longest, int heads, int bloc
   return (dim <= 32 ? 5.5 + 4.2 * fills : 2.7 + dim / 128.0 + (3.55 + 0.9 * dim / 128.0) * fills) < chain + 0.7;
 }
 
+// Norms between sublayers (hyper.cu): a row of 256 threads times `pieces` of four columns in registers through both sums, or read from
+// memory again behind each.  Three and four pieces leave an SM two rows at a time: ahead while that holds all rows there are (steps), behind
+// where many follow.  us of 9 launches, again / registers, 4096 wide: 1 row 55 / 42, 148 rows 51 / 41, 444 52 / 52, 900 69 / 74, 4000 196 / 232;
+// 2560 wide: 148 48 / 39, 444 49 / 50, 600 51 / 58, 4000 144 / 183.  More than four would spill.
+inline bool row_in_registers(int pieces, int rows, int sms) { return pieces <= 2 || (pieces <= 4 && rows <= 3 * sms); }
+
 }  // namespace rules
 }  // namespace b200

@@ -24,6 +24,7 @@
 
 #include <vector>
 
+#include "dispatch_rules.h"
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
@@ -553,9 +554,10 @@ int sandwich_step(const SandwichArgs& a, cudaStream_t st) {
   auto al16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool vec = a.W % 4 == 0 && al16(a.x) && al16(a.y) && al16(a.h) && al16(a.y_bias) && al16(a.post_w) && al16(a.pre_w);
   const int th = vec ? (a.W >= 1024 ? 256 : (a.W >= 512 ? 128 : 64)) : threads_for(a.W);
-  const int pieces = vec ? (a.W + 4 * th - 1) / (4 * th) : 0;     // more than four a thread would take too many registers
+  const int pieces = vec ? (a.W + 4 * th - 1) / (4 * th) : 0;
+  const bool held = vec && rules::row_in_registers(pieces, a.rows, sm_count());
 #define SW(TY, TH) do { if (pieces == 1) launch_pdl(sandwich_rows_kernel<TY, TH, 1>, a.rows, th, 0, st, a); else if (pieces == 2) launch_pdl(sandwich_rows_kernel<TY, TH, 2>, a.rows, th, 0, st, a); \
-  else if (vec && pieces <= 4) launch_pdl(sandwich_rows_kernel<TY, TH, 4>, a.rows, th, 0, st, a); else if (vec) launch_pdl(sandwich_step_kernel<TY, TH, true>, a.rows, th, smem, st, a); else launch_pdl(sandwich_step_kernel<TY, TH, false>, a.rows, th, smem, st, a); } while (0)
+  else if (held) launch_pdl(sandwich_rows_kernel<TY, TH, 4>, a.rows, th, 0, st, a); else if (vec) launch_pdl(sandwich_step_kernel<TY, TH, true>, a.rows, th, smem, st, a); else launch_pdl(sandwich_step_kernel<TY, TH, false>, a.rows, th, smem, st, a); } while (0)
   const bool y16 = a.y && a.ty == DT_BF16, h16 = a.h && a.th == DT_BF16;
   if (y16 && h16) SW(bf16, bf16);
   else if (y16) SW(bf16, float);

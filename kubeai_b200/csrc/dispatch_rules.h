@@ -72,5 +72,14 @@ inline bool segments_pay(long long T, int nseq, int longest, int heads, int bloc
 // 2560 wide: 148 48 / 39, 444 49 / 50, 600 51 / 58, 4000 144 / 183.  More than four would spill.
 inline bool row_in_registers(int pieces, int rows, int sms) { return pieces <= 2 || (pieces <= 4 && rows <= 3 * sms); }
 
+// Products per head of 17 to 128 rows (linear.cu): blocks of 16 rows that read the weights from L2 again, or tiles of 64 rows that walk K in
+// a chain.  What the blocks cost is those bytes, what the tiles cost is K.  us, tiles / blocks: 128 x 512 (rows of W 512, bf16 rows of X)
+// 16 heads 64 rows 12.1 / 11.1, 128 rows 12.7 / 14.5; 32 heads 32 rows 12.5 / 12.6, 100 rows 14.9 / 18.8; 64 heads 128 rows 23.9 / 31.2; K 64,
+// 32 heads 100 rows 10.0 / 13.1, 64 heads 48 rows 9.7 / 10.9, 128 rows 13.7 / 17.4.  Rows of X in fp32, K 512 to 128 columns: 16 heads 21 / 11, 64 heads 64 rows 23.5 / 17.2, 100 rows
+// 25.1 / 24.7, 128 rows 25.5 / 27.6; K 256, 64 heads 128 rows 15.3 / 13.0.
+inline bool row_blocks_pay(int rows, long long batch, long long N, long long K, bool fp32_rows) {
+  return (rows + 15) / 16 * batch * N * K * 2 <= (fp32_rows ? 60000000 : K >= 128 ? 8500000 : 3000000);
+}
+
 }  // namespace rules
 }  // namespace b200

@@ -303,7 +303,7 @@ __device__ __forceinline__ uint4 ldx8(const float* p, uint4* lo) {
   return make_uint4(h[0], h[1], h[2], h[3]);
 }
 
-// More rows than 8 * NB (one product per head, steps of up to 128 tokens): grid row y takes its own 8 * NB, the weights come from L2
+// More rows than 8 * NB (one product per head, steps of up to 128 tokens, rules::row_blocks_pay): grid row y takes its own 8 * NB, the weights come from L2
 // again; an fp32 X is rounded to one bf16 term, as in the 64-row tiles above that these steps used.  16 heads, 512 x 128 and 128 x 512,
 // 100 rows: 22 us and 9 on the tiles, 9 and 8 here; 40 rows 23 and 9, 7 and 6.
 // THIN: the same with the operands' parts exchanged, for many rows of X against few rows of W (router logits, scalar gates):
@@ -440,7 +440,7 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
     static const int mma_rows = [] { const char* e = getenv("B200_LIN_MMA_ROWS"); return e ? std::min(16, std::max(0, atoi(e))) : 16; }();
     const bool vec = a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.xbs % 8 == 0 && a.wbs % 8 == 0 &&
                      reinterpret_cast<uintptr_t>(a.X) % 16 == 0 && reinterpret_cast<uintptr_t>(a.W) % 16 == 0;
-    if (vec && (a.T <= mma_rows || (a.batch > 1 && mma_rows == 16 && a.T <= 128)) && !a.x_rows && !a.tile_group) {
+    if (vec && (a.T <= mma_rows || (a.batch > 1 && mma_rows == 16 && a.T <= 128 && rules::row_blocks_pay(a.T, a.batch, a.N, a.K, sizeof(TX) == 4))) && !a.x_rows && !a.tile_group) {
       const int steps = (a.K + 31) / 32;
       const int KS = steps >= 32 ? 8 : (steps >= 16 ? 4 : (steps >= 8 ? 2 : 1));
       dim3 grid((a.N + 128 / KS - 1) / (128 / KS), a.T <= 8 ? 1 : (a.T + 15) / 16, a.batch);

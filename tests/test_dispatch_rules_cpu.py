@@ -6,7 +6,7 @@ import pytest
 
 from kubeai_b200._lib import lib
 
-PICKED_ALONE, KEY_LANES, STREAM, CLUSTER, SEGMENTS, ROW_REGISTERS = range(6)
+PICKED_ALONE, KEY_LANES, STREAM, CLUSTER, SEGMENTS, ROW_REGISTERS, ROW_BLOCKS = range(7)
 
 
 def rule(which, *v):
@@ -75,3 +75,11 @@ def test_a_chain_is_as_long_as_its_longest_sequence():
 def test_wide_rows_stay_in_registers_in_steps_and_not_in_prompts(pieces, rows, held):
     """4000 rows of 4096 held in registers took 232 us in nine launches, 196 read again behind each sum."""
     assert rule(ROW_REGISTERS, pieces, rows, 148) == held
+
+
+@pytest.mark.parametrize("rows,heads,N,K,fp32,blocks", [(64, 16, 512, 128, 0, 1), (128, 16, 512, 128, 0, 0), (32, 32, 512, 128, 0, 1), (100, 32, 512, 128, 0, 0), (128, 64, 512, 128, 0, 0),
+                                                         (128, 4, 512, 128, 0, 1), (128, 64, 256, 64, 0, 0), (100, 32, 256, 64, 0, 0), (64, 16, 256, 64, 0, 1), (100, 16, 128, 512, 1, 1), (64, 64, 128, 512, 1, 1), (128, 64, 128, 512, 1, 0),
+                                                         (128, 64, 64, 256, 1, 1)])
+def test_products_per_head_in_blocks_of_rows_while_their_reads_of_the_weights_are_few(rows, heads, N, K, fp32, blocks):
+    """Whatever the heads, 100 rows of 32 heads, 128 to 512 columns, took 18.8 us in blocks against 14.9 in tiles."""
+    assert rule(ROW_BLOCKS, rows, heads, N, K, fp32) == blocks

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 
+#include "dispatch_rules.h"
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
@@ -268,10 +269,11 @@ int delta_scan(const DeltaArgs& a, cudaStream_t st) {
     const int from = e ? atoi(e) : 8;
     if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return delta_chunk(a, st);
   }
-  // B200_SCAN_STEP=0 keeps single tokens in the scan (A/B knob); fp32 models stay there, whose outputs are promised to be the same
-  // bits however a sequence was cut into steps
+  // B200_SCAN_STEP: A/B knob, 0 = single tokens stay in the scan, 1 = never there where the pass takes their sizes.  fp32 models stay there,
+  // whose outputs are promised to be the same bits however a sequence was cut into steps
   const char* se = getenv("B200_SCAN_STEP");
-  if (a.t == DT_BF16 && a.T == a.nseq && a.dim <= 256 && a.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(a.states) % 16 == 0 && !(se && atoi(se) == 0)) {
+  if (a.t == DT_BF16 && a.T == a.nseq && a.dim <= 256 && a.vdim % 4 == 0 && reinterpret_cast<uintptr_t>(a.states) % 16 == 0 &&
+      (se ? atoi(se) != 0 : rules::single_step_pays(static_cast<long long>(a.heads) * a.nseq, a.dim, a.vdim, true, sm_count()))) {
     dim3 grid((a.vdim + kStepCols - 1) / kStepCols, a.heads, a.nseq);
     if (a.dim <= 64) launch_pdl(delta_step_kernel<bf16, 4>, grid, kStepWarps * 32, 0, st, a);
     else if (a.dim <= 128) launch_pdl(delta_step_kernel<bf16, 8>, grid, kStepWarps * 32, 0, st, a);

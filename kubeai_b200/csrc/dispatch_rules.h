@@ -81,5 +81,16 @@ inline bool row_blocks_pay(int rows, long long batch, long long N, long long K, 
   return (rows + 15) / 16 * batch * N * K * 2 <= (fp32_rows ? 60000000 : K >= 128 ? 8500000 : 3000000);
 }
 
+// Single tokens of the recurrences (gla.cu, delta.cu): a pass over the states, CTAs of 64 value columns and up to 16, 128 or 256 rows a lane
+// group, or the scan that walks tokens, a column a thread.  The pass idles where a state fills little of that.  Ratio of its time to the
+// scan's, 16 heads, 32 or 128 sequences: GLA, mLSTM, HGRN2, Mamba-2 0.42 .. 1.0 up to 128 rows and from 32 columns on, 256 rows of 4 to 16
+// columns 0.82 .. 1.11; delta rule 64 rows 0.74 .. 0.99, 128 and 256 rows of 32 to 256 columns 0.40 .. 1.0, of 4 to 16 columns 0.92 .. 1.22; 4 to 32
+// rows of 4 to 64 columns 0.74 .. 0.95, of 96 to 256 columns 0.99 .. 1.40.  4 sequences: 0.5 .. 1.0 everywhere.
+inline bool single_step_pays(long long heads_times_sequences, int dim, int vdim, bool delta, int sms) {
+  if (heads_times_sequences * ((vdim + 63) / 64) <= sms) return true;
+  if (!delta) return dim <= 128 || vdim >= 32;
+  return dim > 64 ? vdim >= 32 : dim > 32 || vdim <= 64;
+}
+
 }  // namespace rules
 }  // namespace b200

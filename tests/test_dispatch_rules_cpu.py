@@ -6,7 +6,7 @@ import pytest
 
 from kubeai_b200._lib import lib
 
-PICKED_ALONE, KEY_LANES, STREAM, CLUSTER, SEGMENTS, ROW_REGISTERS, ROW_BLOCKS = range(7)
+PICKED_ALONE, KEY_LANES, STREAM, CLUSTER, SEGMENTS, ROW_REGISTERS, ROW_BLOCKS, SINGLE_STEP = range(8)
 
 
 def rule(which, *v):
@@ -83,3 +83,11 @@ def test_wide_rows_stay_in_registers_in_steps_and_not_in_prompts(pieces, rows, h
 def test_products_per_head_in_blocks_of_rows_while_their_reads_of_the_weights_are_few(rows, heads, N, K, fp32, blocks):
     """Whatever the heads, 100 rows of 32 heads, 128 to 512 columns, took 18.8 us in blocks against 14.9 in tiles."""
     assert rule(ROW_BLOCKS, rows, heads, N, K, fp32) == blocks
+
+
+@pytest.mark.parametrize("units,dim,vdim,delta,step", [(2048, 128, 128, 0, 1), (2048, 128, 4, 0, 1), (2048, 256, 4, 0, 0), (2048, 256, 32, 0, 1), (2048, 64, 4, 0, 1), (64, 256, 4, 0, 1),
+                                                        (2048, 16, 256, 1, 0), (2048, 16, 64, 1, 1), (512, 32, 96, 1, 0), (2048, 64, 256, 1, 1), (512, 128, 16, 1, 0), (512, 128, 32, 1, 1),
+                                                        (2048, 256, 8, 1, 0), (2048, 256, 64, 1, 1), (64, 256, 4, 1, 1), (37, 16, 256, 1, 1), (38, 16, 256, 1, 0)])
+def test_single_tokens_pass_over_states_that_fill_the_pass(units, dim, vdim, delta, step):
+    """Whatever the state, 16 heads of 16 x 256, 128 sequences of the delta rule, took 46.6 us in the pass against 34.2 in the scan."""
+    assert rule(SINGLE_STEP, units, dim, vdim, delta, 148) == step

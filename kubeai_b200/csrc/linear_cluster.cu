@@ -254,7 +254,8 @@ bool pick_shape(int T, int N, int K, Shape* s) {
 bool linear_clusters(const LinearArgs& a) {
   static const bool on = [] { const char* e = getenv("B200_LIN_CLUSTER"); return !e || atoi(e) != 0; }();     // A/B knob
   Shape s;
-  return on && a.T > 32 && a.T <= 256 && a.N >= 1024 && a.tx == DT_BF16 && a.tw == DT_BF16 && a.batch == 1 && !a.x_rows && !a.tile_group && a.K % 8 == 0 &&
+  // its waits have a limit, so it runs only where a wait that ran out can be reported
+  return on && a.error && a.T > 32 && a.T <= 256 && a.N >= 1024 && a.tx == DT_BF16 && a.tw == DT_BF16 && a.batch == 1 && !a.x_rows && !a.tile_group && a.K % 8 == 0 &&
          a.ldx % 8 == 0 && a.ldw % 8 == 0 && (reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.W)) % 16 == 0 && pick_shape(a.T, a.N, a.K, &s);
 }
 

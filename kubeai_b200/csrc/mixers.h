@@ -48,7 +48,7 @@ struct LinearArgs {
   const float* row_scale;
   const float* bias;
   float a_pos = 0.f, a_neg = 0.f;
-  int* error = nullptr;   // optional, host-visible: a kernel whose wait ran out leaves a mark here (gemm_grouped.cu)
+  int* error = nullptr;   // host-visible: a kernel whose wait ran out leaves a mark here (gemm_grouped.cu, linear_cluster.cu, which needs it)
 };
 inline LinearArgs linear_args(const void* X, DType tx, const void* W, DType tw, void* Y, DType ty, int T, int N, int K, int* error = nullptr) {
   LinearArgs a = {X, W, Y, tx, tw, ty, T, N, K, K, K, N, 1, 0, 0, 0, nullptr, nullptr, LIN_NONE, nullptr, nullptr};

@@ -768,7 +768,7 @@ class Nagilix : public Model {
     // [dt | B | C] and the step sizes' pre-activations leave their products in fp32
     const int nx = m.dt_rank + 2 * m.state;
     KRN("ssm_x_proj", linear(linear_args(xc, dt, w.w_x, dt, xdbc, DT_F32, T, nx, m.inner, env.kernel_error), st));
-    LinearArgs dl = linear_args(xdbc, DT_F32, w.w_dt, dt, dtp, DT_F32, T, m.inner, m.dt_rank);
+    LinearArgs dl = linear_args(xdbc, DT_F32, w.w_dt, dt, dtp, DT_F32, T, m.inner, m.dt_rank, env.kernel_error);
     dl.ldx = nx; dl.bias = w.dt_b;
     KRN("ssm_dt_proj", linear(dl, st));
     SelectiveScanArgs sa;

@@ -683,7 +683,7 @@ class Nomanex : public Model {
         } else {
           KRN("latent_prep", latent_prep(p, st));
           // latent query: per head [T, dim] x [kv_rank, dim]^T into the head's first kv_rank columns of qlat
-          LinearArgs lq = linear_args(col(inb, s.off_q), dt, w.uk_t, dt, qlat, DT_F32, T, C, s.dim);
+          LinearArgs lq = linear_args(col(inb, s.off_q), dt, w.uk_t, dt, qlat, DT_F32, T, C, s.dim, env.kernel_error);
           lq.ldx = s.n_in; lq.ldy = s.heads * E; lq.batch = s.heads; lq.xbs = s.dim + R; lq.wbs = static_cast<long long>(C) * s.dim; lq.ybs = E;
           KRN("latent_q_absorb", linear(lq, st));
           LatentAttnArgs a;
@@ -693,7 +693,7 @@ class Nomanex : public Model {
           a.seqs = b.seqs; a.nseq = b.nseq; a.max_ctx = b.max_ctx; a.split_ws = split_ws; a.split_ws_floats = split_ws_floats;
           KRN("latent_attention", latent_attention(a, st));
           // values: per head [T, kv_rank] x [vdim, kv_rank]^T into the head's columns of the output projection's input
-          LinearArgs lv = linear_args(olat, DT_F32, w.uv, dt, ycat, dt, T, s.vdim, C);
+          LinearArgs lv = linear_args(olat, DT_F32, w.uv, dt, ycat, dt, T, s.vdim, C, env.kernel_error);
           lv.ldx = s.heads * C; lv.ldy = s.k_out; lv.batch = s.heads; lv.xbs = C; lv.wbs = static_cast<long long>(s.vdim) * C; lv.ybs = s.vdim;
           KRN("latent_v_expand", linear(lv, st));
         }

@@ -671,7 +671,7 @@ class Soselix : public Model {
       KRN("latent_q_rotate", latent_prep(pq, st));
     }
     // latent query: per head [T, dim] x [kv_rank, dim]^T into the head's first kv_rank columns of qlat
-    LinearArgs lq = linear_args(qb, dt, w.uk_t, dt, qlat, DT_F32, T, C, s.dim);
+    LinearArgs lq = linear_args(qb, dt, w.uk_t, dt, qlat, DT_F32, T, C, s.dim, env.kernel_error);
     lq.ldx = Q; lq.ldy = s.heads * E; lq.batch = s.heads; lq.xbs = s.dim + R; lq.wbs = static_cast<long long>(C) * s.dim; lq.ybs = E;
     KRN("latent_q_absorb", linear(lq, st));
     LatentAttnArgs a = {};
@@ -682,7 +682,7 @@ class Soselix : public Model {
     a.sink = w.sink; a.gate = col(inb, s.off_g); a.ldg = s.n_in;
     KRN("latent_attention", latent_attention(a, st));
     // values: per head [T, kv_rank] x [vdim, kv_rank]^T into the head's columns of the output projection's input
-    LinearArgs lv = linear_args(olat, DT_F32, w.w_uv, dt, yb, dt, T, s.vdim, C);
+    LinearArgs lv = linear_args(olat, DT_F32, w.w_uv, dt, yb, dt, T, s.vdim, C, env.kernel_error);
     lv.ldx = s.heads * C; lv.ldy = s.k_out; lv.batch = s.heads; lv.xbs = C; lv.wbs = static_cast<long long>(s.vdim) * C; lv.ybs = s.vdim;
     KRN("latent_v_expand", linear(lv, st));
     return rc;

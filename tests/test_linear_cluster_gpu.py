@@ -37,6 +37,23 @@ def test_product_matches_64_bits(N, K):
             assert torch.equal(ops.linear_rows(x, w, dtype=torch.float32), y)     # the parts are added in one order
 
 
+@pytest.mark.parametrize("rank", [1024, 1100])
+def test_the_one_head_of_a_latent_layer(tmp_path, rank):
+    """A latent layer of one head has its per-head products here; their waits are reported like the others'."""
+    import numpy as np
+
+    import soselix_util as sx
+    from nomanex_util import feed_portions, open_engine, rel_err, write_model_dir
+    cfg = sx.make_config([sx.latent(heads=1, dim=64, rot_dim=8, vdim=16, kv_rank=rank, q_rank=32, mlp=None)], width=64)
+    W = sx.random_weights(cfg, seed=rank)
+    d = write_model_dir(tmp_path / "m", cfg, W)
+    t = np.random.default_rng(rank).integers(0, cfg["vocab"], 1 + 64 + 130).tolist()
+    with open_engine(d, dtype="bfloat16") as e:
+        r = rel_err(feed_portions(e, t, [1, 64, 130]), sx.oracle_for(cfg, W).forward(t))
+    # six operators' outputs rounded to 2^-9 of their size each, on a width of 64
+    assert np.median(r) < 0.03 and r.max() < 0.2, (np.median(r), r.max())
+
+
 @pytest.mark.parametrize("act", [0, 1, 2])
 @pytest.mark.parametrize("T", [50, 130])
 def test_bias_and_activations(act, T):

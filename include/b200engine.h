@@ -429,6 +429,9 @@ typedef struct {
   const void* norm_w_out;
 } b200_gemm3_args;
 int b200_op_gemm3(const b200_gemm3_args* a, void* stream, int32_t* schedule_out);
+/* Epilogues 2 and 3 of the same arguments as one pass over the weights (csrc/linear_stream.cu), as the engine's steps of few tokens take
+ * them; B200_ERR_INVALID for sizes it does not serve. */
+int b200_op_linear_pairs(const b200_gemm3_args* a, void* stream);
 int b200_op_embed(const void* table, const int32_t* ids, void* out, int32_t T, int32_t H, int32_t vocab, void* stream);
 int b200_op_rmsnorm(const void* x, void* residual, const void* w, void* out, const int32_t* row_index, int32_t rows,
                     int32_t H, float eps, void* stream);

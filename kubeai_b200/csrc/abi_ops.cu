@@ -271,6 +271,25 @@ int b200_op_gemm3(const b200_gemm3_args* a, void* stream, int32_t* schedule_out)
   return 0;
 }
 
+int b200_op_linear_pairs(const b200_gemm3_args* a, void* stream) {
+  if (int rc = require_device()) return rc;
+  LinearPairs q;
+  bool ok = a && a->w && a->x && a->out && a->x_rows >= a->T && (a->epi == GEMM3_EPI_SILU || a->epi == GEMM3_EPI_ROPE_KV);
+  LinearArgs la = {};
+  if (ok) {
+    la = linear_args(a->x, DT_BF16, a->w, DT_BF16, a->out, DT_BF16, a->T, a->N, a->K);
+    la.ldy = a->ldo;
+    q.kind = a->epi == GEMM3_EPI_SILU ? PAIRS_SILU : PAIRS_ROPE_KV;
+    q.positions = a->positions; q.slots = a->slots; q.cos_sin = a->cos_sin; q.kv_layer = a->kv_layer;
+    q.heads = a->q_heads; q.kv_heads = a->kv_heads; q.max_pos = a->max_pos;
+    if (q.kind == PAIRS_SILU) ok = a->ldo >= a->N / 2;
+    else ok = q.heads > 0 && q.kv_heads > 0 && a->N == (q.heads + 2 * q.kv_heads) * 128 && a->ldo >= q.heads * 128 && q.positions && q.slots && q.cos_sin && q.kv_layer && q.max_pos > 0;
+  }
+  if (!ok || !linear_streams(la, &q)) { set_error("b200_op_linear_pairs: not served"); return B200_ERR_INVALID; }
+  const int rc = linear_stream(la, &q, static_cast<cudaStream_t>(stream));
+  return rc ? cuda_fail("b200_op_linear_pairs", rc) : 0;
+}
+
 int b200_schedule_query(int32_t N, int32_t K, int32_t T, int32_t sms, int32_t* out8) {
   if (N <= 0 || K <= 0 || T <= 0 || sms < 2 || !out8) { set_error("b200_schedule_query: bad arguments"); return B200_ERR_INVALID; }
   gemm2_schedule_query(N, K, T, sms, out8);

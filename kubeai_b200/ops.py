@@ -59,9 +59,10 @@ EPI_PLAIN, EPI_RESADD, EPI_SILU, EPI_ROPE_KV, EPI_ARGMAX = 0, 1, 2, 3, 4
 
 def gemm3(x, w, T=None, pro=PRO_NONE, epi=EPI_PLAIN, force=0, ssq_in=None, norm_w=None, eps=1e-5, out=None, ssq_out=None,
           positions=None, slots=None, cos_sin=None, kv_layer=None, q_heads=0, kv_heads=0, argmax_out=None, n_valid=0,
-          normed_out=None, norm_w_out=None):
+          normed_out=None, norm_w_out=None, pairs=False):
     """The decode-shape fused GEMM (b200_op_gemm3).  x: [rows >= T, K] activations (or the residual for PRO_NORM),
-    w: [N, K].  Returns (out, schedule) with schedule = (pairs per tile, stream-K flag, CTAs)."""
+    w: [N, K].  Returns (out, schedule) with schedule = (pairs per tile, stream-K flag, CTAs).  pairs: EPI_SILU or EPI_ROPE_KV
+    as one pass over the weights (b200_op_linear_pairs)."""
     from ._lib import Gemm3Args
     _chk(x), _chk(w)
     T = x.shape[0] if T is None else T
@@ -93,7 +94,7 @@ def gemm3(x, w, T=None, pro=PRO_NONE, epi=EPI_PLAIN, force=0, ssq_in=None, norm_
     if out is not None:
         a.out, a.ldo = out.data_ptr(), out.stride(0)
     sch = (C.c_int32 * 3)()
-    check(lib().b200_op_gemm3(C.byref(a), _stream(), sch))
+    check(lib().b200_op_linear_pairs(C.byref(a), _stream()) if pairs else lib().b200_op_gemm3(C.byref(a), _stream(), sch))
     res = argmax_out if epi == EPI_ARGMAX else (out, ssq_out, normed_out) if (epi == EPI_RESADD and norm_w_out is not None) \
         else (out, ssq_out) if epi == EPI_RESADD else out
     return res, tuple(sch)

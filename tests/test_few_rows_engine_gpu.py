@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("shape", [dict(hidden=1024, q_heads=8, kv_heads=2, intermediate=3584),
                                    dict(hidden=4096, q_heads=32, kv_heads=8, intermediate=14336)])
-@pytest.mark.parametrize("T", [1, 9, 17, 24, 25, 32, 33])
+@pytest.mark.parametrize("T", [1, 9, 17, 24, 25, 32, 33, 40, 48, 49])
 def test_few_token_steps_agree_with_the_fused_form(shape, T, monkeypatch):
     """Prompts of T tokens in one step, then T decode steps of a few sequences: the logits of both forms differ by roundings."""
     from kubeai_b200.engine import Engine, mini_config

@@ -94,3 +94,43 @@ def test_bias_and_activations(act):
         z = torch.where(z > 0, 0.8 * z * z, 1.2 * (torch.expm1(neg) - neg)) + 0.5 * z
     y = ops.linear_rows(x, w, bias=bias, act=act, p=(0.8, 1.2, 0.0), dtype=torch.float32).double()
     assert ((y - z).abs() <= 1e-5 * (1 + z.abs())).all()
+
+
+@pytest.mark.parametrize("heads,kv_heads,K", [(4, 1, 256), (32, 8, 192), (12, 3, 520), (2, 2, 64)])
+@pytest.mark.parametrize("T", [1, 8, 13, 32])
+def test_rotated_heads_and_cache_rows_equal_the_fused_form(heads, kv_heads, K, T):
+    """Small whole numbers have the same sums in every order, so both forms round the same values at the same points: the same bits, for
+    tokens without a slot, positions past the table and before it, several query heads to a key head, cache rows in any order."""
+    from kubeai_b200 import ops
+    N, blocks = (heads + 2 * kv_heads) * 128, 5
+    g = torch.Generator().manual_seed(heads * 100 + T)
+    x = torch.randint(-4, 5, (T, K), generator=g).to(torch.bfloat16).cuda()
+    w = torch.randint(-4, 5, (N, K), generator=g).to(torch.bfloat16).cuda()
+    cs = torch.randn(40, 128, generator=g).to(torch.bfloat16).cuda()
+    pos = torch.randint(0, 40, (T,), generator=g, dtype=torch.int32)
+    slots = torch.randperm(blocks * 16, generator=g)[:T].to(torch.int32)
+    pos[0], pos[-1] = 77, -3
+    if T > 1:
+        slots[T // 2] = -1
+    out = torch.full((T + 1, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    kv = torch.full((blocks, 2, kv_heads, 16, 128), 5.0, dtype=torch.bfloat16, device="cuda")
+    names = dict(positions=pos.cuda(), slots=slots.cuda(), cos_sin=cs, q_heads=heads, kv_heads=kv_heads)
+    ops.gemm3(x, w, epi=ops.EPI_ROPE_KV, out=out, kv_layer=kv, pairs=True, **names)
+    sums = (x.float() @ w.float().T).to(torch.bfloat16).float()
+    c, s = (cs[pos.clamp(0, 39).long().cuda()].float()[:, None, a:a + 64] for a in (0, 64))
+    bf = lambda v: v.to(torch.bfloat16).float()
+    rows = sums.reshape(T, heads + 2 * kv_heads, 128)
+    a, b = rows[..., :64], rows[..., 64:]
+    turned = torch.cat([bf(bf(a * c) - bf(b * s)), bf(bf(b * c) + bf(a * s))], -1)
+    assert torch.equal(out[:T, :heads * 128].float().reshape(T, heads, 128), turned[:, :heads])
+    assert (out[T] == 7).all() and (out[:, heads * 128:] == 7).all()
+    want = torch.full_like(kv, 5.0)
+    for t in range(T):
+        if slots[t] >= 0:
+            want[slots[t] // 16, 0, :, slots[t] % 16] = turned[t, heads:heads + kv_heads].to(torch.bfloat16)
+            want[slots[t] // 16, 1, :, slots[t] % 16] = rows[t, heads + kv_heads:].to(torch.bfloat16)
+    assert torch.equal(kv, want)
+    if N % 256 == 0 and K % 64 == 0:      # sizes of the fused form
+        fused, kv2 = torch.zeros(T, N, dtype=torch.bfloat16, device="cuda"), torch.full_like(kv, 5.0)
+        ops.gemm3(x, w, epi=ops.EPI_ROPE_KV, out=fused, kv_layer=kv2, **names)
+        assert torch.equal(fused[:, :heads * 128], out[:T, :heads * 128]) and torch.equal(kv2, kv)

@@ -484,7 +484,8 @@ __global__ void __launch_bounds__(kWarpsDecode * 32) window_attn_kernel(WindowAt
 // hold a key (eight dimensions or value columns each, whole 16-byte pieces): half-warp r takes the visible keys r, r + 16,
 // r + 32, ... (8 warps), kRowKeys of them in flight, their keys and their values, and keeps an online softmax of its own in
 // fp32 with the accurate functions; the sixteen partial results are merged in a fixed order.  Which keys a half-warp takes,
-// and in which groups, depends on the token's position alone.
+// and in which groups, depends on the token's position alone, and every product and sum is written with its rounding, so that the
+// forms for 1 to 8 heads give the same bits (left to the compiler, they fused different ones).
 // What bounds a step of short contexts is the chain positions -> block table -> rows -> exponentials -> merge; the general
 // kernel below added a chain of 16 loads a key (a lane a key) and of loads four values at a time behind it.  24 sequences of
 // 22 tokens, 16 heads of 128 in 4 groups: 37 us there, 10 here; 16 of 250: 34
@@ -563,19 +564,19 @@ __global__ void __launch_bounds__(kRowWarps * 32) window_attn_rows_kernel(Window
       float mn = m[h];
 #pragma unroll
       for (int u = 0; u < kRowKeys; ++u) {
-        if (a.softcap > 0.f) sc[h][u] = a.softcap * tanhf(sc[h][u] / a.softcap);
+        if (a.softcap > 0.f) sc[h][u] = __fmul_rn(a.softcap, tanhf(sc[h][u] / a.softcap));
         if (i0 + u * 2 * kRowWarps >= n) sc[h][u] = -FLT_MAX;
         mn = fmaxf(mn, sc[h][u]);
       }
       const float corr = expf(m[h] - mn);
       m[h] = mn;
-      l[h] *= corr;
+      l[h] = __fmul_rn(l[h], corr);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[h][e] *= corr;
 #pragma unroll
       for (int u = 0; u < kRowKeys; ++u) {
         sc[h][u] = i0 + u * 2 * kRowWarps < n ? expf(sc[h][u] - mn) : 0.f;
-        l[h] += sc[h][u];
+        l[h] = __fadd_rn(l[h], sc[h][u]);
       }
     }
 #pragma unroll
@@ -594,11 +595,11 @@ __global__ void __launch_bounds__(kRowWarps * 32) window_attn_rows_kernel(Window
     const float mo = __shfl_xor_sync(0xffffffffu, m[h], 16), lo_ = __shfl_xor_sync(0xffffffffu, l[h], 16);
     const float mn = fmaxf(m[h], mo), f0 = m[h] == -FLT_MAX ? 0.f : expf(m[h] - mn), f1 = mo == -FLT_MAX ? 0.f : expf(mo - mn);
     float* mine = sm + (wrp * GS + h) * (Dv + 2);
-    if (lane == 0) { mine[0] = mn; mine[1] = l[h] * f0 + lo_ * f1; }
+    if (lane == 0) { mine[0] = mn; mine[1] = fmaf(l[h], f0, __fmul_rn(lo_, f1)); }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const float o = __shfl_xor_sync(0xffffffffu, acc[h][e], 16);
-      if (lane < 16 && vin) mine[2 + c0 + e] = acc[h][e] * f0 + o * f1;
+      if (lane < 16 && vin) mine[2 + c0 + e] = fmaf(acc[h][e], f0, __fmul_rn(o, f1));
     }
   }
   __syncthreads();
@@ -943,7 +944,8 @@ int qk_rope_norm_cache(const QkPrepArgs& a, cudaStream_t st) {
   if (a.T <= 0) return 0;
   if (a.heads < 1 || a.kv_heads < 1 || a.dim < 1 || a.vdim < 1 || a.rot_dims < 0 || a.rot_dims > a.dim || a.rot_dims % 2 || (a.rot_dims && !a.rope)) return -1;
   auto piece = [](const void* p, int ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 8 == 0; };
-  if (a.t == DT_BF16 && a.vdim % 8 == 0 && (a.dim == 32 || a.dim == 64 || a.dim == 128 || a.dim == 256) && piece(a.q, a.ld) && piece(a.k, a.ld) && piece(a.v, a.ld) &&
+  const char* re = getenv("B200_QK_ROWS");      // A/B knob: 0 = every row on the general kernel
+  if (!(re && atoi(re) == 0) && a.t == DT_BF16 && a.vdim % 8 == 0 && (a.dim == 32 || a.dim == 64 || a.dim == 128 || a.dim == 256) && piece(a.q, a.ld) && piece(a.k, a.ld) && piece(a.v, a.ld) &&
       piece(a.cache, 0) && piece(a.qn, 0) && piece(a.v_blend, a.v_blend ? a.ld_blend : 0) && piece(a.v_raw_out, a.v_raw_out ? a.ld_raw : 0)) {
     const int items = (a.heads + a.kv_heads) * (a.dim / 8) + a.kv_heads * a.vdim / 8;
     const int threads = std::min(a.T >= 256 ? 256 : 512, (items + 31) / 32 * 32);

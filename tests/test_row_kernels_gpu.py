@@ -35,13 +35,15 @@ def test_rows_of_every_number_of_pieces(tmp_path, family, width):
     t = np.random.default_rng(width).integers(0, cfg["vocab"], 21).tolist()
     want = oracle(cfg, W).forward(t)
     # fp32: sums of at most 4100 products, some sixty roundings of 2^-24 each where their signs are random, in about eight sublayers'
-    # worth of operators: 3e-5; small widths divide by sums of few terms
+    # worth of operators: 3e-5; small widths divide by sums of few terms.  Nothing here routes, so that holds for every row
     with nx.open_engine(d) as e:
-        assert np.median(nx.rel_err(nx.feed_whole(e, t), want)) < 1e-4
-        assert np.median(nx.rel_err(nx.feed_portions(e, t, [9] + [1] * 12), want)) < 1e-4
-    # bf16: eight operators' outputs rounded to 2^-9 of their size each
+        assert nx.rel_err(nx.feed_whole(e, t), want).max() < 1e-4
+        assert nx.rel_err(nx.feed_portions(e, t, [9] + [1] * 12), want).max() < 1e-4
+    # bf16: eight operators' outputs rounded to 2^-9 of their size each.  A matrix memory's answer is a quotient, and where its divisor comes
+    # near zero that moves the row and those behind it by more (width 516: four rows by 0.27 to 0.6)
     with nx.open_engine(d, dtype="bfloat16") as e:
-        assert np.median(nx.rel_err(nx.feed_portions(e, t, [9] + [1] * 12), want)) < 0.06
+        r = np.sort(nx.rel_err(nx.feed_portions(e, t, [9] + [1] * 12), want))
+        assert np.median(r) < 0.06 and (r[15] < 0.1 if family == "mulenex" else r[-1] < 0.25), r[-6:]
 
 
 @pytest.mark.parametrize("q_rank,kv_rank", [(1, 1), (127, 129), (1024, 512), (1025, 1023), (40, 1100)])
@@ -51,7 +53,7 @@ def test_latent_rows_that_stay_in_registers_and_longer_ones(tmp_path, q_rank, kv
     d = nx.write_model_dir(tmp_path / "m", cfg, W)
     t = np.random.default_rng(5).integers(0, cfg["vocab"], 17).tolist()
     with nx.open_engine(d) as e:
-        assert np.median(nx.rel_err(nx.feed_portions(e, t, [8] + [1] * 9), sx.oracle_for(cfg, W).forward(t))) < 1e-4
+        assert nx.rel_err(nx.feed_portions(e, t, [8] + [1] * 9), sx.oracle_for(cfg, W).forward(t)).max() < 1e-4
 
 
 @pytest.mark.parametrize("taps", [2, 3, 4])
@@ -69,5 +71,6 @@ def test_short_convolution_over_sequences_that_end_inside_its_rounds(tmp_path, t
             ids = [e.feed_open() for _ in seqs]
             a = e.feed_step([(r, s[:n].tolist(), [n - 1]) for r, s, n in zip(ids, seqs, first)])
             b = e.feed_step([(r, s[n:].tolist(), [len(s) - n - 1]) for r, s, n in zip(ids, seqs, first)])
-        assert np.median(nx.rel_err(np.asarray(a), np.stack([w[n - 1] for w, n in zip(want, first)]))) < tol
-        assert np.median(nx.rel_err(np.asarray(b), np.stack([w[-1] for w in want]))) < tol
+        # every sequence: a fault at one kind of boundary touches few of the sixteen
+        assert nx.rel_err(np.asarray(a), np.stack([w[n - 1] for w, n in zip(want, first)])).max() < tol
+        assert nx.rel_err(np.asarray(b), np.stack([w[-1] for w in want])).max() < tol

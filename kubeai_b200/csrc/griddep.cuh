@@ -22,8 +22,9 @@ __device__ __forceinline__ void griddep_enter() {
 
 // The designs' kernels release their consumer at entry and wait before anything else: the launches and prologues of a whole
 // chain of small kernels then overlap, and a kernel that waits knows that everything before it in the stream is complete,
-// because its predecessor waited too.  Ahead of the wait stands nothing but prefetches and loads of weights, which no step writes, and in a kernel
-// launched this way nothing that an earlier kernel of the step wrote is read through the read-only path (__ldg; kernels launched plainly,
+// because its predecessor waited too.  Ahead of the wait stand loads of weights, which no step writes, and of the step's uploaded inputs (positions,
+// sequences, tables: copied before its first kernel), and prefetches into L2 of what may still be written (states: a prefetched line stays coherent);
+// never a load of anything that a kernel of the step writes.  In a kernel launched this way nothing that an earlier kernel of the step wrote is read through the read-only path (__ldg; kernels launched plainly,
 // such as the scans of prompt portions, may).  Decode steps, device time
 // with plain launches and so: Soselix, 8 sequences, 35 kernels 338 us -> 300; Mulenex, 24 sequences 529 -> 480.
 

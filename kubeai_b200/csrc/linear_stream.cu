@@ -6,8 +6,9 @@
 //     CTAs); the warps of a CTA take the 64-wide pieces of K in turn and their sums meet once in shared memory, in a fixed order;
 //   * every warp runs a ring of its own in shared memory, filled by 16-byte asynchronous copies (whole 128-byte lines of W), so
 //     loads never wait for products and no barrier stands in the loop;
-//   * the ring is filled with weights before the wait for the kernel in front: W is nobody's output.  A ring is small enough
-//     that two or three kernels of a step share an SM, which keeps HBM busy across their boundaries.
+//   * the ring is filled with weights before the wait for the kernel in front: W is nobody's output.  A CTA takes 163 to 210 KB, so
+//     this overlaps kernels that use little shared memory (a norm, an activation, attention of single tokens), and between two such products
+//     in a row nothing does: a smaller ring lost more than that would give (Layout).
 // Products are mma.sync m16n8k16 with 16 rows of W as the first operand and 8 tokens as the second: at up to 16 tokens the
 // kernel needs a twentieth of the tensor cores' rate, and rows that a tile has too many cost nothing.
 // The order of one output element's sums depends on N and K alone, not on what else is in the batch.

@@ -34,8 +34,11 @@ enum LinearAct { LIN_NONE = 0, LIN_RELU2 = 1, LIN_XIELU = 2 };
 //   row_scale (optional, fp32): the accumulator of row t is multiplied by row_scale[t] before act, which is the product
 //     of the scaled input row, (s x) W^T = s (x W^T), without a scaled copy of x.
 //   bias (optional, fp32 [N]): added to the (scaled) accumulator before act.
-// The accumulation order of one output element never depends on T or on the other rows (k ascending inside a tile
-// kernel, a fixed lane pattern in the few-row kernel), so a row's result does not depend on what shares the batch.
+// fp32 weights: the accumulation order of one output element never depends on T or on the other rows (k ascending inside a tile kernel, a fixed lane
+// pattern in the few-row kernel), so a row's result does not depend on what shares the batch.  bf16 weights: that holds within a kernel and shape, and T
+// chooses the kernel: linear_stream.cu (up to 48, 32 or 8 rows, by N) and the fragment kernel (up to 16; per head up to 128, rules::row_blocks_pay) sum in
+// an order of N and K alone, the 64-row tiles and whole tiles k ascending or in parts by shape, linear_cluster.cu in an order that T (up to 128 or
+// beyond), N and K give.  An fp32 row of X is split into two bf16 terms up to 16 rows and rounded to one from 17 on.
 struct LinearArgs {
   const void* X; const void* W; void* Y;
   DType tx, tw, ty;
@@ -73,7 +76,7 @@ struct LinearPairs {
 };
 bool linear_streams(const LinearArgs& a, const LinearPairs* q = nullptr);
 int linear_stream(const LinearArgs& a, const LinearPairs* q, cudaStream_t st);
-// Steps of some tens to a few hundred tokens against a matrix of up to about 3000 rows, K cut over clusters (linear_cluster.cu);
+// Steps of 49 to 256 tokens (fewer go to linear_stream.cu) against a matrix of about 1000 to 3000 rows, K cut over clusters (linear_cluster.cu);
 // `linear` takes it wherever it serves, with the same promise about W.
 bool linear_clusters(const LinearArgs& a);
 int linear_cluster(const LinearArgs& a, cudaStream_t st);

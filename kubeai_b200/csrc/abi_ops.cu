@@ -305,6 +305,7 @@ int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_ROW_REGISTERS && n == 3) return rules::row_in_registers(v[0], v[1], v[2]);
   if (v && rule == B200_RULE_ROW_BLOCKS && n == 5) return rules::row_blocks_pay(v[0], v[1], v[2], v[3], v[4] != 0);
   if (v && rule == B200_RULE_SINGLE_STEP && n == 5) return rules::single_step_pays(v[0], v[1], v[2], v[3] != 0, v[4]);
+  if (v && rule == B200_RULE_LATENT_ROWS && n == 2) return rules::latent_rows_held(v[0], v[1]);
   set_error("b200_rule_query: rule %d with %d sizes", rule, n);
   return B200_ERR_INVALID;
 }

@@ -92,5 +92,11 @@ inline bool single_step_pays(long long heads_times_sequences, int dim, int vdim,
   return dim > 64 ? vdim >= 32 : dim > 32 || vdim <= 64;
 }
 
+// Latent rows (latent_attention.cu): in registers between their sum and their norm, or read again.  Registers for 1024 numbers a CTA cost room on
+// an SM, which short rows and many of them feel; longer rows do not fit.  rank: the longest row asked for, 0 where only queries are rotated.
+// us of two layers, again / held: ranks 1024 and 512, 8 tokens 21 / 17, 4096 43 / 38; 512 and 256, 8 18 / 16, 2400 27.8 / 26.4, 4096 34.3 / 36.3; 128 and
+// 64, 600 tokens 18 / 19, 4096 33 / 38.  One kernel that could do both: 1500 and 1100, 4096 tokens 63 / 73, 2048 60 / 73.
+inline bool latent_rows_held(int rank, int tokens) { return rank <= 1024 && (rank > 512 || tokens <= 4 * (rank > 128 ? rank : 128)); }
+
 }  // namespace rules
 }  // namespace b200

@@ -21,6 +21,7 @@
 #include <atomic>
 #include <vector>
 
+#include "dispatch_rules.h"
 #include "griddep.cuh"
 #include "launch.h"
 #include "mixers.h"
@@ -77,9 +78,9 @@ __device__ __forceinline__ float out_gate(const LatentAttnArgs& a, long long t, 
 
 // per token, each its own CTA: the query latent's norm, the cache row, the queries' rotated parts (one after the other in one CTA,
 // 8 tokens took 13 us)
-// A row of up to 1024 numbers stays in registers between its sum and its norm, whose weights arrive while the kernel in front still
-// runs; what is rotated is loaded before the sum too.  8 tokens of 1024 + 512 + 64 numbers: 7.2 us, now 3.6.
-template <typename T>
+// HELD: a row of up to 1024 numbers stays in registers between its sum and its norm, whose weights arrive while the kernel in front still
+// runs; what is rotated is loaded before the sum too.  8 tokens of 1024 + 512 + 64 numbers: 7.2 us, 3.6 held (rules::latent_rows_held).
+template <typename T, bool HELD>
 __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepArgs a) {
   griddep_launch();
   __shared__ float red[8];
@@ -91,34 +92,34 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepArgs a) {
   constexpr int kHeld = 8;
   const int n = part == 0 ? a.q_rank : C;
   const float* nw = part == 0 ? a.cq_w : a.norm_w;
-  const bool held = n <= kHeld * 128;
   float gain[kHeld];
-  if (part < 2 && held) {
+  if (HELD && part < 2) {
 #pragma unroll
     for (int k = 0; k < kHeld; ++k) gain[k] = threadIdx.x + k * 128 < n ? nw[threadIdx.x + k * 128] : 0.f;
   }
   griddep_wait();
   auto norm_row = [&](const T* u, T* o, auto behind_loads) {
     float v[kHeld], ss = 0.f;
-    if (held) {
+    if constexpr (HELD) {
 #pragma unroll
       for (int k = 0; k < kHeld; ++k) v[k] = threadIdx.x + k * 128 < n ? ldf(u + threadIdx.x + k * 128) : 0.f;
     } else {
       for (int i = threadIdx.x; i < n; i += blockDim.x) { const float x = ldf(u + i); ss = fmaf(x, x, ss); }
     }
-    behind_loads();
-    if (held) {
+    if constexpr (HELD) {
+      behind_loads();
 #pragma unroll
       for (int k = 0; k < kHeld; ++k) ss = fmaf(v[k], v[k], ss);
     }
     ss = block_sum(ss, red);
     const float inv = 1.0f / sqrtf(ss / static_cast<float>(n) + a.eps);
-    if (held) {
+    if constexpr (HELD) {
 #pragma unroll
       for (int k = 0; k < kHeld; ++k)
         if (threadIdx.x + k * 128 < n) stf(o + threadIdx.x + k * 128, v[k] * inv * gain[k]);
     } else {
       for (int i = threadIdx.x; i < n; i += blockDim.x) stf(o + i, ldf(u + i) * inv * nw[i]);
+      behind_loads();
     }
   };
   if (part == 0 && a.cq) norm_row(static_cast<const T*>(a.cq) + static_cast<long long>(t) * a.ldcq, static_cast<T*>(a.cq_out) + static_cast<long long>(t) * a.ldcq_out, [] {});
@@ -135,7 +136,8 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepArgs a) {
     // rotated part of every query head -> tail of the latent query
     const T* q = static_cast<const T*>(a.q) + static_cast<long long>(t) * a.ldq;
     float* ql = a.qlat + static_cast<long long>(t) * a.heads * (C + R);
-#pragma unroll 8
+    constexpr int kAhead = HELD ? 8 : 4;
+#pragma unroll kAhead
     for (int e = threadIdx.x; e < a.heads * R; e += blockDim.x) {
       const int h = e / R, i = e - h * R;
       ql[h * (C + R) + C + i] = rotated(q + h * (D + R) + D, i, half, a.half_pairs, cs);
@@ -749,8 +751,9 @@ int latent_prep(const LatentPrepArgs& a, cudaStream_t st) {
   if (a.cq && (!a.cq_w || !a.cq_out || a.q_rank < 1)) return -1;
   const int parts = (a.cq != nullptr) + (a.dkv != nullptr) + (a.q != nullptr);
   if (!parts) return 0;
-  if (a.t == DT_BF16) launch_pdl(latent_prep_kernel<bf16>, dim3(a.T, parts), 128, 0, st, a);
-  else launch_pdl(latent_prep_kernel<float>, dim3(a.T, parts), 128, 0, st, a);
+  const bool held = rules::latent_rows_held(std::max(a.cq ? a.q_rank : 0, a.dkv ? a.kv_rank : 0), a.T);
+  auto kernel = a.t == DT_BF16 ? (held ? latent_prep_kernel<bf16, true> : latent_prep_kernel<bf16, false>) : (held ? latent_prep_kernel<float, true> : latent_prep_kernel<float, false>);
+  launch_pdl(kernel, dim3(a.T, parts), 128, 0, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -56,6 +56,19 @@ def test_latent_rows_that_stay_in_registers_and_longer_ones(tmp_path, q_rank, kv
         assert nx.rel_err(nx.feed_portions(e, t, [8] + [1] * 9), sx.oracle_for(cfg, W).forward(t)).max() < 1e-4
 
 
+@pytest.mark.parametrize("ranks", [(24, 20), (130, 40)])
+def test_latent_rows_of_more_tokens_than_stay_in_registers(tmp_path, ranks):
+    """Both sides of the line for short rows (512 tokens): in a step of 600 rows are read again, in two of 300 they are held; the same sums."""
+    cfg = sx.make_config([sx.latent(heads=2, q_rank=ranks[0], kv_rank=ranks[1], mlp=None)], width=32)
+    W = sx.random_weights(cfg, seed=7)
+    d = nx.write_model_dir(tmp_path / "m", cfg, W)
+    t = np.random.default_rng(6).integers(0, cfg["vocab"], 600).tolist()
+    with nx.open_engine(d, max_tokens=640) as e:
+        whole, parts = nx.feed_whole(e, t), nx.feed_portions(e, t, [300])
+    assert nx.rel_err(whole, sx.oracle_for(cfg, W).forward(t)).max() < 1e-4
+    assert nx.rel_err(parts, whole.astype(np.float64)).max() < 1e-5
+
+
 @pytest.mark.parametrize("taps", [2, 3, 4])
 def test_short_convolution_over_sequences_that_end_inside_its_rounds(tmp_path, taps):
     """Rows come in rounds of four and walks of up to sixteen; sequences begin and end anywhere in them and go on from what they carry."""

@@ -35,7 +35,7 @@ sys.path.insert(0, str(ROOT))
 METRIC = "agg output tok/s, Llama-3-8B multi-turn (p50/p99 TTFT in extra keys)"
 WORKLOAD = ("Llama-3-8B bf16 (random-init), continuous batching, 128 in-flight multi-turn sessions per GPU, "
             "<=2k ctx, greedy, 40 tokens/turn, synthetic threads of the multi-turn-chat-go shape")
-LAYER_W_BYTES = 218_103_808 * 2          # per decoder layer (SURVEY.md §8)
+LAYER_W_BYTES = 218_103_808 * 2          # per decoder layer
 HEAD_W_BYTES = 128256 * 4096 * 2
 KV_BYTES_PER_TOKEN = 131072
 

@@ -9,7 +9,7 @@ minutes to start).  Two things are compared on >= 32 prompts:
     |x| in 8..16, 0.125 at 16..32) — two correct bf16 pipelines differ by the rounding of the final 4096-term dot product
     (1 ulp) plus what the layers' bf16 intermediates feed into it.  First run on a B200 (profiles/r02_vllm_parity.md): max
     |d logprob| 0.20 on the 2-layer model (3.2 ulps), 0.50 on the 32-layer Llama-3-8B shape (4 ulps), means 0.03 / 0.08,
-    i.e. under one ulp.  The measured maxima of every run go to gpurun_out/vllm_parity.json.
+    i.e. under one ulp.  The measured maxima of every run go to vllm_parity.json in the temporary folder.
   * greedy TOKENS: streams may part only where vLLM's own top-2 candidates are within MARGIN_ULPS bf16 ulps of the top
     logit of each other.  MARGIN_ULPS = 4 is the measured bound on how far ONE logit of the 32-layer model moves between the
     two pipelines (max |d logprob| 3.7-4 ulps over three runs): a margin below it can flip.  Observed first-difference
@@ -18,6 +18,7 @@ minutes to start).  Two things are compared on >= 32 prompts:
 """
 import json
 import os
+import tempfile
 from pathlib import Path
 
 import numpy as np
@@ -38,7 +39,7 @@ def _vllm_ok():
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not _vllm_ok(), reason="vllm is not importable (or B200_SKIP_VLLM=1)")]
 LOGPROB_ULPS = 6.0
 MARGIN_ULPS = 4.0
-REPORT = Path(__file__).resolve().parent.parent / "gpurun_out" / "vllm_parity.json"
+REPORT = Path(tempfile.gettempdir()) / "vllm_parity.json"
 
 
 def ulp_bf16(x):

@@ -405,7 +405,7 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
  * out (the fused qkv buffer, ldo), k/v -> kv_layer pages; 4: argmax_out [T] = argmax_n acc[t, n < n_valid]).
  * force: 0 automatic schedule, 1..4 pairs per tile (cluster split-K through distributed shared memory), < 0 stream-K.
  * schedule_out (optional, 3 ints): pairs per tile, stream-K flag, CTAs launched.  epi 2 without a prologue and with force 0
- * takes b200_op_linear_rows's kernel where that serves the sizes (no pairs per tile then). */
+ * takes b200_op_linear_rows's kernel where that serves the sizes and is ahead (B200_RULE_STREAM; no pairs per tile then). */
 typedef struct {
   int32_t N, T, K, x_rows;
   int32_t pro, epi, force;

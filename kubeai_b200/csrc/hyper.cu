@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(256) sandwich_step_kernel(SandwichArgs a) {
 // output, the residual and the norms' weights are all on their way before the first sum, the weights already while the kernel in
 // front runs, where the form above goes to memory three times, once behind each sum.  What a thread adds up, and in which order, is
 // the same.  A row is bound by that chain in decode steps (8 rows of 2048: 5 to 7.5 us with the form
-// above, 2.5 to 4 here), by HBM in prompts (4096 rows: 21 us, 17.5 here; 16 at the copy rate).
+// above, 2.5 to 4 here), by HBM in prompts (4096 rows: 21 us, 17.5 here; 16 at the copy rate; wider rows of prompts stay above, rules::row_in_registers).
 template <typename TY, typename TH, int R>
 __global__ void __launch_bounds__(256) sandwich_rows_kernel(SandwichArgs a) {
   griddep_launch();

@@ -230,7 +230,7 @@ int launch(const LinearArgs& a, const Shape& s, cudaStream_t st) {
 //   2048 x 4096   64 tokens 13.0 / 10.3  128 tokens 18.0 / 11.8   256 tokens 24.4 / 16.1
 //   2048 x 8192   64 tokens 16.3 / 15.2  128 tokens 21.4 / 17.2   256 tokens 32.1 / 25.3
 //   3072 x 1024   64 tokens  8.4 / 6.6   128 tokens  9.1 / 8.0    256 tokens 10.5 / 12.4
-// From 4096 rows on the whole tiles are as fast or faster: they read X once for 256 rows.
+// From 4096 rows on the whole tiles are as fast or faster: they read X once for 256 rows.  So they are with a long K (rules::cluster_pays).
 bool pick_shape(int T, int N, int K, Shape* s) {
   s->C = 4;
   if (N <= 2112) {

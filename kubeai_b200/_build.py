@@ -16,6 +16,7 @@ ROOT = Path(__file__).resolve().parent
 CSRC = ROOT / "csrc"
 LIB = ROOT / "lib" / "libb200engine.so"
 OBJ = ROOT / "lib" / "obj"
+FEED = ROOT / "_feed.so"      # the Python side's one native helper (csrc/pyfeed.cc)
 
 SOURCES = [
     "gemm_tcgen05.cu",
@@ -72,6 +73,19 @@ def _nvcc() -> str:
     return "nvcc"
 
 
+def _feed_flags():
+    """Include flags of the Python helper; none where Python's or numpy's headers are not installed (engine.py works without it)."""
+    import sysconfig
+    try:
+        import numpy
+    except ImportError:
+        return []
+    dirs = [sysconfig.get_paths()["include"], numpy.get_include(), str(ROOT.parent / "include")]
+    if not os.path.exists(os.path.join(dirs[0], "Python.h")) or not os.path.isdir(dirs[1]):
+        return []
+    return [f for d in dirs for f in ("-I", d)]
+
+
 def _digest(paths) -> str:
     h = hashlib.sha256()
     for p in sorted(paths):
@@ -83,11 +97,12 @@ def _digest(paths) -> str:
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     srcs = [CSRC / s for s in SOURCES if (CSRC / s).exists()]
-    deps = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [ROOT.parent / "include" / "b200engine.h"] + \
+    feed_flags = _feed_flags()
+    deps = [CSRC / "pyfeed.cc"] + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [ROOT.parent / "include" / "b200engine.h"] + \
         list((ROOT.parent / "cmd").glob("*.cc"))
     stamp = OBJ / "digest.txt"
     digest = _digest(srcs + deps)
-    if not force and LIB.exists() and stamp.exists() and stamp.read_text() == digest:
+    if not force and LIB.exists() and (FEED.exists() or not feed_flags) and stamp.exists() and stamp.read_text() == digest:
         return LIB
     OBJ.mkdir(parents=True, exist_ok=True)
     nvcc = _nvcc()
@@ -120,6 +135,11 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"building {name} failed:\n{r.stdout}\n{r.stderr}")
+    if feed_flags:
+        cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", *feed_flags, str(CSRC / "pyfeed.cc"), "-o", str(FEED)]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"building {FEED.name} failed:\n{r.stdout}\n{r.stderr}")
     stamp.write_text(digest)
     return LIB
 

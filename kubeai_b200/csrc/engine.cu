@@ -182,6 +182,7 @@ struct Seq {
   int n_trimmed = 0;     // leading pages already returned to the pool (they lie before every layer's window); blocks[i] = -1 there
   int state_slot = -1;   // recurrent-state slot (models with per-sequence state), held while the sequence holds pages
   bool fed = false;      // tokens come from the caller step by step (b200_feed_*); nothing is sampled into toks
+  uint64_t feed_call = 0;   // number of the last feed_step call that named it
   // shared with API threads: guarded by m (one lock per request, so a step's 128 wake-ups do not convoy on one mutex)
   std::mutex m;
   std::condition_variable cv;
@@ -240,6 +241,7 @@ struct Engine {
   static constexpr size_t kFeedHalf = 2u << 20;
   uint8_t* feed_stage = nullptr;
   cudaEvent_t feed_ev[2] = {nullptr, nullptr};
+  uint64_t feed_calls = 0;
   int init_feed();
   int check_kernels();
   int read_logits_f32(float* out, size_t count);
@@ -1593,6 +1595,17 @@ int Engine::init_feed() {
   return 0;
 }
 
+// Touches the pages of `count` floats the caller will get until `ready` has happened on the device: memory that is new to the
+// process costs 1 to 1.5 us a page, which so passes while the device works and not behind its last kernel.  (A step of 128 sequences of
+// which 16 want 8192 logits each: 168 us from the wait's end to the result without it; 13 such steps 9210 us before, 7370 with this and pyfeed.cc.)
+void touch_pages(float* out, size_t count, cudaEvent_t ready) {
+  constexpr size_t page = 4096 / sizeof(float);
+  for (size_t i = 0, n = 0; i < count; i += page, ++n) {
+    if (n % 16 == 15 && cudaEventQuery(ready) != cudaErrorNotReady) return;
+    *const_cast<volatile float*>(out + i) = 0.f;
+  }
+}
+
 // the first `count` bf16 logits on the device -> fp32 (same values) at `out`
 int Engine::read_logits_f32(float* out, size_t count) {
   constexpr size_t part = kFeedHalf / 2;
@@ -1603,7 +1616,10 @@ int Engine::read_logits_f32(float* out, size_t count) {
       CK(cudaMemcpyAsync(feed_stage + (i & 1) * kFeedHalf, logits + i * part, len(i) * 2, cudaMemcpyDeviceToHost, stream));
       CK(cudaEventRecord(feed_ev[i & 1], stream));
     }
-    if (i == 0) continue;
+    if (i == 0) {
+      touch_pages(out, count, feed_ev[0]);
+      continue;
+    }
     CK(cudaEventSynchronize(feed_ev[(i - 1) & 1]));
     const uint16_t* in = reinterpret_cast<const uint16_t*>(feed_stage + ((i - 1) & 1) * kFeedHalf);
     uint32_t* o = reinterpret_cast<uint32_t*>(out + (i - 1) * part);
@@ -1619,6 +1635,7 @@ int Engine::read_logits_f32(float* out, size_t count) {
 int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, int64_t cap_floats) {
   InFlight& f = inflight_;
   f.sched.clear();
+  ++feed_calls;
   std::vector<std::vector<int>> want(n);
   int T = 0;
   int64_t S = 0;
@@ -1632,7 +1649,8 @@ int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, 
     }
     if (!s || !s->fed) { set_error("feed: request %llu was not opened with b200_feed_open", static_cast<unsigned long long>(en.req_id)); return B200_ERR_NOT_FOUND; }
     if (en.n_tokens <= 0 || !en.tokens || (en.n_want > 0 && !en.want)) { set_error("feed: an entry needs at least one token"); return B200_ERR_INVALID; }
-    for (auto& sc : f.sched) if (sc.s == s) { set_error("feed: a request appears twice in one step"); return B200_ERR_INVALID; }
+    if (s->feed_call == feed_calls) { set_error("feed: a request appears twice in one step"); return B200_ERR_INVALID; }
+    s->feed_call = feed_calls;
     for (int j = 0; j < en.n_tokens; ++j) if (en.tokens[j] < 0 || en.tokens[j] >= V) { set_error("feed: token id out of range"); return B200_ERR_INVALID; }
     for (int j = 0; j < en.n_want; ++j) {
       if (en.want[j] < 0 || en.want[j] >= en.n_tokens) { set_error("feed: wanted position outside the entry's tokens"); return B200_ERR_INVALID; }
@@ -1678,6 +1696,7 @@ int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, 
     }
     if (!rc) {
       CK(cudaEventRecord(ev1, stream));
+      if (staged) touch_pages(logits_out, static_cast<size_t>(S) * V, ev1);
       CK(cudaStreamSynchronize(stream));
       rc = check_kernels();
       if (!rc && staged && S) memcpy(logits_out, feed_stage, static_cast<size_t>(S) * V * sizeof(float));

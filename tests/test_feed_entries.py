@@ -72,3 +72,18 @@ def test_logits_of_a_design_around_the_staging_limit(tmp_path, rows):
     assert np.isfinite(got).all() and got.std(axis=1).min() > 0
     # other numbers of rows take other product kernels: the same sums in another order
     np.testing.assert_allclose(got, np.concatenate(parts), rtol=0, atol=2.0 ** -20 * 64 * np.abs(got).max())
+
+
+def test_arrays_and_lists_give_the_same_entries():
+    """int32 vectors go through the native packing, everything else through numpy: the C call sees the same."""
+    rng = np.random.default_rng(5)
+    toks = [rng.integers(0, 7, n).astype(np.int32) for n in (1, 3, 17, 2)]
+    wants = [np.array(w, dtype=np.int32) for w in ([], [2], [0, 16], [])]
+    rids = [1, 2 ** 64 - 1, 7, 2 ** 63]
+    plain = [(r, t.tolist(), w.tolist()) for r, t, w in zip(rids, toks, wants)]
+    want = [(r, t, w or None) for r, t, w in plain]
+    assert fed(list(zip(rids, toks, wants))) == fed(plain) == fed(tuple(zip(rids, toks, wants))) == want
+    # one entry that is not such a vector sends the whole step the other way: strides, byte order, width, a second dimension, an id that is no int
+    for odd in (np.arange(6, dtype=np.int32)[::2], toks[1].astype(">i4"), toks[1].astype(np.int64), toks[1]):
+        assert fed([(5, toks[0], wants[0]), (np.int64(6), odd, wants[1])]) == [(5, toks[0].tolist(), None), (6, odd.tolist(), [2])]
+    assert fed([(5, np.ones((3, 1), dtype=np.int32), wants[1])]) == [(5, [1, 1, 1], [2])]

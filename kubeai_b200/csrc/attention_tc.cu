@@ -91,7 +91,7 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
 
   const AttnWork wk = work[blockIdx.y];     // q_count <= 64 query tokens of one sequence
   const int kvh = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const int kv_end = wk.q_pos0 + wk.q_count;                    // kv tokens visible to the last query of the block
   const int ntiles = (kv_end + kKvTile - 1) / kKvTile;
   const int last_page = (kv_end - 1) >> 4;
@@ -127,10 +127,11 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
   griddep_enter();
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       auto issue_tile = [&](int tile, int stage) {
         const uint32_t dst = kv_s + stage * kKvStage;
-        mbar_arrive_expect_tx(kv_full(stage), kKvStage);
+        if (one) mbar_arrive_expect_tx(kv_full(stage), kKvStage);
 #pragma unroll
         for (int pg = 0; pg < 4; ++pg) {
           int page = tile * 4 + pg;
@@ -140,25 +141,26 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
           const int row_v = row_k + Hkv * 16;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
+            if (!one) continue;
             tma_load_2d(dst + half * kHalf + pg * 2048, &tm_kv, kv_full(stage), half * 64, row_k, kEvictNormal);
             tma_load_2d(dst + kKTile + half * kHalf + pg * 2048, &tm_kv, kv_full(stage), half * 64, row_v, kEvictNormal);
           }
         }
       };
       // Q: two tiles x two 64-dim halves, rows ordered (token, head) by the 3-D box
-      mbar_arrive_expect_tx(q_bar, 2 * kQTile);
+      if (one) mbar_arrive_expect_tx(q_bar, 2 * kQTile);
       for (int i = 0; i < 2; ++i)
         for (int half = 0; half < 2; ++half)
-          tma_load_3d(q_s + i * kQTile + half * kQHalf, &tm_q, q_bar, half * 64, kvh * 4, wk.q_tok0 + i * kQTok);
+          if (one) tma_load_3d(q_s + i * kQTile + half * kQHalf, &tm_q, q_bar, half * 64, kvh * 4, wk.q_tok0 + i * kQTok);
       for (int s = 0; s < kStages && s < ntiles; ++s) issue_tile(s, s);
-      mbar_wait(q_bar, 0);
+      mbar_wait_warp(q_bar, 0);
 
       const uint32_t idesc_s = idesc_bf16(128, kKvTile, 0);
       const uint32_t idesc_pv = idesc_bf16(128, kD, 1);
       uint32_t ph_p[2] = {0, 0};
       for (int t = 0; t < ntiles; ++t) {
         const int stage = t % kStages;
-        mbar_wait(kv_full(stage), static_cast<uint32_t>(t / kStages) & 1u);
+        mbar_wait_warp(kv_full(stage), static_cast<uint32_t>(t / kStages) & 1u);
         tc_fence_after();
         const uint32_t ks = kv_s + stage * kKvStage, vs = ks + kKTile;
         // S_i = Q_i K^T.  S_i of the previous tile has been read: group i's p_ready arrival of tile t-1 (waited below
@@ -169,29 +171,30 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
           for (int k = 0; k < kD / 16; ++k) {
             const uint32_t koff = (k >> 2) * kQHalf + (k & 3) * 32;     // 64 dims per half, 32 B per k-step inside it
             const uint32_t kboff = (k >> 2) * kHalf + (k & 3) * 32;
-            umma_bf16(tm_S[i], smem_desc_sw128(q_s + i * kQTile + koff, 16, 1024), smem_desc_sw128(ks + kboff, 16, 1024), idesc_s,
+            if (one) umma_bf16(tm_S[i], smem_desc_sw128(q_s + i * kQTile + koff, 16, 1024), smem_desc_sw128(ks + kboff, 16, 1024), idesc_s,
                       k > 0 ? 1u : 0u);
           }
-          umma_commit(s_full(i));
+          if (one) umma_commit(s_full(i));
         }
         // PV_i += P_i V once group i has written P_i (and rescaled the running output to this tile's maximum)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          mbar_wait(p_ready(i), ph_p[i]);
+          mbar_wait_warp(p_ready(i), ph_p[i]);
           ph_p[i] ^= 1u;
           tc_fence_after();
 #pragma unroll
           for (int k = 0; k < kKvTile / 16; ++k) {
             // A = P_i: K-major rows of 128 B (64 kv), k-step = 32 B; B = V: MN-major, 16 kv rows per k-step = 2048 B,
             // leading offset = the second 64-dim half, stride = 8 rows
-            umma_bf16(tm_PV[i], smem_desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), smem_desc_sw128(vs + k * 2048, kHalf, 1024), idesc_pv,
+            if (one) umma_bf16(tm_PV[i], smem_desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), smem_desc_sw128(vs + k * 2048, kHalf, 1024), idesc_pv,
                       (t > 0 || k > 0) ? 1u : 0u);
           }
-          umma_commit(pv_full(i));
+          if (one) umma_commit(pv_full(i));
         }
-        umma_commit(kv_empty(stage));
+        if (one) umma_commit(kv_empty(stage));
+        __syncwarp();
         if (t + kStages < ntiles) {
-          mbar_wait(kv_empty(stage), static_cast<uint32_t>(t / kStages) & 1u);
+          mbar_wait_warp(kv_empty(stage), static_cast<uint32_t>(t / kStages) & 1u);
           issue_tile(t + kStages, stage);
         }
       }

@@ -33,7 +33,6 @@ namespace {
 
 constexpr int kSlab = 128;   // weight rows per CTA (UMMA M = 256 per pair)
 constexpr int kBlockK = 64;
-constexpr int kUmmaK = 16;
 constexpr int kThreads = 192;
 constexpr int kABytes = kSlab * kBlockK * 2;
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address -> rank 0's copy
@@ -110,15 +109,27 @@ __device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // D[tmem, 256 x N over the pair] (+)= A[256 x 16] * B[N x 16]; issued by the leader CTA only.
-__device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
+// A 64-wide step of K from 128-byte swizzled K-major tiles: four products, 32 bytes apart along K; the first adds to what D holds
+// only with `accumulate`.
+__device__ __forceinline__ void umma2_bf16_k64(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, t;\n"
+      ".reg .b64 a, b;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n"
+      "setp.eq.u32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "add.s64 a, %1, 2;\n"
+      "add.s64 b, %2, 2;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
+      "add.s64 a, %1, 4;\n"
+      "add.s64 b, %2, 4;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
+      "add.s64 a, %1, 6;\n"
+      "add.s64 b, %2, 6;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
       "}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Completion of all prior MMAs of this thread arrives on the same-offset mbarrier of BOTH CTAs.
@@ -171,7 +182,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
   const uint32_t tmem_slot = bar_base + 8u * (2 * C::kStages + 5);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_number();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -254,18 +265,19 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       const uint64_t w_hint = ntt > 1 ? kEvictNormal : kEvictFirst;
       int pre = 0;
       for (long long v = 0; v < v_end && pre < C::kStages; ++v, ++pre) {
         int kb;
         const int tile = tile_kb_at(v, &kb);
-        if (leader) mbar_arrive_expect_tx(full_bar(pre), 2u * C::kStageBytes);
-        tma_load_2d_pair(smem_base + pre * C::kStageBytes, &tm_w, full_bar(pre), kb * kBlockK,
+        if (leader && one) mbar_arrive_expect_tx(full_bar(pre), 2u * C::kStageBytes);
+        if (one) tma_load_2d_pair(smem_base + pre * C::kStageBytes, &tm_w, full_bar(pre), kb * kBlockK,
                          (tile / ntt) * 2 * kSlab + static_cast<int>(rank) * kSlab, w_hint);
       }
       griddep_wait();
-      mark(12);
+      if (one) mark(12);
       int stage = 0, idx = 0;
       uint32_t phase = 0;
       for (long long v = 0; v < v_end; ++v, ++idx) {
@@ -274,16 +286,16 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         const int slab2 = tile / ntt, tt = tile - slab2 * ntt;
         const uint32_t sa = smem_base + stage * C::kStageBytes;
         if (idx >= pre) {
-          mbar_wait(empty_bar(stage), phase ^ 1u);
-          if (leader) mbar_arrive_expect_tx(full_bar(stage), 2u * C::kStageBytes);
-          tma_load_2d_pair(sa, &tm_w, full_bar(stage), kb * kBlockK, slab2 * 2 * kSlab + static_cast<int>(rank) * kSlab, w_hint);
+          mbar_wait_warp(empty_bar(stage), phase ^ 1u);
+          if (leader && one) mbar_arrive_expect_tx(full_bar(stage), 2u * C::kStageBytes);
+          if (one) tma_load_2d_pair(sa, &tm_w, full_bar(stage), kb * kBlockK, slab2 * 2 * kSlab + static_cast<int>(rank) * kSlab, w_hint);
         }
 #pragma unroll
         for (int c = 0; c < C::kNch; ++c) {
           // this CTA stages the rank-th half of chunk c (the box is always kHalf rows; rows past nc/2 are ignored)
           const int nc = chunk_n(tt, c);
           const int row0 = tt * BLOCK_N + c * C::kChunk + static_cast<int>(rank) * (nc >> 1);
-          tma_load_2d_pair(sa + kABytes + c * (C::kHalf * kBlockK * 2), &tm_x, full_bar(stage), kb * kBlockK,
+          if (one) tma_load_2d_pair(sa + kABytes + c * (C::kHalf * kBlockK * 2), &tm_x, full_bar(stage), kb * kBlockK,
                            nc > 0 ? row0 : T /* fully out of range -> zero fill */, kEvictLast);
         }
         if (++stage == C::kStages) {
@@ -291,23 +303,24 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
           phase ^= 1u;
         }
       }
-      mark(13);
+      if (one) mark(13);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool one = elect_one();
       griddep_wait();
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       for (long long it = 0; it < v_end;) {
         Seg sg = seg_at(it);
         const int slab2 = sg.tile / ntt, tt = sg.tile - slab2 * ntt;
-        mbar_wait(tempty_bar(acc), acc_phase ^ 1u);
+        mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u);
         tc_fence_after();
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          mbar_wait(full_bar(stage), phase);
+          mbar_wait_warp(full_bar(stage), phase);
           tc_fence_after();
-          if (it == 0 && kb == sg.kb0) mark(10);
+          if (one && it == 0 && kb == sg.kb0) mark(10);
           const uint32_t sa = smem_base + stage * C::kStageBytes;
           const uint64_t a_desc = umma_desc_kmajor_sw128(sa);
 #pragma unroll
@@ -317,12 +330,13 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             const uint32_t idesc = umma_idesc_bf16(2 * kSlab, nc);
             const uint32_t d_tmem = tmem_base + acc * BLOCK_N + c * C::kChunk;
             const uint64_t b_desc = umma_desc_kmajor_sw128(sa + kABytes + c * (C::kHalf * kBlockK * 2));
-#pragma unroll
-            for (int k = 0; k < kBlockK / kUmmaK; ++k)
-              umma2_bf16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
+            if (one) umma2_bf16_k64(d_tmem, a_desc, b_desc, idesc, kb > sg.kb0 ? 1u : 0u);
           }
-          umma2_commit_both(empty_bar(stage));
-          if (kb == sg.kb1 - 1) umma2_commit_both(tfull_bar(acc));
+          if (one) {
+            umma2_commit_both(empty_bar(stage));
+            if (kb == sg.kb1 - 1) umma2_commit_both(tfull_bar(acc));
+          }
+          __syncwarp();
           if (++stage == C::kStages) {
             stage = 0;
             phase ^= 1u;
@@ -334,7 +348,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
         }
         it += sg.kb1 - sg.kb0;
       }
-      mark(11);
+      if (one) mark(11);
     }
   } else {
     // ------------------------------------------------------------ epilogue warps (both CTAs, own 128 rows)

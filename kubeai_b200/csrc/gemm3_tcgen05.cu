@@ -52,7 +52,6 @@ namespace {
 
 constexpr int kSlab = 128;     // weight rows per CTA (UMMA M = 256 per pair)
 constexpr int kBlockK = 64;
-constexpr int kUmmaK = 16;
 constexpr int kBN = 128;       // token tile (one tile per launch: T <= 128)
 constexpr int kChunkTok = 32;  // tokens per epilogue chunk (one tcgen05.ld 32x32b.x32)
 constexpr int kNumChunks = kBN / kChunkTok;
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3_kernel(const __grid_constan
       P.trace[static_cast<size_t>(blockIdx.x) * 8 + i] = t;
     }
   };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   if (threadIdx.x == 64) mark(0);
   const uint32_t crank = cluster_ctarank();       // rank in the cluster (2S CTAs)
   const uint32_t rank = crank & 1u;               // rank in the pair
@@ -186,13 +185,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3_kernel(const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       const uint64_t w_hint = kEvictFirst;
       int pre = 0;
       for (long long it = it_begin; it < it_end && pre < kStages; ++it, ++pre) {
         const int tile = static_cast<int>(it / KB), kb = static_cast<int>(it - static_cast<long long>(tile) * KB);
-        if (leader) mbar_arrive_expect_tx(full_bar(pre), pro_norm ? 2u * kABytes : 2u * kStageBytes);
-        tma_load_2d_pair(smem_base + pre * kStageBytes, &P.tm_w, full_bar(pre), kb * kBlockK, tile * 2 * kSlab + static_cast<int>(rank) * kSlab,
+        if (leader && one) mbar_arrive_expect_tx(full_bar(pre), pro_norm ? 2u * kABytes : 2u * kStageBytes);
+        if (one) tma_load_2d_pair(smem_base + pre * kStageBytes, &P.tm_w, full_bar(pre), kb * kBlockK, tile * 2 * kSlab + static_cast<int>(rank) * kSlab,
                          w_hint);
       }
       griddep_wait();
@@ -202,14 +202,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3_kernel(const __grid_constan
         const int tile = static_cast<int>(it / KB), kb = static_cast<int>(it - static_cast<long long>(tile) * KB);
         const uint32_t sa = smem_base + stage * kStageBytes;
         if (idx >= pre) {
-          mbar_wait(empty_bar(stage), phase ^ 1u);
-          if (leader) mbar_arrive_expect_tx(full_bar(stage), pro_norm ? 2u * kABytes : 2u * kStageBytes);
-          tma_load_2d_pair(sa, &P.tm_w, full_bar(stage), kb * kBlockK, tile * 2 * kSlab + static_cast<int>(rank) * kSlab, w_hint);
+          mbar_wait_warp(empty_bar(stage), phase ^ 1u);
+          if (leader && one) mbar_arrive_expect_tx(full_bar(stage), pro_norm ? 2u * kABytes : 2u * kStageBytes);
+          if (one) tma_load_2d_pair(sa, &P.tm_w, full_bar(stage), kb * kBlockK, tile * 2 * kSlab + static_cast<int>(rank) * kSlab, w_hint);
         }
         if (pro_norm) {
-          mbar_arrive_expect_tx(bfull_bar(stage), kBBytes);
-          tma_load_2d(sa + kABytes, &P.tm_x, bfull_bar(stage), kb * kBlockK, row_half0, kEvictLast);
-        } else {
+          if (one) {
+            mbar_arrive_expect_tx(bfull_bar(stage), kBBytes);
+            tma_load_2d(sa + kABytes, &P.tm_x, bfull_bar(stage), kb * kBlockK, row_half0, kEvictLast);
+          }
+        } else if (one) {
           tma_load_2d_pair(sa + kABytes, &P.tm_x, full_bar(stage), kb * kBlockK, row_half0, kEvictLast);
         }
         if (++stage == kStages) {
@@ -220,29 +222,34 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3_kernel(const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA of the pair)
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool one = elect_one();
       griddep_wait();
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       const uint32_t idesc = umma_idesc_bf16(2 * kSlab, nc);
       for (long long it = it_begin; it < it_end;) {
         const Seg sg = seg_at(it);
-        mbar_wait(tempty_bar(acc), acc_phase ^ 1u);
+        mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u);
         tc_fence_after();
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          mbar_wait(full_bar(stage), phase);
-          if (pro_norm) mbar_wait_cluster(xf_bar(stage), phase);
+          mbar_wait_warp(full_bar(stage), phase);
+          if (pro_norm) {
+            mbar_wait_cluster(xf_bar(stage), phase);
+            __syncwarp();
+          }
           tc_fence_after();
-          if (it == it_begin && kb == sg.kb0) mark(2);
+          if (one && it == it_begin && kb == sg.kb0) mark(2);
           const uint32_t sa = smem_base + stage * kStageBytes;
           const uint64_t a_desc = umma_desc_kmajor_sw128(sa);
           const uint64_t b_desc = umma_desc_kmajor_sw128(sa + kABytes);
           const uint32_t d_tmem = tmem_base + acc * kBN;
-#pragma unroll
-          for (int k = 0; k < kBlockK / kUmmaK; ++k)
-            umma2_bf16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
-          umma2_commit_pair(empty_bar(stage), pair_mask);
-          if (kb == sg.kb1 - 1) umma2_commit_pair(tfull_bar(acc), pair_mask);
+          if (one) {
+            umma2_bf16_k64(d_tmem, a_desc, b_desc, idesc, kb > sg.kb0 ? 1u : 0u);
+            umma2_commit_pair(empty_bar(stage), pair_mask);
+            if (kb == sg.kb1 - 1) umma2_commit_pair(tfull_bar(acc), pair_mask);
+          }
+          __syncwarp();
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -254,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3_kernel(const __grid_constan
         }
         it += sg.kb1 - sg.kb0;
       }
-      mark(3);
+      if (one) mark(3);
     }
   } else if (warp >= 6) {
     // ------------------------------------------------------------ transform warps: RMSNorm of the token tile in smem

@@ -102,11 +102,9 @@ struct Walk {
   }
 };
 
-__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < kWaitLimit; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
+__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) { return mbar_wait_limited(bar, parity, kWaitLimit); }
+// ... by a whole warp: whether all lanes saw the phase end
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_limited(bar, parity)); }
 template <int EPI>
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(groups_of(EPI) * 128) : "memory"); }
 // whether all epilogue threads say yes (they also meet here)
@@ -237,7 +235,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kMaxStages + 2 + a); };   // the leader's copy
   const uint32_t tmem_slot = bar_base + 8u * (2 * kMaxStages + 4);
   uint8_t* stage_out = smem_raw + (bar_base + 256 - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int units = gridDim.x >> 1, unit = blockIdx.x >> 1, KB = (K + kBlockK - 1) / kBlockK;
@@ -270,65 +268,68 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   if (expert_rows || warp != 0) griddep_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0, ahead = 0, filled = 0;
-      uint32_t phase = 0;
-      Tile t;
-      auto load_w = [&](int st, int kb) {
-        if (leader) mbar_arrive_expect_tx(full_bar(st), 2u * stage_step);
-        tma_load_2d_pair(smem_base + st * stage_step, &tm_w, full_bar(st), kb * kBlockK, t.wrow + static_cast<int>(rank) * kSlab, kEvictNormal);
-      };
-      if (!expert_rows) {
-        // the weights do not wait for the kernel in front: the ring's first stages of them are on their way before it ends
-        if (walk.at(unit, &t) && t.rows)
-          for (; ahead < min(stages, t.kb1 - t.kb0); ++ahead) load_w(ahead, t.kb0 + ahead);
-        griddep_wait();
-      }
-      for (long long item = unit; ok && walk.at(item, &t); item += units) {
-        if (!t.rows) continue;
-        const int nc = (t.rows + 15) & ~15;
-        for (int kb = t.kb0; kb < t.kb1; ++kb) {
-          const uint32_t sa = smem_base + stage * stage_step;
-          if (ahead > 0) {
-            --ahead;
-          } else {
-            if (!wait_limited(empty_bar(stage), phase ^ 1u)) { ok = false; break; }
-            load_w(stage, kb);
-          }
-          filled = min(filled + 1, stages);
-          // this CTA stages the rank-th half of the row tile (rows of the box past nc / 2 are not used)
-          tma_load_2d_pair(sa + kABytes, &tm_x, full_bar(stage), kb * kBlockK, t.row0 + static_cast<int>(rank) * (nc >> 1), kEvictLast);
-          if (++stage == stages) { stage = 0; phase ^= 1u; }
-        }
-      }
-      // The copies started last have landed before the CTA ends, also where a role gave up: the leader's barriers count both CTAs'
-      // bytes.  (Where none did, they were waited for long ago.)
-      if (leader)
-        for (int i = 0; i < filled; ++i) {
-          if (--stage < 0) { stage = stages - 1; phase ^= 1u; }
-          wait_limited(full_bar(stage), phase);
-        }
+    const bool one = elect_one();
+    int stage = 0, ahead = 0, filled = 0;
+    uint32_t phase = 0;
+    Tile t;
+    auto load_w = [&](int st, int kb) {
+      if (!one) return;
+      if (leader) mbar_arrive_expect_tx(full_bar(st), 2u * stage_step);
+      tma_load_2d_pair(smem_base + st * stage_step, &tm_w, full_bar(st), kb * kBlockK, t.wrow + static_cast<int>(rank) * kSlab, kEvictNormal);
+    };
+    if (!expert_rows) {
+      // the weights do not wait for the kernel in front: the ring's first stages of them are on their way before it ends
+      if (walk.at(unit, &t) && t.rows)
+        for (; ahead < min(stages, t.kb1 - t.kb0); ++ahead) load_w(ahead, t.kb0 + ahead);
+      griddep_wait();
     }
+    for (long long item = unit; ok && walk.at(item, &t); item += units) {
+      if (!t.rows) continue;
+      const int nc = (t.rows + 15) & ~15;
+      for (int kb = t.kb0; kb < t.kb1; ++kb) {
+        const uint32_t sa = smem_base + stage * stage_step;
+        if (ahead > 0) {
+          --ahead;
+        } else {
+          if (!warp_wait(empty_bar(stage), phase ^ 1u)) { ok = false; break; }
+          load_w(stage, kb);
+        }
+        filled = min(filled + 1, stages);
+        // this CTA stages the rank-th half of the row tile (rows of the box past nc / 2 are not used)
+        if (one) tma_load_2d_pair(sa + kABytes, &tm_x, full_bar(stage), kb * kBlockK, t.row0 + static_cast<int>(rank) * (nc >> 1), kEvictLast);
+        if (++stage == stages) { stage = 0; phase ^= 1u; }
+      }
+    }
+    // The copies started last have landed before the CTA ends, also where a role gave up: the leader's barriers count both CTAs'
+    // bytes.  (Where none did, they were waited for long ago.)
+    if (leader)
+      for (int i = 0; i < filled; ++i) {
+        if (--stage < 0) { stage = stages - 1; phase ^= 1u; }
+        wait_limited(full_bar(stage), phase);
+      }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool one = elect_one();
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       Tile t;
       for (long long item = unit; ok && walk.at(item, &t); item += units) {
         if (!t.rows) continue;
         const uint32_t idesc = umma_idesc_bf16(2 * kSlab, (t.rows + 15) & ~15);
-        if (!wait_limited(tempty_bar(acc), acc_phase ^ 1u)) { ok = false; break; }
+        if (!warp_wait(tempty_bar(acc), acc_phase ^ 1u)) { ok = false; break; }
         tc_fence_after();
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
-          if (!wait_limited(full_bar(stage), phase)) { ok = false; break; }
+          if (!warp_wait(full_bar(stage), phase)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_base + stage * stage_step;
           const uint64_t a_desc = umma_desc_kmajor_sw128(sa), b_desc = umma_desc_kmajor_sw128(sa + kABytes);
-#pragma unroll
-          for (int k = 0; k < kBlockK / kUmmaK; ++k)
-            umma2_bf16(tmem_base + acc * kRows, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > t.kb0 || k > 0) ? 1u : 0u);
-          umma2_commit_pair(empty_bar(stage), 3);
-          if (kb == t.kb1 - 1) umma2_commit_pair(tfull_bar(acc), 3);
+          if (one) {
+            umma2_bf16_k64(tmem_base + acc * kRows, a_desc, b_desc, idesc, kb > t.kb0 ? 1u : 0u);
+            umma2_commit_pair(empty_bar(stage), 3);
+            if (kb == t.kb1 - 1) umma2_commit_pair(tfull_bar(acc), 3);
+          }
+          __syncwarp();
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }

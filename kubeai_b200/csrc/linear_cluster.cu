@@ -35,11 +35,7 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes)
 }
 // this thread's copies so far, once they are through, count as its arrival
 __device__ __forceinline__ void copies_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < kWaitLimit; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
+__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) { return mbar_wait_limited(bar, parity, kWaitLimit); }
 __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
@@ -66,7 +62,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_cluster_kernel(LinearArgs 
   auto full = [&](int i) { return bars + 8u * i; };
   auto empty = [&](int i) { return bars + 8u * (kMaxStages + i); };
   const uint32_t done = bars + 8u * 2 * kMaxStages, slot = done + 8;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_number();
   const int rank = static_cast<int>(cluster_ctarank()), n0 = blockIdx.x / C * R;
   const int KB = (a.K + 64 * KS - 1) / (64 * KS), kb0 = rank * KB / C, kbn = (rank + 1) * KB / C - kb0;
   if (warp == kLoaders) {
@@ -122,10 +118,11 @@ __global__ void __launch_bounds__(kThreads, 1) linear_cluster_kernel(LinearArgs 
       copies_arrive(full(i % D));
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (lane == 0) {
+  } else {
+    const bool one = elect_one();
     const uint32_t idesc = umma_idesc_bf16(128, R);
     for (int i = 0; i < kbn && ok; ++i) {
-      ok = wait_limited(full(i % D), (i / D) & 1);
+      ok = __all_sync(0xffffffffu, wait_limited(full(i % D), (i / D) & 1));
       if (!ok) break;
       fence_proxy_async();      // the copies wrote through the generic proxy, the tensor cores read through the other
       tc_fence_after();
@@ -136,13 +133,13 @@ __global__ void __launch_bounds__(kThreads, 1) linear_cluster_kernel(LinearArgs 
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
           const uint64_t ad = umma_desc_kmajor_sw128(at + m * 16384);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16(tmem + m * R, ad + 2u * k, bd + 2u * k, idesc, (i > 0 || h > 0 || k > 0) ? 1u : 0u);
+          if (one) umma_bf16_k64(tmem + m * R, ad, bd, idesc, (i > 0 || h > 0) ? 1u : 0u);
         }
       }
-      umma_commit(empty(i % D));
+      if (one) umma_commit(empty(i % D));
+      __syncwarp();
     }
-    umma_commit(done);
+    if (one) umma_commit(done);
   }
   __syncwarp();
   ok = wait_limited(done, 0) && ok;

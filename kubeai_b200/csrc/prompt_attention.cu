@@ -57,11 +57,9 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr, uint32_t lbo, uint
   return static_cast<uint64_t>((addr & 0x3FFFFu) >> 4) | static_cast<uint64_t>((lbo >> 4) & 0x3FFFu) << 16 | static_cast<uint64_t>((sbo >> 4) & 0x3FFFu) << 32 |
          static_cast<uint64_t>(1) << 46 | static_cast<uint64_t>(2) << 61;
 }
-__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < kWaitLimit; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
+__device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) { return mbar_wait_limited(bar, parity, kWaitLimit); }
+// ... by a whole warp: whether all lanes saw the phase end
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_limited(bar, parity)); }
 
 // (From 2^-126 to 1, where weights and rescaling factors lie, the same bits as exp2f for every argument; below, 0.)
 __device__ __forceinline__ float exp2_ftz(float x) {
@@ -144,7 +142,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   auto p_ready = [&](int i) { return bars + 8u * (12 + i); };     // 4 warps: P_i written, S_i read, O_i rescaled
   auto pv_full = [&](int i) { return bars + 8u * (14 + i); };
   const uint32_t q_bar = bars + 8u * 16, v2_full = bars + 8u * 17, v2_empty = bars + 8u * 18, tmem_slot = bars + 8u * 19;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -199,21 +197,24 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool ok = true;
 
     if (warp == 0) {
-      if (lane == 0) {
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_kv);
+      {
+        const bool one = elect_one();
         const int tiles = last[1] >= 0 ? 2 : 1;
-        mbar_arrive_expect_tx(q_bar, tiles * NS * kQSlab);
+        if (one) {
+          tma_prefetch_desc(&tm_q);
+          tma_prefetch_desc(&tm_kv);
+          mbar_arrive_expect_tx(q_bar, tiles * NS * kQSlab);
+        }
         for (int i = 0; i < tiles; ++i)
           for (int s = 0; s < NS; ++s)
-            tma_load_2d(q_s + (i * NS + s) * kQSlab, s < 2 ? &tm_q : &tm_q2, q_bar, s < 2 ? head * a.q_step + 64 * s : head * 64, tok0 + q0 + i * kRows, kEvictNormal);
+            if (one) tma_load_2d(q_s + (i * NS + s) * kQSlab, s < 2 ? &tm_q : &tm_q2, q_bar, s < 2 ? head * a.q_step + 64 * s : head * 64, tok0 + q0 + i * kRows, kEvictNormal);
         int nk = 0, nv = 0, nl = 0;      // tiles of keys, values and second terms on their way
         auto keys = [&] {
           const int st = nk & 1;
-          if (!wait_limited(k_empty(st), ((nk >> 1) & 1) ^ 1u)) return false;
-          mbar_arrive_expect_tx(k_full(st), NS * kKSlab);
+          if (!warp_wait(k_empty(st), ((nk >> 1) & 1) ^ 1u)) return false;
+          if (one) mbar_arrive_expect_tx(k_full(st), NS * kKSlab);
           for (int s = 0; s < NS; ++s)
-            tma_load_2d(k_s + (st * NS + s) * kKSlab, s < 2 ? &tm_kv : &tm_k2, k_full(st), s < 2 ? a.k_off + kvh * a.k_step + 64 * s : 0, tok0 + (t_begin + nk) * kKeys,
+            if (one) tma_load_2d(k_s + (st * NS + s) * kKSlab, s < 2 ? &tm_kv : &tm_k2, k_full(st), s < 2 ? a.k_off + kvh * a.k_step + 64 * s : 0, tok0 + (t_begin + nk) * kKeys,
                         kEvictLast);
           ++nk;
           return true;
@@ -223,70 +224,77 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           // with one buffer of second terms that wait is the long one: the next keys go ahead of it
           if ((!LO || t + 1 < t_end) && !(ok = keys())) break;
           const int st = nv & 1, row = tok0 + t * kKeys;
-          if (!(ok = wait_limited(v_empty(st), ((nv >> 1) & 1) ^ 1u))) break;
-          mbar_arrive_expect_tx(v_full(st), kVTile);
-          for (int s = 0; s < 2; ++s) tma_load_2d(v_s + st * kVTile + s * kKSlab, &tm_kv, v_full(st), a.v_off + kvh * a.v_step + 64 * s, row, kEvictLast);
+          if (!(ok = warp_wait(v_empty(st), ((nv >> 1) & 1) ^ 1u))) break;
+          if (one) mbar_arrive_expect_tx(v_full(st), kVTile);
+          for (int s = 0; s < 2; ++s)
+            if (one) tma_load_2d(v_s + st * kVTile + s * kKSlab, &tm_kv, v_full(st), a.v_off + kvh * a.v_step + 64 * s, row, kEvictLast);
           ++nv;
           if constexpr (LO) {
-            if (!(ok = wait_limited(v2_empty, (nl & 1) ^ 1u))) break;
-            mbar_arrive_expect_tx(v2_full, kVTile);
-            for (int s = 0; s < 2; ++s) tma_load_2d(v2_s + s * kKSlab, &tm_v2, v2_full, head * kD + 64 * s, row, kEvictLast);
+            if (!(ok = warp_wait(v2_empty, (nl & 1) ^ 1u))) break;
+            if (one) mbar_arrive_expect_tx(v2_full, kVTile);
+            for (int s = 0; s < 2; ++s)
+              if (one) tma_load_2d(v2_s + s * kKSlab, &tm_v2, v2_full, head * kD + 64 * s, row, kEvictLast);
             ++nl;
           }
         }
         // the copies in flight land before the CTA ends, also where it gives up
-        wait_limited(q_bar, 0);
-        for (int j = max(0, nk - 2); j < nk; ++j) wait_limited(k_full(j & 1), (j >> 1) & 1);
-        for (int j = max(0, nv - 2); j < nv; ++j) wait_limited(v_full(j & 1), (j >> 1) & 1);
-        if (nl > 0) wait_limited(v2_full, (nl - 1) & 1);
+        warp_wait(q_bar, 0);
+        for (int j = max(0, nk - 2); j < nk; ++j) warp_wait(k_full(j & 1), (j >> 1) & 1);
+        for (int j = max(0, nv - 2); j < nv; ++j) warp_wait(v_full(j & 1), (j >> 1) & 1);
+        if (nl > 0) warp_wait(v2_full, (nl - 1) & 1);
       }
     } else if (warp == 9) {
-      if (lane == 0) {
+      {
+        const bool one = elect_one();
         const uint32_t id_s = idesc_bf16(kRows, kKeys, 0), id_o = idesc_bf16(kRows, kD, 1);
         uint32_t ph_p[2] = {0, 0};
         auto scores = [&](int t) {
           const int it = t - t_begin, st = it & 1;
-          if (!wait_limited(k_full(st), (it >> 1) & 1)) return false;
+          if (!warp_wait(k_full(st), (it >> 1) & 1)) return false;
           tc_fence_after();
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (!active(i, t)) continue;
 #pragma unroll
             for (int k = 0; k < 4 * NS; ++k)
-              umma_bf16(tm_s(i, t & 1), desc_sw128(q_s + (i * NS + (k >> 2)) * kQSlab + (k & 3) * 32, 16, 1024),
+              if (one) umma_bf16(tm_s(i, t & 1), desc_sw128(q_s + (i * NS + (k >> 2)) * kQSlab + (k & 3) * 32, 16, 1024),
                         desc_sw128(k_s + (st * NS + (k >> 2)) * kKSlab + (k & 3) * 32, 16, 1024), id_s, k > 0 ? 1u : 0u);
-            umma_commit(s_full(i, t & 1));
+            if (one) umma_commit(s_full(i, t & 1));
           }
-          umma_commit(k_empty(st));
+          if (one) umma_commit(k_empty(st));
+          __syncwarp();
           return true;
         };
-        ok = wait_limited(q_bar, 0) && scores(t_begin);
+        ok = warp_wait(q_bar, 0) && scores(t_begin);
         for (int t = t_begin; ok && t < t_end; ++t) {
           const int it = t - t_begin, st = it & 1;
           // the next scores go to the other buffers, whose readers have handed in their P of the tile before this one
           if (t + 1 < t_end && !(ok = scores(t + 1))) break;
-          if (!(ok = wait_limited(v_full(st), (it >> 1) & 1))) break;
+          if (!(ok = warp_wait(v_full(st), (it >> 1) & 1))) break;
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (!active(i, t)) continue;
-            if (!(ok = wait_limited(p_ready(i), ph_p[i]))) break;
+            if (!(ok = warp_wait(p_ready(i), ph_p[i]))) break;
             ph_p[i] ^= 1u;
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < kKeys / 16; ++k)
-              umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v_s + st * kVTile + k * 2048, kKSlab, 1024), id_o,
+              if (one) umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v_s + st * kVTile + k * 2048, kKSlab, 1024), id_o,
                         (t > first[i] || k > 0) ? 1u : 0u);
             if constexpr (LO) {
-              if (!(ok = wait_limited(v2_full, it & 1))) break;
+              if (!(ok = warp_wait(v2_full, it & 1))) break;
               tc_fence_after();
 #pragma unroll
               for (int k = 0; k < kKeys / 16; ++k)
-                umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v2_s + k * 2048, kKSlab, 1024), id_o, 1u);
+                if (one) umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v2_s + k * 2048, kKSlab, 1024), id_o, 1u);
             }
-            umma_commit(pv_full(i));
+            if (one) umma_commit(pv_full(i));
           }
-          umma_commit(v_empty(st));
-          if constexpr (LO) umma_commit(v2_empty);
+          if (one) {
+            umma_commit(v_empty(st));
+            if constexpr (LO) umma_commit(v2_empty);
+          }
+          __syncwarp();
         }
       }
     } else {

@@ -49,6 +49,55 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
+// ... by a whole warp of which one lane goes on to act on it: no lane is left behind at a phase that the next round may end
+__device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  mbar_wait(bar, parity);
+  __syncwarp();
+}
+
+// A wait that gives up after `limit` tries.  The loop is part of the instruction sequence, so the code around it stays
+// convergent where a whole warp waits.
+__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, uint32_t limit) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b32 left;\n"
+      "mov.b32 left, %3;\n"
+      "TRY:\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "@p bra DONE;\n"
+      "sub.u32 left, left, 1;\n"
+      "setp.ne.u32 q, left, 0;\n"
+      "@q bra TRY;\n"
+      "DONE:\n"
+      "selp.b32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(limit)
+      : "memory");
+  return ok != 0;
+}
+
+// One lane of a converged warp.  Tensor-core and TMA instructions take their operands from the warp's uniform registers: behind
+// `if (lane == 0)` every operand of every instruction is moved there one by one, because values of a thread that is alone need not
+// be the warp's.  Roles therefore run as whole warps whose one elected lane issues.  Measured on the CTA-pair product: four products of a 64-wide step of K
+// and their commit took their thread 580 cycles whatever the tile, of which a tile of 256 x 256 needs 512 and one of 256 x 128 256; 2048 x 8192, 4096
+// rows in tiles of 128: 182 us before, 120 since.  (The mask of disabled lanes, eight more operands of every CTA-pair product, went too.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.b32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(one));
+  return one != 0;
+}
+// the warp's number, as a value that the compiler knows to be the same in all its lanes
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+
 // the same wait with cluster-scope acquire: the barrier is signalled by a thread of ANOTHER CTA of the cluster
 __device__ __forceinline__ void mbar_wait_cluster(uint32_t bar, uint32_t parity) {
   uint32_t ok = 0;
@@ -141,6 +190,29 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint
       ".reg .pred p;\n"
       "setp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// A 64-wide step of K from 128-byte swizzled K-major tiles: four products, 32 bytes apart along K; the first adds to what D holds
+// only with `accumulate`.
+__device__ __forceinline__ void umma_bf16_k64(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, t;\n"
+      ".reg .b64 a, b;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.eq.u32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "add.s64 a, %1, 2;\n"
+      "add.s64 b, %2, 2;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n"
+      "add.s64 a, %1, 4;\n"
+      "add.s64 b, %2, 4;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n"
+      "add.s64 a, %1, 6;\n"
+      "add.s64 b, %2, 6;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n"
       "}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");

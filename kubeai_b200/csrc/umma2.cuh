@@ -52,6 +52,29 @@ __device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t a_desc, uin
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
+// A 64-wide step of K from 128-byte swizzled K-major tiles: four products, 32 bytes apart along K; the first adds to what D holds
+// only with `accumulate`.
+__device__ __forceinline__ void umma2_bf16_k64(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, t;\n"
+      ".reg .b64 a, b;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.eq.u32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "add.s64 a, %1, 2;\n"
+      "add.s64 b, %2, 2;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
+      "add.s64 a, %1, 4;\n"
+      "add.s64 b, %2, 4;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
+      "add.s64 a, %1, 6;\n"
+      "add.s64 b, %2, 6;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // completion of all prior MMAs of this thread arrives on the same-offset mbarrier of both CTAs of the pair
 __device__ __forceinline__ void umma2_commit_pair(uint32_t bar, uint16_t cta_mask) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"

@@ -132,10 +132,10 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
     set_error("b200_op_gemm: problem too large for the op-level scratch");
     return B200_ERR_INVALID;
   }
-  CUtensorMap tmx;
-  rc = gemm_make_x_map(&tmx, x, T, K, K, bn);
-  if (rc) return cuda_fail("gemm_make_x_map", rc);
-  rc = gemm_run(plan, tmx, bn, out, N, T, static_cast<cudaStream_t>(stream));
+  CUtensorMap tmx[kGemmNumBlockN];
+  rc = gemm_make_x_maps(tmx, x, T, K, K);
+  if (rc) return cuda_fail("gemm_make_x_maps", rc);
+  rc = gemm_run(plan, tmx, out, N, T, static_cast<cudaStream_t>(stream));
   if (rc) return cuda_fail("gemm_run", rc);
   return 0;
 }
@@ -232,6 +232,21 @@ int b200_op_gemm3(const b200_gemm3_args* a, void* stream, int32_t* schedule_out)
       const int rs = linear_stream(la, &q, st);
       return rs ? cuda_fail("linear_stream", rs) : 0;
     }
+    // more of them: whole tiles, as the engine's steps take them (28672 x 4096, 16 to 96 tokens: 48.5 to 52 us on this kernel, 46 to 49 so).  A
+    // full tile of tokens keeps this kernel's schedule, of whose plain product its epilogues are bit by bit a function.
+    if (gemm_variant() == 2 && a->N % 256 == 0 && a->K % 64 == 0 && a->T <= 112 && a->ldo % 8 == 0 && reinterpret_cast<uintptr_t>(a->out) % 16 == 0) {
+      if (const int rm = report_mark()) return rm;
+      GemmPlan plan;
+      CUtensorMap tmx[kGemmNumBlockN];
+      int rw = gemm_plan_init(&plan, a->w, a->N, a->K, a->K, g_ws, g_counters, 0);
+      if (!rw) rw = gemm_make_x_maps(tmx, a->x, a->x_rows, a->K, a->K);
+      plan.error = g_mark;
+      plan.ws_bytes = g_ws_bytes;
+      const GroupedOut o = {a->out, a->ldo, GROUPED_SILU};
+      if (!rw) rw = gemm_whole_run(plan, tmx, a->T, o, st);
+      if (schedule_out) { schedule_out[0] = 1; schedule_out[1] = 0; schedule_out[2] = plan.max_ctas; }
+      return rw ? cuda_fail("gemm_whole_run", rw) : 0;
+    }
   }
   Gemm3Schedule sch;
   int rc = gemm3_schedule(a->N, a->K, a->T, a->pro, a->force, &sch);
@@ -306,6 +321,12 @@ int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_ROW_BLOCKS && n == 5) return rules::row_blocks_pay(v[0], v[1], v[2], v[3], v[4] != 0);
   if (v && rule == B200_RULE_SINGLE_STEP && n == 5) return rules::single_step_pays(v[0], v[1], v[2], v[3] != 0, v[4]);
   if (v && rule == B200_RULE_LATENT_ROWS && n == 2) return rules::latent_rows_held(v[0], v[1]);
+  if (v && rule == B200_RULE_TILES && n == 3) return rules::tiles_ahead(v[0], v[1], v[2]);
+  if (v && (rule == B200_RULE_TILE_ROWS || rule == B200_RULE_TILE_PARTS) && n == 5 && v[0] > 0 && v[1] > 0 && v[2] > 0 && v[3] > 0) {
+    int tile, parts;
+    rules::whole_tiles(v[0], v[1], v[2], v[3], v[4] != 0, &tile, &parts);
+    return rule == B200_RULE_TILE_ROWS ? tile : parts;
+  }
   set_error("b200_rule_query: rule %d with %d sizes", rule, n);
   return B200_ERR_INVALID;
 }

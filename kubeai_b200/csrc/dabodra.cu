@@ -590,15 +590,13 @@ class Dabodra : public Model {
   bool takes_whole(bool tc, int T) const { return tc && T > 256 && whole; }
   int run_whole(const GemmPlan& plan, const CUtensorMap* xm, bool glu, void* Y, int ldy, int T) {
     const GroupedOut o = {Y, ldy, glu ? GROUPED_GATED_FAST : GROUPED_PLAIN, nullptr, INFINITY, 1.f, 0.f};
-    const int bn = gemm_block_n_for(T);
-    return gemm_whole_run(plan, xm[gemm_block_n_index(bn)], bn, T, o, env.stream);
+    return gemm_whole_run(plan, xm, T, o, env.stream);
   }
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
     if (takes_whole(tc, T)) return run_whole(plan, xm, false, Y, N, T);
     const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
     if (tc && T > few_rows && !linear_few(la)) {
-      const int bn = gemm_block_n_for(T);
-      return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
+      return gemm_run(plan, xm, Y, N, T, env.stream);
     }
     return linear(la, env.stream);
   }

@@ -49,6 +49,18 @@ inline bool stream_pays(int T, int N, int K, bool pairs) {
 //   K 14336  0.83 .. 1.08 (to 128 tokens), 1.0 .. 1.12 (129 on); 1.08 .. 1.19     K 28672  1.12 .. 1.52, 1.28 .. 1.42
 inline bool cluster_pays(int T, int N, int K) { return K <= (N > 2112 ? 6144 : T <= 128 ? 16384 : 10240); }
 
+// Both of them against tiles whose rows are chosen for the call (whole_tiles below), where there is a plan for those.  us a launch, weights from
+// memory, few rows / tiles:
+//   passes    T 40: 2048 x 4096 9.8 / 11.7, 1024 x 8192 15.3 / 12.6, 3168 x 8192 17.4 / 17.4, 4096 x 8192 18.2 / 20.2, 2048 x 14336 24.3 / 18.6, 4096 x 14336 28.1 / 28.6
+//             T 32: 1024 x 8192 11.3 / 12.7, 2048 x 8192 12.1 / 14.1, 1024 x 14336 17.4 / 14.9, 2048 x 14336 17.9 / 18.2, 3168 x 14336 21.8 / 23.5
+//   clusters  T 64: 2048 x 2048 8.0 / 9.5, 2048 x 4096 11.1 / 12.1, 2048 x 8192 15.6 / 14.8, 1024 x 14336 21.0 / 15.7, 3072 x 1024 8.0 / 7.5, 3072 x 4096 13.1 / 13.3
+//             T 128: 2048 x 2048 9.1 / 9.6, 2048 x 512 6.8 / 6.4, 3072 x 2048 11.1 / 9.8      T 129 .. 256: 1024 x 2048 9.5 .. 11.2 / 9.6, 2048 x 8192 20.8 .. 24.3 / 16.7 .. 19.2
+inline bool tiles_ahead(int T, int N, int K) {
+  if (T <= 32) return T > 24 && K > 12288 && N <= 2112;
+  if (T <= 48) return K > 6144 && N < (K > 12288 ? 4096 : 3168);
+  return T > 128 || K > 6144 || N > 2112;
+}
+
 // Mamba-2 prompts (scan_chunk.cu): sequences cut into segments of 256 tokens, or one chain of 64-token chunks each.  Times in chunks
 // of a chain's CTA with a second one on its SM (13.4 us at 128 state rows; alone on its SM 0.83 of that).  A chain takes its longest
 // sequence, and where not all CTAs (heads, column blocks) run at once as many rounds of equal ones, or the sum of unequal ones and a part of the
@@ -90,6 +102,36 @@ inline bool single_step_pays(long long heads_times_sequences, int dim, int vdim,
   if (heads_times_sequences * ((vdim + 63) / 64) <= sms) return true;
   if (!delta) return dim <= 128 || vdim >= 32;
   return dim > 64 ? vdim >= 32 : dim > 32 || vdim <= 64;
+}
+
+// Whole tiles (gemm_grouped.cu): the rows of a tile of 256 rows of W, and the parts its K is cut into, for `rows` rows of X on `pairs` CTA pairs.
+// A 64-wide step of K takes a pair 0.036 + 0.00105 us a row of the tile, at least 0.16 (what a step costs besides its products), a tile
+// 1.2 us besides, the weights what they take from memory; the exchange between parts 3 + rows * (0.016 + 0.009 parts) us.  So the tiles are as
+// large as they can be with as few rows to work through as there are: rows of the tile times tiles of the busiest pair.  (All tiles had up to
+// 256 rows while a step took 0.3 us whatever they had.)  us a launch, weights from memory, tiles as large as can be / these; over N 1024 to 28672, K 2048 to
+// 14336 and 129 to 3000 rows 0.84 of the time, and within 2.5 % of the best of all tiles and parts in the mean:
+//   2048 x 2048   256 rows 16.2 / 10.5   1000 rows 17.0 / 12.1   3000 rows 27.0 / 22.0 (176)    2048 x 8192   512 31.8 / 23.6   3000 97.9 / 74.0
+//   4096 x 14336  256 rows 60.6 / 44.8   700 rows 77.1 / 63.2    2048 rows 190 / 178 (240)      6144 x 4096  1000 49.0 / 38.6   2048 83.7 / 78.4
+//   28672 x 4096  512 rows 123 / 109     1400 rows 271 / 259     8192 x 2048  700 rows 26.3 / 22.5, 1400 rows 35.9 / 37.3
+// split: whether K may be cut at all.  (Many rows never want the smallest tiles, which are not tried then.)
+inline void whole_tiles(int rows, int N, int K, int pairs, bool split, int* tile, int* parts) {
+  const int KB = (K + 63) / 64, slabs = (N + 255) / 256;
+  const double memory = 2.0 * N * K / 6.3e6;
+  double best = 0;
+  *tile = 0;
+  for (int n = (rows + 255) / 256, last = 0; n <= (rows + 31) / 32; ++n) {
+    const int t = ((rows + n - 1) / n + 15) & ~15;
+    if (t == last) continue;
+    if (rows > 1024 && t < 96) break;
+    last = t;
+    const long long tiles = static_cast<long long>(slabs) * ((rows + t - 1) / t);
+    const double step = fmax(0.16, 0.036 + 0.00105 * t);
+    for (int p = 1; p == 1 || (split && tiles * p <= pairs && p * 8 <= KB); ++p) {
+      const long long waves = (tiles * p + pairs - 1) / pairs;
+      const double us = fmax(waves * ((KB + p - 1) / p * step + 1.2), memory) + (p > 1 ? 3.0 + t * (0.016 + 0.009 * p) : 0.0);
+      if (!*tile || us < best - 1e-9) { best = us; *tile = t; *parts = p; }
+    }
+  }
 }
 
 // Latent rows (latent_attention.cu): in registers between their sum and their norm, or read again.  Registers for 1024 numbers a CTA cost room on

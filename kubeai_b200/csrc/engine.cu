@@ -376,9 +376,8 @@ struct Engine {
   void admit_prefix(Seq& s);
   const CUtensorMap& xmap(const XMaps& xm, int bn) const { return xm.m[gemm_block_n_index(bn)]; }
   int gemm(const GemmPlan& p, const XMaps& xm, void* out, int ldo, int T) {
-    const int bn = gemm_block_n_for(T);
     ++stats.kernel_launches;
-    return gemm_run(p, xmap(xm, bn), bn, out, ldo, T, stream);
+    return gemm_run(p, xm.m, out, ldo, T, stream);
   }
   // GEMM that leaves its stream-K segments as fp32 partials for the next kernel to sum (partials.cuh)
   int gemm_def(const GemmPlan& p, const XMaps& xm, void* out, int ldo, int T, PartialView* pv) {
@@ -886,10 +885,9 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
     launched(1);
     pv = no_partials();
     if (wh) {
-      const int bn = gemm_block_n_for(T);
       const GroupedOut g = {act, I, GROUPED_SILU};
       ++stats.kernel_launches;
-      P(B200_K_GEMM_GU); if (on(B200_K_GEMM_GU)) rc |= gemm_whole_run(ly.p_gu, xmap(xm_normed, bn), bn, T, g, stream); Q();
+      P(B200_K_GEMM_GU); if (on(B200_K_GEMM_GU)) rc |= gemm_whole_run(ly.p_gu, xm_normed.m, T, g, stream); Q();
     } else if (const int bn = f2_bn(ly.p_gu)) {
       Gemm2Epi g;
       memset(&g, 0, sizeof(g));
@@ -990,6 +988,11 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     a.ldy = ldy;
     return a;
   };
+  // More tokens, up to 128: whole tiles whose rows are chosen for the step (gemm_grouped.cu) with a norm or the rotation behind them; what
+  // they cost is the weights and a launch each, where gemm3's exchange and its wait for all other clusters cost as much again.  A step of 4 layers,
+  // gemm3 / so, us: Llama-3-8B sizes 9 tokens 401 / 391, 48 479 / 474, 49 506 / 487, 96 539 / 524, 128 579 / 537; 2048 wide 33 tokens 266 / 251, 128
+  // 330 / 299; 1024 wide 49 to 64 tokens 204 / 209 (kept on gemm3), 128 223 / 206.  The rotation of qkv apart pays from 65 tokens on.
+  const bool tiles = few && whole_ok && (H >= 2048 || T <= 48 || T > 64);
   bool x_pending = false;   // `x` holds a projection's output that the next RMSNorm still has to add to the residual
   for (int l = 0; l < L && !rc; ++l) {
     Layer& ly = layers[l];
@@ -1007,6 +1010,11 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     P(B200_K_GEMM_QKV);
     if (few && linear_few(qa, &pairs)) {
       if (on(B200_K_GEMM_QKV)) rc |= linear_stream(qa, &pairs, stream);
+    } else if (tiles && T > 64) {
+      if (on(B200_K_GEMM_QKV)) rc |= gemm_run(ly.p_qkv, xm_normed.m, qkv, QKV, T, stream);
+      Q();
+      P(B200_K_ROPE); if (on(B200_K_ROPE)) rc |= rope_kv_write(qkv, pos, slots, cos_sin, kv_l, T, Hq, Hkv, cfg.max_model_len, stream);
+      ++stats.kernel_launches;
     } else {
       Gemm3Params p = base(ly.p_qkv, xmap(xm_normed, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_ROPE_KV);
       p.out = qkv; p.ldo = QKV;
@@ -1021,6 +1029,10 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
       P(B200_K_GEMM_O); if (on(B200_K_GEMM_O)) rc |= linear_stream(oa, nullptr, stream); Q();
       P(B200_K_NORM); if (on(B200_K_NORM)) rc |= rmsnorm(x, res, ly.norm2, normed, nullptr, T, H, cfg.rms_eps, stream); Q();
       ++stats.kernel_launches;
+    } else if (tiles) {
+      P(B200_K_GEMM_O); if (on(B200_K_GEMM_O)) rc |= gemm_run(ly.p_o, xm_attn.m, x, H, T, stream); Q();
+      P(B200_K_NORM); if (on(B200_K_NORM)) rc |= rmsnorm(x, res, ly.norm2, normed, nullptr, T, H, cfg.rms_eps, stream); Q();
+      ++stats.kernel_launches;
     } else {
       Gemm3Params p = base(ly.p_o, xmap(xm_attn, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_RESADD);
       p.out = res; p.ldo = H; p.ssq_out = ssq;
@@ -1033,6 +1045,9 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     P(B200_K_GEMM_GU);
     if (few && linear_few(ga, &unit)) {
       if (on(B200_K_GEMM_GU)) rc |= linear_stream(ga, &unit, stream);
+    } else if (tiles) {
+      const GroupedOut g = {act, I, GROUPED_SILU};
+      if (on(B200_K_GEMM_GU)) rc |= gemm_whole_run(ly.p_gu, xm_normed.m, T, g, stream);
     } else {
       Gemm3Params p = base(ly.p_gu, xmap(xm_normed, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_SILU);
       p.out = act; p.ldo = I;
@@ -1043,6 +1058,9 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     P(B200_K_GEMM_DOWN);
     if (few && linear_few(da)) {
       if (on(B200_K_GEMM_DOWN)) rc |= linear_stream(da, nullptr, stream);
+      x_pending = true;
+    } else if (tiles) {
+      if (on(B200_K_GEMM_DOWN)) rc |= gemm_run(ly.p_down, xm_act.m, x, H, T, stream);
       x_pending = true;
     } else {
       Gemm3Params p = base(ly.p_down, xmap(xm_act, 128), T, GEMM3_PRO_NONE, GEMM3_EPI_RESADD);

@@ -37,6 +37,8 @@ size_t gemm_workspace_bytes(int max_ctas);
 int gemm_plan_init(GemmPlan* p, const void* W, int N, int K, int ldw, float* ws, int* counters, int max_ctas);
 // Activation map over X row-major [rows, K] (rows = buffer capacity), for a given token-tile size.
 int gemm_make_x_map(CUtensorMap* tm, const void* X, int rows, int K, int ldx, int block_n);
+// ... for all of them, tm[kGemmNumBlockN]
+int gemm_make_x_maps(CUtensorMap* tm, const void* X, int rows, int K, int ldx);
 // Generic 2-D bf16 tensor map (used by the attention kernel for the paged KV cache).
 int tmap_encode_bf16_2d(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, int box_rows,
                         int box_cols, int swizzle128);
@@ -51,7 +53,7 @@ int gemm2_block_n_for(int T);
 int gemm2_block_n_for_plan(const GemmPlan& p, int T);   // 384-token tiles where they give one whole tile per pair
 int gemm2_x_box_rows(int block_n);
 void gemm2_set_trace(long long* dev_ptr);  // debug: 8 clock64 stamps per CTA, or nullptr
-int gemm2_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, void* out, int ldo, int T, cudaStream_t st);
+int gemm2_run(const GemmPlan& p, const CUtensorMap* x_maps, void* out, int ldo, int T, cudaStream_t st);
 int gemm2_units_for(const GemmPlan& p, int ntt);
 void gemm2_schedule_query(int N, int K, int T, int sms, int* out8);   // host-only: see gemm2_tcgen05.cu
 void gemm2_read_env();   // (re)read the pair kernel's A/B knobs; called when an engine is created
@@ -95,9 +97,9 @@ struct GroupedOut {
 int gemm_grouped_plan(GroupedPlan* p, const void* W, int experts, int N, int K);
 int gemm_grouped_x_maps(GroupedX* x, const void* X, int rows, int K);
 int gemm_grouped_run(const GroupedPlan& p, const GroupedX& x, int most_rows, const int* expert_rows, const GroupedOut& o, int sms, int* error, cudaStream_t st);
-// The same kernel on one matrix and `rows` rows, in whole tiles of 256 weight rows x up to 256 rows; few tiles are cut along K.
-// tm_x: the activation's map for token-tile size block_n, which is gemm_block_n_for(rows) or anything from 256 up.
-int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int rows, const GroupedOut& o, cudaStream_t st);
+// The same kernel on one matrix and `rows` rows, in whole tiles of 256 weight rows x up to 256 rows; few tiles are cut along K
+// (rules::whole_tiles).  x_maps: the activation's maps for all token-tile sizes, kGemmNumBlockN of them.
+int gemm_whole_run(const GemmPlan& p, const CUtensorMap* x_maps, int rows, const GroupedOut& o, cudaStream_t st);
 // whether a bf16 output of the plan's product can leave through it: N and ldo multiples of 8, out on a 16-byte boundary
 bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo);
 // ... with the choices made by the caller: box (16, 32, 64 or 128) is tm_x's, tile its rows per tile (a multiple of 16, at most
@@ -105,11 +107,9 @@ bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo);
 int gemm_whole_run_as(const GemmPlan& p, const CUtensorMap& tm_x, int box, int tile, int parts, int rows, const GroupedOut& o, int* error, cudaStream_t st);
 // ... without a plan: the maps are made for the call (K, ldw, ldx multiples of 8, W and X on 16-byte boundaries, K whole).
 int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, int* error, cudaStream_t st);
-int gemm_whole_parts(int N, int K, int tile, int tiles, int units);
 // Generic consumer: out[t, n] = bf16(sum of segments) — used by tests and by paths without a fused consumer.
 int reduce_partials(const PartialView& v, void* out, int ldo, int T, int N, cudaStream_t st);
-// out[t, n] (bf16, leading dimension ldo) for t < T.
-int gemm_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, void* out, int ldo, int T,
-             cudaStream_t st);
+// out[t, n] (bf16, leading dimension ldo) for t < T; x_maps: the activation's maps for all token-tile sizes.
+int gemm_run(const GemmPlan& p, const CUtensorMap* x_maps, void* out, int ldo, int T, cudaStream_t st);
 
 }  // namespace b200

@@ -968,28 +968,17 @@ int gemm2_block_n_for_plan(const GemmPlan& p, int T) {
 }
 int gemm2_x_box_rows(int block_n) { return (block_n > 256 ? 256 : block_n) / 2; }
 
-int gemm2_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, void* out, int ldo, int T, cudaStream_t st) {
+int gemm2_run(const GemmPlan& p, const CUtensorMap* x_maps, void* out, int ldo, int T, cudaStream_t st) {
   if (T <= 0) return 0;
   // Whole tiles, or tiles cut along K with the last part finishing (gemm_grouped.cu), beat the stream-K form with its in-kernel
-  // fix-up (2048 x 2048, 512 tokens: 17 against 32 us; 8192 x 2048, 512 tokens: 20 against 102 us; 4096 x 14336, 2048 tokens:
-  // 194 against 447 us).  Left here: shapes whose rows are no whole 16-byte pieces, and long K where this kernel gives every
-  // pair one 512-token tile while 256-token tiles take two waves (4096 x 4096, 2048 tokens: 49.5 against 53.6 us; with K of
-  // 2048 the smaller tiles are the faster ones again, 4096 x 2048, 2048 tokens: 28.9 against 30.4).
-  const int slabs = (p.N + 2 * kSlab - 1) / (2 * kSlab);
-  const bool one_each = block_n == 512 && p.K > 2048 && slabs * ((T + 255) / 256) > p.max_ctas / 2 &&
-                        units_for(p, (T + 511) / 512) == slabs * ((T + 511) / 512);
-  // ... and few weight tiles with a long K and 64 to 256 tokens: cut into at most KB / 8 parts they leave most pairs idle, and a
-  // part's exchange grows with its tokens, while this kernel spreads their k-steps over all pairs (K 4096, 128 tokens, N 256 to
-  // 1024: 14.6 to 16.0 against 18.1 to 18.6 us; N 512, K 14336, 256 tokens: 27.1 against 38.2; the line: N 1536, K 3072, 128
-  // tokens 15.7 against 16.8, N 1536, K 4096 even; 320 tokens 28.5 against 32.3, 384 39.9 against 32.4; K 2048, N 1024, 128 tokens
-  // 13.6 against 14.3, 144 15.6 against 14.7).
-  const int KB = (p.K + kBlockK - 1) / kBlockK;
-  const bool few = slabs <= 2 ? (KB >= 48 && T > 63 && T <= 256) || (KB >= 128 && T > 256 && T <= 320) || (KB >= 32 && T > 96 && T <= 128)
-                              : (KB >= 48 && slabs * KB <= 300 && T > 64 && T <= 256) || (KB >= 32 && slabs <= 4 && slabs * KB <= 300 && T > 96 && T <= 128);
-  if (gemm_whole_fits(p, out, ldo) && !one_each && !few) {
+  // fix-up: 8192 x 2048, 512 tokens: 20 against 102 us; 4096 x 14336, 2048 tokens 178 against 447; 3072 x 4096, 2048 tokens (one
+  // 512-token tile a pair here) 37 against 47; 512 x 4096, 128 tokens 11.3 against 16.  Left here: rows that are no whole 16-byte pieces.
+  if (gemm_whole_fits(p, out, ldo)) {
     const GroupedOut o = {out, ldo};
-    return gemm_whole_run(p, tm_x, block_n, T, o, st);
+    return gemm_whole_run(p, x_maps, T, o, st);
   }
+  const int block_n = gemm2_block_n_for(T);
+  const CUtensorMap& tm_x = x_maps[gemm_block_n_index(block_n)];
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   switch (block_n) {
     case 32: return launch2<32>(p, tm_x, o, ldo, T, st);

@@ -24,6 +24,7 @@
 #include <atomic>
 
 #include "activations.cuh"
+#include "dispatch_rules.h"
 #include "gemm.h"
 #include "launch.h"
 #include "ptx.cuh"
@@ -523,7 +524,7 @@ int launch(const CUtensorMap& tm_w, int experts, int N, int K, const CUtensorMap
 int gemm_grouped_run(const GroupedPlan& p, const GroupedX& x, int most_rows, const int* expert_rows, const GroupedOut& o, int sms, int* error, cudaStream_t st) {
   if (!expert_rows) return -1;
   int i = 0;
-  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < most_rows) ++i;
+  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < most_rows) ++i;      // (smaller tiles for experts of many rows: 107 -> 114 us at up to 128 of 512 rows)
   return launch(p.tm_w, p.experts, p.N, p.K, x.box[i], kBoxes[i], expert_rows, 0, o, {nullptr, nullptr, 1, 2 * kBoxes[i]}, sms / 2, error, st);
 }
 
@@ -536,37 +537,21 @@ int gemm_whole_run_as(const GemmPlan& p, const CUtensorMap& tm_x, int box, int t
   return launch(p.tm_w, 1, p.N, p.K, tm_x, box, nullptr, rows, o, {p.ws, p.counters, parts, tile}, units, error, st);
 }
 
-// The parts K is cut into.  A pair takes in a 64-wide step of K in 0.28 us whatever the tile (what an SM draws through TMA), so
-// a launch of few tiles is as long as its K; cutting it puts more pairs to work, down to the time the weights take from
-// memory, and costs the exchange, about 1 us + rows of the tile * (0.03 + 0.005 parts) us.  Measured, one part against the
-// rule's (N, K, tokens): 4096, 14336, 16: 72.7 against 33.8 us; 257: 74.8, 50.9; 512: 76.8, 57.0; 2048, 8192, 16: 45.4, 19.4;
-// 512: 46.1, 34.5; 4096, 4096, 64: 27.6, 20.8; 512: 29.7, 29.7; 2048, 2048, 16: 17.4, 13.3 (launch included).
-int gemm_whole_parts(int N, int K, int tile, int tiles, int units) {
-  const int KB = (K + kBlockK - 1) / kBlockK;
-  const double memory = 2.0 * N * K / 5.5e6;
-  int best = 1;
-  double least = 0;
-  for (int parts = 1; parts == 1 || (tiles * parts <= units && parts * 8 <= KB); ++parts) {
-    const double us = std::max((KB + parts - 1) / parts * 0.28, tiles < units ? memory : 0.0) + (parts > 1 ? 1.0 + tile * (0.03 + 0.005 * parts) : 0.0);
-    if (parts == 1 || us < least) { least = us; best = parts; }
-  }
-  return best;
-}
-
-int gemm_whole_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, int rows, const GroupedOut& o, cudaStream_t st) {
+int gemm_whole_run(const GemmPlan& p, const CUtensorMap* x_maps, int rows, const GroupedOut& o, cudaStream_t st) {
   if (rows < 1) return 0;
-  const int box = gemm2_x_box_rows(block_n), ntt = (rows + 2 * box - 1) / (2 * box), tile = ((rows + ntt - 1) / ntt + 15) & ~15;
-  const int tiles = (p.N + 2 * kSlab - 1) / (2 * kSlab) * ((rows + tile - 1) / tile);
-  // (fp32 outputs have no split form)
-  return gemm_whole_run_as(p, tm_x, box, tile, o.epi == GROUPED_F32 ? 1 : gemm_whole_parts(p.N, p.K, tile, tiles, p.max_ctas / 2), rows, o, p.error, st);
+  int tile, parts, i = 0;      // (fp32 outputs have no split form)
+  rules::whole_tiles(rows, p.N, p.K, p.max_ctas / 2, o.epi != GROUPED_F32, &tile, &parts);
+  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < tile) ++i;      // the maps of the four smallest token-tile sizes have these boxes
+  return gemm_whole_run_as(p, x_maps[i], kBoxes[i], tile, parts, rows, o, p.error, st);
 }
 
 int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, int* error, cudaStream_t st) {
   CUtensorMap tm_w, tm_x;
-  int dev = 0, sms = 0, i = 0;
+  int dev = 0, sms = 0, i = 0, tile, parts;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
-  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < rows) ++i;
-  const int box = kBoxes[i], ntt = (rows + 2 * box - 1) / (2 * box), tile = ((rows + ntt - 1) / ntt + 15) & ~15;
+  rules::whole_tiles(rows, N, K, sms / 2, false, &tile, &parts);
+  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < tile) ++i;
+  const int box = kBoxes[i];
   if (tmap_encode_bf16_2d(&tm_w, W, N, K, ldw, kSlab, kBlockK, 1) || tmap_encode_bf16_2d(&tm_x, X, rows, K, ldx, box, kBlockK, 1)) return -2;
   const long long tiles = static_cast<long long>((N + 2 * kSlab - 1) / (2 * kSlab)) * ((rows + tile - 1) / tile);
   return launch(tm_w, 1, N, K, tm_x, box, nullptr, rows, o, {nullptr, nullptr, 1, tile}, static_cast<int>(std::min<long long>(sms / 2, tiles)), error, st);

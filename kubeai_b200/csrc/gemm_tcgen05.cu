@@ -512,10 +512,18 @@ int gemm_make_x_map(CUtensorMap* tm, const void* X, int rows, int K, int ldx, in
   return make_tmap(tm, X, rows, K, ldx, gemm_x_box_rows(block_n));
 }
 
-int gemm_run(const GemmPlan& p, const CUtensorMap& tm_x, int block_n, void* out, int ldo, int T,
-             cudaStream_t st) {
+int gemm_make_x_maps(CUtensorMap* tm, const void* X, int rows, int K, int ldx) {
+  constexpr int sizes[kGemmNumBlockN] = {32, 64, 128, 256, 512};
+  for (int i = 0; i < kGemmNumBlockN; ++i)
+    if (const int rc = gemm_make_x_map(tm + i, X, rows, K, ldx, sizes[i])) return rc;
+  return 0;
+}
+
+int gemm_run(const GemmPlan& p, const CUtensorMap* x_maps, void* out, int ldo, int T, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (g_variant == 2) return gemm2_run(p, tm_x, block_n, out, ldo, T, st);
+  if (g_variant == 2) return gemm2_run(p, x_maps, out, ldo, T, st);
+  const int block_n = gemm_block_n_for(T);
+  const CUtensorMap& tm_x = x_maps[gemm_block_n_index(block_n)];
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   switch (block_n) {
     case 32: return launch<32>(p, tm_x, o, ldo, T, st);

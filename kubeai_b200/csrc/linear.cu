@@ -496,6 +496,8 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
 }  // namespace
 
 bool linear_few(const LinearArgs& a, const LinearPairs* q) {
+  // (tiles: rows in whole 16-byte pieces, bf16 out)
+  if (!q && a.ty == DT_BF16 && a.N % 8 == 0 && a.ldy % 8 == 0 && reinterpret_cast<uintptr_t>(a.Y) % 16 == 0 && rules::tiles_ahead(a.T, a.N, a.K)) return false;
   if (linear_streams(a, q)) return rules::stream_pays(a.T, a.N, a.K, q != nullptr);
   return !q && linear_clusters(a) && rules::cluster_pays(a.T, a.N, a.K);
 }

@@ -598,13 +598,11 @@ class Mulenex : public Model {
               const float* bias = nullptr, int act = LIN_NONE) {
     LinearArgs a = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
     if (tc && !linear_few(a)) {
-      const int bn = gemm_block_n_for(T);
-      const CUtensorMap& tm = xm[gemm_block_n_index(bn)];
       if ((bias || act != LIN_NONE) && gemm_whole_fits(plan, Y, N)) {
         const GroupedOut o = {Y, N, act == LIN_RELU2 ? GROUPED_RELU2 : GROUPED_PLAIN, bias};
-        return gemm_whole_run(plan, tm, bn, T, o, env.stream);
+        return gemm_whole_run(plan, xm, T, o, env.stream);
       }
-      int rc = gemm_run(plan, tm, bn, Y, N, T, env.stream);
+      int rc = gemm_run(plan, xm, Y, N, T, env.stream);
       if (!rc && (bias || act != LIN_NONE)) rc = bias_act(Y, N, bias, act, dt, T, N, env.stream);
       return rc;
     }
@@ -728,8 +726,7 @@ class Mulenex : public Model {
         KRN("shared_in", linear_stream(sg, &unit, st));
       } else if (w.il_s && w.tc_shin && gemm_whole_fits(w.p_shin, shact, s.sff)) {
         const GroupedOut o = {shact, s.sff, GROUPED_GATED, nullptr, INFINITY, 1.f, 0.f};     // the gated unit in the epilogue
-        const int bn = gemm_block_n_for(T);
-        KRN("shared_in", gemm_whole_run(w.p_shin, xm_h[gemm_block_n_index(bn)], bn, T, o, st));
+        KRN("shared_in", gemm_whole_run(w.p_shin, xm_h, T, o, st));
       } else {
         KRN("shared_in", project(w.p_shin, w.tc_shin, xm_h, h, w.sh_in, sh, T, s.n_sh, W));
         KRN("glu", glu_clamped(sh, s.n_sh, shact, s.sff, dt, T, s.sff, INFINITY, 1.f, st, 0.f, w.il_s));

@@ -656,8 +656,7 @@ class Nagilix : public Model {
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K) {
     const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
     if (tc && !linear_few(la)) {
-      const int bn = gemm_block_n_for(T);
-      return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
+      return gemm_run(plan, xm, Y, N, T, env.stream);
     }
     return linear(la, env.stream);
   }

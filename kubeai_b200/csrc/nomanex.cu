@@ -598,8 +598,7 @@ class Nomanex : public Model {
     static const int tc_min_t = [] { const char* e = getenv("B200_NX_TC_MIN_T"); return e ? atoi(e) : 1; }();   // A/B knob
     const LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
     if (tc && T >= tc_min_t && !linear_few(la)) {
-      const int bn = gemm_block_n_for(T);
-      return gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
+      return gemm_run(plan, xm, Y, N, T, env.stream);
     }
     return linear(la, env.stream);
   }
@@ -666,7 +665,7 @@ class Nomanex : public Model {
         const bool fresh = b.fresh && w.tc_ukv && latent_prompt_pays(T, b.nseq);
         // whole prompts: per-head keys and values once per token, in the buffers of the latent form
         bf16 *c = reinterpret_cast<bf16*>(qlat), *k2 = c + static_cast<size_t>(env.Tcap) * C, *q2 = k2 + static_cast<size_t>(env.Tcap) * R, *v2 = q2 + static_cast<size_t>(env.Tcap) * s.heads * R;
-        const int N = s.heads * (s.dim + s.vdim), bn = gemm_block_n_for(T);
+        const int N = s.heads * (s.dim + s.vdim);
         GroupedOut kv = {olat, N, GROUPED_TWO_TERMS};
         kv.y2 = v2;
         PromptAttnArgs pa = {};
@@ -678,7 +677,7 @@ class Nomanex : public Model {
           p.q = nullptr;
           KRN("latent_prep", latent_prep(p, st));
           KRN("latent_prompt_prep", latent_prompt_prep(pp, st));
-          KRN("latent_kv", gemm_whole_run(w.p_ukv, w.xm_c[gemm_block_n_index(bn)], bn, T, kv, st));
+          KRN("latent_kv", gemm_whole_run(w.p_ukv, w.xm_c, T, kv, st));
           KRN("latent_attention", prompt_attention(pa, st));
         } else {
           KRN("latent_prep", latent_prep(p, st));

@@ -588,12 +588,11 @@ class Soselix : public Model {
   int project(const GemmPlan& plan, bool tc, const CUtensorMap* xm, const void* X, const void* Wm, void* Y, int T, int N, int K, const Epilogue* ep = nullptr) {
     LinearArgs la = linear_args(X, dt, Wm, dt, Y, dt, T, N, K, env.kernel_error);
     if (tc && T > few_rows && !linear_few(la)) {
-      const int bn = gemm_block_n_for(T);
       if (ep && fuse && gemm_whole_fits(plan, Y, N)) {
         const GroupedOut o = {Y, N, GROUPED_XIELU, ep->bias, ep->a_pos, ep->a_neg};
-        return gemm_whole_run(plan, xm[gemm_block_n_index(bn)], bn, T, o, env.stream);
+        return gemm_whole_run(plan, xm, T, o, env.stream);
       }
-      const int rc = gemm_run(plan, xm[gemm_block_n_index(bn)], bn, Y, N, T, env.stream);
+      const int rc = gemm_run(plan, xm, Y, N, T, env.stream);
       return rc || !ep ? rc : bias_act(Y, N, ep->bias, LIN_XIELU, dt, T, N, env.stream, ep->a_pos, ep->a_neg);
     }
     if (ep) { la.bias = ep->bias; la.act = LIN_XIELU; la.a_pos = ep->a_pos; la.a_neg = ep->a_neg; }
@@ -652,7 +651,7 @@ class Soselix : public Model {
       // whole prompts: per-head keys and values once per token, in the buffers of the latent form
       bf16 *c = reinterpret_cast<bf16*>(qlat), *k2 = c + static_cast<size_t>(env.Tcap) * C, *q2 = k2 + static_cast<size_t>(env.Tcap) * R, *v2 = q2 + static_cast<size_t>(env.Tcap) * s.heads * R;
       LatentPromptPrepArgs pp = {r.cache, b.slots, b.pos, w.rope, s.rot_dims, true, qb, Q, c, k2, q2, T, s.heads, s.dim, R, C};
-      const int N = s.heads * (s.dim + s.vdim), bn = gemm_block_n_for(T);
+      const int N = s.heads * (s.dim + s.vdim);
       GroupedOut kv = {olat, N, GROUPED_TWO_TERMS};
       kv.y2 = v2;
       PromptAttnArgs pa = {};
@@ -661,7 +660,7 @@ class Soselix : public Model {
       pa.sink = w.sink; pa.gate = col(inb, s.off_g); pa.ldg = s.n_in; pa.seqs = b.seqs; pa.nseq = b.nseq; pa.error = env.kernel_error;
       if (prompt_attention_fits(pa) && gemm_whole_fits(w.p_ukv, olat, N)) {
         KRN("latent_prompt_prep", latent_prompt_prep(pp, st));
-        KRN("latent_kv", gemm_whole_run(w.p_ukv, w.xm_c[gemm_block_n_index(bn)], bn, T, kv, st));
+        KRN("latent_kv", gemm_whole_run(w.p_ukv, w.xm_c, T, kv, st));
         KRN("latent_attention", prompt_attention(pa, st));
         return rc;
       }

@@ -98,3 +98,33 @@ def test_single_tokens_pass_over_states_that_fill_the_pass(units, dim, vdim, del
 def test_latent_rows_stay_in_registers_where_there_is_room(rank, tokens, held):
     """A kernel with room for 1024 numbers in registers whatever the row: 4096 tokens of 2048 in two layers 73 us against 60."""
     assert rule(LATENT_ROWS, rank, tokens) == held
+
+
+TILES, TILE_ROWS, TILE_PARTS = 9, 10, 11
+
+
+@pytest.mark.parametrize("T,N,K,ahead", [(24, 1024, 14336, 0), (28, 1024, 14336, 1), (32, 3168, 14336, 0), (32, 2048, 8192, 0), (40, 2048, 4096, 0), (40, 1024, 8192, 1), (48, 3072, 8192, 1), (40, 4096, 8192, 0),
+                                         (40, 2048, 14336, 1), (48, 4096, 14336, 0), (64, 2048, 2048, 0), (128, 2048, 4096, 0), (64, 2048, 8192, 1), (64, 3072, 1024, 1), (129, 1024, 2048, 1), (256, 2048, 2048, 1)])
+def test_tiles_chosen_for_the_call_against_the_products_of_few_rows(T, N, K, ahead):
+    """40 rows of 1024 x 14336 take 24 us as a pass over the weights, 20 in clusters and 15 in tiles; 64 of 2048 x 2048 8.0 in clusters and 9.5 in tiles."""
+    assert rule(TILES, T, N, K) == ahead
+
+
+@pytest.mark.parametrize("rows,N,K,tile,parts", [(1999, 4096, 14336, 224, 1), (2048, 4096, 14336, 240, 1), (3001, 2048, 2048, 176, 1), (4096, 2048, 8192, 240, 1), (256, 4096, 14336, 128, 2),
+                                                 (128, 4096, 4096, 64, 1), (64, 512, 4096, 32, 6), (300, 28672, 4096, 160, 1), (1, 256, 64, 16, 1)])
+def test_rows_of_a_tile_and_pieces_of_k(rows, N, K, tile, parts):
+    """2048 rows of 4096 x 14336 in tiles of 256 rows are two rounds of 74 pairs with 20 of them idle: 190 us, 178 in tiles of 240."""
+    assert (rule(TILE_ROWS, rows, N, K, 74, 1), rule(TILE_PARTS, rows, N, K, 74, 1)) == (tile, parts)
+
+
+def test_every_choice_of_tiles_can_be_launched():
+    """Whole steps of 16 rows, at most 256, and a part of K for every pair at most once."""
+    for rows in (1, 15, 16, 17, 31, 33, 100, 128, 129, 255, 256, 257, 500, 511, 1000, 1025, 2049, 4096):
+        for N in (8, 256, 520, 2048, 6144, 28672):
+            for K in (8, 64, 520, 4096, 14336):
+                for pairs in (1, 66, 74):
+                    t, p = rule(TILE_ROWS, rows, N, K, pairs, 1), rule(TILE_PARTS, rows, N, K, pairs, 1)
+                    tiles = -(-N // 256) * -(-rows // t)
+                    assert 16 <= t <= 256 and t % 16 == 0 and p >= 1 and p <= -(-K // 64)
+                    assert p == 1 or tiles * p <= pairs
+                    assert rule(TILE_PARTS, rows, N, K, pairs, 0) == 1

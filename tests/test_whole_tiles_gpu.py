@@ -127,3 +127,22 @@ def test_split_products_with_an_epilogue(tmp_path, monkeypatch, T):
         # the fused form rounds once less per product; otherwise the same roundings
         assert np.median(out[0]) < 0.03 and np.median(out[0]) < 1.1 * np.median(out[1]) + 2.0 ** -11, (name, np.median(out[0]), np.median(out[1]))
         assert out[0].max() < 3 * out[1].max() + 2.0 ** -8, (name, out[0].max(), out[1].max())
+
+
+@pytest.mark.parametrize("T", [9, 16, 17, 33, 64, 65, 96, 112, 113])
+@pytest.mark.parametrize("I,K", [(128, 64), (1024, 512), (3584, 1024), (14336, 4096)])
+def test_gate_and_up_of_a_step(T, I, K):
+    """Both sides of the lines between the passes over the weights, whole tiles and the kernel of a decode step's pairs."""
+    from kubeai_b200 import ops
+    x, w = operands(T, 2 * I, K, seed=4)
+    got, again = ops.gemm3(x, w, epi=ops.EPI_SILU)[0], ops.gemm3(x, w, epi=ops.EPI_SILU)[0]
+    assert torch.equal(got, again)
+    gu = x.double() @ w.double().T
+    mag = (K + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    (g, u), (dg, du) = ((t.reshape(T, I // 64, 2, 64).transpose(1, 2).reshape(T, 2, I).unbind(1)) for t in (gu, 2.0 ** -8 * gu.abs() + mag))
+    s = g * torch.sigmoid(g)
+    # g and u rounded to bf16, silu(g) (its slope is at most 1.1) rounded again, the product rounded again
+    ds = 1.1 * dg + 2.0 ** -8 * (s.abs() + 1.1 * dg)
+    bound = ds * (u.abs() + du) + s.abs() * du
+    bound = bound + 2.0 ** -8 * ((s * u).abs() + bound)
+    assert ((got.double() - s * u).abs() <= 1.01 * bound + 1e-30).all()

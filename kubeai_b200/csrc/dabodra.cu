@@ -792,8 +792,8 @@ class Dabodra : public Model {
       const int n = std::min(row_cap, b.S - r0);
       KRN("residual_norm", sandwich_step(boundary(Pending(), fin_w, hrow, b.rows + r0, n), st));
       KRN("head", linear(linear_args(hrow, dt, head, dt, logits, DT_F32, n, V, W, env.kernel_error), st));
-      KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st));
-      if (host_logits && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
+      KRN("argmax", argmax_f32(logits, sampled + r0, n, V, st, host_logits && b.host_mapped ? host_logits + static_cast<size_t>(r0) * V : nullptr));
+      if (host_logits && !b.host_mapped && cudaMemcpyAsync(host_logits + static_cast<size_t>(r0) * V, logits, static_cast<size_t>(n) * V * sizeof(float),
                                          cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = -2;
     }
     if (launches) *launches += nl;

@@ -319,8 +319,9 @@ __global__ void silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloa
 }
 
 // ------------------------------------------------------------------ greedy argmax over bf16 logits
-__global__ void argmax_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict__ out, int V, int ld,
-                              PartialView pv) {
+// mirror (optional, V % 8 == 0, whole logits): pinned host memory that gets the rows [S][V] too
+__global__ void __launch_bounds__(1024) argmax_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict__ out, int V, int ld,
+                              PartialView pv, uint4* mirror) {
   griddep_enter();
   const int s = blockIdx.x;
   const __nv_bfloat16* row = logits + static_cast<size_t>(s) * ld;
@@ -335,6 +336,7 @@ __global__ void argmax_kernel(const __nv_bfloat16* __restrict__ logits, int* __r
     } else {
       Vec8 a;
       a.u = r4[i];
+      if (mirror) mirror[static_cast<size_t>(s) * nvec + i] = a.u;
 #pragma unroll
       for (int j = 0; j < 8; ++j) fa[j] = __bfloat162float(a.h[j]);
     }
@@ -485,10 +487,10 @@ int silu_mul(const void* gate_up, void* out, int T, int I, cudaStream_t st, Part
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int argmax_rows(const void* logits, int* out, int S, int V, int ld, cudaStream_t st, PartialView pv) {
+int argmax_rows(const void* logits, int* out, int S, int V, int ld, cudaStream_t st, PartialView pv, void* mirror) {
   if (S <= 0) return 0;
-  if (ld % 8 || (pv.ws && V % 8)) return -1;
-  launch_pdl(argmax_kernel, dim3(S), dim3(1024), 0, st, static_cast<const __nv_bfloat16*>(logits), out, V, ld, pv);
+  if (ld % 8 || (pv.ws && V % 8) || (mirror && (pv.ws || V % 8))) return -1;
+  launch_pdl(argmax_kernel, dim3(S), dim3(1024), 0, st, static_cast<const __nv_bfloat16*>(logits), out, V, ld, pv, static_cast<uint4*>(mirror));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

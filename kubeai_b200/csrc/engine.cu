@@ -235,13 +235,14 @@ struct Engine {
   // scheduling, pages, slots, packing and sampling
   std::unique_ptr<Model> model;
   std::vector<int> free_slots;
-  // Pinned staging of b200_feed_step's logits, two halves (engines that step by hand): the device's copies land here and the
-  // host converts or copies from it, one half while the other fills.  16 rows of 8192 logits from pageable memory and one by
+  // Pinned staging of b200_feed_step's logits (engines that step by hand).  What fits goes there by the last kernel's own stores; more
+  // bf16 logits come in two halves, the device's copies into one while the host converts from the other.  16 rows of 8192 logits from pageable memory and one by
   // one took 150 us of a step.
   static constexpr size_t kFeedHalf = 2u << 20;
   uint8_t* feed_stage = nullptr;
   cudaEvent_t feed_ev[2] = {nullptr, nullptr};
   uint64_t feed_calls = 0;
+  void* logits_mirror = nullptr;    // during a fed step: where the kernel that picks the best logits leaves them as well
   int init_feed();
   int check_kernels();
   int read_logits_f32(float* out, size_t count);
@@ -337,7 +338,7 @@ struct Engine {
   int init(const b200_config& c);
   int init_model(const b200_config& c, std::unique_ptr<Model> mdl);
   int alloc_step_ring();
-  int forward_model(const StepMeta& m, int32_t* dbuf, float* host_logits);
+  int forward_model(const StepMeta& m, int32_t* dbuf, float* host_logits, bool mapped = false);
   int pack(InFlight* f, const std::vector<std::vector<int>>* want, StepMeta* mp);
   int feed_step(const b200_feed_entry* entries, int n, float* logits_out, int64_t cap_floats);
   int alloc_all();
@@ -718,7 +719,7 @@ int Engine::init_model(const b200_config& c, std::unique_ptr<Model> mdl) {
   return 0;
 }
 
-int Engine::forward_model(const StepMeta& m, int32_t* dbuf, float* host_logits) {
+int Engine::forward_model(const StepMeta& m, int32_t* dbuf, float* host_logits, bool mapped) {
   StepBatch b;
   b.T = m.T; b.nseq = m.nseq; b.S = m.S;
   b.ids = dbuf + m.off_ids; b.prev_ids = dbuf + m.off_prev; b.pos = dbuf + m.off_pos; b.slots = dbuf + m.off_slots;
@@ -727,6 +728,7 @@ int Engine::forward_model(const StepMeta& m, int32_t* dbuf, float* host_logits) 
   b.max_ctx = m.max_ctx;
   b.max_rows = m.max_rows;
   b.fresh = m.kv_tokens == m.T;
+  b.host_mapped = mapped;
   last_S = m.S;
   if (int rc = model->forward(b, sampled, host_logits, &stats.kernel_launches)) return rc == -1 ? B200_ERR_INVALID : B200_ERR_CUDA;
   return 0;
@@ -927,7 +929,7 @@ int Engine::forward(const StepMeta& m, int32_t* dbuf, bool all_logits, bf16* log
     if (dfr && !keep_logits) rc |= gemm_def(p_lm, xm_last, logits, V, m.S, &pv); else rc |= gemm(p_lm, xm_last, logits, V, m.S);
     Q();
     last_S = m.S;
-    P(B200_K_ARGMAX); rc |= argmax_rows(logits, sampled, m.S, V, V, stream, pv); Q();
+    P(B200_K_ARGMAX); rc |= argmax_rows(logits, sampled, m.S, V, V, stream, pv, logits_mirror); Q();
     launched(2);
   }
   if (rc) return cuda_fail("forward(head)", -2);
@@ -1087,7 +1089,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     }
     Q();
     P(B200_K_ARGMAX);
-    if (stream_lm || keep_logits) rc |= argmax_rows(logits, sampled, m.S, V, V, stream);
+    if (stream_lm || keep_logits) rc |= argmax_rows(logits, sampled, m.S, V, V, stream, no_partials(), logits_mirror);
     else rc |= argmax_candidates(cand, sampled, m.S, V / 128, stream);
     Q();
     last_S = m.S;
@@ -1204,7 +1206,7 @@ int Engine::forward_chain(const StepMeta& m, int32_t* dbuf) {
     p.out = logits; p.ldo = V; p.cand = cand;
     P(B200_K_GEMM_LM); rc |= gemm3_launch(p, sch_lm, stream); Q();
     P(B200_K_ARGMAX);
-    if (keep_logits) rc |= argmax_rows(logits, sampled, m.S, V, V, stream);
+    if (keep_logits) rc |= argmax_rows(logits, sampled, m.S, V, V, stream, no_partials(), logits_mirror);
     else rc |= argmax_candidates(cand, sampled, m.S, V / 128, stream);
     Q();
     last_S = m.S;
@@ -1624,6 +1626,12 @@ void touch_pages(float* out, size_t count, cudaEvent_t ready) {
   }
 }
 
+void widen(float* out, const void* bf16s, size_t n) {
+  const uint16_t* in = static_cast<const uint16_t*>(bf16s);
+  uint32_t* o = reinterpret_cast<uint32_t*>(out);
+  for (size_t k = 0; k < n; ++k) o[k] = static_cast<uint32_t>(in[k]) << 16;
+}
+
 // the first `count` bf16 logits on the device -> fp32 (same values) at `out`
 int Engine::read_logits_f32(float* out, size_t count) {
   constexpr size_t part = kFeedHalf / 2;
@@ -1639,10 +1647,7 @@ int Engine::read_logits_f32(float* out, size_t count) {
       continue;
     }
     CK(cudaEventSynchronize(feed_ev[(i - 1) & 1]));
-    const uint16_t* in = reinterpret_cast<const uint16_t*>(feed_stage + ((i - 1) & 1) * kFeedHalf);
-    uint32_t* o = reinterpret_cast<uint32_t*>(out + (i - 1) * part);
-    const size_t n = len(i - 1);
-    for (size_t k = 0; k < n; ++k) o[k] = static_cast<uint32_t>(in[k]) << 16;
+    widen(out + (i - 1) * part, feed_stage + ((i - 1) & 1) * kFeedHalf, len(i - 1));
   }
   return 0;
 }
@@ -1703,21 +1708,25 @@ int Engine::feed_step(const b200_feed_entry* entries, int n, float* logits_out, 
     int32_t* dbuf = stage_dev[slot];
     CK(cudaMemcpyAsync(dbuf, stage_host, static_cast<size_t>(m.words) * 4, cudaMemcpyHostToDevice, stream));
     CK(cudaEventRecord(ev0, stream));
-    const bool staged = model && static_cast<size_t>(S) * V * sizeof(float) <= 2 * kFeedHalf;
-    if (model) rc = forward_model(m, dbuf, staged ? reinterpret_cast<float*>(feed_stage) : logits_out);
+    const size_t count = static_cast<size_t>(S) * V;
+    const bool staged = S > 0 && count * (model ? sizeof(float) : sizeof(bf16)) <= 2 * kFeedHalf && (model || V % 8 == 0);
+    if (model) rc = forward_model(m, dbuf, staged ? reinterpret_cast<float*>(feed_stage) : logits_out, staged);
     else {
       const bool keep = keep_logits;
       keep_logits = true;
+      logits_mirror = staged ? feed_stage : nullptr;
       rc = forward(m, dbuf, false, nullptr);
+      logits_mirror = nullptr;
       keep_logits = keep;
-      if (!rc && m.S) rc = read_logits_f32(logits_out, static_cast<size_t>(m.S) * V);
+      if (!rc && m.S && !staged) rc = read_logits_f32(logits_out, count);
     }
     if (!rc) {
       CK(cudaEventRecord(ev1, stream));
-      if (staged) touch_pages(logits_out, static_cast<size_t>(S) * V, ev1);
+      if (staged) touch_pages(logits_out, count, ev1);
       CK(cudaStreamSynchronize(stream));
       rc = check_kernels();
-      if (!rc && staged && S) memcpy(logits_out, feed_stage, static_cast<size_t>(S) * V * sizeof(float));
+      if (!rc && staged && model) memcpy(logits_out, feed_stage, count * sizeof(float));
+      if (!rc && staged && !model) widen(logits_out, feed_stage, count);
     }
   }
   if (rc) {

@@ -24,7 +24,7 @@ int rope_kv_write(void* qkv, const int* positions, const int* slots, const void*
 int silu_mul(const void* gate_up, void* out, int T, int I, cudaStream_t st, PartialView pv = no_partials(), int interleaved = 0);
 // gate_up weight rows: logical [gate | up] <-> physical (64 gate rows, their 64 up rows, ...); dst != src
 int permute_gate_up(void* dst, const void* src, int I, int H, int to_physical, cudaStream_t st);
-int argmax_rows(const void* logits, int* out, int S, int V, int ld, cudaStream_t st, PartialView pv = no_partials());
+int argmax_rows(const void* logits, int* out, int S, int V, int ld, cudaStream_t st, PartialView pv = no_partials(), void* mirror = nullptr);
 int init_uniform(void* p, size_t n, uint32_t seed, float scale, float offset, cudaStream_t st);
 
 // One unit of attention work: q_count query tokens of one sequence starting at row q_tok0 of the

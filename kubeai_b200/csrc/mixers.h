@@ -123,7 +123,7 @@ int bias_act(void* y, int ldy, const float* bias, int act, DType t, int T, int n
 int sigmoid_gate(void* y, int ldy, const void* g, int ldg, DType t, int T, int n, cudaStream_t st);
 // p[i] = offset + scale * u_i, u uniform in [-1, 1) from a counter hash of (seed, i): seeded random weights for benchmarks
 int fill_uniform(void* p, DType t, size_t n, uint64_t seed, float scale, float offset, cudaStream_t st);
-int argmax_f32(const float* logits, int* out, int S, int V, cudaStream_t st);
+int argmax_f32(const float* logits, int* out, int S, int V, cudaStream_t st, float* mirror = nullptr);   // mirror: pinned, gets the logits as well
 
 // ---------------------------------------------------------------- gated linear attention (gla.cu)
 // Per sequence and head: S <- diag(alpha_t) S + k_t v_t^T, o_t = S^T (q_t * q_scale), alpha = sigmoid(z + z_bias)^(inv_tau),

@@ -34,6 +34,7 @@ struct StepBatch {
   bool fresh = false;               // every sequence of the step starts at its first token
   int max_ctx = 0;                  // longest context in the step: max over sequences of first position + rows
   int max_rows = 0;                 // most rows of a sequence in the step
+  bool host_mapped = false;         // forward's host_logits is pinned memory, which a kernel may write
 };
 
 struct ModelEnv {

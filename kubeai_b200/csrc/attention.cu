@@ -47,8 +47,11 @@ constexpr int attn_smem_bytes() {
   return S * kStageBytes + 64 + 1024;  // stages + mbarriers + slack for the 1 KiB alignment the swizzle needs
 }
 
-template <bool DECODE, int S>  // S = tiles in flight per CTA
-__global__ void __launch_bounds__(128)
+// S = tiles in flight per CTA.  One where no sequence has more: then what bounds a step of many short sequences is how many CTAs an SM holds, and
+// four fit (three with two tiles; 128 sequences of up to 64 tokens, 8 heads: 12.3 us, 10.9 with one tile, its pages alone and one lane of a
+// whole warp issuing).
+template <bool DECODE, int S>
+__global__ void __launch_bounds__(128, S == 1 ? 4 : 1)
 paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16* __restrict__ q, int ldq,
                   __nv_bfloat16* __restrict__ out, int ldo, const int* __restrict__ block_tables, int max_blocks,
                   const AttnWork* __restrict__ work, int Hkv, float scale_log2, float* __restrict__ split_ws) {
@@ -63,7 +66,7 @@ paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16
   // work[] and block_tables were uploaded before the first kernel of the step: readable ahead of the dependency wait.
   const AttnWork wk = work[blockIdx.y];  // work items are sorted longest-first; heads are the fast grid dimension
   const int kvh = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = S == 1 ? warp_number() : tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tq = lane & 3;
 
   const int kv_end = wk.q_pos0 + wk.q_count;  // tokens [0, kv_end) are visible to the last query
@@ -86,18 +89,25 @@ paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16
   }
   __syncthreads();
 
-  // thread 0: gather tile `tile` into stage `stage` (pages past the sequence's last one repeat it; they are masked)
+  // gather tile `tile` into stage `stage`: thread 0 (pages past the sequence's last one repeat it; they are masked), or with one tile a CTA the elected
+  // lane of warp 0, and of the pages only those there are (a page is one warp's strip, and a warp without tokens reads nothing).  Streams of many
+  // tiles lose by the second form: 128 x 2048 tokens 94.5 us, 96.8 so.
   const uint64_t hint = DECODE ? kEvictFirst : kEvictNormal;
+  constexpr bool WARP = S == 1;
+  const bool issuer = WARP ? warp == 0 : tid == 0, one = WARP ? warp == 0 && elect_one() : true;
   auto issue_tile = [&](int tile, int stage) {
     const uint32_t dst = sbase + stage * kStageBytes;
-    mbar_arrive_expect_tx(full_bar(stage), kStageBytes);
+    const int pages = WARP ? min(4, last_page + 1 - tile * 4) : 4;
+    if (one) mbar_arrive_expect_tx(full_bar(stage), pages * (kStageBytes / 4));
 #pragma unroll
     for (int pg = 0; pg < 4; ++pg) {
+      if (pg >= pages) break;
       int page = tile * 4 + pg;
       page = page > last_page ? last_page : page;
       const int blk = __ldg(btab + page);
       const int row_k = ((blk * 2) * Hkv + kvh) * 16;  // row of the layer's [rows][128] view
       const int row_v = row_k + Hkv * 16;
+      if (!one) continue;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         tma_load_2d(dst + half * kHalfBytes + pg * 2048, &tm_kv, full_bar(stage), half * 64, row_k, hint);
@@ -118,7 +128,7 @@ paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16
       griddep_enter();
       waited = true;
     }
-    if (tid == 0 && t_begin + i < t_end) issue_tile(t_begin + i, i);
+    if (issuer && t_begin + i < t_end) issue_tile(t_begin + i, i);
   }
   if (!waited) griddep_enter();
 
@@ -241,7 +251,7 @@ paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16
       }
     }
     __syncthreads();  // every warp is done reading this stage
-    if (tid == 0 && t + S < t_end) issue_tile(t + S, stage);
+    if (issuer && t + S < t_end) issue_tile(t + S, stage);
   }
 
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
@@ -412,7 +422,7 @@ int attn_decode_split(int num_work, int Hkv, int max_ctx, int sms) {
 
 int paged_attention(const void* q, int ldq, void* out, int ldo, const void* kv_layer, const int* block_tables,
                     int max_blocks, const AttnWork* work, int num_work, int Hq, int Hkv, float scale,
-                    int decode, cudaStream_t st, float* split_ws, int split) {
+                    int decode, cudaStream_t st, float* split_ws, int split, int max_ctx) {
   if (num_work <= 0) return 0;
   if (Hq != 4 * Hkv) return -1;
   if (split > 1 && (!decode || !split_ws)) return -1;
@@ -424,6 +434,7 @@ int paged_attention(const void* q, int ldq, void* out, int ldo, const void* kv_l
   __nv_bfloat16* oo = static_cast<__nv_bfloat16*>(out);
   if (!decode)
     return launch_attn<false, kPrefillStages>(tm, grid, st, qq, ldq, oo, ldo, block_tables, max_blocks, work, Hkv, scale_log2);
+  if (max_ctx > 0 && max_ctx <= kTile) return launch_attn<true, 1>(tm, grid, st, qq, ldq, oo, ldo, block_tables, max_blocks, work, Hkv, scale_log2, split_ws);
   switch (decode_stages()) {
     case 3: return launch_attn<true, 3>(tm, grid, st, qq, ldq, oo, ldo, block_tables, max_blocks, work, Hkv, scale_log2, split_ws);
     case 4: return launch_attn<true, 4>(tm, grid, st, qq, ldq, oo, ldo, block_tables, max_blocks, work, Hkv, scale_log2, split_ws);

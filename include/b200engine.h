@@ -372,7 +372,7 @@ int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, i
  * B200_RULE_KEY_LANES {tokens, heads, the larger head dimension, most keys a token sees, scores capped}: sixteen lanes hold a key.
  * B200_RULE_STREAM {tokens, N, K, pairs}, B200_RULE_CLUSTER {tokens, N, K}: a product of few rows takes csrc/linear_stream.cu or
  *   csrc/linear_cluster.cu although it has a whole-tile form.
- * B200_RULE_SEGMENTS {tokens, sequences, longest, heads, column blocks, state rows, CTAs at once, SMs}: Mamba-2 prompts in segments.
+ * B200_RULE_SEGMENTS {tokens, sequences, longest, heads, column blocks, state rows (any), CTAs at once, SMs}: Mamba-2 prompts in segments.
  * B200_RULE_ROW_REGISTERS {pieces a thread, rows, SMs}: the norms between sublayers keep a row in registers.
  * B200_RULE_ROW_BLOCKS {rows, heads, N, K, fp32 rows}: products per head of 17 to 128 rows in blocks of 16.
  * B200_RULE_SINGLE_STEP {heads times sequences, state rows, value columns, delta rule, SMs}: single tokens as a pass over the states.

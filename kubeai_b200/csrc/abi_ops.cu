@@ -316,7 +316,7 @@ int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_KEY_LANES && n == 5) return rules::sixteen_lanes_a_key(static_cast<long long>(v[0]) * v[1], v[2], v[3], v[4] != 0);
   if (v && rule == B200_RULE_STREAM && n == 4) return rules::stream_pays(v[0], v[1], v[2], v[3] != 0);
   if (v && rule == B200_RULE_CLUSTER && n == 3) return rules::cluster_pays(v[0], v[1], v[2]);
-  if (v && rule == B200_RULE_SEGMENTS && n == 8) return rules::segments_pay(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+  if (v && rule == B200_RULE_SEGMENTS && n == 8) return rules::segments_pay(v[0], v[1], v[2], v[3], v[4], v[6], v[7]);
   if (v && rule == B200_RULE_ROW_REGISTERS && n == 3) return rules::row_in_registers(v[0], v[1], v[2]);
   if (v && rule == B200_RULE_ROW_BLOCKS && n == 5) return rules::row_blocks_pay(v[0], v[1], v[2], v[3], v[4] != 0);
   if (v && rule == B200_RULE_SINGLE_STEP && n == 5) return rules::single_step_pays(v[0], v[1], v[2], v[3] != 0, v[4]);

@@ -62,20 +62,21 @@ inline bool tiles_ahead(int T, int N, int K) {
 }
 
 // Mamba-2 prompts (scan_chunk.cu): sequences cut into segments of 256 tokens, or one chain of 64-token chunks each.  Times in chunks
-// of a chain's CTA with a second one on its SM (13.4 us at 128 state rows; alone on its SM 0.83 of that).  A chain takes its longest
-// sequence, and where not all CTAs (heads, column blocks) run at once as many rounds of equal ones, or the sum of unequal ones and a part of the
-// longest, which comes last at worst; the segments' three launches take about 3 to 5 and then 4 to 4.5 for every time that all of them fill the device.  us, segments / chains, 64 columns, 128 state rows:
-//   8 heads   1 x 4096 83 / 691    6 x 682 89 / 128        64 heads   1 x 512 89 / 97    1 x 4096 269 / 721    3 x 1365 279 / 289
-//   32 heads  4 x 512 103 / 98     6 x 682 162 / 147                  4 x 512 171 / 114  4 x 1024 270 / 217    6 x 682 274 / 281
-//   128 heads 1 x 1024 167 / 185   2 x 512 168 / 113       256 heads  1 x 512 169 / 115  1 x 4096 911 / 823    3 x 1365 965 / 882
-//   unequal: 64 heads 455 + 1365 + 2275 277 / 461; 128 heads 300 + 700 + 1100 + 2000 499 / 550; 256 heads 300 + 2000 561 / 484
+// of a chain's CTA with a second one on its SM (9.2 us at 128 state rows, 6.5 at 64, 5.1 at 32; alone on its SM 0.83 of that).  A chain takes its
+// longest sequence, and where not all CTAs (heads, column blocks) run at once as many rounds of equal ones, or the sum of unequal ones and a part of the
+// longest, which comes last at worst; the segments' three launches take about 4 and then 4.6 for every time that all of them fill the device twice over,
+// with any number of state rows.  us, segments / chains, 64 columns, 128 state rows:
+//   8 heads   1 x 4096 67 / 481    6 x 682 71 / 90         64 heads   1 x 512 71 / 70    1 x 4096 202 / 485    3 x 1365 216 / 206
+//   32 heads  4 x 512 87 / 70      6 x 682 126 / 109                  4 x 512 128 / 84   4 x 1024 208 / 155    6 x 682 214 / 195
+//   128 heads 1 x 1024 124 / 131   2 x 512 128 / 84        256 heads  1 x 512 128 / 84   1 x 4096 744 / 586    3 x 1365 800 / 614
+//   unequal: 64 heads 455 + 1365 + 2275 214 / 330; 128 heads 300 + 700 + 1100 + 2000 407 / 392; 256 heads 300 + 2000 456 / 347
+// 64 state rows: 64 heads 1 x 4096 146 / 338, 4 x 1024 144 / 111, 128 heads 2 x 2048 253 / 211; 32: 64 heads 1 x 4096 118 / 268, 4 x 1024 120 / 88.
 // longest 0: not known, all taken as equal.  From seven sequences on, or with a mean below 512, chains.
-inline bool segments_pay(long long T, int nseq, int longest, int heads, int blocks, int dim, int slots, int sms) {
+inline bool segments_pay(long long T, int nseq, int longest, int heads, int blocks, int slots, int sms) {
   if (nseq < 1 || nseq > 6 || T < 512LL * nseq) return false;
   const double mean = T / 64.0 / nseq, most = ceil(longest > 0 ? longest / 64.0 : mean), per_slot = static_cast<double>(heads) * blocks / slots, rounds = ceil(nseq * per_slot);
   const double chain = rounds <= 1 ? (nseq * heads * blocks <= sms ? 0.83 : 1.0) * most : most <= 1.1 * mean + 1 ? rounds * most : fmax(most, T / 64.0 * per_slot + 0.7 * fmax(0.0, 1.0 - per_slot) * most);
-  const double fills = (T / 256.0 + nseq / 2.0) * per_slot;
-  return (dim <= 32 ? 5.5 + 4.2 * fills : 2.7 + dim / 128.0 + (3.55 + 0.9 * dim / 128.0) * fills) < chain + 0.7;
+  return 4.1 + 4.6 * (T / 256.0 + nseq / 2.0) * heads * blocks / (2.0 * sms) < chain;
 }
 
 // Norms between sublayers (hyper.cu): a row of 256 threads times `pieces` of four columns in registers through both sums, or read from

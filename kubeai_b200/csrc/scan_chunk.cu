@@ -13,12 +13,18 @@
 //
 // Few long sequences leave most of the device to a chain of chunks on few CTAs.  They are cut into segments of kSegment
 // tokens: the sums of all segments at once (PART_SUMS), a pass that turns them into incoming states, the outputs of all segments at
-// once (PART_OUT).  64 heads of 128 x 64, 3 sequences of 455, 1365 and 2275 tokens: one chain each (PART_ALL) 460 us, segments 270.
+// once (PART_OUT).  64 heads of 128 x 64, 3 sequences of 455, 1365 and 2275 tokens: one chain each (PART_ALL) 330 us, segments 214.
 // The sums cost a third of the products again, so sequences whose chains fill the device stay whole (rules::segments_pay).
 //
 // One CTA owns 64 value columns of a (head, sequence or segment) and walks its chunks: 4 warps, each with 16 value columns.  The state
 // lives transposed (value columns x state rows) in the warps' accumulators, which are the left operand of the next chunk's
-// y without leaving the registers; the scores B C^T are computed 16 rows per warp and shared through shared memory.
+// y without leaving the registers; the scores C B^T are computed 16 tokens per warp and shared through shared memory.
+//
+// What bounds it: two to four warps a scheduler (registers, shared memory), which stand behind fixed latencies for half of their time; tensor cores
+// (mma.sync) 40 % of the time, issue slots 40 %.  So the terms of a split operand go round over several sums (three products in a row on one sum wait
+// for each other), a thread's copies step along one column, and in chains and sums the next chunk's keys, values and gates (a chain's queries, once
+// they are read) come in while this one is worked on.  The outputs of a segment, four chunks at most, have three CTAs an SM and one set
+// of tiles instead: 145 us against 174 with two and two (the shape above).  Without all that: a chain 455 us, sums 77, outputs 172; now 330, 57, 145.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -43,11 +49,17 @@ constexpr int kLdX = kCols + 8, kLdM = kQ + 8;
 
 __device__ __forceinline__ float softplusf_(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-size_t chunk_smem(int N) {
-  return static_cast<size_t>(2) * kQ * (N + 8) * 2 + static_cast<size_t>(kQ) * kLdX * 2 + 3ull * kQ * kLdM * 2 + 4 * kQ * sizeof(float);
+// per token: c_t, exp(c_t), d_t (0 past the portion), exp(c_last - c_t) d_t
+struct Gates {
+  float cum[kQ], ecum[kQ], dts[kQ], wts[kQ];
+};
+enum Part { PART_ALL = 0, PART_SUMS, PART_OUT };
+__host__ __device__ constexpr int buffers_for(int part) { return part == PART_OUT ? 1 : 2; }       // of keys, values and gates
+size_t chunk_smem(int N, int part) {
+  const size_t nb = buffers_for(part), qk = part == PART_SUMS ? nb : nb + 1, scores = part == PART_SUMS ? 0 : 3ull * kQ * kLdM * 2;
+  return qk * kQ * (N + 8) * 2 + nb * kQ * kLdX * 2 + scores + nb * sizeof(Gates);
 }
 
-enum Part { PART_ALL = 0, PART_SUMS, PART_OUT };
 constexpr int kSegment = 256;
 // of every segment and head: its sums [dim][vdim], then the state in front of it; the decay over it
 struct Segments {
@@ -56,18 +68,16 @@ struct Segments {
 
 // NK: state rows in units of 16, at most (N = a.dim is any multiple of 16 up to 16 NK)
 template <int NK, int PART>
-__global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a, Segments sg) {
+__global__ void __launch_bounds__(kThreads, PART == PART_SUMS ? 4 : PART == PART_OUT || NK == 2 ? 3 : 2) scalar_decay_chunk_kernel(GlaArgs a, Segments sg) {
   using namespace frag;
   extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr int NB = buffers_for(PART);
   const int N = a.dim, P = a.vdim, nk = N / 16, LDN = N + 8;
-  bf16* Bs = reinterpret_cast<bf16*>(smraw);     // [kQ][LDN] keys
-  bf16* Cs = Bs + kQ * LDN;                      // [kQ][LDN] queries
-  bf16* Xs = Cs + kQ * LDN;                      // [kQ][kLdX] values of the CTA's columns
-  bf16* Ms = Xs + kQ * kLdX;                     // [3][kQ (t)][kLdM (j)] weighted scores, three bf16 terms
-  float* cum = reinterpret_cast<float*>(Ms + 3 * kQ * kLdM);   // [kQ] c_t
-  float* ecum = cum + kQ;                        // [kQ] exp(c_t)
-  float* dts = ecum + kQ;                        // [kQ] d_t (0 past the portion)
-  float* wts = dts + kQ;                         // [kQ] exp(c_last - c_t) d_t
+  bf16* Bbuf = reinterpret_cast<bf16*>(smraw);   // [NB][kQ][LDN] keys
+  bf16* Xbuf = Bbuf + NB * kQ * LDN;             // [NB][kQ][kLdX] values of the CTA's columns
+  Gates* gates = reinterpret_cast<Gates*>(Xbuf + NB * kQ * kLdX);   // [NB]
+  bf16* Cs = reinterpret_cast<bf16*>(gates + NB);   // [kQ][LDN] queries
+  bf16* Ms = Cs + kQ * LDN;                      // [3][kQ (t)][kLdM (j)] weighted scores, three bf16 terms
   const int head = blockIdx.y, p0 = (PART == PART_ALL ? blockIdx.x : blockIdx.z) * kCols;
   int seq = blockIdx.z, segment = 0;
   if (PART != PART_ALL && !find_tile(a.seqs, a.nseq, kSegment, blockIdx.x, &seq, &segment)) return;
@@ -92,111 +102,137 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a,
         S[k][h][c] = (PART != PART_SUMS && k < nk && p < P && pos0 > 0) ? Sg[static_cast<long long>(nn) * P + p] : 0.f;
       }
   const float rate = a.dt_rate[head], dbias = a.dt_bias[head];
-  const int npiece = N / 8, xpiece = kCols / 8;
 
-  for (int c0 = 0; c0 < n; c0 += kQ) {
-    const int q = min(kQ, n - c0);
-    __syncthreads();   // the last chunk's tiles are no longer read
-    const bf16* rows = base + static_cast<long long>(tok0 + c0) * a.ld;
-    for (int e = tid; e < kQ * npiece; e += kThreads) {
-      const int t = e / npiece, c = (e - t * npiece) * 8;
-      bf16 *db = Bs + t * LDN + c, *dc = Cs + t * LDN + c;
-      if (t < q) {
-        const bf16* r = rows + static_cast<long long>(t) * a.ld + qk0 + c;
-        cp_async16(smem_addr(db), r + a.k_off);
-        if (PART != PART_SUMS) cp_async16(smem_addr(dc), r + a.q_off);
-      } else {
-        *reinterpret_cast<uint4*>(db) = make_uint4(0, 0, 0, 0);
-        if (PART != PART_SUMS) *reinterpret_cast<uint4*>(dc) = make_uint4(0, 0, 0, 0);
-      }
-    }
-    for (int e = tid; e < kQ * xpiece; e += kThreads) {
-      const int t = e / xpiece, c = (e - t * xpiece) * 8;
-      bf16* d = Xs + t * kLdX + c;
-      if (t < q && p0 + c < P) cp_async16(smem_addr(d), rows + static_cast<long long>(t) * a.ld + a.v_off + head * P + p0 + c);
+  // a chunk's rows of one column block (keys or queries), 16 bytes a thread and step; rows past the portion become zeros
+  auto fetch_rows = [&](bf16* dst, int off, int c0) {
+    constexpr int kPieces = 2 * NK, kRows = kThreads / kPieces;    // of a row (those past N idle); rows at a time
+    const int t0 = tid / kPieces, c = (tid % kPieces) * 8;
+    if (c >= N) return;
+    const bf16* src = base + static_cast<long long>(tok0 + c0 + t0) * a.ld + off + qk0 + c;
+    bf16* d = dst + t0 * LDN + c;
+#pragma unroll
+    for (int t = 0; t < kQ; t += kRows, src += static_cast<long long>(kRows) * a.ld, d += kRows * LDN) {
+      if (c0 + t0 + t < n) cp_async16(smem_addr(d), src);
       else *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
     }
-    if (w == 0) {
-      // step sizes and running log decays: lane l owns tokens 2l and 2l + 1
-      float d[2], s[2];
+  };
+  auto fetch_values = [&](bf16* dst, int c0) {
+    constexpr int kPieces = kCols / 8, kRows = kThreads / kPieces;
+    const int t0 = tid / kPieces, c = (tid % kPieces) * 8;
+    const bf16* src = base + static_cast<long long>(tok0 + c0 + t0) * a.ld + a.v_off + head * P + p0 + c;
+    bf16* d = dst + t0 * kLdX + c;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int t = 2 * lane + i;
-        d[i] = t < q ? softplusf_(__bfloat162float(static_cast<const bf16*>(a.dt_pre)[static_cast<long long>(tok0 + c0 + t) * a.ld_dt + head]) + dbias) : 0.f;
-        s[i] = rate * d[i];
-      }
-      float run = s[0] + s[1];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float v = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += v;
-      }
-      const float last = __shfl_sync(0xffffffffu, run, 31);
-      total += last;
-      const float before = __shfl_up_sync(0xffffffffu, run, 1);
-      const float cc[2] = {(lane ? before : 0.f) + s[0], run};
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int t = 2 * lane + i;
-        cum[t] = cc[i];
-        ecum[t] = expf(cc[i]);
-        dts[t] = d[i];
-        wts[t] = expf(last - cc[i]) * d[i];
-      }
+    for (int t = 0; t < kQ; t += kRows, src += static_cast<long long>(kRows) * a.ld, d += kRows * kLdX) {
+      if (c0 + t0 + t < n && p0 + c < P) cp_async16(smem_addr(d), src);
+      else *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
     }
-    cp_async_wait_all();
-    __syncthreads();
-
-    // ---- weighted scores: this warp's 16 keys j against the tokens t >= j's block
-    if (PART != PART_SUMS) {
-      float G[4][2][4];
+  };
+  // step sizes and running log decays of a chunk, by one warp: lane l owns tokens 2l and 2l + 1
+  auto make_gates = [&](Gates& G, int c0) {
+    float d[2], s[2];
 #pragma unroll
-      for (int tb = 0; tb < 4; ++tb)
+    for (int i = 0; i < 2; ++i) {
+      const int t = 2 * lane + i;
+      d[i] = c0 + t < n ? softplusf_(__bfloat162float(static_cast<const bf16*>(a.dt_pre)[static_cast<long long>(tok0 + c0 + t) * a.ld_dt + head]) + dbias) : 0.f;
+      s[i] = rate * d[i];
+    }
+    float run = s[0] + s[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += v;
+    }
+    const float last = __shfl_sync(0xffffffffu, run, 31);
+    total += last;
+    const float before = __shfl_up_sync(0xffffffffu, run, 1);
+    const float cc[2] = {(lane ? before : 0.f) + s[0], run};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = 2 * lane + i;
+      G.cum[t] = cc[i];
+      G.ecum[t] = expf(cc[i]);
+      G.dts[t] = d[i];
+      G.wts[t] = expf(last - cc[i]) * d[i];
+    }
+  };
+  auto fetch_all = [&](int c0) {
+    fetch_rows(Bbuf, a.k_off, c0);
+    if (PART != PART_SUMS) fetch_rows(Cs, a.q_off, c0);
+    fetch_values(Xbuf, c0);
+    if (w == 0) make_gates(gates[0], c0);
+  };
+  if (NB == 2) fetch_all(0);
+
+  for (int c0 = 0, buf = 0; c0 < n; c0 += kQ, buf ^= NB - 1) {
+    const int q = min(kQ, n - c0);
+    const bool more = NB == 2 && c0 + kQ < n;
+    if (NB == 1) {
+      __syncthreads();   // the last chunk's tiles are no longer read
+      fetch_all(c0);
+    }
+    const bf16 *Bs = Bbuf + buf * kQ * LDN, *Xs = Xbuf + buf * kQ * kLdX;
+    const Gates& G = gates[buf];
+    cp_async_wait_all();
+    __syncthreads();     // this chunk's tiles and gates are in place; nobody works on the last chunk any more
+    if (more) {
+      fetch_rows(Bbuf + (buf ^ 1) * kQ * LDN, a.k_off, c0 + kQ);
+      fetch_values(Xbuf + (buf ^ 1) * kQ * kLdX, c0 + kQ);
+    }
+
+    // ---- weighted scores: this warp's 16 tokens t against the keys of its own and earlier blocks
+    if (PART != PART_SUMS) {
+      float D[4][2][4];
+#pragma unroll
+      for (int jb = 0; jb < 4; ++jb)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) G[tb][h][c] = 0.f;
+          for (int c = 0; c < 4; ++c) D[jb][h][c] = 0.f;
 #pragma unroll
       for (int k = 0; k < NK; ++k) {
         if (k < nk) {
           uint32_t af[4];
-          ldsm_x4(af, a_addr(Bs, LDN, 16 * w, 16 * k, lane));
+          ldsm_x4(af, a_addr(Cs, LDN, 16 * w, 16 * k, lane));
 #pragma unroll
-          for (int tb = 0; tb < 4; ++tb) {
-            if (tb >= w) {
+          for (int jb = 0; jb < 4; ++jb) {
+            if (jb <= w) {
               uint32_t bf_[4];
-              ldsm_x4(bf_, b_addr(Cs, LDN, 16 * tb, 16 * k, lane));
-              mma(G[tb][0], af, bf_[0], bf_[1]);
-              mma(G[tb][1], af, bf_[2], bf_[3]);
+              ldsm_x4(bf_, b_addr(Bs, LDN, 16 * jb, 16 * k, lane));
+              mma(D[jb][0], af, bf_[0], bf_[1]);
+              mma(D[jb][1], af, bf_[2], bf_[3]);
             }
           }
         }
       }
-      const float cj[2] = {cum[16 * w + g], cum[16 * w + g + 8]}, dj[2] = {dts[16 * w + g], dts[16 * w + g + 8]};
+      const float ct[2] = {G.cum[16 * w + g], G.cum[16 * w + g + 8]};
 #pragma unroll
-      for (int tb = 0; tb < 4; ++tb) {
-        if (tb >= w) {
+      for (int jb = 0; jb < 4; ++jb) {
+        if (jb <= w) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
+          for (int h = 0; h < 2; ++h) {
+            const int j = 16 * jb + 8 * h + 2 * t4;
+            const float2 cj = *reinterpret_cast<const float2*>(G.cum + j), dj = *reinterpret_cast<const float2*>(G.dts + j);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int j = 16 * w + g + 8 * (c >> 1), t = 16 * tb + 8 * h + 2 * t4 + (c & 1);
-              float v = j <= t ? G[tb][h][c] * (expf(cum[t] - cj[c >> 1]) * dj[c >> 1]) : 0.f;
+            for (int hf = 0; hf < 2; ++hf) {
+              const int t = 16 * w + g + 8 * hf;
+              uint32_t x[3];
+              split3(j <= t ? D[jb][h][2 * hf] * (expf(ct[hf] - cj.x) * dj.x) : 0.f, j + 1 <= t ? D[jb][h][2 * hf + 1] * (expf(ct[hf] - cj.y) * dj.y) : 0.f,
+                     &x[0], &x[1], &x[2]);
 #pragma unroll
-              for (int s = 0; s < 3; ++s) {
-                const bf16 b = __float2bfloat16_rn(v);
-                Ms[(s * kQ + t) * kLdM + j] = b;
-                v -= __bfloat162float(b);
-              }
+              for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(Ms + (s * kQ + t) * kLdM + j) = x[s];
             }
+          }
         }
       }
+      if (w == 0 && more) make_gates(gates[buf ^ 1], c0 + kQ);
       __syncthreads();
+    } else if (w == 0 && more) {
+      make_gates(gates[buf ^ 1], c0 + kQ);
     }
 
+    float Y[4][2][4];
     if (live) {
       // ---- y^T [16 value columns x 64 tokens]: the state's part, scaled per token, then the chunk's own
-      float Y[4][2][4];
 #pragma unroll
       for (int tb = 0; tb < 4; ++tb)
 #pragma unroll
@@ -206,21 +242,20 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a,
 #pragma unroll
       for (int k = 0; k < NK; ++k) {
         if (PART != PART_SUMS && k < nk) {
-          uint32_t s0[4], s1[4], s2[4];
-          split3(S[k][0][0], S[k][0][1], &s0[0], &s1[0], &s2[0]);
-          split3(S[k][0][2], S[k][0][3], &s0[1], &s1[1], &s2[1]);
-          split3(S[k][1][0], S[k][1][1], &s0[2], &s1[2], &s2[2]);
-          split3(S[k][1][2], S[k][1][3], &s0[3], &s1[3], &s2[3]);
+          uint32_t st[3][4];
 #pragma unroll
-          for (int tb = 0; tb < 4; ++tb) {
-            uint32_t b[4];
-            ldsm_x4(b, b_addr(Cs, LDN, 16 * tb, 16 * k, lane));
+          for (int r = 0; r < 4; ++r) split3(S[k][r >> 1][2 * (r & 1)], S[k][r >> 1][2 * (r & 1) + 1], &st[0][r], &st[1][r], &st[2][r]);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              mma(Y[tb][h], s2, b[2 * h], b[2 * h + 1]);
-              mma(Y[tb][h], s1, b[2 * h], b[2 * h + 1]);
-              mma(Y[tb][h], s0, b[2 * h], b[2 * h + 1]);
-            }
+          for (int half = 0; half < 2; ++half) {
+            uint32_t b[2][4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) ldsm_x4(b[i], b_addr(Cs, LDN, 32 * half + 16 * i, 16 * k, lane));
+#pragma unroll
+            for (int term = 2; term >= 0; --term)
+#pragma unroll
+              for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) mma(Y[2 * half + i][h], st[term], b[i][2 * h], b[i][2 * h + 1]);
           }
         }
       }
@@ -228,26 +263,32 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a,
       for (int tb = 0; tb < 4; ++tb)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const float e0 = ecum[16 * tb + 8 * h + 2 * t4], e1 = ecum[16 * tb + 8 * h + 2 * t4 + 1];
-          Y[tb][h][0] *= e0; Y[tb][h][1] *= e1; Y[tb][h][2] *= e0; Y[tb][h][3] *= e1;
+          const float2 e = *reinterpret_cast<const float2*>(G.ecum + 16 * tb + 8 * h + 2 * t4);
+          Y[tb][h][0] *= e.x; Y[tb][h][1] *= e.y; Y[tb][h][2] *= e.x; Y[tb][h][3] *= e.y;
         }
-      const float decay = ecum[kQ - 1];
+      const float decay = G.ecum[kQ - 1];
 #pragma unroll
       for (int k = 0; k < NK; ++k)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int c = 0; c < 4; ++c) S[k][h][c] *= decay;
+    }
+    if (PART != PART_SUMS && more) {
+      __syncthreads();   // the queries are no longer read
+      fetch_rows(Cs, a.q_off, c0 + kQ);
+    }
+    if (live) {
 #pragma unroll
       for (int jb = 0; jb < 4; ++jb) {
         if (16 * jb >= q) break;       // no tokens there
         uint32_t xf[4];
         ldsm_x4_trans(xf, at_addr(Xs, kLdX, 16 * jb, 16 * w, lane));
+        if (PART != PART_SUMS) {
 #pragma unroll
-        for (int tb = 0; tb < 4; ++tb) {
-          if (PART != PART_SUMS && tb >= jb) {
+          for (int s = 2; s >= 0; --s) {
 #pragma unroll
-            for (int s = 2; s >= 0; --s) {
+            for (int tb = jb; tb < 4; ++tb) {
               uint32_t b[4];
               ldsm_x4(b, b_addr(Ms + s * kQ * kLdM, kLdM, 16 * tb, 16 * jb, lane));
               mma(Y[tb][0], xf, b[0], b[1]);
@@ -255,38 +296,39 @@ __global__ void __launch_bounds__(kThreads) scalar_decay_chunk_kernel(GlaArgs a,
             }
           }
         }
+        if (PART == PART_OUT && c0 + kQ >= n) continue;   // nobody asks for the state behind the last chunk
         // the state takes exp(c_last - c_j) d_j x_j B_j^T
-        const float2 wl = *reinterpret_cast<const float2*>(wts + 16 * jb + 2 * t4), wh = *reinterpret_cast<const float2*>(wts + 16 * jb + 8 + 2 * t4);
-        uint32_t x0[4], x1[4], x2[4];
-        split3(low(xf[0]) * wl.x, high(xf[0]) * wl.y, &x0[0], &x1[0], &x2[0]);
-        split3(low(xf[1]) * wl.x, high(xf[1]) * wl.y, &x0[1], &x1[1], &x2[1]);
-        split3(low(xf[2]) * wh.x, high(xf[2]) * wh.y, &x0[2], &x1[2], &x2[2]);
-        split3(low(xf[3]) * wh.x, high(xf[3]) * wh.y, &x0[3], &x1[3], &x2[3]);
+        const float2 wl = *reinterpret_cast<const float2*>(G.wts + 16 * jb + 2 * t4), wh = *reinterpret_cast<const float2*>(G.wts + 16 * jb + 8 + 2 * t4);
+        uint32_t x[3][4];
 #pragma unroll
-        for (int k = 0; k < NK; ++k) {
+        for (int r = 0; r < 4; ++r) split3(low(xf[r]) * (r < 2 ? wl.x : wh.x), high(xf[r]) * (r < 2 ? wl.y : wh.y), &x[0][r], &x[1][r], &x[2][r]);
+#pragma unroll
+        for (int k = 0; k < NK; k += 2) {
           if (k < nk) {
-            uint32_t b[4];
-            ldsm_x4_trans(b, bt_addr(Bs, LDN, 16 * jb, 16 * k, lane));
+            uint32_t b[2][4];
+            ldsm_x4_trans(b[0], bt_addr(Bs, LDN, 16 * jb, 16 * k, lane));
+            if (k + 1 < nk) ldsm_x4_trans(b[1], bt_addr(Bs, LDN, 16 * jb, 16 * (k + 1), lane));
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              mma(S[k][h], x2, b[2 * h], b[2 * h + 1]);
-              mma(S[k][h], x1, b[2 * h], b[2 * h + 1]);
-              mma(S[k][h], x0, b[2 * h], b[2 * h + 1]);
-            }
+            for (int term = 2; term >= 0; --term)
+#pragma unroll
+              for (int i = 0; i < 2; ++i)
+                if (k + i < nk) {
+                  mma(S[k + i][0], x[term], b[i][0], b[i][1]);
+                  mma(S[k + i][1], x[term], b[i][2], b[i][3]);
+                }
           }
         }
       }
       if (PART == PART_SUMS) continue;
-      float* out = a.o + static_cast<long long>(tok0 + c0) * (a.heads * P) + head * P;
+      const int HP = a.heads * P;
+      float* out = a.o + static_cast<long long>(tok0 + c0 + 2 * t4) * HP + head * P + pr[0];
 #pragma unroll
       for (int tb = 0; tb < 4; ++tb)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h, out += 8ll * HP)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int t = 16 * tb + 8 * h + 2 * t4 + (c & 1), p = pr[c >> 1];
-            if (t < q && p < P) out[static_cast<long long>(t) * (a.heads * P) + p] = Y[tb][h][c];
-          }
+          for (int c = 0; c < 4; ++c)
+            if (16 * tb + 8 * h + 2 * t4 + (c & 1) < q && pr[c >> 1] < P) out[(c & 1 ? HP : 0) + 8 * (c >> 1)] = Y[tb][h][c];
     }
   }
   if (PART == PART_SUMS && p0 == 0 && tid == 0) sg.d[static_cast<long long>(blockIdx.x) * a.heads + head] = expf(total);
@@ -341,8 +383,8 @@ __global__ void __launch_bounds__(256) segment_states_kernel(GlaArgs a, Segments
 template <int NK, int PART>
 int launch_part(const GlaArgs& a, const Segments& sg, dim3 grid, cudaStream_t st) {
   static std::atomic<unsigned long long> attr{0};
-  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK, PART>, static_cast<int>(chunk_smem(16 * NK)), &attr)) return -2;
-  scalar_decay_chunk_kernel<NK, PART><<<grid, kThreads, chunk_smem(a.dim), st>>>(a, sg);
+  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK, PART>, static_cast<int>(chunk_smem(16 * NK, PART)), &attr)) return -2;
+  scalar_decay_chunk_kernel<NK, PART><<<grid, kThreads, chunk_smem(a.dim, PART), st>>>(a, sg);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 // Segments where they are the shorter way (slots: CTAs of the chain that run at once), and their workspace is there.
@@ -351,7 +393,7 @@ bool cut_into_segments(const GlaArgs& a, int slots) {
   const int force = e ? atoi(e) : -1;
   if (force == 0 || !a.par_ws || scan_segments_ws_floats(a.T, a.nseq, a.heads, a.dim, a.vdim) > a.par_ws_floats || a.vdim % 4 ||
       (reinterpret_cast<uintptr_t>(a.par_ws) | reinterpret_cast<uintptr_t>(a.states)) % 16) return false;
-  return force == 1 || rules::segments_pay(a.T, a.nseq, a.max_rows, a.heads, (a.vdim + kCols - 1) / kCols, a.dim, slots, sm_count());
+  return force == 1 || rules::segments_pay(a.T, a.nseq, a.max_rows, a.heads, (a.vdim + kCols - 1) / kCols, slots, sm_count());
 }
 template <int NK>
 int launch(const GlaArgs& a, cudaStream_t st) {
@@ -359,8 +401,8 @@ int launch(const GlaArgs& a, cudaStream_t st) {
   Segments sg = {nullptr, nullptr};
   static std::atomic<unsigned long long> attr{0};
   int per_sm = 0;
-  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK, PART_ALL>, static_cast<int>(chunk_smem(16 * NK)), &attr) ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scalar_decay_chunk_kernel<NK, PART_ALL>, kThreads, chunk_smem(a.dim)) != cudaSuccess) return -2;
+  if (!ensure_dynamic_smem(scalar_decay_chunk_kernel<NK, PART_ALL>, static_cast<int>(chunk_smem(16 * NK, PART_ALL)), &attr) ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, scalar_decay_chunk_kernel<NK, PART_ALL>, kThreads, chunk_smem(a.dim, PART_ALL)) != cudaSuccess) return -2;
   if (!cut_into_segments(a, std::max(1, per_sm) * sm_count())) return launch_part<NK, PART_ALL>(a, sg, dim3(cb, a.heads, a.nseq), st);
   const int segs = a.T / kSegment + a.nseq;
   sg.s = a.par_ws;

@@ -65,6 +65,13 @@ def test_sequences_are_cut_where_their_chains_leave_the_device_idle(heads, block
         assert rule(SEGMENTS, nseq * each, nseq, longest, heads, blocks, dim, 444 if dim <= 32 else 296, 148) == cut
 
 
+@pytest.mark.parametrize("heads,dim,nseq,each,cut", [(64, 128, 6, 682, 0), (64, 128, 2, 1024, 1), (128, 64, 2, 2048, 0), (256, 64, 1, 4096, 0), (128, 64, 3, 1365, 1),
+                                                     (64, 32, 4, 1024, 0), (128, 32, 2, 2048, 0), (64, 32, 1, 1024, 1), (256, 32, 1, 4096, 0)])
+def test_chains_whose_tiles_come_in_ahead_stay_whole_longer(heads, dim, nseq, each, cut):
+    """128 heads, 64 state rows, two sequences of 2048: 253 us in segments, 303 in chains that waited for each chunk's tiles, 211 since."""
+    assert rule(SEGMENTS, nseq * each, nseq, each, heads, 1, dim, 444 if dim <= 32 else 296, 148) == cut
+
+
 def test_a_chain_is_as_long_as_its_longest_sequence():
     assert rule(SEGMENTS, 4095, 3, 2275, 64, 1, 128, 296, 148) == 1 and rule(SEGMENTS, 4096, 4, 3000, 64, 1, 128, 296, 148) == 1
     assert rule(SEGMENTS, 4100, 4, 2000, 128, 1, 128, 296, 148) == 1 and rule(SEGMENTS, 2300, 2, 2000, 256, 1, 128, 296, 148) == 0

@@ -112,39 +112,198 @@ __global__ void moe_route_kernel(float* scores, int* topk_ids, float* topk_w, in
   }
 }
 
-// single CTA: histogram, padded offsets, scatter
-__global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, int pairs, int top, int E, int* sorted_rows, int* tile_group,
-                                                         int* pair_pos, int cap, int* expert_rows, const float* topk_w, float* sorted_w, int matrices) {
+// The same with the token's scores in registers, lane l holding experts l, l + 32, ...: at most 32 R experts and 32 choices.  A step through
+// the scratch row above is a trip to the cache, several of them one behind the other for each choice; here only the groups' ranks meet, in
+// shared memory.  16 experts, two choices: 4096 tokens 9.8 us above, 4.1 here; 24 tokens 4.2 and 2.1.
+template <int R>
+__global__ void __launch_bounds__(128) moe_route_few_kernel(const float* scores, int* topk_ids, float* topk_w, int T, int E, int groups, int keep, int top, int score_fn,
+                                                            int ld, const float* bias, MoeRouteForm form) {
+  __shared__ float ranks[4][32 * R];
+  const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, t = blockIdx.x * 4 + wrp;
+  float b[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) b[r] = bias && lane + 32 * r < E ? bias[lane + 32 * r] : 0.f;
   griddep_launch();
   griddep_wait();
-  extern __shared__ int sh[];   // count[E], start[E + 1], fill[E]
+  if (t >= T) return;
+  float s[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) s[r] = lane + 32 * r < E ? scores[static_cast<long long>(t) * ld + lane + 32 * r] : 0.f;
+  if (score_fn == MOE_SIGMOID) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = 1.0f / (1.0f + expf(-s[r]));
+  } else if (score_fn == MOE_TOP_SOFTMAX) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = fmaxf(s[r], -0.5f * FLT_MAX);   // a logit stays above the mark
+  } else {
+    float mx = -FLT_MAX, sum = 0.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) if (lane + 32 * r < E) mx = fmaxf(mx, s[r]);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+    for (int r = 0; r < R; ++r) if (lane + 32 * r < E) { s[r] = expf(s[r] - mx); sum += s[r]; }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float inv = 1.0f / sum;
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] *= inv;
+  }
+  // what an expert is ranked by; at `lowest`: not there, not eligible or chosen already
+  const float lowest = bias || score_fn == MOE_TOP_SOFTMAX ? -FLT_MAX : -1.f;
+  float v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = lane + 32 * r < E ? (bias ? s[r] + b[r] : s[r]) : lowest;
+  if (keep < groups || form.group_best == 2) {
+    const int per = E / groups;
+#pragma unroll
+    for (int r = 0; r < R; ++r) ranks[wrp][lane + 32 * r] = v[r];
+    __syncwarp();
+    float gm[2];           // of groups lane and lane + 32
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      gm[i] = lowest;
+      const int g = lane + 32 * i;
+      if (g < groups) {
+        float second = lowest;
+        for (int e = g * per; e < (g + 1) * per; ++e) {
+          const float x = ranks[wrp][e];
+          second = fmaxf(second, fminf(gm[i], x));
+          gm[i] = fmaxf(gm[i], x);
+        }
+        if (form.group_best == 2 && per > 1) gm[i] += second;
+      }
+    }
+    unsigned long long kept = 0;
+    for (int k = 0; k < keep; ++k) {
+      float best = lowest;
+      int bg = 0x7fffffff;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (gm[i] > best) { best = gm[i]; bg = lane + 32 * i; }
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int og = __shfl_xor_sync(0xffffffffu, bg, o);
+        if (ob > best || (ob == best && og < bg)) { best = ob; bg = og; }
+      }
+      if (bg == 0x7fffffff) break;
+      kept |= 1ull << bg;
+      if (bg == lane) gm[0] = lowest;
+      if (bg == lane + 32) gm[1] = lowest;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (lane + 32 * r < E && !(kept >> ((lane + 32 * r) / per) & 1ull)) v[r] = lowest;
+  }
+  float first = 0.f, sum = 0.f, mine = 0.f;   // choice k stays with lane k
+  int my_id = 0;
+  for (int k = 0; k < top; ++k) {
+    float best = lowest;
+    int be = 0x7fffffff;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (v[r] > best) { best = v[r]; be = lane + 32 * r; }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oe = __shfl_xor_sync(0xffffffffu, be, o);
+      if (ob > best || (ob == best && oe < be)) { best = ob; be = oe; }
+    }
+    if (be == 0x7fffffff) { be = 0; best = 0.f; }
+    else {
+      float weight = 0.f;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (be == lane + 32 * r) { weight = s[r]; v[r] = lowest; }
+      if (bias) best = __shfl_sync(0xffffffffu, weight, be & 31);     // the weight is the score without the bias
+    }
+    if (k == 0) first = best;
+    sum += score_fn == MOE_TOP_SOFTMAX ? expf(best - first) : best;
+    if (lane == k) { my_id = be; mine = best; }
+  }
+  if (score_fn == MOE_TOP_SOFTMAX) {
+    const float inv = 1.0f / sum;
+    mine = expf(mine - first) * inv;
+  } else if (form.normalize) {
+    mine = mine / (sum + form.sum_eps) * form.scale;
+  }
+  if (lane < top) {
+    topk_ids[static_cast<long long>(t) * top + lane] = my_id;
+    topk_w[static_cast<long long>(t) * top + lane] = mine;
+  }
+}
+
+// Single CTA: a pair's rank among its expert's from a count that the lanes of a warp with the same expert raise together, padded
+// offsets, scatter.  What bounds it is one SM's latencies in a row, so a thread has its pairs' loads under way at once and meets the counts
+// once.  16 experts, 48 pairs: 4.2 us with a count and a place per pair and one thread that laid out the tiles, 3.1 now; 8192 pairs take 10 as before.
+__global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, int pairs, int top, int E, int* sorted_rows, int* tile_group,
+                                                         int* pair_pos, int cap, int* expert_rows, const float* topk_w, float* sorted_w, int matrices) {
+  extern __shared__ int sh[];   // count[E], start[E]
   int* count = sh;
   int* start = sh + E;
-  int* fill = sh + 2 * E + 1;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) { count[e] = 0; fill[e] = 0; }
+  const int lane = threadIdx.x & 31;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+  griddep_launch();
+  griddep_wait();
+  constexpr int U = 8;          // pairs a thread holds; with more than that in all, ranks wait in pair_pos
+  const int held = U * 1024;
+  int id[U], rank[U];
+  auto load_ids = [&](int p0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int p = p0 + u * 1024 + threadIdx.x;
+      id[u] = p < pairs ? topk_ids[p] : -1;
+    }
+  };
+  load_ids(0);
   for (int i = threadIdx.x; i < cap; i += blockDim.x) { sorted_rows[i] = -1; if (sorted_w) sorted_w[i] = 0.f; }
   for (int i = threadIdx.x; i < cap / 64; i += blockDim.x) tile_group[i] = -1;
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&count[topk_ids[p]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int e = 0; e < E; ++e) {
-      start[e] = at;
-      if (expert_rows) { expert_rows[2 * e] = at; expert_rows[2 * e + 1] = count[e]; }
-      const int tiles = (count[e] + 63) / 64;
-      for (int i = 0; i < tiles; ++i) tile_group[at / 64 + i] = e < matrices ? e : -1;   // an expert without matrices: its tiles are skipped
-      at += tiles * 64;
+  for (int p0 = 0; p0 < pairs; p0 += held) {
+    if (p0) load_ids(p0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (p0 + u * 1024 < pairs) {
+        const unsigned same = __match_any_sync(0xffffffffu, id[u]);
+        const int leader = __ffs(same) - 1;
+        int before = 0;
+        if (lane == leader && id[u] >= 0) before = atomicAdd(&count[id[u]], __popc(same));
+        rank[u] = __shfl_sync(0xffffffffu, before, leader) + __popc(same & ((1u << lane) - 1));
+        const int p = p0 + u * 1024 + threadIdx.x;
+        if (pairs > held && p < pairs) pair_pos[p] = rank[u];
+      }
     }
-    start[E] = at;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int e = topk_ids[p];
-    const int r = start[e] + atomicAdd(&fill[e], 1);
-    sorted_rows[r] = p / top;
-    pair_pos[p] = r;
-    if (sorted_w) sorted_w[r] = topk_w[p];
+  if (threadIdx.x < 32) {
+    int at = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, rows = e < E ? count[e] : 0;
+      int end = (rows + 63) / 64 * 64;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += x;
+      }
+      if (e < E) {
+        start[e] = at + end - (rows + 63) / 64 * 64;
+        if (expert_rows) { expert_rows[2 * e] = start[e]; expert_rows[2 * e + 1] = rows; }
+      }
+      at += __shfl_sync(0xffffffffu, end, 31);
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x >> 5; e < E && e < matrices; e += 32)     // an expert without matrices: its tiles are skipped
+    for (int i = lane; i < (count[e] + 63) / 64; i += 32) tile_group[start[e] / 64 + i] = e;
+  for (int p0 = 0; p0 < pairs; p0 += held) {
+    if (pairs > held) load_ids(p0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int p = p0 + u * 1024 + threadIdx.x;
+      if (p < pairs) {
+        const int r = start[id[u]] + (pairs > held ? pair_pos[p] : rank[u]);
+        sorted_rows[r] = p / top;
+        pair_pos[p] = r;
+        if (sorted_w) sorted_w[r] = topk_w[p];
+      }
+    }
   }
 }
 
@@ -219,7 +378,12 @@ int moe_route(float* scores, int* topk_ids, float* topk_w, int T, int E, int gro
   if (E < 1 || groups < 1 || groups > 64 || E % groups || keep < 1 || keep > groups || top < 1 || top > keep * (E / groups)) return -1;
   if ((select_bias || form.normalize) && score_fn == MOE_TOP_SOFTMAX) return -1;
   if (form.group_best < 1 || form.group_best > 2) return -1;
-  launch_pdl(moe_route_kernel, (T + 3) / 4, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, ld > 0 ? ld : E, select_bias, form);
+  const int blocks = (T + 3) / 4, lds = ld > 0 ? ld : E;
+  if (E <= 32 && top <= 32) launch_pdl(moe_route_few_kernel<1>, blocks, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, lds, select_bias, form);
+  else if (E <= 64 && top <= 32) launch_pdl(moe_route_few_kernel<2>, blocks, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, lds, select_bias, form);
+  else if (E <= 128 && top <= 32) launch_pdl(moe_route_few_kernel<4>, blocks, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, lds, select_bias, form);
+  else if (E <= 256 && top <= 32) launch_pdl(moe_route_few_kernel<8>, blocks, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, lds, select_bias, form);
+  else launch_pdl(moe_route_kernel, blocks, 128, 0, st, scores, topk_ids, topk_w, T, E, groups, keep, top, score_fn, lds, select_bias, form);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -227,9 +391,8 @@ int moe_align(const int* topk_ids, int T, int top, int E, int* sorted_rows, int*
               int* expert_rows, const float* topk_w, float* sorted_w, int matrices) {
   if (T <= 0) return 0;
   if (cap % 64 || cap < T * top + E * 64 || (sorted_w && !topk_w)) return -1;
-  const size_t smem = static_cast<size_t>(3 * E + 1) * sizeof(int);
-  if (smem > 48 * 1024) return -1;
-  launch_pdl(moe_align_kernel, 1, 1024, smem, st, topk_ids, T * top, top, E, sorted_rows, tile_group, pair_pos, cap, expert_rows, topk_w, sorted_w, matrices > 0 ? matrices : E);
+  if (E > 4095) return -1;
+  launch_pdl(moe_align_kernel, 1, 1024, 2 * E * sizeof(int), st, topk_ids, T * top, top, E, sorted_rows, tile_group, pair_pos, cap, expert_rows, topk_w, sorted_w, matrices > 0 ? matrices : E);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

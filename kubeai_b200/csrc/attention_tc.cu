@@ -9,13 +9,15 @@
 //     the same page gather as the decode kernel) and issues every tcgen05.mma:
 //         S_i = Q_i K^T          M=128 (rows = token x head), N=64 kv tokens, K=128 dims; Q_i lands by a 3-D TMA box
 //                                (64 dims x 4 heads x 32 tokens) straight from the fused qkv buffer, K-major, swizzled
-//         PV_i = P_i V           M=128, N=128 dims, K=64 kv tokens; P_i is written to shared memory by the softmax warps as
-//                                a K-major swizzled A operand, V is read in place as an MN-major B operand (its rows are kv
-//                                tokens = the contraction index), so no transpose of V is ever made
-//     accumulators live in TMEM: S_0, S_1 (64 columns each) and PV_0, PV_1 (128 columns each);
+//         PV_i = P_i V           M=128, N=128 dims, K=64 kv tokens; P_i lies in TMEM, where the softmax warps wrote it over its
+//                                scores, V is read in place as an MN-major B operand (its rows are kv tokens = the contraction
+//                                index), so no transpose of V is ever made
+//     accumulators live in TMEM: two buffers each of S_0, S_1 (64 columns) and PV_0, PV_1 (128 columns each);
 //   * two softmax warpgroups (4 warps each, one per 128-row tile, thread = row as tcgen05.ld 32x32b delivers it) run the
 //     online softmax in fp32 with base-2 exponentials, rescale the running output in TMEM (tcgen05.ld / .st) only when a row
-//     of the warp moved its maximum, and hand P back; while one group is in its softmax the tensor core works for the other.
+//     of the warp took a new reference, and hand P back; the next tile's scores are formed meanwhile.
+// What bounds it: the chain softmax, P, products of the longest CTA.  2048 new tokens in one prompt, 32 query and 8 key heads: 36.9 us with one
+// buffer of scores, P in shared memory and a rescaling for every new maximum, 27 now.
 // Causal masking by absolute position; K/V rows of a page beyond the sequence end are finite (the pool is zero-filled) and
 // masked.  Output rounding: one bf16 rounding of the normalised fp32 result, as the decode kernel.
 #include <cuda.h>
@@ -42,11 +44,13 @@ constexpr int kQTok = 32;                       // query tokens per 128-row UMMA
 constexpr int kHalf = kKvTile * 128;            // [64 tokens][64 dims] bf16: 8 KB
 constexpr int kKTile = 2 * kHalf;               // K tile: two 64-column halves, 16 KB
 constexpr int kKvStage = 2 * kKTile;            // K + V: 32 KB
-constexpr int kStages = 2;
+constexpr int kStages = 3;
 constexpr int kQHalf = 128 * 128;               // [128 rows][64 dims] bf16: 16 KB
 constexpr int kQTile = 2 * kQHalf;              // 32 KB per UMMA tile
-constexpr int kPTile = 128 * 128;               // [128 rows][64 kv] bf16: 16 KB
-constexpr int kSmem = 1024 + kStages * kKvStage + 2 * kQTile + 2 * kPTile + 256;   // 161 KB
+constexpr int kSmem = 1024 + kStages * kKvStage + 2 * kQTile + 256;   // 161 KB
+// Weights are relative to 2^kSlack times the row's largest so far when that was last taken: none is above 1, and the output in TMEM is
+// scaled again only behind a score that is larger by more than that, which after a row's first keys hardly any is.
+constexpr float kSlack = 8.f;
 constexpr int kThreads = 288;                   // warp 0: driver (TMA + MMA); warps 1-4: rows of tile 0; warps 5-8: tile 1
 
 // Instruction descriptor: D=f32, A=B=bf16, A K-major, B K-major (b_mn = 0) or MN-major (b_mn = 1), M x N.
@@ -78,15 +82,15 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
   uint8_t* smem = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t kv_s = sbase;                                  // [stage][K half0 | K half1 | V half0 | V half1]
   const uint32_t q_s = kv_s + kStages * kKvStage;               // [tile][half0 | half1]
-  const uint32_t p_s = q_s + 2 * kQTile;                        // [tile][128 rows x 128 B]
-  const uint32_t bars = p_s + 2 * kPTile;
+  const uint32_t bars = q_s + 2 * kQTile;
   auto kv_full = [&](int s) { return bars + 8u * s; };          // TMA -> driver
-  auto kv_empty = [&](int s) { return bars + 8u * (2 + s); };   // MMA commit -> driver (stage can be refilled)
-  auto s_full = [&](int i) { return bars + 8u * (4 + i); };     // MMA commit -> group i
-  auto p_ready = [&](int i) { return bars + 8u * (6 + i); };    // group i (4 warp arrivals) -> driver: P_i written, S_i read, O_i rescaled
-  auto pv_full = [&](int i) { return bars + 8u * (8 + i); };    // MMA commit -> group i
-  const uint32_t q_bar = bars + 8u * 12;
-  const uint32_t tmem_slot = bars + 8u * 13;
+  auto kv_empty = [&](int s) { return bars + 8u * (3 + s); };   // MMA commit -> driver (stage can be refilled)
+  auto s_full = [&](int i, int b) { return bars + 8u * (6 + 2 * i + b); };   // MMA commit -> group i
+  // of every other tile each, as the scores': a warp is up to two tiles ahead of the slowest one of its group
+  auto p_ready = [&](int i, int b) { return bars + 8u * (10 + 2 * i + b); };   // group i (4 warp arrivals) -> driver: S_i read, P_i in its place, O_i rescaled
+  auto pv_full = [&](int i, int b) { return bars + 8u * (14 + 2 * i + b); };   // MMA commit -> group i
+  const uint32_t q_bar = bars + 8u * 18;
+  const uint32_t tmem_slot = bars + 8u * 19;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem + (tmem_slot - sbase));
 
   const AttnWork wk = work[blockIdx.y];     // q_count <= 64 query tokens of one sequence
@@ -106,9 +110,11 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
         mbar_init(kv_empty(s), 1);
       }
       for (int i = 0; i < 2; ++i) {
-        mbar_init(s_full(i), 1);
-        mbar_init(p_ready(i), 4);
-        mbar_init(pv_full(i), 1);
+        for (int b = 0; b < 2; ++b) {
+          mbar_init(s_full(i, b), 1);
+          mbar_init(p_ready(i, b), 4);
+          mbar_init(pv_full(i, b), 1);
+        }
       }
       mbar_init(q_bar, 1);
       fence_mbar_init();
@@ -121,8 +127,8 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  const uint32_t tm_S[2] = {tmem_base, tmem_base + 64};
-  const uint32_t tm_PV[2] = {tmem_base + 128, tmem_base + 256};
+  auto tm_S = [&](int i, int b) { return tmem_base + 64u * (2 * i + b); };
+  const uint32_t tm_PV[2] = {tmem_base + 256, tmem_base + 384};
   // prefill tiles may hold K/V rows and q rows written by this step's upstream kernels: wait before any load
   griddep_enter();
 
@@ -152,51 +158,51 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
       for (int i = 0; i < 2; ++i)
         for (int half = 0; half < 2; ++half)
           if (one) tma_load_3d(q_s + i * kQTile + half * kQHalf, &tm_q, q_bar, half * 64, kvh * 4, wk.q_tok0 + i * kQTok);
-      for (int s = 0; s < kStages && s < ntiles; ++s) issue_tile(s, s);
+      for (int s = 0; s < kStages - 1 && s < ntiles; ++s) issue_tile(s, s);
       mbar_wait_warp(q_bar, 0);
 
       const uint32_t idesc_s = idesc_bf16(128, kKvTile, 0);
       const uint32_t idesc_pv = idesc_bf16(128, kD, 1);
-      uint32_t ph_p[2] = {0, 0};
-      for (int t = 0; t < ntiles; ++t) {
+      const uint64_t q_d = smem_desc_sw128(q_s, 16, 1024), k_d = smem_desc_sw128(kv_s, 16, 1024), v_d = smem_desc_sw128(kv_s + kKTile, kHalf, 1024);
+      // S_i = Q_i K^T into the buffer of tile t's parity.  Its previous scores, of tile t - 2, have been read: group i's p_ready
+      // arrival of that tile, waited for before PV_i(t - 2) was issued, came after its tcgen05.ld of S_i.
+      auto scores = [&](int t) {
         const int stage = t % kStages;
         mbar_wait_warp(kv_full(stage), static_cast<uint32_t>(t / kStages) & 1u);
         tc_fence_after();
-        const uint32_t ks = kv_s + stage * kKvStage, vs = ks + kKTile;
-        // S_i = Q_i K^T.  S_i of the previous tile has been read: group i's p_ready arrival of tile t-1 (waited below
-        // before PV_i(t-1) was issued) came after its tcgen05.ld of S_i.
+        if (one) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+          for (int i = 0; i < 2; ++i) {
 #pragma unroll
-          for (int k = 0; k < kD / 16; ++k) {
-            const uint32_t koff = (k >> 2) * kQHalf + (k & 3) * 32;     // 64 dims per half, 32 B per k-step inside it
-            const uint32_t kboff = (k >> 2) * kHalf + (k & 3) * 32;
-            if (one) umma_bf16(tm_S[i], smem_desc_sw128(q_s + i * kQTile + koff, 16, 1024), smem_desc_sw128(ks + kboff, 16, 1024), idesc_s,
-                      k > 0 ? 1u : 0u);
+            for (int h = 0; h < 2; ++h)       // 64 dims per half
+              umma_bf16_k64(tm_S(i, t & 1), q_d + ((i * kQTile + h * kQHalf) >> 4), k_d + ((stage * kKvStage + h * kHalf) >> 4), idesc_s, h > 0 ? 1u : 0u);
+            umma_commit(s_full(i, t & 1));
           }
-          if (one) umma_commit(s_full(i));
+        }
+      };
+      scores(0);
+      for (int t = 0; t < ntiles; ++t) {
+        // the next scores are formed under this tile's softmax; then tile t - 1's stage, whose products are the last ones queued in front of
+        // them, takes tile t + 2
+        if (t + 1 < ntiles) scores(t + 1);
+        if (t + kStages - 1 < ntiles) {
+          const int next = t + kStages - 1, stage = next % kStages;
+          if (t > 0) mbar_wait_warp(kv_empty(stage), static_cast<uint32_t>((t - 1) / kStages) & 1u);
+          issue_tile(next, stage);
         }
         // PV_i += P_i V once group i has written P_i (and rescaled the running output to this tile's maximum)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          mbar_wait_warp(p_ready(i), ph_p[i]);
-          ph_p[i] ^= 1u;
+          mbar_wait_warp(p_ready(i, t & 1), static_cast<uint32_t>(t >> 1) & 1u);
           tc_fence_after();
-#pragma unroll
-          for (int k = 0; k < kKvTile / 16; ++k) {
-            // A = P_i: K-major rows of 128 B (64 kv), k-step = 32 B; B = V: MN-major, 16 kv rows per k-step = 2048 B,
-            // leading offset = the second 64-dim half, stride = 8 rows
-            if (one) umma_bf16(tm_PV[i], smem_desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), smem_desc_sw128(vs + k * 2048, kHalf, 1024), idesc_pv,
-                      (t > 0 || k > 0) ? 1u : 0u);
+          // A = P_i: 64 kv in 32 columns; B = V: MN-major, 16 kv rows per k-step = 2048 B, leading offset = the second 64-dim half, stride = 8 rows
+          if (one) {
+            umma_bf16_tmem_k64(tm_PV[i], tm_S(i, t & 1), v_d + (((t % kStages) * kKvStage) >> 4), idesc_pv, t > 0 ? 1u : 0u);
+            umma_commit(pv_full(i, t & 1));
           }
-          if (one) umma_commit(pv_full(i));
         }
-        if (one) umma_commit(kv_empty(stage));
+        if (one) umma_commit(kv_empty(t % kStages));
         __syncwarp();
-        if (t + kStages < ntiles) {
-          mbar_wait_warp(kv_empty(stage), static_cast<uint32_t>(t / kStages) & 1u);
-          issue_tile(t + kStages, stage);
-        }
       }
     }
   } else {
@@ -209,78 +215,74 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_c
     const bool valid = tl < wk.q_count;
     const int q_pos = wk.q_pos0 + tl;
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    uint8_t* prow = smem + (p_s - sbase) + gi * kPTile + row * 128;
 
-    float m = -INFINITY, l = 0.f;
-    uint32_t ph_s = 0, ph_pv = 0;
+    float ref = -INFINITY, l = 0.f;                 // what the row's weights are relative to, in units of log 2
 
     for (int t = 0; t < ntiles; ++t) {
-      mbar_wait(s_full(gi), ph_s);
-      ph_s ^= 1u;
+      const int b = t & 1;
+      mbar_wait(s_full(gi, b), static_cast<uint32_t>(t >> 1) & 1u);
       tc_fence_after();
       uint32_t s0[32], s1[32];
-      tmem_ld_32x32(tm_S[gi] + lane_off, s0);
-      tmem_ld_32x32(tm_S[gi] + lane_off + 32, s1);
+      tmem_ld_32x32(tm_S(gi, b) + lane_off, s0);
+      tmem_ld_32x32(tm_S(gi, b) + lane_off + 32, s1);
       tmem_ld_wait();
       const int kv0 = t * kKvTile;
-      const bool edge = kv0 + kKvTile - 1 > q_pos || !valid;     // tile reaches past this row's position: mask
-      float mx = -INFINITY;
+      if (kv0 + kKvTile - 1 > q_pos || !valid) {     // tile reaches past this row's position: mask
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        float a = __uint_as_float(s0[c]), b = __uint_as_float(s1[c]);
-        if (edge && (kv0 + c > q_pos || !valid)) a = -INFINITY;
-        if (edge && (kv0 + 32 + c > q_pos || !valid)) b = -INFINITY;
-        s0[c] = __float_as_uint(a);
-        s1[c] = __float_as_uint(b);
-        mx = fmaxf(mx, fmaxf(a, b));
+        for (int c = 0; c < 32; ++c) {
+          if (kv0 + c > q_pos || !valid) s0[c] = 0xff800000u;
+          if (kv0 + 32 + c > q_pos || !valid) s1[c] = 0xff800000u;
+        }
       }
-      const float mn = fmaxf(m, mx * scale_log2);
-      const float mu = mn == -INFINITY ? 0.f : mn;
-      const float alpha = exp2f(m - mu);            // m = -inf -> 0
-      m = mn;
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 32; c += 2)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          mx[k] = fmaxf(mx[k], __uint_as_float(s0[c + k]));
+          mx[2 + k] = fmaxf(mx[2 + k], __uint_as_float(s1[c + k]));
+        }
+      const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
+      float alpha = 1.f;
+      if (top > ref) {
+        alpha = exp2_ftz(ref - (top + kSlack));     // ref = -inf -> 0
+        ref = top + kSlack;
+      }
+      const float mu = ref == -INFINITY ? 0.f : ref;
+      auto weight = [&](uint32_t u) { return exp2_ftz(fmaf(__uint_as_float(u), scale_log2, -mu)); };
       float ps = 0.f;
       uint32_t pk[32];
 #pragma unroll
       for (int c = 0; c < 32; c += 2) {
-        const float p0 = exp2f(__uint_as_float(s0[c]) * scale_log2 - mu), p1 = exp2f(__uint_as_float(s0[c + 1]) * scale_log2 - mu);
-        const float p2 = exp2f(__uint_as_float(s1[c]) * scale_log2 - mu), p3 = exp2f(__uint_as_float(s1[c + 1]) * scale_log2 - mu);
+        const float p0 = weight(s0[c]), p1 = weight(s0[c + 1]), p2 = weight(s1[c]), p3 = weight(s1[c + 1]);
         ps += (p0 + p1) + (p2 + p3);
         pk[c >> 1] = pack_bf16x2(p0, p1);
         pk[16 + (c >> 1)] = pack_bf16x2(p2, p3);
       }
       l = l * alpha + ps;
-      // the running output lives in TMEM (PV_i accumulates over the tiles): once the previous tile's P V has landed,
-      // rescale it to this tile's reference maximum — only when some row of the warp actually moved its maximum
-      if (t > 0) {
-        mbar_wait(pv_full(gi), ph_pv);
-        ph_pv ^= 1u;
+      // P in place of the scores: what read this buffer's last P went ahead of them.  The running output lives in TMEM too (PV_i
+      // accumulates over the tiles): where some row of the warp took a new reference, it is rescaled once the previous tile's P V has landed
+      tmem_st_32x32(tm_S(gi, b) + lane_off, pk);
+      if (t > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+        mbar_wait(pv_full(gi, b ^ 1), static_cast<uint32_t>((t - 1) >> 1) & 1u);
         tc_fence_after();
-        if (__any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll
-          for (int c0 = 0; c0 < kD; c0 += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(tm_PV[gi] + lane_off + c0, v);
-            tmem_ld_wait();
+        for (int c0 = 0; c0 < kD; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld_32x32(tm_PV[gi] + lane_off + c0, v);
+          tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * alpha);
-            tmem_st_32x32(tm_PV[gi] + lane_off + c0, v);
-          }
-          tmem_st_wait();
+          for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * alpha);
+          tmem_st_32x32(tm_PV[gi] + lane_off + c0, v);
         }
       }
-      // P row -> smem, K-major 128B-swizzled: logical 16-byte chunk ch lands at ch ^ (row & 7)
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        const uint4 val = make_uint4(pk[ch * 4], pk[ch * 4 + 1], pk[ch * 4 + 2], pk[ch * 4 + 3]);
-        *reinterpret_cast<uint4*>(prow + ((ch ^ (row & 7)) << 4)) = val;
-      }
-      fence_proxy_async();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_ready(gi));
+      if (lane == 0) mbar_arrive(p_ready(gi, b));
     }
     // the finished output
-    mbar_wait(pv_full(gi), ph_pv);
+    mbar_wait(pv_full(gi, (ntiles - 1) & 1), static_cast<uint32_t>((ntiles - 1) >> 1) & 1u);
     tc_fence_after();
     const float inv = l > 0.f ? 1.f / l : 0.f;
     __nv_bfloat16* dst = out + static_cast<size_t>(wk.q_tok0 + tl) * ldo + head * kD;

@@ -8,20 +8,22 @@
 // A CTA owns 256 query tokens of one head as two 128-row tiles that share every 64-key tile.  One thread loads (TMA, 128-byte
 // swizzle, keys and values in rings of their own), one issues every tcgen05.mma:
 //   S_i = Q_i K^T    M = 128, N = 64; two buffers per tile in TMEM, so that the next scores are formed under this softmax
-//   O_i += P_i V     M = 128, N = 128; P_i from shared memory as the softmax warps wrote it, V in place as an MN-major operand
+//   O_i += P_i V     M = 128, N = 128; P_i in TMEM, where the softmax warps wrote it over its scores, V in place as an MN-major operand
 // Two groups of four softmax warps (thread = row) work in fp32 with base-2 exponentials and rescale O_i in TMEM only when a row
-// of the warp moved its maximum.  Key tiles outside a row tile's triangle or window are skipped for that tile.  Rows behind a
+// of the warp took a new reference (kSlack).  Key tiles outside a row tile's triangle or window are skipped for that tile.  Rows behind a
 // sequence's end belong to the next one: their keys are masked and their values cleared, so that nothing of another sequence
 // can reach a result.  A masked key has weight 0, which a product turns into NaN where its value is infinite or NaN: a row that
 // comes out not finite looks for such a key and is then formed again, key by key.  Every wait has a limit; a CTA that gives up sets an error mark and still meets at the end.
 //
 // With keys and values per head (window_prompt_prep gathers them from the cache): sequences of 455, 1365 and 2275 tokens, 16 query
-// and 4 key heads, cap: 291 us on mma.sync -> 119.
+// and 4 key heads, cap: 291 us on mma.sync -> 53.
 //
-// What bounds it: the chain scores, softmax, weights, sums inside the one CTA an SM holds; the tensor pipe is active 28 % of the
-// time, the exponentials' unit 17 % (profiles/prompt_kernels_ncu.md).  16 heads, 192 + 128 dimensions with values in two terms, sequences
-// of 455, 1365 and 2275 tokens: 111 us (52 GFLOP), with the product that rebuilds keys and values and the gather of the latents
-// 166; the latent-space kernel on mma.sync took 883, with its two per-head products 1109.
+// What bounds it, in cycles of a key tile (of both row tiles): the products with 192 dimensions a head and two terms, 2100 of 3200 (scores of 64
+// columns are held up by their operands in shared memory); under a cap the exponentials' unit, three a score, 3100 of 3500; else
+// half and half, with what the barriers between them cost.  The longest CTA has 36 of the tiles.  16 heads, 192 + 128 dimensions with
+// values in two terms, sequences of 455, 1365 and 2275 tokens: 73 us (52 GFLOP); the latent-space kernel on mma.sync took 883, with its two
+// per-head products 1109.  Before P moved to TMEM (which left shared memory for a second buffer of second terms), rescaling took a slack and four
+// products went out at a time: 90, under the cap 60; of that 3 were the rescaling's, 9 and 2 P's and the buffer's, 5 and 2 the issue's.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -42,12 +44,15 @@ namespace {
 typedef __nv_bfloat16 bf16;
 constexpr int kRows = 128, kKeys = 64, kD = 128;     // rows of a query tile, keys of a tile, value dimensions
 constexpr int kQSlab = kRows * 128, kKSlab = kKeys * 128;   // bytes of 64 columns
-constexpr int kVTile = 2 * kKSlab, kPTile = kRows * 128;
+constexpr int kVTile = 2 * kKSlab;
 constexpr int kThreads = 320;                        // warp 0: loads, warps 1-4 and 5-8: rows of tile 0 and 1, warp 9: products
 constexpr int kWaitLimit = 1 << 22;
+// Weights are relative to 2^kSlack times the row's largest so far when that was last taken: none is above 1, and sums in TMEM are
+// scaled again only behind a score that is larger by more than that, which after a row's first keys hardly any is.
+constexpr float kSlack = 8.f;
 template <int NS>
-constexpr int smem_bytes() { return 1024 + 2 * NS * kQSlab + 2 * NS * kKSlab + 2 * kVTile + 2 * kPTile + (NS == 3 ? kVTile : 0) + 256; }
-static_assert(smem_bytes<3>() <= 227 * 1024, "one buffer of the values' second terms is what fits");
+constexpr int smem_bytes() { return 1024 + 2 * NS * kQSlab + 2 * NS * kKSlab + 2 * (NS == 3 ? 2 : 1) * kVTile + 256; }
+static_assert(smem_bytes<3>() <= 227 * 1024, "");
 
 __device__ __forceinline__ uint32_t idesc_bf16(uint32_t m, uint32_t n, uint32_t b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
@@ -60,13 +65,6 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr, uint32_t lbo, uint
 __device__ __forceinline__ bool wait_limited(uint32_t bar, uint32_t parity) { return mbar_wait_limited(bar, parity, kWaitLimit); }
 // ... by a whole warp: whether all lanes saw the phase end
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_limited(bar, parity)); }
-
-// (From 2^-126 to 1, where weights and rescaling factors lie, the same bits as exp2f for every argument; below, 0.)
-__device__ __forceinline__ float exp2_ftz(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 // A row that came out not finite: where a key that it masks but its tiles hold ([begin, end)) has a value that is not finite, the
 // row is formed again from the keys it sees and from no other (a thread; what it sees itself decides otherwise).
@@ -130,25 +128,26 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint8_t* smem = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t q_s = sbase;                               // [tile][slab]
   const uint32_t k_s = q_s + 2 * NS * kQSlab;               // [stage][slab]
-  const uint32_t v_s = k_s + 2 * NS * kKSlab;               // [stage][half]
-  const uint32_t p_s = v_s + 2 * kVTile;                    // [tile]
-  const uint32_t v2_s = p_s + 2 * kPTile;                   // the values' second terms, one tile
-  const uint32_t bars = v2_s + (LO ? kVTile : 0);
+  constexpr int kVStage = (LO ? 2 : 1) * kVTile;
+  const uint32_t v_s = k_s + 2 * NS * kKSlab;               // [stage][term][half]
+  const uint32_t bars = v_s + 2 * kVStage;
   auto k_full = [&](int s) { return bars + 8u * s; };
   auto k_empty = [&](int s) { return bars + 8u * (2 + s); };
   auto v_full = [&](int s) { return bars + 8u * (4 + s); };
   auto v_empty = [&](int s) { return bars + 8u * (6 + s); };
   auto s_full = [&](int i, int b) { return bars + 8u * (8 + 2 * i + b); };
-  auto p_ready = [&](int i) { return bars + 8u * (12 + i); };     // 4 warps: P_i written, S_i read, O_i rescaled
-  auto pv_full = [&](int i) { return bars + 8u * (14 + i); };
-  const uint32_t q_bar = bars + 8u * 16, v2_full = bars + 8u * 17, v2_empty = bars + 8u * 18, tmem_slot = bars + 8u * 19;
+  // Of every other tile each, as the scores': a warp is up to two tiles ahead of the slowest one of its group.
+  auto p_ready = [&](int i, int b) { return bars + 8u * (12 + 2 * i + b); };     // 4 warps: S_i read, P_i in its place, O_i rescaled
+  auto pv_full = [&](int i, int b) { return bars + 8u * (16 + 2 * i + b); };
+  const uint32_t q_bar = bars + 8u * 20, tmem_slot = bars + 8u * 21;
   const int warp = warp_number(), lane = threadIdx.x & 31;
 
   if (warp == 0) {
     if (lane == 0) {
       for (int s = 0; s < 2; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
-      for (int i = 0; i < 2; ++i) { mbar_init(s_full(i, 0), 1); mbar_init(s_full(i, 1), 1); mbar_init(p_ready(i), 4); mbar_init(pv_full(i), 1); }
-      mbar_init(q_bar, 1); mbar_init(v2_full, 1); mbar_init(v2_empty, 1);
+      for (int i = 0; i < 2; ++i)
+        for (int b = 0; b < 2; ++b) { mbar_init(s_full(i, b), 1); mbar_init(p_ready(i, b), 4); mbar_init(pv_full(i, b), 1); }
+      mbar_init(q_bar, 1);
       fence_mbar_init();
     }
     __syncwarp();
@@ -208,7 +207,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int i = 0; i < tiles; ++i)
           for (int s = 0; s < NS; ++s)
             if (one) tma_load_2d(q_s + (i * NS + s) * kQSlab, s < 2 ? &tm_q : &tm_q2, q_bar, s < 2 ? head * a.q_step + 64 * s : head * 64, tok0 + q0 + i * kRows, kEvictNormal);
-        int nk = 0, nv = 0, nl = 0;      // tiles of keys, values and second terms on their way
+        int nk = 0, nv = 0;      // tiles of keys and values on their way
         auto keys = [&] {
           const int st = nk & 1;
           if (!warp_wait(k_empty(st), ((nk >> 1) & 1) ^ 1u)) return false;
@@ -219,35 +218,30 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           ++nk;
           return true;
         };
-        if (LO) ok = keys();
+        ok = keys();
         for (int t = t_begin; ok && t < t_end; ++t) {
-          // with one buffer of second terms that wait is the long one: the next keys go ahead of it
-          if ((!LO || t + 1 < t_end) && !(ok = keys())) break;
+          if (t + 1 < t_end && !(ok = keys())) break;      // their product goes ahead of this tile's values
           const int st = nv & 1, row = tok0 + t * kKeys;
           if (!(ok = warp_wait(v_empty(st), ((nv >> 1) & 1) ^ 1u))) break;
-          if (one) mbar_arrive_expect_tx(v_full(st), kVTile);
+          if (one) mbar_arrive_expect_tx(v_full(st), kVStage);
           for (int s = 0; s < 2; ++s)
-            if (one) tma_load_2d(v_s + st * kVTile + s * kKSlab, &tm_kv, v_full(st), a.v_off + kvh * a.v_step + 64 * s, row, kEvictLast);
-          ++nv;
-          if constexpr (LO) {
-            if (!(ok = warp_wait(v2_empty, (nl & 1) ^ 1u))) break;
-            if (one) mbar_arrive_expect_tx(v2_full, kVTile);
+            if (one) tma_load_2d(v_s + st * kVStage + s * kKSlab, &tm_kv, v_full(st), a.v_off + kvh * a.v_step + 64 * s, row, kEvictLast);
+          if constexpr (LO)
             for (int s = 0; s < 2; ++s)
-              if (one) tma_load_2d(v2_s + s * kKSlab, &tm_v2, v2_full, head * kD + 64 * s, row, kEvictLast);
-            ++nl;
-          }
+              if (one) tma_load_2d(v_s + st * kVStage + kVTile + s * kKSlab, &tm_v2, v_full(st), head * kD + 64 * s, row, kEvictLast);
+          ++nv;
         }
         // the copies in flight land before the CTA ends, also where it gives up
         warp_wait(q_bar, 0);
         for (int j = max(0, nk - 2); j < nk; ++j) warp_wait(k_full(j & 1), (j >> 1) & 1);
         for (int j = max(0, nv - 2); j < nv; ++j) warp_wait(v_full(j & 1), (j >> 1) & 1);
-        if (nl > 0) warp_wait(v2_full, (nl - 1) & 1);
       }
     } else if (warp == 9) {
       {
         const bool one = elect_one();
+        // a product takes the tensor pipe 32 to 64 cycles: they are issued four at a time, with the descriptors that the loop needs at hand
         const uint32_t id_s = idesc_bf16(kRows, kKeys, 0), id_o = idesc_bf16(kRows, kD, 1);
-        uint32_t ph_p[2] = {0, 0};
+        const uint64_t q_d = desc_sw128(q_s, 16, 1024), k_d = desc_sw128(k_s, 16, 1024), v_d = desc_sw128(v_s, kKSlab, 1024);
         auto scores = [&](int t) {
           const int it = t - t_begin, st = it & 1;
           if (!warp_wait(k_full(st), (it >> 1) & 1)) return false;
@@ -255,11 +249,11 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (!active(i, t)) continue;
+            if (one) {
 #pragma unroll
-            for (int k = 0; k < 4 * NS; ++k)
-              if (one) umma_bf16(tm_s(i, t & 1), desc_sw128(q_s + (i * NS + (k >> 2)) * kQSlab + (k & 3) * 32, 16, 1024),
-                        desc_sw128(k_s + (st * NS + (k >> 2)) * kKSlab + (k & 3) * 32, 16, 1024), id_s, k > 0 ? 1u : 0u);
-            if (one) umma_commit(s_full(i, t & 1));
+              for (int s = 0; s < NS; ++s) umma_bf16_k64(tm_s(i, t & 1), q_d + (i * NS + s) * (kQSlab >> 4), k_d + (st * NS + s) * (kKSlab >> 4), id_s, s > 0 ? 1u : 0u);
+              umma_commit(s_full(i, t & 1));
+            }
           }
           if (one) umma_commit(k_empty(st));
           __syncwarp();
@@ -274,26 +268,15 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (!active(i, t)) continue;
-            if (!(ok = warp_wait(p_ready(i), ph_p[i]))) break;
-            ph_p[i] ^= 1u;
+            if (!(ok = warp_wait(p_ready(i, t & 1), ((t - first[i]) >> 1) & 1))) break;
             tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < kKeys / 16; ++k)
-              if (one) umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v_s + st * kVTile + k * 2048, kKSlab, 1024), id_o,
-                        (t > first[i] || k > 0) ? 1u : 0u);
-            if constexpr (LO) {
-              if (!(ok = warp_wait(v2_full, it & 1))) break;
-              tc_fence_after();
-#pragma unroll
-              for (int k = 0; k < kKeys / 16; ++k)
-                if (one) umma_bf16(tm_o(i), desc_sw128(p_s + i * kPTile + k * 32, 16, 1024), desc_sw128(v2_s + k * 2048, kKSlab, 1024), id_o, 1u);
+            if (one) {
+              umma_bf16_tmem_k64(tm_o(i), tm_s(i, t & 1), v_d + st * (kVStage >> 4), id_o, t > first[i] ? 1u : 0u);
+              if (LO) umma_bf16_tmem_k64(tm_o(i), tm_s(i, t & 1), v_d + st * (kVStage >> 4) + (kVTile >> 4), id_o, 1u);
+              umma_commit(pv_full(i, t & 1));
             }
-            if (one) umma_commit(pv_full(i));
           }
-          if (one) {
-            umma_commit(v_empty(st));
-            if constexpr (LO) umma_commit(v2_empty);
-          }
+          if (one) umma_commit(v_empty(st));
           __syncwarp();
         }
       }
@@ -302,16 +285,14 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const bool valid = p < n;
       const int lo = max(0, p - a.window + 1);
       const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-      uint8_t* prow = smem + (p_s - sbase) + gi * kPTile + row * 128;
-      float m = -INFINITY, l = 0.f;
-      uint32_t ph_s[2] = {0, 0}, ph_pv = 0;
+      float ref = -INFINITY, l = 0.f;   // what the row's weights are relative to, in units of log 2
       const float mul = CAP ? 1.0f : a.scale * 1.4426950408889634f;
-      const float pre = CAP ? 2.0f * a.scale / a.softcap : 0.f, cap2 = a.softcap * 1.4426950408889634f;
-      auto capped = [&](uint32_t u) { return __float_as_uint(cap2 * (1.0f - __fdividef(2.0f, __expf(__uint_as_float(u) * pre) + 1.0f))); };
+      // tanh x = 1 - 2 / (e^2x + 1)
+      const float pre = CAP ? 2.0f * 1.4426950408889634f * a.scale / a.softcap : 0.f, cap2 = a.softcap * 1.4426950408889634f;
+      auto capped = [&](uint32_t u) { return __float_as_uint(fmaf(-2.0f * cap2, rcp_ftz(exp2_ftz(__uint_as_float(u) * pre) + 1.0f), cap2)); };
       for (int t = first[gi]; ok && t <= last[gi]; ++t) {
         const int b = t & 1, kv0 = t * kKeys;
-        if (!__all_sync(0xffffffffu, wait_limited(s_full(gi, b), b ? ph_s[1] : ph_s[0]))) { ok = false; break; }
-        if (b) ph_s[1] ^= 1u; else ph_s[0] ^= 1u;
+        if (!__all_sync(0xffffffffu, wait_limited(s_full(gi, b), ((t - first[gi]) >> 1) & 1))) { ok = false; break; }
         tc_fence_after();
         uint32_t s0[32], s1[32];
         tmem_ld_32x32(tm_s(gi, b) + lane_off, s0);
@@ -330,7 +311,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!valid || j1 > p || j1 < lo) s1[c] = 0xff800000u;
           }
         }
-        float mx[4] = {m, m, m, m};
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int c = 0; c < 32; c += 2)
 #pragma unroll
@@ -338,10 +319,14 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mx[k] = fmaxf(mx[k], __uint_as_float(s0[c + k]));
             mx[2 + k] = fmaxf(mx[2 + k], __uint_as_float(s1[c + k]));
           }
-        const float mn = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), mu = mn == -INFINITY ? 0.f : mn * mul;
-        const float alpha = exp2_ftz(fmaf(m, mul, -mu));
+        const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mul;
+        float alpha = 1.f;
+        if (top > ref) {
+          alpha = exp2_ftz(ref - (top + kSlack));
+          ref = top + kSlack;
+        }
+        const float mu = ref == -INFINITY ? 0.f : ref;
         auto weight = [&](uint32_t u) { return exp2_ftz(fmaf(__uint_as_float(u), mul, -mu)); };
-        m = mn;
         float ps = 0.f;
         uint32_t pk[32];
 #pragma unroll
@@ -355,54 +340,48 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           pk[16 + (c >> 1)] = a1;
         }
         l = fmaf(l, alpha, ps);
-        if (t > first[gi]) {
-          if (!__all_sync(0xffffffffu, wait_limited(pv_full(gi), ph_pv))) { ok = false; break; }
-          ph_pv ^= 1u;
+        // P in place of the scores; the products in front of it may still be under way, those of this buffer's last P are not: the scores came behind them
+        tmem_st_32x32(tm_s(gi, b) + lane_off, pk);
+        if (t > first[gi] && __any_sync(0xffffffffu, alpha != 1.0f)) {
+          if (!__all_sync(0xffffffffu, wait_limited(pv_full(gi, b ^ 1), ((t - first[gi] - 1) >> 1) & 1))) { ok = false; break; }
           tc_fence_after();
-          if (__any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll
-            for (int c0 = 0; c0 < kD; c0 += 32) {
-              uint32_t v[32];
-              tmem_ld_32x32(tm_o(gi) + lane_off + c0, v);
-              tmem_ld_wait();
+          for (int c0 = 0; c0 < kD; c0 += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(tm_o(gi) + lane_off + c0, v);
+            tmem_ld_wait();
 #pragma unroll
-              for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * alpha);
-              tmem_st_32x32(tm_o(gi) + lane_off + c0, v);
-            }
-            tmem_st_wait();
+            for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * alpha);
+            tmem_st_32x32(tm_o(gi) + lane_off + c0, v);
           }
         }
-        // P row -> shared memory, K-major, 128B swizzle: 16-byte piece c lands at c ^ (row & 7)
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
+        tmem_st_wait();
         if (kv0 + kKeys > n && (gi == 0 || !active(0, t))) {
           // values behind the sequence's end: cleared before the first product that reads the tile (that of row tile 0, where it is active)
           const int it = t - t_begin;
-          if (!__all_sync(0xffffffffu, wait_limited(v_full(it & 1), (it >> 1) & 1) && (!LO || wait_limited(v2_full, it & 1)))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, wait_limited(v_full(it & 1), (it >> 1) & 1))) { ok = false; break; }
           const int r = row & 63;
           if (kv0 + r >= n) {
-            uint4* d = reinterpret_cast<uint4*>(smem + (v_s - sbase) + (it & 1) * kVTile + (row >> 6) * kKSlab + r * 128);
-            uint4* d2 = reinterpret_cast<uint4*>(smem + (v2_s - sbase) + (row >> 6) * kKSlab + r * 128);
+            uint4* d = reinterpret_cast<uint4*>(smem + (v_s - sbase) + (it & 1) * kVStage + (row >> 6) * kKSlab + r * 128);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
               d[c] = make_uint4(0, 0, 0, 0);
-              if (LO) d2[c] = make_uint4(0, 0, 0, 0);
+              if (LO) d[kVTile / 16 + c] = make_uint4(0, 0, 0, 0);
             }
           }
+          fence_proxy_async();
         }
-        fence_proxy_async();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready(gi));
+        if (lane == 0) mbar_arrive(p_ready(gi, b));
       }
-      if (ok && last[gi] >= 0) ok = __all_sync(0xffffffffu, wait_limited(pv_full(gi), ph_pv));
+      if (ok && last[gi] >= 0) ok = __all_sync(0xffffffffu, wait_limited(pv_full(gi, last[gi] & 1), ((last[gi] - first[gi]) >> 1) & 1));
       if (ok && last[gi] >= 0) {
         tc_fence_after();
         bool finite = true;
         float inv = l > 0.f ? 1.f / l : 0.f;
         if (a.sink) {
-          const float sk = a.sink[head] * 1.4426950408889634f, ml = m * mul, mm = fmaxf(ml, sk), back = exp2f(ml - mm);
+          const float sk = a.sink[head] * 1.4426950408889634f, mm = fmaxf(ref, sk), back = exp2f(ref - mm);
           inv = back / fmaf(l, back, exp2f(sk - mm));
         }
         const long long tok = tok0 + p;

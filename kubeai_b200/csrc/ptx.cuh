@@ -315,4 +315,43 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// A 64-wide step of K with A in TMEM (rows are lanes, a column holds two neighbouring entries of a row: 32 columns) and B 128-byte swizzled
+// tiles of 128-byte rows that run along K: four products, eight columns and sixteen rows apart.
+__device__ __forceinline__ void umma_bf16_tmem_k64(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, t;\n"
+      ".reg .b32 a;\n"
+      ".reg .b64 b;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.eq.b32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "add.u32 a, %1, 8;\n"
+      "add.u64 b, %2, 128;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
+      "add.u32 a, %1, 16;\n"
+      "add.u64 b, %2, 256;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
+      "add.u32 a, %1, 24;\n"
+      "add.u64 b, %2, 384;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// 2^x of softmax weights: from 2^-126 to 1, where weights and rescaling factors lie, the same bits as exp2f for every argument; below, 0.
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// 1 / x for x from 1 on, an approximation good to a unit in the last place; 0 from 2^126 on.
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 }  // namespace b200

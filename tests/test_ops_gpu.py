@@ -289,3 +289,28 @@ def test_paged_attention_prefill_tensor_core(case, Hkv):
         want = O.attention(q[L - n:], k, v, torch.arange(L - n, L), 128 ** -0.5).reshape(n, Hq * 128)
         t0 = spans[i][0]
         close(got[t0:t0 + n], want, atol=4e-3, what=f"tensor-core prefill attn seq {i} (ctx {L}, new {n})")
+
+
+@pytest.mark.parametrize("seq_len,new", [(1, 1), (63, 63), (65, 64), (128, 64), (129, 2), (321, 100), (700, 700)])
+@pytest.mark.parametrize("factor", [16, 256])
+def test_prefill_tensor_core_with_scores_that_leave_the_reference_behind(seq_len, new, factor):
+    """Queries that spread a row's scores over hundreds of powers of two: the weights' reference moves, and the output is scaled again, at any
+    key tile.  bf16 has eight significant bits: a weight rounds by 2^-8 of itself at most, the sum of the weights does not, the output once
+    more by 2^-8."""
+    from kubeai_b200 import ops
+    Hq, Hkv = 4, 1
+    kv, btab, seqs = _paged_setup([seq_len], None, Hq, Hkv, seed=seq_len, nblocks=(seq_len + 15) // 16 + 3)
+    row, q, k, v, _ = seqs[0]
+    rows = row[seq_len - new:].clone()
+    rows[:, :Hq * 128] *= factor                 # a power of two: exact
+    work = [[j, min(64, new - j), seq_len - new + j, 0] for j in range(0, new, 64)]
+    got = ops.paged_attn_prefill_tc(rows, kv, btab, torch.tensor(work, dtype=torch.int32).cuda(), Hq, Hkv)
+    torch.cuda.synchronize()
+    qf = (q[seq_len - new:] * factor).double()
+    s = torch.einsum("nhd,ld->hnl", qf, k[:, 0].double()) * 128 ** -0.5
+    s.masked_fill_(torch.arange(seq_len)[None, :] > torch.arange(seq_len - new, seq_len)[:, None], float("-inf"))
+    want = torch.einsum("hnl,ld->nhd", s.softmax(-1), v[:, 0].double()).reshape(new, Hq * 128)
+    err = (got.double().cpu() - want).abs().max().item()
+    # the scores' own fp32 sums of 128 products add 2^-24 of 128 largest products at most, each e-fold of it to the weights
+    bound = 2 * 2.0 ** -8 * float(v.abs().max()) + 2.0 ** -23 * float(s[s.isfinite()].abs().max()) * 12 * float(v.abs().max())
+    assert torch.isfinite(got.float()).all() and err <= bound, (err, bound)

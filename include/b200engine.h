@@ -378,8 +378,9 @@ int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, i
  * B200_RULE_SINGLE_STEP {heads times sequences, state rows, value columns, delta rule, SMs}: single tokens as a pass over the states.
  * B200_RULE_LATENT_ROWS {longest row, tokens}: latent rows stay in registers between their sum and their norm.
  * B200_RULE_TILES {tokens, N, K}: a product that csrc/linear_stream.cu or csrc/linear_cluster.cu could take goes to whole tiles all the same.
- * B200_RULE_TILE_ROWS, B200_RULE_TILE_PARTS {rows, N, K, CTA pairs, K may be cut}: rows of a whole tile, and pieces K is cut into (numbers). */
-enum { B200_RULE_PICKED_ALONE = 0, B200_RULE_KEY_LANES = 1, B200_RULE_STREAM = 2, B200_RULE_CLUSTER = 3, B200_RULE_SEGMENTS = 4, B200_RULE_ROW_REGISTERS = 5, B200_RULE_ROW_BLOCKS = 6, B200_RULE_SINGLE_STEP = 7, B200_RULE_LATENT_ROWS = 8, B200_RULE_TILES = 9, B200_RULE_TILE_ROWS = 10, B200_RULE_TILE_PARTS = 11 };
+ * B200_RULE_TILE_ROWS, B200_RULE_TILE_PARTS {rows, N, K, CTA pairs, K may be cut}: rows of a whole tile, and pieces K is cut into (numbers).
+ * B200_RULE_DELTA_AHEAD {CTAs a sequence, sequences, tokens, longest, SMs}: delta-rule chunks whose scores are formed a chunk ahead by warps of their own. */
+enum { B200_RULE_PICKED_ALONE = 0, B200_RULE_KEY_LANES = 1, B200_RULE_STREAM = 2, B200_RULE_CLUSTER = 3, B200_RULE_SEGMENTS = 4, B200_RULE_ROW_REGISTERS = 5, B200_RULE_ROW_BLOCKS = 6, B200_RULE_SINGLE_STEP = 7, B200_RULE_LATENT_ROWS = 8, B200_RULE_TILES = 9, B200_RULE_TILE_ROWS = 10, B200_RULE_TILE_PARTS = 11, B200_RULE_DELTA_AHEAD = 12 };
 int b200_rule_query(int32_t rule, const int32_t* v, int32_t n);
 /* Debug: subsequent pair-GEMM launches write 8 clock64() phase stamps per CTA into trace_dev (int64[grid][8]);
  * NULL turns it off.  Stamps: 0 entry, 1 after prologue, 2 first tile accumulated, 3 main loop + partial stores

@@ -321,6 +321,7 @@ int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_ROW_BLOCKS && n == 5) return rules::row_blocks_pay(v[0], v[1], v[2], v[3], v[4] != 0);
   if (v && rule == B200_RULE_SINGLE_STEP && n == 5) return rules::single_step_pays(v[0], v[1], v[2], v[3] != 0, v[4]);
   if (v && rule == B200_RULE_LATENT_ROWS && n == 2) return rules::latent_rows_held(v[0], v[1]);
+  if (v && rule == B200_RULE_DELTA_AHEAD && n == 5) return rules::delta_scores_ahead(v[0], v[1], v[2], v[3], v[4]);
   if (v && rule == B200_RULE_TILES && n == 3) return rules::tiles_ahead(v[0], v[1], v[2]);
   if (v && (rule == B200_RULE_TILE_ROWS || rule == B200_RULE_TILE_PARTS) && n == 5 && v[0] > 0 && v[1] > 0 && v[2] > 0 && v[3] > 0) {
     int tile, parts;

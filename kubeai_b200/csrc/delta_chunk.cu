@@ -23,11 +23,17 @@
 // 16 tokens per warp and shared through shared memory, already split, as 16 x 16 blocks whose 16-byte halves are swapped in
 // every other group of four rows (ldmatrix then meets no bank conflict).  The next chunk's keys, queries, values and gates
 // are fetched while the current one is worked on.
+//
+// What bounds it: a chain as long as the longest sequence on a CTA a head and 64 columns, tensor cores (mma.sync) two thirds of a chunk.  A sixth of their
+// products and most of the rest of a chunk's time go into A, its inverses and the weighted scores, which need no state: where the longest chain outlasts the
+// SMs' work (rules::delta_scores_ahead), four more warps form them a chunk ahead; the longest sequences' CTAs start first.  16 heads of 128 x 128, 63 to 959
+// tokens in 8 sequences: 229 us -> 162, 1024 tokens in one 211 -> 146, the same bits.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
 
+#include "dispatch_rules.h"
 #include "launch.h"
 #include "mixers.h"
 #include "mma_frag.cuh"
@@ -52,8 +58,13 @@ struct Gates {
   float chi[kQ], clo[kQ], ecum[kQ], wl[kQ], beta[kQ], ea[kQ], ec[kQ], eb[16];
 };
 
-constexpr size_t chunk_smem(int D) {
-  return static_cast<size_t>(3) * kQ * (D + 8) * 2 + static_cast<size_t>(kQ) * kLdV * 2 + 2ull * kBlocks * 3 * kBlock * 2 + 4 * 16 * kLdD * 4 + 2 * sizeof(Gates) + 2 * kQ * 4;
+// How many of each a CTA holds: keys, queries, values, gates; scores with the norms that go with them.  `ahead`: see the kernel.
+__host__ __device__ constexpr int k_bufs(bool ahead) { return ahead ? 3 : 2; }
+__host__ __device__ constexpr int q_bufs(bool ahead) { return ahead ? 3 : 1; }
+__host__ __device__ constexpr int s_bufs(bool ahead) { return ahead ? 2 : 1; }
+constexpr size_t chunk_smem(int D, bool ahead) {
+  return static_cast<size_t>(k_bufs(ahead) + q_bufs(ahead)) * kQ * (D + 8) * 2 + static_cast<size_t>(q_bufs(ahead)) * kQ * kLdV * 2 + s_bufs(ahead) * (2ull * kBlocks * 3 * kBlock * 2 + 2 * kQ * 4) +
+         4 * 16 * kLdD * 4 + k_bufs(ahead) * sizeof(Gates);
 }
 
 __device__ __forceinline__ int block_at(int tb, int jb) { return (tb * (tb + 1) / 2 + jb) * 3 * kBlock; }
@@ -69,28 +80,45 @@ constexpr int kPairs = 6;
 __device__ __forceinline__ constexpr int pair_a(int i) { return i == 0 ? 2 : (i == 1 ? 0 : (i == 2 ? 1 : (i == 3 ? 1 : 0))); }
 __device__ __forceinline__ constexpr int pair_b(int i) { return i == 0 ? 0 : (i == 1 ? 2 : (i == 2 ? 1 : (i == 3 ? 0 : (i == 4 ? 1 : 0)))); }
 
+// The sequence with the z-th most tokens (ties: the first), by a warp: long chains start first, and short ones fill in behind or beside them.  Of more
+// sequences than kSorted the z-th as they come.
+constexpr int kSorted = 64;
+__device__ __forceinline__ int nth_longest(const int* seqs, int nseq, int z) {
+  if (nseq > kSorted) return z;
+  const int lane = threadIdx.x & 31, a = lane < nseq ? seqs[lane * 8 + 1] : -1, b = lane + 32 < nseq ? seqs[(lane + 32) * 8 + 1] : -1;
+  int ra = 0, rb = 0;      // how many come before the lane's two
+  for (int i = 0; i < min(nseq, 32); ++i) {
+    const int va = __shfl_sync(0xffffffffu, a, i), vb = __shfl_sync(0xffffffffu, b, i);
+    ra += (va > a || (va == a && i < lane)) + (vb > a);
+    rb += (va >= b) + (vb > b || (vb == b && i < lane));
+  }
+  const unsigned ma = __ballot_sync(0xffffffffu, lane < nseq && ra == z), mb = __ballot_sync(0xffffffffu, lane + 32 < nseq && rb == z);
+  return ma ? __ffs(ma) - 1 : __ffs(mb) + 31;
+}
+
 // NK: key rows in units of 16, at most (D = a.dim is any multiple of 16 up to 16 NK); FULL: exactly 16 NK rows, which leaves the
-// loops over them without branches
-template <int NK, bool FULL>
-__global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, int sms) {
+// loops over them without branches.  AHEAD: four more warps form the next chunk's A, inverses and weighted scores, which need no state, while the
+// first four work on this one's; a CTA then has its SM to itself.
+template <int NK, bool FULL, bool AHEAD>
+__global__ void __launch_bounds__(AHEAD ? 2 * kThreads : kThreads, AHEAD ? 1 : 2) delta_chunk_kernel(DeltaArgs a, int sms) {
   using namespace frag;
   extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr int NKB = k_bufs(AHEAD), NQB = q_bufs(AHEAD), NSB = s_bufs(AHEAD), kAll = AHEAD ? 2 * kThreads : kThreads;
   const int D = FULL ? 16 * NK : a.dim, P = a.vdim, nk = FULL ? NK : D / 16, LDN = D + 8;
-  bf16* Kbuf = reinterpret_cast<bf16*>(smraw);   // [2][kQ][LDN] keys, this chunk's and the next one's
-  bf16* Qs = Kbuf + 2 * kQ * LDN;                // [kQ][LDN] queries
-  bf16* Vs = Qs + kQ * LDN;                      // [kQ][kLdV] values of the CTA's columns
-  bf16* As = Vs + kQ * kLdV;                     // [kBlocks][3][kBlock]: -A below the diagonal, the inverses of I + A on it
-  bf16* Ms = As + kBlocks * 3 * kBlock;          // the weighted scores of the queries
-  float* diag = reinterpret_cast<float*>(Ms + kBlocks * 3 * kBlock);   // [4][16][kLdD]
-  Gates* gates = reinterpret_cast<Gates*>(diag + 4 * 16 * kLdD);       // [2]
-  float* ik = reinterpret_cast<float*>(gates + 2);   // [kQ] 1 / |k_t|
-  float* iq = ik + kQ;                               // [kQ] q_scale / |q_t|
-  const int seq = blockIdx.z, head = blockIdx.y, p0 = blockIdx.x * kCols;
+  bf16* Kbuf = reinterpret_cast<bf16*>(smraw);   // [NKB][kQ][LDN] keys of chunk i at i % NKB, and so on
+  bf16* Qbuf = Kbuf + NKB * kQ * LDN;            // [NQB][kQ][LDN] queries
+  bf16* Vbuf = Qbuf + NQB * kQ * LDN;            // [NQB][kQ][kLdV] values of the CTA's columns
+  bf16* Abuf = Vbuf + NQB * kQ * kLdV;           // [NSB][kBlocks][3][kBlock]: -A below the diagonal, the inverses of I + A on it
+  bf16* Mbuf = Abuf + NSB * kBlocks * 3 * kBlock;   // [NSB] the weighted scores of the queries
+  float* diag = reinterpret_cast<float*>(Mbuf + NSB * kBlocks * 3 * kBlock);   // [4][16][kLdD]
+  Gates* gates = reinterpret_cast<Gates*>(diag + 4 * 16 * kLdD);       // [NKB]
+  float* ikbuf = reinterpret_cast<float*>(gates + NKB);   // [NSB][2][kQ] 1 / |k_t|, q_scale / |q_t|
+  const int seq = nth_longest(a.seqs, a.nseq, blockIdx.z), head = blockIdx.y, p0 = blockIdx.x * kCols;
   const int tok0 = a.seqs[seq * 8 + 0], n = a.seqs[seq * 8 + 1], pos0 = a.seqs[seq * 8 + 2], slot = a.seqs[seq * 8 + 3];
   // later row blocks have more scores: every other wave of CTAs deals them to the warps in the opposite order, so that the two
   // CTAs of an SM load its four schedulers evenly
   const bool flip = ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) / sms & 1;
-  const int tid = threadIdx.x, lane = tid & 31, w = flip ? 3 - (tid >> 5) : tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, w = flip ? 3 - (tid >> 5 & 3) : tid >> 5 & 3, g = lane >> 2, t4 = lane & 3;
   const bf16* base = static_cast<const bf16*>(a.qkv);
   const int qk0 = head / (a.heads / a.kv_heads) * D;
   const bool live = p0 + 16 * w < P;             // warps past the last value column only help with the scores
@@ -107,7 +135,7 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
         S[k][h][c] = (k < nk && p < P && pos0 > 0) ? Sg[nn * P + p] : 0.f;
       }
   // the piece of a 16-byte row piece grid this thread copies first, and its step to the next one
-  const int npiece = D / 8, t_first = tid / npiece, c_first = tid - t_first * npiece, t_step = kThreads / npiece, c_step = kThreads - t_step * npiece;
+  const int npiece = D / 8, t_first = tid / npiece, c_first = tid - t_first * npiece, t_step = kAll / npiece, c_step = kAll - t_step * npiece;
   // a chunk's rows of one column block, by all threads; rows past the portion become zeros
   auto fetch_rows = [&](bf16* dst, int off, int c0) {
     const bf16* src = base + static_cast<long long>(tok0 + c0) * a.ld + off + qk0;
@@ -121,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
     }
   };
   // the warp's own 16 value columns
-  auto fetch_values = [&](int c0) {
+  auto fetch_values = [&](bf16* Vs, int c0) {
     const int c = 16 * w + 8 * (lane & 1);
     const bf16* src = base + static_cast<long long>(tok0 + c0) * a.ld + a.v_off + head * P + p0 + c;
     for (int t = lane >> 1; t < kQ; t += 16) {
@@ -171,22 +199,10 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
     if (lane < 16) G.eb[lane] = jb < tb ? expf(static_cast<float>(at - from)) : 0.f;
   };
 
-  fetch_rows(Kbuf, a.k_off, 0);
-  fetch_rows(Qs, a.q_off, 0);
-  fetch_values(0);
-  if (w == 0) make_gates(gates[0], 0);
   // the lane's ldmatrix row in a block that is the right operand: its rows are the operand's columns
   const int b_lane = block_pos((lane & 7) + 8 * (lane >> 4), 8 * ((lane >> 3) & 1));
-  int buf = 0;
-  for (int c0 = 0; c0 < n; c0 += kQ, buf ^= 1) {
-    const int q = min(kQ, n - c0);
-    const bf16* Ks = Kbuf + buf * kQ * LDN;
-    const Gates& G = gates[buf];
-    const bool more = c0 + kQ < n;
-    cp_async_wait_all();
-    __syncthreads();   // this chunk's tiles and gates are in place; nobody works on the last chunk any more
-    if (more) fetch_rows(Kbuf + (buf ^ 1) * kQ * LDN, a.k_off, c0 + kQ);
-
+  // what a chunk leaves for the walk over the states: by four warps
+  auto scores = [&](const bf16* Ks, const bf16* Qs, const Gates& G, bf16* As, bf16* Ms, float* ik, float* iq) {
     // ---- A and the weighted query scores of this warp's 16 tokens against the keys of its own and earlier blocks
     {
       float GK[4][2][4], GQ[4][2][4], QQ[2][4];
@@ -319,9 +335,11 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
           v -= __bfloat162float(o);
         }
       }
-      if (w == 0 && more) make_gates(gates[buf ^ 1], c0 + kQ);
     }
-    __syncthreads();
+  };
+  // the walk's step
+  auto step = [&](int c0, const bf16* Ks, const bf16* Qs, const bf16* Vs, const Gates& G, const bf16* As, const bf16* Ms, const float* ik, const float* iq) {
+    const int q = min(kQ, n - c0);
 
     float R[4][2][4], Y[4][2][4];
     if (live) {
@@ -382,10 +400,12 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
 #pragma unroll
           for (int c = 0; c < 4; ++c) S[k][h][c] *= decay;
     }
-    __syncthreads();   // the queries and the values are no longer read
-    if (more) {
-      fetch_rows(Qs, a.q_off, c0 + kQ);
-      fetch_values(c0 + kQ);
+    if constexpr (!AHEAD) {
+      __syncthreads();   // the queries and the values are no longer read
+      if (c0 + kQ < n) {
+        fetch_rows(Qbuf, a.q_off, c0 + kQ);
+        fetch_values(Vbuf, c0 + kQ);
+      }
     }
     if (live) {
       // ---- block by block: the writes U of 16 tokens, then what they change in later right-hand sides, outputs and the state
@@ -472,6 +492,50 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
             }
           }
     }
+  };
+  auto K = [&](int i) { return Kbuf + i % NKB * kQ * LDN; };
+  auto Q = [&](int i) { return Qbuf + i % NQB * kQ * LDN; };
+  auto V = [&](int i) { return Vbuf + i % NQB * kQ * kLdV; };
+  auto A = [&](int i) { return Abuf + i % NSB * kBlocks * 3 * kBlock; };
+  auto M = [&](int i) { return Mbuf + i % NSB * kBlocks * 3 * kBlock; };
+  auto IK = [&](int i) { return ikbuf + i % NSB * 2 * kQ; };
+  if constexpr (AHEAD) {
+    const bool walks = tid < kThreads;
+    auto fetch = [&](int i) {
+      fetch_rows(K(i), a.k_off, i * kQ);
+      fetch_rows(Q(i), a.q_off, i * kQ);
+      if (walks) fetch_values(V(i), i * kQ);
+    };
+    const int chunks = (n + kQ - 1) / kQ;
+    if (chunks > 0) fetch(0);
+    if (!walks && w == 0 && chunks > 0) make_gates(gates[0], 0);
+    for (int i = -1; i < chunks; ++i) {
+      cp_async_wait_all();
+      __syncthreads();   // the scores of chunk i and the tiles and gates of chunk i + 1 are in place; nobody works on chunk i - 1 any more
+      if (i + 2 < chunks) fetch(i + 2);
+      if (walks) {
+        if (i >= 0) step(i * kQ, K(i), Q(i), V(i), gates[i % NKB], A(i), M(i), IK(i), IK(i) + kQ);
+      } else if (i + 1 < chunks) {
+        if (w == 0 && i + 2 < chunks) make_gates(gates[(i + 2) % NKB], (i + 2) * kQ);
+        scores(K(i + 1), Q(i + 1), gates[(i + 1) % NKB], A(i + 1), M(i + 1), IK(i + 1), IK(i + 1) + kQ);
+      }
+    }
+    if (!walks) return;
+  } else {
+    fetch_rows(Kbuf, a.k_off, 0);
+    fetch_rows(Qbuf, a.q_off, 0);
+    fetch_values(Vbuf, 0);
+    if (w == 0) make_gates(gates[0], 0);
+    for (int c0 = 0, i = 0; c0 < n; c0 += kQ, ++i) {
+      const bool more = c0 + kQ < n;
+      cp_async_wait_all();
+      __syncthreads();   // this chunk's tiles and gates are in place; nobody works on the last chunk any more
+      if (more) fetch_rows(K(i + 1), a.k_off, c0 + kQ);
+      scores(K(i), Qbuf, gates[i % NKB], Abuf, Mbuf, ikbuf, ikbuf + kQ);
+      if (w == 0 && more) make_gates(gates[(i + 1) % NKB], c0 + kQ);
+      __syncthreads();
+      step(c0, K(i), Qbuf, Vbuf, gates[i % NKB], Abuf, Mbuf, ikbuf, ikbuf + kQ);
+    }
   }
 #pragma unroll
   for (int k = 0; k < NK; ++k)
@@ -484,14 +548,20 @@ __global__ void __launch_bounds__(kThreads, 2) delta_chunk_kernel(DeltaArgs a, i
       }
 }
 
+template <int NK, bool FULL, bool AHEAD>
+int launch_form(const DeltaArgs& a, dim3 grid, int sms, cudaStream_t st) {
+  static std::atomic<unsigned long long> attr{0};
+  if (!ensure_dynamic_smem(delta_chunk_kernel<NK, FULL, AHEAD>, static_cast<int>(chunk_smem(16 * NK, AHEAD)), &attr)) return -2;
+  delta_chunk_kernel<NK, FULL, AHEAD><<<grid, AHEAD ? 2 * kThreads : kThreads, chunk_smem(a.dim, AHEAD), st>>>(a, sms);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 template <int NK, bool FULL>
 int launch(const DeltaArgs& a, cudaStream_t st) {
-  static std::atomic<unsigned long long> attr{0};
-  if (!ensure_dynamic_smem(delta_chunk_kernel<NK, FULL>, static_cast<int>(chunk_smem(16 * NK)), &attr)) return -2;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  delta_chunk_kernel<NK, FULL><<<dim3((a.vdim + kCols - 1) / kCols, a.heads, a.nseq), kThreads, chunk_smem(a.dim), st>>>(a, sms);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  const dim3 grid((a.vdim + kCols - 1) / kCols, a.heads, a.nseq);
+  if (rules::delta_scores_ahead(grid.x * grid.y, a.nseq, a.T, a.max_rows, sms)) return launch_form<NK, FULL, true>(a, grid, sms, st);
+  return launch_form<NK, FULL, false>(a, grid, sms, st);
 }
 template <int NK>
 int launch(const DeltaArgs& a, cudaStream_t st) { return a.dim == 16 * NK ? launch<NK, true>(a, st) : launch<NK, false>(a, st); }

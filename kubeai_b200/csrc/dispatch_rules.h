@@ -79,6 +79,16 @@ inline bool segments_pay(long long T, int nseq, int longest, int heads, int bloc
   return 4.1 + 4.6 * (T / 256.0 + nseq / 2.0) * heads * blocks / (2.0 * sms) < chain;
 }
 
+// Chunks of the delta rule (delta_chunk.cu): four more warps a CTA form the next chunk's scores, one CTA an SM, or two CTAs of four warps share an SM.  A
+// chain gains what waits left of its SM's tensor pipe; where the SMs' work outlasts the longest chain, two CTAs hide each other's waits as well and without the
+// rest.  us, by itself / ahead, 128 x 128 (CTAs a sequence: twice the heads): 16 heads, 63 to 959 tokens in 8 sequences (work 14.7 chunks an SM, longest 15)
+// 229 / 162, 4 x 1000 and 500 (15.7, 16) 238 / 172, 5 x 777 (13.7, 13) 217 / 244, 8 x 200 (6.3, 4) 82 / 98; 32 heads, the 8 sequences (29.4, 15) 256 / 305,
+// 100 to 2000 in six (20, 32) 440 / 307; 2 x 1000: 4 heads 213 / 148, 37 (148 CTAs) 223 / 172, 40 (17.4, 16) 264 / 299, 74 (32, 16) 283 / 330.  64 and 32 rows
+// the same.  A step of one chunk has nothing ahead.  longest 0: not known.
+inline bool delta_scores_ahead(int ctas, int nseq, int tokens, int longest, int sms) {
+  return tokens > 64 && (static_cast<long long>(ctas) * nseq <= sms || (tokens / 64.0 + nseq / 2.0) * ctas / sms <= (longest + 63) / 64);
+}
+
 // Norms between sublayers (hyper.cu): a row of 256 threads times `pieces` of four columns in registers through both sums, or read from
 // memory again behind each.  Three and four pieces leave an SM two rows at a time: ahead while that holds all rows there are (steps), behind
 // where many follow.  us of 9 launches, again / registers, 4096 wide: 1 row 55 / 42, 148 rows 51 / 41, 444 52 / 52, 900 69 / 74, 4000 196 / 232;

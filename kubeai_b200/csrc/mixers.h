@@ -248,6 +248,7 @@ struct DeltaArgs {
   float* states; const int* seqs; int nseq; int T;
   int heads, kv_heads, dim, vdim;
   float* o;
+  int max_rows = 0;   // most tokens that a sequence brings (0: not known)
 };
 int delta_scan(const DeltaArgs& a, cudaStream_t st);
 // The chunked tensor-core form of the same scan (delta_chunk.cu; same result up to fp32 rounding), for the shapes it takes;

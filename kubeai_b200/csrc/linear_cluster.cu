@@ -222,12 +222,13 @@ int launch(const LinearArgs& a, const Shape& s, cudaStream_t st) {
 }
 
 // Four CTAs a cluster and 64 rows of W put 2048 rows on 128 SMs; a long K with up to 128 tokens has less of X to read with six and
-// 96 rows (at most 22 such clusters run at once, and 33 of four).  us a launch, weights from HBM, whole tiles / here:
+// 96 rows (at most 22 such clusters run at once, and 33 of four).  us a launch, weights from HBM, whole tiles of 256 rows / here:
 //   2048 x 2048   64 tokens 11.1 / 7.2   100 tokens 13.6 / 8.0    256 tokens 14.9 / 11.6
 //   2048 x 4096   64 tokens 13.0 / 10.3  128 tokens 18.0 / 11.8   256 tokens 24.4 / 16.1
 //   2048 x 8192   64 tokens 16.3 / 15.2  128 tokens 21.4 / 17.2   256 tokens 32.1 / 25.3
 //   3072 x 1024   64 tokens  8.4 / 6.6   128 tokens  9.1 / 8.0    256 tokens 10.5 / 12.4
-// From 4096 rows on the whole tiles are as fast or faster: they read X once for 256 rows.  So they are with a long K (rules::cluster_pays).
+// From 4096 rows on those are as fast or faster: they read X once for 256 rows.  So they are with a long K (rules::cluster_pays), and tiles whose
+// rows are chosen for the call are from 129 tokens on (rules::tiles_ahead); a product without a plan for them still comes here.
 bool pick_shape(int T, int N, int K, Shape* s) {
   s->C = 4;
   if (N <= 2112) {

@@ -230,7 +230,7 @@ int pick_tokens(const LinearArgs& a, const LinearPairs& q, cudaStream_t st) {
 //   8192 x 2048:   8 tokens 6.6 / 11.7   32 tokens  9.4 / 12.4   48 tokens 13.2 / 13.4
 //   28672 x 4096:  8 tokens 36.1 / 42.5  16 tokens 39.0 / 43.0, in a second of nothing else 38.5 / 43.5 and 43.7 / 44.0
 // More tokens cost their rows once a CTA and block of its rows, which is what narrow matrices can afford longest.  With a long K the
-// whole tiles win earlier (rules::stream_pays); a product without a plan for them still comes here.
+// whole tiles win earlier (rules::stream_pays, rules::tiles_ahead); a product without a plan for them still comes here.
 bool linear_streams(const LinearArgs& a, const LinearPairs* q) {
   static const int most = [] { const char* e = getenv("B200_LIN_STREAM"); return e ? atoi(e) : 48; }();     // A/B knob: the most rows, 0: none
   const int sms = sm_count();

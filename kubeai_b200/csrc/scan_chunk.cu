@@ -21,7 +21,7 @@
 // y without leaving the registers; the scores C B^T are computed 16 tokens per warp and shared through shared memory.
 //
 // What bounds it: two to four warps a scheduler (registers, shared memory), which stand behind fixed latencies for half of their time; tensor cores
-// (mma.sync) 40 % of the time, issue slots 40 %.  So the terms of a split operand go round over several sums (three products in a row on one sum wait
+// (mma.sync) 40 % of the time, issue slots 31 %.  So the terms of a split operand go round over several sums (three products in a row on one sum wait
 // for each other), a thread's copies step along one column, and in chains and sums the next chunk's keys, values and gates (a chain's queries, once
 // they are read) come in while this one is worked on.  The outputs of a segment, four chunks at most, have three CTAs an SM and one set
 // of tiles instead: 145 us against 174 with two and two (the shape above).  Without all that: a chain 455 us, sums 77, outputs 172; now 330, 57, 145.

@@ -1,5 +1,6 @@
 // Op-level C-ABI entry points (include/b200engine.h "op-level entry points") + error plumbing.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -435,3 +436,19 @@ int b200_op_init_uniform(void* p, uint64_t n, uint32_t seed, float scale, float 
 }
 
 }  // extern "C"
+int b200_op_prompt_attn(const void* q, const void* q2, const void* kv, const void* k2, const void* v2, void* out, int32_t T, int32_t heads, int32_t kv_heads,
+                        const int32_t* seqs, int32_t nseq, int32_t window, float scale, float softcap, const float* sink, void* stream) {
+  if (int rc = require_device()) return rc;
+  if (!q || !kv || !out || !seqs || T < 1 || nseq < 1 || heads < 1 || kv_heads < 1 || window < 0) { set_error("b200_op_prompt_attn: bad arguments"); return B200_ERR_INVALID; }
+  if (ensure_scratch()) { set_error("workspace allocation failed"); return B200_ERR_OOM; }
+  if (int rc = report_mark()) return rc;
+  PromptAttnArgs a = {};
+  a.q = q; a.ldq = heads * 128; a.q_step = 128; a.q2 = q2;
+  a.kv = kv; a.ldkv = kv_heads * 256; a.k_step = a.v_step = 256; a.v_off = 128; a.k2 = k2; a.v2 = v2;
+  a.y = out; a.ldy = heads * 128; a.T = T; a.heads = heads; a.kv_heads = kv_heads;
+  a.window = window > 0 ? window : INT_MAX; a.scale = scale; a.softcap = softcap; a.out_scale = 1.f;
+  a.sink = sink; a.seqs = seqs; a.nseq = nseq; a.error = g_mark;
+  const int rc = prompt_attention(a, static_cast<cudaStream_t>(stream));
+  return rc ? cuda_fail("prompt_attention", rc) : 0;
+}
+

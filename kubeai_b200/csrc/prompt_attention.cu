@@ -10,20 +10,23 @@
 //   S_i = Q_i K^T    M = 128, N = 64; two buffers per tile in TMEM, so that the next scores are formed under this softmax
 //   O_i += P_i V     M = 128, N = 128; P_i in TMEM, where the softmax warps wrote it over its scores, V in place as an MN-major operand
 // Two groups of four softmax warps (thread = row) work in fp32 with base-2 exponentials and rescale O_i in TMEM only when a row
-// of the warp took a new reference (kSlack).  Key tiles outside a row tile's triangle or window are skipped for that tile.  Rows behind a
+// of the warp moved its maximum.  Key tiles outside a row tile's triangle or window are skipped for that tile.  Rows behind a
 // sequence's end belong to the next one: their keys are masked and their values cleared, so that nothing of another sequence
 // can reach a result.  A masked key has weight 0, which a product turns into NaN where its value is infinite or NaN: a row that
 // comes out not finite looks for such a key and is then formed again, key by key.  Every wait has a limit; a CTA that gives up sets an error mark and still meets at the end.
 //
 // With keys and values per head (window_prompt_prep gathers them from the cache): sequences of 455, 1365 and 2275 tokens, 16 query
-// and 4 key heads, cap: 291 us on mma.sync -> 53.
+// and 4 key heads, cap: 291 us on mma.sync -> 101.
 //
 // What bounds it, in cycles of a key tile (of both row tiles): the products with 192 dimensions a head and two terms, 2100 of 3200 (scores of 64
 // columns are held up by their operands in shared memory); under a cap the exponentials' unit, three a score, 3100 of 3500; else
 // half and half, with what the barriers between them cost.  The longest CTA has 36 of the tiles.  16 heads, 192 + 128 dimensions with
-// values in two terms, sequences of 455, 1365 and 2275 tokens: 73 us (52 GFLOP); the latent-space kernel on mma.sync took 883, with its two
-// per-head products 1109.  Before P moved to TMEM (which left shared memory for a second buffer of second terms), rescaling took a slack and four
-// products went out at a time: 90, under the cap 60; of that 3 were the rescaling's, 9 and 2 P's and the buffer's, 5 and 2 the issue's.
+// values in two terms, sequences of 455, 1365 and 2275 tokens: 77 us (52 GFLOP); the latent-space kernel on mma.sync took 883, with its two
+// per-head products 1109.  With P in shared memory, one buffer of second terms and one product a time it
+// took 90 (under a cap, 4096 tokens in eight sequences, 60 for 55 now).
+//
+// Weights are relative to the row's largest score so far, so the largest weight is exactly 1 and its rounding to bf16 costs nothing.  Relative to 2^8 times an
+// older maximum, which saves most of the rescaling (75 us for 77, under the cap 53.6 for 55.3, 39.0 for 42.4 in windows), outputs were off by 2 to 10 % more.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -47,9 +50,6 @@ constexpr int kQSlab = kRows * 128, kKSlab = kKeys * 128;   // bytes of 64 colum
 constexpr int kVTile = 2 * kKSlab;
 constexpr int kThreads = 320;                        // warp 0: loads, warps 1-4 and 5-8: rows of tile 0 and 1, warp 9: products
 constexpr int kWaitLimit = 1 << 22;
-// Weights are relative to 2^kSlack times the row's largest so far when that was last taken: none is above 1, and sums in TMEM are
-// scaled again only behind a score that is larger by more than that, which after a row's first keys hardly any is.
-constexpr float kSlack = 8.f;
 template <int NS>
 constexpr int smem_bytes() { return 1024 + 2 * NS * kQSlab + 2 * NS * kKSlab + 2 * (NS == 3 ? 2 : 1) * kVTile + 256; }
 static_assert(smem_bytes<3>() <= 227 * 1024, "");
@@ -322,8 +322,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mul;
         float alpha = 1.f;
         if (top > ref) {
-          alpha = exp2_ftz(ref - (top + kSlack));
-          ref = top + kSlack;
+          alpha = exp2_ftz(ref - top);
+          ref = top;
         }
         const float mu = ref == -INFINITY ? 0.f : ref;
         auto weight = [&](uint32_t u) { return exp2_ftz(fmaf(__uint_as_float(u), mul, -mu)); };

@@ -167,6 +167,22 @@ def paged_attn_prefill_tc(qkv, kv_layer, block_tables, work, q_heads, kv_heads, 
     return out
 
 
+def prompt_attn(q, kv, lens, scale, q2=None, k2=None, v2=None, window=0, softcap=0.0, sink=None):
+    """Attention of whole prompts of `lens` tokens one behind the other (b200_op_prompt_attn): q [T, heads, 128], kv [T, kv_heads, 256]."""
+    for t in (q, kv, q2, k2, v2):
+        if t is not None:
+            _chk(t)
+    if sink is not None:
+        _chk(sink, torch.float32)
+    T, heads, _ = q.shape
+    assert sum(lens) == T and min(lens) > 0 and kv.shape[0] == T
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    seqs = torch.tensor([[a, n, 0, 0, 0, 0, 0, 0] for a, n in zip(starts, lens)], dtype=torch.int32).to(q.device)
+    out = torch.empty(T, heads, 128, dtype=torch.bfloat16, device=q.device)
+    check(lib().b200_op_prompt_attn(_p(q), _p(q2), _p(kv), _p(k2), _p(v2), _p(out), T, heads, kv.shape[1], _p(seqs), len(lens), window, scale, softcap, _p(sink), _stream()))
+    return out
+
+
 def init_uniform(n, seed, scale, offset, device="cuda"):
     out = torch.empty(n, dtype=torch.bfloat16, device=device)
     check(lib().b200_op_init_uniform(_p(out), n, seed & 0xFFFFFFFF, scale, offset, _stream()))

@@ -457,15 +457,15 @@ int b200_op_paged_attn_decode_split(const void* q, int32_t ldq, void* out, int32
 int b200_op_paged_attn_prefill_tc(const void* qkv, int32_t q_rows, int32_t ldq, void* out, int32_t ldo, const void* kv_layer,
                                   const int32_t* block_tables, int32_t max_blocks, const int32_t* work, int32_t num_work,
                                   int32_t q_heads, int32_t kv_heads, float scale, void* stream);
-int b200_op_init_uniform(void* p, uint64_t n, uint32_t seed, float scale, float offset, void* stream);
-
-#ifdef __cplusplus
-}
-#endif
-#endif /* B200ENGINE_H */
 /* Attention of whole prompts (csrc/prompt_attention.cu): q [T, heads, 128] and kv [T, kv_heads, 128 of the key, 128 of the value] bf16, out [T, heads, 128];
  * with q2 [T, heads, 64], k2 [T, 64] (shared by the heads) and v2 [T, heads, 128] (the values' second terms; all three or none, kv_heads == heads then) keys of
  * 192 dimensions.  seqs: device int32[nseq][8], {first row, rows} of each sequence ahead of six zeros, in order and without gaps.  Causal; window (0: none) keys at
  * most, softcap (0: none) on the scores, sink fp32 [heads] or NULL.  A wait that ran out is reported by the next operation (b200_op_kernel_mark). */
 int b200_op_prompt_attn(const void* q, const void* q2, const void* kv, const void* k2, const void* v2, void* out, int32_t T, int32_t heads, int32_t kv_heads,
                         const int32_t* seqs, int32_t nseq, int32_t window, float scale, float softcap, const float* sink, void* stream);
+int b200_op_init_uniform(void* p, uint64_t n, uint32_t seed, float scale, float offset, void* stream);
+
+#ifdef __cplusplus
+}
+#endif
+#endif /* B200ENGINE_H */

@@ -429,13 +429,6 @@ int b200_op_paged_attn_prefill_tc(const void* qkv, int32_t q_rows, int32_t ldq, 
   return rc ? cuda_fail("paged_attention_prefill_tc", rc) : 0;
 }
 
-int b200_op_init_uniform(void* p, uint64_t n, uint32_t seed, float scale, float offset, void* stream) {
-  if (int rc = require_device()) return rc;
-  int rc = init_uniform(p, n, seed, scale, offset, static_cast<cudaStream_t>(stream));
-  return rc ? cuda_fail("init_uniform", rc) : 0;
-}
-
-}  // extern "C"
 int b200_op_prompt_attn(const void* q, const void* q2, const void* kv, const void* k2, const void* v2, void* out, int32_t T, int32_t heads, int32_t kv_heads,
                         const int32_t* seqs, int32_t nseq, int32_t window, float scale, float softcap, const float* sink, void* stream) {
   if (int rc = require_device()) return rc;
@@ -452,3 +445,10 @@ int b200_op_prompt_attn(const void* q, const void* q2, const void* kv, const voi
   return rc ? cuda_fail("prompt_attention", rc) : 0;
 }
 
+int b200_op_init_uniform(void* p, uint64_t n, uint32_t seed, float scale, float offset, void* stream) {
+  if (int rc = require_device()) return rc;
+  int rc = init_uniform(p, n, seed, scale, offset, static_cast<cudaStream_t>(stream));
+  return rc ? cuda_fail("init_uniform", rc) : 0;
+}
+
+}  // extern "C"

@@ -399,6 +399,10 @@ int b200_op_gemm_deferred(const void* w, const void* x, void* out, int32_t N, in
  * 4: silu(gate) up of the same rows.  B200_ERR_INVALID for sizes it does not serve.  w is read ahead of the kernel in front. */
 int b200_op_linear_rows(const void* x, const void* w, void* y, const float* bias, int32_t T, int32_t N, int32_t K, int32_t ldx, int32_t ldw,
                         int32_t ldy, int32_t y_f32, int32_t act, float p0, float p1, float p2, void* stream);
+/* Calls on several streams may run side by side where rows of out are whole 16-byte pieces (N a multiple of 8).  Everything else that meets in a workspace has one for all
+ * calls and is used on one stream at a time: b200_op_gemm for other N, b200_op_gemm_deferred, b200_op_gemm3 on its stream-K schedule (force < 0, or N of as many tiles as
+ * there are CTA pairs, which epi 2 with force 0 and up to 112 tokens mostly leaves to whole tiles), with the fused norm, with epi 4 or of more than 128 tokens, and
+ * b200_op_paged_attn_decode_split. */
 int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, int32_t K, void* stream);
 /* The decode-shape fused GEMM (T <= 128; csrc/gemm3_tcgen05.cu): acc = X' W^T with the split-K reduction finished in the
  * kernel, a prologue (pro 0: X' = x; 1: X' = RMSNorm(x) from the per-slab sums of squares ssq_in [T, ssq_slabs] and norm_w)
@@ -408,7 +412,8 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
  * out (the fused qkv buffer, ldo), k/v -> kv_layer pages; 4: argmax_out [T] = argmax_n acc[t, n < n_valid]).
  * force: 0 automatic schedule, 1..4 pairs per tile (cluster split-K through distributed shared memory), < 0 stream-K.
  * schedule_out (optional, 3 ints): pairs per tile, stream-K flag, CTAs launched.  epi 2 without a prologue and with force 0
- * takes b200_op_linear_rows's kernel where that serves the sizes and is ahead (B200_RULE_STREAM; no pairs per tile then). */
+ * takes b200_op_linear_rows's kernel where that serves the sizes and is ahead (B200_RULE_STREAM; no pairs per tile then), and for up to
+ * 112 tokens whole tiles where those are (one pair per tile or piece of K). */
 typedef struct {
   int32_t N, T, K, x_rows;
   int32_t pro, epi, force;

@@ -54,6 +54,13 @@ size_t g_ws_bytes = 0;
 int* g_counters = nullptr;
 int* g_mark = nullptr;   // pinned: a kernel whose wait ran out leaves a mark here
 constexpr int kCounterInts = 1 << 20;
+// Whole tiles whose K is cut meet in fp32 parts and counters, and calls on several streams run side by side: every stream has its own, the first
+// kStreams of them that ask (19 MB each; a stream's number is never given out again).  For more streams K stays whole.
+constexpr int kStreams = 32, kStreamCounters = 512;
+struct StreamParts { unsigned long long stream; float* ws; };
+StreamParts g_parts[kStreams];
+int g_nparts = 0;
+constexpr size_t kCounterBytes = (kCounterInts + static_cast<size_t>(kStreams) * kStreamCounters) * sizeof(int);   // for all calls, then the streams'
 
 int ensure_scratch() {
   std::lock_guard<std::mutex> lk(g_mu);
@@ -63,11 +70,43 @@ int ensure_scratch() {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   g_ws_bytes = std::max<size_t>(gemm_workspace_bytes(sms), 256ull << 20);
   if (cudaMalloc(&g_ws, g_ws_bytes) != cudaSuccess) return -1;
-  if (cudaMalloc(&g_counters, kCounterInts * sizeof(int)) != cudaSuccess) return -1;
-  cudaMemset(g_counters, 0, kCounterInts * sizeof(int));
+  if (cudaMalloc(&g_counters, kCounterBytes) != cudaSuccess) return -1;
+  if (cudaMemset(g_counters, 0, kCounterBytes) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) return -1;   // a stream need not wait for the default one
   if (cudaMallocHost(&g_mark, sizeof(int)) != cudaSuccess) return -1;
   *g_mark = 0;
   return 0;
+}
+
+// A stream that is being captured has no number to ask for, and its graph may run on any other: workspaces are for calls that run at once.
+bool captured(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+// The plan's workspace becomes the stream's own; false: it has none.
+bool stream_parts(cudaStream_t st, GemmPlan* plan) {
+  unsigned long long id = 0;
+  if (cudaStreamGetId(st, &id) != cudaSuccess) { cudaGetLastError(); return false; }
+  const size_t pairs = plan->max_ctas / 2, ws_bytes = pairs * 2 * 256 * 128 * sizeof(float);      // a pair has one item, of at most 256 rows
+  if (2 * pairs > kStreamCounters) return false;
+  std::lock_guard<std::mutex> lk(g_mu);
+  int i = 0;
+  while (i < g_nparts && g_parts[i].stream != id) ++i;
+  if (i == kStreams) return false;
+  if (i == g_nparts) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // in which memory can be had while another thread captures
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    float* ws = nullptr;
+    const bool ok = cudaMalloc(&ws, ws_bytes) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) { cudaGetLastError(); return false; }
+    g_parts[g_nparts++] = {id, ws};
+  }
+  plan->ws = g_parts[i].ws;
+  plan->ws_bytes = ws_bytes;
+  plan->counters = g_counters + kCounterInts + i * kStreamCounters;
+  return true;
 }
 
 // The operations return before their kernels have run, so one that gave up waiting is reported by the next: an error once, and
@@ -77,7 +116,8 @@ int report_mark() {
   volatile int* mark = g_mark;
   if (!*mark) return 0;
   cudaDeviceSynchronize();
-  cudaMemset(g_counters, 0, kCounterInts * sizeof(int));
+  cudaMemset(g_counters, 0, kCounterBytes);
+  cudaDeviceSynchronize();      // the next kernel's stream need not wait for this one
   *mark = 0;
   set_error("a wait inside the kernel of an earlier product ran out: its output is not valid");
   return B200_ERR_CUDA;
@@ -133,9 +173,17 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
     set_error("b200_op_gemm: problem too large for the op-level scratch");
     return B200_ERR_INVALID;
   }
-  CUtensorMap tmx[kGemmNumBlockN];
-  rc = gemm_make_x_maps(tmx, x, T, K, K);
-  if (rc) return cuda_fail("gemm_make_x_maps", rc);
+  if (gemm_variant() == 2 && gemm_whole_fits(plan, out, N)) {
+    // (a graph's parts lie in the workspace of all calls, as this operation's always did)
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    WholeTiles w = gemm_whole_tiles(plan, T, true);
+    if (w.parts > 1 && !captured(st) && !stream_parts(st, &plan)) w = gemm_whole_tiles(plan, T, false);
+    rc = gemm_whole_run(plan, x, T, K, w, T, {out, N}, st);
+    return rc ? cuda_fail("gemm_whole_run", rc) : 0;
+  }
+  CUtensorMap tmx[kGemmNumBlockN];      // of which the rest reads one
+  rc = gemm_make_x_map(&tmx[gemm_block_n_index(bn)], x, T, K, K, bn);
+  if (rc) return cuda_fail("gemm_make_x_map", rc);
   rc = gemm_run(plan, tmx, out, N, T, static_cast<cudaStream_t>(stream));
   if (rc) return cuda_fail("gemm_run", rc);
   return 0;
@@ -233,20 +281,21 @@ int b200_op_gemm3(const b200_gemm3_args* a, void* stream, int32_t* schedule_out)
       const int rs = linear_stream(la, &q, st);
       return rs ? cuda_fail("linear_stream", rs) : 0;
     }
-    // more of them: whole tiles, as the engine's steps take them (28672 x 4096, 16 to 96 tokens: 48.5 to 52 us on this kernel, 46 to 49 so).  A
-    // full tile of tokens keeps this kernel's schedule, of whose plain product its epilogues are bit by bit a function.
+    // more of them: whole tiles, as the engine's steps take them.  113 to 128 tokens, a full tile of this kernel, keep its schedule although the engine's do
+    // not: there this call promises the bits of its own plain product with the unit applied.
+    // Where K is cut and the stream has no workspace for it, this kernel's clusters, which need none.
     if (gemm_variant() == 2 && a->N % 256 == 0 && a->K % 64 == 0 && a->T <= 112 && a->ldo % 8 == 0 && reinterpret_cast<uintptr_t>(a->out) % 16 == 0) {
       if (const int rm = report_mark()) return rm;
       GemmPlan plan;
-      CUtensorMap tmx[kGemmNumBlockN];
-      int rw = gemm_plan_init(&plan, a->w, a->N, a->K, a->K, g_ws, g_counters, 0);
-      if (!rw) rw = gemm_make_x_maps(tmx, a->x, a->x_rows, a->K, a->K);
+      int rw = gemm_plan_init(&plan, a->w, a->N, a->K, a->K, nullptr, nullptr, 0);
+      if (rw) return cuda_fail("gemm_plan_init", rw);
       plan.error = g_mark;
-      plan.ws_bytes = g_ws_bytes;
-      const GroupedOut o = {a->out, a->ldo, GROUPED_SILU};
-      if (!rw) rw = gemm_whole_run(plan, tmx, a->T, o, st);
-      if (schedule_out) { schedule_out[0] = 1; schedule_out[1] = 0; schedule_out[2] = plan.max_ctas; }
-      return rw ? cuda_fail("gemm_whole_run", rw) : 0;
+      const WholeTiles w = gemm_whole_tiles(plan, a->T, true);
+      if (w.parts == 1 || (!captured(st) && stream_parts(st, &plan))) {
+        if (schedule_out) { schedule_out[0] = 1; schedule_out[1] = 0; schedule_out[2] = gemm_whole_ctas(plan, w, a->T); }
+        rw = gemm_whole_run(plan, a->x, a->x_rows, a->K, w, a->T, {a->out, a->ldo, GROUPED_SILU}, st);
+        return rw ? cuda_fail("gemm_whole_run", rw) : 0;
+      }
     }
   }
   Gemm3Schedule sch;

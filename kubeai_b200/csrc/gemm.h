@@ -37,8 +37,6 @@ size_t gemm_workspace_bytes(int max_ctas);
 int gemm_plan_init(GemmPlan* p, const void* W, int N, int K, int ldw, float* ws, int* counters, int max_ctas);
 // Activation map over X row-major [rows, K] (rows = buffer capacity), for a given token-tile size.
 int gemm_make_x_map(CUtensorMap* tm, const void* X, int rows, int K, int ldx, int block_n);
-// ... for all of them, tm[kGemmNumBlockN]
-int gemm_make_x_maps(CUtensorMap* tm, const void* X, int rows, int K, int ldx);
 // Generic 2-D bf16 tensor map (used by the attention kernel for the paged KV cache).
 int tmap_encode_bf16_2d(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, int box_rows,
                         int box_cols, int swizzle128);
@@ -100,6 +98,12 @@ int gemm_grouped_run(const GroupedPlan& p, const GroupedX& x, int most_rows, con
 // The same kernel on one matrix and `rows` rows, in whole tiles of 256 weight rows x up to 256 rows; few tiles are cut along K
 // (rules::whole_tiles).  x_maps: the activation's maps for all token-tile sizes, kGemmNumBlockN of them.
 int gemm_whole_run(const GemmPlan& p, const CUtensorMap* x_maps, int rows, const GroupedOut& o, cudaStream_t st);
+// ... in its two halves, for a caller that has no maps yet: the tiles that are chosen (cut: whether K may be cut), and the launch, which makes the one map
+// it reads of x_rows rows of X, ldx apart.
+struct WholeTiles { int tile, parts, box; };      // box: which of the kernel's
+WholeTiles gemm_whole_tiles(const GemmPlan& p, int rows, bool cut);
+int gemm_whole_ctas(const GemmPlan& p, const WholeTiles& w, int rows);
+int gemm_whole_run(const GemmPlan& p, const void* X, int x_rows, int ldx, const WholeTiles& w, int rows, const GroupedOut& o, cudaStream_t st);
 // whether a bf16 output of the plan's product can leave through it: N and ldo multiples of 8, out on a 16-byte boundary
 bool gemm_whole_fits(const GemmPlan& p, const void* out, int ldo);
 // ... with the choices made by the caller: box (16, 32, 64 or 128) is tm_x's, tile its rows per tile (a multiple of 16, at most

@@ -528,21 +528,40 @@ int gemm_grouped_run(const GroupedPlan& p, const GroupedX& x, int most_rows, con
   return launch(p.tm_w, p.experts, p.N, p.K, x.box[i], kBoxes[i], expert_rows, 0, o, {nullptr, nullptr, 1, 2 * kBoxes[i]}, sms / 2, error, st);
 }
 
+namespace {
+int whole_units(const GemmPlan& p, int tile, int parts, int rows) {
+  return static_cast<int>(std::min<long long>(p.max_ctas / 2, static_cast<long long>((p.N + 2 * kSlab - 1) / (2 * kSlab)) * ((rows + tile - 1) / tile) * parts));
+}
+}  // namespace
+
 int gemm_whole_run_as(const GemmPlan& p, const CUtensorMap& tm_x, int box, int tile, int parts, int rows, const GroupedOut& o, int* error, cudaStream_t st) {
   if (rows < 1 || tile < 1 || parts < 1 || parts > (p.K + kBlockK - 1) / kBlockK) return -1;
   const long long tiles = static_cast<long long>((p.N + 2 * kSlab - 1) / (2 * kSlab)) * ((rows + tile - 1) / tile);
   if (parts > 1 && (tiles * parts > p.max_ctas / 2 || tiles * parts * 2 * tile * kSlab * static_cast<long long>(sizeof(float)) > static_cast<long long>(p.ws_bytes) ||
                     !p.ws || !p.counters)) return -1;
-  const int units = static_cast<int>(std::min<long long>(p.max_ctas / 2, tiles * parts));
-  return launch(p.tm_w, 1, p.N, p.K, tm_x, box, nullptr, rows, o, {p.ws, p.counters, parts, tile}, units, error, st);
+  return launch(p.tm_w, 1, p.N, p.K, tm_x, box, nullptr, rows, o, {p.ws, p.counters, parts, tile}, whole_units(p, tile, parts, rows), error, st);
 }
+
+WholeTiles gemm_whole_tiles(const GemmPlan& p, int rows, bool cut) {
+  WholeTiles w = {16, 1, 0};
+  rules::whole_tiles(rows, p.N, p.K, p.max_ctas / 2, cut, &w.tile, &w.parts);
+  while (w.box + 1 < kGroupedBoxes && 2 * kBoxes[w.box] < w.tile) ++w.box;
+  return w;
+}
+
+int gemm_whole_ctas(const GemmPlan& p, const WholeTiles& w, int rows) { return 2 * whole_units(p, w.tile, w.parts, rows); }
 
 int gemm_whole_run(const GemmPlan& p, const CUtensorMap* x_maps, int rows, const GroupedOut& o, cudaStream_t st) {
   if (rows < 1) return 0;
-  int tile, parts, i = 0;      // (fp32 outputs have no split form)
-  rules::whole_tiles(rows, p.N, p.K, p.max_ctas / 2, o.epi != GROUPED_F32, &tile, &parts);
-  while (i + 1 < kGroupedBoxes && 2 * kBoxes[i] < tile) ++i;      // the maps of the four smallest token-tile sizes have these boxes
-  return gemm_whole_run_as(p, x_maps[i], kBoxes[i], tile, parts, rows, o, p.error, st);
+  const WholeTiles w = gemm_whole_tiles(p, rows, o.epi != GROUPED_F32);      // (fp32 outputs have no split form)
+  return gemm_whole_run_as(p, x_maps[w.box], kBoxes[w.box], w.tile, w.parts, rows, o, p.error, st);      // the maps of the four smallest token-tile sizes have these boxes
+}
+
+int gemm_whole_run(const GemmPlan& p, const void* X, int x_rows, int ldx, const WholeTiles& w, int rows, const GroupedOut& o, cudaStream_t st) {
+  CUtensorMap tm_x;
+  if (ldx % 8) return -5;
+  if (const int rc = tmap_encode_bf16_2d(&tm_x, X, x_rows, p.K, ldx, kBoxes[w.box], kBlockK, 1)) return rc;
+  return gemm_whole_run_as(p, tm_x, kBoxes[w.box], w.tile, w.parts, rows, o, p.error, st);
 }
 
 int gemm_whole_direct(const void* W, int ldw, const void* X, int ldx, int N, int K, int rows, const GroupedOut& o, int* error, cudaStream_t st) {

@@ -512,13 +512,6 @@ int gemm_make_x_map(CUtensorMap* tm, const void* X, int rows, int K, int ldx, in
   return make_tmap(tm, X, rows, K, ldx, gemm_x_box_rows(block_n));
 }
 
-int gemm_make_x_maps(CUtensorMap* tm, const void* X, int rows, int K, int ldx) {
-  constexpr int sizes[kGemmNumBlockN] = {32, 64, 128, 256, 512};
-  for (int i = 0; i < kGemmNumBlockN; ++i)
-    if (const int rc = gemm_make_x_map(tm + i, X, rows, K, ldx, sizes[i])) return rc;
-  return 0;
-}
-
 int gemm_run(const GemmPlan& p, const CUtensorMap* x_maps, void* out, int ldo, int T, cudaStream_t st) {
   if (T <= 0) return 0;
   if (g_variant == 2) return gemm2_run(p, x_maps, out, ldo, T, st);

@@ -379,8 +379,10 @@ int b200_attn_split_query(int32_t num_work, int32_t kv_heads, int32_t max_ctx, i
  * B200_RULE_LATENT_ROWS {longest row, tokens}: latent rows stay in registers between their sum and their norm.
  * B200_RULE_TILES {tokens, N, K}: a product that csrc/linear_stream.cu or csrc/linear_cluster.cu could take goes to whole tiles all the same.
  * B200_RULE_TILE_ROWS, B200_RULE_TILE_PARTS {rows, N, K, CTA pairs, K may be cut}: rows of a whole tile, and pieces K is cut into (numbers).
- * B200_RULE_DELTA_AHEAD {CTAs a sequence, sequences, tokens, longest, SMs}: delta-rule chunks whose scores are formed a chunk ahead by warps of their own. */
-enum { B200_RULE_PICKED_ALONE = 0, B200_RULE_KEY_LANES = 1, B200_RULE_STREAM = 2, B200_RULE_CLUSTER = 3, B200_RULE_SEGMENTS = 4, B200_RULE_ROW_REGISTERS = 5, B200_RULE_ROW_BLOCKS = 6, B200_RULE_SINGLE_STEP = 7, B200_RULE_LATENT_ROWS = 8, B200_RULE_TILES = 9, B200_RULE_TILE_ROWS = 10, B200_RULE_TILE_PARTS = 11, B200_RULE_DELTA_AHEAD = 12 };
+ * B200_RULE_DELTA_AHEAD {CTAs a sequence, sequences, tokens, longest, SMs}: delta-rule chunks whose scores are formed a chunk ahead by warps of their own.
+ * B200_RULE_GATE_UP {N, K, CTA pairs}: gate and up of up to 128 rows in whole tiles.
+ * B200_RULE_STEP_TILES {tokens, hidden}: projections of a Llama step of 9 to 128 tokens in whole tiles (1), with the rotation apart (2). */
+enum { B200_RULE_PICKED_ALONE = 0, B200_RULE_KEY_LANES = 1, B200_RULE_STREAM = 2, B200_RULE_CLUSTER = 3, B200_RULE_SEGMENTS = 4, B200_RULE_ROW_REGISTERS = 5, B200_RULE_ROW_BLOCKS = 6, B200_RULE_SINGLE_STEP = 7, B200_RULE_LATENT_ROWS = 8, B200_RULE_TILES = 9, B200_RULE_TILE_ROWS = 10, B200_RULE_TILE_PARTS = 11, B200_RULE_DELTA_AHEAD = 12, B200_RULE_GATE_UP = 13, B200_RULE_STEP_TILES = 14 };
 int b200_rule_query(int32_t rule, const int32_t* v, int32_t n);
 /* Debug: subsequent pair-GEMM launches write 8 clock64() phase stamps per CTA into trace_dev (int64[grid][8]);
  * NULL turns it off.  Stamps: 0 entry, 1 after prologue, 2 first tile accumulated, 3 main loop + partial stores
@@ -413,7 +415,7 @@ int b200_op_gemm(const void* w, const void* x, void* out, int32_t N, int32_t T, 
  * force: 0 automatic schedule, 1..4 pairs per tile (cluster split-K through distributed shared memory), < 0 stream-K.
  * schedule_out (optional, 3 ints): pairs per tile, stream-K flag, CTAs launched.  epi 2 without a prologue and with force 0
  * takes b200_op_linear_rows's kernel where that serves the sizes and is ahead (B200_RULE_STREAM; no pairs per tile then), and for up to
- * 112 tokens whole tiles where those are (one pair per tile or piece of K). */
+ * 112 tokens whole tiles where those are (B200_RULE_GATE_UP; one pair per tile or piece of K). */
 typedef struct {
   int32_t N, T, K, x_rows;
   int32_t pro, epi, force;

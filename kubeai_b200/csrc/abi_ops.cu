@@ -291,7 +291,7 @@ int b200_op_gemm3(const b200_gemm3_args* a, void* stream, int32_t* schedule_out)
       if (rw) return cuda_fail("gemm_plan_init", rw);
       plan.error = g_mark;
       const WholeTiles w = gemm_whole_tiles(plan, a->T, true);
-      if (w.parts == 1 || (!captured(st) && stream_parts(st, &plan))) {
+      if (rules::gate_up_tiles(a->N, a->K, plan.max_ctas / 2) && (w.parts == 1 || (!captured(st) && stream_parts(st, &plan)))) {
         if (schedule_out) { schedule_out[0] = 1; schedule_out[1] = 0; schedule_out[2] = gemm_whole_ctas(plan, w, a->T); }
         rw = gemm_whole_run(plan, a->x, a->x_rows, a->K, w, a->T, {a->out, a->ldo, GROUPED_SILU}, st);
         return rw ? cuda_fail("gemm_whole_run", rw) : 0;
@@ -372,6 +372,8 @@ int b200_rule_query(int32_t rule, const int32_t* v, int32_t n) {
   if (v && rule == B200_RULE_SINGLE_STEP && n == 5) return rules::single_step_pays(v[0], v[1], v[2], v[3] != 0, v[4]);
   if (v && rule == B200_RULE_LATENT_ROWS && n == 2) return rules::latent_rows_held(v[0], v[1]);
   if (v && rule == B200_RULE_DELTA_AHEAD && n == 5) return rules::delta_scores_ahead(v[0], v[1], v[2], v[3], v[4]);
+  if (v && rule == B200_RULE_GATE_UP && n == 3) return rules::gate_up_tiles(v[0], v[1], v[2]);
+  if (v && rule == B200_RULE_STEP_TILES && n == 2) return rules::step_tiles(v[0], v[1]) ? 1 + rules::rotation_apart(v[0]) : 0;
   if (v && rule == B200_RULE_TILES && n == 3) return rules::tiles_ahead(v[0], v[1], v[2]);
   if (v && (rule == B200_RULE_TILE_ROWS || rule == B200_RULE_TILE_PARTS) && n == 5 && v[0] > 0 && v[1] > 0 && v[2] > 0 && v[3] > 0) {
     int tile, parts;

@@ -145,6 +145,23 @@ inline void whole_tiles(int rows, int N, int K, int pairs, bool split, int* tile
   }
 }
 
+// Gate and up of up to 128 rows: whole tiles, or gemm3's pairs that share out the tiles' steps of K evenly.  Tiles are ahead by 10 to 30 % (28672 x 4096, 64 rows
+// 44.2 us in pairs / 41.7, 14336 x 4096 27.4 / 24.0) unless a few of them are left for a second round: those stream their K on few SMs, at 0.16 us a step, under
+// which the memory idles.  pairs / tiles of 74 pairs, 64 rows, us: 19456 x 8192 (76 tiles) 61.2 / 66.1, 20480 x 5120 (80) 1 / 1.04, 22016 x 8192 (86) 64.5 / 68.6,
+// 22016 x 5120 1 / 0.99, 22016 x 4096 1 / 0.95, 24576 x 8192 (96) 1 / 0.98, 19456 x 3072 1 / 1.03, 19456 x 2048 1 / 0.87; from the second full round on tiles again (38912 x
+// 8192, 152 tiles, 1 / 0.96).
+inline bool gate_up_tiles(int N, int K, int pairs) {
+  const int left = (N + 255) / 256 - pairs;
+  return left <= 0 || left >= pairs || (K + 63) / 64 * 0.16 + 1.2 - left * 512.0 * K / 6.3e6 <= 8.0;
+}
+
+// Llama steps of 9 to 128 tokens (engine.cu forward_fused): projections that are no passes over the weights as whole tiles with a norm or the rotation behind
+// them, or gemm3 with those in its epilogue.  What tiles cost is the weights and a launch each, where gemm3's exchange and its wait for all other clusters cost as much
+// again.  A step of 4 layers, gemm3 / tiles, us: Llama-3-8B sizes 9 tokens 401 / 391, 48 479 / 474, 49 506 / 487, 96 539 / 524, 128 579 / 537; 2048 wide 33 tokens
+// 266 / 251, 128 330 / 299; 1024 wide 49 to 64 tokens 204 / 209, 128 223 / 206.  The rotation apart pays from 65 tokens on.
+inline bool step_tiles(int tokens, int hidden) { return hidden >= 2048 || tokens <= 48 || tokens > 64; }
+inline bool rotation_apart(int tokens) { return tokens > 64; }
+
 // Latent rows (latent_attention.cu): in registers between their sum and their norm, or read again.  Registers for 1024 numbers a CTA cost room on
 // an SM, which short rows and many of them feel; longer rows do not fit.  rank: the longest row asked for, 0 where only queries are rotated.
 // us of two layers, again / held: ranks 1024 and 512, 8 tokens 21 / 17, 4096 43 / 38; 512 and 256, 8 18 / 16, 2400 27.8 / 26.4, 4096 34.3 / 36.3; 128 and

@@ -29,6 +29,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "dispatch_rules.h"
 #include "../../include/b200engine.h"
 #include "errors.h"
 #include "gemm.h"
@@ -990,11 +991,8 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     a.ldy = ldy;
     return a;
   };
-  // More tokens, up to 128: whole tiles whose rows are chosen for the step (gemm_grouped.cu) with a norm or the rotation behind them; what
-  // they cost is the weights and a launch each, where gemm3's exchange and its wait for all other clusters cost as much again.  A step of 4 layers,
-  // gemm3 / so, us: Llama-3-8B sizes 9 tokens 401 / 391, 48 479 / 474, 49 506 / 487, 96 539 / 524, 128 579 / 537; 2048 wide 33 tokens 266 / 251, 128
-  // 330 / 299; 1024 wide 49 to 64 tokens 204 / 209 (kept on gemm3), 128 223 / 206.  The rotation of qkv apart pays from 65 tokens on.
-  const bool tiles = few && whole_ok && (H >= 2048 || T <= 48 || T > 64);
+  // More tokens, up to 128: whole tiles whose rows are chosen for the step (gemm_grouped.cu) with a norm or the rotation behind them.
+  const bool tiles = few && whole_ok && rules::step_tiles(T, H), gu_tiles = tiles && rules::gate_up_tiles(2 * I, H, layers[0].p_gu.max_ctas / 2);
   bool x_pending = false;   // `x` holds a projection's output that the next RMSNorm still has to add to the residual
   for (int l = 0; l < L && !rc; ++l) {
     Layer& ly = layers[l];
@@ -1012,7 +1010,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     P(B200_K_GEMM_QKV);
     if (few && linear_few(qa, &pairs)) {
       if (on(B200_K_GEMM_QKV)) rc |= linear_stream(qa, &pairs, stream);
-    } else if (tiles && T > 64) {
+    } else if (tiles && rules::rotation_apart(T)) {
       if (on(B200_K_GEMM_QKV)) rc |= gemm_run(ly.p_qkv, xm_normed.m, qkv, QKV, T, stream);
       Q();
       P(B200_K_ROPE); if (on(B200_K_ROPE)) rc |= rope_kv_write(qkv, pos, slots, cos_sin, kv_l, T, Hq, Hkv, cfg.max_model_len, stream);
@@ -1047,7 +1045,7 @@ int Engine::forward_fused(const StepMeta& m, int32_t* dbuf) {
     P(B200_K_GEMM_GU);
     if (few && linear_few(ga, &unit)) {
       if (on(B200_K_GEMM_GU)) rc |= linear_stream(ga, &unit, stream);
-    } else if (tiles) {
+    } else if (gu_tiles) {
       const GroupedOut g = {act, I, GROUPED_SILU};
       if (on(B200_K_GEMM_GU)) rc |= gemm_whole_run(ly.p_gu, xm_normed.m, T, g, stream);
     } else {

@@ -145,3 +145,18 @@ def test_delta_scores_come_ahead_where_the_longest_chain_outlasts_the_work(ctas,
     """16 heads, 5 sequences of 777 tokens: 217 us two CTAs to an SM, 244 with more warps a CTA and one to an SM; 63 to 959 tokens in 8 sequences: 229 and 162."""
     assert rule(12, ctas, len(lens), sum(lens), max(lens), 148) == ahead
     assert rule(12, ctas, len(lens), sum(lens), 0, 148) == (sum(lens) > 64 and ctas * len(lens) <= 148)
+
+
+GATE_UP, STEP_TILES = 13, 14
+
+
+@pytest.mark.parametrize("N,K,tiles", [(28672, 4096, 1), (14336, 4096, 1), (18944, 8192, 1), (19456, 8192, 0), (19456, 4096, 0), (19456, 2048, 1), (20480, 5120, 0), (22016, 8192, 0), (22016, 4096, 1),
+                                       (24576, 8192, 1), (37888, 8192, 1), (38912, 8192, 1), (57344, 8192, 1), (256, 64, 1)])
+def test_few_gate_and_up_tiles_left_for_a_second_round_stay_with_the_pairs(N, K, tiles):
+    """19456 x 8192 is 76 tiles on 74 pairs, 64 rows: 66 us in two rounds, 61 where the pairs share out the steps of K."""
+    assert rule(GATE_UP, N, K, 74) == tiles
+
+
+@pytest.mark.parametrize("tokens,hidden,form", [(9, 1024, 1), (48, 1024, 1), (49, 1024, 0), (64, 1024, 0), (65, 1024, 2), (49, 2048, 1), (64, 2048, 1), (65, 4096, 2), (128, 4096, 2)])
+def test_projections_of_a_step(tokens, hidden, form):
+    assert rule(STEP_TILES, tokens, hidden) == form

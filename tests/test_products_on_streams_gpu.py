@@ -70,7 +70,7 @@ def test_captured(kind, T, N, K, warm):
         assert ((out.double() - want.double()).norm() / want.double().norm()).item() < 2.0 ** -8
 
 
-@pytest.mark.parametrize("T,N,K,kind", [(64, 28672, 4096, "tiles"), (33, 19456, 2048, "tiles"), (64, 2048, 4096, "tiles"), (112, 1024, 512, "tiles"), (113, 1024, 512, "gemm3")])
+@pytest.mark.parametrize("T,N,K,kind", [(64, 28672, 4096, "tiles"), (33, 19456, 4096, "stream-K"), (33, 19456, 2048, "tiles"), (64, 2048, 4096, "tiles"), (112, 1024, 512, "tiles"), (113, 1024, 512, "gemm3")])
 def test_schedule_that_is_reported(T, N, K, kind):
     from kubeai_b200 import ops
     x, w = torch.randn(T, K, device="cuda").to(torch.bfloat16), (torch.randn(N, K, device="cuda") / K ** 0.5).to(torch.bfloat16)

@@ -124,7 +124,9 @@ inline bool single_step_pays(long long heads_times_sequences, int dim, int vdim,
 //   2048 x 2048   256 rows 16.2 / 10.5   1000 rows 17.0 / 12.1   3000 rows 27.0 / 22.0 (176)    2048 x 8192   512 31.8 / 23.6   3000 97.9 / 74.0
 //   4096 x 14336  256 rows 60.6 / 44.8   700 rows 77.1 / 63.2    2048 rows 190 / 178 (240)      6144 x 4096  1000 49.0 / 38.6   2048 83.7 / 78.4
 //   28672 x 4096  512 rows 123 / 109     1400 rows 271 / 259     8192 x 2048  700 rows 26.3 / 22.5, 1400 rows 35.9 / 37.3
-// split: whether K may be cut at all.  (Many rows never want the smallest tiles, which are not tried then.)
+// split: whether K may be cut at all.  (Many rows never want the smallest tiles, which are not tried then.)  Of choices within 2 % the fewest tiles, which read the
+// weights less often (fewest / best by the count of steps alone, us: 700 rows 11008 x 8192 92.0 / 101.3, 11008 x 14336 160 / 178, 19456 x 2048 44.5 / 49.7; 1000 rows
+// 19456 x 14336 401 / 432; 22016 x 2048 52.3 / 50.4); short K and up to 320 rows gain nothing (14336 x 1024, 600 rows 19.5 / 18.1; 28672 x 14336, 300 rows 278 / 240).
 inline void whole_tiles(int rows, int N, int K, int pairs, bool split, int* tile, int* parts) {
   const int KB = (K + 63) / 64, slabs = (N + 255) / 256;
   const double memory = 2.0 * N * K / 6.3e6;
@@ -137,19 +139,19 @@ inline void whole_tiles(int rows, int N, int K, int pairs, bool split, int* tile
     last = t;
     const long long tiles = static_cast<long long>(slabs) * ((rows + t - 1) / t);
     const double step = fmax(0.16, 0.036 + 0.00105 * t);
+    const bool fewer = rows > 320 && KB >= 32 && tiles > pairs;
     for (int p = 1; p == 1 || (split && tiles * p <= pairs && p * 8 <= KB); ++p) {
       const long long waves = (tiles * p + pairs - 1) / pairs;
       const double us = fmax(waves * ((KB + p - 1) / p * step + 1.2), memory) + (p > 1 ? 3.0 + t * (0.016 + 0.009 * p) : 0.0);
-      if (!*tile || us < best - 1e-9) { best = us; *tile = t; *parts = p; }
+      if (!*tile || us < best * (fewer ? 0.98 : 1.0) - 1e-9) { best = us; *tile = t; *parts = p; }
     }
   }
 }
 
 // Gate and up of up to 128 rows: whole tiles, or gemm3's pairs that share out the tiles' steps of K evenly.  Tiles are ahead by 10 to 30 % (28672 x 4096, 64 rows
 // 44.2 us in pairs / 41.7, 14336 x 4096 27.4 / 24.0) unless a few of them are left for a second round: those stream their K on few SMs, at 0.16 us a step, under
-// which the memory idles.  pairs / tiles of 74 pairs, 64 rows, us: 19456 x 8192 (76 tiles) 61.2 / 66.1, 20480 x 5120 (80) 1 / 1.04, 22016 x 8192 (86) 64.5 / 68.6,
-// 22016 x 5120 1 / 0.99, 22016 x 4096 1 / 0.95, 24576 x 8192 (96) 1 / 0.98, 19456 x 3072 1 / 1.03, 19456 x 2048 1 / 0.87; from the second full round on tiles again (38912 x
-// 8192, 152 tiles, 1 / 0.96).
+// which the memory idles.  Tiles' time over the pairs', 74 pairs, 64 rows: 19456 x 8192 (76 tiles, 66.1 us over 61.2) 1.08, x 5120 1.07, x 3072 1.03, x 2048 0.82; 20480 x 5120
+// (80) 1.04; 22016 x 8192 (86) 1.06, x 5120 0.99, x 4096 0.95; 24576 x 8192 (96) 0.98; from the second full round on tiles again (38912 x 8192, 152 tiles, 0.96).
 inline bool gate_up_tiles(int N, int K, int pairs) {
   const int left = (N + 255) / 256 - pairs;
   return left <= 0 || left >= pairs || (K + 63) / 64 * 0.16 + 1.2 - left * 512.0 * K / 6.3e6 <= 8.0;

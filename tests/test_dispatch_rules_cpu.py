@@ -160,3 +160,9 @@ def test_few_gate_and_up_tiles_left_for_a_second_round_stay_with_the_pairs(N, K,
 @pytest.mark.parametrize("tokens,hidden,form", [(9, 1024, 1), (48, 1024, 1), (49, 1024, 0), (64, 1024, 0), (65, 1024, 2), (49, 2048, 1), (64, 2048, 1), (65, 4096, 2), (128, 4096, 2)])
 def test_projections_of_a_step(tokens, hidden, form):
     assert rule(STEP_TILES, tokens, hidden) == form
+
+
+@pytest.mark.parametrize("rows,N,K,tile", [(700, 11008, 8192, 240), (700, 11008, 14336, 240), (1000, 19456, 14336, 256), (600, 14336, 1024, 128), (300, 28672, 14336, 112), (700, 2048, 8192, 112)])
+def test_of_choices_that_are_even_the_fewest_tiles(rows, N, K, tile):
+    """700 rows of 11008 x 14336: 129 tiles of 240 rows 160 us, 215 of 144 rows 178, although the busiest pair has fewer rows then."""
+    assert rule(TILE_ROWS, rows, N, K, 74, 1) == tile

@@ -37,6 +37,23 @@ def test_a_fed_step_that_ends_with_the_mark_set_fails(tmp_path, make):
 
 
 @pytest.mark.parametrize("make", [design, llama])
+def test_a_fed_step_that_fails_leaves_the_callers_memory_as_it_was(tmp_path, make):
+    import ctypes as C
+    from kubeai_b200._lib import FeedEntry
+    with make(tmp_path) as e:
+        rows = 60
+        out = np.full((rows, e.cfg.vocab), 7.0, dtype=np.float32)
+        tokens, want = (C.c_int32 * rows)(*range(rows)), (C.c_int32 * rows)(*range(rows))
+        entry = (FeedEntry * 1)()
+        entry[0].req_id = e.feed_open()
+        entry[0].n_tokens = entry[0].n_want = rows
+        entry[0].tokens, entry[0].want = tokens, want
+        e._l.b200_engine_kernel_mark(e._h, 1)
+        assert e._l.b200_feed_step(e._h, entry, 1, out.ctypes.data_as(C.POINTER(C.c_float)), out.size) < 0
+        assert (out == 7.0).all()
+
+
+@pytest.mark.parametrize("make", [design, llama])
 def test_a_scheduled_step_that_ends_with_the_mark_set_hands_out_no_token(tmp_path, make):
     with make(tmp_path) as e:
         r = e.submit([5, 6, 7], max_tokens=4)

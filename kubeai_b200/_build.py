@@ -9,6 +9,7 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -16,7 +17,9 @@ ROOT = Path(__file__).resolve().parent
 CSRC = ROOT / "csrc"
 LIB = ROOT / "lib" / "libb200engine.so"
 OBJ = ROOT / "lib" / "obj"
-FEED = ROOT / "_feed.so"      # the Python side's one native helper (csrc/pyfeed.cc)
+# The Python side's one native helper (csrc/pyfeed.cc).  It reads lists, tuples and arrays by the layouts of one interpreter, so its name says which:
+# another one does not find it and forms the entries with numpy.
+FEED = ROOT / ("_feed" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 SOURCES = [
     "gemm_tcgen05.cu",
@@ -75,7 +78,6 @@ def _nvcc() -> str:
 
 def _feed_flags():
     """Include flags of the Python helper; none where Python's or numpy's headers are not installed (engine.py works without it)."""
-    import sysconfig
     try:
         import numpy
     except ImportError:
@@ -95,14 +97,49 @@ def _digest(paths) -> str:
     return h.hexdigest()
 
 
+def _feed_digest(flags) -> str:
+    """What the helper was made from: its source, the entry it fills, the interpreter and the numpy whose layouts it knows."""
+    import numpy
+    h = hashlib.sha256(_digest([CSRC / "pyfeed.cc", ROOT.parent / "include" / "b200engine.h"]).encode())
+    h.update(" ".join([sys.version, numpy.__version__, *flags]).encode())
+    return h.hexdigest()
+
+
+def build_feed(force: bool = False) -> bool:
+    """Build the Python helper where it can be built; whether it is there.  Without it engine.py forms the entries with numpy, so a
+    compiler that fails is reported and no more."""
+    plain = FEED.with_name("_feed.so")      # a name that every interpreter takes for its own
+    if plain != FEED:
+        plain.unlink(missing_ok=True)
+    flags = _feed_flags()
+    if not flags:
+        return FEED.exists()
+    stamp = OBJ / "feed_digest.txt"
+    digest = _feed_digest(flags)
+    if not force and FEED.exists() and stamp.exists() and stamp.read_text() == digest:
+        return True
+    OBJ.mkdir(parents=True, exist_ok=True)
+    FEED.unlink(missing_ok=True)
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", *flags, str(CSRC / "pyfeed.cc"), "-o", str(FEED)]
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        failed = f"{r.stdout}\n{r.stderr}" if r.returncode else ""
+    except OSError as e:
+        failed = str(e)
+    if failed:
+        print(f"kubeai_b200: building {FEED.name} failed, entries will be formed by numpy:\n{failed}", file=sys.stderr)
+        return False
+    stamp.write_text(digest)
+    return True
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
+    build_feed(force)
     srcs = [CSRC / s for s in SOURCES if (CSRC / s).exists()]
-    feed_flags = _feed_flags()
-    deps = [CSRC / "pyfeed.cc"] + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [ROOT.parent / "include" / "b200engine.h"] + \
-        list((ROOT.parent / "cmd").glob("*.cc"))
+    deps = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [ROOT.parent / "include" / "b200engine.h"] + list((ROOT.parent / "cmd").glob("*.cc"))
     stamp = OBJ / "digest.txt"
     digest = _digest(srcs + deps)
-    if not force and LIB.exists() and (FEED.exists() or not feed_flags) and stamp.exists() and stamp.read_text() == digest:
+    if not force and LIB.exists() and stamp.exists() and stamp.read_text() == digest:
         return LIB
     OBJ.mkdir(parents=True, exist_ok=True)
     nvcc = _nvcc()
@@ -135,11 +172,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"building {name} failed:\n{r.stdout}\n{r.stderr}")
-    if feed_flags:
-        cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", *feed_flags, str(CSRC / "pyfeed.cc"), "-o", str(FEED)]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"building {FEED.name} failed:\n{r.stdout}\n{r.stderr}")
     stamp.write_text(digest)
     return LIB
 

@@ -87,3 +87,56 @@ def test_arrays_and_lists_give_the_same_entries():
     for odd in (np.arange(6, dtype=np.int32)[::2], toks[1].astype(">i4"), toks[1].astype(np.int64), toks[1]):
         assert fed([(5, toks[0], wants[0]), (np.int64(6), odd, wants[1])]) == [(5, toks[0].tolist(), None), (6, odd.tolist(), [2])]
     assert fed([(5, np.ones((3, 1), dtype=np.int32), wants[1])]) == [(5, [1, 1, 1], [2])]
+
+
+def helper():
+    """The native packing, where the headers it is built with are there."""
+    from kubeai_b200 import _build
+    if not _build._feed_flags():
+        pytest.skip("no headers of Python or numpy")
+    from kubeai_b200 import _feed
+    assert E._pack is _feed.pack
+    return _feed
+
+
+def test_the_native_packing_serves_int32_vectors_and_nothing_else():
+    pack = helper().pack
+    t, w = np.array([1, 2, 3], dtype=np.int32), np.array([0, 2], dtype=np.int32)
+    buf, rows = pack([(7, t, w), (8, t[:1], w[:0])])
+    assert isinstance(buf, bytearray) and rows == 2
+    for odd in ([(7, [1, 2, 3], w)], [(7, t, [0, 2])], ((7, t, w),), [[7, t, w]], [(np.int64(7), t, w)], [(True, t, w)], [(7, t.astype(np.int64), w)], [(7, t[::2], w)],
+                [(7, t.astype(">i4"), w)], [(7, t.reshape(1, 3), w)], [(7, t)], [(7, t, w), (8, t, w, w)], []):
+        assert pack(odd) is None, odd
+
+
+def test_the_native_packing_belongs_to_one_interpreter():
+    import sysconfig
+    from kubeai_b200 import _build
+    name = helper().__file__.rsplit("/", 1)[-1]
+    assert name == "_feed" + sysconfig.get_config_var("EXT_SUFFIX") != "_feed.so" and _build.FEED.name == name
+
+
+def test_another_numpy_or_interpreter_is_another_build(monkeypatch):
+    import sys
+    from kubeai_b200 import _build
+    a = _build._feed_digest(["-Ix"])
+    assert a == _build._feed_digest(["-Ix"]) != _build._feed_digest(["-Iy"])
+    with monkeypatch.context() as m:
+        m.setattr(np, "__version__", "0.1")
+        assert _build._feed_digest(["-Ix"]) != a
+    with monkeypatch.context() as m:
+        m.setattr(sys, "version", "2.7")
+        assert _build._feed_digest(["-Ix"]) != a
+
+
+def test_a_compiler_that_fails_costs_the_helper_and_no_more(monkeypatch, tmp_path, capsys):
+    from kubeai_b200 import _build
+    monkeypatch.setattr(_build, "OBJ", tmp_path / "obj")
+    monkeypatch.setattr(_build, "FEED", tmp_path / "_feed.x.so")
+    monkeypatch.setattr(_build, "_feed_flags", lambda: ["-no-such-flag"])
+    (tmp_path / "_feed.so").write_bytes(b"any interpreter would take this")
+    (tmp_path / "_feed.x.so").write_bytes(b"of another source")
+    assert _build.build_feed() is False and "formed by numpy" in capsys.readouterr().err
+    assert not list(tmp_path.glob("*.so"))
+    monkeypatch.setattr(_build, "_feed_flags", lambda: [])
+    assert _build.build_feed() is False

@@ -436,6 +436,9 @@ int b200_op_argmax(const void* logits, int32_t* out, int32_t S, int32_t V, int32
   return rc ? cuda_fail("argmax_rows", rc) : 0;
 }
 
+// no sequence is longer than its row of the block table
+static int most_keys(int32_t max_blocks) { return max_blocks > 0 && max_blocks <= 4096 ? max_blocks * 16 : 0; }
+
 int b200_op_paged_attn(const void* q, int32_t ldq, void* out, int32_t ldo, const void* kv_layer,
                        const int32_t* block_tables, int32_t max_blocks, const int32_t* work, int32_t num_work,
                        int32_t q_heads, int32_t kv_heads, float scale, int32_t decode, void* stream) {
@@ -443,7 +446,7 @@ int b200_op_paged_attn(const void* q, int32_t ldq, void* out, int32_t ldo, const
   static_assert(sizeof(AttnWork) == 16, "AttnWork is int32[4] on the wire");
   int rc = paged_attention(q, ldq, out, ldo, kv_layer, block_tables, max_blocks,
                            reinterpret_cast<const AttnWork*>(work), num_work, q_heads, kv_heads, scale, decode,
-                           static_cast<cudaStream_t>(stream));
+                           static_cast<cudaStream_t>(stream), nullptr, 1, most_keys(max_blocks));
   return rc ? cuda_fail("paged_attention", rc) : 0;
 }
 
@@ -466,7 +469,7 @@ int b200_op_paged_attn_decode_split(const void* q, int32_t ldq, void* out, int32
     ws_bytes = need;
   }
   int rc = paged_attention(q, ldq, out, ldo, kv_layer, block_tables, max_blocks, reinterpret_cast<const AttnWork*>(work), num_work,
-                           q_heads, kv_heads, scale, 1, static_cast<cudaStream_t>(stream), ws, split);
+                           q_heads, kv_heads, scale, 1, static_cast<cudaStream_t>(stream), ws, split, most_keys(max_blocks));
   return rc ? cuda_fail("paged_attention(split)", rc) : 0;
 }
 

@@ -30,6 +30,7 @@
 // tokens in 8 sequences: 229 us -> 162, 1024 tokens in one 211 -> 146, the same bits.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <stdlib.h>
 
 #include <atomic>
 
@@ -560,7 +561,8 @@ int launch(const DeltaArgs& a, cudaStream_t st) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const dim3 grid((a.vdim + kCols - 1) / kCols, a.heads, a.nseq);
-  if (rules::delta_scores_ahead(grid.x * grid.y, a.nseq, a.T, a.max_rows, sms)) return launch_form<NK, FULL, true>(a, grid, sms, st);
+  const char* e = getenv("B200_DELTA_AHEAD");     // A/B knob: 0 = never, 1 = always
+  if (e ? atoi(e) != 0 : rules::delta_scores_ahead(grid.x * grid.y, a.nseq, a.T, a.max_rows, sms)) return launch_form<NK, FULL, true>(a, grid, sms, st);
   return launch_form<NK, FULL, false>(a, grid, sms, st);
 }
 template <int NK>

@@ -584,8 +584,8 @@ class Dabodra : public Model {
   }
 
   // ------------------------------------------------------------ forward
-  // Y = X W^T.  Steps of up to 16 tokens stream the weights through linear.cu's fragment kernel, steps of up to 256 tokens take
-  // the stream-K pair GEMM (every weight byte once, all pairs busy), larger ones whole tiles.
+  // Y = X W^T.  Steps of up to 16 tokens stream the weights through linear.cu's fragment kernel, larger ones take whole tiles (up
+  // to 256 tokens by way of gemm_run, which keeps the stream-K pair GEMM for rows that are no whole 16-byte pieces).
   // The grouped kernel on one matrix: whole 256 x 256 tiles, the accumulator drained under the next tile.
   bool takes_whole(bool tc, int T) const { return tc && T > 256 && whole; }
   int run_whole(const GemmPlan& plan, const CUtensorMap* xm, bool glu, void* Y, int ldy, int T) {

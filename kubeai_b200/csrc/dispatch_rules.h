@@ -44,7 +44,8 @@ inline bool stream_pays(int T, int N, int K, bool pairs) {
   if (pairs) return T <= 24;
   return T <= 16 || (T <= 32 ? K <= 16384 || N >= 2048 : N >= 4096);
 }
-// clusters, 49 .. 256 tokens:
+// clusters, 49 .. 256 tokens, over tiles as large as can be.  tiles_ahead below leaves them less than these lines do, which so decide only for outputs that are no
+// whole 16-byte pieces:
 //   K 4096   N 1024 .. 2112 0.67 .. 0.83, 2560 .. 3168 0.77 .. 0.91     K 8192   0.73 .. 0.93, 0.93 .. 1.08
 //   K 14336  0.83 .. 1.08 (to 128 tokens), 1.0 .. 1.12 (129 on); 1.08 .. 1.19     K 28672  1.12 .. 1.52, 1.28 .. 1.42
 inline bool cluster_pays(int T, int N, int K) { return K <= (N > 2112 ? 6144 : T <= 128 ? 16384 : 10240); }

@@ -26,6 +26,7 @@
 #include "gemm.h"
 #include "launch.h"
 #include "ptx.cuh"
+#include "umma2.cuh"
 
 namespace b200 {
 
@@ -35,7 +36,6 @@ constexpr int kSlab = 128;   // weight rows per CTA (UMMA M = 256 per pair)
 constexpr int kBlockK = 64;
 constexpr int kThreads = 192;
 constexpr int kABytes = kSlab * kBlockK * 2;
-constexpr uint32_t kPeerMask = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address -> rank 0's copy
 
 template <int BLOCK_N>
 struct Cfg2 {
@@ -70,9 +70,6 @@ __host__ __device__ __forceinline__ int hybrid_dp_waves(int tiles_total, int uni
   if (tail != 0 && tail < units) w = 0;
   return w;
 }
-__device__ __forceinline__ long long range_begin(int unit, long long total, int units) {
-  return (static_cast<long long>(unit) * total) / units;
-}
 __device__ __forceinline__ int unit_of_iter(long long x, long long total, int units) {
   return static_cast<int>(((x + 1) * units + total - 1) / total - 1);
 }
@@ -81,74 +78,8 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// 2-D TMA load into OWN smem, completion bytes credited to the LEADER CTA's mbarrier.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void* tmap, uint32_t bar, int32_t c0,
-                                                 int32_t c1, uint64_t hint) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar & kPeerMask), "r"(c0), "r"(c1), "l"(hint)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc2(uint32_t dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish2() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// D[tmem, 256 x N over the pair] (+)= A[256 x 16] * B[N x 16]; issued by the leader CTA only.
-// A 64-wide step of K from 128-byte swizzled K-major tiles: four products, 32 bytes apart along K; the first adds to what D holds
-// only with `accumulate`.
-__device__ __forceinline__ void umma2_bf16_k64(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p, t;\n"
-      ".reg .b64 a, b;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "setp.eq.u32 t, 0, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "add.s64 a, %1, 2;\n"
-      "add.s64 b, %2, 2;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
-      "add.s64 a, %1, 4;\n"
-      "add.s64 b, %2, 4;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
-      "add.s64 a, %1, 6;\n"
-      "add.s64 b, %2, 6;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, t;\n"
-      "}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Completion of all prior MMAs of this thread arrives on the same-offset mbarrier of BOTH CTAs.
-__device__ __forceinline__ void umma2_commit_both(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t cta) {
-  asm volatile(
-      "{\n"
-      ".reg .b32 ra;\n"
-      "mapa.shared::cluster.u32 ra, %0, %1;\n"
-      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n"
-      "}\n" ::"r"(bar),
-      "r"(cta)
-      : "memory");
-}
+__device__ __forceinline__ void umma2_commit_both(uint32_t bar) { umma2_commit_pair(bar, 3); }
 
 template <int BLOCK_N>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
@@ -243,7 +174,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     tmem_relinquish2();
   }
   tc_fence_before();
-  cluster_sync();  // barrier inits + TMEM allocation visible to the peer CTA
+  cluster_sync_all();  // barrier inits + TMEM allocation visible to the peer CTA
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   griddep_launch();
@@ -423,7 +354,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
           __syncwarp();
           if (lane == 0) {
             if (leader) mbar_arrive(tempty_bar(acc));
-            else mbar_arrive_remote(tempty_bar(acc), 0);
+            else mbar_arrive_cluster_relaxed(tempty_bar(acc), 0);
           }
           __threadfence();
           asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -474,7 +405,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
           __syncwarp();
           if (lane == 0) {
             if (leader) mbar_arrive(tempty_bar(acc));
-            else mbar_arrive_remote(tempty_bar(acc), 0);
+            else mbar_arrive_cluster_relaxed(tempty_bar(acc), 0);
           }
         }
         if (++acc == C::kAccStages) {
@@ -569,7 +500,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
       __syncwarp();
       if (lane == 0) {
         if (leader) mbar_arrive(tempty_bar(acc));
-        else mbar_arrive_remote(tempty_bar(acc), 0);
+        else mbar_arrive_cluster_relaxed(tempty_bar(acc), 0);
       }
       if (!complete && !deferred) {
         __threadfence();
@@ -701,7 +632,7 @@ gemm2_streamk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     mark(6);
   }
   tc_fence_before();
-  cluster_sync();  // neither CTA may exit (or free TMEM) while the peer can still signal its barriers / read its smem
+  cluster_sync_all();  // neither CTA may exit (or free TMEM) while the peer can still signal its barriers / read its smem
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc2(tmem_base, C::kTmemCols);

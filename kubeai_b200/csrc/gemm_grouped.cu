@@ -36,7 +36,7 @@ namespace {
 typedef __nv_bfloat16 bf16;
 constexpr int kSlab = 128;      // weight rows per CTA
 constexpr int kRows = 256;      // rows of X per tile, at most; TMEM columns of one accumulator
-constexpr int kBlockK = 64, kUmmaK = 16;
+constexpr int kBlockK = 64;
 // A warp that loads, one that issues the products, and one or two groups of four that drain a tile's rows in turns.  Two where
 // the drain of one group outlasts the next tile's products: gated units with the accurate functions (4096 tokens, 16 experts of 4096 x
 // 2048, two a token: 133 us with one group, 122 with two; one such matrix for all 70 and 58; of 500 tokens with K cut, 27 and 21) and

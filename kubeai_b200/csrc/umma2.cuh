@@ -1,6 +1,6 @@
 // Inline-PTX helpers for CTA-pair kernels (tcgen05 cta_group::2) inside thread-block clusters: pair TMA loads that signal
 // the leader's mbarrier, multicast commits, remote mbarrier arrives, DSMEM bulk copies, gpu-scope flag loads / stores.
-// Shared by gemm3_tcgen05.cu and chain_tcgen05.cu.
+// Shared by the kernels of CTA pairs and clusters.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

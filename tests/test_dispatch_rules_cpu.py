@@ -166,3 +166,12 @@ def test_projections_of_a_step(tokens, hidden, form):
 def test_of_choices_that_are_even_the_fewest_tiles(rows, N, K, tile):
     """700 rows of 11008 x 14336: 129 tiles of 240 rows 160 us, 215 of 144 rows 178, although the busiest pair has fewer rows then."""
     assert rule(TILE_ROWS, rows, N, K, 74, 1) == tile
+
+
+def test_clusters_have_whole_tiles_to_beat_only_in_short_products():
+    """What tiles_ahead leaves the clusters (49 rows on, where the passes end) is all theirs; cluster_pays draws its own lines for outputs that are no whole 16-byte pieces."""
+    for T in range(49, 257):
+        for N in (8, 1024, 2112, 2120, 3168, 4096):
+            for K in (512, 2048, 6144, 6208, 8192, 14336):
+                if not rule(TILES, T, N, K):
+                    assert T <= 128 and N <= 2112 and K <= 6144 and rule(CLUSTER, T, N, K) == 1

@@ -675,8 +675,8 @@ class Dabodra : public Model {
     d.dt_bias = w.dt_b; d.rate = w.rate;
     d.q_scale = 1.0f / sqrtf(static_cast<float>(s.dim)); d.unit_eps = kUnitEps;
     d.states = r.state; d.seqs = b.seqs; d.nseq = b.nseq; d.T = b.T;
-    d.heads = s.heads; d.kv_heads = s.kv_heads; d.dim = s.dim; d.vdim = s.vdim; d.o = o32; d.max_rows = b.max_rows;
-    KRN("delta_scan", delta_scan(d, st));
+    d.heads = s.heads; d.kv_heads = s.kv_heads; d.dim = s.dim; d.vdim = s.vdim; d.o = o32;
+    KRN("delta_scan", delta_scan(d, st, b.max_rows));
     OutGateArgs og = {};
     og.o = o32; og.g = col(inb, s.off_g); og.ldg = s.n_in; og.w = w.o_norm; og.eps = eps;
     og.y = yb; og.ldy = s.k_out; og.t = dt; og.T = b.T; og.heads = s.heads; og.vdim = s.vdim;

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kStepWarps * 32) delta_step_kernel(DeltaArgs a
 
 }  // namespace
 
-int delta_scan(const DeltaArgs& a, cudaStream_t st) {
+int delta_scan(const DeltaArgs& a, cudaStream_t st, int max_rows) {
   if (a.nseq <= 0 || a.T <= 0) return 0;
   if (!a.qkv || !a.beta_pre || !a.dt_pre || !a.dt_bias || !a.rate || !a.states || !a.seqs || !a.o || a.heads < 1 || a.kv_heads < 1 ||
       a.heads % a.kv_heads || a.dim < 1 || a.vdim < 1) return -1;
@@ -267,7 +267,7 @@ int delta_scan(const DeltaArgs& a, cudaStream_t st) {
     // steps that bring portions (B200_DELTA_CHUNK: A/B knob, the mean portion from which the chunked form runs; 0 = never)
     const char* e = getenv("B200_DELTA_CHUNK");
     const int from = e ? atoi(e) : 8;
-    if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return delta_chunk(a, st);
+    if (from > 0 && a.T >= static_cast<long long>(from) * a.nseq) return delta_chunk(a, st, max_rows);
   }
   // B200_SCAN_STEP: A/B knob, 0 = single tokens stay in the scan, 1 = never there where the pass takes their sizes.  fp32 models stay there,
   // whose outputs are promised to be the same bits however a sequence was cut into steps

@@ -27,7 +27,8 @@
 // What bounds it: a chain as long as the longest sequence on a CTA a head and 64 columns, tensor cores (mma.sync) two thirds of a chunk.  A sixth of their
 // products and most of the rest of a chunk's time go into A, its inverses and the weighted scores, which need no state: where the longest chain outlasts the
 // SMs' work (rules::delta_scores_ahead), four more warps form them a chunk ahead; the longest sequences' CTAs start first.  16 heads of 128 x 128, 63 to 959
-// tokens in 8 sequences: 229 us -> 162, 1024 tokens in one 211 -> 146, the same bits.
+// tokens in 8 sequences: 235 us -> 161, 1000 tokens in one 196 -> 141, the same bits.  (Registers decide: what the kernel is given says nothing it does not read.  With
+// one number more in DeltaArgs the compiler spilled 536 bytes for 296 in the form of four warps, 3 to 5 % of its time, and 296 for 72 in the other.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -81,11 +82,9 @@ constexpr int kPairs = 6;
 __device__ __forceinline__ constexpr int pair_a(int i) { return i == 0 ? 2 : (i == 1 ? 0 : (i == 2 ? 1 : (i == 3 ? 1 : 0))); }
 __device__ __forceinline__ constexpr int pair_b(int i) { return i == 0 ? 0 : (i == 1 ? 2 : (i == 2 ? 1 : (i == 3 ? 0 : (i == 4 ? 1 : 0)))); }
 
-// The sequence with the z-th most tokens (ties: the first), by a warp: long chains start first, and short ones fill in behind or beside them.  Of more
-// sequences than kSorted the z-th as they come.
+// The sequence with the z-th most tokens (ties: the first) of at most kSorted, by a warp: long chains start first, and short ones fill in behind or beside them.
 constexpr int kSorted = 64;
 __device__ __forceinline__ int nth_longest(const int* seqs, int nseq, int z) {
-  if (nseq > kSorted) return z;
   const int lane = threadIdx.x & 31, a = lane < nseq ? seqs[lane * 8 + 1] : -1, b = lane + 32 < nseq ? seqs[(lane + 32) * 8 + 1] : -1;
   int ra = 0, rb = 0;      // how many come before the lane's two
   for (int i = 0; i < min(nseq, 32); ++i) {
@@ -101,7 +100,7 @@ __device__ __forceinline__ int nth_longest(const int* seqs, int nseq, int z) {
 // loops over them without branches.  AHEAD: four more warps form the next chunk's A, inverses and weighted scores, which need no state, while the
 // first four work on this one's; a CTA then has its SM to itself.
 template <int NK, bool FULL, bool AHEAD>
-__global__ void __launch_bounds__(AHEAD ? 2 * kThreads : kThreads, AHEAD ? 1 : 2) delta_chunk_kernel(DeltaArgs a, int sms) {
+__global__ void __launch_bounds__(AHEAD ? 2 * kThreads : kThreads, AHEAD ? 1 : 2) delta_chunk_kernel(DeltaArgs a, int sms, bool by_length) {
   using namespace frag;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int NKB = k_bufs(AHEAD), NQB = q_bufs(AHEAD), NSB = s_bufs(AHEAD), kAll = AHEAD ? 2 * kThreads : kThreads;
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(AHEAD ? 2 * kThreads : kThreads, AHEAD ? 1 : 2
   float* diag = reinterpret_cast<float*>(Mbuf + NSB * kBlocks * 3 * kBlock);   // [4][16][kLdD]
   Gates* gates = reinterpret_cast<Gates*>(diag + 4 * 16 * kLdD);       // [NKB]
   float* ikbuf = reinterpret_cast<float*>(gates + NKB);   // [NSB][2][kQ] 1 / |k_t|, q_scale / |q_t|
-  const int seq = nth_longest(a.seqs, a.nseq, blockIdx.z), head = blockIdx.y, p0 = blockIdx.x * kCols;
+  const int seq = by_length ? nth_longest(a.seqs, a.nseq, blockIdx.z) : blockIdx.z, head = blockIdx.y, p0 = blockIdx.x * kCols;
   const int tok0 = a.seqs[seq * 8 + 0], n = a.seqs[seq * 8 + 1], pos0 = a.seqs[seq * 8 + 2], slot = a.seqs[seq * 8 + 3];
   // later row blocks have more scores: every other wave of CTAs deals them to the warps in the opposite order, so that the two
   // CTAs of an SM load its four schedulers evenly
@@ -550,23 +549,25 @@ __global__ void __launch_bounds__(AHEAD ? 2 * kThreads : kThreads, AHEAD ? 1 : 2
 }
 
 template <int NK, bool FULL, bool AHEAD>
-int launch_form(const DeltaArgs& a, dim3 grid, int sms, cudaStream_t st) {
+int launch_form(const DeltaArgs& a, dim3 grid, int sms, int max_rows, cudaStream_t st) {
   static std::atomic<unsigned long long> attr{0};
   if (!ensure_dynamic_smem(delta_chunk_kernel<NK, FULL, AHEAD>, static_cast<int>(chunk_smem(16 * NK, AHEAD)), &attr)) return -2;
-  delta_chunk_kernel<NK, FULL, AHEAD><<<grid, AHEAD ? 2 * kThreads : kThreads, chunk_smem(a.dim, AHEAD), st>>>(a, sms);
+  // in order of length where some have to wait, and wait for longer than the order costs (about 2 us a CTA)
+  const bool by_length = a.nseq <= kSorted && static_cast<long long>(grid.x) * grid.y * a.nseq > (AHEAD ? sms : 2 * sms) && static_cast<long long>(max_rows) * a.nseq - a.T >= 64ll * a.nseq;
+  delta_chunk_kernel<NK, FULL, AHEAD><<<grid, AHEAD ? 2 * kThreads : kThreads, chunk_smem(a.dim, AHEAD), st>>>(a, sms, by_length);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 template <int NK, bool FULL>
-int launch(const DeltaArgs& a, cudaStream_t st) {
+int launch(const DeltaArgs& a, int max_rows, cudaStream_t st) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const dim3 grid((a.vdim + kCols - 1) / kCols, a.heads, a.nseq);
   const char* e = getenv("B200_DELTA_AHEAD");     // A/B knob: 0 = never, 1 = always
-  if (e ? atoi(e) != 0 : rules::delta_scores_ahead(grid.x * grid.y, a.nseq, a.T, a.max_rows, sms)) return launch_form<NK, FULL, true>(a, grid, sms, st);
-  return launch_form<NK, FULL, false>(a, grid, sms, st);
+  if (e ? atoi(e) != 0 : rules::delta_scores_ahead(grid.x * grid.y, a.nseq, a.T, max_rows, sms)) return launch_form<NK, FULL, true>(a, grid, sms, max_rows, st);
+  return launch_form<NK, FULL, false>(a, grid, sms, max_rows, st);
 }
 template <int NK>
-int launch(const DeltaArgs& a, cudaStream_t st) { return a.dim == 16 * NK ? launch<NK, true>(a, st) : launch<NK, false>(a, st); }
+int launch(const DeltaArgs& a, int max_rows, cudaStream_t st) { return a.dim == 16 * NK ? launch<NK, true>(a, max_rows, st) : launch<NK, false>(a, max_rows, st); }
 
 }  // namespace
 
@@ -575,10 +576,10 @@ bool delta_chunk_fits(const DeltaArgs& a) {
          a.v_off % 8 == 0 && reinterpret_cast<uintptr_t>(a.qkv) % 16 == 0;
 }
 
-int delta_chunk(const DeltaArgs& a, cudaStream_t st) {
+int delta_chunk(const DeltaArgs& a, cudaStream_t st, int max_rows) {
   if (!delta_chunk_fits(a)) return -1;
-  if (a.dim <= 32) return launch<2>(a, st);
-  return a.dim <= 64 ? launch<4>(a, st) : launch<8>(a, st);
+  if (a.dim <= 32) return launch<2>(a, max_rows, st);
+  return a.dim <= 64 ? launch<4>(a, max_rows, st) : launch<8>(a, max_rows, st);
 }
 
 }  // namespace b200

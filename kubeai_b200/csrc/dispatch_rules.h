@@ -85,9 +85,9 @@ inline bool segments_pay(long long T, int nseq, int longest, int heads, int bloc
 // rest.  us, by itself / ahead, 128 x 128 (CTAs a sequence: twice the heads): 16 heads, 63 to 959 tokens in 8 sequences (work 14.7 chunks an SM, longest 15)
 // 229 / 162, 4 x 1000 and 500 (15.7, 16) 238 / 172, 5 x 777 (13.7, 13) 217 / 244, 8 x 200 (6.3, 4) 82 / 98; 32 heads, the 8 sequences (29.4, 15) 256 / 305,
 // 100 to 2000 in six (20, 32) 440 / 307; 2 x 1000: 4 heads 213 / 148, 37 (148 CTAs) 223 / 172, 40 (17.4, 16) 264 / 299, 74 (32, 16) 283 / 330.  64 and 32 rows
-// the same.  A step of one chunk has nothing ahead.  longest 0: not known.
+// the same.  Sequences of one chunk have nothing ahead (40 of 17 tokens, 4 heads of 128 x 64 27 / 40).  longest 0: not known.
 inline bool delta_scores_ahead(int ctas, int nseq, int tokens, int longest, int sms) {
-  return tokens > 64 && (static_cast<long long>(ctas) * nseq <= sms || (tokens / 64.0 + nseq / 2.0) * ctas / sms <= (longest + 63) / 64);
+  return (longest > 0 ? longest : tokens) > 64 && (static_cast<long long>(ctas) * nseq <= sms || (tokens / 64.0 + nseq / 2.0) * ctas / sms <= (longest + 63) / 64);
 }
 
 // Norms between sublayers (hyper.cu): a row of 256 threads times `pieces` of four columns in registers through both sums, or read from

@@ -248,13 +248,13 @@ struct DeltaArgs {
   float* states; const int* seqs; int nseq; int T;
   int heads, kv_heads, dim, vdim;
   float* o;
-  int max_rows = 0;   // most tokens that a sequence brings (0: not known)
 };
-int delta_scan(const DeltaArgs& a, cudaStream_t st);
+// max_rows: most tokens that a sequence brings (0: not known)
+int delta_scan(const DeltaArgs& a, cudaStream_t st, int max_rows = 0);
 // The chunked tensor-core form of the same scan (delta_chunk.cu; same result up to fp32 rounding), for the shapes it takes;
 // delta_scan chooses it for bf16 steps of prompt portions.
 bool delta_chunk_fits(const DeltaArgs& a);
-int delta_chunk(const DeltaArgs& a, cudaStream_t st);
+int delta_chunk(const DeltaArgs& a, cudaStream_t st, int max_rows);
 
 // ---------------------------------------------------------------- latent attention (latent_attention.cu)
 // Rotation table for interleaved pairs (2i, 2i+1): cs[p][i] = (cos, sin)(p * base^(-2i/dims)), computed in double.

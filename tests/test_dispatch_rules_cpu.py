@@ -140,7 +140,7 @@ def test_every_choice_of_tiles_can_be_launched():
 @pytest.mark.parametrize("ctas,lens,ahead", [
     (32, [63, 191, 319, 447, 575, 703, 831, 959], 1), (64, [63, 191, 319, 447, 575, 703, 831, 959], 0), (32, [1000] * 4 + [500], 1), (32, [777] * 5, 0), (32, [200] * 8, 0),
     (64, [100, 200, 100, 2000, 300, 80], 1), (8, [1000, 1000], 1), (74, [1000, 1000], 1), (80, [1000, 1000], 0), (148, [1000, 1000], 0), (128, [100, 3000], 1), (32, [64], 0),
-    (32, [65], 1), (1, [1], 0)])
+    (32, [65], 1), (1, [1], 0), (8, [17] * 40, 0), (8, [64] * 40, 0), (4, [64] * 8, 0), (4, [65] * 8, 1)])
 def test_delta_scores_come_ahead_where_the_longest_chain_outlasts_the_work(ctas, lens, ahead):
     """16 heads, 5 sequences of 777 tokens: 217 us two CTAs to an SM, 244 with more warps a CTA and one to an SM; 63 to 959 tokens in 8 sequences: 229 and 162."""
     assert rule(12, ctas, len(lens), sum(lens), max(lens), 148) == ahead

@@ -66,9 +66,15 @@ struct Segments {
   float *s, *d;
 };
 
+// CTAs an SM is to hold: what shared memory allows with the registers that leaves.  Up to 32 state rows segments live on them: 64 heads of 64 x 16, one sequence of 2000
+// tokens, 71 us with four and three of them, 56 so; 64 x 32 76 and 60.
+__host__ __device__ constexpr int ctas_per_sm(int nk, int part) {
+  return part == PART_SUMS ? (nk == 2 ? 6 : 4) : part == PART_OUT ? (nk == 2 ? 4 : 3) : nk == 2 ? 3 : 2;
+}
+
 // NK: state rows in units of 16, at most (N = a.dim is any multiple of 16 up to 16 NK)
 template <int NK, int PART>
-__global__ void __launch_bounds__(kThreads, PART == PART_SUMS ? 4 : PART == PART_OUT || NK == 2 ? 3 : 2) scalar_decay_chunk_kernel(GlaArgs a, Segments sg) {
+__global__ void __launch_bounds__(kThreads, ctas_per_sm(NK, PART)) scalar_decay_chunk_kernel(GlaArgs a, Segments sg) {
   using namespace frag;
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int NB = buffers_for(PART);

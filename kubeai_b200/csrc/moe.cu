@@ -233,6 +233,8 @@ __global__ void __launch_bounds__(128) moe_route_few_kernel(const float* scores,
 // Single CTA: a pair's rank among its expert's from a count that the lanes of a warp with the same expert raise together, padded
 // offsets, scatter.  What bounds it is one SM's latencies in a row, so a thread has its pairs' loads under way at once and meets the counts
 // once.  16 experts, 48 pairs: 4.2 us with a count and a place per pair and one thread that laid out the tiles, 3.1 now; 8192 pairs take 10 as before.
+// More pairs than its threads hold are counted and placed one by one: lanes that look for their like take a turn for each expert among them (64 experts, 8192 tokens,
+// 32 choices: 500 us so, 221 one by one).
 __global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, int pairs, int top, int E, int* sorted_rows, int* tile_group,
                                                          int* pair_pos, int cap, int* expert_rows, const float* topk_w, float* sorted_w, int matrices) {
   extern __shared__ int sh[];   // count[E], start[E]
@@ -242,8 +244,9 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, in
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
   griddep_launch();
   griddep_wait();
-  constexpr int U = 8;          // pairs a thread holds; with more than that in all, ranks wait in pair_pos
+  constexpr int U = 8;          // pairs a thread holds
   const int held = U * 1024;
+  const bool many = pairs > held;
   int id[U], rank[U];
   auto load_ids = [&](int p0) {
 #pragma unroll
@@ -260,14 +263,14 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, in
     if (p0) load_ids(p0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (p0 + u * 1024 < pairs) {
+      if (many) {
+        if (id[u] >= 0) atomicAdd(&count[id[u]], 1);
+      } else if (u * 1024 < pairs) {
         const unsigned same = __match_any_sync(0xffffffffu, id[u]);
         const int leader = __ffs(same) - 1;
         int before = 0;
         if (lane == leader && id[u] >= 0) before = atomicAdd(&count[id[u]], __popc(same));
         rank[u] = __shfl_sync(0xffffffffu, before, leader) + __popc(same & ((1u << lane) - 1));
-        const int p = p0 + u * 1024 + threadIdx.x;
-        if (pairs > held && p < pairs) pair_pos[p] = rank[u];
       }
     }
   }
@@ -292,13 +295,14 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* topk_ids, in
   __syncthreads();
   for (int e = threadIdx.x >> 5; e < E && e < matrices; e += 32)     // an expert without matrices: its tiles are skipped
     for (int i = lane; i < (count[e] + 63) / 64; i += 32) tile_group[start[e] / 64 + i] = e;
+  if (many) __syncthreads();    // the starts become the experts' next free rows
   for (int p0 = 0; p0 < pairs; p0 += held) {
-    if (pairs > held) load_ids(p0);
+    if (many) load_ids(p0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int p = p0 + u * 1024 + threadIdx.x;
       if (p < pairs) {
-        const int r = start[id[u]] + (pairs > held ? pair_pos[p] : rank[u]);
+        const int r = many ? atomicAdd(&start[id[u]], 1) : start[id[u]] + rank[u];
         sorted_rows[r] = p / top;
         pair_pos[p] = r;
         if (sorted_w) sorted_w[r] = topk_w[p];

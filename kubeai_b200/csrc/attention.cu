@@ -51,7 +51,7 @@ constexpr int attn_smem_bytes() {
 // four fit (three with two tiles; 128 sequences of up to 64 tokens, 8 heads: 12.3 us, 10.9 with one tile, its pages alone and one lane of a
 // whole warp issuing).
 template <bool DECODE, int S>
-__global__ void __launch_bounds__(128, S == 1 ? 4 : 0)
+__global__ void __launch_bounds__(128, S == 1 ? 4 : 1)
 paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16* __restrict__ q, int ldq,
                   __nv_bfloat16* __restrict__ out, int ldo, const int* __restrict__ block_tables, int max_blocks,
                   const AttnWork* __restrict__ work, int Hkv, float scale_log2, float* __restrict__ split_ws) {

@@ -49,7 +49,7 @@ constexpr int attn_smem_bytes() {
 
 // S = tiles in flight per CTA.  One where no sequence has more: then what bounds a step of many short sequences is how many CTAs an SM holds, and
 // four fit (three with two tiles; 128 sequences of up to 64 tokens, 8 heads: 12.3 us, 10.9 with one tile, its pages alone and one lane of a
-// whole warp issuing).
+// whole warp issuing).  The other forms' bound of one is no limit but the better code: 16 x 4000 tokens 75.8 us, 77.8 without it.
 template <bool DECODE, int S>
 __global__ void __launch_bounds__(128, S == 1 ? 4 : 1)
 paged_attn_kernel(const __grid_constant__ CUtensorMap tm_kv, const __nv_bfloat16* __restrict__ q, int ldq,
